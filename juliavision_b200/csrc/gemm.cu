@@ -940,6 +940,8 @@ int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, 
     if (!tc) {
         B200_REQUIRE(N < 65536 && nbatch < 65536, B200_DECLINE_EXTENT,
                      "gemm: unaligned operands with N or nbatch >= 65536");
+        if (gemm_rows_takes(M, N, K, nbatch))
+            return gemm_rows_launch(ctx, M, N, K, A, lda, B, ldb, bias, bias_per_n, out, ldo, out_dtype, epilogue);
         dim3 grid((unsigned)cdiv(M, 128), (unsigned)N, (unsigned)nbatch), block(128);
         if (out_dtype == B200_F16)
             gemm_f16_scalar_kernel<__half><<<grid, block, 0, ctx->stream>>>(

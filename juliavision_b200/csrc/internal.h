@@ -117,6 +117,11 @@ int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, 
                  int epilogue, int64_t nbatch, int64_t strideA, int64_t strideB, int64_t strideO,
                  int use_workspace = 1);
 
+// GEMM over operands a tensor map cannot express, from a few tens of thousands of elements of A up (gemm_rows.cu).
+bool gemm_rows_takes(int64_t M, int64_t N, int64_t K, int64_t nbatch);
+int gemm_rows_launch(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda, const void* B, int64_t ldb,
+                     const void* bias, int bias_per_n, void* out, int64_t ldo, int out_dtype, int epilogue);
+
 inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // Launch with the programmatic-serialization attribute (and a cluster width when > 1).  Only

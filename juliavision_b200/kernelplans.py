@@ -30,8 +30,9 @@ class MMTilePlan:
 
 @dataclass(frozen=True)
 class MMScalarPlan:
-    """fp16 operands a tensor map cannot express (unaligned leading dimension or pointer): the
-    one-thread-per-output kernel with mm2's arithmetic (matmul.jl:17-28), still on the GPU."""
+    """fp16 operands a tensor map cannot express (unaligned leading dimension or pointer), still on the GPU: from
+    32 k elements of A up the warp-level tensor-core kernel that reads A at any alignment, below that the
+    one-thread-per-output kernel with mm2's arithmetic (matmul.jl:17-28)."""
     reason: str
 
 

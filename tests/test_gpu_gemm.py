@@ -78,6 +78,37 @@ def test_unaligned_operands_take_the_scalar_kernel_bit_exact(ctx, ora):
     assert np.array_equal(got, ora.linear(X, Wt, b, epi="relu"))
 
 
+# (tokens, out, K) with an odd `out`: one to eight token tiles and a second block of them, fewer columns than one step,
+# reductions split over a cluster or staged in several chunks, a leading dimension of the tokens off 8 elements
+UNALIGNED = [(2, 65, 512), (5, 4099, 1280), (8, 121, 640), (9, 1001, 72), (17, 1337, 712), (33, 57003, 16), (64, 1001, 1408),
+             (65, 333, 403), (130, 113, 2000), (7, 51865, 129)]
+
+
+@pytest.mark.parametrize("tokens,out,K", UNALIGNED)
+@pytest.mark.parametrize("out_dtype,epi", [(np.float16, "gelu"), (np.float32, "identity")])
+def test_unaligned_rows_on_the_tensor_cores(ctx, ora, tokens, out, K, out_dtype, epi):
+    """Operands no tensor map can express, from 32 k elements of A up: A and the output start one element into an
+    allocation whose neighbours hold NaN, so every column has its own offset from a 16-byte boundary."""
+    rng = np.random.default_rng(tokens + out + K)
+    X, Wt, b = _case(rng, tokens, out, K, scale=0.25)
+    pad = np.full(K * out + 16, np.nan, np.float16)
+    pad[1:1 + K * out] = Wt.reshape(-1)
+    base = ctx.toback(pad)
+    A = jv.DeviceArray(ctx, base.ptr + 2, np.float16, (out, K), owner=base)
+    es = np.dtype(out_dtype).itemsize
+    dest = ctx.allocate(out_dtype, out * tokens + 2)
+    ctx.fill_bytes(dest, 0xFF)
+    Y = jv.DeviceArray(ctx, dest.ptr + es, out_dtype, (out, tokens), owner=dest)
+    jv.matmul_(ctx, Y, A, ctx.toback(X), ctx.toback(b), epi=epi)
+    ctx.synchronize()
+    flat = dest.to_host()
+    got, ref = flat[1:-1].reshape(tokens, out), ora.linear(X, Wt, b, epi=epi, out_dtype=out_dtype)
+    assert np.isnan(flat[0]) and np.isnan(flat[-1]), "wrote outside the output"
+    # fp32 sums in another order: sqrt(K) eps32 against the sums' own size, one fp16 rounding step for fp16 results
+    tol = 2e-3 if out_dtype == np.float16 else 2e-5
+    assert relerr(got, ref) < tol, describe(got, ref, tol)
+
+
 def test_batched(ctx, ora):
     rng = np.random.default_rng(7)
     nb, m, k, n = 6, 70, 64, 136
