@@ -38,19 +38,28 @@ constexpr int ATT_TILE_BYTES = 128 * 128; // one swizzle atom of an operand tile
 //                              has pulled S into registers, and a tile's Q K'(j+1) is issued after its P V(j)
 //                              (the two tiles' chains interleave on the tensor core); K/V rings of 2 stages x 32 KB
 // The reference's own fused tiling is E = 72 padded to 80 (flash.jl:1149-1157, flashepad kernelplans.jl).
-template <int EP> struct AttCfg {
+// With an additive mask each tile also stages a block's 128 x 128 mask entries (BIAS_ROW_WORDS words per row, see
+// the softmax); at EP = 128 the room for it comes from the V ring, which keeps one stage: V(j+1) is asked for when
+// both tiles' P V(j) are done and needed a softmax later, more than a fetch takes.
+// A staged mask row: 128 entries.  Rows on 8-byte boundaries are copied and read 8 bytes at a time, 66 words apart
+// (an odd number of 8-byte units, so that a warp's 32 rows lie in all banks); others word by word, from the 4-byte
+// boundary at or one entry before the first, 65 words apart (odd, for the same reason).
+constexpr int BIAS_ROW_WORDS = 66;
+template <int EP, bool BIAS = false> struct AttCfg {
     static_assert(EP == 64 || EP == 128, "head dim is padded to one or two swizzle atoms");
     static constexpr int ATOMS = EP / 64;              // 16 KB atoms per operand tile
     static constexpr int NT = 2;                       // query tiles per CTA
-    static constexpr int KV_STAGES = EP == 64 ? 4 : 2;
+    static constexpr int K_STAGES = EP == 64 ? 4 : 2;
+    static constexpr int V_STAGES = EP == 64 ? 4 : (BIAS ? 1 : 2);
     static constexpr bool P_IN_S = EP == 128;          // P shares its tile's S columns (tensor memory is full otherwise)
     static constexpr int OP_BYTES = ATOMS * ATT_TILE_BYTES;   // one Q, K or V tile
     // shared-memory map, in 16 KB atoms
     static constexpr int T_Q = 0;                              // NT tiles
-    static constexpr int T_K = NT * ATOMS;                     // KV_STAGES tiles
-    static constexpr int T_V = T_K + KV_STAGES * ATOMS;        // KV_STAGES tiles
-    static constexpr int T_END = T_V + KV_STAGES * ATOMS;
-    static constexpr int SMEM_BYTES = T_END * ATT_TILE_BYTES + 256;
+    static constexpr int T_K = NT * ATOMS;                     // K_STAGES tiles
+    static constexpr int T_V = T_K + K_STAGES * ATOMS;         // V_STAGES tiles
+    static constexpr int T_END = T_V + V_STAGES * ATOMS;
+    static constexpr int BIAS_TILE_BYTES = BIAS ? ATT_BR * BIAS_ROW_WORDS * 4 : 0;
+    static constexpr int SMEM_BYTES = T_END * ATT_TILE_BYTES + NT * BIAS_TILE_BYTES + 256;
     static_assert(SMEM_BYTES <= 232448, "shared memory over budget");
 };
 // tensor-memory map (512 columns): S of tile t, fp32, at [128 t, 128 t + 128); O of tile t, fp32, at
@@ -63,7 +72,7 @@ constexpr int ATT_P_COL = 384;
 
 struct AttnParams {
     int E, Lq, Lk, H, B;
-    float scale_log2;   // scale * log2(e)
+    float scale, scale_log2;   // scale_log2 = scale * log2(e)
     void* out;
     int64_t osL, osH, osB;  // element strides of out along L, H, B (E is contiguous)
     int out_f32;
@@ -72,10 +81,11 @@ struct AttnParams {
     int* d_status;
     unsigned long long* trace;  // optional timeline of CTA (0,0,0) (globaltimer ns), null in normal use
     // Additive mask of the mem-efficient variant (attention.jl:55-59), (Lk,Lq,H,B) fp16 with element
-    // strides (0 on a broadcast axis); null when absent.  bias_vec: rows can be read 8 keys at a time.
+    // strides (0 on a broadcast axis); null when absent.
     const __half* bias;
     int64_t bsK, bsQ, bsH, bsB;
-    int bias_vec;
+    int bias_async;     // keys contiguous: the mask's blocks are copied to shared memory ahead of use, 1: by words,
+                        // 2: every row starts on an 8-byte boundary
     // Keys split over nsplit CTAs per query pair (few queries, many keys): each writes its unnormalised
     // fp32 O rows to part_o[split][tail pair][256 rows][E] and (reference point, row sum) to part_ml[...][2];
     // attention_merge_kernel combines them (the reference's attn_flash_cm_merge!, flash.jl:1398-1421).
@@ -116,6 +126,14 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -146,8 +164,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 1)
 attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                         const __grid_constant__ CUtensorMap tmapK,
                         const __grid_constant__ CUtensorMap tmapV, const AttnParams p) {
-    using Cfg = AttCfg<EP>;
-    constexpr int ATT_KV_STAGES = Cfg::KV_STAGES;
+    using Cfg = AttCfg<EP, BIAS>;
+    constexpr int K_STAGES = Cfg::K_STAGES, V_STAGES = Cfg::V_STAGES;
     constexpr int NT = Cfg::NT;
     constexpr int ITEM_ROWS = NT * ATT_BR;   // queries one whole work item covers
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -158,13 +176,13 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
         return;
     }
     auto tile_ptr = [&](int t) { return smem + t * ATT_TILE_BYTES; };
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::T_END * ATT_TILE_BYTES);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::T_END * ATT_TILE_BYTES + NT * Cfg::BIAS_TILE_BYTES);
     uint64_t* q_full = bars + 0;                           // [2]
-    uint64_t* k_full = bars + 2;                           // [STAGES]
-    uint64_t* k_empty = k_full + ATT_KV_STAGES;            // [STAGES]
-    uint64_t* v_full = k_empty + ATT_KV_STAGES;            // [STAGES]
-    uint64_t* v_empty = v_full + ATT_KV_STAGES;            // [STAGES]
-    uint64_t* s_full = v_empty + ATT_KV_STAGES;            // [2]
+    uint64_t* k_full = bars + 2;                           // [K_STAGES]
+    uint64_t* k_empty = k_full + K_STAGES;                 // [K_STAGES]
+    uint64_t* v_full = k_empty + K_STAGES;                 // [V_STAGES]
+    uint64_t* v_empty = v_full + V_STAGES;                 // [V_STAGES]
+    uint64_t* s_full = v_empty + V_STAGES;                 // [2]
     uint64_t* s_empty = s_full + 2;                        // [2]
     uint64_t* p_full = s_empty + 2;                        // [2]
     uint64_t* pv_done = p_full + 2;                        // [2]
@@ -212,9 +230,11 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             mbar_init(&pv_done[t], 1);
             mbar_init(&exp_turn[t], 4);
         }
-        for (int s = 0; s < ATT_KV_STAGES; ++s) {
+        for (int s = 0; s < K_STAGES; ++s) {
             mbar_init(&k_full[s], 1);
             mbar_init(&k_empty[s], ntiles);   // freed when every tile's issuer is done with it
+        }
+        for (int s = 0; s < V_STAGES; ++s) {
             mbar_init(&v_full[s], 1);
             mbar_init(&v_empty[s], ntiles);
         }
@@ -252,18 +272,18 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                     tma_load_4d(tile_ptr(Cfg::T_Q + t * Cfg::ATOMS + a), &tmapQ, &q_full[t], a * 64, q0 + t * ATT_BR, h, b);
             }
             for (int j = 0; j < nblk; ++j) {
-                const int s = j % ATT_KV_STAGES;
-                const uint32_t ph = (uint32_t)((j / ATT_KV_STAGES) & 1);
+                const int s = j % K_STAGES, sv = j % V_STAGES;
+                const uint32_t ph = (uint32_t)((j / K_STAGES) & 1), phv = (uint32_t)((j / V_STAGES) & 1);
                 if (!mbar_wait(&k_empty[s], ph ^ 1, p.d_status, KST_WAIT_EMPTY, abort_flag)) break;
                 mbar_arrive_expect_tx(&k_full[s], Cfg::OP_BYTES);
 #pragma unroll
                 for (int a = 0; a < Cfg::ATOMS; ++a)
                     tma_load_4d(tile_ptr(Cfg::T_K + s * Cfg::ATOMS + a), &tmapK, &k_full[s], a * 64, (jb0 + j) * ATT_BC, h, b);
-                if (!mbar_wait(&v_empty[s], ph ^ 1, p.d_status, KST_WAIT_EMPTY, abort_flag)) break;
-                mbar_arrive_expect_tx(&v_full[s], Cfg::OP_BYTES);
+                if (!mbar_wait(&v_empty[sv], phv ^ 1, p.d_status, KST_WAIT_EMPTY, abort_flag)) break;
+                mbar_arrive_expect_tx(&v_full[sv], Cfg::OP_BYTES);
 #pragma unroll
                 for (int a = 0; a < Cfg::ATOMS; ++a)
-                    tma_load_4d(tile_ptr(Cfg::T_V + s * Cfg::ATOMS + a), &tmapV, &v_full[s], a * 64, (jb0 + j) * ATT_BC, h, b);
+                    tma_load_4d(tile_ptr(Cfg::T_V + sv * Cfg::ATOMS + a), &tmapV, &v_full[sv], a * 64, (jb0 + j) * ATT_BC, h, b);
             }
         }
     } else if (warp == 9 || warp == 10) {
@@ -288,8 +308,8 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             const uint32_t p_tmem = Cfg::P_IN_S ? s_tmem : tmem_base + ATT_P_COL + t * 64;
 
             auto issue_qk = [&](int j) -> bool {
-                const int sk = j % ATT_KV_STAGES;
-                if (!mbar_wait(&k_full[sk], (uint32_t)((j / ATT_KV_STAGES) & 1), p.d_status, KST_WAIT_FULL, abort_flag))
+                const int sk = j % K_STAGES;
+                if (!mbar_wait(&k_full[sk], (uint32_t)((j / K_STAGES) & 1), p.d_status, KST_WAIT_FULL, abort_flag))
                     return false;
                 // With P in S's columns this product is issued after P V(j-1), which read P after the softmax had taken
                 // S(j-1), and UMMAs of one thread run in issue order: nothing else to wait for.
@@ -314,8 +334,8 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             if (ok && nblk > 0) ok = issue_qk(0);
             for (int j = 0; ok && j < nblk; ++j) {
                 if (!Cfg::P_IN_S && j + 1 < nblk && !issue_qk(j + 1)) break;
-                const int sv = j % ATT_KV_STAGES;
-                if (!mbar_wait(&v_full[sv], (uint32_t)((j / ATT_KV_STAGES) & 1), p.d_status, KST_WAIT_FULL, abort_flag)) break;
+                const int sv = j % V_STAGES;
+                if (!mbar_wait(&v_full[sv], (uint32_t)((j / V_STAGES) & 1), p.d_status, KST_WAIT_FULL, abort_flag)) break;
                 if (j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 7);   // issuer reaches its wait for P(j)
                 if (!mbar_wait(&p_full[t], (uint32_t)(j & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag)) break;
                 tc_fence_after();
@@ -343,8 +363,8 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             const uint32_t s_tmem = tmem_base + lane_base + ATT_S_COL + t * 128;
             const uint32_t o_tmem = tmem_base + lane_base + ATT_O_COL + t * EP;
             const uint32_t p_tmem = Cfg::P_IN_S ? s_tmem : tmem_base + lane_base + ATT_P_COL + t * 64;
-            const float sc = p.scale_log2;
-            const float sce = BIAS ? 1.0f : sc;   // with a bias the scores are rescaled when it is added
+            const float sc = BIAS ? p.scale : p.scale_log2;
+            const float sce = BIAS ? 1.4426950408889634f : sc;   // with a bias the scores are scaled when it is added
             float m_run = -INFINITY, l_run = 0.f;
             bool ok = true;
             // Both tiles take the same time per block, and left alone they fall into step: both
@@ -353,7 +373,47 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             // j+1, ...): while one tile owns the MUFU pipe the other does its max / rescale / waits
             // and its tensor-core work runs.
             const bool pingpong = ntiles == 2 && ATT_TURN_AT >= 0;
-
+            // The mask, when its keys are contiguous: each warp copies the next block's entries of its own 32 rows to
+            // shared memory (cp.async, a row's entries across the lanes) while it works on this block, and every thread
+            // then reads its row back.  Nothing but the warp itself is involved, so no barrier is.  Rows may start at
+            // any element: when not all of them lie on 8-byte boundaries (an odd number of keys puts every other row in
+            // the middle of a word) words are copied from the 4-byte boundary at or below a row's first entry and
+            // shifted when read.  Every piece copied holds an entry of the mask.  Read straight from global memory, one
+            // row per thread, 20 heads x 1500 x 1500 took 152 us, with words copied 56, with 8 bytes at a time 45 (24
+            // without a mask: adding it is 64 more packed FMAs, 128 conversions and the reads per thread and block).
+            uint32_t* bias_rows = reinterpret_cast<uint32_t*>(smem + Cfg::T_END * ATT_TILE_BYTES) + (t * ATT_BR + quad * 32) * BIAS_ROW_WORDS;
+            const bool bias_async = BIAS && p.bias != nullptr && p.bias_async;
+            const bool bias8 = BIAS && p.bias_async == 2;
+            auto bias_fetch = [&](int j) {
+                const int keys = min(ATT_BC, p.Lk - (jb0 + j) * ATT_BC);
+                const int rows = min(32, p.Lq - (q0 + t * ATT_BR + quad * 32));   // rows of this warp that exist
+                const char* src = reinterpret_cast<const char*>(p.bias + (int64_t)(q0 + t * ATT_BR + quad * 32) * p.bsQ +
+                                                                (int64_t)h * p.bsH + (int64_t)b * p.bsB + (int64_t)(jb0 + j) * ATT_BC);
+                const uint32_t dst = smem_u32(bias_rows);
+                if (bias8) {
+                    if (4 * lane < keys) {
+                        src += lane * 8;
+#pragma unroll 8
+                        for (int r = 0; r < rows; ++r, src += p.bsQ * 2) cp_async8(dst + lane * 8 + r * 264, src);
+                    }
+                } else {
+                    const char* s = src;
+#pragma unroll 4
+                    for (int r = 0; r < rows; ++r, s += p.bsQ * 2) {
+                        const int words = (keys + 1 + (int)((reinterpret_cast<uintptr_t>(s) >> 1) & 1)) >> 1;
+                        const char* a = reinterpret_cast<const char*>(reinterpret_cast<uintptr_t>(s) & ~(uintptr_t)3) + lane * 4;
+                        if (lane < words) cp_async4(dst + lane * 4 + r * 260, a);
+                        if (lane + 32 < words) cp_async4(dst + lane * 4 + r * 260 + 128, a + 128);
+                    }
+                    if (lane < rows) {   // a row's 65th word, when its 128 entries start in the middle of a word
+                        const uintptr_t a = reinterpret_cast<uintptr_t>(src) + (int64_t)lane * p.bsQ * 2;
+                        if ((a & 2) && keys == ATT_BC)
+                            cp_async4(dst + lane * 260 + 256, reinterpret_cast<const char*>((a & ~(uintptr_t)3) + 256));
+                    }
+                }
+                cp_async_commit();
+            };
+            if (bias_async) bias_fetch(0);
 
             for (int j = 0; ok && j < nblk; ++j) {
                 if (!mbar_wait(&s_full[t], (uint32_t)(j & 1), p.d_status, KST_WAIT_TMEM_FULL, abort_flag)) { ok = false; break; }
@@ -373,10 +433,8 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                 if (lane == 0 && quad == 0 && j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 3);  // S in registers
 
                 if constexpr (BIAS) {
-                    // r <- s * scale * log2(e) (+ bias * log2(e)): from here on the scores are in the
-                    // exponent's own units and the scale below is one.
+                    // r <- s * scale + bias: from here on the scores are in the mask's units and the scale below is log2(e).
                     const int lq = q0 + t * ATT_BR + row;
-                    const float L2E = 1.4426950408889634f;
                     if (p.bias == nullptr) {
 #pragma unroll
                         for (int c = 0; c < 4; ++c)
@@ -385,27 +443,51 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                     } else {
                         const __half* brow = p.bias + (int64_t)(lq < p.Lq ? lq : 0) * p.bsQ + (int64_t)h * p.bsH +
                                              (int64_t)b * p.bsB + (int64_t)(jb0 + j) * ATT_BC * p.bsK;
-                        if (p.bias_vec && nvalid >= ATT_BC) {
+                        if (bias_async) {
+                            cp_async_wait_all();
+                            __syncwarp();
+                            const uint64_t sc2b = pack2(sc, sc);
+                            // score * scale + mask for two keys: the mask's units, the exponent's factor follows later
+                            auto add = [&](int c, int i, uint32_t two) {
+                                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&two));
+                                float x0, x1;
+                                unpack2(fma2(pack2(__uint_as_float(r[c][2 * i]), __uint_as_float(r[c][2 * i + 1])), sc2b, pack2(f.x, f.y)),
+                                        x0, x1);
+                                r[c][2 * i] = __float_as_uint(x0);
+                                r[c][2 * i + 1] = __float_as_uint(x1);
+                            };
+                            if (bias8) {
+                                const uint2* w = reinterpret_cast<const uint2*>(bias_rows + lane * 66);
 #pragma unroll
-                            for (int c = 0; c < 4; ++c)
+                                for (int c = 0; c < 4; ++c)
 #pragma unroll
-                                for (int g = 0; g < 4; ++g) {
-                                    const uint4 w = __ldg(reinterpret_cast<const uint4*>(brow + c * 32 + g * 8));
-                                    const __half2* hh = reinterpret_cast<const __half2*>(&w);
-#pragma unroll
-                                    for (int u = 0; u < 4; ++u) {
-                                        const float2 f = __half22float2(hh[u]);
-                                        r[c][g * 8 + 2 * u] = __float_as_uint(fmaf(__uint_as_float(r[c][g * 8 + 2 * u]), sc, f.x * L2E));
-                                        r[c][g * 8 + 2 * u + 1] = __float_as_uint(fmaf(__uint_as_float(r[c][g * 8 + 2 * u + 1]), sc, f.y * L2E));
+                                    for (int i = 0; i < 16; i += 2) {
+                                        const uint2 four = w[c * 8 + i / 2];
+                                        add(c, i, four.x);
+                                        add(c, i + 1, four.y);
                                     }
-                                }
+                            } else {
+                                const uint32_t* w = bias_rows + lane * 65;
+                                const uint32_t shift = (uint32_t)(reinterpret_cast<uintptr_t>(brow) & 2) * 8;   // 16: the row starts mid-word
+                                uint32_t lo = w[0];
+#pragma unroll
+                                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                                    for (int i = 0; i < 16; ++i) {
+                                        const uint32_t hi = w[c * 16 + i + 1];
+                                        add(c, i, __funnelshift_r(lo, hi, shift));
+                                        lo = hi;
+                                    }
+                            }
+                            __syncwarp();   // every lane has read its row
+                            if (j + 1 < nblk) bias_fetch(j + 1);
                         } else {
 #pragma unroll
                             for (int c = 0; c < 4; ++c)
 #pragma unroll
                                 for (int i = 0; i < 32; ++i) {
                                     const float bv = (c * 32 + i < nvalid) ? __half2float(brow[(int64_t)(c * 32 + i) * p.bsK]) : 0.f;
-                                    r[c][i] = __float_as_uint(fmaf(__uint_as_float(r[c][i]), sc, bv * L2E));
+                                    r[c][i] = __float_as_uint(fmaf(__uint_as_float(r[c][i]), sc, bv));
                                 }
                         }
                     }
@@ -913,11 +995,11 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
         B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        AttCfg<64>::SMEM_BYTES));
         B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       AttCfg<64>::SMEM_BYTES));
+                                       AttCfg<64, true>::SMEM_BYTES));
         B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        AttCfg<128>::SMEM_BYTES));
         B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       AttCfg<128>::SMEM_BYTES));
+                                       AttCfg<128, true>::SMEM_BYTES));
         attr_done[ctx->device & 15] = true;
     }
     // Many windows of at most 64 keys: bound by HBM and latency, not by the tensor pipe; the small-tile
@@ -931,6 +1013,7 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     if ((rc = make_qkv_map(ctx, &tv, v, E, Lk, H, B))) return rc;
     AttnParams p;
     p.E = (int)E; p.Lq = (int)Lq; p.Lk = (int)Lk; p.H = (int)H; p.B = (int)B;
+    p.scale = scale;
     p.scale_log2 = scale * 1.4426950408889634f;
     p.out = out;
     p.osL = o->stride[1]; p.osH = o->stride[2]; p.osB = o->stride[3];
@@ -939,10 +1022,11 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     p.trace = ctx->gemm_trace;
     p.bias = bptr;
     p.bsK = bs[0]; p.bsQ = bs[1]; p.bsH = bs[2]; p.bsB = bs[3];
-    p.bias_vec = bptr && bs[0] == 1 && al16(bptr) && bs[1] % 8 == 0 && bs[2] % 8 == 0 && bs[3] % 8 == 0;
+    p.bias_async = !bptr || !(bs[0] == 1 || Lk == 1) ? 0 : 1 + (reinterpret_cast<uintptr_t>(bptr) % 8 == 0 && bs[1] % 4 == 0 && bs[2] % 4 == 0 && bs[3] % 4 == 0);
     const bool wide = E > 64;                              // two swizzle atoms along E
     const int64_t item_rows = wide ? AttCfg<128>::NT * ATT_BR : AttCfg<64>::NT * ATT_BR;
-    const size_t smem_bytes = wide ? AttCfg<128>::SMEM_BYTES : AttCfg<64>::SMEM_BYTES;
+    const size_t smem_bytes = wide ? (bptr ? AttCfg<128, true>::SMEM_BYTES : AttCfg<128>::SMEM_BYTES)
+                                   : (bptr ? AttCfg<64, true>::SMEM_BYTES : AttCfg<64>::SMEM_BYTES);
     auto launch = [&](dim3 grid) -> cudaError_t {
         if (wide)
             return bptr ? launch_dep(attention_f16_tc_kernel<128, true>, grid, dim3(ATT_THREADS, 1, 1), smem_bytes, ctx->stream, 1, tq, tk, tv, p)
@@ -963,7 +1047,7 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     p.part_o = p.part_ml = nullptr;
     const int64_t nblk_all = cdiv(Lk, ATT_BC);
     const int64_t rem = pairs % sms;
-    if (bptr == nullptr && nblk_all >= 4) {
+    if (nblk_all >= 4) {
         int64_t ntail = 0, ns = 1;
         if (2 * pairs <= sms) {
             ntail = pairs;

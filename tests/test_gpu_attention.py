@@ -336,3 +336,38 @@ def test_few_queries_many_keys_split_and_merged(ctx, ora, B, H, Lq, Lk, E):
         got, plan = attention_gpu(ctx, q, k, v, scale, out_dtype)
         assert isinstance(plan, jv.FlashTCPlan)
         assert relerr(got, ref) < TOL, describe(got, ref, TOL)
+
+
+# masked, keys contiguous: even and odd row strides of the mask (rows that start in the middle of a word), one key
+# more and less than a block, a mask wider than its rows, and shapes whose keys are split and merged
+MASKED = [((1, 2, 300, 1500, 64), (1, 1, 300, 1500), 0), ((1, 1, 257, 129, 64), (1, 1, 257, 129), 0),
+          ((1, 2, 129, 127, 72), (1, 2, 129, 127), 0), ((1, 1, 130, 1, 64), (1, 1, 130, 1), 0),
+          ((2, 2, 140, 383, 128), (2, 1, 140, 383), 3), ((1, 3, 3, 477, 64), (1, 1, 3, 477), 0),
+          ((1, 4, 23, 2049, 72), (1, 1, 23, 2049), 1), ((1, 2, 260, 1030, 96), (1, 1, 1, 1030), 0)]
+
+
+@pytest.mark.parametrize("shape,bshape,extra", MASKED)
+def test_masked_blocks_staged_ahead(ctx, ora, shape, bshape, extra):
+    B, H, Lq, Lk, E = shape
+    rng = np.random.default_rng(sum(shape) + extra)
+    q, k, v = (np.float16(rng.standard_normal((B, H, n, E))) for n in (Lq, Lk, Lk))
+    bias = np.float16(rng.standard_normal(bshape))
+    bias[rng.random(bshape) < 0.2] = -np.inf
+    bias[rng.random(bshape) < 0.1] = -65504
+    bias[..., -1, :Lk // 2] = -np.inf          # a row that has seen nothing after its first blocks (or split)
+    if bshape[2] > 2:
+        bias[..., 1, :] = -np.inf
+    wide = np.full(bshape[:3] + (Lk + extra,), np.nan, np.float16)      # the mask as a slice of a wider array
+    wide[..., :Lk] = bias
+    dq, dk, dv = (ctx.toback(a) for a in (q, k, v))
+    db = ctx.toback(wide).slice(0, 0, Lk)
+    out = ctx.allocate(np.float32, E, Lq, H, B)
+    ctx.fill_bytes(out, 0xFF)
+    ctx.ws.reset()
+    jv.sdpa(ctx, dq, dk, dv, db, 1 / np.sqrt(E), out=out)
+    ctx.synchronize()
+    got, ref = out.to_host(), ora.attention_ref(q, k, v, 1 / np.sqrt(E), bias=bias)
+    assert np.all(np.isfinite(got))
+    assert relerr(got, ref) < TOL, describe(got, ref, TOL)
+    if bshape[2] > 2:
+        assert np.all(got[:, :, 1] == 0)
