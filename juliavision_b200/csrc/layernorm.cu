@@ -7,6 +7,7 @@
 // group, shared-memory tree reductions and three strided passes over the group.
 #include <cuda_fp16.h>
 
+#include "act.cuh"
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -58,6 +59,8 @@ template <int N> __device__ __forceinline__ void store_vec(float* dst, const flo
         *reinterpret_cast<float4*>(dst + i) = make_float4(f[i], f[i + 1], f[i + 2], f[i + 3]);
 }
 
+constexpr int LN_WIDE_THREADS = 256;   // block of a row too wide for one warp
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -70,6 +73,65 @@ __device__ __forceinline__ float group_sum(float v) {
 #pragma unroll
     for (int o = LPG / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+// What every form of the warp kernel does with a row's elements once they are in registers, as packed fp32 pairs (one
+// instruction for two: at 65536 x 1280 the scalar form issued for about 25 us of the launch's 62, half of them in
+// these steps; 62.2 -> 58.1 us, 5.4 -> 5.8 TB/s).  The vectors of a lane are v = first, first + stride, ...; `x` is left holding x - mean after ln_moments.
+// One definition, so that the layer norm alone and the one behind a residual add give the same bits.
+__device__ __forceinline__ float pairs_sum(unsigned long long s2) {
+    float a, b;
+    act_detail::upk(s2, a, b);
+    return a + b;
+}
+template <int VPL, int VN, int LPG>
+__device__ __forceinline__ void ln_moments(unsigned long long (&x)[VPL][VN / 2], int first, int nvec, int C, float eps, float& mu,
+                                           float& r) {
+    using namespace act_detail;
+    unsigned long long s = pk(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < VPL; ++i)
+        if (first + 32 * i < nvec) {
+#pragma unroll
+            for (int j = 0; j < VN / 2; ++j) s = add2(s, x[i][j]);
+        }
+    const float n = (float)C;
+    mu = group_sum<LPG>(pairs_sum(s)) / n;
+    const unsigned long long nmu = pk(-mu, -mu);
+    unsigned long long s2 = pk(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < VPL; ++i)
+        if (first + 32 * i < nvec) {
+#pragma unroll
+            for (int j = 0; j < VN / 2; ++j) {
+                x[i][j] = add2(x[i][j], nmu);
+                s2 = fma2(x[i][j], x[i][j], s2);
+            }
+        }
+    r = 1.0f / sqrtf(group_sum<LPG>(pairs_sum(s2)) / n + eps);
+}
+// One vector of the result: d = x - mean; y = d r, then gamma and beta in one rounding where both are there.
+template <typename InT, typename OutT>
+__device__ __forceinline__ void ln_write(OutT* dst, const unsigned long long* d, float r, bool has_g, const uint4& g, bool has_b,
+                                         const uint4& b) {
+    using namespace act_detail;
+    constexpr int VN = Vec16<InT>::N;
+    Vec16<InT> tg, tb;
+    float gf[VN], bf[VN], y[VN];
+    tg.raw = g;
+    tb.raw = b;
+    if (has_g) tg.to_f32(gf);
+    if (has_b) tb.to_f32(bf);
+    const unsigned long long rr = pk(r, r);
+#pragma unroll
+    for (int j = 0; j < VN / 2; ++j) {
+        unsigned long long v = mul2(d[j], rr);
+        if (has_g && has_b) v = fma2(v, pk(gf[2 * j], gf[2 * j + 1]), pk(bf[2 * j], bf[2 * j + 1]));
+        else if (has_g) v = mul2(v, pk(gf[2 * j], gf[2 * j + 1]));
+        else if (has_b) v = add2(v, pk(bf[2 * j], bf[2 * j + 1]));
+        upk(v, y[2 * j], y[2 * j + 1]);
+    }
+    store_vec<VN>(dst, y);
 }
 
 // One warp per group; lane l owns vectors l, l+32, ... (VPL of them at most).  Narrow groups (at most
@@ -106,61 +168,35 @@ ln_warp_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
         }
     }
 
-    float x[VPL][VN];
-    float s = 0.f;
+    unsigned long long x[VPL][VN / 2];
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
-        int v = lane + 32 * i;
+        const int v = lane + 32 * i;
         if (v < nvec) {
             Vec16<InT> t;
+            float f[VN];
             t.raw = __ldg(reinterpret_cast<const uint4*>(src) + v);
-            t.to_f32(x[i]);
+            t.to_f32(f);
 #pragma unroll
-            for (int j = 0; j < VN; ++j) s += x[i][j];
+            for (int j = 0; j < VN / 2; ++j) x[i][j] = act_detail::pk(f[2 * j], f[2 * j + 1]);
         }
     }
-    const float n = (float)C;
-    const float mu = group_sum<LPG>(s) / n;
-    float s2 = 0.f;
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-        if (lane + 32 * i < nvec) {
-#pragma unroll
-            for (int j = 0; j < VN; ++j) {
-                float d = x[i][j] - mu;
-                s2 += d * d;
-            }
-        }
-    }
-    const float r = 1.0f / sqrtf(group_sum<LPG>(s2) / n + eps);
-
+    float mu, r;
+    ln_moments<VPL, VN, LPG>(x, lane, nvec, C, eps, mu, r);
     OutT* dst = out + g * (int64_t)C;
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
-        int v = lane + 32 * i;
+        const int v = lane + 32 * i;
         if (v < nvec) {
-            float y[VN];
-#pragma unroll
-            for (int j = 0; j < VN; ++j) y[j] = (x[i][j] - mu) * r;
-            if (gamma) {
-                Vec16<InT> t;
-                float gf[VN];
-                if constexpr (HOIST) t.raw = gw[i];
-                else t.raw = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
-                t.to_f32(gf);
-#pragma unroll
-                for (int j = 0; j < VN; ++j) y[j] *= gf[j];
+            uint4 gv = make_uint4(0u, 0u, 0u, 0u), bv = gv;
+            if constexpr (HOIST) {
+                gv = gw[i];
+                bv = bw[i];
+            } else {
+                if (gamma) gv = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
+                if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + v);
             }
-            if (beta) {
-                Vec16<InT> t;
-                float bf[VN];
-                if constexpr (HOIST) t.raw = bw[i];
-                else t.raw = __ldg(reinterpret_cast<const uint4*>(beta) + v);
-                t.to_f32(bf);
-#pragma unroll
-                for (int j = 0; j < VN; ++j) y[j] += bf[j];
-            }
-            store_vec<VN>(dst + (int64_t)v * VN, y);
+            ln_write<InT, OutT>(dst + (int64_t)v * VN, x[i], r, gamma != nullptr, gv, beta != nullptr, bv);
         }
     }
     if (lane == 0 && g < groups) {
@@ -203,8 +239,7 @@ ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half*
     __half* xr = x + g * (int64_t)C;
     const __half* hr = h + g * (int64_t)C;
 
-    float v[VPL][VN];
-    float s = 0.f;
+    unsigned long long v[VPL][VN / 2];
     // every load of the row first, then the arithmetic: one round trip for the row whatever the compiler would
     // have made of loads and stores through the same pointer
     // (the latency form; the lean one reads each vector where it uses it)
@@ -238,52 +273,29 @@ ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half*
             for (int j = 0; j < VN; ++j) {
                 float t = __half2float(__float2half_rn(fa[j] + fb[j]));        // add.Tensor rounds here
                 if (use_clamp) t = __half2float(__float2half_rn(fminf(fmaxf(t, lo), hi)));
-                v[i][j] = t;
-                s += t;
+                fa[j] = t;
             }
-            store_vec<VN>(xr + (int64_t)vi * VN, v[i]);                         // exact: already fp16 values
+            store_vec<VN>(xr + (int64_t)vi * VN, fa);                           // exact: already fp16 values
+#pragma unroll
+            for (int j = 0; j < VN / 2; ++j) v[i][j] = act_detail::pk(fa[2 * j], fa[2 * j + 1]);
         }
     }
-    const float n = (float)C;
-    const float mu = group_sum<LPG>(s) / n;
-    float s2 = 0.f;
-#pragma unroll
-    for (int i = 0; i < VPL; ++i)
-        if (lane + 32 * i < nvec) {
-#pragma unroll
-            for (int j = 0; j < VN; ++j) {
-                float d = v[i][j] - mu;
-                s2 += d * d;
-            }
-        }
-    const float r = 1.0f / sqrtf(group_sum<LPG>(s2) / n + eps);
+    float mu, r;
+    ln_moments<VPL, VN, LPG>(v, lane, nvec, C, eps, mu, r);
     __half* dst = out + g * (int64_t)C;
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
         const int vi = lane + 32 * i;
         if (vi < nvec) {
-            float y[VN];
-#pragma unroll
-            for (int j = 0; j < VN; ++j) y[j] = (v[i][j] - mu) * r;
-            if (gamma) {
-                Vec16<__half> t;
-                float gf[VN];
-                if constexpr (HOIST) t.raw = gw[i];
-                else t.raw = __ldg(reinterpret_cast<const uint4*>(gamma) + vi);
-                t.to_f32(gf);
-#pragma unroll
-                for (int j = 0; j < VN; ++j) y[j] *= gf[j];
+            uint4 gv = make_uint4(0u, 0u, 0u, 0u), bv = gv;
+            if constexpr (HOIST) {
+                gv = gw[i];
+                bv = bw[i];
+            } else {
+                if (gamma) gv = __ldg(reinterpret_cast<const uint4*>(gamma) + vi);
+                if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + vi);
             }
-            if (beta) {
-                Vec16<__half> t;
-                float bf[VN];
-                if constexpr (HOIST) t.raw = bw[i];
-                else t.raw = __ldg(reinterpret_cast<const uint4*>(beta) + vi);
-                t.to_f32(bf);
-#pragma unroll
-                for (int j = 0; j < VN; ++j) y[j] += bf[j];
-            }
-            store_vec<VN>(dst + (int64_t)vi * VN, y);
+            ln_write<__half, __half>(dst + (int64_t)vi * VN, v[i], r, gamma != nullptr, gv, beta != nullptr, bv);
         }
     }
     if (lane == 0 && g < groups) {
@@ -305,6 +317,79 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
     __syncthreads();
     float t = l < nw ? red[l] : 0.f;
     return warp_sum(t);
+}
+
+// Rows too wide for one warp's registers (more than 16 vectors per lane): one block per row, the row in registers as
+// above, the two sums over the block through shared memory.  Bound by HBM; with scalar accesses and the row read three
+// times these rows took 71 us for 7112 x 4280 in fp32, now 42.7 (5.7 TB/s); 79 x 3168 4.9 -> 2.9.
+template <typename InT, typename OutT, int VPT>
+__global__ void __launch_bounds__(LN_WIDE_THREADS)
+ln_wide_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restrict__ mean, float* __restrict__ rstd,
+               const InT* __restrict__ gamma, const InT* __restrict__ beta, int C, float eps) {
+    constexpr int VN = Vec16<InT>::N;
+    __shared__ float red[32];
+    const int64_t g = blockIdx.x;
+    const int nvec = C / VN, tid = threadIdx.x;
+    const uint4* src = reinterpret_cast<const uint4*>(a + g * (int64_t)C);
+    grid_dep_wait();     // the input is the previous kernel's output
+    grid_dep_launch();
+    Vec16<InT> raw[VPT];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+        if (tid + LN_WIDE_THREADS * i < nvec) raw[i].raw = __ldg(src + tid + LN_WIDE_THREADS * i);
+    float x[VPT][VN];
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+        if (tid + LN_WIDE_THREADS * i < nvec) {
+            raw[i].to_f32(x[i]);
+#pragma unroll
+            for (int j = 0; j < VN; ++j) s += x[i][j];
+        }
+    const float n = (float)C;
+    const float mu = block_sum(s, red) / n;
+    float s2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+        if (tid + LN_WIDE_THREADS * i < nvec) {
+#pragma unroll
+            for (int j = 0; j < VN; ++j) {
+                const float d = x[i][j] - mu;
+                s2 += d * d;
+            }
+        }
+    const float r = 1.0f / sqrtf(block_sum(s2, red) / n + eps);
+    OutT* dst = out + g * (int64_t)C;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int v = tid + LN_WIDE_THREADS * i;
+        if (v < nvec) {
+            float y[VN];
+#pragma unroll
+            for (int j = 0; j < VN; ++j) y[j] = (x[i][j] - mu) * r;
+            if (gamma) {
+                Vec16<InT> t;
+                float gf[VN];
+                t.raw = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
+                t.to_f32(gf);
+#pragma unroll
+                for (int j = 0; j < VN; ++j) y[j] *= gf[j];
+            }
+            if (beta) {
+                Vec16<InT> t;
+                float bf[VN];
+                t.raw = __ldg(reinterpret_cast<const uint4*>(beta) + v);
+                t.to_f32(bf);
+#pragma unroll
+                for (int j = 0; j < VN; ++j) y[j] += bf[j];
+            }
+            store_vec<VN>(dst + (int64_t)v * VN, y);
+        }
+    }
+    if (tid == 0) {
+        mean[g] = mu;
+        rstd[g] = r;
+    }
 }
 
 // Any C, any alignment: one block per group, scalar accesses, the group re-read from
@@ -350,7 +435,7 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
     const InT* bp = static_cast<const InT*>(beta);
     auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     const size_t out_vec_bytes = VN * sizeof(OutT);
-    bool vec_ok = C % VN == 0 && C / VN <= 32 * 16 && al16(a) && (!gamma || al16(gamma)) &&
+    const bool vec_ok = C % VN == 0 && C / VN <= 8 * LN_WIDE_THREADS && al16(a) && (!gamma || al16(gamma)) &&
                   (!beta || al16(beta)) &&
                   (reinterpret_cast<uintptr_t>(out) % (out_vec_bytes > 16 ? 16 : out_vec_bytes)) == 0;
     if (vec_ok) {
@@ -382,7 +467,13 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
         else if (vpl <= 6) LN_GO(6);
         else if (vpl <= 8) LN_GO(8);
         else if (vpl <= 12) LN_GO(12);
-        else LN_GO(16);
+        else if (vpl <= 16) LN_GO(16);
+        else if (nvec <= 4 * LN_WIDE_THREADS)
+            B200_CUDA(launch_dep(ln_wide_kernel<InT, OutT, 4>, dim3((unsigned)groups), dim3(LN_WIDE_THREADS), 0, ctx->stream, 1, ap,
+                                 op, mean, rstd, gp, bp, (int)C, eps));
+        else
+            B200_CUDA(launch_dep(ln_wide_kernel<InT, OutT, 8>, dim3((unsigned)groups), dim3(LN_WIDE_THREADS), 0, ctx->stream, 1, ap,
+                                 op, mean, rstd, gp, bp, (int)C, eps));
 #undef LN_GO
 #undef LN_GO_SHARED
     } else {

@@ -39,6 +39,21 @@ def test_vs_oracle(ctx, ora, groups, C, dt_in, dt_out):
         assert np.max(np.abs(mean - rmean)) < 1e-5 and relerr(rstd, rrstd) < 1e-5
 
 
+@pytest.mark.parametrize("dt,C", [(np.float16, 4104), (np.float16, 8192), (np.float16, 8200), (np.float16, 16384),
+                                  (np.float16, 16392), (np.float32, 2052), (np.float32, 4096), (np.float32, 4280),
+                                  (np.float32, 8192), (np.float32, 8196)])
+def test_rows_wider_than_a_warp_holds(ctx, ora, dt, C):
+    """A block per row: the smallest and largest widths of its two forms, and the next ones on either side."""
+    rng = np.random.default_rng(C)
+    a = (rng.standard_normal((37, C)) * 2 + 0.5).astype(dt)
+    gam, bet = ((o + 0.1 * rng.standard_normal(C)).astype(dt) for o in (1, 0))
+    got, mean, rstd = layernorm_gpu(ctx, a, gam, bet, 1e-5)
+    ref, rmean, rrstd = ora.layernorm(a, gam, bet, 1e-5, out_dtype=dt)
+    tol = 1.5e-3 if dt == np.float16 else 2e-6      # as above: a few fp32 ulps of the sums, at most one output ulp
+    assert relerr(got, ref) < tol, describe(got, ref, tol)
+    assert np.max(np.abs(mean - rmean)) < 1e-5 and relerr(rstd, rrstd) < 1e-5
+
+
 def test_mean_dominates_variance(ctx, ora):
     a = (np.float32(1000.0) + np.float32(0.5) * np.sin(np.arange(4 * 256, dtype=np.float32))).reshape(4, 256)
     got, _, _ = layernorm_gpu(ctx, a, eps=1e-5)
