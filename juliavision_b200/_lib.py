@@ -6,10 +6,13 @@ symbol cannot be resolved, importing the product fails loudly.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SO_PATH = os.path.join(HERE, "csrc", "libb200dnn.so")
+HOST_PATH = os.path.join(HERE, "csrc", "hostcalls.so")
 
 OK, EINVAL, ECUDA, ENOMEM, EKERNEL = 0, 1, 2, 3, 4
 DECLINE = {16: "operands", 17: "extent", 18: "wrapped", 19: "bias", 20: "eltype", 21: "tiling"}
@@ -127,6 +130,27 @@ def lib() -> C.CDLL:
             fn.argtypes = args
         _lib = L
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The entry points' host side as a native module (csrc/hostcalls.c): checks and call in one step for the
+    operands programs ordinarily pass, None for any others."""
+    global _host
+    if _host is None:
+        L = lib()
+        if not os.path.exists(HOST_PATH):
+            raise ImportError(f"{HOST_PATH} is missing: build it with `python -m juliavision_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("hostcalls", HOST_PATH)
+        m = importlib.util.module_from_spec(importlib.util.spec_from_file_location("hostcalls", HOST_PATH, loader=loader))
+        loader.exec_module(m)
+        at = lambda f: C.cast(f, C.c_void_p).value
+        m.bind(at(L.b200_gemm_f16), at(L.b200_gemv), at(L.b200_attention_f16_bias), at(L.b200_layernorm),
+               at(L.b200_conv2d_grouped_f16))
+        _host = m
+    return _host
 
 
 def last_error() -> str:

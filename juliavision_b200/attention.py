@@ -86,4 +86,8 @@ def sdpa(ctx: Ctx, q, k, v, bias=None, scale: Optional[float] = None, out: Optio
     """sdpa(ctx, q, k, v, bias, scale; out) (attention.jl:712-719)."""
     if scale is None:
         scale = 1.0 / sqrt(q.shape[0])
+    rc = _lib.host().sdpa(ctx.handle, out, q, k, v, bias, scale)
+    if rc is not None:
+        check(rc)
+        return out
     return sdpa_(ctx, sdpaplan(ctx, q, k, v, bias), out, q, k, v, bias, scale)

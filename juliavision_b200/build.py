@@ -10,12 +10,15 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 SO = os.path.join(CSRC, "libb200dnn.so")
 SOURCES = ["ctx.cu", "layernorm.cu", "gemm.cu", "attention.cu", "glue.cu", "conv.cu", "gemv.cu", "gemm_rows.cu", "attention_window.cu", "selftest.cu"]
 HEADERS = ["internal.h", "ptx.cuh", "act.cuh", os.path.join("..", "..", "include", "b200dnn.h")]
+HOST_SRC = os.path.join(CSRC, "hostcalls.c")   # the entry points' host side, a CPython extension
+HOST_SO = os.path.join(CSRC, "hostcalls.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -53,6 +56,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
         failed |= p.returncode != 0
     if failed:
         raise RuntimeError("nvcc failed; see output above")
+    if force or _stale(HOST_SO, [HOST_SRC, hdrs[-1]]):
+        subprocess.run(["/usr/bin/gcc", "-O2", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], "-o", HOST_SO,
+                        HOST_SRC], check=True)
     if force or procs or _stale(SO, objs):
         cmd = [NVCC, "-shared", "-o", SO, *objs, "-ccbin", "/usr/bin/g++", "-cudart", "static",
                "-gencode", "arch=compute_100a,code=sm_100a"]

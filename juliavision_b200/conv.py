@@ -27,6 +27,10 @@ def convolution_(ctx: Ctx, out: DeviceArray, x: DeviceArray, w: DeviceArray, bia
                  act: str = "identity") -> DeviceArray:
     """convolution!(ctx, out, x, w, bias, stride, padding, dilation, groups; act); stride etc. are
     (x, y) in the reference's reversed order."""
+    rc = _lib.host().convolution(ctx.handle, out, x, w, bias, stride, padding, dilation, groups, _lib.EPI.get(act))
+    if rc is not None:
+        check(rc)
+        return out
     if x.dtype != np.float16 or w.dtype != np.float16:
         raise B200Error(16, "convolution!: Decline(:operands)")
     if not (x.isdense() and w.isdense() and out.isdense()):

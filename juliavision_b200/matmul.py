@@ -79,6 +79,10 @@ def matmul_(ctx: Ctx, out: DeviceArray, A: DeviceArray, B: DeviceArray, bias: Op
             epi: str = "identity") -> DeviceArray:
     """matmul!(ctx, out, A, B, bias; epi) (matmul.jl:78-79). An unsupported operand is an error:
     there is no CPU path behind this entry point."""
+    rc = _lib.host().matmul(ctx.handle, out, A, B, bias, _lib.EPI.get(epi))
+    if rc is not None:
+        check(rc)
+        return out
     plan = mmplan(ctx, out, A, B, bias)
     if isinstance(plan, Decline):
         raise B200Error(16, f"matmul!: Decline(:{plan.reason}) for A{A.shape}:{A.dtype} B{B.shape}:{B.dtype}")
