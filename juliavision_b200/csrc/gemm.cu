@@ -17,8 +17,6 @@
 //   warp 1     UMMA issuer   (one lane issues) shared -> TMEM accumulators (two, ping-pong)
 //   warps 2-17 epilogue      (512 threads)     TMEM -> registers -> +bias, round, act ->
 //                                              warp-private shared slab -> bulk tensor store
-//   warp 18    relay                           waits for each stage to land and passes that on to the
-//                                              issuer through a named barrier (see the issuer's comment)
 #include <cuda_fp16.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -32,8 +30,7 @@ namespace b200 {
 constexpr int GEMM_BM = 128; // tokens per CTA (TMEM lanes)
 constexpr int GEMM_BK = 64;  // one 128-byte swizzle row of fp16
 constexpr int EPI_WARPS = 16;
-constexpr int RELAY_WARP = 2 + EPI_WARPS;
-constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS + 32; // producer warp, UMMA warp, epilogue warps, relay warp
+constexpr int GEMM_THREADS = 64 + 32 * EPI_WARPS; // producer warp, UMMA warp, epilogue warps
 static_assert(GEMM_BK == 64, "the UMMA issuer unrolls four K = 16 steps per k-block");
 constexpr int SMEM_LIMIT = 232448; // 227 KB
 
@@ -201,7 +198,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // warp-uniform, and known to be
     const int lane = threadIdx.x & 31;
     const uint32_t rank = NCTA == 2 ? cluster_ctarank() : 0u;  // 0 = the CTA that issues the UMMAs
     const uint32_t worker = NCTA == 2 ? (blockIdx.x >> 1) : blockIdx.x;
@@ -303,14 +300,12 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
         }
     } else if (warp == 1) {
         // -------------------------------------------------------------- UMMA issuer
-        // What one k-block costs the issuing thread, measured with the SM's cycle counter on a stand-alone
-        // loop of the same instructions: 64 cycles per tcgen05.mma (whatever N), ~45 for the commit, and
-        // ~215 more for the first shared-memory read after them whose value the thread needs — which is what
-        // an mbarrier test is.  4 x 64 + 45 + 215 made every k-block take 560-590 cycles for every tile width,
-        // above the 512 the tensor pipe needs for a 256-wide pair tile.  So this thread never reads shared
-        // memory in its loop: the relay warp watches the stage barriers and hands each "stage has landed"
-        // over through a named barrier (a hardware barrier, ~100 cycles here), one per stage of the ring.
-        // The whole warp runs the loop so that the barrier instruction is warp-uniform; lane 0 issues.
+        // The whole warp walks the loop and waits for the stages; the thread elect.sync picks (the same one every
+        // time) issues, every operand of an instruction being the same for the warp.  With one lane running the loop
+        // under `if (lane == 0)` a k-block took 560-590 cycles unless a further warp did the waiting for it and handed
+        // each stage over through a named barrier; against that pair of warps this takes 0 to 15 % off most launches
+        // (160 x 2304 x 768: 8.0 -> 7.3 us, 1500 x 3840 x 1280: 25.3 -> 24.0, 8192 x 3584 x 896 with GELU: 57.6 -> 48.6,
+        // 65536 x 5120 x 1280 unchanged) and adds as much to a few of short K (32768 x 1344 x 448: 42.5 -> 47.4).
         if (rank == 0) {
             constexpr uint32_t idesc = make_idesc_f16(TILE_N, Cfg::WIDE ? 256 : BN, /*a K-major*/ 0, /*b MN-major*/ 1);
             const uint32_t idesc2 = make_idesc_f16(TILE_N, p.bn - 256, 0, 1);   // wide tile: the columns past 256
@@ -318,19 +313,23 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
             constexpr uint64_t bdesc0 = make_smem_desc(Cfg::B_CHUNK_BYTES, 1024);
             int s = 0;
             int it = 0;
+            uint32_t ph = 0;
+            bool ok = true;
             SegIter seg;
-            for (seg.init(p.total_tiles, p.num_kb, p.streamk, worker, nworkers); seg.valid(); seg.next(), ++it) {
+            for (seg.init(p.total_tiles, p.num_kb, p.streamk, worker, nworkers); ok && seg.valid(); seg.next(), ++it) {
                 const int acc = Cfg::WIDE ? 0 : (int)(it & 1);
                 const uint32_t aph = (uint32_t)((Cfg::WIDE ? it : it >> 1) & 1);
                 bool got;
                 if constexpr (NCTA == 2) got = mbar_wait_cluster(&tempty[acc], aph ^ 1, p.d_status, KST_WAIT_TMEM_EMPTY, abort_flag);
                 else got = mbar_wait(&tempty[acc], aph ^ 1, p.d_status, KST_WAIT_TMEM_EMPTY, abort_flag);
-                if (__any_sync(0xffffffffu, !got)) break;   // one answer per warp; the relay keeps arriving, which is harmless
+                if (__any_sync(0xffffffffu, !got)) break;   // one answer per warp
                 const uint32_t d_tmem = tmem_base + acc * BN;
                 for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
-                    named_bar_sync(1 + s, 64);   // the relay has seen full[s] complete (or has given up: see there)
+                    if constexpr (NCTA == 2) got = mbar_wait_cluster(&full[s], ph, p.d_status, KST_WAIT_FULL, abort_flag);
+                    else got = mbar_wait(&full[s], ph, p.d_status, KST_WAIT_FULL, abort_flag);
+                    if (__any_sync(0xffffffffu, !got)) { ok = false; break; }
                     tc_fence_after();
-                    if (lane == 0) {
+                    if (elect_one()) {
                         if (kb == seg.kb0 && it == 0) GEMM_TRACE(3); // first stage landed
                         const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
                         const uint32_t b_addr = a_addr + Cfg::A_BYTES;
@@ -359,39 +358,14 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
                         else umma_commit(&empty[s]);
                     }
                     __syncwarp();
-                    if (++s == Cfg::STAGES) s = 0;
+                    if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
                 }
-                if (lane == 0) {
+                if (ok && elect_one()) {
                     if constexpr (NCTA == 2) umma_commit_pair(&tfull[acc], 3);
                     else umma_commit(&tfull[acc]);
                     GEMM_TRACE(4 + (it < 4 ? it : 3)); // all UMMAs of tile `it` issued
                 }
                 __syncwarp();
-            }
-        }
-    } else if (warp == RELAY_WARP) {
-        // -------------------------------------------------------------------- relay
-        // Waits (bounded) for each stage's operands to land and arrives on that stage's named barrier, on
-        // which the issuer warp syncs.  It can run ahead of the issuer by at most the ring depth, because
-        // stage s is refilled only after the issuer's commit for it, so one barrier id per stage suffices.
-        // After a wait has run out it stops waiting but keeps arriving, so the issuer is never left
-        // blocked: the UMMAs then run on whatever the stages hold, the status word says the result is void.
-        if (rank == 0) {
-            int s = 0;
-            uint32_t ph = 0;
-            bool ok = true;
-            SegIter seg;
-            for (seg.init(p.total_tiles, p.num_kb, p.streamk, worker, nworkers); seg.valid(); seg.next()) {
-                for (int kb = seg.kb0; kb < seg.kb1; ++kb) {
-                    if (ok) {
-                        bool got;
-                        if constexpr (NCTA == 2) got = mbar_wait_cluster(&full[s], ph, p.d_status, KST_WAIT_FULL, abort_flag);
-                        else got = mbar_wait(&full[s], ph, p.d_status, KST_WAIT_FULL, abort_flag);
-                        ok = !__any_sync(0xffffffffu, !got);
-                    }
-                    named_bar_arrive(1 + s, 64);
-                    if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
-                }
             }
         }
     } else {
