@@ -57,6 +57,7 @@ template <int BN, typename OutT, int NCTA> struct GemmCfg {
     static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + TAIL_BYTES;
     static constexpr int TMEM_COLS = WIDE ? 512 : (2 * BN < 32 ? 32 : 2 * BN);
+    static_assert(NCTA == 2 || STAGES * STAGE_BYTES >= GEMM_BM * BN * 4, "a tile's fp32 accumulator fits over the ring");
     static_assert(STAGES >= 2, "ring too shallow");
     static_assert(SMEM_BYTES <= SMEM_LIMIT, "shared memory over budget");
     static_assert(TMEM_COLS == 128 || TMEM_COLS == 256 || TMEM_COLS == 512, "TMEM columns");
@@ -76,6 +77,7 @@ template <typename OutT> struct GemmParams {
     const __half* bias;
     int bias_per_n;        // 0: bias[i] over features (M); 1: bias[j] over tokens (N)
     int epilogue;
+    int ksplit;            // KSPLIT: CTAs (a cluster) per tile
     int streamk;           // 0: whole tiles, strided over the workers; 1 + lean: contiguous k-block ranges per worker (see SegIter)
     float* sk_part;        // stream-K: fp32 partial accumulators, one 128 x BN block per (worker, CTA rank)
     int* sk_flag;          // stream-K: one flag per (worker, CTA rank, epilogue warp), zero between launches
@@ -172,7 +174,17 @@ __device__ __forceinline__ void st_release_gpu(int* p, int v) {
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-template <int BN, typename OutT, int NCTA>
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
+// KSPLIT: a cluster of p.ksplit CTAs (NCTA = 1) takes one tile, each a contiguous part of its k-blocks.  The fp32
+// accumulators are laid over the drained operand ring and every CTA finishes its share of the tile's chunks from all
+// of them, read through distributed shared memory and added in rank order: no workspace, no flags, and a hand-off of
+// a cluster barrier where the stream-K one through L2 costs ~6 us.
+template <int BN, typename OutT, int NCTA, bool KSPLIT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, tokens, batch}
                    const __grid_constant__ CUtensorMap tmapW,   // A(M,K): {features, K, batch}
@@ -200,9 +212,11 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // warp-uniform, and known to be
     const int lane = threadIdx.x & 31;
+    static_assert(!KSPLIT || NCTA == 1, "a K split is over single CTAs");
     const uint32_t rank = NCTA == 2 ? cluster_ctarank() : 0u;  // 0 = the CTA that issues the UMMAs
-    const uint32_t worker = NCTA == 2 ? (blockIdx.x >> 1) : blockIdx.x;
-    const uint32_t nworkers = NCTA == 2 ? (gridDim.x >> 1) : gridDim.x;
+    const uint32_t kpart = KSPLIT ? cluster_ctarank() : 0u;    // which part of the tile's k-blocks
+    const uint32_t worker = NCTA == 2 ? (blockIdx.x >> 1) : (KSPLIT ? blockIdx.x / (uint32_t)p.ksplit : blockIdx.x);
+    const uint32_t nworkers = NCTA == 2 ? (gridDim.x >> 1) : (KSPLIT ? gridDim.x / (uint32_t)p.ksplit : gridDim.x);
 
     if (threadIdx.x == 0) {
         GEMM_TRACE(0); // kernel entry
@@ -233,6 +247,13 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
     if constexpr (NCTA == 2) cluster_sync_all(); // both CTAs' barriers and TMEM exist before any use
     else __syncthreads();
     tc_fence_after();
+    // KSPLIT: this CTA's k-blocks (at least one: the host keeps ksplit <= num_kb), its worker's only tile
+    auto narrow = [&](SegIter& seg) {
+        if constexpr (KSPLIT) {
+            seg.kb0 = (int)(kpart * (uint32_t)p.num_kb / (uint32_t)p.ksplit);
+            seg.kb1 = (int)((kpart + 1) * (uint32_t)p.num_kb / (uint32_t)p.ksplit);
+        }
+    };
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tiles_per_batch = (uint32_t)p.tiles_m * (uint32_t)p.tiles_n;
     const bool one_plane = tiles_per_batch == p.total_tiles;
@@ -243,6 +264,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
     grid_dep_launch();
 
     if (threadIdx.x == 0) GEMM_TRACE(1); // setup done
+    bool met = false;   // KSPLIT: this warp has passed the barrier inside the epilogue
 
     if (warp == 0) {
         // ------------------------------------------------------------- TMA producer
@@ -252,6 +274,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
             bool ok = true;
             SegIter seg;
             for (seg.init(p.total_tiles, p.num_kb, p.streamk, worker, nworkers); ok && seg.valid(); seg.next()) {
+                narrow(seg);
                 const TileAt at = tile_at(seg.tile, (uint32_t)p.tiles_m, tiles_per_batch, one_plane);
                 const int batch = at.batch;
                 const int m0 = Cfg::WIDE ? at.tm * p.bn : at.tm * BN + (int)rank * Cfg::B_COLS;
@@ -317,6 +340,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
             bool ok = true;
             SegIter seg;
             for (seg.init(p.total_tiles, p.num_kb, p.streamk, worker, nworkers); ok && seg.valid(); seg.next(), ++it) {
+                narrow(seg);
                 const int acc = Cfg::WIDE ? 0 : (int)(it & 1);
                 const uint32_t aph = (uint32_t)((Cfg::WIDE ? it : it >> 1) & 1);
                 bool got;
@@ -401,9 +425,9 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
             // Stream-K roles of this segment: a contributor holds later k-blocks of a tile some other
             // worker finishes; a finisher holds the tile's first k-block and collects what the
             // following workers left for it.
-            const bool contributor = seg.kb0 > 0;
+            const bool contributor = seg.kb0 > 0;   // (never with KSPLIT, whose ranges `narrow` does not touch here)
             int ncontrib = 0;
-            if (!contributor && seg.kb1 < seg.nkb) {
+            if (!KSPLIT && !contributor && seg.kb1 < seg.nkb) {
                 const uint32_t units = p.total_tiles * (uint32_t)seg.nkb, tile_end = (tile + 1) * (uint32_t)seg.nkb;
                 while (worker + 1 + (uint32_t)ncontrib < nworkers &&
                        SegIter::range_start(units, worker + 1 + (uint32_t)ncontrib, nworkers, (uint32_t)p.streamk - 1u) < tile_end)
@@ -457,18 +481,50 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
             // spreads a warp's 16-byte stores over all banks: four wavefronts per instruction instead of eight.
             const int swz = RB == 32 ? ((lane >> 2) & 1) : ((lane >> 1) & 3);
 
+            // KSPLIT: the accumulator over the operand ring, [chunk][quarter][row] of 16 bytes
+            const uint32_t dump = smem_u32(smem) + row * 16;
+            if constexpr (KSPLIT) {
+#pragma unroll 1
+                for (int c = 0; c < NCH; ++c) {
+                    uint32_t r[CH];
+                    tmem_ld16(tacc + chunk_col(c), r);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int q = 0; q < CH / 4; ++q)
+                        st_shared_v4(dump + (uint32_t)(chunk_col(c) / 4 + q) * (GEMM_BM * 16), r + 4 * q);
+                }
+                __syncwarp();
+                met = true;
+                cluster_sync_all();   // every part's accumulator is in its shared memory (the other roles arrive below)
+            }
 #pragma unroll 1
             for (int c = 0; c < NCH; ++c) {
                 const int col0 = chunk_col(c);
+                if (KSPLIT && (uint32_t)(col0 / CH) % (uint32_t)p.ksplit != kpart) continue;   // another part finishes this chunk
                 float v[CH];
-                {
+                if constexpr (KSPLIT) {
+#pragma unroll
+                    for (int t = 0; t < CH; ++t) v[t] = 0.f;
+#pragma unroll 4
+                    for (uint32_t k = 0; k < (uint32_t)p.ksplit; ++k) {
+                        const uint32_t src = mapa_u32(dump + (uint32_t)(col0 / 4) * (GEMM_BM * 16), k);
+#pragma unroll
+                        for (int q = 0; q < CH / 4; ++q) {
+                            const float4 f = ld_cluster_f4(src + q * (GEMM_BM * 16));
+                            v[4 * q] += f.x;
+                            v[4 * q + 1] += f.y;
+                            v[4 * q + 2] += f.z;
+                            v[4 * q + 3] += f.w;
+                        }
+                    }
+                } else {
                     uint32_t r[CH];
                     tmem_ld16(tacc + col0, r);
                     tmem_wait_ld();
 #pragma unroll
                     for (int t = 0; t < CH; ++t) v[t] = __uint_as_float(r[t]);
                 }
-                if (c == NCH - 1) {
+                if (!KSPLIT && c == NCH - 1) {
                     // This warp has read all it needs of the accumulator: hand it back (leader CTA).
                     tc_fence_before();
                     __syncwarp();
@@ -582,12 +638,17 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
     }
 
     // Teardown: every role arrives here whether it finished or gave up.
+    if constexpr (KSPLIT) {
+        // the barrier between the two halves of the epilogue: the roles without one, and epilogue warps that gave up
+        __syncwarp();
+        if (!met) cluster_sync_all();
+    }
     if (*abort_flag) {
         // Let any TMA copy still in flight into this CTA's shared memory land before exit.
         for (int i = 0; i < 4; ++i) __nanosleep(1000000);
     }
     tc_fence_before();
-    if constexpr (NCTA == 2) cluster_sync_all(); // neither CTA leaves while its peer may still signal it
+    if constexpr (NCTA == 2 || KSPLIT) cluster_sync_all(); // no CTA leaves while a peer may still signal it or read its accumulator
     else __syncthreads();
     if (warp == 1) {
         tc_fence_after();
@@ -629,6 +690,7 @@ struct TilePick {
     int ncta;    // 1: 128-token tiles, one CTA each; 2: 256-token tiles, one CTA pair each
     int streamk; // 1: equal k-block ranges per worker instead of whole tiles
     int width;   // bn == 512 (the wide tile): feature columns per tile, a multiple of 16 in (256, 512]
+    int ksplit;  // > 1: CTAs of a cluster that share a tile's k-blocks (ncta == 1)
 };
 
 // Tile planner.  Candidates are (BN, NCTA, whole-tile | stream-K); the estimate for each is
@@ -645,19 +707,22 @@ static int64_t streamk_workers(int64_t tiles, int64_t workers_max) {
 
 static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int sms, bool allow_streamk = true,
                           int epilogue = B200_EPI_NONE) {
-    if (const char* f = getenv("B200_GEMM_TILE")) { // debugging aid: "<bn>x<ncta>[s]", e.g. 256x2 or 256x2s
-        int bn = 0, nc = 0;
+    if (const char* f = getenv("B200_GEMM_TILE")) { // debugging aid: "<bn>x<ncta>[s|k<parts>]", e.g. 256x2, 256x2s or 64x1k4
+        int bn = 0, nc = 0, ks = 1;
         char sk = 0;
-        const int got = sscanf(f, "%dx%d%c", &bn, &nc, &sk);
+        const int got = sscanf(f, "%dx%d%c%d", &bn, &nc, &sk, &ks);
+        if (got == 4 && sk == 'k' && nc == 1 && (bn == 128 || bn == 64) && ks >= 2 && ks <= 8 && ks <= cdiv(K, GEMM_BK) &&
+            cdiv(M, bn) * cdiv(N, (int64_t)GEMM_BM) * nbatch * ks <= sms)
+            return {bn, 1, 0, 0, ks};
         if (got >= 2 && (bn == 256 || bn == 128 || (bn == 64 && nc == 1)) && (nc == 1 || nc == 2))
-            return {bn, nc, allow_streamk && got == 3 && sk == 's', 0};
-        if (got >= 2 && bn > 256 && bn <= 512 && bn % 16 == 0 && nc == 2) return {512, 2, 0, bn};   // "<width>x2": the wide tile
+            return {bn, nc, allow_streamk && got == 3 && sk == 's', 0, 1};
+        if (got >= 2 && bn > 256 && bn <= 512 && bn % 16 == 0 && nc == 2) return {512, 2, 0, bn, 1};   // "<width>x2": the wide tile
     }
     struct Cand { int bn, ncta; double t_kb; };
     const Cand cands[5] = {{256, 2, 0.39}, {128, 2, 0.38}, {256, 1, 0.50}, {128, 1, 0.38}, {64, 1, 0.32}};
     const int64_t nkb = cdiv(K, GEMM_BK);
     const double t_tile = 2.0, t_fix = 8.0;  // measured: partial dump + fence + flag + read-back
-    TilePick best{256, 1, 0, 0};
+    TilePick best{256, 1, 0, 0, 1};
     double best_cost = 1e300;
     for (const Cand& c : cands) {   // whole-tile schedules first: stream-K has to beat the best of them clearly
         const int64_t tiles = cdiv(M, c.bn) * cdiv(N, (int64_t)GEMM_BM * c.ncta) * nbatch;
@@ -665,7 +730,7 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
         const double dp = (double)waves * ((double)nkb * c.t_kb + t_tile);
         if (dp < best_cost - 1e-9) {
             best_cost = dp;
-            best = {c.bn, c.ncta, 0, 0};
+            best = {c.bn, c.ncta, 0, 0, 1};
         }
     }
     {
@@ -685,13 +750,29 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
                 const double wide = 7.0 + (double)nkb * 0.3 * (rel < 1.25 ? 1.25 : rel) + (gelu ? 0.85 : 0.25) * (double)width / 64.0;
                 if (wide < 0.92 * best_cost) {
                     best_cost = wide;
-                    best = {512, 2, 0, (int)width};
+                    best = {512, 2, 0, (int)width, 1};
                 }
             }
         }
     }
+    // Few tiles with long reductions: the k-blocks of a tile over a cluster of 2, 4 or 8 CTAs, as long as every CTA
+    // has an SM and three k-blocks.  t_join is what the accumulators' way through shared memory adds.  Reductions of
+    // fewer than 24 k-blocks stay whole: they gain a microsecond or two, and the rows of a product computed in shards
+    // keep the bits they have in the whole.  160 x 768 x 3072: 17.0 -> 11.1 us, 18 x 304 x 2144: 11 -> 7.0,
+    // 9 x 1056 x 4488: 20 -> 14.
+    for (const int bn : {128, 64}) {
+        const int64_t tiles = cdiv(M, bn) * cdiv(N, (int64_t)GEMM_BM) * nbatch;
+        const double t_kb = bn == 128 ? 0.38 : 0.32, t_join = 1.5;
+        for (int ks = 2; ks <= 8 && nkb >= 24 && tiles * ks <= sms; ks *= 2) {
+            const double cost = (double)cdiv(nkb, ks) * t_kb + t_tile + t_join;
+            if (cost < 0.95 * best_cost) {
+                best_cost = cost;
+                best = {bn, 1, 0, 0, ks};
+            }
+        }
+    }
     best_cost *= 0.85;
-    if (!allow_streamk) return best;
+    if (!allow_streamk || best.ksplit > 1) return best;
     for (const Cand& c : cands) {
         const int64_t tiles = cdiv(M, c.bn) * cdiv(N, (int64_t)GEMM_BM * c.ncta) * nbatch;
         const int64_t workers = sms / c.ncta;
@@ -704,24 +785,25 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
             const double sk = (double)(tiles * nkb) / (double)skw * c.t_kb + t_tile + t_fix;
             if (sk < best_cost - 1e-9) {
                 best_cost = sk;
-                best = {c.bn, c.ncta, 1, 0};
+                best = {c.bn, c.ncta, 1, 0, 1};
             }
         }
     }
     return best;
 }
 
-template <int BN, typename OutT, int NCTA>
+template <int BN, typename OutT, int NCTA, bool KSPLIT = false>
 static int launch_tc(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda,
                      const void* B, int64_t ldb, const void* bias, int bias_per_n, void* out, int64_t ldo,
-                     int epi, int64_t nbatch, int64_t sA, int64_t sB, int64_t sO, int streamk, int width) {
+                     int epi, int64_t nbatch, int64_t sA, int64_t sB, int64_t sO, int streamk, int width,
+                     int ksplit) {
     using Cfg = GemmCfg<BN, OutT, NCTA>;
     if (Cfg::WIDE) {
         B200_REQUIRE(width > 256 && width <= 512 && width % 16 == 0, B200_EINVAL, "gemm: wide tile of %d columns", width);
         streamk = 0;
     }
     static bool attr_done[16] = {};
-    auto kern = gemm_f16_tc_kernel<BN, OutT, NCTA>;
+    auto kern = gemm_f16_tc_kernel<BN, OutT, NCTA, KSPLIT>;
     if (!attr_done[ctx->device & 15]) {
         B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
         attr_done[ctx->device & 15] = true;
@@ -802,6 +884,14 @@ static int launch_tc(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void*
         if (resident[ctx->device & 15] < workers_max) workers_max = resident[ctx->device & 15];
     }
     int workers = (int)((int64_t)p.total_tiles < workers_max ? (int64_t)p.total_tiles : workers_max);
+    p.ksplit = 1;
+    if (KSPLIT) {
+        B200_REQUIRE(ksplit >= 2 && ksplit <= 8 && ksplit <= p.num_kb && (int64_t)p.total_tiles * ksplit <= ctx->prop.multiProcessorCount,
+                     B200_EINVAL, "gemm: K split in %d", ksplit);
+        p.ksplit = ksplit;
+        workers = (int)p.total_tiles;
+        streamk = 0;
+    }
     p.streamk = 0;
     p.sk_part = nullptr;
     p.sk_flag = ctx->sk_flags;
@@ -821,8 +911,8 @@ static int launch_tc(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void*
         p.streamk = 1 + lean;
         p.sk_part = static_cast<float*>(part);
     }
-    B200_CUDA(launch_dep(kern, dim3((unsigned)(workers * NCTA), 1, 1), dim3(GEMM_THREADS, 1, 1), Cfg::SMEM_BYTES,
-                         ctx->stream, NCTA, tX, tW, tO, p));
+    B200_CUDA(launch_dep(kern, dim3((unsigned)(workers * NCTA * p.ksplit), 1, 1), dim3(GEMM_THREADS, 1, 1), Cfg::SMEM_BYTES,
+                         ctx->stream, NCTA * p.ksplit, tX, tW, tO, p));
     ctx->launches++;
     return B200_OK;
 }
@@ -876,7 +966,7 @@ int b200_gemm_f16_plan(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, int64_t n
     plan->tiles_n = (int)cdiv(N, (int64_t)GEMM_BM * t.ncta);
     const int64_t tiles = (int64_t)plan->tiles_m * plan->tiles_n * nbatch;
     const int64_t workers = sms / t.ncta;
-    plan->ctas = (int)((tiles < workers ? tiles : workers) * t.ncta);
+    plan->ctas = (int)((tiles < workers ? tiles : workers) * t.ncta) * t.ksplit;
     return B200_OK;
 }
 
@@ -932,7 +1022,18 @@ int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, 
     const TilePick t = pick_tile(M, N, K, nbatch, ctx->prop.multiProcessorCount, use_workspace != 0, epilogue);
 #define GEMM_GO(BN_, T_, NC_)                                                                                     \
     return launch_tc<BN_, T_, NC_>(ctx, M, N, K, A, lda, B, ldb, bias, bias_per_n, out, ldo, epilogue, nbatch, strideA, \
-                                   strideB, strideO, t.streamk, t.width)
+                                   strideB, strideO, t.streamk, t.width, t.ksplit)
+#define GEMM_GO_SPLIT(BN_, T_)                                                                                    \
+    return launch_tc<BN_, T_, 1, true>(ctx, M, N, K, A, lda, B, ldb, bias, bias_per_n, out, ldo, epilogue, nbatch, strideA, \
+                                       strideB, strideO, 0, 0, t.ksplit)
+    if (t.ksplit > 1) {
+        if (out_dtype == B200_F16) {
+            if (t.bn == 128) GEMM_GO_SPLIT(128, __half);
+            GEMM_GO_SPLIT(64, __half);
+        }
+        if (t.bn == 128) GEMM_GO_SPLIT(128, float);
+        GEMM_GO_SPLIT(64, float);
+    }
     if (out_dtype == B200_F16) {
         if (t.bn == 512) GEMM_GO(512, __half, 2);
         if (t.ncta == 2 && t.bn == 256) GEMM_GO(256, __half, 2);
@@ -949,6 +1050,7 @@ int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, 
         GEMM_GO(64, float, 1);
     }
 #undef GEMM_GO
+#undef GEMM_GO_SPLIT
 }
 
 } // namespace b200

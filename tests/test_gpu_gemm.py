@@ -200,6 +200,29 @@ def test_every_tile_shape_and_schedule(ctx, ora, tile, monkeypatch):
         assert relerr(got, ref) < TOL, (tile, tokens, out, K, describe(got, ref, TOL))
 
 
+@pytest.mark.parametrize("tile", ["64x1k2", "64x1k8", "128x1k2", "128x1k3", "128x1k8"])
+@pytest.mark.parametrize("tokens,out,K", [(2, 8, 512), (129, 264, 530), (300, 200, 1288), (17, 1000, 4264)])
+def test_tiles_shared_by_a_cluster(ctx, ora, tile, tokens, out, K, monkeypatch):
+    """K split over a cluster's CTAs: even and uneven parts (one k-block each at the least), ragged tiles both ways,
+    fp16 with an activation and fp32; the same bits every time, and two planes at once."""
+    monkeypatch.setenv("B200_GEMM_TILE", tile)
+    rng = np.random.default_rng(tokens + out + K)
+    X, Wt, b = _case(rng, tokens, out, K, scale=0.25)
+    got = linear_gpu(ctx, X, Wt, b, epi="gelu")
+    assert relerr(got, ora.linear(X, Wt, b, epi="gelu")) < 2e-3          # one rounding step of fp16
+    f32 = linear_gpu(ctx, X, Wt, b, out_dtype=np.float32)
+    ref = ora.linear(X, Wt, b, out_dtype=np.float32)
+    assert relerr(f32, ref) < 2e-5, describe(f32, ref, 2e-5)             # sqrt(K) eps32
+    assert np.array_equal(f32, linear_gpu(ctx, X, Wt, b, out_dtype=np.float32))
+    A, B = np.stack([Wt, -Wt]), np.stack([X, 2 * X])
+    two = ctx.allocate(np.float32, out, tokens, 2)
+    ctx.fill_bytes(two, 0xFF)
+    jv.batchedmatmul_(ctx, two, ctx.toback(A), ctx.toback(B))
+    ctx.synchronize()
+    zero = ora.linear(X, Wt, out_dtype=np.float32)
+    assert relerr(two.to_host(), np.stack([zero, -2 * zero])) < 2e-5
+
+
 def test_streamk_is_deterministic(ctx, monkeypatch):
     monkeypatch.setenv("B200_GEMM_TILE", "256x2s")
     rng = np.random.default_rng(77)
