@@ -215,8 +215,11 @@ gemm_rows_kernel(const GrParams p) {
     for (int i = tid + (int)rank * 32 * GR_WARPS; i < ntok * Cfg::ROWS; i += (int)nparts * 32 * GR_WARPS) {
         const int tok = i / Cfg::ROWS, r = i - tok * Cfg::ROWS;
         if (m0 + r >= p.M) continue;
-        float v = 0.f;
-        for (uint32_t q = 0; q < nparts; ++q) v += ld_cluster_f32(mapa_u32(mine + i * 4, q));
+        float a[8], v = 0.f;   // every part's load in flight together: a remote load takes a few hundred nanoseconds
+#pragma unroll
+        for (uint32_t q = 0; q < 8; ++q) a[q] = q < nparts ? ld_cluster_f32(mapa_u32(mine + i * 4, q)) : 0.f;
+#pragma unroll
+        for (uint32_t q = 0; q < 8; ++q) v += a[q];
         store(tok, r, v);
     }
     cluster_sync_all();   // nobody leaves while its sums may still be read
