@@ -705,8 +705,10 @@ static int64_t streamk_workers(int64_t tiles, int64_t workers_max) {
     return 0;
 }
 
-static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int sms, bool allow_streamk = true,
-                          int epilogue = B200_EPI_NONE) {
+struct KsplitRoom { int clusters[4]; };   // [l]: clusters of 2^l CTAs the GPU holds at once
+
+static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int sms, const KsplitRoom& room,
+                          bool allow_streamk = true, int epilogue = B200_EPI_NONE) {
     if (const char* f = getenv("B200_GEMM_TILE")) { // debugging aid: "<bn>x<ncta>[s|k<parts>]", e.g. 256x2, 256x2s or 64x1k4
         int bn = 0, nc = 0, ks = 1;
         char sk = 0;
@@ -755,19 +757,22 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
             }
         }
     }
-    // Few tiles with long reductions: the k-blocks of a tile over a cluster of 2, 4 or 8 CTAs, as long as every CTA
-    // has an SM and three k-blocks.  t_join is what the accumulators' way through shared memory adds.  Reductions of
-    // fewer than 24 k-blocks stay whole: they gain a microsecond or two, and the rows of a product computed in shards
-    // keep the bits they have in the whole.  160 x 768 x 3072: 17.0 -> 11.1 us, 18 x 304 x 2144: 11 -> 7.0,
-    // 9 x 1056 x 4488: 20 -> 14.
+    // Few tiles with long reductions: the k-blocks of a tile over a cluster of 2, 4 or 8 CTAs, as long as every cluster
+    // is resident at once (a GPC's SMs do not divide into clusters of 8 without a rest: 17 of them take two rounds,
+    // 17.3 us for 42 x 2112 x 3152 where clusters of 4 take 8.6).  t_join is what the accumulators' way through shared
+    // memory adds, fitted to 25 shapes.  Reductions of fewer than 24 k-blocks stay whole: they gain a microsecond or
+    // two, and the rows of a product computed in shards keep the bits they have in the whole.
+    // 160 x 768 x 3072: 17.0 -> 11.1 us, 18 x 304 x 2144: 11 -> 7.0, 9 x 1056 x 4488: 20 -> 14.
     for (const int bn : {128, 64}) {
         const int64_t tiles = cdiv(M, bn) * cdiv(N, (int64_t)GEMM_BM) * nbatch;
-        const double t_kb = bn == 128 ? 0.38 : 0.32, t_join = 1.5;
-        for (int ks = 2; ks <= 8 && nkb >= 24 && tiles * ks <= sms; ks *= 2) {
-            const double cost = (double)cdiv(nkb, ks) * t_kb + t_tile + t_join;
+        const double t_kb = bn == 128 ? 0.38 : 0.32;
+        const double t_join[4] = {0.0, 1.2, bn == 128 ? 2.7 : 2.2, bn == 128 ? 4.3 : 3.1};
+        for (int l = 1; l <= 3 && nkb >= 24; ++l) {
+            if (tiles > room.clusters[l]) break;
+            const double cost = (double)cdiv(nkb, (int64_t)1 << l) * t_kb + t_tile + t_join[l];
             if (cost < 0.95 * best_cost) {
                 best_cost = cost;
-                best = {bn, 1, 0, 0, ks};
+                best = {bn, 1, 0, 0, 1 << l};
             }
         }
     }
@@ -790,6 +795,37 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
         }
     }
     return best;
+}
+
+// How many clusters of 2, 4 and 8 single-CTA tiles are resident at once: asked of the runtime once per device.
+static KsplitRoom ksplit_room(b200_ctx* ctx) {
+    static KsplitRoom room[16] = {};
+    KsplitRoom& r = room[ctx->device & 15];
+    if (r.clusters[0]) return r;
+    using Cfg = GemmCfg<64, __half, 1>;
+    auto kern = gemm_f16_tc_kernel<64, __half, 1, true>;
+    KsplitRoom got = {{ctx->prop.multiProcessorCount, 0, 0, 0}};
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) == cudaSuccess)
+        for (int l = 1; l <= 3; ++l) {
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = 1u << l;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
+            cfg.gridDim = dim3((unsigned)((ctx->prop.multiProcessorCount >> l) << l), 1, 1);
+            cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+            cfg.stream = ctx->stream;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess) got.clusters[l] = n;
+            else cudaGetLastError();
+        }
+    else
+        cudaGetLastError();
+    return r = got;
 }
 
 template <int BN, typename OutT, int NCTA, bool KSPLIT = false>
@@ -944,7 +980,7 @@ int b200_gemm_f16_plan(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, int64_t n
     B200_REQUIRE(ctx && plan, B200_EINVAL, "gemm_plan: null argument");
     B200_REQUIRE(M >= 1 && N >= 1 && K >= 1 && nbatch >= 1, B200_DECLINE_EXTENT, "gemm_plan: empty extent");
     const int sms = ctx->prop.multiProcessorCount;
-    const TilePick t = pick_tile(M, N, K, nbatch, sms);
+    const TilePick t = pick_tile(M, N, K, nbatch, sms, ksplit_room(ctx));
     const int bn = t.bn == 512 ? t.width : t.bn;
     plan->block_m = GEMM_BM * t.ncta;
     plan->block_n = bn;
@@ -1019,7 +1055,7 @@ int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, 
         B200_CUDA(cudaGetLastError());
         return B200_OK;
     }
-    const TilePick t = pick_tile(M, N, K, nbatch, ctx->prop.multiProcessorCount, use_workspace != 0, epilogue);
+    const TilePick t = pick_tile(M, N, K, nbatch, ctx->prop.multiProcessorCount, ksplit_room(ctx), use_workspace != 0, epilogue);
 #define GEMM_GO(BN_, T_, NC_)                                                                                     \
     return launch_tc<BN_, T_, NC_>(ctx, M, N, K, A, lda, B, ldb, bias, bias_per_n, out, ldo, epilogue, nbatch, strideA, \
                                    strideB, strideO, t.streamk, t.width, t.ksplit)
