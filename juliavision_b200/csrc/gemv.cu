@@ -1,15 +1,17 @@
 // Matrix-vector product for the one-token case of matmul! (reference kernels/extern/matmul.jl:103-137,
 // the MMGemvPlan / Lava.gemv! path): out[m] = epi(T(bias[m] + sum_k A[m,k] x[k])), A (M,K) with M
-// contiguous (what hoistpermutes leaves), fp32 accumulation.  Bandwidth-bound: every byte of A is read
-// once, as aligned 16-byte vectors whatever the leading dimension (a vocabulary of 51865 rows gives
-// every column its own misalignment), a warp covering 512 contiguous bytes of a column, the K axis
-// split over the warps of a block and, when M alone cannot fill the GPU, over blocks as well (partials
-// in the workspace, summed in a fixed order by whichever block of a row range finishes last, so the
-// result does not depend on timing).
+// contiguous (what hoistpermutes leaves), fp32 accumulation.  Bandwidth-bound when A is large, a chain of round trips
+// when it is not: every byte of A is read once, as aligned 16-byte vectors whatever the leading dimension (a
+// vocabulary of 51865 rows gives every column its own misalignment), a warp covering 512 contiguous bytes of a
+// column, the K axis split over the warps of a block and, when M alone cannot fill the GPU, over the blocks of a
+// cluster as well, whose sums meet in distributed shared memory and are added in rank order (so the result does not
+// depend on timing).  1280 x 1280 in fp16 6.3 -> 5.0 us and 594 x 1685 in fp32 6.0 -> 4.1 against partial sums through
+// the workspace and half as many columns in flight.
 #include <cuda_fp16.h>
 
 #include "act.cuh"
 #include "internal.h"
+#include "ptx.cuh"
 
 namespace b200 {
 
@@ -24,16 +26,22 @@ __device__ __forceinline__ void gemv_store(OutT* out, int64_t m, float acc, int 
     else out[m] = apply_act(epi, acc);
 }
 
-constexpr int GEMV_WARPS = 8;
-constexpr int GEMV_UNROLL = 4;          // columns in flight per lane: 64 bytes (8 measured no faster)
-constexpr int GEMV_BLOCKS_PER_SM = 6;   // resident blocks of 256 threads at 40 registers
-constexpr int GEMV_MIN_COLS = 16;       // columns per warp below which a further K split only adds launch work
-#define GEMV_SPLIT_ROUND(a, b) ((a) / (b))
+constexpr int GEMV_WARPS = 16;          // a multiple of 8: a warp's columns share their offset from a 16-byte boundary
+constexpr int GEMV_UNROLL = 8;          // columns in flight per lane: 128 bytes
+constexpr int GEMV_BLOCKS_PER_SM = 2;   // resident blocks of 512 threads at 64 registers
+constexpr int GEMV_SPLIT_MIN_K = 4096;  // see gemv_run
+constexpr int GEMV_MIN_COLS = 8;        // columns per warp below which a further K split only adds the join
 
-// grid (m blocks, k splits); block (32, GEMV_WARPS).
+__device__ __forceinline__ float gemv_ld_cluster(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+// grid (m blocks, k parts); block (32, GEMV_WARPS); the k parts of an m block form a cluster.
 //
-// Warp w takes columns k0 + w, k0 + w + 8, ...  Their start addresses differ by multiples of
-// 8 * lda * sizeof(T), a multiple of 16 bytes, so all of one warp's columns sit at the same offset s
+// Warp w takes columns k0 + w, k0 + w + 16, ...  Their start addresses differ by multiples of
+// 16 * lda * sizeof(T), a multiple of 16 bytes, so all of one warp's columns sit at the same offset s
 // (in elements) from a 16-byte boundary.  The warp therefore keeps its accumulators aligned to memory,
 // not to rows: lane l reads the aligned vector j = 31 * block + l of each column, whose VEC elements
 // are rows VEC * j - s ... VEC * j - s + VEC - 1, with no shifting or masking in the loop.  A block owns
@@ -45,10 +53,94 @@ constexpr int GEMV_MIN_COLS = 16;       // columns per warp below which a furthe
 template <typename T, typename OutT>
 __global__ void __launch_bounds__(32 * GEMV_WARPS, GEMV_BLOCKS_PER_SM)
 gemv_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const T* __restrict__ bias, OutT* __restrict__ out,
-            float* __restrict__ partial, int* __restrict__ arrived, int64_t M, int64_t K, int64_t kchunk, int epi) {
+            int64_t M, int64_t K, int64_t kchunk, int epi) {
     constexpr int VEC = 16 / (int)sizeof(T);
     constexpr int ROWS = 31 * VEC;
     __shared__ float red[GEMV_WARPS][ROWS];
+    __shared__ float sums[ROWS];
+    const int lane = threadIdx.x, warp = threadIdx.y, tid = warp * 32 + lane;
+    const int parts = gridDim.y;
+    const int64_t k0 = (int64_t)blockIdx.y * kchunk;
+    const int64_t k1 = k0 + kchunk < K ? k0 + kchunk : K;
+    const int64_t j = (int64_t)blockIdx.x * 31 + lane;
+    grid_dep_wait();
+    grid_dep_launch();
+    float acc[VEC];
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) acc[v] = 0.f;
+    int s = 0;
+    int64_t k = k0 + warp;
+    if (k < k1) {
+        s = (int)((reinterpret_cast<uintptr_t>(A + k * lda) & 15u) / sizeof(T));
+        if (VEC * j - s < M) {
+            // first aligned vector of column k, then + j; columns are 16 * lda elements apart
+            const uint4* vp = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(A + k * lda) - s * sizeof(T)) + j;
+            const int64_t vstep = GEMV_WARPS * lda * (int64_t)sizeof(T) / 16;
+            constexpr int UN = GEMV_UNROLL;
+            for (; k < k1; k += UN * GEMV_WARPS, vp += UN * vstep) {
+                uint4 a[UN];
+                float xv[UN];
+#pragma unroll
+                for (int u = 0; u < UN; ++u) {
+                    const bool in = k + u * GEMV_WARPS < k1;
+                    a[u] = in ? __ldg(vp + u * vstep) : make_uint4(0u, 0u, 0u, 0u);
+                    xv[u] = in ? gemv_tof<T>(x[k + u * GEMV_WARPS]) : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < UN; ++u) {
+                    const T* e = reinterpret_cast<const T*>(&a[u]);
+#pragma unroll
+                    for (int v = 0; v < VEC; ++v) acc[v] = fmaf(gemv_tof<T>(e[v]), xv[u], acc[v]);
+                }
+            }
+        }
+    }
+    // accumulator v of lane l is row VEC * l + v - s of the block
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) {
+        const int r = VEC * lane + v - s;
+        if (r >= 0 && r < ROWS) red[warp][r] = acc[v];
+    }
+    __syncthreads();
+    auto finish = [&](int r, float t) {
+        const int64_t m = (int64_t)blockIdx.x * ROWS + r;
+        if (m >= M) return;
+        if (bias != nullptr) t += gemv_tof<T>(bias[m]);
+        gemv_store<OutT>(out, m, t, epi);
+    };
+    for (int r = tid; r < ROWS; r += 32 * GEMV_WARPS) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < GEMV_WARPS; ++w) t += red[w][r];
+        if (parts > 1) sums[r] = t;
+        else finish(r, t);
+    }
+    if (parts == 1) return;
+    cluster_sync_all();   // every part's sums are in its shared memory
+    const int rank = (int)blockIdx.y;
+    const uint32_t mine = smem_u32(sums);
+    for (int r = tid * parts + rank; r < ROWS; r += 32 * GEMV_WARPS * parts) {
+        float v[8], t = 0.f;   // every part's load in flight together: a remote load takes a few hundred nanoseconds
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = q < parts ? gemv_ld_cluster(mapa_u32(mine + r * 4, (uint32_t)q)) : 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) t += v[q];
+        finish(r, t);
+    }
+    cluster_sync_all();   // nobody leaves while its sums may still be read
+}
+
+// The same with the K axis over up to 64 blocks that are not a cluster: for a few row blocks and a long reduction, which
+// eight parts leave most of the GPU out of.  Partial sums go through the workspace and are added in split order by
+// whichever block of a row range finishes last, so the result does not depend on timing.
+constexpr int GEMV_SPLIT_WARPS = 8;
+template <typename T, typename OutT>
+__global__ void __launch_bounds__(32 * GEMV_SPLIT_WARPS, 6)
+gemv_split_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const T* __restrict__ bias, OutT* __restrict__ out,
+            float* __restrict__ partial, int* __restrict__ arrived, int64_t M, int64_t K, int64_t kchunk, int epi) {
+    constexpr int VEC = 16 / (int)sizeof(T);
+    constexpr int ROWS = 31 * VEC;
+    __shared__ float red[GEMV_SPLIT_WARPS][ROWS];
     __shared__ int last;
     const int lane = threadIdx.x, warp = threadIdx.y;
     const int64_t k0 = (int64_t)blockIdx.y * kchunk;
@@ -64,15 +156,15 @@ gemv_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const
         if (VEC * j - s < M) {
             // first aligned vector of column k, then + j; columns are 8 * lda elements apart
             const uint4* vp = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(A + k * lda) - s * sizeof(T)) + j;
-            const int64_t vstep = GEMV_WARPS * lda * (int64_t)sizeof(T) / 16;
-            constexpr int UN = GEMV_UNROLL;
-            for (; k + (UN - 1) * GEMV_WARPS < k1; k += UN * GEMV_WARPS, vp += UN * vstep) {
+            const int64_t vstep = GEMV_SPLIT_WARPS * lda * (int64_t)sizeof(T) / 16;
+            constexpr int UN = 4;
+            for (; k + (UN - 1) * GEMV_SPLIT_WARPS < k1; k += UN * GEMV_SPLIT_WARPS, vp += UN * vstep) {
                 uint4 a[UN];
                 float xv[UN];
 #pragma unroll
                 for (int u = 0; u < UN; ++u) {
                     a[u] = __ldg(vp + u * vstep);
-                    xv[u] = gemv_tof<T>(x[k + u * GEMV_WARPS]);
+                    xv[u] = gemv_tof<T>(x[k + u * GEMV_SPLIT_WARPS]);
                 }
 #pragma unroll
                 for (int u = 0; u < UN; ++u) {
@@ -81,7 +173,7 @@ gemv_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const
                     for (int v = 0; v < VEC; ++v) acc[v] = fmaf(gemv_tof<T>(e[v]), xv[u], acc[v]);
                 }
             }
-            for (; k < k1; k += GEMV_WARPS, vp += vstep) {
+            for (; k < k1; k += GEMV_SPLIT_WARPS, vp += vstep) {
                 const uint4 a = __ldg(vp);
                 const float xv = gemv_tof<T>(x[k]);
                 const T* e = reinterpret_cast<const T*>(&a);
@@ -97,20 +189,14 @@ gemv_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const
         if (r >= 0 && r < ROWS) red[warp][r] = acc[v];
     }
     __syncthreads();
-    for (int r = warp * 32 + lane; r < ROWS; r += 32 * GEMV_WARPS) {
+    for (int r = warp * 32 + lane; r < ROWS; r += 32 * GEMV_SPLIT_WARPS) {
         const int64_t m = (int64_t)blockIdx.x * ROWS + r;
         if (m >= M) continue;
         float t = 0.f;
 #pragma unroll
-        for (int w = 0; w < GEMV_WARPS; ++w) t += red[w][r];
-        if (partial != nullptr) {
-            partial[(int64_t)blockIdx.y * M + m] = t;
-        } else {
-            if (bias != nullptr) t += gemv_tof<T>(bias[m]);
-            gemv_store<OutT>(out, m, t, epi);
-        }
+        for (int w = 0; w < GEMV_SPLIT_WARPS; ++w) t += red[w][r];
+        partial[(int64_t)blockIdx.y * M + m] = t;
     }
-    if (partial == nullptr || arrived == nullptr) return;
     // K was split over gridDim.y blocks: the one that arrives last adds the partial sums of these rows in
     // split order (so the result does not depend on which block that is) and puts the counter back to zero
     // for the next launch.  Nobody waits on anybody.
@@ -120,7 +206,7 @@ gemv_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const
     __syncthreads();
     if (!last) return;
     __threadfence();
-    for (int r = warp * 32 + lane; r < ROWS; r += 32 * GEMV_WARPS) {
+    for (int r = warp * 32 + lane; r < ROWS; r += 32 * GEMV_SPLIT_WARPS) {
         const int64_t m = (int64_t)blockIdx.x * ROWS + r;
         if (m >= M) continue;
         float t = 0.f;
@@ -132,51 +218,57 @@ gemv_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const
 }
 
 template <typename T, typename OutT>
-__global__ void __launch_bounds__(256)
-gemv_finish_kernel(const float* __restrict__ partial, int ksplit, const T* __restrict__ bias, OutT* __restrict__ out, int64_t M,
-                   int epi) {
-    const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (m >= M) return;
-    float s = 0.f;
-    for (int j = 0; j < ksplit; ++j) s += partial[(int64_t)j * M + m];
-    if (bias != nullptr) s += gemv_tof<T>(bias[m]);
-    gemv_store<OutT>(out, m, s, epi);
-}
-
-template <typename T, typename OutT>
 static int gemv_run(b200_ctx* ctx, int64_t M, int64_t K, const void* A, int64_t lda, const void* x, const void* bias, void* out,
                     int epi) {
     constexpr int ROWS = 31 * (16 / (int)sizeof(T));
     const int64_t mblocks = cdiv(M, ROWS);
-    // Split K over blocks until the grid is one resident wave (a second, partial wave would cost a whole
-    // extra pass of latency), keeping at least GEMV_MIN_COLS columns per warp in every split.
-    const int64_t wave = (int64_t)ctx->prop.multiProcessorCount * GEMV_BLOCKS_PER_SM;
-    int64_t ksplit = mblocks >= wave ? 1 : GEMV_SPLIT_ROUND(wave, mblocks);
-    const int64_t maxsplit = K / (GEMV_MIN_COLS * GEMV_WARPS) > 0 ? K / (GEMV_MIN_COLS * GEMV_WARPS) : 1;
-    if (ksplit > maxsplit) ksplit = maxsplit;
-    if (ksplit > 64) ksplit = 64;
-    const int64_t kchunk = K > 0 ? cdiv(K, ksplit) : 1;   // K = 0: one block per row range writes the bias
-    ksplit = K > 0 ? cdiv(K, kchunk) : 1;
-    float* partial = nullptr;
-    if (ksplit > 1) {
+    B200_REQUIRE(mblocks < (1ll << 31), B200_DECLINE_EXTENT, "gemv: M = %lld", (long long)M);
+    // Split K over a cluster's blocks as long as that shortens the time in waves of resident blocks (a last, partial
+    // wave costs a whole one) and every warp keeps GEMV_MIN_COLS columns.
+    // (Up to an SM per block while there are that many SMs: a second block on some of them is a longer chain there.)
+    const int64_t wave = (int64_t)ctx->prop.multiProcessorCount * (mblocks > ctx->prop.multiProcessorCount ? GEMV_BLOCKS_PER_SM : 1);
+    int64_t parts = 1;
+    double best = (double)cdiv(mblocks, wave);
+    for (int64_t p = 2; p <= 8 && K >= p * GEMV_WARPS * GEMV_MIN_COLS; p *= 2) {
+        const double t = (double)cdiv(p * mblocks, wave) / (double)p;
+        if (t < 0.9 * best) {
+            best = t;
+            parts = p;
+        }
+    }
+    // Eight parts of so few row blocks would leave nine tenths of the SMs idle over a long chain (256 x 4096: 6.35 us
+    // this way, 6.44 as a cluster; 480 x 2500: 6.8 against 5.7).
+    if (mblocks * 8 * 8 <= ctx->prop.multiProcessorCount && K >= GEMV_SPLIT_MIN_K && ctx->sk_flags != nullptr) {
+        int64_t ksplit = K / (16 * GEMV_SPLIT_WARPS);
+        if (ksplit > 64) ksplit = 64;
+        const int64_t chunk = cdiv(K, ksplit);
+        ksplit = cdiv(K, chunk);
         void* ws = nullptr;
         int rc = ws_scratch(ctx, (size_t)ksplit * M * sizeof(float), &ws);
         if (rc) return rc;
-        partial = static_cast<float*>(ws);
-    }
-    B200_REQUIRE(mblocks < (1ll << 31), B200_DECLINE_EXTENT, "gemv: M = %lld", (long long)M);
-    dim3 grid((unsigned)mblocks, (unsigned)ksplit), block(32, GEMV_WARPS);
-    int* arrived = partial != nullptr && mblocks <= GEMV_COUNTER_COUNT && ctx->sk_flags != nullptr ? ctx->sk_flags + SK_FLAG_COUNT : nullptr;
-    gemv_kernel<T, OutT><<<grid, block, 0, ctx->stream>>>((const T*)A, lda, (const T*)x, (const T*)bias, (OutT*)out, partial,
-                                                          arrived, M, K, kchunk, epi);
-    ctx->launches++;
-    B200_CUDA(cudaGetLastError());
-    if (partial != nullptr && arrived == nullptr) {
-        gemv_finish_kernel<T, OutT><<<(unsigned)cdiv(M, 256), 256, 0, ctx->stream>>>(partial, (int)ksplit, (const T*)bias,
-                                                                                  (OutT*)out, M, epi);
+        gemv_split_kernel<T, OutT><<<dim3((unsigned)mblocks, (unsigned)ksplit), dim3(32, GEMV_SPLIT_WARPS), 0, ctx->stream>>>(
+            (const T*)A, lda, (const T*)x, (const T*)bias, (OutT*)out, static_cast<float*>(ws), ctx->sk_flags + SK_FLAG_COUNT, M, K,
+            chunk, epi);
         ctx->launches++;
         B200_CUDA(cudaGetLastError());
+        return B200_OK;
     }
+    const int64_t kchunk = K > 0 ? cdiv(K, parts) : 1;   // K = 0: one block per row range writes the bias
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)mblocks, (unsigned)parts, 1);
+    cfg.blockDim = dim3(32, GEMV_WARPS, 1);
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = (unsigned)parts;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    B200_CUDA(cudaLaunchKernelEx(&cfg, gemv_kernel<T, OutT>, (const T*)A, lda, (const T*)x, (const T*)bias, (OutT*)out, M, K, kchunk, epi));
+    ctx->launches++;
     return B200_OK;
 }
 
