@@ -108,6 +108,12 @@ int attention_window_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
                             const b200_strided4* k, const b200_strided4* v, const b200_strided4* o, int out_dtype,
                             float scale);
 
+// Attention of at most 32 queries (attention_few.cu); operands as above, E <= 128.  bs: the mask's element strides
+// (keys, queries, heads, batch; 0 on a broadcast axis).
+int attention_few_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B, const b200_strided4* q,
+                         const b200_strided4* k, const b200_strided4* v, const void* bias, const int64_t* bs,
+                         const b200_strided4* o, int out_dtype, float scale);
+
 // GEMM with the bias broadcast along either axis (bias_per_n = 1: one value per column j,
 // which is what a convolution lowered to a GEMM over pixels needs).  use_workspace = 0 keeps the
 // planner to schedules that need no scratch memory (whole tiles only), so the call touches neither

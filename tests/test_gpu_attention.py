@@ -371,3 +371,34 @@ def test_masked_blocks_staged_ahead(ctx, ora, shape, bshape, extra):
     assert relerr(got, ref) < TOL, describe(got, ref, TOL)
     if bshape[2] > 2:
         assert np.all(got[:, :, 1] == 0)
+
+
+# (B, H, Lq, Lk, E): the edges of the query tiles (16, 32) and of the key blocks (64), one block and 128 of them, every
+# width of head, parts of a cluster that get different numbers of blocks
+FEW = [(1, 1, 1, 1, 8), (1, 2, 16, 63, 64), (2, 3, 17, 64, 56), (1, 5, 16, 65, 72), (1, 2, 9, 129, 128), (1, 1, 32, 8192, 64),
+       (1, 5, 32, 65, 40), (1, 19, 7, 345, 56), (1, 8, 13, 4096, 80), (3, 4, 5, 1003, 128), (40, 8, 16, 49, 72)]
+
+
+@pytest.mark.parametrize("B,H,Lq,Lk,E", FEW)
+@pytest.mark.parametrize("masked", [False, True])
+def test_few_queries_in_one_launch(ctx, ora, B, H, Lq, Lk, E, masked):
+    rng = np.random.default_rng(B + H + Lq + Lk + E)
+    buf = np.float16(rng.standard_normal((B, Lk, 2, H, E)))              # keys and values side by side
+    k, v = (buf[:, :, i].transpose(0, 2, 1, 3) for i in range(2))
+    q = np.float16(rng.standard_normal((B, H, Lq, E)))
+    bias = None
+    if masked:
+        bias = np.float16(rng.standard_normal((B, 1, Lq, Lk)))
+        bias[rng.random(bias.shape) < 0.2] = -np.inf
+        bias[:, :, 0, : Lk // 2] = -np.inf
+        bias[:, :, Lq - 1] = -np.inf
+    ref = ora.attention_ref(q, k, v, 1 / np.sqrt(E), bias=bias)
+    for out_dtype in (np.float16, np.float32):
+        n0 = ctx.launch_count()
+        got, plan = attention_gpu(ctx, q, k, v, 1 / np.sqrt(E), out_dtype, bias=bias)
+        assert isinstance(plan, jv.FlashTCPlan) and ctx.launch_count() - n0 == 1
+        assert np.all(np.isfinite(got))
+        # P is rounded to fp16 (2^-11 per key, averaged over them) and, for fp16, the result once more
+        assert relerr(got, ref) < 2e-3, describe(got, ref, 2e-3)
+        if masked:
+            assert np.all(got[:, :, Lq - 1] == 0)
