@@ -23,13 +23,13 @@
 namespace b200 {
 
 constexpr int ATT_BR = 128;  // queries per tile (TMEM lanes)
-constexpr int ATT_BC = 128;  // keys per block
-constexpr int ATT_THREADS = 384;  // warps 0-3, 4-7: softmax of tile 0, 1; warp 8: TMA; warps 9, 10: UMMA; 11 idle
 constexpr int ATT_TILE_BYTES = 128 * 128; // one swizzle atom of an operand tile: 128 rows x 128 B (64 fp16 of E)
 #ifndef ATT_TURN_AT
 #define ATT_TURN_AT 2   // after which quarter (0..3) of its exponentials a tile passes the turn
 #endif
-// Two shapes of CTA, chosen by the head dimension:
+// Two shapes of CTA, chosen by the head dimension, and a third for short keys:
+//   EP = 64, NT = 1:           one query tile, key blocks of 64, P over S, 128 tensor-memory columns and 48 KB, so that
+//                              four CTAs share an SM
 //   EP = 64  (E <= 64):        two query tiles of 128 per CTA, K/V rings of 4 stages x 16 KB
 //   EP = 128 (64 < E <= 128):  two query tiles of 128 per CTA as well; every operand tile is two swizzle atoms along
 //                              E (columns 0-63, 64-127, the second zero-filled past E by the tensor map), S = Q K'
@@ -45,30 +45,37 @@ constexpr int ATT_TILE_BYTES = 128 * 128; // one swizzle atom of an operand tile
 // (an odd number of 8-byte units, so that a warp's 32 rows lie in all banks); others word by word, from the 4-byte
 // boundary at or one entry before the first, 65 words apart (odd, for the same reason).
 constexpr int BIAS_ROW_WORDS = 66;
-template <int EP, bool BIAS = false> struct AttCfg {
+template <int EP, bool BIAS = false, int NT_ = 2> struct AttCfg {
     static_assert(EP == 64 || EP == 128, "head dim is padded to one or two swizzle atoms");
     static constexpr int ATOMS = EP / 64;              // 16 KB atoms per operand tile
-    static constexpr int NT = 2;                       // query tiles per CTA
-    static constexpr int K_STAGES = EP == 64 ? 4 : 2;
-    static constexpr int V_STAGES = EP == 64 ? 4 : (BIAS ? 1 : 2);
-    static constexpr bool P_IN_S = EP == 128;          // P shares its tile's S columns (tensor memory is full otherwise)
-    static constexpr int OP_BYTES = ATOMS * ATT_TILE_BYTES;   // one Q, K or V tile
-    // shared-memory map, in 16 KB atoms
-    static constexpr int T_Q = 0;                              // NT tiles
-    static constexpr int T_K = NT * ATOMS;                     // K_STAGES tiles
-    static constexpr int T_V = T_K + K_STAGES * ATOMS;         // V_STAGES tiles
-    static constexpr int T_END = T_V + V_STAGES * ATOMS;
+    static constexpr int NT = NT_;                     // query tiles per CTA
+    static_assert(NT == 2 || (NT == 1 && EP == 64 && !BIAS), "one tile per CTA is built for E <= 64 without a mask");
+    static constexpr int BC = NT == 2 ? 128 : 64;      // keys per block
+    static constexpr int CTAS_PER_SM = NT == 2 ? 1 : 4;
+    static constexpr int THREADS = 128 * NT + 128;     // NT softmax warpgroups, then TMA, UMMA and idle warps
+    static constexpr int TMA_WARP = 4 * NT, ISSUE_WARP = 4 * NT + 1;
+    // registers of a softmax thread and of the others: (NT x 128 x one + 128 x the other) is what the launch holds
+    static constexpr int SOFTMAX_REGS = NT == 2 ? 232 : 96, OTHER_REGS = NT == 2 ? 40 : 32;
+    static constexpr int TMEM_COLS = NT == 2 ? 512 : 128;
+    // S of tile t at BC t, O at O_COL + EP t, P of its own at P_COL + 64 t
+    static constexpr int O_COL = NT * BC, P_COL = 384;
+    static constexpr int K_STAGES = NT == 2 && EP == 64 ? 4 : 2;
+    static constexpr int V_STAGES = NT == 2 && EP == 64 ? 4 : (BIAS ? 1 : 2);
+    static constexpr bool P_IN_S = EP == 128 || NT == 1;   // P shares its tile's S columns (tensor memory is full otherwise)
+    static constexpr int Q_BYTES = ATOMS * ATT_TILE_BYTES;    // one Q tile
+    static constexpr int KV_ATOM = BC * 128, KV_BYTES = ATOMS * KV_ATOM;   // one K or V tile
+    // shared-memory map
+    static constexpr int S_Q = 0;                              // NT tiles
+    static constexpr int S_K = NT * Q_BYTES;                   // K_STAGES tiles
+    static constexpr int S_V = S_K + K_STAGES * KV_BYTES;      // V_STAGES tiles
+    static constexpr int S_END = S_V + V_STAGES * KV_BYTES;
     static constexpr int BIAS_TILE_BYTES = BIAS ? ATT_BR * BIAS_ROW_WORDS * 4 : 0;
-    static constexpr int SMEM_BYTES = T_END * ATT_TILE_BYTES + NT * BIAS_TILE_BYTES + 256;
-    static_assert(SMEM_BYTES <= 232448, "shared memory over budget");
+    static constexpr int SMEM_BYTES = S_END + NT * BIAS_TILE_BYTES + 256;
+    static_assert(CTAS_PER_SM * (SMEM_BYTES + 1024) <= 233472, "shared memory over budget");
 };
-// tensor-memory map (512 columns): S of tile t, fp32, at [128 t, 128 t + 128); O of tile t, fp32, at
+// tensor-memory map of two tiles (512 columns): S of tile t, fp32, at [128 t, 128 t + 128); O of tile t, fp32, at
 // [256 + EP t, ... + EP); P of tile t, fp16 packed two keys per column, at [384 + 64 t, ... + 64) for EP = 64 and
 // over the first 64 columns of S_t for EP = 128
-constexpr int ATT_TMEM_COLS = 512;
-constexpr int ATT_S_COL = 0;
-constexpr int ATT_O_COL = 256;
-constexpr int ATT_P_COL = 384;
 
 struct AttnParams {
     int E, Lq, Lk, H, B;
@@ -126,6 +133,11 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -159,13 +171,14 @@ __device__ __forceinline__ void tmem_st16_raw(uint32_t taddr, const uint32_t* r)
 // the P V product takes its A operand from there, so the shared-memory port only feeds K and V.
 // BIAS: the scaled score gets an additive fp16 mask before the softmax; a row whose keys are all
 // blocked (-inf everywhere) comes out as zeros, as in attn_softmax (attention.jl:73-100).
-template <int EP, bool BIAS>
-__global__ void __launch_bounds__(ATT_THREADS, 1)
+template <int EP, bool BIAS, int NT_>
+__global__ void __launch_bounds__(AttCfg<EP, BIAS, NT_>::THREADS, AttCfg<EP, BIAS, NT_>::CTAS_PER_SM)
 attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                         const __grid_constant__ CUtensorMap tmapK,
                         const __grid_constant__ CUtensorMap tmapV, const AttnParams p) {
-    using Cfg = AttCfg<EP, BIAS>;
+    using Cfg = AttCfg<EP, BIAS, NT_>;
     constexpr int K_STAGES = Cfg::K_STAGES, V_STAGES = Cfg::V_STAGES;
+    constexpr int BC = Cfg::BC, NC = BC / 32;   // keys per block, and per-thread pieces of 32 of them
     constexpr int NT = Cfg::NT;
     constexpr int ITEM_ROWS = NT * ATT_BR;   // queries one whole work item covers
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -175,8 +188,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
         if (threadIdx.x == 0) atomicCAS(p.d_status, 0, KST_SMEM_LAYOUT);
         return;
     }
-    auto tile_ptr = [&](int t) { return smem + t * ATT_TILE_BYTES; };
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::T_END * ATT_TILE_BYTES + NT * Cfg::BIAS_TILE_BYTES);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::S_END + NT * Cfg::BIAS_TILE_BYTES);
     uint64_t* q_full = bars + 0;                           // [2]
     uint64_t* k_full = bars + 2;                           // [K_STAGES]
     uint64_t* k_empty = k_full + K_STAGES;                 // [K_STAGES]
@@ -215,7 +227,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
     const int h = (item / p.qpairs) % p.H;
     const int b = item / (p.qpairs * p.H);
     const int q0 = qp * ITEM_ROWS + (half > 0 ? ATT_BR : 0);
-    const int nblk_all = (p.Lk + ATT_BC - 1) / ATT_BC;
+    const int nblk_all = (p.Lk + BC - 1) / BC;
     const int jb0 = (int)((int64_t)split * nblk_all / nsp);           // first key block of this CTA
     const int nblk = (int)((int64_t)(split + 1) * nblk_all / nsp) - jb0;
     const int ntiles = (NT == 2 && half < 0 && q0 + ATT_BR < p.Lq) ? 2 : 1;   // the second tile may lie wholly past Lq
@@ -244,8 +256,8 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
         prefetch_tmap(&tmapK);
         prefetch_tmap(&tmapV);
     }
-    if (warp == 8) {
-        tmem_alloc(tmem_slot, ATT_TMEM_COLS);
+    if (warp == Cfg::TMA_WARP) {
+        tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -259,53 +271,53 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
     // Register budget: the two softmax warpgroups hold a full score row per thread; the third
     // warpgroup (one TMA lane, one UMMA lane, two idle warps) needs almost nothing and hands its
     // share over (setmaxnreg at the head of each role's branch).
-    if (warp == 11) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    } else if (warp == 8) {
+    if (warp == 4 * NT + 3 || (NT == 1 && warp == 6)) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::OTHER_REGS));
+    } else if (warp == Cfg::TMA_WARP) {
         // ------------------------------------------------------------- TMA producer
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::OTHER_REGS));
         if (lane == 0) {
             for (int t = 0; t < ntiles; ++t) {
-                mbar_arrive_expect_tx(&q_full[t], Cfg::OP_BYTES);
+                mbar_arrive_expect_tx(&q_full[t], Cfg::Q_BYTES);
 #pragma unroll
                 for (int a = 0; a < Cfg::ATOMS; ++a)
-                    tma_load_4d(tile_ptr(Cfg::T_Q + t * Cfg::ATOMS + a), &tmapQ, &q_full[t], a * 64, q0 + t * ATT_BR, h, b);
+                    tma_load_4d(smem + Cfg::S_Q + t * Cfg::Q_BYTES + a * ATT_TILE_BYTES, &tmapQ, &q_full[t], a * 64, q0 + t * ATT_BR, h, b);
             }
             for (int j = 0; j < nblk; ++j) {
                 const int s = j % K_STAGES, sv = j % V_STAGES;
                 const uint32_t ph = (uint32_t)((j / K_STAGES) & 1), phv = (uint32_t)((j / V_STAGES) & 1);
                 if (!mbar_wait(&k_empty[s], ph ^ 1, p.d_status, KST_WAIT_EMPTY, abort_flag)) break;
-                mbar_arrive_expect_tx(&k_full[s], Cfg::OP_BYTES);
+                mbar_arrive_expect_tx(&k_full[s], Cfg::KV_BYTES);
 #pragma unroll
                 for (int a = 0; a < Cfg::ATOMS; ++a)
-                    tma_load_4d(tile_ptr(Cfg::T_K + s * Cfg::ATOMS + a), &tmapK, &k_full[s], a * 64, (jb0 + j) * ATT_BC, h, b);
+                    tma_load_4d(smem + Cfg::S_K + s * Cfg::KV_BYTES + a * Cfg::KV_ATOM, &tmapK, &k_full[s], a * 64, (jb0 + j) * BC, h, b);
                 if (!mbar_wait(&v_empty[sv], phv ^ 1, p.d_status, KST_WAIT_EMPTY, abort_flag)) break;
-                mbar_arrive_expect_tx(&v_full[sv], Cfg::OP_BYTES);
+                mbar_arrive_expect_tx(&v_full[sv], Cfg::KV_BYTES);
 #pragma unroll
                 for (int a = 0; a < Cfg::ATOMS; ++a)
-                    tma_load_4d(tile_ptr(Cfg::T_V + sv * Cfg::ATOMS + a), &tmapV, &v_full[sv], a * 64, (jb0 + j) * ATT_BC, h, b);
+                    tma_load_4d(smem + Cfg::S_V + sv * Cfg::KV_BYTES + a * Cfg::KV_ATOM, &tmapV, &v_full[sv], a * 64, (jb0 + j) * BC, h, b);
             }
         }
-    } else if (warp == 9 || warp == 10) {
+    } else if (warp == Cfg::ISSUE_WARP || (NT == 2 && warp == Cfg::ISSUE_WARP + 1)) {
         // ------------------------------------------------------------- UMMA issuers
         // One issuing lane per query tile (warp 9: tile 0, warp 10: tile 1).  Each walks its own
         // chain  S_t(j+1) = Q_t K(j+1)'  as soon as the softmax has pulled S_t(j) into registers,
         // then  O_t += P_t(j) V(j)  once P_t(j) is written.  The two chains share only the
         // K/V rings.  (Issuing a UMMA blocks while the tensor pipe is busy, so the issuing lanes
         // are not softmax threads.)
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-        const int t = warp - 9;
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::OTHER_REGS));
+        const int t = warp - Cfg::ISSUE_WARP;
         if (lane == 0 && t < ntiles) {
             // S = Q K': both operands K-major (E contiguous), from shared memory.  O += P V: P from
             // tensor memory, V MN-major (E contiguous per key) from shared memory.
-            constexpr uint32_t idesc_s = make_idesc_f16(ATT_BR, ATT_BC, 0, 0);
+            constexpr uint32_t idesc_s = make_idesc_f16(ATT_BR, BC, 0, 0);
             constexpr uint32_t idesc_o = make_idesc_f16(ATT_BR, EP, 0, 1);
             constexpr uint64_t kdesc0 = make_smem_desc(16, 1024);
-            constexpr uint64_t vdesc0 = make_smem_desc(ATT_TILE_BYTES, 1024);
-            const uint32_t q_addr = smem_u32(tile_ptr(Cfg::T_Q + t * Cfg::ATOMS));
-            const uint32_t s_tmem = tmem_base + ATT_S_COL + t * 128;
-            const uint32_t o_tmem = tmem_base + ATT_O_COL + t * EP;
-            const uint32_t p_tmem = Cfg::P_IN_S ? s_tmem : tmem_base + ATT_P_COL + t * 64;
+            constexpr uint64_t vdesc0 = make_smem_desc(Cfg::KV_ATOM, 1024);
+            const uint32_t q_addr = smem_u32(smem + Cfg::S_Q + t * Cfg::Q_BYTES);
+            const uint32_t s_tmem = tmem_base + t * BC;
+            const uint32_t o_tmem = tmem_base + Cfg::O_COL + t * EP;
+            const uint32_t p_tmem = Cfg::P_IN_S ? s_tmem : tmem_base + Cfg::P_COL + t * 64;
 
             auto issue_qk = [&](int j) -> bool {
                 const int sk = j % K_STAGES;
@@ -317,12 +329,14 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                     !mbar_wait(&s_empty[t], (uint32_t)((j - 1) & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag))
                     return false;
                 tc_fence_after();
-                const uint32_t k_addr = smem_u32(tile_ptr(Cfg::T_K + sk * Cfg::ATOMS));
+                const uint32_t k_addr = smem_u32(smem + Cfg::S_K + sk * Cfg::KV_BYTES);
 #pragma unroll
                 for (int k = 0; k < EP / 16; ++k) {
+                    if (k * 16 >= p.E) break;   // past the head dim both operands are zeros (E = 72: five of eight steps)
                     // 16 elements of E = 32 B inside the swizzle row; every fourth step moves to the next atom
-                    const uint32_t off = (uint32_t)(k >> 2) * ATT_TILE_BYTES + (uint32_t)(k & 3) * 32;
-                    umma_ss(s_tmem, smem_desc_at(kdesc0, q_addr + off), smem_desc_at(kdesc0, k_addr + off), idesc_s, k != 0);
+                    const uint32_t in = (uint32_t)(k & 3) * 32;
+                    umma_ss(s_tmem, smem_desc_at(kdesc0, q_addr + (uint32_t)(k >> 2) * ATT_TILE_BYTES + in),
+                            smem_desc_at(kdesc0, k_addr + (uint32_t)(k >> 2) * Cfg::KV_ATOM + in), idesc_s, k != 0);
                 }
                 umma_commit(&s_full[t]);
                 umma_commit(&k_empty[sk]);   // one of `ntiles` arrivals that free this K stage
@@ -339,9 +353,9 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                 if (j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 7);   // issuer reaches its wait for P(j)
                 if (!mbar_wait(&p_full[t], (uint32_t)(j & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag)) break;
                 tc_fence_after();
-                const uint32_t v_addr = smem_u32(tile_ptr(Cfg::T_V + sv * Cfg::ATOMS));
+                const uint32_t v_addr = smem_u32(smem + Cfg::S_V + sv * Cfg::KV_BYTES);
 #pragma unroll
-                for (int k = 0; k < ATT_BC / 16; ++k) {
+                for (int k = 0; k < BC / 16; ++k) {
                     // P comes from tensor memory: 16 keys = 8 packed columns per step.
                     // V: 16 key rows = two 8-row groups = 2048 B.
                     umma_ts(o_tmem, p_tmem + k * 8, smem_desc_at(vdesc0, v_addr + k * 2048), idesc_o, (j | k) != 0);
@@ -354,15 +368,15 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
         }
     } else {
         // ------------------------------------------------------- softmax + epilogue
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::SOFTMAX_REGS));
         const int t = warp >> 2;               // which query tile this warpgroup owns
         const int quad = warp & 3;             // TMEM lane quadrant
         const int row = quad * 32 + lane;
         if (t < ntiles) {
             const uint32_t lane_base = uint32_t(quad * 32) << 16;
-            const uint32_t s_tmem = tmem_base + lane_base + ATT_S_COL + t * 128;
-            const uint32_t o_tmem = tmem_base + lane_base + ATT_O_COL + t * EP;
-            const uint32_t p_tmem = Cfg::P_IN_S ? s_tmem : tmem_base + lane_base + ATT_P_COL + t * 64;
+            const uint32_t s_tmem = tmem_base + lane_base + t * BC;
+            const uint32_t o_tmem = tmem_base + lane_base + Cfg::O_COL + t * EP;
+            const uint32_t p_tmem = Cfg::P_IN_S ? s_tmem : tmem_base + lane_base + Cfg::P_COL + t * 64;
             const float sc = BIAS ? p.scale : p.scale_log2;
             const float sce = BIAS ? 1.4426950408889634f : sc;   // with a bias the scores are scaled when it is added
             float m_run = -INFINITY, l_run = 0.f;
@@ -381,14 +395,14 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             // shifted when read.  Every piece copied holds an entry of the mask.  Read straight from global memory, one
             // row per thread, 20 heads x 1500 x 1500 took 152 us, with words copied 56, with 8 bytes at a time 45 (24
             // without a mask: adding it is 64 more packed FMAs, 128 conversions and the reads per thread and block).
-            uint32_t* bias_rows = reinterpret_cast<uint32_t*>(smem + Cfg::T_END * ATT_TILE_BYTES) + (t * ATT_BR + quad * 32) * BIAS_ROW_WORDS;
+            uint32_t* bias_rows = reinterpret_cast<uint32_t*>(smem + Cfg::S_END) + (t * ATT_BR + quad * 32) * BIAS_ROW_WORDS;
             const bool bias_async = BIAS && p.bias != nullptr && p.bias_async;
             const bool bias8 = BIAS && p.bias_async == 2;
             auto bias_fetch = [&](int j) {
-                const int keys = min(ATT_BC, p.Lk - (jb0 + j) * ATT_BC);
+                const int keys = min(BC, p.Lk - (jb0 + j) * BC);
                 const int rows = min(32, p.Lq - (q0 + t * ATT_BR + quad * 32));   // rows of this warp that exist
                 const char* src = reinterpret_cast<const char*>(p.bias + (int64_t)(q0 + t * ATT_BR + quad * 32) * p.bsQ +
-                                                                (int64_t)h * p.bsH + (int64_t)b * p.bsB + (int64_t)(jb0 + j) * ATT_BC);
+                                                                (int64_t)h * p.bsH + (int64_t)b * p.bsB + (int64_t)(jb0 + j) * BC);
                 const uint32_t dst = smem_u32(bias_rows);
                 if (bias8) {
                     if (4 * lane < keys) {
@@ -407,7 +421,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                     }
                     if (lane < rows) {   // a row's 65th word, when its 128 entries start in the middle of a word
                         const uintptr_t a = reinterpret_cast<uintptr_t>(src) + (int64_t)lane * p.bsQ * 2;
-                        if ((a & 2) && keys == ATT_BC)
+                        if ((a & 2) && keys == BC)
                             cp_async4(dst + lane * 260 + 256, reinterpret_cast<const char*>((a & ~(uintptr_t)3) + 256));
                     }
                 }
@@ -418,14 +432,14 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             for (int j = 0; ok && j < nblk; ++j) {
                 if (!mbar_wait(&s_full[t], (uint32_t)(j & 1), p.d_status, KST_WAIT_TMEM_FULL, abort_flag)) { ok = false; break; }
                 tc_fence_after();
-                const int nvalid = p.Lk - (jb0 + j) * ATT_BC; // keys of this block that exist (>= 128 when full)
+                const int nvalid = p.Lk - (jb0 + j) * BC; // keys of this block that exist (>= BC when full)
                 if (lane == 0 && quad == 0 && j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 2);  // S(0, j) ready
 
                 // The whole row of S (128 fp32) comes into registers in one round trip; S is then
                 // free for the next Q K' of this tile.
-                uint32_t r[4][32];
+                uint32_t r[NC][32];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) tmem_ld32(s_tmem + c * 32, r[c]);
+                for (int c = 0; c < NC; ++c) tmem_ld32(s_tmem + c * 32, r[c]);
                 tmem_wait_ld();
                 tc_fence_before();
                 __syncwarp();
@@ -437,12 +451,12 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                     const int lq = q0 + t * ATT_BR + row;
                     if (p.bias == nullptr) {
 #pragma unroll
-                        for (int c = 0; c < 4; ++c)
+                        for (int c = 0; c < NC; ++c)
 #pragma unroll
                             for (int i = 0; i < 32; ++i) r[c][i] = __float_as_uint(__uint_as_float(r[c][i]) * sc);
                     } else {
                         const __half* brow = p.bias + (int64_t)(lq < p.Lq ? lq : 0) * p.bsQ + (int64_t)h * p.bsH +
-                                             (int64_t)b * p.bsB + (int64_t)(jb0 + j) * ATT_BC * p.bsK;
+                                             (int64_t)b * p.bsB + (int64_t)(jb0 + j) * BC * p.bsK;
                         if (bias_async) {
                             cp_async_wait_all();
                             __syncwarp();
@@ -459,7 +473,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                             if (bias8) {
                                 const uint2* w = reinterpret_cast<const uint2*>(bias_rows + lane * 66);
 #pragma unroll
-                                for (int c = 0; c < 4; ++c)
+                                for (int c = 0; c < NC; ++c)
 #pragma unroll
                                     for (int i = 0; i < 16; i += 2) {
                                         const uint2 four = w[c * 8 + i / 2];
@@ -471,7 +485,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                                 const uint32_t shift = (uint32_t)(reinterpret_cast<uintptr_t>(brow) & 2) * 8;   // 16: the row starts mid-word
                                 uint32_t lo = w[0];
 #pragma unroll
-                                for (int c = 0; c < 4; ++c)
+                                for (int c = 0; c < NC; ++c)
 #pragma unroll
                                     for (int i = 0; i < 16; ++i) {
                                         const uint32_t hi = w[c * 16 + i + 1];
@@ -483,7 +497,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                             if (j + 1 < nblk) bias_fetch(j + 1);
                         } else {
 #pragma unroll
-                            for (int c = 0; c < 4; ++c)
+                            for (int c = 0; c < NC; ++c)
 #pragma unroll
                                 for (int i = 0; i < 32; ++i) {
                                     const float bv = (c * 32 + i < nvalid) ? __half2float(brow[(int64_t)(c * 32 + i) * p.bsK]) : 0.f;
@@ -494,16 +508,16 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                 }
                 // Row maximum of the raw scores (the scale is positive, so it commutes with max);
                 // eight independent chains instead of one 128-long dependent one.
-                if (nvalid < ATT_BC) {
+                if (nvalid < BC) {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c)
+                    for (int c = 0; c < NC; ++c)
 #pragma unroll
                         for (int i = 0; i < 32; ++i)
                             if (c * 32 + i >= nvalid) r[c][i] = 0xff800000u; // -inf: a key that does not exist gives 2^-inf = 0
                 }
                 float mxa = -INFINITY, mxb = -INFINITY, mxc = -INFINITY, mxd = -INFINITY;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < NC; ++c) {
 #pragma unroll
                     for (int i = 0; i < 32; i += 8) {   // three-input max: two scores per instruction
                         mxa = fmax3(mxa, __uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1]));
@@ -557,7 +571,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                 const uint64_t sc2 = pack2(sce, sce), nm2 = pack2(-m_sub, -m_sub);
                 uint64_t lsa = pack2(0.f, 0.f), lsb = pack2(0.f, 0.f);
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < NC; ++c) {
                     uint32_t pk[16];
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
@@ -574,7 +588,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                     tmem_st16_raw(p_tmem + c * 16, pk);
                     // Hand the turn over part way: the other tile's exponentials then overlap the
                     // rest of these, which keeps the MUFU pipe fed without falling in step.
-                    if (c == ATT_TURN_AT && pingpong) {
+                    if (c == ATT_TURN_AT && NC == 4 && pingpong) {
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&exp_turn[1 - t]);
                     }
@@ -666,9 +680,9 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 8) {
+    if (warp == Cfg::TMA_WARP) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, ATT_TMEM_COLS);
+        tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
     }
 }
 
@@ -884,7 +898,7 @@ static int tc_reason(int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B, co
 }
 
 static int make_qkv_map(b200_ctx* ctx, CUtensorMap* m, const b200_strided4* t, int64_t E, int64_t L,
-                        int64_t H, int64_t B) {
+                        int64_t H, int64_t B, uint32_t rows) {
     uint64_t dims[4] = {(uint64_t)E, (uint64_t)L, (uint64_t)H, (uint64_t)B};
     // A unit-extent axis may carry any stride; give the encoder a legal one.
     auto st = [&](int d, uint64_t fallback) {
@@ -895,7 +909,7 @@ static int make_qkv_map(b200_ctx* ctx, CUtensorMap* m, const b200_strided4* t, i
     uint64_t s2 = st(2, s1 * (uint64_t)L);
     uint64_t s3 = st(3, s2 * (uint64_t)H);
     uint64_t str[3] = {s1, s2, s3};
-    uint32_t box[4] = {64, 128, 1, 1};   // one swizzle atom; a head dim above 64 takes two boxes per tile
+    uint32_t box[4] = {64, rows, 1, 1};   // one swizzle atom; a head dim above 64 takes two boxes per tile
     return make_tmap(ctx, m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, t->ptr, dims, str, box,
                      CU_TENSOR_MAP_SWIZZLE_128B);
 }
@@ -992,13 +1006,15 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     }
     static bool attr_done[16] = {};
     if (!attr_done[ctx->device & 15]) {
-        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<64, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       AttCfg<64, false, 1>::SMEM_BYTES));
+        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<64, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        AttCfg<64>::SMEM_BYTES));
-        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<64, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        AttCfg<64, true>::SMEM_BYTES));
-        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<128, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        AttCfg<128>::SMEM_BYTES));
-        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<128, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        AttCfg<128, true>::SMEM_BYTES));
         attr_done[ctx->device & 15] = true;
     }
@@ -1009,11 +1025,19 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     // A few queries: their tile would be mostly empty (see attention_few.cu).  Past 16, and past 32 with E <= 64, a warp
     // has too much of the chain to itself: 40 x 1500, E = 72, 20 heads took 19.5 us there and 13.1 here.
     if (Lq <= (E <= 64 ? 32 : 16)) return attention_few_launch(ctx, E, Lq, Lk, H, B, q, k, v, bptr, bs, o, out_dtype, scale);
+    const bool wide = E > 64;                              // two swizzle atoms along E
+    const int64_t sms = ctx->prop.multiProcessorCount;
+    // Up to 256 keys and more than two tiles per SM (16 x 16 windows): one tile per CTA, four CTAs per SM, so that one's
+    // set-up, loads and hand-offs run under the others' arithmetic: 1024 of 256 x 256, E = 56: 65 -> 54 us, 287 of 196 x
+    // 196: 17.0 -> 15.4.  With long keys its blocks of 64 hold the tensor pipe as long as blocks of 128 (64 cycles a UMMA
+    // whatever N), and it loses: 12 heads x 4096 x 4096 85.7 -> 126.7.
+    const bool single = !wide && bptr == nullptr && Lk <= 256 && cdiv(Lq, ATT_BR) * H * B > 2 * sms;
+    const int block = single ? AttCfg<64, false, 1>::BC : AttCfg<64>::BC;
     CUtensorMap tq, tk, tv;
     int rc;
-    if ((rc = make_qkv_map(ctx, &tq, q, E, Lq, H, B))) return rc;
-    if ((rc = make_qkv_map(ctx, &tk, k, E, Lk, H, B))) return rc;
-    if ((rc = make_qkv_map(ctx, &tv, v, E, Lk, H, B))) return rc;
+    if ((rc = make_qkv_map(ctx, &tq, q, E, Lq, H, B, ATT_BR))) return rc;
+    if ((rc = make_qkv_map(ctx, &tk, k, E, Lk, H, B, block))) return rc;
+    if ((rc = make_qkv_map(ctx, &tv, v, E, Lk, H, B, block))) return rc;
     AttnParams p;
     p.E = (int)E; p.Lq = (int)Lq; p.Lk = (int)Lk; p.H = (int)H; p.B = (int)B;
     p.scale = scale;
@@ -1026,21 +1050,22 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     p.bias = bptr;
     p.bsK = bs[0]; p.bsQ = bs[1]; p.bsH = bs[2]; p.bsB = bs[3];
     p.bias_async = !bptr || !(bs[0] == 1 || Lk == 1) ? 0 : 1 + (reinterpret_cast<uintptr_t>(bptr) % 8 == 0 && bs[1] % 4 == 0 && bs[2] % 4 == 0 && bs[3] % 4 == 0);
-    const bool wide = E > 64;                              // two swizzle atoms along E
-    const int64_t item_rows = wide ? AttCfg<128>::NT * ATT_BR : AttCfg<64>::NT * ATT_BR;
-    const size_t smem_bytes = wide ? (bptr ? AttCfg<128, true>::SMEM_BYTES : AttCfg<128>::SMEM_BYTES)
-                                   : (bptr ? AttCfg<64, true>::SMEM_BYTES : AttCfg<64>::SMEM_BYTES);
+    const int64_t nblk_all = cdiv(Lk, block);
+    const int64_t item_rows = single ? ATT_BR : 2 * ATT_BR;
     auto launch = [&](dim3 grid) -> cudaError_t {
+        auto go = [&](auto kern, int threads, size_t smem) {
+            return launch_dep(kern, grid, dim3(threads, 1, 1), smem, ctx->stream, 1, tq, tk, tv, p);
+        };
+        if (single) return go(attention_f16_tc_kernel<64, false, 1>, AttCfg<64, false, 1>::THREADS, AttCfg<64, false, 1>::SMEM_BYTES);
         if (wide)
-            return bptr ? launch_dep(attention_f16_tc_kernel<128, true>, grid, dim3(ATT_THREADS, 1, 1), smem_bytes, ctx->stream, 1, tq, tk, tv, p)
-                        : launch_dep(attention_f16_tc_kernel<128, false>, grid, dim3(ATT_THREADS, 1, 1), smem_bytes, ctx->stream, 1, tq, tk, tv, p);
-        return bptr ? launch_dep(attention_f16_tc_kernel<64, true>, grid, dim3(ATT_THREADS, 1, 1), smem_bytes, ctx->stream, 1, tq, tk, tv, p)
-                    : launch_dep(attention_f16_tc_kernel<64, false>, grid, dim3(ATT_THREADS, 1, 1), smem_bytes, ctx->stream, 1, tq, tk, tv, p);
+            return bptr ? go(attention_f16_tc_kernel<128, true, 2>, AttCfg<128, true>::THREADS, AttCfg<128, true>::SMEM_BYTES)
+                        : go(attention_f16_tc_kernel<128, false, 2>, AttCfg<128>::THREADS, AttCfg<128>::SMEM_BYTES);
+        return bptr ? go(attention_f16_tc_kernel<64, true, 2>, AttCfg<64, true>::THREADS, AttCfg<64, true>::SMEM_BYTES)
+                    : go(attention_f16_tc_kernel<64, false, 2>, AttCfg<64>::THREADS, AttCfg<64>::SMEM_BYTES);
     };
     p.qpairs = (int)cdiv(Lq, item_rows);
     const int64_t pairs = (int64_t)p.qpairs * H * B;      // work items: pairs of query tiles, or single tiles when wide
     B200_REQUIRE(pairs < (1ll << 30), B200_DECLINE_EXTENT, "attention: too many query tiles");
-    const int64_t sms = ctx->prop.multiProcessorCount;
     // Two cases cut pairs along the keys (at least two key blocks per piece) and merge afterwards:
     // few queries over many keys (a decode step, Lq = 23, Lk = 4096: every pair is cut so that the
     // SMs are all used), and a last wave that would leave most SMs idle (its pairs are cut so that
@@ -1048,9 +1073,8 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     p.nsplit = 1;
     p.ntail = 0;
     p.part_o = p.part_ml = nullptr;
-    const int64_t nblk_all = cdiv(Lk, ATT_BC);
     const int64_t rem = pairs % sms;
-    if (nblk_all >= 4) {
+    if (!single && nblk_all >= 4) {
         int64_t ntail = 0, ns = 1;
         if (2 * pairs <= sms) {
             ntail = pairs;
@@ -1085,7 +1109,7 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     }
     // Split the pairs of a last wave that would leave more than half of the SMs idle — but not a
     // pair whose second tile does not exist.
-    int64_t nsplit = (pairs > sms && rem > 0 && 2 * rem <= sms && Lq % (2 * ATT_BR) == 0) ? rem : 0;
+    int64_t nsplit = (!single && pairs > sms && rem > 0 && 2 * rem <= sms && Lq % (2 * ATT_BR) == 0) ? rem : 0;
     p.pair_ctas = (int)(pairs - nsplit);
     B200_CUDA(launch(dim3((unsigned)(pairs + nsplit), 1, 1)));
     ctx->launches++;
