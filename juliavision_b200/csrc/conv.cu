@@ -118,11 +118,17 @@ static int conv2d_group(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_
     const bool onebyone = KW == 1 && KH == 1 && sx == 1 && sy == 1 && px == 0 && py == 0;
     int rc;
 
-    // Weight operand: (CRS, Cout) with CRS contiguous; pad its leading dimension to a
-    // multiple of 8 elements when it is not one already.
+    // Weight operand: (CRS, Cout) with CRS contiguous; copied with a leading dimension that is a multiple of 8
+    // elements when it does not already lie as a tensor map wants it.
+    auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
     const void* wB = w;
     int64_t ldw = CRS;
-    if (CRS % 8 != 0) {
+    // The implicit kernel where the GEMM cannot store the result, and where it has two pixel tiles per SM or more; a small
+    // image the GEMM can store is as fast through a small im2col matrix (64 x 58 x 24 -> 64: 7.5 us, implicit 12).
+    const bool aligned = P % 8 == 0 && out_img * osz % 16 == 0 && al16(out);   // the GEMM can store the result
+    const bool implicit = conv_implicit_takes(W, H, Cin, N, KW, KH, Cout, P) &&
+                          (onebyone ? !(aligned && x_img % 8 == 0 && al16(x)) : !aligned || cdiv(P, 128) * N >= 2 * ctx->prop.multiProcessorCount);
+    if (CRS % 8 != 0 || (implicit && !al16(w))) {
         ldw = (CRS + 7) / 8 * 8;
         void* wp = nullptr;
         if ((rc = ws_scratch(ctx, (size_t)(ldw * Cout) * 2, &wp))) return rc;
@@ -132,6 +138,9 @@ static int conv2d_group(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_
         B200_CUDA(cudaGetLastError());
         wB = wp;
     }
+    if (implicit)
+        return conv_implicit_launch(ctx, W, H, Cin, N, KW, KH, Cout, sx, sy, px, py, dx, dy, OW, P, x, x_img, wB, ldw, bias, out,
+                                    out_img, out_dtype, epilogue);
     if (onebyone) {
         for (int64_t n = 0; n < N; ++n) {
             const __half* xa = x + n * x_img; // (P, Cin) ld = P

@@ -1,0 +1,374 @@
+// Convolution as an implicit GEMM on the sm_100a tensor cores: the im2col matrix exists only as the shared-memory
+// tiles the UMMAs read.  out(OW,OH,Cout,N) = act(bias + w * x); x (W,H,Cin,N), w (KW,KH,Cin,Cout), the general form of
+// the reference's im2col + GEMM route (kernels/extern/conv_coopmat.jl:246-392).
+//
+// What bounds it: the gather, element by element, because a tap moves the image by one element and a TMA copy or a
+// vector load by multiples of eight; and, with few input channels, the output's way to HBM.  Against the materialised
+// matrix it saves that matrix's write and read and a launch; and because the pixels sit on the tensor-memory lanes,
+// the store of one channel is 32 consecutive elements per warp whatever the alignment, so an image of any size runs
+// on the tensor cores.
+//
+// One CTA takes 128 pixels of one image and up to 256 output channels, two CTAs per SM so that one's gather runs under
+// the other's waits and store:
+//   warps 0-7  gather: D's A operand, 64 rows (cin, kh, kw) x 128 pixels per k-block, pixels contiguous (MN-major),
+//              written with the 128-byte swizzle.  A warp takes eight rows, whose tap is then uniform, and a lane two
+//              pairs of neighbouring pixels of each, so that a load instruction touches one or two lines and a store
+//              every bank once; four rows are loaded while the four before them are stored.
+//              Afterwards the epilogue, TMEM -> +bias, round, act -> global
+//   warp 8     TMA producer of the weight tile (K-major, straight from w)
+//   warp 9     UMMA issuer
+// Measured (us, B200) against the im2col + GEMM route: 1024 x 1024 x 3 -> 112, 7 x 7 / 4: 35 -> 23.6; 300 x 296 x 16 -> 64,
+// 3 x 3: 42.5 -> 24.6; against the scalar GEMM odd pixel counts had: 43 x 42 x 256 -> 256, 3 x 3 / 2: 229 -> 14.2, two of
+// 230 x 225 x 32 -> 80, 3 x 3: 890 -> 43.  What is left is the gather's load latency.
+// A small image (fewer CTAs than the GPU holds) splits the reduction over the CTAs of a cluster, whose fp32 tiles
+// meet in distributed shared memory, added in rank order.
+#include <cuda_fp16.h>
+
+#include "act.cuh"
+#include "internal.h"
+#include "ptx.cuh"
+
+namespace b200 {
+
+constexpr int CI_PIX = 128;              // pixels per CTA (TMEM lanes)
+constexpr int CI_BK = 64;                // one 128-byte swizzle row of the weight tile
+constexpr int CI_GATHER = 256;           // gather / epilogue threads
+constexpr int CI_THREADS = CI_GATHER + 64;
+constexpr int CI_A_BYTES = CI_PIX * CI_BK * 2;
+
+template <int BN> struct CiCfg {
+    static constexpr int STAGES = BN == 256 ? 2 : (BN == 128 ? 3 : 4);
+    static constexpr int B_BYTES = BN * CI_BK * 2;
+    static constexpr int STAGE_BYTES = CI_A_BYTES + B_BYTES;
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BN * 4 + 128;
+    static constexpr bool SPLITS = BN * CI_PIX * 4 <= STAGES * STAGE_BYTES;   // the fp32 tile fits over the drained ring
+    static_assert(2 * (SMEM_BYTES + 1024) <= 233472, "two CTAs per SM");
+};
+
+struct ConvParams {
+    const __half* x;
+    const __half* bias;
+    void* out;
+    int64_t x_img, out_img;   // elements from one image to the next
+    int W, H, CRS, Cout, OW, P, tiles;   // tiles of CI_PIX pixels per image
+    int sx, sy, px, py, dx, dy;
+    int KW, KH;
+    uint32_t mKW, mKH;        // ceil(2^32 / KW), ceil(2^32 / KH): exact quotients below 2^16
+    int epi;
+    int* d_status;
+};
+
+__device__ __forceinline__ uint32_t div_magic(uint32_t v, uint32_t d, uint32_t magic) {
+    return d == 1 ? v : __umulhi(v, magic);
+}
+
+// The element at p, or zero: a predicated load, no branch.
+__device__ __forceinline__ uint32_t ldg_u16_if(const uint16_t* p, bool in) {
+    uint32_t v;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred P;\n\t"
+        ".reg .b16 h;\n\t"
+        "setp.ne.u32 P, %2, 0;\n\t"
+        "mov.b16 h, 0;\n\t"
+        "@P ld.global.nc.b16 h, [%1];\n\t"
+        "cvt.u32.u16 %0, h;\n\t"
+        "}\n"
+        : "=r"(v)
+        : "l"(p), "r"((uint32_t)in));
+    return v;
+}
+__device__ __forceinline__ float ci_ld_cluster(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+// grid (K parts, pixel tiles of all images, channel tiles); the K parts of a tile form a cluster.
+template <int BN, typename OutT>
+__global__ void __launch_bounds__(CI_THREADS, 2)
+conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Cout}, boxes of 64 x BN
+                     const ConvParams p) {
+    using Cfg = CiCfg<BN>;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    if ((smem_u32(smem) & 1023u) != 0) {
+        if (threadIdx.x == 0) atomicCAS(p.d_status, 0, KST_SMEM_LAYOUT);
+        return;
+    }
+    float* sbias = reinterpret_cast<float*>(smem + Cfg::STAGES * Cfg::STAGE_BYTES);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sbias + BN);
+    uint64_t* full = bars;
+    uint64_t* empty = bars + Cfg::STAGES;
+    uint64_t* tfull = bars + 2 * Cfg::STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int img = blockIdx.y / p.tiles, m0 = (blockIdx.y - img * p.tiles) * CI_PIX, c0 = blockIdx.z * BN;
+    const int parts = gridDim.x, rank = blockIdx.x;
+    const int nkb_all = (p.CRS + CI_BK - 1) / CI_BK;
+    const int kb0 = rank * nkb_all / parts, nkb = (rank + 1) * nkb_all / parts - kb0;
+
+    if (tid == 0) {
+        for (int s = 0; s < Cfg::STAGES; ++s) {
+            mbar_init(&full[s], CI_GATHER / 32 + 1);   // the gather warps and the weight tile's bytes
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(tfull, 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+        prefetch_tmap(&tmapW);
+    }
+    if (warp == 8) {
+        tmem_alloc(tmem_slot, BN);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    grid_dep_wait();
+    grid_dep_launch();
+
+    // Channel c of the tile at pixel pix, rounded before the activation sees it.  The activation is a template
+    // argument: a switch in the unrolled store cost more than the gather.
+    OutT* const out0 = static_cast<OutT*>(p.out) + (int64_t)img * p.out_img + (int64_t)c0 * p.P;
+    auto store = [&](OutT* dst, float o, auto act) {
+        if constexpr (sizeof(OutT) == 2) *dst = __float2half_rn(act(__half2float(__float2half_rn(o))));
+        else *dst = act(o);
+    };
+    auto by_act = [&](auto body) {
+        switch (p.epi) {
+            case B200_EPI_NONE: body([](float v) { return v; }); break;
+            case B200_EPI_RELU: body([](float v) { return fmaxf(v, 0.f); }); break;
+            case B200_EPI_GELU: body([](float v) { return gelu_exact(v); }); break;
+            default: body([](float v) { return apply_act(B200_EPI_GELU_TANH, v); }); break;
+        }
+    };
+    if (warp == 8) {
+        if (lane == 0) {
+            for (int kb = 0; kb < nkb; ++kb) {
+                const int s = kb % Cfg::STAGES;
+                if (!mbar_wait(&empty[s], (uint32_t)((kb / Cfg::STAGES) & 1) ^ 1, p.d_status, KST_WAIT_EMPTY, abort_flag)) break;
+                mbar_arrive_expect_tx(&full[s], Cfg::B_BYTES);
+                tma_load_2d(smem + s * Cfg::STAGE_BYTES + CI_A_BYTES, &tmapW, &full[s], (kb0 + kb) * CI_BK, c0);
+            }
+        }
+    } else if (warp == 9) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = make_idesc_f16(CI_PIX, BN, /*a MN-major*/ 1, /*b K-major*/ 0);
+            constexpr uint64_t adesc0 = make_smem_desc(64 * CI_BK * 2, 1024);
+            constexpr uint64_t bdesc0 = make_smem_desc(16, 1024);
+            bool ok = true;
+            for (int kb = 0; kb < nkb; ++kb) {
+                const int s = kb % Cfg::STAGES;
+                if (!mbar_wait(&full[s], (uint32_t)((kb / Cfg::STAGES) & 1), p.d_status, KST_WAIT_FULL, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t a = smem_u32(smem + s * Cfg::STAGE_BYTES), b = a + CI_A_BYTES;
+#pragma unroll
+                for (int k = 0; k < CI_BK / 16; ++k)   // 16 k: two 8-row groups of A, 32 bytes inside B's swizzle row
+                    umma_ss(tmem_base, smem_desc_at(adesc0, a + k * 2048), smem_desc_at(bdesc0, b + k * 32), idesc, (kb | k) != 0);
+                umma_commit(&empty[s]);
+            }
+            if (ok) umma_commit(tfull);
+        }
+    } else {
+        for (int j = tid; j < BN; j += CI_GATHER)   // read in the epilogue, a barrier among these warps later
+            sbias[j] = p.bias != nullptr && c0 + j < p.Cout ? __half2float(p.bias[c0 + j]) : 0.f;
+        // Pixels 2 lane, 2 lane + 1 of either half of the tile.
+        int bx[4], by[4], base[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int m = m0 + 64 * (q >> 1) + 2 * lane + (q & 1);
+            const int oh = m / p.OW, ow = m - oh * p.OW;
+            bx[q] = ow * p.sx - p.px;
+            by[q] = m < p.P ? oh * p.sy - p.py : -(1 << 30);   // never inside the image
+            base[q] = by[q] * p.W + bx[q];
+        }
+        const uint16_t* xi = reinterpret_cast<const uint16_t*>(p.x) + (int64_t)img * p.x_img;
+        const int row_off = warp * 128 + (((lane >> 2) ^ warp) << 4) + (lane & 3) * 4;   // row warp + 8 r: r * 1024 further
+        // The taps of the warp's eight rows of a k-block, row r by lane r: offset in the image and (x, y) shift.  A row
+        // past the reduction gets a shift that is never inside.
+        int koff, kx, ky;
+        auto taps = [&](int kb) {
+            const uint32_t k = (uint32_t)((kb0 + kb) * CI_BK + warp + 8 * (lane & 7));
+            const uint32_t t = div_magic(k, p.KW, p.mKW), cin = div_magic(t, p.KH, p.mKH);
+            kx = k < (uint32_t)p.CRS ? (int)(k - t * p.KW) * p.dx : -(1 << 30);
+            ky = (int)(t - cin * p.KH) * p.dy;
+            koff = ((int)cin * p.H + ky) * p.W + kx;
+        };
+        auto load = [&](uint32_t (&v)[4][4], int half) {   // rows 4 half ... of the k-block whose taps are held
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int o = __shfl_sync(0xffffffffu, koff, 4 * half + i), x = __shfl_sync(0xffffffffu, kx, 4 * half + i),
+                          y = __shfl_sync(0xffffffffu, ky, 4 * half + i);
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    v[i][q] = ldg_u16_if(xi + (base[q] + o), (uint32_t)(bx[q] + x) < (uint32_t)p.W && (uint32_t)(by[q] + y) < (uint32_t)p.H);
+            }
+        };
+        auto put = [&](const uint32_t (&v)[4][4], int step) {
+            uint8_t* a = smem + ((step >> 1) % Cfg::STAGES) * Cfg::STAGE_BYTES + (step & 1) * 4096 + row_off;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    *reinterpret_cast<uint32_t*>(a + h * (64 * CI_BK * 2) + i * 1024) = v[i][2 * h] | (v[i][2 * h + 1] << 16);
+        };
+        bool ok = true;
+        uint32_t va[4][4], vb[4][4];
+        taps(0);
+        load(va, 0);
+        for (int kb = 0; kb < nkb; ++kb) {
+            const int s = kb % Cfg::STAGES;
+            load(vb, 1);
+            if (ok && !mbar_wait(&empty[s], (uint32_t)((kb / Cfg::STAGES) & 1) ^ 1, p.d_status, KST_WAIT_EMPTY, abort_flag)) ok = false;
+            if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+            put(va, 2 * kb);
+            if (kb + 1 < nkb) {
+                taps(kb + 1);
+                load(va, 0);
+            }
+            put(vb, 2 * kb + 1);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[s]);
+        }
+        // ------------------------------------------------------------------ epilogue
+        named_bar_sync(1, CI_GATHER);   // sbias
+        if (ok && !mbar_wait(tfull, 0, p.d_status, KST_WAIT_TMEM_FULL, abort_flag)) ok = false;
+        if (!__any_sync(0xffffffffu, !ok)) {
+            tc_fence_after();
+            const int quad = warp & 3, part = warp >> 2;   // tensor-memory lane quadrant, half of the channels
+            const int pix = m0 + quad * 32 + lane;
+            const uint32_t tacc = tmem_base + (uint32_t(quad * 32) << 16);
+            const int cend = min((part + 1) * (BN / 2), p.Cout - c0);
+            if (Cfg::SPLITS && parts > 1) {
+                float* acc = reinterpret_cast<float*>(smem) + quad * 32 + lane;   // [channel][pixel], over the drained ring
+#pragma unroll 1
+                for (int c = part * (BN / 2); c < cend; c += 16) {
+                    uint32_t r[16];
+                    tmem_ld16(tacc + c, r);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int t = 0; t < 16; ++t) acc[(c + t) * CI_PIX] = __uint_as_float(r[t]);
+                }
+            } else {
+                by_act([&](auto act) {
+#pragma unroll 1
+                    for (int c = part * (BN / 2); c < cend; c += 16) {
+                        uint32_t r[16];
+                        tmem_ld16(tacc + c, r);
+                        tmem_wait_ld();
+                        OutT* dst = out0 + (int64_t)c * p.P + pix;
+                        if (pix < p.P) {
+                            if (c + 16 <= cend) {
+#pragma unroll
+                                for (int t = 0; t < 16; ++t, dst += p.P) store(dst, __uint_as_float(r[t]) + sbias[c + t], act);
+                            } else {
+#pragma unroll
+                                for (int t = 0; t < 16; ++t, dst += p.P)
+                                    if (c + t < cend) store(dst, __uint_as_float(r[t]) + sbias[c + t], act);
+                            }
+                        }
+                        __syncwarp();
+                    }
+                });
+            }
+        }
+    }
+    if (Cfg::SPLITS && parts > 1) {
+        __syncwarp();
+        cluster_sync_all();   // every part's tile is in its shared memory
+        if (warp < 8) {
+            const uint32_t mine = smem_u32(smem) + (tid & 127) * 4;
+            const int pix = m0 + (tid & 127);
+            // four channels' loads from every part in flight together: a remote load takes a few hundred nanoseconds
+            for (int c = rank * (BN / parts) + (tid >> 7); c < (rank + 1) * (BN / parts); c += 8) {
+                float v[4][8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const uint32_t src = mapa_u32(mine + c * (CI_PIX * 4), q < parts ? q : 0);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) v[u][q] = q < parts ? ci_ld_cluster(src + u * (2 * CI_PIX * 4)) : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    float o = 0.f;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) o += v[u][q];
+                    if (pix < p.P && c0 + c + 2 * u < p.Cout)
+                        by_act([&](auto act) { store(out0 + (int64_t)(c + 2 * u) * p.P + pix, o + sbias[c + 2 * u], act); });
+                }
+            }
+        }
+        __syncwarp();
+        cluster_sync_all();   // nobody leaves while its tile may still be read
+    }
+    if (*abort_flag) {   // let any TMA copy still in flight into this CTA's shared memory land before exit
+        for (int i = 0; i < 4; ++i) __nanosleep(1000000);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 8) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, BN);
+    }
+}
+
+template <int BN, typename OutT>
+static int ci_launch(b200_ctx* ctx, const CUtensorMap& tw, const ConvParams& p, int64_t N, int parts) {
+    using Cfg = CiCfg<BN>;
+    static bool attr_done[16] = {};
+    auto kern = conv_implicit_kernel<BN, OutT>;
+    if (!attr_done[ctx->device & 15]) {
+        B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+        attr_done[ctx->device & 15] = true;
+    }
+    dim3 grid((unsigned)parts, (unsigned)(p.tiles * N), (unsigned)cdiv(p.Cout, BN));
+    B200_CUDA(launch_dep(kern, grid, dim3(CI_THREADS, 1, 1), Cfg::SMEM_BYTES, ctx->stream, parts, tw, p));
+    ctx->launches++;
+    return B200_OK;
+}
+
+bool conv_implicit_takes(int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t KW, int64_t KH, int64_t Cout, int64_t P) {
+    return cdiv(P, CI_PIX) * N < 65536 && P < (1ll << 30) && W * H * Cin < (1ll << 31) && KW * KH * Cin < 65536 && KW < 65536 && KH < 65536 &&
+           Cout < (1 << 20) && W < (1 << 28) && H < (1 << 28);
+}
+
+int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t KW, int64_t KH, int64_t Cout,
+                         int64_t sx, int64_t sy, int64_t px, int64_t py, int64_t dx, int64_t dy, int64_t OW, int64_t P,
+                         const void* x, int64_t x_img, const void* w, int64_t ldw, const void* bias, void* out,
+                         int64_t out_img, int out_dtype, int epilogue) {
+    ConvParams p;
+    p.x = static_cast<const __half*>(x);
+    p.bias = static_cast<const __half*>(bias);
+    p.out = out;
+    p.x_img = x_img; p.out_img = out_img;
+    p.W = (int)W; p.H = (int)H; p.CRS = (int)(KW * KH * Cin); p.Cout = (int)Cout; p.OW = (int)OW; p.P = (int)P;
+    p.sx = (int)sx; p.sy = (int)sy; p.px = (int)px; p.py = (int)py; p.dx = (int)dx; p.dy = (int)dy;
+    p.KW = (int)KW; p.KH = (int)KH;
+    p.mKW = KW > 1 ? (uint32_t)(((1ull << 32) + KW - 1) / KW) : 0;
+    p.mKH = KH > 1 ? (uint32_t)(((1ull << 32) + KH - 1) / KH) : 0;
+    p.epi = epilogue;
+    p.d_status = ctx->d_status;
+    p.tiles = (int)cdiv(P, CI_PIX);
+    // Channels per CTA: all of them up to 256, since every channel tile gathers the pixels again; but a launch that
+    // leaves half of the GPU's CTAs unused splits the reduction, two k-blocks a part at least, which the 256-wide
+    // tile has no shared memory for.
+    const int64_t tiles = p.tiles * N, room = 2 * (int64_t)ctx->prop.multiProcessorCount, nkb = cdiv(p.CRS, CI_BK);
+    int bn = Cout <= 64 ? 64 : (Cout <= 128 || (2 * tiles * cdiv(Cout, 128) <= room && nkb >= 4) ? 128 : 256), parts = 1;
+    if (bn < 256)
+        while (parts < 8 && 2 * parts * tiles * cdiv(Cout, bn) <= room && nkb >= 4 * parts) parts *= 2;
+    CUtensorMap tw;
+    uint64_t dims[2] = {(uint64_t)p.CRS, (uint64_t)Cout};
+    uint64_t str[1] = {(uint64_t)ldw * 2};
+    uint32_t box[2] = {CI_BK, (uint32_t)bn};
+    int rc = make_tmap(ctx, &tw, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, w, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
+    const bool h = out_dtype == B200_F16;
+    if (bn == 256) return h ? ci_launch<256, __half>(ctx, tw, p, N, 1) : ci_launch<256, float>(ctx, tw, p, N, 1);
+    if (bn == 128) return h ? ci_launch<128, __half>(ctx, tw, p, N, parts) : ci_launch<128, float>(ctx, tw, p, N, parts);
+    return h ? ci_launch<64, __half>(ctx, tw, p, N, parts) : ci_launch<64, float>(ctx, tw, p, N, parts);
+}
+
+} // namespace b200

@@ -123,6 +123,14 @@ int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, 
                  int epilogue, int64_t nbatch, int64_t strideA, int64_t strideB, int64_t strideO,
                  int use_workspace = 1);
 
+// Convolution without a materialised im2col matrix (conv_implicit.cu).  w: (CRS, Cout), 16-byte aligned, leading
+// dimension ldw a multiple of 8; x and out at any alignment.
+bool conv_implicit_takes(int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t KW, int64_t KH, int64_t Cout, int64_t P);
+int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t KW, int64_t KH, int64_t Cout,
+                         int64_t sx, int64_t sy, int64_t px, int64_t py, int64_t dx, int64_t dy, int64_t OW, int64_t P,
+                         const void* x, int64_t x_img, const void* w, int64_t ldw, const void* bias, void* out,
+                         int64_t out_img, int out_dtype, int epilogue);
+
 // GEMM over operands a tensor map cannot express, from a few tens of thousands of elements of A up (gemm_rows.cu).
 bool gemm_rows_takes(int64_t M, int64_t N, int64_t K, int64_t nbatch);
 int gemm_rows_launch(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda, const void* B, int64_t ldb,

@@ -63,6 +63,36 @@ def test_conv_1x1_is_a_gemm(ctx, ora, W, H, Cin, Cout):
     assert relerr(got, ref) < 5e-3, describe(got, ref, 5e-3)
 
 
+# (N, Cin, H, W, Cout, KH, KW, stride, padding, dilation), torch order: pixel counts off 8 and 128, rows shorter than a
+# chunk of 8 pixels, channel counts on both sides of a tile, every stride form, dilation, wide padding, a 1x1 of odd size
+IMPLICIT = [(1, 3, 33, 41, 40, 7, 7, (4, 4), (3, 3), (1, 1)), (2, 8, 5, 6, 33, 3, 3, (1, 1), (1, 1), (1, 1)),
+            (1, 16, 31, 29, 130, 3, 3, (2, 2), (1, 1), (1, 1)), (1, 24, 17, 19, 257, 1, 1, (1, 1), (0, 0), (1, 1)),
+            (1, 5, 40, 37, 64, 3, 5, (3, 1), (2, 4), (2, 2)), (3, 8, 64, 128, 64, 3, 3, (1, 1), (1, 1), (1, 1)),
+            (1, 200, 13, 150, 300, 3, 3, (1, 3), (1, 1), (1, 1)), (1, 1, 9, 200, 16, 2, 2, (1, 1), (5, 9), (1, 1))]
+
+
+@pytest.mark.parametrize("N,Cin,H,W,Cout,KH,KW,stride,padding,dilation", IMPLICIT)
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+def test_conv_gathered_into_the_tiles(ctx, ora, N, Cin, H, W, Cout, KH, KW, stride, padding, dilation, dt):
+    rng = np.random.default_rng(Cin + Cout + W)
+    x = np.float16(rng.standard_normal((N, Cin, H, W)) * 0.5)
+    w = np.float16(rng.standard_normal((Cout, Cin, KH, KW)) * 0.2)
+    b = np.float16(rng.standard_normal(Cout) * 0.2)
+    ref = ora.conv2d(x, w, b, stride, padding, dilation, epi="relu", out_dtype=dt)
+    flat = ctx.allocate(dt, ref.size + 1)      # the output one element off its allocation's alignment
+    ctx.fill_bytes(flat, 0xFF)
+    out = jv.DeviceArray(ctx, flat.ptr + np.dtype(dt).itemsize, dt, tuple(reversed(ref.shape)), owner=flat)
+    ctx.ws.reset()
+    jv.convolution_(ctx, out, ctx.toback(x), ctx.toback(w), ctx.toback(b), stride[::-1], padding[::-1], dilation[::-1], act="relu")
+    ctx.synchronize()
+    host = flat.to_host()
+    assert np.isnan(host[0]), "wrote before the output"
+    got = host[1:].reshape(ref.shape)
+    # fp32 sums in another order (sqrt(CRS) eps32), then one fp16 rounding step
+    tol = 2e-3 if dt == np.float16 else 2e-5
+    assert relerr(got, ref) < tol, describe(got, ref, tol)
+
+
 def test_im2col_bit_exact(ctx, ora):
     import ctypes as C
     from juliavision_b200 import _lib
