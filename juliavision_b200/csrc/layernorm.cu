@@ -75,10 +75,12 @@ __device__ __forceinline__ float group_sum(float v) {
     return v;
 }
 
-// What every form of the warp kernel does with a row's elements once they are in registers, as packed fp32 pairs (one
-// instruction for two: at 65536 x 1280 the scalar form issued for about 25 us of the launch's 62, half of them in
-// these steps; 62.2 -> 58.1 us, 5.4 -> 5.8 TB/s).  The vectors of a lane are v = first, first + stride, ...; `x` is left holding x - mean after ln_moments.
-// One definition, so that the layer norm alone and the one behind a residual add give the same bits.
+// The packed form (PACK): a row's moments and its output two elements per instruction, gamma and beta in one rounding.
+// It is for launches whose rows come from and go to HBM (more than the L2 holds): 65536 x 1280 in fp16 62.2 -> 58.1 us
+// (5.4 -> 5.8 TB/s), where the scalar form issues for about 25 us of the launch.  Rows that stay in the L2 are faster
+// in the scalar form (14736 x 1176: 11.7 us, packed 12.9), so the row bytes decide, the same for the layer norm alone
+// and the one behind a residual add, which therefore give the same bits.  The vectors of a lane are v = first,
+// first + 32, ...; `x` is left holding x - mean.
 __device__ __forceinline__ float pairs_sum(unsigned long long s2) {
     float a, b;
     act_detail::upk(s2, a, b);
@@ -140,7 +142,7 @@ __device__ __forceinline__ void ln_write(OutT* dst, const unsigned long long* d,
 // LAT: the latency form, for launches small enough that every CTA is resident at once and what the kernel takes
 // is a chain of round trips, not bytes (the encoder's 1500 rows): everything the row needs is asked for up front.
 // It costs ~40 registers; launches of many waves, which want occupancy, take the lean form.
-template <typename InT, typename OutT, int VPL, int LPG = 32, bool LAT = false>
+template <typename InT, typename OutT, int VPL, int LPG = 32, bool LAT = false, bool PACK = false>
 __global__ void __launch_bounds__(128)
 ln_warp_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restrict__ mean,
                float* __restrict__ rstd, const InT* __restrict__ gamma,
@@ -168,35 +170,95 @@ ln_warp_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
         }
     }
 
-    unsigned long long x[VPL][VN / 2];
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-        const int v = lane + 32 * i;
-        if (v < nvec) {
-            Vec16<InT> t;
-            float f[VN];
-            t.raw = __ldg(reinterpret_cast<const uint4*>(src) + v);
-            t.to_f32(f);
-#pragma unroll
-            for (int j = 0; j < VN / 2; ++j) x[i][j] = act_detail::pk(f[2 * j], f[2 * j + 1]);
-        }
-    }
     float mu, r;
-    ln_moments<VPL, VN, LPG>(x, lane, nvec, C, eps, mu, r);
-    OutT* dst = out + g * (int64_t)C;
+    if constexpr (PACK) {
+        unsigned long long x[VPL][VN / 2];
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-        const int v = lane + 32 * i;
-        if (v < nvec) {
-            uint4 gv = make_uint4(0u, 0u, 0u, 0u), bv = gv;
-            if constexpr (HOIST) {
-                gv = gw[i];
-                bv = bw[i];
-            } else {
-                if (gamma) gv = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
-                if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + v);
+        for (int i = 0; i < VPL; ++i) {
+            const int v = lane + 32 * i;
+            if (v < nvec) {
+                Vec16<InT> t;
+                float f[VN];
+                t.raw = __ldg(reinterpret_cast<const uint4*>(src) + v);
+                t.to_f32(f);
+#pragma unroll
+                for (int j = 0; j < VN / 2; ++j) x[i][j] = act_detail::pk(f[2 * j], f[2 * j + 1]);
             }
-            ln_write<InT, OutT>(dst + (int64_t)v * VN, x[i], r, gamma != nullptr, gv, beta != nullptr, bv);
+        }
+        ln_moments<VPL, VN, LPG>(x, lane, nvec, C, eps, mu, r);
+        OutT* dst = out + g * (int64_t)C;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+            const int v = lane + 32 * i;
+            if (v < nvec) {
+                uint4 gv = make_uint4(0u, 0u, 0u, 0u), bv = gv;
+                if constexpr (HOIST) {
+                    gv = gw[i];
+                    bv = bw[i];
+                } else {
+                    if (gamma) gv = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
+                    if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + v);
+                }
+                ln_write<InT, OutT>(dst + (int64_t)v * VN, x[i], r, gamma != nullptr, gv, beta != nullptr, bv);
+            }
+        }
+    } else {
+        float x[VPL][VN];
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+            int v = lane + 32 * i;
+            if (v < nvec) {
+                Vec16<InT> t;
+                t.raw = __ldg(reinterpret_cast<const uint4*>(src) + v);
+                t.to_f32(x[i]);
+#pragma unroll
+                for (int j = 0; j < VN; ++j) s += x[i][j];
+            }
+        }
+        const float n = (float)C;
+        mu = group_sum<LPG>(s) / n;
+        float s2 = 0.f;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+            if (lane + 32 * i < nvec) {
+#pragma unroll
+                for (int j = 0; j < VN; ++j) {
+                    float d = x[i][j] - mu;
+                    s2 += d * d;
+                }
+            }
+        }
+        r = 1.0f / sqrtf(group_sum<LPG>(s2) / n + eps);
+
+        OutT* dst = out + g * (int64_t)C;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+            int v = lane + 32 * i;
+            if (v < nvec) {
+                float y[VN];
+#pragma unroll
+                for (int j = 0; j < VN; ++j) y[j] = (x[i][j] - mu) * r;
+                if (gamma) {
+                    Vec16<InT> t;
+                    float gf[VN];
+                    if constexpr (HOIST) t.raw = gw[i];
+                    else t.raw = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
+                    t.to_f32(gf);
+#pragma unroll
+                    for (int j = 0; j < VN; ++j) y[j] *= gf[j];
+                }
+                if (beta) {
+                    Vec16<InT> t;
+                    float bf[VN];
+                    if constexpr (HOIST) t.raw = bw[i];
+                    else t.raw = __ldg(reinterpret_cast<const uint4*>(beta) + v);
+                    t.to_f32(bf);
+#pragma unroll
+                    for (int j = 0; j < VN; ++j) y[j] += bf[j];
+                }
+                store_vec<VN>(dst + (int64_t)v * VN, y);
+            }
         }
     }
     if (lane == 0 && g < groups) {
@@ -210,7 +272,7 @@ ln_warp_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
 // Bit-identical to running add.Tensor, clamp.default and native_layer_norm one after another
 // (each rounds to fp16 where the separate ops would), but x and h are read once and the three
 // launches become one.
-template <int VPL, int LPG = 32, bool LAT = false>
+template <int VPL, int LPG = 32, bool LAT = false, bool PACK = false>
 __global__ void __launch_bounds__(128)
 ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half* __restrict__ out,
                    float* __restrict__ mean, float* __restrict__ rstd, const __half* __restrict__ gamma,
@@ -239,7 +301,6 @@ ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half*
     __half* xr = x + g * (int64_t)C;
     const __half* hr = h + g * (int64_t)C;
 
-    unsigned long long v[VPL][VN / 2];
     // every load of the row first, then the arithmetic: one round trip for the row whatever the compiler would
     // have made of loads and stores through the same pointer
     // (the latency form; the lean one reads each vector where it uses it)
@@ -254,48 +315,121 @@ ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half*
             }
         }
     }
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-        const int vi = lane + 32 * i;
-        if (vi < nvec) {
-            Vec16<__half> a, b;
-            if constexpr (HOIST) {
-                a.raw = xraw[i];
-                b.raw = hraw[i];
-            } else {
-                a.raw = *(reinterpret_cast<const uint4*>(xr) + vi);
-                b.raw = __ldg(reinterpret_cast<const uint4*>(hr) + vi);
-            }
-            float fa[VN], fb[VN];
-            a.to_f32(fa);
-            b.to_f32(fb);
-#pragma unroll
-            for (int j = 0; j < VN; ++j) {
-                float t = __half2float(__float2half_rn(fa[j] + fb[j]));        // add.Tensor rounds here
-                if (use_clamp) t = __half2float(__float2half_rn(fminf(fmaxf(t, lo), hi)));
-                fa[j] = t;
-            }
-            store_vec<VN>(xr + (int64_t)vi * VN, fa);                           // exact: already fp16 values
-#pragma unroll
-            for (int j = 0; j < VN / 2; ++j) v[i][j] = act_detail::pk(fa[2 * j], fa[2 * j + 1]);
-        }
-    }
     float mu, r;
-    ln_moments<VPL, VN, LPG>(v, lane, nvec, C, eps, mu, r);
-    __half* dst = out + g * (int64_t)C;
+    if constexpr (PACK) {
+        unsigned long long v[VPL][VN / 2];
 #pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-        const int vi = lane + 32 * i;
-        if (vi < nvec) {
-            uint4 gv = make_uint4(0u, 0u, 0u, 0u), bv = gv;
-            if constexpr (HOIST) {
-                gv = gw[i];
-                bv = bw[i];
-            } else {
-                if (gamma) gv = __ldg(reinterpret_cast<const uint4*>(gamma) + vi);
-                if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + vi);
+        for (int i = 0; i < VPL; ++i) {
+            const int vi = lane + 32 * i;
+            if (vi < nvec) {
+                Vec16<__half> a, b;
+                if constexpr (HOIST) {
+                    a.raw = xraw[i];
+                    b.raw = hraw[i];
+                } else {
+                    a.raw = *(reinterpret_cast<const uint4*>(xr) + vi);
+                    b.raw = __ldg(reinterpret_cast<const uint4*>(hr) + vi);
+                }
+                float fa[VN], fb[VN];
+                a.to_f32(fa);
+                b.to_f32(fb);
+#pragma unroll
+                for (int j = 0; j < VN; ++j) {
+                    float t = __half2float(__float2half_rn(fa[j] + fb[j]));        // add.Tensor rounds here
+                    if (use_clamp) t = __half2float(__float2half_rn(fminf(fmaxf(t, lo), hi)));
+                    fa[j] = t;
+                }
+                store_vec<VN>(xr + (int64_t)vi * VN, fa);                           // exact: already fp16 values
+#pragma unroll
+                for (int j = 0; j < VN / 2; ++j) v[i][j] = act_detail::pk(fa[2 * j], fa[2 * j + 1]);
             }
-            ln_write<__half, __half>(dst + (int64_t)vi * VN, v[i], r, gamma != nullptr, gv, beta != nullptr, bv);
+        }
+        ln_moments<VPL, VN, LPG>(v, lane, nvec, C, eps, mu, r);
+        __half* dst = out + g * (int64_t)C;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+            const int vi = lane + 32 * i;
+            if (vi < nvec) {
+                uint4 gv = make_uint4(0u, 0u, 0u, 0u), bv = gv;
+                if constexpr (HOIST) {
+                    gv = gw[i];
+                    bv = bw[i];
+                } else {
+                    if (gamma) gv = __ldg(reinterpret_cast<const uint4*>(gamma) + vi);
+                    if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + vi);
+                }
+                ln_write<__half, __half>(dst + (int64_t)vi * VN, v[i], r, gamma != nullptr, gv, beta != nullptr, bv);
+            }
+        }
+    } else {
+        float v[VPL][VN];
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+            const int vi = lane + 32 * i;
+            if (vi < nvec) {
+                Vec16<__half> a, b;
+                if constexpr (HOIST) {
+                    a.raw = xraw[i];
+                    b.raw = hraw[i];
+                } else {
+                    a.raw = *(reinterpret_cast<const uint4*>(xr) + vi);
+                    b.raw = __ldg(reinterpret_cast<const uint4*>(hr) + vi);
+                }
+                float fa[VN], fb[VN];
+                a.to_f32(fa);
+                b.to_f32(fb);
+#pragma unroll
+                for (int j = 0; j < VN; ++j) {
+                    float t = __half2float(__float2half_rn(fa[j] + fb[j]));        // add.Tensor rounds here
+                    if (use_clamp) t = __half2float(__float2half_rn(fminf(fmaxf(t, lo), hi)));
+                    v[i][j] = t;
+                    s += t;
+                }
+                store_vec<VN>(xr + (int64_t)vi * VN, v[i]);                         // exact: already fp16 values
+            }
+        }
+        const float n = (float)C;
+        mu = group_sum<LPG>(s) / n;
+        float s2 = 0.f;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i)
+            if (lane + 32 * i < nvec) {
+#pragma unroll
+                for (int j = 0; j < VN; ++j) {
+                    float d = v[i][j] - mu;
+                    s2 += d * d;
+                }
+            }
+        r = 1.0f / sqrtf(group_sum<LPG>(s2) / n + eps);
+        __half* dst = out + g * (int64_t)C;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+            const int vi = lane + 32 * i;
+            if (vi < nvec) {
+                float y[VN];
+#pragma unroll
+                for (int j = 0; j < VN; ++j) y[j] = (v[i][j] - mu) * r;
+                if (gamma) {
+                    Vec16<__half> t;
+                    float gf[VN];
+                    if constexpr (HOIST) t.raw = gw[i];
+                    else t.raw = __ldg(reinterpret_cast<const uint4*>(gamma) + vi);
+                    t.to_f32(gf);
+#pragma unroll
+                    for (int j = 0; j < VN; ++j) y[j] *= gf[j];
+                }
+                if (beta) {
+                    Vec16<__half> t;
+                    float bf[VN];
+                    if constexpr (HOIST) t.raw = bw[i];
+                    else t.raw = __ldg(reinterpret_cast<const uint4*>(beta) + vi);
+                    t.to_f32(bf);
+#pragma unroll
+                    for (int j = 0; j < VN; ++j) y[j] += bf[j];
+                }
+                store_vec<VN>(dst + (int64_t)vi * VN, y);
+            }
         }
     }
     if (lane == 0 && g < groups) {
@@ -425,6 +559,9 @@ ln_block_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __rest
     }
 }
 
+// fp16 rows of more than 96 MB, and as many bytes of results: they do not stay in the L2 (see the packed form).
+static bool ln_packs(int64_t groups, int64_t C) { return groups * C >= (int64_t)48 << 20; }
+
 template <typename InT, typename OutT>
 static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, void* out, float* mean,
                      float* rstd, const void* gamma, const void* beta, float eps) {
@@ -443,6 +580,7 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
         const int vpl = (nvec + 31) / 32;
         const int wpb = 4;
         dim3 grid((unsigned)cdiv(groups, wpb)), block(32 * wpb);
+        constexpr bool PACKS = sizeof(InT) == 2 && sizeof(OutT) == 2;
         // few enough rows that every CTA is resident at once: the latency form (see the kernel)
         const bool lat = groups <= (int64_t)4 * wpb * ctx->prop.multiProcessorCount;
 #define LN_GO(V)                                                                                            \
@@ -450,6 +588,9 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
         if (lat)                                                                                            \
             B200_CUDA(launch_dep(ln_warp_kernel<InT, OutT, V, 32, true>, grid, block, 0, ctx->stream, 1, ap, op, mean, rstd, gp, \
                                  bp, groups, (int)C, eps));                                                 \
+        else if (PACKS && (V) >= 4 && (V) <= 8 && ln_packs(groups, C))                                      \
+            B200_CUDA(launch_dep(ln_warp_kernel<InT, OutT, V, 32, false, PACKS && (V) >= 4 && (V) <= 8>, grid, block, 0, ctx->stream, 1, \
+                                 ap, op, mean, rstd, gp, bp, groups, (int)C, eps));                         \
         else                                                                                                \
             B200_CUDA(launch_dep(ln_warp_kernel<InT, OutT, V>, grid, block, 0, ctx->stream, 1, ap, op, mean, rstd, gp, bp, \
                                  groups, (int)C, eps));                                                     \
@@ -518,6 +659,10 @@ extern "C" int b200_add_layernorm_f16(b200_ctx* ctx, int64_t groups, int64_t C, 
             B200_CUDA(launch_dep(ln_add_warp_kernel<V, 32, true>, grid, block, 0, ctx->stream, 1, (__half*)x, (const __half*)h, \
                                  (__half*)out, mean, rstd, (const __half*)gamma, (const __half*)beta, groups, (int)C, eps, \
                                  use_clamp, lo, hi));                                                             \
+        else if ((V) >= 4 && (V) <= 8 && ln_packs(groups, C))                                                     \
+            B200_CUDA(launch_dep(ln_add_warp_kernel<V, 32, false, (V) >= 4 && (V) <= 8>, grid, block, 0, ctx->stream, 1, (__half*)x, \
+                                 (const __half*)h, (__half*)out, mean, rstd, (const __half*)gamma, (const __half*)beta, groups, (int)C, \
+                                 eps, use_clamp, lo, hi));                                                        \
         else                                                                                                      \
             B200_CUDA(launch_dep(ln_add_warp_kernel<V>, grid, block, 0, ctx->stream, 1, (__half*)x, (const __half*)h,   \
                                  (__half*)out, mean, rstd, (const __half*)gamma, (const __half*)beta, groups, (int)C, eps, \
