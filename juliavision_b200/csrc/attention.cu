@@ -332,7 +332,8 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                 const uint32_t k_addr = smem_u32(smem + Cfg::S_K + sk * Cfg::KV_BYTES);
 #pragma unroll
                 for (int k = 0; k < EP / 16; ++k) {
-                    if (k * 16 >= p.E) break;   // past the head dim both operands are zeros (E = 72: five of eight steps)
+                    // past the head dim both operands are zeros (E = 72: five of eight steps; the fifth always has some)
+                    if (EP == 128 && k >= 5 && k * 16 >= p.E) break;
                     // 16 elements of E = 32 B inside the swizzle row; every fourth step moves to the next atom
                     const uint32_t in = (uint32_t)(k & 3) * 32;
                     umma_ss(s_tmem, smem_desc_at(kdesc0, q_addr + (uint32_t)(k >> 2) * ATT_TILE_BYTES + in),
