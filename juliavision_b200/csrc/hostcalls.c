@@ -61,7 +61,10 @@ static int load(PyObject* o, Arr* a) {
         Py_XDECREF(sh);
         Py_XDECREF(st);
     }
-    if (PyErr_Occurred()) PyErr_Clear();   // the Python route meets it again and reports it
+    if (PyErr_Occurred()) {   // an attribute that is missing or out of range: the Python route meets it again
+        PyErr_Clear();
+        ok = 0;
+    }
     return ok && (a->code == B200_F16 || a->code == B200_F32);
 }
 

@@ -99,6 +99,7 @@ def test_matmul(both):
     agree(both(jv.matmul_, arr(f16, (8, 3)), arr(f16, (8, 4)), arr(f16, (4, 3)), arr(f16, (2, 4))))      # a bias of two axes
     agree(both(jv.matmul_, arr(f16, (8, 3)), arr(f16, (8, 4)), arr(f16, (4, 3)), arr(f16, (8,), (2,))))  # a strided bias
     agree(both(jv.matmul_, arr(f16, (8, 3)), arr(f16, (8, 4)), arr(f16, (4, 3)), None, epi="tanh"))
+    agree(both(jv.matmul_, arr(f16, (8, 3)), arr(f16, (8, 4), ptr=1 << 63), arr(f16, (4, 3)), None))     # past a signed 64-bit integer
     assert taken > 100
 
 
