@@ -29,7 +29,7 @@ __device__ __forceinline__ void gemv_store(OutT* out, int64_t m, float acc, int 
 constexpr int GEMV_WARPS = 16;          // a multiple of 8: a warp's columns share their offset from a 16-byte boundary
 constexpr int GEMV_UNROLL = 8;          // columns in flight per lane: 128 bytes
 constexpr int GEMV_BLOCKS_PER_SM = 2;   // resident blocks of 512 threads at 64 registers
-constexpr int GEMV_SPLIT_MIN_K = 4096;  // see gemv_run
+constexpr int GEMV_SPLIT_MIN_K = 4096;  // (gemv_run)
 constexpr int GEMV_MIN_COLS = 8;        // columns per warp below which a further K split only adds the join
 
 __device__ __forceinline__ float gemv_ld_cluster(uint32_t addr) {
@@ -130,8 +130,8 @@ gemv_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const
     cluster_sync_all();   // nobody leaves while its sums may still be read
 }
 
-// The same with the K axis over up to 64 blocks that are not a cluster: for a few row blocks and a long reduction, which
-// eight parts leave most of the GPU out of.  Partial sums go through the workspace and are added in split order by
+// The same in blocks of eight warps, four columns in flight, with the K axis over up to 64 blocks that are not a cluster
+// (gemv_run says when).  Partial sums go through the workspace and are added in split order by
 // whichever block of a row range finishes last, so the result does not depend on timing.
 constexpr int GEMV_SPLIT_WARPS = 8;
 template <typename T, typename OutT>
@@ -195,8 +195,14 @@ gemv_split_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x,
         float t = 0.f;
 #pragma unroll
         for (int w = 0; w < GEMV_SPLIT_WARPS; ++w) t += red[w][r];
-        partial[(int64_t)blockIdx.y * M + m] = t;
+        if (partial != nullptr) {
+            partial[(int64_t)blockIdx.y * M + m] = t;
+        } else {
+            if (bias != nullptr) t += gemv_tof<T>(bias[m]);
+            gemv_store<OutT>(out, m, t, epi);
+        }
     }
+    if (partial == nullptr) return;
     // K was split over gridDim.y blocks: the one that arrives last adds the partial sums of these rows in
     // split order (so the result does not depend on which block that is) and puts the counter back to zero
     // for the next launch.  Nobody waits on anybody.
@@ -223,29 +229,32 @@ static int gemv_run(b200_ctx* ctx, int64_t M, int64_t K, const void* A, int64_t 
     constexpr int ROWS = 31 * (16 / (int)sizeof(T));
     const int64_t mblocks = cdiv(M, ROWS);
     B200_REQUIRE(mblocks < (1ll << 31), B200_DECLINE_EXTENT, "gemv: M = %lld", (long long)M);
-    // Split K over a cluster's blocks as long as that shortens the time in waves of resident blocks (a last, partial
-    // wave costs a whole one) and every warp keeps GEMV_MIN_COLS columns.
-    // (Up to an SM per block while there are that many SMs: a second block on some of them is a longer chain there.)
-    const int64_t wave = (int64_t)ctx->prop.multiProcessorCount * (mblocks > ctx->prop.multiProcessorCount ? GEMV_BLOCKS_PER_SM : 1);
+    // A cluster's parts: a power of two (clusters of 3 or 7 fill the GPCs badly: 7000 x 3000 in fp32 12 -> 15 us) that
+    // leaves every block an SM of its own and every warp GEMV_MIN_COLS columns.
+    const int64_t sms = ctx->prop.multiProcessorCount;
     int64_t parts = 1;
-    double best = (double)cdiv(mblocks, wave);
-    for (int64_t p = 2; p <= 8 && K >= p * GEMV_WARPS * GEMV_MIN_COLS; p *= 2) {
-        const double t = (double)cdiv(p * mblocks, wave) / (double)p;
-        if (t < 0.9 * best) {
-            best = t;
-            parts = p;
-        }
-    }
-    // Eight parts of so few row blocks would leave nine tenths of the SMs idle over a long chain (256 x 4096: 6.35 us
-    // this way, 6.44 as a cluster; 480 x 2500: 6.8 against 5.7).
-    if (mblocks * 8 * 8 <= ctx->prop.multiProcessorCount && K >= GEMV_SPLIT_MIN_K && ctx->sk_flags != nullptr) {
-        int64_t ksplit = K / (16 * GEMV_SPLIT_WARPS);
+    while (parts < 8 && 2 * parts * mblocks <= sms && K >= 2 * parts * GEMV_WARPS * GEMV_MIN_COLS) parts *= 2;
+    // Taken while a block has up to 290 KB to read, where round trips are what a call waits for (1280 x 1280 in fp16
+    // 6.3 -> 5.0 us, 4390 x 721 in fp32 6.6 -> 5.5, 3000 x 5000 in fp16 10.0 -> 7.6).  With more to read, or more row
+    // blocks than SMs, blocks of eight warps, six to an SM, stream with fewer gaps (9956 x 1817 in fp16 8.9 us against
+    // 9.8, 51865 x 1280 25.3 against 31); and so few row blocks that eight parts would leave nine tenths of the SMs idle
+    // over a long chain are split further that way (256 x 4096: 6.35 us, 6.44 as a cluster).
+    const bool few = mblocks * 8 * 8 <= sms && K >= GEMV_SPLIT_MIN_K;
+    const bool cluster = K == 0 || (!few && mblocks <= sms && M * K * (int64_t)sizeof(T) <= 290 * 1024 * mblocks * parts);
+    if (!cluster && ctx->sk_flags != nullptr) {
+        // K over blocks until the grid is one resident wave, sixteen columns a warp at least
+        const int64_t slots = sms * 6;
+        int64_t ksplit = mblocks >= slots || mblocks > GEMV_COUNTER_COUNT ? 1 : slots / mblocks;
+        const int64_t most = K / (16 * GEMV_SPLIT_WARPS) > 0 ? K / (16 * GEMV_SPLIT_WARPS) : 1;
+        if (ksplit > most) ksplit = most;
         if (ksplit > 64) ksplit = 64;
         const int64_t chunk = cdiv(K, ksplit);
         ksplit = cdiv(K, chunk);
         void* ws = nullptr;
-        int rc = ws_scratch(ctx, (size_t)ksplit * M * sizeof(float), &ws);
-        if (rc) return rc;
+        if (ksplit > 1) {
+            int rc = ws_scratch(ctx, (size_t)ksplit * M * sizeof(float), &ws);
+            if (rc) return rc;
+        }
         gemv_split_kernel<T, OutT><<<dim3((unsigned)mblocks, (unsigned)ksplit), dim3(32, GEMV_SPLIT_WARPS), 0, ctx->stream>>>(
             (const T*)A, lda, (const T*)x, (const T*)bias, (OutT*)out, static_cast<float*>(ws), ctx->sk_flags + SK_FLAG_COUNT, M, K,
             chunk, epi);

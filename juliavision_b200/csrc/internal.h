@@ -77,7 +77,7 @@ struct b200_ctx {
 };
 
 constexpr int SK_FLAG_COUNT = 4096;
-constexpr int GEMV_COUNTER_COUNT = 64;     // arrival counters of the split matrix-vector product, after the flags
+constexpr int GEMV_COUNTER_COUNT = 1024;    // arrival counters of the split matrix-vector product, after the flags
 
 struct b200_event {
     cudaEvent_t ev = nullptr;
