@@ -328,7 +328,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
         // under `if (lane == 0)` a k-block took 560-590 cycles unless a further warp did the waiting for it and handed
         // each stage over through a named barrier; against that pair of warps this takes 0 to 15 % off most launches
         // (160 x 2304 x 768: 8.0 -> 7.3 us, 1500 x 3840 x 1280: 25.3 -> 24.0, 8192 x 3584 x 896 with GELU: 57.6 -> 48.6,
-        // 65536 x 5120 x 1280 unchanged) and adds as much to a few of short K (32768 x 1344 x 448: 42.5 -> 47.4).
+        // 65536 x 5120 x 1280 unchanged; 32768 x 1344 x 448 moves between 42 and 47 on either side).
         if (rank == 0) {
             constexpr uint32_t idesc = make_idesc_f16(TILE_N, Cfg::WIDE ? 256 : BN, /*a K-major*/ 0, /*b MN-major*/ 1);
             const uint32_t idesc2 = make_idesc_f16(TILE_N, p.bn - 256, 0, 1);   // wide tile: the columns past 256
@@ -729,7 +729,14 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
     for (const Cand& c : cands) {   // whole-tile schedules first: stream-K has to beat the best of them clearly
         const int64_t tiles = cdiv(M, c.bn) * cdiv(N, (int64_t)GEMM_BM * c.ncta) * nbatch;
         const int64_t waves = cdiv(tiles, (int64_t)(sms / c.ncta));
-        const double dp = (double)waves * ((double)nkb * c.t_kb + t_tile);
+        // One to three rounds: t_tile per round, and a pair's set-up and hand-overs show where a tile is only a few k-blocks
+        // long (1067 x 1224 x 144: 5.9 us on 128x2 tiles, 5.2 on 128x1; 18600 x 160 x 192: 6.6 on 256x2, 5.6 on 256x1).
+        // Over many rounds a tile's epilogue runs under the next one's main loop and only a part of it shows, less than
+        // half as much for half the columns (524288 x 336 x 112: 2.5 us a round on 256x2 tiles, 1.4 on 128x2; with four
+        // to fifteen rounds the same estimate picked worse tiles as often as better ones).
+        const bool many = waves >= 16;
+        const double tile = many ? (c.bn == 256 ? 1.3 : 0.5) : t_tile + (c.ncta == 2 && nkb <= 8 ? 0.4 : 0.0);
+        const double dp = (double)waves * ((double)nkb * c.t_kb + tile);
         if (dp < best_cost - 1e-9) {
             best_cost = dp;
             best = {c.bn, c.ncta, 0, 0, 1};

@@ -6,7 +6,7 @@ import pytest
 import juliavision_b200 as jv
 
 from .conftest import relerr
-from .gpu_helpers import attention_gpu, describe
+from .gpu_helpers import attention_gpu, describe, qkv_views
 
 pytestmark = pytest.mark.gpu
 G = os.path.join(os.path.dirname(__file__), "golden")
@@ -402,3 +402,29 @@ def test_few_queries_in_one_launch(ctx, ora, B, H, Lq, Lk, E, masked):
         assert relerr(got, ref) < 2e-3, describe(got, ref, 2e-3)
         if masked:
             assert np.all(got[:, :, Lq - 1] == 0)
+
+
+# (B, H, Lq, Lk, E) with more than 296 query tiles: one key past the window kernel's, one block and four of them, ragged
+# tiles, one query past the few-query kernel's
+SHORT = [(150, 2, 65, 65, 64), (300, 1, 33, 129, 32), (100, 3, 130, 200, 56), (75, 4, 256, 256, 64), (160, 2, 100, 64 * 3, 8)]
+
+
+@pytest.mark.parametrize("B,H,Lq,Lk,E", SHORT)
+def test_short_keys_share_an_sm(ctx, ora, B, H, Lq, Lk, E):
+    """One query tile per CTA, four CTAs per SM; operands side by side in one projection, result token-major."""
+    rng = np.random.default_rng(B + Lq + Lk)
+    buf = np.float16(rng.standard_normal((B, max(Lq, Lk), 3, H, E)))
+    q, k, v = (buf[:, :n, i].transpose(0, 2, 1, 3) for i, n in enumerate((Lq, Lk, Lk)))
+    dq, dk, dv = qkv_views(ctx, q, k, v)
+    ref = ora.attention_ref(q, k, v, 1 / np.sqrt(E))
+    for dt in (np.float16, np.float32):
+        flat = ctx.allocate(dt, E * H, Lq * B)
+        ctx.fill_bytes(flat, 0xFF)
+        out = jv.DeviceArray(ctx, flat.ptr, dt, (E, Lq, H, B), (1, E * H, E, E * H * Lq), owner=flat)
+        ctx.ws.reset()
+        jv.sdpa(ctx, dq, dk, dv, None, 1 / np.sqrt(E), out=out)
+        ctx.synchronize()
+        got = flat.to_host().reshape(B, Lq, H, E).transpose(0, 2, 1, 3)
+        assert np.all(np.isfinite(got))
+        # P is rounded to fp16 (2^-11 per key, averaged over them) and, for fp16, the result once more
+        assert relerr(got, ref) < 2e-3, describe(got, ref, 2e-3)
