@@ -532,8 +532,12 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                 // it follows the true maximum lazily, moving (and rescaling O and the running sum)
                 // only when the maximum has grown by more than 2^8.  Any reference point gives the
                 // same quotient O / l; the lazy one makes rescales rare after the first blocks.
+                // The key at the reference point has P = 1, which fp16 holds exactly, and it is the key with the largest
+                // weight: so the first 128 keys give their maximum in every form, also where they are two blocks (left
+                // lazy there, the result of 256-key windows was 1.6 to 2 % further from 64 bits, for 2 % of their time).
                 const float m_blk = mx * sce;
-                const float m_new = (m_blk > m_run + 8.0f) ? m_blk : m_run;
+                const float slack = (BC < 128 && j == 1) ? 0.0f : 8.0f;
+                const float m_new = (m_blk > m_run + slack) ? m_blk : m_run;
                 // 0 on the first block (m_run = -inf), else 1 or < 2^-8.  With a mask a row may have seen
                 // nothing but -inf so far: then the reference point stays -inf and nothing is rescaled.
                 const float alpha = (BIAS && m_run == m_new) ? 1.0f : ex2(m_run - m_new);
@@ -1029,8 +1033,8 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     const bool wide = E > 64;                              // two swizzle atoms along E
     const int64_t sms = ctx->prop.multiProcessorCount;
     // Up to 256 keys and more than two tiles per SM (16 x 16 windows): one tile per CTA, four CTAs per SM, so that one's
-    // set-up, loads and hand-offs run under the others' arithmetic: 1024 of 256 x 256, E = 56: 65 -> 54 us, 287 of 196 x
-    // 196: 17.0 -> 15.4.  With long keys its blocks of 64 hold the tensor pipe as long as blocks of 128 (64 cycles a UMMA
+    // set-up, loads and hand-offs run under the others' arithmetic: 1024 x 2 heads of 256 x 256, E = 56: 118 -> 91 us,
+    // 287 x 2 heads of 196 x 196, E = 64: 30.5 -> 26.9.  With long keys its blocks of 64 hold the tensor pipe as long as blocks of 128 (64 cycles a UMMA
     // whatever N), and it loses: 12 heads x 4096 x 4096 85.7 -> 126.7.
     const bool single = !wide && bptr == nullptr && Lk <= 256 && cdiv(Lq, ATT_BR) * H * B > 2 * sms;
     const int block = single ? AttCfg<64, false, 1>::BC : AttCfg<64>::BC;

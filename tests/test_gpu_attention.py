@@ -428,3 +428,26 @@ def test_short_keys_share_an_sm(ctx, ora, B, H, Lq, Lk, E):
         assert np.all(np.isfinite(got))
         # P is rounded to fp16 (2^-11 per key, averaged over them) and, for fp16, the result once more
         assert relerr(got, ref) < 2e-3, describe(got, ref, 2e-3)
+
+
+@pytest.mark.parametrize("first,best", [(3, 5), (3, 64), (63, 127), (10, 100)])
+@pytest.mark.parametrize("Lk", [128, 196, 256])
+def test_the_heaviest_of_the_first_128_keys_is_not_rounded(ctx, Lk, first, best):
+    """One key holds nearly all of a row's weight, another up to 2^8 less, the rest nothing.  The heavy one lies in the
+    first 128 keys, so its probability is the reference point of the exponentials and exact: what is left is the
+    rounding of the light one (at least 2^-6 of the weight at 2^-11) and of fp32.  Whole tiles, four CTAs per SM."""
+    B, H, Lq, E = 160, 2, 128, 64
+    rng = np.random.default_rng(Lk + best)
+    q, k = np.zeros((B, H, Lq, E), np.float16), np.zeros((B, H, Lk, E), np.float16)
+    q[..., 0] = 1
+    k[..., 0] = -20                                    # 2^-28 of the first key
+    k[:, :, first, 0] = 0
+    k[:, :, best, 0] = 4.2 + 1.3 * rng.random((B, H))   # 2^6 to 2^7.95 times the first key
+    v = np.float16(rng.standard_normal((B, H, Lk, E)))
+    got, _ = attention_gpu(ctx, q, k, v, 1.0, np.float32)
+    s = k[..., 0].astype(np.float64)
+    p = np.exp(s - s.max(-1, keepdims=True))
+    ref = np.einsum("bhk,bhke->bhe", p / p.sum(-1, keepdims=True), v.astype(np.float64))[:, :, None]
+    # 2^-6 * 2^-11 of the light key's value, plus a few fp32 roundings, against values of size one
+    err = np.abs(got - ref).max() / np.abs(ref).max()
+    assert err < 1.2e-5, err
