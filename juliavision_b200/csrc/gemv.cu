@@ -4,7 +4,7 @@
 // when it is not: every byte of A is read once, as aligned 16-byte vectors whatever the leading dimension (a
 // vocabulary of 51865 rows gives every column its own misalignment), a warp covering 512 contiguous bytes of a
 // column, the K axis split over the warps of a block and, when M alone cannot fill the GPU, over the blocks of a
-// cluster as well, whose sums meet in distributed shared memory and are added in rank order (so the result does not
+// cluster as well, whose sums meet in distributed shared memory and are added in one fixed order (so the result does not
 // depend on timing).  1280 x 1280 in fp16 6.3 -> 5.0 us and 594 x 1685 in fp32 6.0 -> 4.1 against partial sums through
 // the workspace and half as many columns in flight.
 #include <cuda_fp16.h>
@@ -36,6 +36,18 @@ __device__ __forceinline__ float gemv_ld_cluster(uint32_t addr) {
     float v;
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
     return v;
+}
+
+// Pairwise sum.  With results kept in fp32 the columns of a warp are added two at a time as well: as one chain over them
+// and one over the warps, those results were up to 17 % further from 64 bits than with the fewer columns that a warp of
+// gemv_split_kernel takes (10428 x 429: 1.24e-7 against 1.06e-7).  Rounded to fp16 none of this shows, and there the
+// shorter chains would cost 2 to 4 % of the time.
+template <int N> __device__ __forceinline__ float gemv_pairs(float (&v)[N]) {
+#pragma unroll
+    for (int h = N / 2; h > 0; h /= 2)
+#pragma unroll
+        for (int i = 0; i < h; ++i) v[i] += v[i + h];
+    return v[0];
 }
 
 // grid (m blocks, k parts); block (32, GEMV_WARPS); the k parts of an m block form a cluster.
@@ -87,10 +99,18 @@ gemv_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const
                     xv[u] = in ? gemv_tof<T>(x[k + u * GEMV_WARPS]) : 0.f;
                 }
 #pragma unroll
-                for (int u = 0; u < UN; ++u) {
+                for (int u = 0; u < UN; u += 2) {
                     const T* e = reinterpret_cast<const T*>(&a[u]);
+                    const T* f = reinterpret_cast<const T*>(&a[u + 1]);
 #pragma unroll
-                    for (int v = 0; v < VEC; ++v) acc[v] = fmaf(gemv_tof<T>(e[v]), xv[u], acc[v]);
+                    for (int v = 0; v < VEC; ++v) {
+                        if constexpr (sizeof(OutT) == 4) {   // two columns at a time: half the chain (see gemv_pairs)
+                            acc[v] += fmaf(gemv_tof<T>(f[v]), xv[u + 1], gemv_tof<T>(e[v]) * xv[u]);
+                        } else {
+                            acc[v] = fmaf(gemv_tof<T>(e[v]), xv[u], acc[v]);
+                            acc[v] = fmaf(gemv_tof<T>(f[v]), xv[u + 1], acc[v]);
+                        }
+                    }
                 }
             }
         }
@@ -109,9 +129,10 @@ gemv_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const
         gemv_store<OutT>(out, m, t, epi);
     };
     for (int r = tid; r < ROWS; r += 32 * GEMV_WARPS) {
-        float t = 0.f;
+        float v[GEMV_WARPS];
 #pragma unroll
-        for (int w = 0; w < GEMV_WARPS; ++w) t += red[w][r];
+        for (int w = 0; w < GEMV_WARPS; ++w) v[w] = red[w][r];
+        const float t = gemv_pairs(v);
         if (parts > 1) sums[r] = t;
         else finish(r, t);
     }
@@ -120,12 +141,10 @@ gemv_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const
     const int rank = (int)blockIdx.y;
     const uint32_t mine = smem_u32(sums);
     for (int r = tid * parts + rank; r < ROWS; r += 32 * GEMV_WARPS * parts) {
-        float v[8], t = 0.f;   // every part's load in flight together: a remote load takes a few hundred nanoseconds
+        float v[8];   // every part's load in flight together: a remote load takes a few hundred nanoseconds
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] = q < parts ? gemv_ld_cluster(mapa_u32(mine + r * 4, (uint32_t)q)) : 0.f;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) t += v[q];
-        finish(r, t);
+        finish(r, gemv_pairs(v));
     }
     cluster_sync_all();   // nobody leaves while its sums may still be read
 }
