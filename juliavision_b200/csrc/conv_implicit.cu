@@ -277,7 +277,6 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
         }
     }
     if (Cfg::SPLITS && parts > 1) {
-        __syncwarp();
         cluster_sync_all();   // every part's tile is in its shared memory
         if (warp < 8) {
             const uint32_t mine = smem_u32(smem) + (tid & 127) * 4;
@@ -301,7 +300,6 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
                 }
             }
         }
-        __syncwarp();
         cluster_sync_all();   // nobody leaves while its tile may still be read
     }
     if (*abort_flag) {   // let any TMA copy still in flight into this CTA's shared memory land before exit

@@ -493,7 +493,6 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
                     for (int q = 0; q < CH / 4; ++q)
                         st_shared_v4(dump + (uint32_t)(chunk_col(c) / 4 + q) * (GEMM_BM * 16), r + 4 * q);
                 }
-                __syncwarp();
                 met = true;
                 cluster_sync_all();   // every part's accumulator is in its shared memory (the other roles arrive below)
             }
@@ -640,7 +639,6 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
     // Teardown: every role arrives here whether it finished or gave up.
     if constexpr (KSPLIT) {
         // the barrier between the two halves of the epilogue: the roles without one, and epilogue warps that gave up
-        __syncwarp();
         if (!met) cluster_sync_all();
     }
     if (*abort_flag) {

@@ -345,7 +345,10 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
+// The barrier's aligned form wants the lanes of a warp together: callers come here out of loops and branches that differ by
+// lane, after which nothing else brings them back together.
 __device__ __forceinline__ void cluster_sync_all() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // shared::cluster address of `local_smem_addr` as seen in CTA `rank` of the cluster.

@@ -1,0 +1,24 @@
+"""Rules of the instruction set that a GPU run cannot show to be kept, read off the sources (no GPU)."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "juliavision_b200", "csrc")
+
+
+def sources():
+    for name in sorted(os.listdir(CSRC)):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, name)) as f:
+                yield name, re.sub(r"//[^\n]*", "", f.read())
+
+
+def test_cluster_barriers_bring_the_warp_together_first():
+    """barrier.cluster.arrive.aligned is undefined when the lanes of a warp arrive apart, and its callers come out of loops
+    whose trip counts differ by lane: whoever issues it converges the warp in the statement before."""
+    seen = 0
+    for name, text in sources():
+        for m in re.finditer(r"[^;{}]*[;{}]\s*asm volatile\(\s*\"[^;]*barrier\.cluster\.arrive", text):
+            assert m.group(0).split(";")[0].strip() == "__syncwarp()", (name, m.group(0))
+            seen += 1
+        assert len(re.findall(r"barrier\.cluster\.arrive", text)) == (1 if name == "ptx.cuh" else 0), name
+    assert seen == 1
