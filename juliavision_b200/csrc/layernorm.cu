@@ -501,6 +501,20 @@ ln_wide_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
             float y[VN];
 #pragma unroll
             for (int j = 0; j < VN; ++j) y[j] = (x[i][j] - mu) * r;
+            if (sizeof(OutT) == 4 && gamma && beta) {
+                // gamma and beta in one rounding, as in ln_block_kernel: with two, fp32 results were 7 % further from 64
+                // bits (rounded to fp16 it does not show, and there both vectors at once cost registers and 17 % of the time)
+                Vec16<InT> tg, tb;
+                float gf[VN], bf[VN];
+                tg.raw = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
+                tb.raw = __ldg(reinterpret_cast<const uint4*>(beta) + v);
+                tg.to_f32(gf);
+                tb.to_f32(bf);
+#pragma unroll
+                for (int j = 0; j < VN; ++j) y[j] = fmaf(y[j], gf[j], bf[j]);
+                store_vec<VN>(dst + (int64_t)v * VN, y);
+                continue;
+            }
             if (gamma) {
                 Vec16<InT> t;
                 float gf[VN];

@@ -54,6 +54,19 @@ def test_rows_wider_than_a_warp_holds(ctx, ora, dt, C):
     assert np.max(np.abs(mean - rmean)) < 1e-5 and relerr(rstd, rrstd) < 1e-5
 
 
+@pytest.mark.parametrize("C", [2052, 4280, 8192, 8196])
+def test_rows_wider_than_a_warp_holds_round_gamma_and_beta_once(ctx, C):
+    """fp32, where it shows: y gamma + beta is one rounding of the row's own y = (x - mean) rstd, in the form of a block
+    per row as in the general one (C = 8196).  64 bits hold the product of two fp32 numbers exactly."""
+    rng = np.random.default_rng(C)
+    a = np.float32(rng.standard_normal((37, C)) * 2 + 0.5)
+    gam, bet = np.float32(1 + 0.1 * rng.standard_normal(C)), np.float32(rng.standard_normal(C))
+    got, mean, rstd = layernorm_gpu(ctx, a, gam, bet, 1e-5)
+    y = (a - mean.reshape(-1, 1)) * rstd.reshape(-1, 1)
+    once = np.float32(y.astype(np.float64) * gam + bet)
+    assert np.mean(got != once) < 1e-4      # a double rounding where 64 bits end on a tie
+
+
 def test_mean_dominates_variance(ctx, ora):
     a = (np.float32(1000.0) + np.float32(0.5) * np.sin(np.arange(4 * 256, dtype=np.float32))).reshape(4, 256)
     got, _, _ = layernorm_gpu(ctx, a, eps=1e-5)
