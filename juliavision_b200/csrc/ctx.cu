@@ -142,14 +142,14 @@ int ws_scratch(b200_ctx* ctx, size_t bytes, void** out) {
     size_t off = round_up(ctx->ws_used, 256);
     size_t need = off + bytes;
     if (!ctx->ws_buf || need > ctx->ws_cap) {
-        // Retire, never release here: pointers handed out earlier in this op still point
-        // into the old block and their kernels may not have run yet.
-        if (ctx->ws_buf) ctx->ws_retired.push_back({ctx->ws_buf, ctx->ws_cap});
         size_t cap = need + need / 2;
         if (cap < (1u << 20)) cap = 1u << 20;
         void* p = nullptr;
         int rc = pool_alloc(ctx, cap, &p);
-        if (rc) return rc;
+        if (rc) return rc;   // the block at hand stays the workspace
+        // Retire, never release here: pointers handed out earlier in this op still point
+        // into the old block and their kernels may not have run yet.
+        if (ctx->ws_buf) ctx->ws_retired.push_back({ctx->ws_buf, ctx->ws_cap});
         ctx->ws_buf = p;
         ctx->ws_cap = cap;
         // A fresh block starts at offset 0, as the reference's does: `off` was computed

@@ -172,6 +172,29 @@ def test_memory_a_graph_uses_is_not_handed_to_anyone_else(ctx):
         assert res2.value == res.value, "the released workspace block was not reused"
 
 
+def test_a_refused_workspace_request_leaves_the_workspace_as_it_was(ctx):
+    """Growth is refused while a graph is recorded.  The block at hand must stay the workspace's own: were it retired on
+    the way, the next reset would give it to the pool while scratch is still handed out from it."""
+    import ctypes as C
+    with jv.Ctx(0) as c:
+        L = _lib.lib()
+        first = c.ws.scratch(np.uint8, 1 << 12)
+        c.ws.reset()
+        before = c.ws.stats()
+        _lib.check(L.b200_graph_begin(c.handle))
+        p, g = C.c_void_p(), C.c_void_p()
+        rc = L.b200_workspace_scratch(c.handle, 64 * before[1], C.byref(p))
+        _lib.check(L.b200_graph_end(c.handle, C.byref(g)))
+        _lib.check(L.b200_graph_destroy(g))
+        assert rc == _lib.ENOMEM and c.ws.stats() == before
+        c.ws.reset()
+        other = [c.allocate(np.uint8, before[1]) for _ in range(2)]
+        again = c.ws.scratch(np.uint8, 1 << 12)
+        assert again.ptr == first.ptr and c.ws.stats()[1] == before[1]
+        for a in other:
+            assert a.ptr + a.nbytes <= again.ptr or again.ptr + before[1] <= a.ptr, "the pool gave the workspace away"
+
+
 def test_a_wait_that_cannot_be_satisfied_runs_out_and_the_context_carries_on(ctx):
     """Bounded waits: a one-warp kernel waits 2 ms on a barrier nothing arrives at.  It must return, the
     next sync must report the kernel status once, and the same context must then compute correctly."""
