@@ -1079,6 +1079,7 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     p.ntail = 0;
     p.part_o = p.part_ml = nullptr;
     const int64_t rem = pairs % sms;
+    const size_t ws_mark = ctx->ws_used;
     if (!single && nblk_all >= 4) {
         int64_t ntail = 0, ns = 1;
         if (2 * pairs <= sms) {
@@ -1094,11 +1095,15 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
             const int64_t rows = ntail * item_rows;
             void* ws = nullptr;
             rc = ws_scratch(ctx, (size_t)(ns * rows * (E + 2)) * sizeof(float), &ws);
-            if (rc) return rc;
-            p.nsplit = (int)ns;
-            p.ntail = (int)ntail;
-            p.part_o = static_cast<float*>(ws);
-            p.part_ml = p.part_o + ns * rows * E;
+            // A masked call does not depend on the workspace: it runs unsplit when that is refused (a graph recorded
+            // without an eager call before), and gives its share back below.
+            if (rc && !(bptr && rc == B200_ENOMEM)) return rc;
+            if (!rc) {
+                p.nsplit = (int)ns;
+                p.ntail = (int)ntail;
+                p.part_o = static_cast<float*>(ws);
+                p.part_ml = p.part_o + ns * rows * E;
+            }
         }
     }
     if (p.nsplit > 1) {
@@ -1110,6 +1115,7 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
                              (const float*)p.part_o, (const float*)p.part_ml, p.nsplit, p.ntail, p.pair_ctas, p.qpairs, (int)item_rows, (int)E,
                              (int)Lq, (int)H, out, o->stride[1], o->stride[2], o->stride[3], (int)(out_dtype == B200_F32)));
         ctx->launches += 2;
+        if (bptr) ctx->ws_used = ws_mark;   // what comes next on the stream runs after the merge has read the partial rows
         return B200_OK;
     }
     // Split the pairs of a last wave that would leave more than half of the SMs idle — but not a
