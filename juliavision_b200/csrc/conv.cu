@@ -126,21 +126,33 @@ static int conv2d_group(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_
     // The implicit kernel where the GEMM cannot store the result, and where it has two pixel tiles per SM or more; a small
     // image the GEMM can store is as fast through a small im2col matrix (64 x 58 x 24 -> 64: 7.5 us, implicit 12).
     const bool aligned = P % 8 == 0 && out_img * osz % 16 == 0 && al16(out);   // the GEMM can store the result
-    const bool implicit = conv_implicit_takes(W, H, Cin, N, KW, KH, Cout, P) &&
-                          (onebyone ? !(aligned && x_img % 8 == 0 && al16(x)) : !aligned || cdiv(P, 128) * N >= 2 * ctx->prop.multiProcessorCount);
-    if (CRS % 8 != 0 || (implicit && !al16(w))) {
+    bool implicit = conv_implicit_takes(W, H, Cin, N, KW, KH, Cout, P) &&
+                    (onebyone ? !(aligned && x_img % 8 == 0 && al16(x)) : !aligned || cdiv(P, 128) * N >= 2 * ctx->prop.multiProcessorCount);
+    const size_t ws_mark = ctx->ws_used;
+    const bool padded = CRS % 8 != 0;
+    if (padded || (implicit && !al16(w))) {
         ldw = (CRS + 7) / 8 * 8;
         void* wp = nullptr;
-        if ((rc = ws_scratch(ctx, (size_t)(ldw * Cout) * 2, &wp))) return rc;
-        padrows_f16_kernel<<<grid_for(ctx, ldw * Cout), 256, 0, ctx->stream>>>((__half*)wp, (const __half*)w,
-                                                                                (int)CRS, (int)ldw, ldw * Cout);
-        ctx->launches++;
-        B200_CUDA(cudaGetLastError());
-        wB = wp;
+        rc = ws_scratch(ctx, (size_t)(ldw * Cout) * 2, &wp);
+        // A weight that only lies off a 16-byte boundary is copied for the implicit kernel alone; the other route takes
+        // it as it is, so a refusal (a graph recorded without an eager call before) is no reason to fail.
+        if (rc && (padded || rc != B200_ENOMEM)) return rc;
+        if (rc) {
+            implicit = false;
+        } else {
+            padrows_f16_kernel<<<grid_for(ctx, ldw * Cout), 256, 0, ctx->stream>>>((__half*)wp, (const __half*)w,
+                                                                                    (int)CRS, (int)ldw, ldw * Cout);
+            ctx->launches++;
+            B200_CUDA(cudaGetLastError());
+            wB = wp;
+        }
     }
-    if (implicit)
-        return conv_implicit_launch(ctx, W, H, Cin, N, KW, KH, Cout, sx, sy, px, py, dx, dy, OW, P, x, x_img, wB, ldw, bias, out,
-                                    out_img, out_dtype, epilogue);
+    if (implicit) {
+        rc = conv_implicit_launch(ctx, W, H, Cin, N, KW, KH, Cout, sx, sy, px, py, dx, dy, OW, P, x, x_img, wB, ldw, bias, out,
+                                  out_img, out_dtype, epilogue);
+        if (!padded) ctx->ws_used = ws_mark;   // that copy is not kept: what comes next on the stream runs after it was read
+        return rc;
+    }
     if (onebyone) {
         for (int64_t n = 0; n < N; ++n) {
             const __half* xa = x + n * x_img; // (P, Cin) ld = P

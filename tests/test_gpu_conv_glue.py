@@ -93,6 +93,37 @@ def test_conv_gathered_into_the_tiles(ctx, ora, N, Cin, H, W, Cout, KH, KW, stri
     assert relerr(got, ref) < tol, describe(got, ref, tol)
 
 
+@pytest.mark.parametrize("Cin,Cout,H,W", [(24, 40, 17, 19), (8, 257, 33, 31)])
+def test_a_weight_off_its_boundary_does_not_depend_on_the_workspace(ora, Cin, Cout, H, W):
+    """A 1x1 convolution of an odd image needs no scratch but for a weight that starts off a 16-byte boundary, which the
+    implicit kernel wants copied.  Recorded on a context that has no workspace yet it runs all the same; in a loop
+    without a reset it leaves the workspace as it found it."""
+    rng = np.random.default_rng(Cout)
+    x = np.float16(rng.standard_normal((1, Cin, H, W)) * 0.5)
+    w = np.float16(rng.standard_normal((Cout, Cin, 1, 1)) * 0.2)
+    ref = ora.conv2d(x, w, None, out_dtype=np.float32)
+    with jv.Ctx(0) as c:
+        dx, base = c.toback(x), c.toback(np.concatenate([np.float16([0]), w.reshape(-1)]))
+        dw = jv.DeviceArray(c, base.ptr + 2, np.float16, (1, 1, Cin, Cout), owner=base)
+        out = c.allocate(np.float32, W, H, Cout, 1)
+        call = lambda: jv.convolution_(c, out, dx, dw, None, (1, 1), (0, 0), (1, 1))
+        c.fill_bytes(out, 0xFF)
+        g = c.capture(call)
+        assert c.ws.stats()[1] == 0
+        g.replay()
+        c.synchronize()
+        assert relerr(out.to_host(), ref) < 2e-5      # fp32 sums in another order
+        c.fill_bytes(out, 0xFF)
+        call()
+        cap = c.ws.stats()
+        assert cap[0] == 0 and cap[1] > 0
+        for _ in range(20):
+            call()
+        c.synchronize()
+        assert c.ws.stats() == cap
+        assert relerr(out.to_host(), ref) < 2e-5
+
+
 def test_im2col_bit_exact(ctx, ora):
     import ctypes as C
     from juliavision_b200 import _lib
