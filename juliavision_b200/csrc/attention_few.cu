@@ -11,6 +11,9 @@
 // products are warp-level m16n8k16 tiles in registers, four warps sharing a block by queries and keys.  Measured against
 // that: 23 x 4096, 8 heads 14.5 -> 9.2 us; masked, 3 x 477, 13 heads 29 -> 6, 2 x 7763, E = 128, 8 heads 419 -> 21.
 #include <cuda_fp16.h>
+#include <stdlib.h>
+
+#include <atomic>
 
 #include "internal.h"
 #include "ptx.cuh"
@@ -323,16 +326,41 @@ attention_few_kernel(const FewParams p) {
     if (parts > 1) cluster_sync_all();   // nobody leaves while its rows may still be read
 }
 
+// The largest cluster of this kernel, up to AF_PARTS, of which the device can hold one: 16 is beyond the portable size,
+// and a slice of a GPU may have fewer SMs to a GPC.  Asked of the runtime once per device.
+template <typename Kern> static int af_largest(Kern kern, size_t smem) {
+    for (int n = AF_PARTS; n > 8; n /= 2) {
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)n;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)n, 1, 1);
+        cfg.blockDim = dim3(AF_THREADS, 1, 1);
+        cfg.dynamicSmemBytes = smem;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess && fit > 0) return n;
+        cudaGetLastError();
+    }
+    return 8;   // portable
+}
+
 template <int EP, int KS, bool BIAS>
 static int af_launch(b200_ctx* ctx, const FewParams& p, int64_t H, int64_t B, int parts) {
     using Cfg = AfCfg<EP, KS>;
-    static bool attr_done[16] = {};
+    static std::atomic<int> largest[16] = {};
     auto kern = attention_few_kernel<EP, KS, BIAS>;
-    if (!attr_done[ctx->device & 15]) {
+    int most = largest[ctx->device & 15].load(std::memory_order_acquire);
+    if (most == 0) {
         B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
-        B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        attr_done[ctx->device & 15] = true;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) most = af_largest(kern, Cfg::SMEM_BYTES);
+        else most = 8, cudaGetLastError();
+        largest[ctx->device & 15].store(most, std::memory_order_release);
     }
+    if (parts > most) parts = most;
     B200_CUDA(launch_dep(kern, dim3((unsigned)parts, (unsigned)H, (unsigned)B), dim3(AF_THREADS, 1, 1), Cfg::SMEM_BYTES, ctx->stream,
                          parts, p));
     ctx->launches++;
@@ -368,8 +396,9 @@ int attention_few_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64
     p.scale_log2 = scale * 1.4426950408889634f;
     // Key parts: as many as keep every CTA resident at once (two per SM) with two blocks or more each.
     const int64_t nblk = cdiv(Lk, AF_BC), room = 2 * (int64_t)ctx->prop.multiProcessorCount;
-    int parts = 1;
-    while (parts < AF_PARTS && 2 * parts * H * B <= room && nblk >= 4 * parts) parts *= 2;
+    int parts = 1, most = AF_PARTS;
+    if (const char* f = getenv("B200_ATTENTION_PARTS")) most = atoi(f);   // debugging aid: the largest cluster to form
+    while (2 * parts <= most && 2 * parts * H * B <= room && nblk >= 4 * parts) parts *= 2;
     return E <= 64 ? af_slots<64>(ctx, p, H, B, parts) : af_slots<128>(ctx, p, H, B, parts);
 }
 

@@ -481,3 +481,19 @@ def test_masked_calls_do_not_depend_on_the_workspace(ora, B, H, Lq, Lk, E):
         c.synchronize()
         assert c.ws.stats() == cap
         assert relerr(out.to_host(), ref) < 2e-3
+
+
+@pytest.mark.parametrize("B,H,Lq,Lk,E", [(1, 2, 23, 4096, 64), (1, 3, 5, 4500, 128)])
+def test_few_queries_with_smaller_clusters(ctx, ora, B, H, Lq, Lk, E, monkeypatch):
+    """Clusters of sixteen are more than every device must hold: the same kernel with the keys over eight CTAs and fewer,
+    down to one, which walk the ring up to sixteen times as often.  fp32 shows that the split did change."""
+    rng = np.random.default_rng(Lk)
+    q, k, v = (np.float16(rng.standard_normal((B, H, n, E))) for n in (Lq, Lk, Lk))
+    ref = ora.attention_ref(q, k, v, 1 / np.sqrt(E))
+    seen = []
+    for most in (16, 8, 4, 2, 1):
+        monkeypatch.setenv("B200_ATTENTION_PARTS", str(most))
+        got, _ = attention_gpu(ctx, q, k, v, 1 / np.sqrt(E), np.float32)
+        assert relerr(got, ref) < 2e-3, (most, describe(got, ref, 2e-3))     # P rounded to fp16
+        assert not any(np.array_equal(got, s) for s in seen), most
+        seen.append(got)
