@@ -379,6 +379,31 @@ def test_timeline_records_time_and_cycles(ctx):
     assert not tl.to_host().any()
 
 
+@pytest.mark.parametrize("tile", ["64x1k2", "128x1k8"])
+def test_timeline_of_a_cluster_is_one_cta(ctx, tile, monkeypatch):
+    """With a K split the worker is a cluster, and its first CTA records: events in order and a plausible clock from first
+    to last, one exit per tile, launch after launch."""
+    from juliavision_b200 import _lib
+    monkeypatch.setenv("B200_GEMM_TILE", tile)
+    rng = np.random.default_rng(2)
+    X = ctx.toback(np.float16(rng.standard_normal((128, 2048)) * 0.05))
+    W = ctx.toback(np.float16(rng.standard_normal((2048, 512)) * 0.05))
+    out = ctx.allocate(np.float16, 512, 128)
+    tl = ctx.allocate(np.uint64, 256)
+    for _ in range(8):
+        ctx.fill_bytes(tl, 0)
+        _lib.check(_lib.lib().b200_timeline(ctx.handle, tl.ptr))
+        jv.matmul_(ctx, out, W, X, None)
+        ctx.synchronize()
+        _lib.check(_lib.lib().b200_timeline(ctx.handle, None))
+        t = tl.to_host().astype(np.int64)
+        assert 0 < t[0] <= t[1] <= t[3] <= t[4] <= t[8] <= t[12] <= t[16]
+        for a, b in ((0, 16), (0, 8), (4, 12)):
+            ns, clk = t[b] - t[a], t[64 + b] - t[64 + a]
+            assert ns >= 0 and abs(clk / 1.4 - ns) < 1000 + 0.8 * ns       # 0.8 to 2.2 GHz, the clock ticks in steps
+        assert np.count_nonzero(t[128:]) == 512 // int(tile.split("x")[0])
+
+
 def test_weight_operand_produced_by_the_previous_launch(ctx):
     """Launches overlap their predecessor's tail (programmatic dependent launch) and must not read an operand
     before the dependency wait.  Here the first product is the second one's A operand (as in a batched

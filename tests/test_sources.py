@@ -22,3 +22,13 @@ def test_cluster_barriers_bring_the_warp_together_first():
             seen += 1
         assert len(re.findall(r"barrier\.cluster\.arrive", text)) == (1 if name == "ptx.cuh" else 0), name
     assert seen == 1
+
+
+def test_one_cta_of_a_worker_writes_the_timeline():
+    """Every CTA of a worker (a pair, or a cluster along K) runs the lines that record events; only one may write."""
+    text = dict(sources())["gemm.cu"]
+    writes = [m.start() for m in re.finditer(r"p\.trace\[[^\]]*\] =", text)]
+    assert len(writes) == 3
+    for at in writes:
+        guard = text[text.rindex("if (", 0, at):at]
+        assert "rank == 0" in guard and "kpart == 0" in guard and "worker" in guard, guard
