@@ -22,6 +22,15 @@ def onebyone(w: DeviceArray, stride, padding, dilation, groups: int) -> bool:
             and tuple(dilation) == (1, 1) and groups == 1)
 
 
+def _biasptr(bias: Optional[DeviceArray], cout: int, what: str) -> Optional[int]:
+    """The kernels read one fp16 value per output channel, side by side."""
+    if bias is None:
+        return None
+    if bias.dtype != np.float16 or not bias.isdense() or bias.size < cout:
+        raise B200Error(19, f"{what}: Decline(:bias) for {bias.shape}:{bias.dtype} and {cout} channels")
+    return bias.ptr
+
+
 def convolution_(ctx: Ctx, out: DeviceArray, x: DeviceArray, w: DeviceArray, bias: Optional[DeviceArray],
                  stride: Sequence[int], padding: Sequence[int], dilation: Sequence[int], groups: int = 1,
                  act: str = "identity") -> DeviceArray:
@@ -45,7 +54,7 @@ def convolution_(ctx: Ctx, out: DeviceArray, x: DeviceArray, w: DeviceArray, bia
         raise B200Error(17, f"convolution!: out is {out.shape}, expected {(OW, OH, Cout, N)}")
     check(_lib.lib().b200_conv2d_grouped_f16(ctx.handle, W, H, Cin, N, KW, KH, Cout, stride[0], stride[1], padding[0],
                                              padding[1], dilation[0], dilation[1], groups, x.ptr, w.ptr,
-                                             bias.ptr if bias is not None else None, out.ptr, dtcode(out.dtype),
+                                             _biasptr(bias, Cout, "convolution!"), out.ptr, dtcode(out.dtype),
                                              _lib.EPI[act]))
     return out
 
@@ -81,5 +90,5 @@ def convolutiontranspose_(ctx: Ctx, out: DeviceArray, x: DeviceArray, w: DeviceA
         raise B200Error(17, f"convolutiontranspose!: out is {out.shape}, expected {(OW, OH, Cout, N)}")
     check(_lib.lib().b200_convtranspose2d_f16(ctx.handle, W, H, Cin, N, KW, KH, Cout, stride[0], stride[1], padding[0],
                                               padding[1], dilation[0], dilation[1], outpad[0], outpad[1], groups, x.ptr,
-                                              w.ptr, bias.ptr if bias is not None else None, out.ptr, dtcode(out.dtype)))
+                                              w.ptr, _biasptr(bias, Cout, "convolutiontranspose!"), out.ptr, dtcode(out.dtype)))
     return out

@@ -196,7 +196,7 @@ static PyObject* h_layernorm(PyObject* self, PyObject* const* v, Py_ssize_t n) {
 
 // convolution(handle, out, x, w, bias, stride, padding, dilation, groups, act)
 static PyObject* h_convolution(PyObject* self, PyObject* const* v, Py_ssize_t n) {
-    Arr out, x, w, b;
+    Arr out, x, w;
     int64_t s[2], p[2], d[2];
     b200_ctx* c;
     int act, rc, over;
@@ -208,11 +208,8 @@ static PyObject* h_convolution(PyObject* self, PyObject* const* v, Py_ssize_t n)
     }
     if (!load(v[1], &out) || !load(v[2], &x) || !load(v[3], &w) || out.nd != 4 || x.nd != 4 || w.nd != 4) Py_RETURN_NONE;
     if (x.code != B200_F16 || w.code != B200_F16 || !dense(&x) || !dense(&w) || !dense(&out)) Py_RETURN_NONE;
-    const void* bias = NULL;
-    if (v[4] != Py_None) {
-        if (!load(v[4], &b)) Py_RETURN_NONE;
-        bias = P(b);
-    }
+    const void* bias;
+    if (!vector(v[4], B200_F16, w.shape[3], &bias)) Py_RETURN_NONE;
     if (groups < 1 || w.shape[2] * groups != x.shape[2] || w.shape[3] % groups || out.shape[2] != w.shape[3] || out.shape[3] != x.shape[3])
         Py_RETURN_NONE;
     for (int i = 0; i < 2; ++i) {

@@ -154,3 +154,21 @@ def test_convolution(both):
                                   (out, arr(f16, (9, 9, 4, 1), (1, 9, 90, 400)), w, (1, 1), 1, None), (out, x, arr(f16, (3, 3, 5, 8)), (1, 1), 1, None)):
         agree(both(jv.convolution_, o, xx, ww, None, st, (0, 0), (1, 1), g, act=act))
     assert taken > 50
+
+
+def test_convolution_bias(both, monkeypatch):
+    """One fp16 value per channel, side by side: any other type, fewer of them or a stride is refused on both routes, and
+    in the transposed form; a vector of more axes, or one that goes on behind the channels, is read as it always was."""
+    f16, f32 = np.float16, np.float32
+    x, w, out = arr(f16, (9, 9, 4, 1)), arr(f16, (3, 3, 4, 8)), arr(f16, (7, 7, 8, 1))
+    args = ((1, 1), (0, 0), (1, 1))
+    for b in (arr(f32, (8,)), arr(np.uint8, (8,)), arr(f16, (7,)), arr(f16, (8,), (2,)), arr(f16, (1,))):
+        assert both(jv.convolution_, out, x, w, b, *args) == [jv.B200Error, jv.B200Error], b
+    for b in (arr(f16, (8,)), arr(f16, (1, 1, 8, 1)), arr(f16, (8,), ptr=2), arr(f16, (9,)), None):
+        assert agree(both(jv.convolution_, out, x, w, b, *args)), b
+    wt, wide = arr(f16, (3, 3, 8, 4)), arr(f16, (11, 11, 8, 1))
+    monkeypatch.setattr(_lib._lib, "b200_convtranspose2d_f16", lambda *a: 0, raising=False)
+    for b in (arr(f32, (8,)), arr(f16, (7,)), arr(f16, (8,), (2,))):
+        with pytest.raises(jv.B200Error):
+            jv.convolutiontranspose_(FakeCtx, wide, x, wt, b, *args)
+    jv.convolutiontranspose_(FakeCtx, wide, x, wt, arr(f16, (8,)), *args)
