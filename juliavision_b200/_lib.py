@@ -12,7 +12,7 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SO_PATH = os.path.join(HERE, "csrc", "libb200dnn.so")
-HOST_PATH = os.path.join(HERE, "csrc", "hostcalls.so")
+HOST_PATH = os.path.join(HERE, "csrc", "hostcalls" + importlib.machinery.EXTENSION_SUFFIXES[0])
 
 OK, EINVAL, ECUDA, ENOMEM, EKERNEL = 0, 1, 2, 3, 4
 DECLINE = {16: "operands", 17: "extent", 18: "wrapped", 19: "bias", 20: "eltype", 21: "tiling"}

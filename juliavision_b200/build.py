@@ -11,6 +11,7 @@ import os
 import subprocess
 import sys
 import sysconfig
+from importlib.machinery import EXTENSION_SUFFIXES
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -18,7 +19,7 @@ SO = os.path.join(CSRC, "libb200dnn.so")
 SOURCES = ["ctx.cu", "layernorm.cu", "gemm.cu", "attention.cu", "glue.cu", "conv.cu", "conv_implicit.cu", "gemv.cu", "gemm_rows.cu", "attention_window.cu", "attention_few.cu", "selftest.cu"]
 HEADERS = ["internal.h", "ptx.cuh", "act.cuh", os.path.join("..", "..", "include", "b200dnn.h")]
 HOST_SRC = os.path.join(CSRC, "hostcalls.c")   # the entry points' host side, a CPython extension
-HOST_SO = os.path.join(CSRC, "hostcalls.so")
+HOST_SO = os.path.join(CSRC, "hostcalls" + EXTENSION_SUFFIXES[0])   # for this interpreter: another builds its own
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -56,13 +57,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
         failed |= p.returncode != 0
     if failed:
         raise RuntimeError("nvcc failed; see output above")
-    if force or _stale(HOST_SO, [HOST_SRC, hdrs[-1]]):
-        subprocess.run(["/usr/bin/gcc", "-O2", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], "-o", HOST_SO,
-                        HOST_SRC], check=True)
     if force or procs or _stale(SO, objs):
         cmd = [NVCC, "-shared", "-o", SO, *objs, "-ccbin", "/usr/bin/g++", "-cudart", "static",
                "-gencode", "arch=compute_100a,code=sm_100a"]
         subprocess.run(cmd, check=True)
+    if force or _stale(HOST_SO, [HOST_SRC, hdrs[-1]]):
+        subprocess.run(["/usr/bin/gcc", "-O2", "-Wall", "-shared", "-fPIC", "-I", sysconfig.get_paths()["include"], "-o", HOST_SO,
+                        HOST_SRC], check=True)
     return SO
 
 
