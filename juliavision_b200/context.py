@@ -58,7 +58,6 @@ class DeviceArray:
         self.ctx = ctx
         self.ptr = int(ptr)
         self.dtype = np.dtype(dtype)
-        self.code = _DT.get(self.dtype)     # the library's code for it (F16, F32), None for any other
         self.shape = tuple(int(s) for s in shape)
         if strides is None:
             st, acc = [], 1

@@ -18,7 +18,8 @@ typedef struct {
     int nd, code;
 } Arr;
 
-static PyObject *s_ptr, *s_code, *s_shape, *s_strides;
+static PyObject *s_ptr, *s_dtype, *s_shape, *s_strides;
+static PyObject *dt_f16, *dt_f32;   // numpy's own dtype objects; an equal one that is not the same goes the Python route
 
 static int (*p_gemm)(b200_ctx*, int64_t, int64_t, int64_t, const void*, int64_t, const void*, int64_t, const void*, void*,
                      int64_t, int, int, int64_t, int64_t, int64_t, int64_t);
@@ -51,8 +52,11 @@ static int ints(PyObject* t, int64_t* out, int n) {   // a tuple of n integers
 
 // A DeviceArray of fp16 or fp32 with one to four axes; 0 for anything else.
 static int load(PyObject* o, Arr* a) {
-    int ok = 1;
-    a->code = (int)attr_int(o, s_code, &ok);
+    int ok;
+    PyObject* dt = PyObject_GetAttr(o, s_dtype);
+    a->code = dt == dt_f16 ? B200_F16 : dt == dt_f32 ? B200_F32 : -1;
+    Py_XDECREF(dt);   // numpy holds the two that count
+    ok = a->code >= 0;
     a->ptr = ok ? attr_int(o, s_ptr, &ok) : 0;
     if (ok) {
         PyObject *sh = PyObject_GetAttr(o, s_shape), *st = PyObject_GetAttr(o, s_strides);
@@ -65,7 +69,7 @@ static int load(PyObject* o, Arr* a) {
         PyErr_Clear();
         ok = 0;
     }
-    return ok && (a->code == B200_F16 || a->code == B200_F32);
+    return ok;
 }
 
 static int dense(const Arr* a) {
@@ -243,9 +247,15 @@ static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "hostcalls", NULL, -1
 
 PyMODINIT_FUNC PyInit_hostcalls(void) {
     s_ptr = PyUnicode_InternFromString("ptr");
-    s_code = PyUnicode_InternFromString("code");
+    s_dtype = PyUnicode_InternFromString("dtype");
     s_shape = PyUnicode_InternFromString("shape");
     s_strides = PyUnicode_InternFromString("strides");
-    if (!s_ptr || !s_code || !s_shape || !s_strides) return NULL;
+    if (!s_ptr || !s_dtype || !s_shape || !s_strides) return NULL;
+    PyObject* np = PyImport_ImportModule("numpy");
+    if (!np) return NULL;
+    dt_f16 = PyObject_CallMethod(np, "dtype", "s", "float16");
+    dt_f32 = PyObject_CallMethod(np, "dtype", "s", "float32");
+    Py_DECREF(np);
+    if (!dt_f16 || !dt_f32) return NULL;
     return PyModule_Create(&module);
 }

@@ -172,3 +172,17 @@ def test_convolution_bias(both, monkeypatch):
         with pytest.raises(jv.B200Error):
             jv.convolutiontranspose_(FakeCtx, wide, x, wt, b, *args)
     jv.convolutiontranspose_(FakeCtx, wide, x, wt, arr(f16, (8,)), *args)
+
+
+def test_an_array_has_one_element_type(both):
+    """The native route reads the dtype the array shows, as the Python route does: also after it was assigned."""
+    f16, f32 = np.float16, np.float32
+    A, B, out = arr(f32, (8, 4)), arr(f32, (4, 3)), arr(f16, (8, 3))
+    assert not agree(both(jv.matmul_, out, A, B, None))                # fp32 products of several tokens are declined
+    A.dtype = B.dtype = np.dtype(f16)
+    assert agree(both(jv.matmul_, out, A, B, None))
+    out.dtype = np.dtype(f32)
+    assert agree(both(jv.matmul_, out, A, B, None))
+    for d in (">f2", "i2", "f8"):
+        A.dtype = np.dtype(d)
+        assert not agree(both(jv.matmul_, out, A, B, None)), d
