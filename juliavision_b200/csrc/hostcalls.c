@@ -14,7 +14,7 @@
 #include "../../include/b200dnn.h"
 
 typedef struct {
-    int64_t ptr, shape[4], stride[4];
+    int64_t ptr, shape[4], stride[4], size;
     int nd, code;
 } Arr;
 
@@ -50,7 +50,7 @@ static int ints(PyObject* t, int64_t* out, int n) {   // a tuple of n integers
     return !PyErr_Occurred();
 }
 
-// A DeviceArray of fp16 or fp32 with one to four axes; 0 for anything else.
+// A DeviceArray of fp16 or fp32 with one to four axes and a size that is a number here; 0 for anything else.
 static int load(PyObject* o, Arr* a) {
     int ok;
     PyObject* dt = PyObject_GetAttr(o, s_dtype);
@@ -62,6 +62,8 @@ static int load(PyObject* o, Arr* a) {
         PyObject *sh = PyObject_GetAttr(o, s_shape), *st = PyObject_GetAttr(o, s_strides);
         a->nd = sh && PyTuple_Check(sh) ? (int)PyTuple_GET_SIZE(sh) : 0;
         ok = a->nd >= 1 && a->nd <= 4 && ints(sh, a->shape, a->nd) && ints(st, a->stride, a->nd);
+        a->size = 1;
+        for (int i = 0; ok && i < a->nd; ++i) ok = a->shape[i] >= 0 && !__builtin_mul_overflow(a->size, a->shape[i], &a->size);
         Py_XDECREF(sh);
         Py_XDECREF(st);
     }
@@ -80,11 +82,6 @@ static int dense(const Arr* a) {
     }
     return 1;
 }
-static int64_t size(const Arr* a) {
-    int64_t n = 1;
-    for (int i = 0; i < a->nd; ++i) n *= a->shape[i];
-    return n;
-}
 static int64_t colmajor(const Arr* a) {   // leading dimension of a 2-D view with a unit first stride, else -1
     if (a->shape[0] != 1 && a->stride[0] != 1) return -1;
     const int64_t ld = a->shape[1] != 1 ? a->stride[1] : (a->shape[0] > 1 ? a->shape[0] : 1);
@@ -95,7 +92,7 @@ static int vector(PyObject* o, int code, int64_t n, const void** p) {
     Arr a;
     *p = NULL;
     if (o == Py_None) return 1;
-    if (!load(o, &a) || a.code != code || size(&a) != n || !dense(&a)) return 0;
+    if (!load(o, &a) || a.code != code || a.size != n || !dense(&a)) return 0;
     *p = (const void*)a.ptr;
     return 1;
 }
@@ -188,10 +185,10 @@ static PyObject* h_layernorm(PyObject* self, PyObject* const* v, Py_ssize_t n) {
     if (n != 9 || !(c = handle(v[0])) || !PyLong_Check(v[7]) || !PyFloat_Check(v[8])) Py_RETURN_NONE;
     if (!load(v[1], &out) || !load(v[2], &mean) || !load(v[3], &rstd) || !load(v[4], &a)) Py_RETURN_NONE;
     int over;
-    const int64_t C = PyLong_AsLongLongAndOverflow(v[7], &over), total = size(&a);
-    if (over || C < 1 || total % C || size(&out) != total || !dense(&a) || !dense(&out) || !dense(&mean) || !dense(&rstd)) Py_RETURN_NONE;
+    const int64_t C = PyLong_AsLongLongAndOverflow(v[7], &over), total = a.size;
+    if (over || C < 1 || total % C || out.size != total || !dense(&a) || !dense(&out) || !dense(&mean) || !dense(&rstd)) Py_RETURN_NONE;
     const int64_t groups = total / C;
-    if (mean.code != B200_F32 || rstd.code != B200_F32 || size(&mean) < groups || size(&rstd) < groups) Py_RETURN_NONE;
+    if (mean.code != B200_F32 || rstd.code != B200_F32 || mean.size < groups || rstd.size < groups) Py_RETURN_NONE;
     if (!vector(v[5], a.code, C, &gamma) || !vector(v[6], a.code, C, &beta)) Py_RETURN_NONE;
     const float eps = (float)PyFloat_AS_DOUBLE(v[8]);
     ENTER(rc, p_layernorm(c, groups, C, P(a), a.code, P(out), out.code, (float*)P(mean), (float*)P(rstd), gamma, beta, eps));
@@ -216,7 +213,9 @@ static PyObject* h_convolution(PyObject* self, PyObject* const* v, Py_ssize_t n)
     if (!vector(v[4], B200_F16, w.shape[3], &bias)) Py_RETURN_NONE;
     if (groups < 1 || w.shape[2] * groups != x.shape[2] || w.shape[3] % groups || out.shape[2] != w.shape[3] || out.shape[3] != x.shape[3])
         Py_RETURN_NONE;
+    const int64_t lim = (int64_t)1 << 31;   // past it (no extent of a real convolution) the sums below could wrap
     for (int i = 0; i < 2; ++i) {
+        if (x.shape[i] >= lim || w.shape[i] >= lim || s[i] >= lim || p[i] >= lim || d[i] >= lim) Py_RETURN_NONE;
         const int64_t span = x.shape[i] + 2 * p[i] - d[i] * (w.shape[i] - 1) - 1;
         if (s[i] < 1 || d[i] < 1 || p[i] < 0 || span < 0 || out.shape[i] != span / s[i] + 1) Py_RETURN_NONE;
     }

@@ -186,3 +186,14 @@ def test_an_array_has_one_element_type(both):
     for d in (">f2", "i2", "f8"):
         A.dtype = np.dtype(d)
         assert not agree(both(jv.matmul_, out, A, B, None)), d
+
+
+def test_numbers_that_wrap_in_64_bits_go_the_python_route(both):
+    """Python's integers do not wrap: what it refuses for its size must not be read as a small number."""
+    f16, f32, big = np.float16, np.float32, 1 << 32
+    a, m = arr(f16, (big, big)), arr(f32, (4,))
+    assert both(jv.layernorm_, arr(f16, (big, big)), m, m, a, None, None, 1, 1e-5) == [jv.B200Error] * 2     # 2^64 elements
+    x, w = arr(f16, (9, 9, 4, 1)), arr(f16, (3, 3, 4, 8))
+    for out, p, d in ((arr(f16, (5, 5, 8, 1)), (1 << 63) - 1, 1), (arr(f16, (7, 7, 8, 1)), 0, (1 << 63) + 1), (arr(f16, (5, 5, 8, 1)), 1, (1 << 62) + 2)):
+        assert not agree(both(jv.convolution_, out, x, w, None, (1, 1), (p, p), (d, d))), (p, d)
+    assert agree(both(jv.convolution_, arr(f16, (7, 7, 8, 1)), x, w, None, (1, 1), (0, 0), (1, 1)))
