@@ -803,35 +803,42 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
     return best;
 }
 
-// How many clusters of 2, 4 and 8 single-CTA tiles are resident at once: asked of the runtime once per device.
-static KsplitRoom ksplit_room(b200_ctx* ctx) {
-    static KsplitRoom room[16] = {};
-    KsplitRoom& r = room[ctx->device & 15];
-    if (r.clusters[0]) return r;
+// How many clusters of 2, 4 and 8 single-CTA tiles are resident at once: asked of the runtime once per device, about the
+// context's device whichever is current (the plan entry comes here without a launch), by one thread while others wait.
+static KsplitRoom ksplit_ask(b200_ctx* ctx) {
     using Cfg = GemmCfg<64, __half, 1>;
     auto kern = gemm_f16_tc_kernel<64, __half, 1, true>;
     KsplitRoom got = {{ctx->prop.multiProcessorCount, 0, 0, 0}};
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) == cudaSuccess)
-        for (int l = 1; l <= 3; ++l) {
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = 1u << l;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cudaLaunchConfig_t cfg = {};
-            cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
-            cfg.gridDim = dim3((unsigned)((ctx->prop.multiProcessorCount >> l) << l), 1, 1);
-            cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-            cfg.stream = ctx->stream;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess) got.clusters[l] = n;
-            else cudaGetLastError();
-        }
-    else
+    if (cudaSetDevice(ctx->device) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess) {
         cudaGetLastError();
-    return r = got;
+        return got;
+    }
+    for (int l = 1; l <= 3; ++l) {
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1u << l;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
+        cfg.gridDim = dim3((unsigned)((ctx->prop.multiProcessorCount >> l) << l), 1, 1);
+        cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+        cfg.stream = ctx->stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess) got.clusters[l] = n;
+        else cudaGetLastError();
+    }
+    return got;
+}
+static const KsplitRoom& ksplit_room(b200_ctx* ctx) {
+    static std::once_flag once[16];
+    static KsplitRoom room[16];
+    const int d = ctx->device & 15;
+    std::call_once(once[d], [&] { room[d] = ksplit_ask(ctx); });
+    return room[d];
 }
 
 template <int BN, typename OutT, int NCTA, bool KSPLIT = false>

@@ -223,6 +223,29 @@ def test_tiles_shared_by_a_cluster(ctx, ora, tile, tokens, out, K, monkeypatch):
     assert relerr(two.to_host(), np.stack([zero, -2 * zero])) < 2e-5
 
 
+def test_plans_made_by_several_threads_agree(ctx):
+    """The plan entry asks the runtime once per device and keeps the answer for every thread."""
+    import ctypes as C
+    import threading
+    from juliavision_b200 import _lib
+    shapes = [(768, 160, 3072), (2112, 42, 3152), (304, 18, 2144), (3072, 4096, 768)]
+    def plans(c):
+        out = []
+        for M, N, K in shapes:
+            p = _lib.GemmPlan()
+            _lib.check(_lib.lib().b200_gemm_f16_plan(c.handle, M, N, K, 1, C.byref(p)))
+            out.append((p.block_m, p.block_n, p.ctas))
+        return out
+    want, got = plans(ctx), []
+    ts = [threading.Thread(target=lambda: got.append(plans(ctx))) for _ in range(8)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert got == [want] * 8
+    assert any(p[2] > -(-M // p[1]) * -(-N // p[0]) for p, (M, N, K) in zip(want, shapes)), "no shape splits K here"
+
+
 def test_streamk_is_deterministic(ctx, monkeypatch):
     monkeypatch.setenv("B200_GEMM_TILE", "256x2s")
     rng = np.random.default_rng(77)

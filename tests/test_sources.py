@@ -32,3 +32,13 @@ def test_one_cta_of_a_worker_writes_the_timeline():
     for at in writes:
         guard = text[text.rindex("if (", 0, at):at]
         assert "rank == 0" in guard and "kpart == 0" in guard and "worker" in guard, guard
+
+
+def test_what_the_runtime_is_asked_once_is_asked_of_the_right_device_by_one_thread():
+    """The K split's room is kept per device and asked for by the plan entry too, with any device current and from any
+    thread: the device is set before the question, and the answer is published whole."""
+    text = dict(sources())["gemm.cu"]
+    ask = text[text.index("static KsplitRoom ksplit_ask("):]
+    assert 0 < ask.index("cudaSetDevice(ctx->device)") < ask.index("cudaFuncSetAttribute(") < ask.index("cudaOccupancyMaxActiveClusters(")
+    room = text[text.index("ksplit_room(b200_ctx* ctx) {"):]
+    assert "std::call_once(" in room[:room.index("\n}\n")]
