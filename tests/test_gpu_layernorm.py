@@ -3,6 +3,8 @@ import os
 import numpy as np
 import pytest
 
+import juliavision_b200 as jv
+
 from .conftest import relerr
 from .gpu_helpers import describe, layernorm_gpu
 
@@ -83,3 +85,50 @@ def test_empty_and_errors(ctx):
     b = ctx.allocate(np.float16, 10, 3)
     with pytest.raises(jv.B200Error):
         jv.layernorm_(ctx, b, m, m, b, None, None, 7, 1e-5)  # 30 is not a multiple of 7
+
+
+PACKED = [1000, 1024, 1176, 1480, 1800, 2048]    # 4, 4, 5, 6 and 8 vectors per lane, the last one ragged or full
+
+
+def _packed_rows(C):
+    """Rows just past the 48 Mi elements from which fp16 launches take the packed form, the last block of four ragged."""
+    groups = ((48 << 20) + C - 1) // C + 1
+    return groups + (groups % 4 == 0)
+
+
+@pytest.mark.parametrize("C", PACKED)
+def test_rows_the_cache_does_not_hold(ctx, ora, C):
+    """The packed form: first and last rows and a sample in between, with gamma and beta, one of them and neither."""
+    groups = _packed_rows(C)
+    rng = np.random.default_rng(C)
+    a = np.float16(rng.standard_normal((groups, C), dtype=np.float32) * 2 + 0.5)
+    gam, bet = (np.float16(o + 0.1 * rng.standard_normal(C)) for o in (1, 0))
+    rows = np.unique(np.concatenate([np.arange(9), groups - 1 - np.arange(9), rng.integers(0, groups, 400)]))
+    for g, b in ((gam, bet), (gam, None), (None, bet), (None, None)):
+        got, mean, rstd = layernorm_gpu(ctx, a, g, b, 1e-5)
+        ref, rmean, rrstd = ora.layernorm(a[rows], g, b, 1e-5)
+        assert np.all(np.isfinite(got)) and np.all(np.isfinite(mean)) and np.all(np.isfinite(rstd))
+        assert relerr(got[rows], ref) < 1.5e-3, describe(got[rows], ref, 1.5e-3)    # as above: at most one output ulp
+        assert np.max(np.abs(mean[rows] - rmean)) < 1e-5 and relerr(rstd[rows], rrstd) < 1e-5
+
+
+@pytest.mark.parametrize("C", [1000, 1176, 1480, 1800])
+def test_add_layernorm_equals_the_three_ops_where_the_cache_does_not_hold_them(ctx, C):
+    """The promise of equal bits at the size where both take the packed form, and one row short of it, where neither does."""
+    rng = np.random.default_rng(C)
+    least = ((48 << 20) + C - 1) // C
+    g, b = (ctx.toback(np.float16(o + 0.1 * rng.standard_normal(C))) for o in (1, 0))
+    for groups, clamp, gb in ((_packed_rows(C), (-500.0, 500.0), (g, b)), (least, None, (g, None)), (least - 1, None, (g, b))):
+        x0, h0 = (np.float16(rng.standard_normal((groups, C), dtype=np.float32) * 300) for _ in range(2))
+        mean, rstd, m2, r2 = (ctx.allocate(np.float32, groups) for _ in range(4))
+        xa, ha, oa = ctx.toback(x0), ctx.toback(h0), ctx.allocate(np.float16, C, groups)
+        jv.add_(ctx, xa, xa, ha)
+        if clamp:
+            jv.clamp_(ctx, xa, xa, *clamp)
+        jv.layernorm_(ctx, oa, mean, rstd, xa, *gb, C, 1e-5)
+        xb, ob = ctx.toback(x0), ctx.allocate(np.float16, C, groups)
+        ctx.fill_bytes(ob, 0xFF)
+        jv.add_layernorm_(ctx, ob, m2, r2, xb, ha, *gb, C, 1e-5, clamp=clamp)
+        ctx.synchronize()
+        for one, other in ((xa, xb), (oa, ob), (mean, m2), (rstd, r2)):
+            assert np.array_equal(one.to_host(), other.to_host()), (groups, C)
