@@ -26,7 +26,7 @@ constexpr int AF_PARTS = 16; // CTAs of a cluster at most
 
 // KS: key slots, i.e. how many of the four warps share a tile of 16 queries (4 / KS tiles per CTA, one or two).
 template <int EP, int KS> struct AfCfg {
-    static_assert(KS == 2 || KS == 4, "two or one query tiles");
+    static_assert(KS == 4 || (KS == 2 && EP == 64), "one query tile, or two of them at E <= 64");
     static constexpr int QT = 4 / KS, QR = 16 * QT;           // query tiles and rows of a CTA
     static constexpr int PITCH = EP + 8;                      // halves per shared row: an odd number of 16-byte units
     static constexpr int STAGES = EP == 64 ? 4 : 3;
@@ -373,8 +373,9 @@ static int af_bias(b200_ctx* ctx, const FewParams& p, int64_t H, int64_t B, int 
 }
 template <int EP>
 static int af_slots(b200_ctx* ctx, const FewParams& p, int64_t H, int64_t B, int parts) {
-    if (p.Lq <= 16) return af_bias<EP, 4>(ctx, p, H, B, parts);
-    return af_bias<EP, 2>(ctx, p, H, B, parts);
+    if constexpr (EP == 64)   // wider heads come here with up to 16 queries
+        if (p.Lq > 16) return af_bias<EP, 2>(ctx, p, H, B, parts);
+    return af_bias<EP, 4>(ctx, p, H, B, parts);
 }
 
 int attention_few_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B, const b200_strided4* q,

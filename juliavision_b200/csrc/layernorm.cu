@@ -149,6 +149,7 @@ ln_warp_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
                const InT* __restrict__ beta, int64_t groups, int C, float eps) {
     constexpr int VN = Vec16<InT>::N;
     static_assert(LPG == 32 || VPL == 1, "only single-vector groups share a warp");
+    static_assert(!(PACK && LAT), "the packed form is for launches of many waves");
     const int lane = threadIdx.x & (LPG - 1);
     const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / LPG;
     const int nvec = g < groups ? C / VN : 0;   // lanes past the last group idle through the shuffles
@@ -192,13 +193,8 @@ ln_warp_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
             const int v = lane + 32 * i;
             if (v < nvec) {
                 uint4 gv = make_uint4(0u, 0u, 0u, 0u), bv = gv;
-                if constexpr (HOIST) {
-                    gv = gw[i];
-                    bv = bw[i];
-                } else {
-                    if (gamma) gv = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
-                    if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + v);
-                }
+                if (gamma) gv = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
+                if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + v);
                 ln_write<InT, OutT>(dst + (int64_t)v * VN, x[i], r, gamma != nullptr, gv, beta != nullptr, bv);
             }
         }
@@ -280,6 +276,7 @@ ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half*
                    float hi) {
     constexpr int VN = 8;
     static_assert(LPG == 32 || VPL == 1, "only single-vector groups share a warp");
+    static_assert(!(PACK && LAT), "the packed form is for launches of many waves");
     const int lane = threadIdx.x & (LPG - 1);
     const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / LPG;
     const int nvec = g < groups ? C / VN : 0;
@@ -323,13 +320,8 @@ ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half*
             const int vi = lane + 32 * i;
             if (vi < nvec) {
                 Vec16<__half> a, b;
-                if constexpr (HOIST) {
-                    a.raw = xraw[i];
-                    b.raw = hraw[i];
-                } else {
-                    a.raw = *(reinterpret_cast<const uint4*>(xr) + vi);
-                    b.raw = __ldg(reinterpret_cast<const uint4*>(hr) + vi);
-                }
+                a.raw = *(reinterpret_cast<const uint4*>(xr) + vi);
+                b.raw = __ldg(reinterpret_cast<const uint4*>(hr) + vi);
                 float fa[VN], fb[VN];
                 a.to_f32(fa);
                 b.to_f32(fb);
@@ -351,13 +343,8 @@ ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half*
             const int vi = lane + 32 * i;
             if (vi < nvec) {
                 uint4 gv = make_uint4(0u, 0u, 0u, 0u), bv = gv;
-                if constexpr (HOIST) {
-                    gv = gw[i];
-                    bv = bw[i];
-                } else {
-                    if (gamma) gv = __ldg(reinterpret_cast<const uint4*>(gamma) + vi);
-                    if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + vi);
-                }
+                if (gamma) gv = __ldg(reinterpret_cast<const uint4*>(gamma) + vi);
+                if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + vi);
                 ln_write<__half, __half>(dst + (int64_t)vi * VN, v[i], r, gamma != nullptr, gv, beta != nullptr, bv);
             }
         }
