@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 
 #include "../../include/b200dnn.h"
+#include "ptx.cuh"
 
 namespace b200 {
 
@@ -32,59 +33,33 @@ __device__ __forceinline__ float gelu_exact(float x) {
 
 // The same function on a pair, with the multiplies and FMAs as packed fp32-pair instructions (sm_100): half
 // the instructions per element in the GEMM store, where the activation is what a short-K tile waits for.
-namespace act_detail {
-__device__ __forceinline__ unsigned long long pk(float lo, float hi) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void upk(unsigned long long v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned long long dup(float c) { return pk(c, c); }
-} // namespace act_detail
+__device__ __forceinline__ uint64_t dup2(float c) { return pack2(c, c); }
 
 __device__ __forceinline__ float2 gelu_exact2(float2 x) {
-    using namespace act_detail;
-    const unsigned long long x2 = pk(x.x, x.y);
+    const uint64_t x2 = pack2(x.x, x.y);
     float z0, z1;
-    upk(mul2(x2, dup(0.70710678118654752f)), z0, z1);
+    unpack2(mul2(x2, dup2(0.70710678118654752f)), z0, z1);
     const float a0 = fabsf(z0), a1 = fabsf(z1);
-    const unsigned long long a2 = pk(a0, a1);
+    const uint64_t a2 = pack2(a0, a1);
     float d0, d1, t0, t1, u0, u1, e0, e1;
-    upk(fma2(dup(0.3275911f), a2, dup(1.0f)), d0, d1);
+    unpack2(fma2(dup2(0.3275911f), a2, dup2(1.0f)), d0, d1);
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t0) : "f"(d0));
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t1) : "f"(d1));
-    upk(mul2(mul2(a2, a2), dup(-1.4426950408889634f)), u0, u1);
+    unpack2(mul2(mul2(a2, a2), dup2(-1.4426950408889634f)), u0, u1);
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(u0));
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(u1));
-    const unsigned long long t2 = pk(t0, t1);
-    unsigned long long poly = fma2(dup(1.061405429f), t2, dup(-1.453152027f));
-    poly = fma2(poly, t2, dup(1.421413741f));
-    poly = fma2(poly, t2, dup(-0.284496736f));
-    poly = fma2(poly, t2, dup(0.254829592f));
+    const uint64_t t2 = pack2(t0, t1);
+    uint64_t poly = fma2(dup2(1.061405429f), t2, dup2(-1.453152027f));
+    poly = fma2(poly, t2, dup2(1.421413741f));
+    poly = fma2(poly, t2, dup2(-0.284496736f));
+    poly = fma2(poly, t2, dup2(0.254829592f));
     poly = mul2(poly, t2);
     float p0, p1, y0, y1;
-    upk(poly, p0, p1);
-    upk(fma2(pk(-p0, -p1), pk(e0, e1), dup(1.0f)), y0, y1);
-    const unsigned long long hx = mul2(dup(0.5f), x2);
+    unpack2(poly, p0, p1);
+    unpack2(fma2(pack2(-p0, -p1), pack2(e0, e1), dup2(1.0f)), y0, y1);
+    const uint64_t hx = mul2(dup2(0.5f), x2);
     float r0, r1;
-    upk(fma2(hx, pk(copysignf(y0, z0), copysignf(y1, z1)), hx), r0, r1);
+    unpack2(fma2(hx, pack2(copysignf(y0, z0), copysignf(y1, z1)), hx), r0, r1);
     return make_float2(r0, r1);
 }
 __device__ __forceinline__ float apply_act(int epi, float v) {

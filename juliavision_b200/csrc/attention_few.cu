@@ -51,11 +51,6 @@ struct FewParams {
     float scale_log2;
 };
 
-__device__ __forceinline__ void af_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 template <bool TRANS> __device__ __forceinline__ void af_ldmatrix(uint32_t (&r)[4], const __half* row) {
     const uint32_t addr = smem_u32(row);
     if constexpr (TRANS)
@@ -68,16 +63,6 @@ template <bool TRANS> __device__ __forceinline__ void af_ldmatrix(uint32_t (&r)[
 // 16 bytes to shared memory, zeros when `live` is false (the address is then not read)
 __device__ __forceinline__ void af_copy16(const __half* dst, const __half* src, bool live) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ float2 af_ld_cluster2(uint32_t addr) {
-    float2 v;
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
-    return v;
-}
-__device__ __forceinline__ float4 af_ld_cluster4(uint32_t addr) {
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-    return v;
 }
 __device__ __forceinline__ uint32_t af_pack(float lo, float hi) {
     const __half2 h = __floats2half2_rn(lo, hi);
@@ -169,8 +154,8 @@ attention_few_kernel(const FewParams p) {
             for (int ks = 0; ks < EP / 16; ++ks) {
                 uint32_t kb[4];
                 af_ldmatrix<false>(kb, Ks + ((n + (lane >> 4)) * 8 + (lane & 7)) * PITCH + ks * 16 + ((lane >> 3) & 1) * 8);
-                af_mma(s[n], qa[ks], kb[0], kb[1]);
-                af_mma(s[n + 1], qa[ks], kb[2], kb[3]);
+                mma_16816(s[n], qa[ks], kb[0], kb[1]);
+                mma_16816(s[n + 1], qa[ks], kb[2], kb[3]);
             }
         float x0 = -INFINITY, x1 = -INFINITY;
 #pragma unroll
@@ -219,8 +204,8 @@ attention_few_kernel(const FewParams p) {
             for (int n = 0; n < EP / 8; n += 2) {
                 uint32_t vb[4];
                 af_ldmatrix<true>(vb, Vs + (kk * 16 + (lane & 15)) * PITCH + (n + (lane >> 4)) * 8);
-                af_mma(o[n], pa[kk], vb[0], vb[1]);
-                af_mma(o[n + 1], pa[kk], vb[2], vb[3]);
+                mma_16816(o[n], pa[kk], vb[0], vb[1]);
+                mma_16816(o[n + 1], pa[kk], vb[2], vb[3]);
             }
     }
 #pragma unroll
@@ -274,7 +259,7 @@ attention_few_kernel(const FewParams p) {
 #pragma unroll
             for (int r = 0; r < RB; ++r) {
                 const uint32_t at = base + (row0 + r < p.Lq ? row0 + r : row0) * (ROW * 4) + EP * 4;
-                const float2 ml = lane < parts ? af_ld_cluster2(mapa_u32(at, (uint32_t)lane)) : make_float2(-INFINITY, 0.f);
+                const float2 ml = lane < parts ? ld_cluster_f32x2(mapa_u32(at, (uint32_t)lane)) : make_float2(-INFINITY, 0.f);
                 w[r] = ml.x;
                 inv[r] = ml.y;
                 acc[r] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -298,7 +283,7 @@ attention_few_kernel(const FewParams p) {
                     const uint32_t src = mapa_u32(base + lane * 16, (uint32_t)(in ? q0 + u : 0));
 #pragma unroll
                     for (int r = 0; r < RB; ++r)
-                        v[r][u] = in ? af_ld_cluster4(src + (row0 + r < p.Lq ? row0 + r : row0) * (ROW * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        v[r][u] = in ? ld_cluster_f32x4(src + (row0 + r < p.Lq ? row0 + r : row0) * (ROW * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
                 for (int u = 0; u < PB; ++u)

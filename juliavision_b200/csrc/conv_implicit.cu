@@ -78,11 +78,6 @@ __device__ __forceinline__ uint32_t ldg_u16_if(const uint16_t* p, bool in) {
         : "l"(p), "r"((uint32_t)in));
     return v;
 }
-__device__ __forceinline__ float ci_ld_cluster(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-    return v;
-}
 
 // grid (K parts, pixel tiles of all images, channel tiles); the K parts of a tile form a cluster.
 template <int BN, typename OutT>
@@ -288,7 +283,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
                 for (int q = 0; q < 8; ++q) {
                     const uint32_t src = mapa_u32(mine + c * (CI_PIX * 4), q < parts ? q : 0);
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) v[u][q] = q < parts ? ci_ld_cluster(src + u * (2 * CI_PIX * 4)) : 0.f;
+                    for (int u = 0; u < 4; ++u) v[u][q] = q < parts ? ld_cluster_f32(src + u * (2 * CI_PIX * 4)) : 0.f;
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {

@@ -175,12 +175,6 @@ __device__ __forceinline__ void st_release_gpu(int* p, int v) {
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-
 // KSPLIT: a cluster of p.ksplit CTAs (NCTA = 1) takes one tile, each a contiguous part of its k-blocks.  The fp32
 // accumulators are laid over the drained operand ring and every CTA finishes its share of the tile's chunks from all
 // of them, read through distributed shared memory and added in rank order: no workspace, no flags, and a hand-off of
@@ -510,7 +504,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
                         const uint32_t src = mapa_u32(dump + (uint32_t)(col0 / 4) * (GEMM_BM * 16), k);
 #pragma unroll
                         for (int q = 0; q < CH / 4; ++q) {
-                            const float4 f = ld_cluster_f4(src + q * (GEMM_BM * 16));
+                            const float4 f = ld_cluster_f32x4(src + q * (GEMM_BM * 16));
                             v[4 * q] += f.x;
                             v[4 * q + 1] += f.y;
                             v[4 * q + 2] += f.z;

@@ -52,22 +52,6 @@ struct GrParams {
     int steps_per_cta;   // steps of GR_STEP columns each CTA of a cluster takes
 };
 
-__device__ __forceinline__ void gr_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-    return v;
-}
-__device__ __forceinline__ uint32_t cluster_nctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
-
 // grid (K parts, row blocks, token blocks), the K parts of a row block forming a cluster; 256 threads.
 template <int NT, typename OutT>
 __global__ void __launch_bounds__(32 * GR_WARPS, GrCfg<NT>::MIN_BLOCKS)
@@ -164,7 +148,7 @@ gemm_rows_kernel(const GrParams p) {
                         const uint32_t a0 = __byte_perm(w0[q], w1[q], 0x5410), a1 = __byte_perm(w0[q], w1[q], 0x7632);
                         const uint32_t a2 = __byte_perm(w2[q], w3[q], 0x5410), a3 = __byte_perm(w2[q], w3[q], 0x7632);
 #pragma unroll
-                        for (int u = 0; u < (NT < 4 ? NT : 4); ++u) gr_mma(acc[mi][q][nt0 + u], a0, a1, a2, a3, b[u].x, b[u].y);
+                        for (int u = 0; u < (NT < 4 ? NT : 4); ++u) mma_16816(acc[mi][q][nt0 + u], a0, a1, a2, a3, b[u].x, b[u].y);
                     }
                 }
             }

@@ -32,12 +32,6 @@ constexpr int GEMV_BLOCKS_PER_SM = 2;   // resident blocks of 512 threads at 64 
 constexpr int GEMV_SPLIT_MIN_K = 4096;  // (gemv_run)
 constexpr int GEMV_MIN_COLS = 8;        // columns per warp below which a further K split only adds the join
 
-__device__ __forceinline__ float gemv_ld_cluster(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-    return v;
-}
-
 // Pairwise sum.  With results kept in fp32 the columns of a warp are added two at a time as well: as one chain over them
 // and one over the warps, those results were up to 17 % further from 64 bits than with the fewer columns that a warp of
 // gemv_split_kernel takes (10428 x 429: 1.24e-7 against 1.06e-7).  Rounded to fp16 none of this shows, and there the
@@ -143,7 +137,7 @@ gemv_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const
     for (int r = tid * parts + rank; r < ROWS; r += 32 * GEMV_WARPS * parts) {
         float v[8];   // every part's load in flight together: a remote load takes a few hundred nanoseconds
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = q < parts ? gemv_ld_cluster(mapa_u32(mine + r * 4, (uint32_t)q)) : 0.f;
+        for (int q = 0; q < 8; ++q) v[q] = q < parts ? ld_cluster_f32(mapa_u32(mine + r * 4, (uint32_t)q)) : 0.f;
         finish(r, gemv_pairs(v));
     }
     cluster_sync_all();   // nobody leaves while its sums may still be read

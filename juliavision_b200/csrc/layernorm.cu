@@ -7,7 +7,6 @@
 // group, shared-memory tree reductions and three strided passes over the group.
 #include <cuda_fp16.h>
 
-#include "act.cuh"
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -81,16 +80,15 @@ __device__ __forceinline__ float group_sum(float v) {
 // in the scalar form (14736 x 1176: 11.7 us, packed 12.9), so the row bytes decide, the same for the layer norm alone
 // and the one behind a residual add, which therefore give the same bits.  The vectors of a lane are v = first,
 // first + 32, ...; `x` is left holding x - mean.
-__device__ __forceinline__ float pairs_sum(unsigned long long s2) {
+__device__ __forceinline__ float pairs_sum(uint64_t s2) {
     float a, b;
-    act_detail::upk(s2, a, b);
+    unpack2(s2, a, b);
     return a + b;
 }
 template <int VPL, int VN, int LPG>
-__device__ __forceinline__ void ln_moments(unsigned long long (&x)[VPL][VN / 2], int first, int nvec, int C, float eps, float& mu,
+__device__ __forceinline__ void ln_moments(uint64_t (&x)[VPL][VN / 2], int first, int nvec, int C, float eps, float& mu,
                                            float& r) {
-    using namespace act_detail;
-    unsigned long long s = pk(0.f, 0.f);
+    uint64_t s = pack2(0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < VPL; ++i)
         if (first + 32 * i < nvec) {
@@ -99,8 +97,8 @@ __device__ __forceinline__ void ln_moments(unsigned long long (&x)[VPL][VN / 2],
         }
     const float n = (float)C;
     mu = group_sum<LPG>(pairs_sum(s)) / n;
-    const unsigned long long nmu = pk(-mu, -mu);
-    unsigned long long s2 = pk(0.f, 0.f);
+    const uint64_t nmu = pack2(-mu, -mu);
+    uint64_t s2 = pack2(0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < VPL; ++i)
         if (first + 32 * i < nvec) {
@@ -114,9 +112,8 @@ __device__ __forceinline__ void ln_moments(unsigned long long (&x)[VPL][VN / 2],
 }
 // One vector of the result: d = x - mean; y = d r, then gamma and beta in one rounding where both are there.
 template <typename InT, typename OutT>
-__device__ __forceinline__ void ln_write(OutT* dst, const unsigned long long* d, float r, bool has_g, const uint4& g, bool has_b,
+__device__ __forceinline__ void ln_write(OutT* dst, const uint64_t* d, float r, bool has_g, const uint4& g, bool has_b,
                                          const uint4& b) {
-    using namespace act_detail;
     constexpr int VN = Vec16<InT>::N;
     Vec16<InT> tg, tb;
     float gf[VN], bf[VN], y[VN];
@@ -124,14 +121,14 @@ __device__ __forceinline__ void ln_write(OutT* dst, const unsigned long long* d,
     tb.raw = b;
     if (has_g) tg.to_f32(gf);
     if (has_b) tb.to_f32(bf);
-    const unsigned long long rr = pk(r, r);
+    const uint64_t rr = pack2(r, r);
 #pragma unroll
     for (int j = 0; j < VN / 2; ++j) {
-        unsigned long long v = mul2(d[j], rr);
-        if (has_g && has_b) v = fma2(v, pk(gf[2 * j], gf[2 * j + 1]), pk(bf[2 * j], bf[2 * j + 1]));
-        else if (has_g) v = mul2(v, pk(gf[2 * j], gf[2 * j + 1]));
-        else if (has_b) v = add2(v, pk(bf[2 * j], bf[2 * j + 1]));
-        upk(v, y[2 * j], y[2 * j + 1]);
+        uint64_t v = mul2(d[j], rr);
+        if (has_g && has_b) v = fma2(v, pack2(gf[2 * j], gf[2 * j + 1]), pack2(bf[2 * j], bf[2 * j + 1]));
+        else if (has_g) v = mul2(v, pack2(gf[2 * j], gf[2 * j + 1]));
+        else if (has_b) v = add2(v, pack2(bf[2 * j], bf[2 * j + 1]));
+        unpack2(v, y[2 * j], y[2 * j + 1]);
     }
     store_vec<VN>(dst, y);
 }
@@ -173,7 +170,7 @@ ln_warp_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
 
     float mu, r;
     if constexpr (PACK) {
-        unsigned long long x[VPL][VN / 2];
+        uint64_t x[VPL][VN / 2];
 #pragma unroll
         for (int i = 0; i < VPL; ++i) {
             const int v = lane + 32 * i;
@@ -183,7 +180,7 @@ ln_warp_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
                 t.raw = __ldg(reinterpret_cast<const uint4*>(src) + v);
                 t.to_f32(f);
 #pragma unroll
-                for (int j = 0; j < VN / 2; ++j) x[i][j] = act_detail::pk(f[2 * j], f[2 * j + 1]);
+                for (int j = 0; j < VN / 2; ++j) x[i][j] = pack2(f[2 * j], f[2 * j + 1]);
             }
         }
         ln_moments<VPL, VN, LPG>(x, lane, nvec, C, eps, mu, r);
@@ -314,7 +311,7 @@ ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half*
     }
     float mu, r;
     if constexpr (PACK) {
-        unsigned long long v[VPL][VN / 2];
+        uint64_t v[VPL][VN / 2];
 #pragma unroll
         for (int i = 0; i < VPL; ++i) {
             const int vi = lane + 32 * i;
@@ -333,7 +330,7 @@ ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half*
                 }
                 store_vec<VN>(xr + (int64_t)vi * VN, fa);                           // exact: already fp16 values
 #pragma unroll
-                for (int j = 0; j < VN / 2; ++j) v[i][j] = act_detail::pk(fa[2 * j], fa[2 * j + 1]);
+                for (int j = 0; j < VN / 2; ++j) v[i][j] = pack2(fa[2 * j], fa[2 * j + 1]);
             }
         }
         ln_moments<VPL, VN, LPG>(v, lane, nvec, C, eps, mu, r);
