@@ -233,7 +233,8 @@ int b200_attention_f16_route(int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64
 /*
  * layernorm!/layernorm_kernel! (layernorm.jl:44-135): a is (C, groups) contiguous,
  * in_dtype/out_dtype fp16 or fp32; gamma/beta are (C,) in in_dtype or NULL; mean and
- * rstd are fp32 (groups,).  fp32 statistics, variance about the mean.
+ * rstd are fp32 (groups,).  fp32 statistics, variance about the mean.  fp16 launches of 48 Mi elements and
+ * more add in another order than smaller ones: a row's last bits may differ between the two.
  */
 int b200_layernorm(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, int in_dtype, void* out,
                    int out_dtype, float* mean, float* rstd, const void* gamma, const void* beta,

@@ -12,9 +12,9 @@
 // Replaces matmul_coopmat! + Lava.coopmat_gemm! + padcols_kernel! + mm_epilogue_kernel!
 // (reference kernels/extern/matmul.jl:172-273).
 //
-// Roles inside one persistent CTA (608 threads):
+// Roles inside one persistent CTA (576 threads):
 //   warp 0     TMA producer  (one lane)        global -> shared ring, STAGES deep
-//   warp 1     UMMA issuer   (one lane issues) shared -> TMEM accumulators (two, ping-pong)
+//   warp 1     UMMA issuer   (waits together, an elected thread issues) shared -> TMEM accumulators (two, ping-pong)
 //   warps 2-17 epilogue      (512 threads)     TMEM -> registers -> +bias, round, act ->
 //                                              warp-private shared slab -> bulk tensor store
 #include <cuda_fp16.h>

@@ -250,7 +250,7 @@ static int gemv_run(b200_ctx* ctx, int64_t M, int64_t K, const void* A, int64_t 
     // Taken while a block has up to 290 KB to read, where round trips are what a call waits for (1280 x 1280 in fp16
     // 6.3 -> 5.0 us, 4390 x 721 in fp32 6.6 -> 5.5, 3000 x 5000 in fp16 10.0 -> 7.6).  With more to read, or more row
     // blocks than SMs, blocks of eight warps, six to an SM, stream with fewer gaps (9956 x 1817 in fp16 8.9 us against
-    // 9.8, 51865 x 1280 25.3 against 31); and so few row blocks that eight parts would leave nine tenths of the SMs idle
+    // 9.8, 51865 x 1280 25 against 31); and so few row blocks that eight parts would leave nine tenths of the SMs idle
     // over a long chain are split further that way (256 x 4096: 6.35 us, 6.44 as a cluster).
     const bool few = mblocks * 8 * 8 <= sms && K >= GEMV_SPLIT_MIN_K;
     const bool cluster = K == 0 || (!few && mblocks <= sms && M * K * (int64_t)sizeof(T) <= 290 * 1024 * mblocks * parts);

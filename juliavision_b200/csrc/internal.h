@@ -116,8 +116,8 @@ int attention_few_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64
 
 // GEMM with the bias broadcast along either axis (bias_per_n = 1: one value per column j,
 // which is what a convolution lowered to a GEMM over pixels needs).  use_workspace = 0 keeps the
-// planner to schedules that need no scratch memory (whole tiles only), so the call touches neither
-// the workspace nor the pool.
+// planner to schedules that need no scratch memory (whole tiles, and tiles whose k-blocks a cluster
+// shares), so the call touches neither the workspace nor the pool.
 int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda, const void* B,
                  int64_t ldb, const void* bias, int bias_per_n, void* out, int64_t ldo, int out_dtype,
                  int epilogue, int64_t nbatch, int64_t strideA, int64_t strideB, int64_t strideO,

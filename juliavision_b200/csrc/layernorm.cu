@@ -75,8 +75,8 @@ __device__ __forceinline__ float group_sum(float v) {
 }
 
 // The packed form (PACK): a row's moments and its output two elements per instruction, gamma and beta in one rounding.
-// It is for launches whose rows come from and go to HBM (more than the L2 holds): 65536 x 1280 in fp16 62.2 -> 58.1 us
-// (5.4 -> 5.8 TB/s), where the scalar form issues for about 25 us of the launch.  Rows that stay in the L2 are faster
+// It is for launches whose rows come from and go to HBM (more than the L2 holds): 65536 x 1280 in fp16 63.1 -> 59.6 us
+// (5.3 -> 5.6 TB/s, replayed over four operand sets), where the scalar form issues for about 25 us of the launch.  Rows that stay in the L2 are faster
 // in the scalar form (14736 x 1176: 11.7 us, packed 12.9), so the row bytes decide, the same for the layer norm alone
 // and the one behind a residual add, which therefore give the same bits.  The vectors of a lane are v = first,
 // first + 32, ...; `x` is left holding x - mean.
@@ -439,7 +439,8 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 
 // Rows too wide for one warp's registers (more than 16 vectors per lane): one block per row, the row in registers as
 // above, the two sums over the block through shared memory.  Bound by HBM; with scalar accesses and the row read three
-// times these rows took 71 us for 7112 x 4280 in fp32, now 42.7 (5.7 TB/s); 79 x 3168 4.9 -> 2.9.
+// times these rows took 71.6 us for 7112 x 4280 in fp32, now 44.5 (5.5 TB/s); 79 x 3168 5.4 -> 3.3, 20000 x 5120 in fp16
+// 206 -> 106 (replayed over four operand sets).
 template <typename InT, typename OutT, int VPT>
 __global__ void __launch_bounds__(LN_WIDE_THREADS)
 ln_wide_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restrict__ mean, float* __restrict__ rstd,
@@ -557,7 +558,8 @@ ln_block_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __rest
     }
 }
 
-// fp16 rows of more than 96 MB, and as many bytes of results: they do not stay in the L2 (see the packed form).
+// fp16 rows of more than 96 MB, and as many bytes of results: they do not stay in the L2 (see the packed form).  A row's
+// last bits therefore depend on the launch being this large, as they do on which kernel its width and alignment choose.
 static bool ln_packs(int64_t groups, int64_t C) { return groups * C >= (int64_t)48 << 20; }
 
 template <typename InT, typename OutT>
