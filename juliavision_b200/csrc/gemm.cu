@@ -87,11 +87,11 @@ template <typename OutT> struct GemmParams {
 
 // Timeline slots written by worker 0 when tracing (b200_timeline): globaltimer ns at [slot] and
 // the SM's own cycle counter at [64 + slot], so a phase can be read both in time and in cycles (their
-// ratio is the clock the SM actually ran at).  One CTA writes: a pair's leader, the first part of a K split.  Costs one
-// predictable branch per event otherwise.
+// ratio is the clock the SM actually ran at).  One CTA writes, the grid's first: worker 0, a pair's leader, the first part
+// of a K split.  Costs one predictable branch per event otherwise.
 #define GEMM_TRACE(slot)                                                   \
     do {                                                                   \
-        if (p.trace != nullptr && worker == 0 && rank == 0 && kpart == 0) { \
+        if (p.trace != nullptr && blockIdx.x == 0) {                       \
             p.trace[(slot)] = globaltimer_ns();                            \
             p.trace[64 + (slot)] = (unsigned long long)clock64();          \
         }                                                                  \
