@@ -514,7 +514,9 @@ ln_wide_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
                 t.raw = __ldg(reinterpret_cast<const uint4*>(beta) + v);
                 t.to_f32(bf);
 #pragma unroll
-                for (int j = 0; j < VN; ++j) y[j] += bf[j];
+                for (int j = 0; j < VN; ++j)   // fp32 without gamma: one rounding too (with two, 14 % further)
+                    if constexpr (sizeof(OutT) == 4) y[j] = fmaf(x[i][j] - mu, r, bf[j]);
+                    else y[j] += bf[j];
             }
             store_vec<VN>(dst + (int64_t)v * VN, y);
         }

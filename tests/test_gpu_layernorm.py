@@ -67,6 +67,9 @@ def test_rows_wider_than_a_warp_holds_round_gamma_and_beta_once(ctx, C):
     y = (a - mean.reshape(-1, 1)) * rstd.reshape(-1, 1)
     once = np.float32(y.astype(np.float64) * gam + bet)
     assert np.mean(got != once) < 1e-4      # a double rounding where 64 bits end on a tie
+    got, mean, rstd = layernorm_gpu(ctx, a, None, bet, 1e-5)      # beta alone: added to the product with rstd
+    once = np.float32((a - mean.reshape(-1, 1)).astype(np.float64) * rstd.reshape(-1, 1) + bet)
+    assert np.mean(got != once) < 1e-4
 
 
 def test_mean_dominates_variance(ctx, ora):
