@@ -425,6 +425,8 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
 
                 if constexpr (BIAS) {
                     // r <- s * scale + bias: from here on the scores are in the mask's units and the scale below is log2(e).
+                    // (A reference point beyond 2^12, where every key of a row carries the type's lowest value, is itself
+                    // rounded by more than fp16 tells from one: there the heaviest key's P is rounded like the others'.)
                     const int lq = q0 + t * ATT_BR + row;
                     if (p.bias == nullptr) {
 #pragma unroll
