@@ -110,7 +110,7 @@ __device__ __forceinline__ void ln_moments(uint64_t (&x)[VPL][VN / 2], int first
         }
     r = 1.0f / sqrtf(group_sum<LPG>(pairs_sum(s2)) / n + eps);
 }
-// One vector of the result: d = x - mean; y = d r, then gamma and beta in one rounding where both are there.
+// One vector of the result: d = x - mean; y = d r, then gamma and beta in one rounding, or d r and beta in one.
 template <typename InT, typename OutT>
 __device__ __forceinline__ void ln_write(OutT* dst, const uint64_t* d, float r, bool has_g, const uint4& g, bool has_b,
                                          const uint4& b) {
@@ -124,10 +124,11 @@ __device__ __forceinline__ void ln_write(OutT* dst, const uint64_t* d, float r, 
     const uint64_t rr = pack2(r, r);
 #pragma unroll
     for (int j = 0; j < VN / 2; ++j) {
-        uint64_t v = mul2(d[j], rr);
-        if (has_g && has_b) v = fma2(v, pack2(gf[2 * j], gf[2 * j + 1]), pack2(bf[2 * j], bf[2 * j + 1]));
-        else if (has_g) v = mul2(v, pack2(gf[2 * j], gf[2 * j + 1]));
-        else if (has_b) v = add2(v, pack2(bf[2 * j], bf[2 * j + 1]));
+        uint64_t v;
+        if (has_g && has_b) v = fma2(mul2(d[j], rr), pack2(gf[2 * j], gf[2 * j + 1]), pack2(bf[2 * j], bf[2 * j + 1]));
+        else if (has_g) v = mul2(mul2(d[j], rr), pack2(gf[2 * j], gf[2 * j + 1]));
+        else if (has_b) v = fma2(d[j], rr, pack2(bf[2 * j], bf[2 * j + 1]));
+        else v = mul2(d[j], rr);
         unpack2(v, y[2 * j], y[2 * j + 1]);
     }
     store_vec<VN>(dst, y);
@@ -265,15 +266,19 @@ ln_warp_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
 // Bit-identical to running add.Tensor, clamp.default and native_layer_norm one after another
 // (each rounds to fp16 where the separate ops would), but x and h are read once and the three
 // launches become one.
-template <int VPL, int LPG = 32, bool LAT = false, bool PACK = false>
-__global__ void __launch_bounds__(128)
+// PAIRS: the order of the packed form, whose bits these are to be where the layer norm alone takes it, in scalar
+// instructions: even and odd elements summed apart, gamma and beta (or the deviation and beta) in one rounding.  As packed
+// instructions the row's two inputs and its pairs left a third fewer warps in flight (65536 x 1280: 136 us, 118.6 this way,
+// 117.2 in the plain order; 43000 x 1480: 121, 104.0, 102.4); the bound on registers is the plain order's own count.
+template <int VPL, int LPG = 32, bool LAT = false, bool PAIRS = false>
+__global__ void __launch_bounds__(128, PAIRS ? (VPL <= 5 ? 8 : 7) : 0)
 ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half* __restrict__ out,
                    float* __restrict__ mean, float* __restrict__ rstd, const __half* __restrict__ gamma,
                    const __half* __restrict__ beta, int64_t groups, int C, float eps, int use_clamp, float lo,
                    float hi) {
     constexpr int VN = 8;
     static_assert(LPG == 32 || VPL == 1, "only single-vector groups share a warp");
-    static_assert(!(PACK && LAT), "the packed form is for launches of many waves");
+    static_assert(!(PAIRS && LAT), "the packed form is for launches of many waves");
     const int lane = threadIdx.x & (LPG - 1);
     const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / LPG;
     const int nvec = g < groups ? C / VN : 0;
@@ -309,111 +314,100 @@ ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half*
             }
         }
     }
-    float mu, r;
-    if constexpr (PACK) {
-        uint64_t v[VPL][VN / 2];
+    float v[VPL][VN];
+    float s = 0.f, so = 0.f;   // so: the odd elements' sum with PAIRS
 #pragma unroll
-        for (int i = 0; i < VPL; ++i) {
-            const int vi = lane + 32 * i;
-            if (vi < nvec) {
-                Vec16<__half> a, b;
+    for (int i = 0; i < VPL; ++i) {
+        const int vi = lane + 32 * i;
+        if (vi < nvec) {
+            Vec16<__half> a, b;
+            if constexpr (HOIST) {
+                a.raw = xraw[i];
+                b.raw = hraw[i];
+            } else {
                 a.raw = *(reinterpret_cast<const uint4*>(xr) + vi);
                 b.raw = __ldg(reinterpret_cast<const uint4*>(hr) + vi);
-                float fa[VN], fb[VN];
-                a.to_f32(fa);
-                b.to_f32(fb);
+            }
+            float fa[VN], fb[VN];
+            a.to_f32(fa);
+            b.to_f32(fb);
 #pragma unroll
-                for (int j = 0; j < VN; ++j) {
-                    float t = __half2float(__float2half_rn(fa[j] + fb[j]));        // add.Tensor rounds here
-                    if (use_clamp) t = __half2float(__float2half_rn(fminf(fmaxf(t, lo), hi)));
-                    fa[j] = t;
-                }
-                store_vec<VN>(xr + (int64_t)vi * VN, fa);                           // exact: already fp16 values
+            for (int j = 0; j < VN; ++j) {
+                float t = __half2float(__float2half_rn(fa[j] + fb[j]));        // add.Tensor rounds here
+                if (use_clamp) t = __half2float(__float2half_rn(fminf(fmaxf(t, lo), hi)));
+                v[i][j] = t;
+                if (PAIRS && (j & 1)) so += t;
+                else s += t;
+            }
+            store_vec<VN>(xr + (int64_t)vi * VN, v[i]);                         // exact: already fp16 values
+        }
+    }
+    const float n = (float)C;
+    const float mu = group_sum<LPG>(PAIRS ? s + so : s) / n;
+    float s2 = 0.f, s2o = 0.f;
 #pragma unroll
-                for (int j = 0; j < VN / 2; ++j) v[i][j] = pack2(fa[2 * j], fa[2 * j + 1]);
+    for (int i = 0; i < VPL; ++i)
+        if (lane + 32 * i < nvec) {
+#pragma unroll
+            for (int j = 0; j < VN; ++j) {
+                float d = v[i][j] - mu;
+                if (PAIRS && (j & 1)) s2o = fmaf(d, d, s2o);
+                else s2 = fmaf(d, d, s2);
             }
         }
-        ln_moments<VPL, VN, LPG>(v, lane, nvec, C, eps, mu, r);
-        __half* dst = out + g * (int64_t)C;
+    const float r = 1.0f / sqrtf(group_sum<LPG>(PAIRS ? s2 + s2o : s2) / n + eps);
+    __half* dst = out + g * (int64_t)C;
 #pragma unroll
-        for (int i = 0; i < VPL; ++i) {
-            const int vi = lane + 32 * i;
-            if (vi < nvec) {
-                uint4 gv = make_uint4(0u, 0u, 0u, 0u), bv = gv;
+    for (int i = 0; i < VPL; ++i) {
+        const int vi = lane + 32 * i;
+        if (vi < nvec) {
+            if constexpr (PAIRS) {   // two elements at a time: whole vectors of gamma and beta beside the row would spill
+                uint4 gv = make_uint4(0u, 0u, 0u, 0u), bv = gv, ov;
                 if (gamma) gv = __ldg(reinterpret_cast<const uint4*>(gamma) + vi);
                 if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + vi);
-                ln_write<__half, __half>(dst + (int64_t)vi * VN, v[i], r, gamma != nullptr, gv, beta != nullptr, bv);
+                const __half2 *gh = reinterpret_cast<const __half2*>(&gv), *bh = reinterpret_cast<const __half2*>(&bv);
+#pragma unroll
+                for (int j = 0; j < VN / 2; ++j) {
+                    const float2 g2 = __half22float2(gh[j]), b2 = __half22float2(bh[j]);
+                    const float d0 = v[i][2 * j] - mu, d1 = v[i][2 * j + 1] - mu;
+                    float y0 = __fmul_rn(d0, r), y1 = __fmul_rn(d1, r);
+                    if (gamma && beta) {
+                        y0 = fmaf(y0, g2.x, b2.x);
+                        y1 = fmaf(y1, g2.y, b2.y);
+                    } else if (gamma) {
+                        y0 *= g2.x;
+                        y1 *= g2.y;
+                    } else if (beta) {
+                        y0 = fmaf(d0, r, b2.x);
+                        y1 = fmaf(d1, r, b2.y);
+                    }
+                    reinterpret_cast<__half2*>(&ov)[j] = __floats2half2_rn(y0, y1);
+                }
+                *(reinterpret_cast<uint4*>(dst) + vi) = ov;
+                continue;
             }
-        }
-    } else {
-        float v[VPL][VN];
-        float s = 0.f;
+            float y[VN];
 #pragma unroll
-        for (int i = 0; i < VPL; ++i) {
-            const int vi = lane + 32 * i;
-            if (vi < nvec) {
-                Vec16<__half> a, b;
-                if constexpr (HOIST) {
-                    a.raw = xraw[i];
-                    b.raw = hraw[i];
-                } else {
-                    a.raw = *(reinterpret_cast<const uint4*>(xr) + vi);
-                    b.raw = __ldg(reinterpret_cast<const uint4*>(hr) + vi);
-                }
-                float fa[VN], fb[VN];
-                a.to_f32(fa);
-                b.to_f32(fb);
+            for (int j = 0; j < VN; ++j) y[j] = (v[i][j] - mu) * r;
+            if (gamma) {
+                Vec16<__half> t;
+                float gf[VN];
+                if constexpr (HOIST) t.raw = gw[i];
+                else t.raw = __ldg(reinterpret_cast<const uint4*>(gamma) + vi);
+                t.to_f32(gf);
 #pragma unroll
-                for (int j = 0; j < VN; ++j) {
-                    float t = __half2float(__float2half_rn(fa[j] + fb[j]));        // add.Tensor rounds here
-                    if (use_clamp) t = __half2float(__float2half_rn(fminf(fmaxf(t, lo), hi)));
-                    v[i][j] = t;
-                    s += t;
-                }
-                store_vec<VN>(xr + (int64_t)vi * VN, v[i]);                         // exact: already fp16 values
+                for (int j = 0; j < VN; ++j) y[j] *= gf[j];
             }
-        }
-        const float n = (float)C;
-        mu = group_sum<LPG>(s) / n;
-        float s2 = 0.f;
+            if (beta) {
+                Vec16<__half> t;
+                float bf[VN];
+                if constexpr (HOIST) t.raw = bw[i];
+                else t.raw = __ldg(reinterpret_cast<const uint4*>(beta) + vi);
+                t.to_f32(bf);
 #pragma unroll
-        for (int i = 0; i < VPL; ++i)
-            if (lane + 32 * i < nvec) {
-#pragma unroll
-                for (int j = 0; j < VN; ++j) {
-                    float d = v[i][j] - mu;
-                    s2 += d * d;
-                }
+                for (int j = 0; j < VN; ++j) y[j] += bf[j];
             }
-        r = 1.0f / sqrtf(group_sum<LPG>(s2) / n + eps);
-        __half* dst = out + g * (int64_t)C;
-#pragma unroll
-        for (int i = 0; i < VPL; ++i) {
-            const int vi = lane + 32 * i;
-            if (vi < nvec) {
-                float y[VN];
-#pragma unroll
-                for (int j = 0; j < VN; ++j) y[j] = (v[i][j] - mu) * r;
-                if (gamma) {
-                    Vec16<__half> t;
-                    float gf[VN];
-                    if constexpr (HOIST) t.raw = gw[i];
-                    else t.raw = __ldg(reinterpret_cast<const uint4*>(gamma) + vi);
-                    t.to_f32(gf);
-#pragma unroll
-                    for (int j = 0; j < VN; ++j) y[j] *= gf[j];
-                }
-                if (beta) {
-                    Vec16<__half> t;
-                    float bf[VN];
-                    if constexpr (HOIST) t.raw = bw[i];
-                    else t.raw = __ldg(reinterpret_cast<const uint4*>(beta) + vi);
-                    t.to_f32(bf);
-#pragma unroll
-                    for (int j = 0; j < VN; ++j) y[j] += bf[j];
-                }
-                store_vec<VN>(dst + (int64_t)vi * VN, y);
-            }
+            store_vec<VN>(dst + (int64_t)vi * VN, y);
         }
     }
     if (lane == 0 && g < groups) {
@@ -563,6 +557,10 @@ ln_block_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __rest
 // fp16 rows of more than 96 MB, and as many bytes of results: they do not stay in the L2 (see the packed form).  A row's
 // last bits therefore depend on the launch being this large, as they do on which kernel its width and alignment choose.
 static bool ln_packs(int64_t groups, int64_t C) { return groups * C >= (int64_t)48 << 20; }
+// The widths for which the packed form was measured to pay, as vectors per lane.  Four (60000 x 1000: 43.9 us scalar, 47.0
+// packed) and eight (36000 x 1800: 60.0, 62.3; 32000 x 2048: 55.2, 57.2) lose: there its registers cost more warps than its
+// instructions save; five and six gain (50000 x 1280: 51.8 -> 49.1, 43000 x 1480: 55.2 -> 52.1).
+constexpr bool ln_pack_width(int vpl) { return vpl == 5 || vpl == 6; }
 
 template <typename InT, typename OutT>
 static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, void* out, float* mean,
@@ -590,8 +588,8 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
         if (lat)                                                                                            \
             B200_CUDA(launch_dep(ln_warp_kernel<InT, OutT, V, 32, true>, grid, block, 0, ctx->stream, 1, ap, op, mean, rstd, gp, \
                                  bp, groups, (int)C, eps));                                                 \
-        else if (PACKS && (V) >= 4 && (V) <= 8 && ln_packs(groups, C))                                      \
-            B200_CUDA(launch_dep(ln_warp_kernel<InT, OutT, V, 32, false, PACKS && (V) >= 4 && (V) <= 8>, grid, block, 0, ctx->stream, 1, \
+        else if (PACKS && ln_pack_width(V) && ln_packs(groups, C))                                          \
+            B200_CUDA(launch_dep(ln_warp_kernel<InT, OutT, V, 32, false, PACKS && ln_pack_width(V)>, grid, block, 0, ctx->stream, 1, \
                                  ap, op, mean, rstd, gp, bp, groups, (int)C, eps));                         \
         else                                                                                                \
             B200_CUDA(launch_dep(ln_warp_kernel<InT, OutT, V>, grid, block, 0, ctx->stream, 1, ap, op, mean, rstd, gp, bp, \
@@ -661,8 +659,8 @@ extern "C" int b200_add_layernorm_f16(b200_ctx* ctx, int64_t groups, int64_t C, 
             B200_CUDA(launch_dep(ln_add_warp_kernel<V, 32, true>, grid, block, 0, ctx->stream, 1, (__half*)x, (const __half*)h, \
                                  (__half*)out, mean, rstd, (const __half*)gamma, (const __half*)beta, groups, (int)C, eps, \
                                  use_clamp, lo, hi));                                                             \
-        else if ((V) >= 4 && (V) <= 8 && ln_packs(groups, C))                                                     \
-            B200_CUDA(launch_dep(ln_add_warp_kernel<V, 32, false, (V) >= 4 && (V) <= 8>, grid, block, 0, ctx->stream, 1, (__half*)x, \
+        else if (ln_pack_width(V) && ln_packs(groups, C))                                                         \
+            B200_CUDA(launch_dep(ln_add_warp_kernel<V, 32, false, ln_pack_width(V)>, grid, block, 0, ctx->stream, 1, (__half*)x, \
                                  (const __half*)h, (__half*)out, mean, rstd, (const __half*)gamma, (const __half*)beta, groups, (int)C, \
                                  eps, use_clamp, lo, hi));                                                        \
         else                                                                                                      \

@@ -90,7 +90,7 @@ def test_empty_and_errors(ctx):
         jv.layernorm_(ctx, b, m, m, b, None, None, 7, 1e-5)  # 30 is not a multiple of 7
 
 
-PACKED = [1000, 1024, 1176, 1480, 1800, 2048]    # 4, 4, 5, 6 and 8 vectors per lane, the last one ragged or full
+PACKED = [1000, 1024, 1176, 1480, 1800, 2048]    # 4, 4, 5, 6 and 8 vectors per lane, the last one ragged or full; 5 and 6 pack
 
 
 def _packed_rows(C):
@@ -101,7 +101,7 @@ def _packed_rows(C):
 
 @pytest.mark.parametrize("C", PACKED)
 def test_rows_the_cache_does_not_hold(ctx, ora, C):
-    """The packed form: first and last rows and a sample in between, with gamma and beta, one of them and neither."""
+    """The packed form and its neighbours: first and last rows and a sample, with gamma and beta, one of them and neither."""
     groups = _packed_rows(C)
     rng = np.random.default_rng(C)
     a = np.float16(rng.standard_normal((groups, C), dtype=np.float32) * 2 + 0.5)
@@ -121,7 +121,8 @@ def test_add_layernorm_equals_the_three_ops_where_the_cache_does_not_hold_them(c
     rng = np.random.default_rng(C)
     least = ((48 << 20) + C - 1) // C
     g, b = (ctx.toback(np.float16(o + 0.1 * rng.standard_normal(C))) for o in (1, 0))
-    for groups, clamp, gb in ((_packed_rows(C), (-500.0, 500.0), (g, b)), (least, None, (g, None)), (least - 1, None, (g, b))):
+    for groups, clamp, gb in ((_packed_rows(C), (-500.0, 500.0), (g, b)), (least, None, (g, None)), (least, None, (None, b)),
+                              (least - 1, None, (g, b)), (least - 1, None, (None, b))):
         x0, h0 = (np.float16(rng.standard_normal((groups, C), dtype=np.float32) * 300) for _ in range(2))
         mean, rstd, m2, r2 = (ctx.allocate(np.float32, groups) for _ in range(4))
         xa, ha, oa = ctx.toback(x0), ctx.toback(h0), ctx.allocate(np.float16, C, groups)
@@ -135,3 +136,15 @@ def test_add_layernorm_equals_the_three_ops_where_the_cache_does_not_hold_them(c
         ctx.synchronize()
         for one, other in ((xa, xb), (oa, ob), (mean, m2), (rstd, r2)):
             assert np.array_equal(one.to_host(), other.to_host()), (groups, C)
+
+
+@pytest.mark.parametrize("C,same", [(1000, True), (1024, True), (1176, False), (1480, False), (1800, True), (2048, True)])
+def test_only_the_widths_that_gain_take_the_packed_form(ctx, C, same):
+    """Five and six vectors per lane are faster packed, four and eight slower: there a row keeps its bits whatever the launch."""
+    rng = np.random.default_rng(C)
+    part = np.float16(rng.standard_normal((4096, C)) * 2 + 0.5)
+    gam, bet = (np.float16(o + 0.1 * rng.standard_normal(C)) for o in (1, 0))
+    small = layernorm_gpu(ctx, part, gam, bet, 1e-5)
+    large = layernorm_gpu(ctx, np.tile(part, (-(-_packed_rows(C) // 4096), 1)), gam, bet, 1e-5)
+    equal = [np.array_equal(a, b[:len(a)]) for a, b in zip(small, large)]
+    assert equal == [True] * 3 if same else not all(equal)
