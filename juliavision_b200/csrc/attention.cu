@@ -1005,9 +1005,9 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     // kernel keeps six CTAs per SM in flight where this one's set-up would cost more than the arithmetic.
     if (bptr == nullptr && E <= 64 && Lk <= 64 && B * H * cdiv(Lq, 64) > 2 * ctx->prop.multiProcessorCount)
         return attention_window_launch(ctx, E, Lq, Lk, H, B, q, k, v, o, out_dtype, scale);
-    // A few queries: their tile would be mostly empty (see attention_few.cu).  Past 16, and past 32 with E <= 64, a warp
-    // has too much of the chain to itself: 40 x 1500, E = 72, 20 heads took 19.5 us there and 13.1 here.
-    if (Lq <= (E <= 64 ? 32 : 16)) return attention_few_launch(ctx, E, Lq, Lk, H, B, q, k, v, bptr, bs, o, out_dtype, scale);
+    // A few queries: their tile would be mostly empty (see attention_few.cu).
+    if (attention_few_takes(ctx, E, Lq, Lk, H, B, bptr != nullptr))
+        return attention_few_launch(ctx, E, Lq, Lk, H, B, q, k, v, bptr, bs, o, out_dtype, scale);
     const bool wide = E > 64;                              // two swizzle atoms along E
     const int64_t sms = ctx->prop.multiProcessorCount;
     // Up to 256 keys and more than two tiles per SM (16 x 16 windows): one tile per CTA, four CTAs per SM, so that one's
@@ -1059,6 +1059,7 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     p.part_o = p.part_ml = nullptr;
     const int64_t rem = pairs % sms;
     const size_t ws_mark = ctx->ws_used;
+    const bool frugal = bptr != nullptr || Lq <= (E <= 64 ? 32 : 16);
     if (!single && nblk_all >= 4) {
         int64_t ntail = 0, ns = 1;
         if (2 * pairs <= sms) {
@@ -1074,9 +1075,9 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
             const int64_t rows = ntail * item_rows;
             void* ws = nullptr;
             rc = ws_scratch(ctx, (size_t)(ns * rows * (E + 2)) * sizeof(float), &ws);
-            // A masked call does not depend on the workspace: it runs unsplit when that is refused (a graph recorded
-            // without an eager call before), and gives its share back below.
-            if (rc && !(bptr && rc == B200_ENOMEM)) return rc;
+            // A masked call, and one of as few queries as attention_few.cu takes, does not depend on the workspace: it runs
+            // unsplit when that is refused (a graph recorded without an eager call before), and gives its share back below.
+            if (rc && !(frugal && rc == B200_ENOMEM)) return rc;
             if (!rc) {
                 p.nsplit = (int)ns;
                 p.ntail = (int)ntail;
@@ -1094,7 +1095,7 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
                              (const float*)p.part_o, (const float*)p.part_ml, p.nsplit, p.ntail, p.pair_ctas, p.qpairs, (int)item_rows, (int)E,
                              (int)Lq, (int)H, out, o->stride[1], o->stride[2], o->stride[3], (int)(out_dtype == B200_F32)));
         ctx->launches += 2;
-        if (bptr) ctx->ws_used = ws_mark;   // what comes next on the stream runs after the merge has read the partial rows
+        if (frugal) ctx->ws_used = ws_mark;   // what comes next on the stream runs after the merge has read the partial rows
         return B200_OK;
     }
     // Split the pairs of a last wave that would leave more than half of the SMs idle — but not a

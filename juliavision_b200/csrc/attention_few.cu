@@ -13,7 +13,8 @@
 #include <cuda_fp16.h>
 #include <stdlib.h>
 
-#include <atomic>
+#include <mutex>
+#include <type_traits>
 
 #include "internal.h"
 #include "ptx.cuh"
@@ -311,56 +312,122 @@ attention_few_kernel(const FewParams p) {
     if (parts > 1) cluster_sync_all();   // nobody leaves while its rows may still be read
 }
 
-// The largest cluster of this kernel, up to AF_PARTS, of which the device can hold one: 16 is beyond the portable size,
-// and a slice of a GPU may have fewer SMs to a GPC.  Asked of the runtime once per device.
-template <typename Kern> static int af_largest(Kern kern, size_t smem) {
-    for (int n = AF_PARTS; n > 8; n /= 2) {
+// How many CTAs of this kernel, and clusters of 2, 4, 8 and 16 of them, the device holds at once: [l] for 2^l, asked of the
+// runtime once per device.  A GPC's SMs do not divide into large clusters without a rest, so that twice the SMs over the size is too many;
+// sixteen is beyond the portable size besides, and a slice of a GPU may hold none.
+struct AfRoom {
+    int clusters[5];
+};
+template <typename Kern> static AfRoom af_ask(b200_ctx* ctx, Kern kern, size_t smem) {
+    AfRoom room = {};
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, AF_THREADS, smem) != cudaSuccess) cudaGetLastError();
+    room.clusters[0] = ctx->prop.multiProcessorCount * (per_sm > 0 ? per_sm : 1);
+    const bool wide = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    for (int l = 1; l <= (wide ? 4 : 3); ++l) {
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)n;
+        attr[0].val.clusterDim.x = 1u << l;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)n, 1, 1);
+        cfg.gridDim = dim3(1u << l, 1, 1);
         cfg.blockDim = dim3(AF_THREADS, 1, 1);
         cfg.dynamicSmemBytes = smem;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int fit = 0;
-        if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess && fit > 0) return n;
-        cudaGetLastError();
+        if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess) room.clusters[l] = fit;
+        else cudaGetLastError();
     }
-    return 8;   // portable
+    if (!wide) cudaGetLastError();
+    return room;
+}
+
+template <int EP, int KS, bool BIAS> static cudaError_t af_rooms(b200_ctx* ctx, const AfRoom*& room) {
+    static std::once_flag once[16];
+    static AfRoom rooms[16];
+    static cudaError_t set[16];
+    auto kern = attention_few_kernel<EP, KS, BIAS>;
+    const int d = ctx->device & 15;
+    std::call_once(once[d], [&] {
+        set[d] = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AfCfg<EP, KS>::SMEM_BYTES);
+        if (set[d] == cudaSuccess) rooms[d] = af_ask(ctx, kern, AfCfg<EP, KS>::SMEM_BYTES);
+    });
+    room = &rooms[d];
+    return set[d];
+}
+
+static const char* af_forced() { return getenv("B200_ATTENTION_PARTS"); }   // debugging aid: this kernel, with clusters up to that size
+
+// Key parts: as many, with two blocks or more each, as keep every cluster resident at once.  A second round of clusters
+// costs more than the shorter walk saves (17 heads, 25 x 2405: 15.7 us with sixteen parts, of which sixteen clusters fit).
+static int af_parts(const AfRoom& room, int64_t nblk, int64_t items) {
+    const char* f = af_forced();
+    const int most = f ? atoi(f) : AF_PARTS;
+    int parts = 1;
+    for (int l = 1; l <= 4 && (1 << l) <= most && nblk >= 2 << l; ++l)
+        if (items <= room.clusters[l]) parts = 1 << l;
+    return parts;
 }
 
 template <int EP, int KS, bool BIAS>
-static int af_launch(b200_ctx* ctx, const FewParams& p, int64_t H, int64_t B, int parts) {
-    using Cfg = AfCfg<EP, KS>;
-    static std::atomic<int> largest[16] = {};
-    auto kern = attention_few_kernel<EP, KS, BIAS>;
-    int most = largest[ctx->device & 15].load(std::memory_order_acquire);
-    if (most == 0) {
-        B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) most = af_largest(kern, Cfg::SMEM_BYTES);
-        else most = 8, cudaGetLastError();
-        largest[ctx->device & 15].store(most, std::memory_order_release);
-    }
-    if (parts > most) parts = most;
-    B200_CUDA(launch_dep(kern, dim3((unsigned)parts, (unsigned)H, (unsigned)B), dim3(AF_THREADS, 1, 1), Cfg::SMEM_BYTES, ctx->stream,
-                         parts, p));
+static int af_launch(b200_ctx* ctx, const FewParams& p, int64_t H, int64_t B) {
+    const AfRoom* room;
+    B200_CUDA((af_rooms<EP, KS, BIAS>(ctx, room)));
+    const int parts = af_parts(*room, cdiv(p.Lk, AF_BC), H * B);
+    B200_CUDA(launch_dep(attention_few_kernel<EP, KS, BIAS>, dim3((unsigned)parts, (unsigned)H, (unsigned)B), dim3(AF_THREADS, 1, 1),
+                         AfCfg<EP, KS>::SMEM_BYTES, ctx->stream, parts, p));
     ctx->launches++;
     return B200_OK;
 }
 
-template <int EP, int KS>
-static int af_bias(b200_ctx* ctx, const FewParams& p, int64_t H, int64_t B, int parts) {
-    return p.bias ? af_launch<EP, KS, true>(ctx, p, H, B, parts) : af_launch<EP, KS, false>(ctx, p, H, B, parts);
+// f(head dim tier, key slots, mask) with the three as constants
+template <typename F> static auto af_dispatch(int64_t E, int64_t Lq, bool masked, F f) {
+    auto mask = [&](auto ep, auto ks) { return masked ? f(ep, ks, std::true_type{}) : f(ep, ks, std::false_type{}); };
+    if (E > 64) return mask(AfInt<128>{}, AfInt<4>{});       // up to 16 queries
+    return Lq <= 16 ? mask(AfInt<64>{}, AfInt<4>{}) : mask(AfInt<64>{}, AfInt<2>{});
 }
-template <int EP>
-static int af_slots(b200_ctx* ctx, const FewParams& p, int64_t H, int64_t B, int parts) {
-    if constexpr (EP == 64)   // wider heads come here with up to 16 queries
-        if (p.Lq > 16) return af_bias<EP, 2>(ctx, p, H, B, parts);
-    return af_bias<EP, 4>(ctx, p, H, B, parts);
+
+// Whether a call of few queries is faster here than as tiles of 128 queries (attention_f16_tc_kernel, which cuts the keys
+// too, and merges in a second launch).  Both times in us, fitted to 5060 shapes timed on both (4 to 290 heads in all, 1 to
+// 32 queries, 16 to 8192 keys): the large kernel takes as long for 128 keys as this one for 64, but sets up tensor memory
+// and merges.  16 to 32 queries over up to 384 keys are its (20 heads, 32 x 128: 4.4 us there, 7.2 here; 32 x 256 5.7, 6.7),
+// and many heads over long keys with more than 16 queries (36 heads, 32 x 8192: 31, 36); up to 8 queries are nearly always
+// this one's (8 heads, 1 x 1000: 9.5, 5.0).  Over 4154 further shapes the choice leaves two more than 4 % behind the large
+// kernel, where taking every call here left 350, by up to three quarters.
+bool attention_few_takes(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B, bool masked) {
+    if (Lq > (E <= 64 ? 32 : 16)) return false;
+    if (af_forced()) return true;
+    struct Large { double wave, split, part, block; };
+    struct Few { double start, join, finish, one, two; };   // per block: one CTA on an SM, or two
+    static const Large large[2][2] = {{{3.16, 2.76, 0.34, 1.42}, {3.04, 2.72, 0.37, 2.22}}, {{3.05, 2.72, 0.40, 2.22}, {2.95, 2.73, 0.41, 3.09}}};
+    static const Few few[3][2] = {{{3.41, 0.84, 0.83, 0.46, 0.78}, {3.47, 1.08, 1.07, 0.86, 1.21}},
+                                  {{6.17, -0.51, 0.33, 0.50, 0.99}, {5.77, -0.66, 0.15, 1.77, 2.60}},
+                                  {{4.58, 0.86, 0.79, 0.92, 1.52}, {3.90, 0.97, 1.16, 1.69, 2.46}}};
+    const int64_t items = H * B, sms = ctx->prop.multiProcessorCount, blocks = cdiv(Lk, 128), nblk = cdiv(Lk, AF_BC);
+    const Large& m = large[E > 64][masked];
+    double there = m.wave * (double)cdiv(items, sms) + m.block * (double)(blocks * cdiv(items, sms));
+    const int64_t rem = items % sms, cut = 2 * items <= sms ? items : (items > sms && rem > 0 && 2 * rem <= sms ? rem : 0);
+    if (blocks >= 4 && cut > 0) {   // the keys of `cut` items over ns CTAs each, as the large kernel's launch does
+        int64_t ns = sms / cut;
+        if (ns > blocks / 2) ns = blocks / 2;
+        if (ns > 64) ns = 64;
+        if (ns >= 2)
+            there = m.wave * (double)(items / sms + 1) + m.split + m.part * (double)ns + m.block * (double)(blocks * (items / sms) + cdiv(blocks, ns));
+    }
+    const AfRoom* room = nullptr;
+    const cudaError_t e = af_dispatch(E, Lq, masked, [&](auto ep, auto ks, auto bias) {
+        return af_rooms<decltype(ep)::value, decltype(ks)::value, decltype(bias)::value>(ctx, room);
+    });
+    if (e != cudaSuccess) return true;   // the launch reports it
+    const int parts = af_parts(*room, nblk, items);
+    const bool wide = E <= 64 && Lq > 16;   // two query tiles
+    const Few& q = few[E > 64 ? 2 : wide][masked];
+    const int64_t ctas = items * parts, waves = parts > 1 ? 1 : cdiv(items, room->clusters[0]);
+    const double each = ctas <= (wide ? sms * 7 / 8 : sms) ? q.one : q.two * (double)waves;
+    const double here = q.start * (double)waves + (parts > 1 ? q.join : 0.0) + (Lq > 4 * parts ? q.finish : 0.0) + each * (double)cdiv(nblk, parts);
+    return here <= (masked ? 1.06 : 1.03) * there;   // past the fits' own error the simpler launch
 }
 
 int attention_few_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B, const b200_strided4* q,
@@ -380,12 +447,9 @@ int attention_few_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64
     p.E = (int)E; p.Lq = (int)Lq; p.Lk = (int)Lk;
     p.out_f32 = out_dtype == B200_F32;
     p.scale_log2 = scale * 1.4426950408889634f;
-    // Key parts: as many as keep every CTA resident at once (two per SM) with two blocks or more each.
-    const int64_t nblk = cdiv(Lk, AF_BC), room = 2 * (int64_t)ctx->prop.multiProcessorCount;
-    int parts = 1, most = AF_PARTS;
-    if (const char* f = getenv("B200_ATTENTION_PARTS")) most = atoi(f);   // debugging aid: the largest cluster to form
-    while (2 * parts <= most && 2 * parts * H * B <= room && nblk >= 4 * parts) parts *= 2;
-    return E <= 64 ? af_slots<64>(ctx, p, H, B, parts) : af_slots<128>(ctx, p, H, B, parts);
+    return af_dispatch(E, Lq, bias != nullptr, [&](auto ep, auto ks, auto masked) {
+        return af_launch<decltype(ep)::value, decltype(ks)::value, decltype(masked)::value>(ctx, p, H, B);
+    });
 }
 
 } // namespace b200

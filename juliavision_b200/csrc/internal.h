@@ -108,8 +108,10 @@ int attention_window_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
                             const b200_strided4* k, const b200_strided4* v, const b200_strided4* o, int out_dtype,
                             float scale);
 
-// Attention of at most 32 queries (attention_few.cu); operands as above, E <= 128.  bs: the mask's element strides
+// Attention of at most 32 queries, 16 above E = 64 (attention_few.cu), where that is faster than the large kernel;
+// operands as above, E <= 128.  bs: the mask's element strides
 // (keys, queries, heads, batch; 0 on a broadcast axis).
+bool attention_few_takes(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B, bool masked);
 int attention_few_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B, const b200_strided4* q,
                          const b200_strided4* k, const b200_strided4* v, const void* bias, const int64_t* bs,
                          const b200_strided4* o, int out_dtype, float scale);

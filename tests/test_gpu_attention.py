@@ -453,17 +453,20 @@ def test_the_heaviest_of_the_first_128_keys_is_not_rounded(ctx, Lk, first, best)
     assert err < 1.2e-5, err
 
 
-@pytest.mark.parametrize("B,H,Lq,Lk,E", [(1, 2, 300, 1500, 64), (1, 3, 40, 2000, 128)])
-def test_masked_calls_do_not_depend_on_the_workspace(ora, B, H, Lq, Lk, E):
-    """Shapes whose keys are split.  Recorded on a context that has no workspace yet, a masked call runs (unsplit); run
-    eagerly again and again without a reset, it leaves the workspace as it found it."""
+@pytest.mark.parametrize("B,H,Lq,Lk,E,masked", [(1, 2, 300, 1500, 64, True), (1, 3, 40, 2000, 128, True), (1, 36, 32, 4096, 64, False),
+                                                (1, 36, 16, 8192, 72, True)])
+def test_masked_calls_and_few_queries_do_not_depend_on_the_workspace(ora, B, H, Lq, Lk, E, masked):
+    """Shapes whose keys the large kernel splits.  Recorded on a context that has no workspace yet, a masked call and one of
+    few queries run (unsplit); run eagerly again and again without a reset, they leave the workspace as they found it."""
     rng = np.random.default_rng(Lq)
     q, k, v = (np.float16(rng.standard_normal((B, H, n, E))) for n in (Lq, Lk, Lk))
-    bias = np.float16(rng.standard_normal((1, 1, Lq, Lk)))
-    bias[rng.random(bias.shape) < 0.2] = -np.inf
+    bias = None
+    if masked:
+        bias = np.float16(rng.standard_normal((1, 1, Lq, Lk)))
+        bias[rng.random(bias.shape) < 0.2] = -np.inf
     ref = ora.attention_ref(q, k, v, 1 / np.sqrt(E), bias=bias)
     with jv.Ctx(0) as c:
-        dq, dk, dv, db = (c.toback(a) for a in (q, k, v, bias))
+        dq, dk, dv, db = (None if a is None else c.toback(a) for a in (q, k, v, bias))
         out = c.allocate(np.float32, E, Lq, H, B)
         call = lambda: jv.sdpa(c, dq, dk, dv, db, 1 / np.sqrt(E), out=out)
         c.fill_bytes(out, 0xFF)
@@ -481,6 +484,16 @@ def test_masked_calls_do_not_depend_on_the_workspace(ora, B, H, Lq, Lk, E):
         c.synchronize()
         assert c.ws.stats() == cap
         assert relerr(out.to_host(), ref) < 2e-3
+
+
+@pytest.mark.parametrize("B,H,Lq,Lk,E", FEW)
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("most", [16, 1])
+def test_few_queries_whatever_is_faster(ctx, ora, B, H, Lq, Lk, E, masked, most, monkeypatch):
+    """The shapes above on the kernel of few queries also where the large one is the faster, cut as far as the keys
+    allow and not at all."""
+    monkeypatch.setenv("B200_ATTENTION_PARTS", str(most))
+    test_few_queries_in_one_launch(ctx, ora, B, H, Lq, Lk, E, masked)
 
 
 @pytest.mark.parametrize("B,H,Lq,Lk,E", [(1, 2, 23, 4096, 64), (1, 3, 5, 4500, 128)])
