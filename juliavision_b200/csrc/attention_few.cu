@@ -394,7 +394,7 @@ template <typename F> static auto af_dispatch(int64_t E, int64_t Lq, bool masked
 // 32 queries, 16 to 8192 keys): the large kernel takes as long for 128 keys as this one for 64, but sets up tensor memory
 // and merges.  16 to 32 queries over up to 384 keys are its (20 heads, 32 x 128: 4.4 us there, 7.2 here; 32 x 256 5.7, 6.7),
 // and many heads over long keys with more than 16 queries (36 heads, 32 x 8192: 31, 36); up to 8 queries are nearly always
-// this one's (8 heads, 1 x 1000: 9.5, 5.0).  Over 4154 further shapes the choice leaves two more than 4 % behind the large
+// this one's (8 heads, 1 x 1000: 9.5, 5.0).  Over 4154 further shapes the choice leaves three more than 4 % behind the large
 // kernel, where taking every call here left 350, by up to three quarters.
 bool attention_few_takes(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B, bool masked) {
     if (Lq > (E <= 64 ? 32 : 16)) return false;
@@ -404,7 +404,7 @@ bool attention_few_takes(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64
     static const Large large[2][2] = {{{3.16, 2.76, 0.34, 1.42}, {3.04, 2.72, 0.37, 2.22}}, {{3.05, 2.72, 0.40, 2.22}, {2.95, 2.73, 0.41, 3.09}}};
     static const Few few[3][2] = {{{3.41, 0.84, 0.83, 0.46, 0.78}, {3.47, 1.08, 1.07, 0.86, 1.21}},
                                   {{6.17, -0.51, 0.33, 0.50, 0.99}, {5.77, -0.66, 0.15, 1.77, 2.60}},
-                                  {{4.58, 0.86, 0.79, 0.92, 1.52}, {3.90, 0.97, 1.16, 1.69, 2.46}}};
+                                  {{4.58, 0.86, 0.79, 0.92, 1.52}, {4.27, 1.10, 1.25, 1.41, 2.35}}};
     const int64_t items = H * B, sms = ctx->prop.multiProcessorCount, blocks = cdiv(Lk, 128), nblk = cdiv(Lk, AF_BC);
     const Large& m = large[E > 64][masked];
     double there = m.wave * (double)cdiv(items, sms) + m.block * (double)(blocks * cdiv(items, sms));
@@ -425,9 +425,11 @@ bool attention_few_takes(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64
     const bool wide = E <= 64 && Lq > 16;   // two query tiles
     const Few& q = few[E > 64 ? 2 : wide][masked];
     const int64_t ctas = items * parts, waves = parts > 1 ? 1 : cdiv(items, room->clusters[0]);
-    const double each = ctas <= (wide ? sms * 7 / 8 : sms) ? q.one : q.two * (double)waves;
-    const double here = q.start * (double)waves + (parts > 1 ? q.join : 0.0) + (Lq > 4 * parts ? q.finish : 0.0) + each * (double)cdiv(nblk, parts);
-    return here <= (masked ? 1.06 : 1.03) * there;   // past the fits' own error the simpler launch
+    // (further rounds start under the ones before; a CTA's walk is its own up to an SM each, the heavier ones' up to seven
+    // eighths of that: clusters do not spread evenly)
+    const double each = ctas <= (wide || (masked && E > 64) ? sms * 7 / 8 : sms) ? q.one : q.two * (double)waves;
+    const double here = q.start * 0.5 * (double)(waves + 1) + (parts > 1 ? q.join : 0.0) + (Lq > 4 * parts ? q.finish : 0.0) + each * (double)cdiv(nblk, parts);
+    return here <= 1.03 * there;   // within the fits' own error the simpler launch
 }
 
 int attention_few_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B, const b200_strided4* q,
