@@ -360,14 +360,15 @@ template <int EP, int KS, bool BIAS> static cudaError_t af_rooms(b200_ctx* ctx, 
 
 static const char* af_forced() { return getenv("B200_ATTENTION_PARTS"); }   // debugging aid: this kernel, with clusters up to that size
 
-// Key parts: as many, with two blocks or more each, as keep every cluster resident at once.  A second round of clusters
-// costs more than the shorter walk saves (17 heads, 25 x 2405: 15.7 us with sixteen parts, of which sixteen clusters fit).
-static int af_parts(const AfRoom& room, int64_t nblk, int64_t items) {
+// Key parts: as many, with two blocks or more each, as keep every cluster resident at once, two CTAs to an SM.  A second
+// round of clusters costs more than the shorter walk saves (17 heads, 25 x 2405: 15.7 us with sixteen parts, of which
+// sixteen clusters fit), and so does a third CTA on an SM (20 heads, 12 x 2003: 7.1 us with eight parts, 7.4 with sixteen).
+static int af_parts(const AfRoom& room, int64_t sms, int64_t nblk, int64_t items) {
     const char* f = af_forced();
     const int most = f ? atoi(f) : AF_PARTS;
     int parts = 1;
     for (int l = 1; l <= 4 && (1 << l) <= most && nblk >= 2 << l; ++l)
-        if (items <= room.clusters[l]) parts = 1 << l;
+        if (items <= room.clusters[l] && items << l <= 2 * sms) parts = 1 << l;
     return parts;
 }
 
@@ -375,7 +376,7 @@ template <int EP, int KS, bool BIAS>
 static int af_launch(b200_ctx* ctx, const FewParams& p, int64_t H, int64_t B) {
     const AfRoom* room;
     B200_CUDA((af_rooms<EP, KS, BIAS>(ctx, room)));
-    const int parts = af_parts(*room, cdiv(p.Lk, AF_BC), H * B);
+    const int parts = af_parts(*room, ctx->prop.multiProcessorCount, cdiv(p.Lk, AF_BC), H * B);
     B200_CUDA(launch_dep(attention_few_kernel<EP, KS, BIAS>, dim3((unsigned)parts, (unsigned)H, (unsigned)B), dim3(AF_THREADS, 1, 1),
                          AfCfg<EP, KS>::SMEM_BYTES, ctx->stream, parts, p));
     ctx->launches++;
@@ -421,7 +422,7 @@ bool attention_few_takes(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64
         return af_rooms<decltype(ep)::value, decltype(ks)::value, decltype(bias)::value>(ctx, room);
     });
     if (e != cudaSuccess) return true;   // the launch reports it
-    const int parts = af_parts(*room, nblk, items);
+    const int parts = af_parts(*room, sms, nblk, items);
     const bool wide = E <= 64 && Lq > 16;   // two query tiles
     const Few& q = few[E > 64 ? 2 : wide][masked];
     const int64_t ctas = items * parts, waves = parts > 1 ? 1 : cdiv(items, room->clusters[0]);

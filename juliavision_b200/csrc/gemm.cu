@@ -87,11 +87,12 @@ template <typename OutT> struct GemmParams {
 
 // Timeline slots written by worker 0 when tracing (b200_timeline): globaltimer ns at [slot] and
 // the SM's own cycle counter at [64 + slot], so a phase can be read both in time and in cycles (their
-// ratio is the clock the SM actually ran at).  One CTA writes, the grid's first: worker 0, a pair's leader, the first part
-// of a K split.  Costs one predictable branch per event otherwise.
+// ratio is the clock the SM actually ran at).  One CTA writes: a pair's leader, the first part of a K split (asked for behind
+// the branch: kept in a register for it, the part cost short launches 2 %).  Costs one predictable branch per event otherwise.
 #define GEMM_TRACE(slot)                                                   \
     do {                                                                   \
-        if (p.trace != nullptr && blockIdx.x == 0) {                       \
+        if (p.trace != nullptr && worker == 0 && rank == 0 &&              \
+            (!KSPLIT || cluster_ctarank() == 0)) {                         \
             p.trace[(slot)] = globaltimer_ns();                            \
             p.trace[64 + (slot)] = (unsigned long long)clock64();          \
         }                                                                  \
@@ -649,7 +650,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
         else tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
     }
     if (threadIdx.x == 0) GEMM_TRACE(16); // exit
-    if (threadIdx.x == 0 && rank == 0 && kpart == 0 && p.trace != nullptr && worker < 120)
+    if (threadIdx.x == 0 && rank == 0 && p.trace != nullptr && worker < 120 && (!KSPLIT || cluster_ctarank() == 0))
         p.trace[128 + worker] = globaltimer_ns();   // when each worker left, to see how evenly the work was dealt
 }
 

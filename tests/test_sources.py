@@ -31,7 +31,7 @@ def test_one_cta_of_a_worker_writes_the_timeline():
     assert len(writes) == 3
     for at in writes:
         guard = text[text.rindex("if (", 0, at):at]
-        assert "blockIdx.x == 0" in guard or all(c in guard for c in ("rank == 0", "kpart == 0", "worker")), guard
+        assert all(c in guard for c in ("rank == 0", "(!KSPLIT || cluster_ctarank() == 0)", "worker")), guard
 
 
 def test_what_the_runtime_is_asked_once_is_asked_of_the_right_device_by_one_thread():
