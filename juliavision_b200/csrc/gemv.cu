@@ -32,10 +32,10 @@ constexpr int GEMV_BLOCKS_PER_SM = 2;   // resident blocks of 512 threads at 64 
 constexpr int GEMV_SPLIT_MIN_K = 4096;  // (gemv_run)
 constexpr int GEMV_MIN_COLS = 8;        // columns per warp below which a further K split only adds the join
 
-// Pairwise sum.  With results kept in fp32 the columns of a warp are added two at a time as well: as one chain over them
-// and one over the warps, those results were up to 17 % further from 64 bits than with the fewer columns that a warp of
-// gemv_split_kernel takes (10428 x 429: 1.24e-7 against 1.06e-7).  Rounded to fp16 none of this shows, and there the
-// shorter chains would cost 2 to 4 % of the time.
+// Pairwise sum of the warps, and of the parts.  With results kept in fp32 and K over fewer than eight parts (PAIRS) a warp's
+// columns are added two at a time as well: as one chain over them and one over the warps, those results were up to 17 %
+// further from 64 bits than with the fewer columns that a warp of gemv_split_kernel takes (10428 x 429: 1.24e-7 against
+// 1.06e-7).  Eight parts leave a warp few enough (492 x 4415: 5.45 us, 5.68 in pairs), and rounded to fp16 none of this shows.
 template <int N> __device__ __forceinline__ float gemv_pairs(float (&v)[N]) {
 #pragma unroll
     for (int h = N / 2; h > 0; h /= 2)
@@ -56,7 +56,7 @@ template <int N> __device__ __forceinline__ float gemv_pairs(float (&v)[N]) {
 // previous column, the start of the next, or the rest of an aligned 16-byte block at either end of the
 // array) only reach accumulators that are thrown away; every vector read holds at least one element of
 // A, so no read leaves the 16-byte blocks the array occupies.
-template <typename T, typename OutT>
+template <typename T, typename OutT, bool PAIRS>
 __global__ void __launch_bounds__(32 * GEMV_WARPS, GEMV_BLOCKS_PER_SM)
 gemv_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const T* __restrict__ bias, OutT* __restrict__ out,
             int64_t M, int64_t K, int64_t kchunk, int epi) {
@@ -98,7 +98,7 @@ gemv_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ x, const
                     const T* f = reinterpret_cast<const T*>(&a[u + 1]);
 #pragma unroll
                     for (int v = 0; v < VEC; ++v) {
-                        if constexpr (sizeof(OutT) == 4) {   // two columns at a time: half the chain (see gemv_pairs)
+                        if constexpr (PAIRS) {   // two columns at a time: half the chain (see gemv_pairs)
                             acc[v] += fmaf(gemv_tof<T>(f[v]), xv[u + 1], gemv_tof<T>(e[v]) * xv[u]);
                         } else {
                             acc[v] = fmaf(gemv_tof<T>(e[v]), xv[u], acc[v]);
@@ -289,7 +289,8 @@ static int gemv_run(b200_ctx* ctx, int64_t M, int64_t K, const void* A, int64_t 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    B200_CUDA(cudaLaunchKernelEx(&cfg, gemv_kernel<T, OutT>, (const T*)A, lda, (const T*)x, (const T*)bias, (OutT*)out, M, K, kchunk, epi));
+    const auto kern = sizeof(OutT) == 4 && parts < 8 ? gemv_kernel<T, OutT, sizeof(OutT) == 4> : gemv_kernel<T, OutT, false>;
+    B200_CUDA(cudaLaunchKernelEx(&cfg, kern, (const T*)A, lda, (const T*)x, (const T*)bias, (OutT*)out, M, K, kchunk, epi));
     ctx->launches++;
     return B200_OK;
 }
