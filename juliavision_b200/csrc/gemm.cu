@@ -720,16 +720,31 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
     const double t_tile = 2.0, t_fix = 8.0;  // measured: partial dump + fence + flag + read-back
     TilePick best{256, 1, 0, 0, 1};
     double best_cost = 1e300;
+    // What a tile costs beside its k-blocks, fitted to 620 products of 100 to 530,000 tokens with K = 112 to 4600 timed on
+    // every tile (the tile chosen is 1.1% slower than the fastest in the mean; one t_tile for all of them is 2.5% slower).
+    // A launch of up to three rounds: t_tile, and a pair's set-up and hand-overs where a tile is only a few k-blocks long
+    // (1067 x 1224 x 144: 5.9 us on 128x2 tiles, 5.2 on 128x1; 18600 x 160 x 192: 6.6 on 256x2, 5.6 on 256x1), which
+    // show once, so not over several rounds of one feature tile (51442 x 184 x 168: 18.2 us on 256x1, 15.1 on 256x2).
+    // Over more rounds a tile's epilogue runs under the next one's main loop and only a part of it shows, less than
+    // half as much for half the columns (524288 x 336 x 112: 2.5 us a round on 256x2 tiles, 1.4 on 128x2).  The line is drawn once,
+    // by the rounds of the widest tile: drawn for each candidate it set tiles of a few long rounds, at the full t_tile,
+    // against tiles of many short ones (57732 x 736 x 216: 47.7 us on 128x2, 37.0 on 256x2).
+    // Rows of fp16 results that start off a 32-byte sector cost the wider tile more where it is short, unless the
+    // arithmetic of a GELU is what takes the time (46572 x 2408 x 128: 97.7 us on 256x2, 73.8 on 128x2; at 2432 features
+    // 62 on 256x2).
+    const bool many = cdiv(cdiv(M, 256) * cdiv(N, (int64_t)GEMM_BM * 2) * nbatch, (int64_t)(sms / 2)) >= 4;
+    const bool gelu = epilogue == B200_EPI_GELU || epilogue == B200_EPI_GELU_TANH;
+    const double ragged = nkb <= 4 && M % 16 != 0 && !gelu ? 0.5 : 0.0;
     for (const Cand& c : cands) {   // whole-tile schedules first: stream-K has to beat the best of them clearly
         const int64_t tiles = cdiv(M, c.bn) * cdiv(N, (int64_t)GEMM_BM * c.ncta) * nbatch;
         const int64_t waves = cdiv(tiles, (int64_t)(sms / c.ncta));
-        // One to three rounds: t_tile per round, and a pair's set-up and hand-overs show where a tile is only a few k-blocks
-        // long (1067 x 1224 x 144: 5.9 us on 128x2 tiles, 5.2 on 128x1; 18600 x 160 x 192: 6.6 on 256x2, 5.6 on 256x1).
-        // Over many rounds a tile's epilogue runs under the next one's main loop and only a part of it shows, less than
-        // half as much for half the columns (524288 x 336 x 112: 2.5 us a round on 256x2 tiles, 1.4 on 128x2; with four
-        // to fifteen rounds the same estimate picked worse tiles as often as better ones).
-        const bool many = waves >= 16;
-        const double tile = many ? (c.bn == 256 ? 1.3 : 0.5) : t_tile + (c.ncta == 2 && nkb <= 8 ? 0.4 : 0.0);
+        double tile;
+        if (many) {
+            tile = c.bn == 256 ? 1.6 + ragged : 0.7;
+        } else {
+            tile = t_tile;
+            if (c.ncta == 2 && nkb <= 8 && (waves == 1 || (waves <= 3 && cdiv(M, c.bn) > 1))) tile += 0.4;
+        }
         const double dp = (double)waves * ((double)nkb * c.t_kb + tile);
         if (dp < best_cost - 1e-9) {
             best_cost = dp;
@@ -749,7 +764,6 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
             const int64_t width = cdiv(cdiv(M, fm), 16) * 16;
             if (width > 256 && width <= 512) {
                 const double rel = (double)width / 256.0;
-                const bool gelu = epilogue == B200_EPI_GELU || epilogue == B200_EPI_GELU_TANH;
                 const double wide = 7.0 + (double)nkb * 0.3 * (rel < 1.25 ? 1.25 : rel) + (gelu ? 0.85 : 0.25) * (double)width / 64.0;
                 if (wide < 0.92 * best_cost) {
                     best_cost = wide;

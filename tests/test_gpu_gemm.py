@@ -246,6 +246,22 @@ def test_plans_made_by_several_threads_agree(ctx):
     assert any(p[2] > -(-M // p[1]) * -(-N // p[0]) for p, (M, N, K) in zip(want, shapes)), "no shape splits K here"
 
 
+@pytest.mark.parametrize("tokens,out,K,tile", [
+    (57732, 736, 216, (256, 256)),    # several rounds of wide tiles: every width is held to the same share of its epilogue
+    (131072, 336, 112, (256, 128)),   # a width that three narrow tiles cover and two wide ones overshoot
+    (46572, 2408, 128, (256, 128)),   # rows of results off 32-byte sectors, two k-blocks
+    (46572, 2432, 128, (256, 256)),   # the same on sectors
+    (7287, 528, 128, (128, 128)),     # one round: no pairs
+    (51442, 184, 168, (256, 256)),    # three rounds of one feature tile: pairs
+])
+def test_tiles_for_short_reductions(ctx, tokens, out, K, tile):
+    import ctypes as C
+    from juliavision_b200 import _lib
+    p = _lib.GemmPlan()
+    _lib.check(_lib.lib().b200_gemm_f16_plan(ctx.handle, out, tokens, K, 1, C.byref(p)))
+    assert (p.block_m, p.block_n) == tile
+
+
 def test_streamk_is_deterministic(ctx, monkeypatch):
     monkeypatch.setenv("B200_GEMM_TILE", "256x2s")
     rng = np.random.default_rng(77)
