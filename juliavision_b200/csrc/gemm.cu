@@ -720,19 +720,22 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
     const double t_tile = 2.0, t_fix = 8.0;  // measured: partial dump + fence + flag + read-back
     TilePick best{256, 1, 0, 0, 1};
     double best_cost = 1e300;
-    // What a tile costs beside its k-blocks, fitted to 620 products of 100 to 530,000 tokens with K = 112 to 4600 timed on
-    // every tile (the tile chosen is 1.1% slower than the fastest in the mean; one t_tile for all of them is 2.5% slower).
+    // What a tile costs beside its k-blocks, fitted to 1150 products of 8 to 300,000 tokens and 16 to 500,000 features, K = 1
+    // to 4600, timed on every tile (the tile chosen is 1.2% slower than the fastest in the mean; with one t_tile for
+    // all of them 2.1%).
     // A launch of up to three rounds: t_tile, and a pair's set-up and hand-overs where a tile is only a few k-blocks long
     // (1067 x 1224 x 144: 5.9 us on 128x2 tiles, 5.2 on 128x1; 18600 x 160 x 192: 6.6 on 256x2, 5.6 on 256x1), which
     // show once, so not over several rounds of one feature tile (51442 x 184 x 168: 18.2 us on 256x1, 15.1 on 256x2).
     // Over more rounds a tile's epilogue runs under the next one's main loop and only a part of it shows, less than
-    // half as much for half the columns (524288 x 336 x 112: 2.5 us a round on 256x2 tiles, 1.4 on 128x2).  The line is drawn once,
-    // by the rounds of the widest tile: drawn for each candidate it set tiles of a few long rounds, at the full t_tile,
-    // against tiles of many short ones (57732 x 736 x 216: 47.7 us on 128x2, 37.0 on 256x2).
+    // half as much for half the columns (524288 x 336 x 112: 2.5 us a round on 256x2 tiles, 1.4 on 128x2).  The line is
+    // drawn once, by the rounds of the widest tile: drawn for each candidate it set tiles of a few long rounds, at the full
+    // t_tile, against tiles of many short ones (57732 x 736 x 216: 47.7 us on 128x2, 37.0 on 256x2).  Rows of results of
+    // more than some 2500 features are written a tile's width at a time, and half the width costs as much: t_tile again
+    // (24 x 378840 x 8: 146 us on 128x1, 88 on 256x1).
     // Rows of fp16 results that start off a 32-byte sector cost the wider tile more where it is short, unless the
     // arithmetic of a GELU is what takes the time (46572 x 2408 x 128: 97.7 us on 256x2, 73.8 on 128x2; at 2432 features
     // 62 on 256x2).
-    const bool many = cdiv(cdiv(M, 256) * cdiv(N, (int64_t)GEMM_BM * 2) * nbatch, (int64_t)(sms / 2)) >= 4;
+    const bool many = M <= 2560 && cdiv(cdiv(M, 256) * cdiv(N, (int64_t)GEMM_BM * 2) * nbatch, (int64_t)(sms / 2)) >= 4;
     const bool gelu = epilogue == B200_EPI_GELU || epilogue == B200_EPI_GELU_TANH;
     const double ragged = nkb <= 4 && M % 16 != 0 && !gelu ? 0.5 : 0.0;
     for (const Cand& c : cands) {   // whole-tile schedules first: stream-K has to beat the best of them clearly
