@@ -193,6 +193,7 @@ int b200_conv2d_grouped_f16(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, in
     B200_REQUIRE(Cin % groups == 0 && Cout % groups == 0, B200_DECLINE_EXTENT, "conv2d: %lld groups do not divide the channels",
                  (long long)groups);
     B200_REQUIRE(out_dtype == B200_F16 || out_dtype == B200_F32, B200_DECLINE_ELTYPE, "conv2d: out dtype %d", out_dtype);
+    B200_REQUIRE(epilogue >= B200_EPI_NONE && epilogue <= B200_EPI_GELU_TANH, B200_EINVAL, "conv2d: epilogue %d", epilogue);
     const int64_t OW = convsize(W, KW, sx, px, dx), OH = convsize(H, KH, sy, py, dy);
     B200_REQUIRE(OW > 0 && OH > 0, B200_DECLINE_EXTENT, "conv2d: empty output");
     B200_CUDA(cudaSetDevice(ctx->device));

@@ -124,6 +124,16 @@ def test_a_weight_off_its_boundary_does_not_depend_on_the_workspace(ora, Cin, Co
         assert relerr(out.to_host(), ref) < 2e-5
 
 
+@pytest.mark.parametrize("side", [16, 17])      # through the GEMM, through the implicit kernel
+@pytest.mark.parametrize("epilogue", [-1, 4])
+def test_an_epilogue_that_does_not_exist_is_refused(ctx, side, epilogue):
+    from juliavision_b200 import _lib
+    x, w = ctx.toback(np.zeros((1, 8, side, side), np.float16)), ctx.toback(np.zeros((8, 8, 1, 1), np.float16))
+    out = ctx.allocate(np.float16, side, side, 8, 1)
+    rc = _lib.lib().b200_conv2d_f16(ctx.handle, side, side, 8, 1, 1, 1, 8, 1, 1, 0, 0, 1, 1, x.ptr, w.ptr, None, out.ptr, 0, epilogue)
+    assert rc == _lib.lib().b200_conv2d_f16(ctx.handle, side, side, 8, 1, 1, 1, 8, 0, 1, 0, 0, 1, 1, x.ptr, w.ptr, None, out.ptr, 0, 0) != 0
+
+
 def test_im2col_bit_exact(ctx, ora):
     import ctypes as C
     from juliavision_b200 import _lib
