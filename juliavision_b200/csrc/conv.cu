@@ -105,6 +105,20 @@ int b200_im2col_f16(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_t N,
     return B200_OK;
 }
 
+// A 1x1 convolution the tensor-core GEMM cannot run: the scalar GEMM (a launch per image, a thread per output) against
+// the implicit kernel, in microseconds as fitted to 350 of 40 to 450,000 pixels, 1 to 512 -> 8 to 1000 channels.  The first
+// starts sooner and multiplies one channel after the other (1 -> 88, 315 pixels: 3.9 us, implicit 6.5; 512 -> 88, 100 pixels:
+// 43, implicit 9.4); the second pays for whole tiles of 64, 128 or 256 channels (8 -> 8, 49284 pixels: 4.6 us, implicit
+// 9.4).  Taking the cheaper one is 0.3% off the faster of the two in the mean, always the implicit one was 10% off.
+static bool scalar_1x1_is_faster(b200_ctx* ctx, int64_t P, int64_t Cin, int64_t Cout, int64_t N) {
+    const int64_t sms = ctx->prop.multiProcessorCount, nkb = cdiv(Cin, 64), bn = Cout <= 64 ? 64 : (Cout <= 128 ? 128 : 256);
+    const int64_t waves = cdiv(cdiv(P, 128) * N * cdiv(Cout, bn), bn == 256 ? sms : 2 * sms);
+    const double scalar = (double)N * (1.8 + 0.077 * (double)Cin + (double)(P * Cout) * (3.2e-6 + 2.8e-7 * (double)Cin));
+    const double implicit = 2.8 + 0.0075 * (double)(Cout < 256 ? Cout : 256) + 0.8 * (double)waves +
+                            (double)nkb * (4.7 * (double)waves - 3.6);
+    return Cout < 65536 && scalar < implicit;
+}
+
 // One group of a convolution: Cin_g input channels starting at x (image n at x + n * x_img), Cout_g output
 // channels starting at out (image n at out + n * out_img elements), weight (KW,KH,Cin_g,Cout_g) dense.
 static int conv2d_group(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t KW, int64_t KH,
@@ -126,8 +140,16 @@ static int conv2d_group(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_
     // The implicit kernel where the GEMM cannot store the result, and where it has two pixel tiles per SM or more; a small
     // image the GEMM can store is as fast through a small im2col matrix (64 x 58 x 24 -> 64: 7.5 us, implicit 12).
     const bool aligned = P % 8 == 0 && out_img * osz % 16 == 0 && al16(out);   // the GEMM can store the result
+    const bool gemm_1x1 = onebyone && aligned && x_img % 8 == 0 && al16(x);
+    if (onebyone && !gemm_1x1 && scalar_1x1_is_faster(ctx, P, Cin, Cout, N)) {
+        for (int64_t n = 0; n < N; ++n)
+            if ((rc = gemm_f16_scalar_launch(ctx, P, Cout, Cin, x + n * x_img, P, w, Cin, bias, 1, (char*)out + (size_t)(n * out_img) * osz,
+                                             P, out_dtype, epilogue, 1, 0, 0, 0)))
+                return rc;
+        return B200_OK;
+    }
     bool implicit = conv_implicit_takes(W, H, Cin, N, KW, KH, Cout, P) &&
-                    (onebyone ? !(aligned && x_img % 8 == 0 && al16(x)) : !aligned || cdiv(P, 128) * N >= 2 * ctx->prop.multiProcessorCount);
+                    (onebyone ? !gemm_1x1 : !aligned || cdiv(P, 128) * N >= 2 * ctx->prop.multiProcessorCount);
     const size_t ws_mark = ctx->ws_used;
     const bool padded = CRS % 8 != 0;
     if (padded || (implicit && !al16(w))) {

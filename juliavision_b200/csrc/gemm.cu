@@ -1042,6 +1042,23 @@ int b200_gemm_f16(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A,
 
 namespace b200 {
 
+int gemm_f16_scalar_launch(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda, const void* B, int64_t ldb,
+                           const void* bias, int bias_per_n, void* out, int64_t ldo, int out_dtype, int epilogue, int64_t nbatch,
+                           int64_t strideA, int64_t strideB, int64_t strideO) {
+    dim3 grid((unsigned)cdiv(M, 128), (unsigned)N, (unsigned)nbatch), block(128);
+    if (out_dtype == B200_F16)
+        gemm_f16_scalar_kernel<__half><<<grid, block, 0, ctx->stream>>>(
+            M, N, K, (const __half*)A, lda, (const __half*)B, ldb, (const __half*)bias, bias_per_n, (__half*)out,
+            ldo, epilogue, strideA, strideB, strideO);
+    else
+        gemm_f16_scalar_kernel<float><<<grid, block, 0, ctx->stream>>>(
+            M, N, K, (const __half*)A, lda, (const __half*)B, ldb, (const __half*)bias, bias_per_n, (float*)out,
+            ldo, epilogue, strideA, strideB, strideO);
+    ctx->launches++;
+    B200_CUDA(cudaGetLastError());
+    return B200_OK;
+}
+
 int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda, const void* B,
                  int64_t ldb, const void* bias, int bias_per_n, void* out, int64_t ldo, int out_dtype,
                  int epilogue, int64_t nbatch, int64_t strideA, int64_t strideB, int64_t strideO, int use_workspace) {
@@ -1067,18 +1084,8 @@ int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, 
                      "gemm: unaligned operands with N or nbatch >= 65536");
         if (gemm_rows_takes(M, N, K, nbatch))
             return gemm_rows_launch(ctx, M, N, K, A, lda, B, ldb, bias, bias_per_n, out, ldo, out_dtype, epilogue);
-        dim3 grid((unsigned)cdiv(M, 128), (unsigned)N, (unsigned)nbatch), block(128);
-        if (out_dtype == B200_F16)
-            gemm_f16_scalar_kernel<__half><<<grid, block, 0, ctx->stream>>>(
-                M, N, K, (const __half*)A, lda, (const __half*)B, ldb, (const __half*)bias, bias_per_n, (__half*)out,
-                ldo, epilogue, strideA, strideB, strideO);
-        else
-            gemm_f16_scalar_kernel<float><<<grid, block, 0, ctx->stream>>>(
-                M, N, K, (const __half*)A, lda, (const __half*)B, ldb, (const __half*)bias, bias_per_n, (float*)out,
-                ldo, epilogue, strideA, strideB, strideO);
-        ctx->launches++;
-        B200_CUDA(cudaGetLastError());
-        return B200_OK;
+        return gemm_f16_scalar_launch(ctx, M, N, K, A, lda, B, ldb, bias, bias_per_n, out, ldo, out_dtype, epilogue, nbatch,
+                                      strideA, strideB, strideO);
     }
     const TilePick t = pick_tile(M, N, K, nbatch, ctx->prop.multiProcessorCount, ksplit_room(ctx), use_workspace != 0, epilogue);
 #define GEMM_GO(BN_, T_, NC_)                                                                                     \

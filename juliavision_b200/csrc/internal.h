@@ -124,6 +124,10 @@ int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, 
                  int64_t ldb, const void* bias, int bias_per_n, void* out, int64_t ldo, int out_dtype,
                  int epilogue, int64_t nbatch, int64_t strideA, int64_t strideB, int64_t strideO,
                  int use_workspace = 1);
+// The same on one thread per output, for operands at any alignment (N and nbatch below 65536).
+int gemm_f16_scalar_launch(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda, const void* B, int64_t ldb,
+                           const void* bias, int bias_per_n, void* out, int64_t ldo, int out_dtype, int epilogue, int64_t nbatch,
+                           int64_t strideA, int64_t strideB, int64_t strideO);
 
 // Convolution without a materialised im2col matrix (conv_implicit.cu).  w: (CRS, Cout), 16-byte aligned, leading
 // dimension ldw a multiple of 8; x and out at any alignment.

@@ -93,7 +93,7 @@ def test_conv_gathered_into_the_tiles(ctx, ora, N, Cin, H, W, Cout, KH, KW, stri
     assert relerr(got, ref) < tol, describe(got, ref, tol)
 
 
-@pytest.mark.parametrize("Cin,Cout,H,W", [(24, 40, 17, 19), (8, 257, 33, 31)])
+@pytest.mark.parametrize("Cin,Cout,H,W", [(136, 40, 17, 19), (72, 257, 33, 31)])
 def test_a_weight_off_its_boundary_does_not_depend_on_the_workspace(ora, Cin, Cout, H, W):
     """A 1x1 convolution of an odd image needs no scratch but for a weight that starts off a 16-byte boundary, which the
     implicit kernel wants copied.  Recorded on a context that has no workspace yet it runs all the same; in a loop
@@ -124,7 +124,7 @@ def test_a_weight_off_its_boundary_does_not_depend_on_the_workspace(ora, Cin, Co
         assert relerr(out.to_host(), ref) < 2e-5
 
 
-@pytest.mark.parametrize("side", [16, 17])      # through the GEMM, through the implicit kernel
+@pytest.mark.parametrize("side", [16, 17])      # an image the GEMM can store, one it cannot
 @pytest.mark.parametrize("epilogue", [-1, 4])
 def test_an_epilogue_that_does_not_exist_is_refused(ctx, side, epilogue):
     from juliavision_b200 import _lib
@@ -132,6 +132,26 @@ def test_an_epilogue_that_does_not_exist_is_refused(ctx, side, epilogue):
     out = ctx.allocate(np.float16, side, side, 8, 1)
     rc = _lib.lib().b200_conv2d_f16(ctx.handle, side, side, 8, 1, 1, 1, 8, 1, 1, 0, 0, 1, 1, x.ptr, w.ptr, None, out.ptr, 0, epilogue)
     assert rc == _lib.lib().b200_conv2d_f16(ctx.handle, side, side, 8, 1, 1, 1, 8, 0, 1, 0, 0, 1, 1, x.ptr, w.ptr, None, out.ptr, 0, 0) != 0
+
+
+# 1x1 convolutions of odd images: (N, Cin, H, W, Cout, whether the scalar GEMM takes them, a launch per image, rather than the
+# implicit kernel)
+@pytest.mark.parametrize("N,Cin,H,W,Cout,scalar", [(1, 1, 15, 21, 88, True), (1, 16, 45, 53, 96, True), (1, 40, 7, 9, 512, True),
+                                                   (2, 3, 321, 235, 8, True), (1, 40, 21, 25, 24, False), (4, 8, 7, 7, 64, False),
+                                                   (1, 512, 9, 11, 88, False), (1, 128, 51, 37, 64, False)])
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+def test_conv_1x1_of_odd_images(ctx, ora, N, Cin, H, W, Cout, scalar, dt):
+    rng = np.random.default_rng(Cin + Cout + W)
+    x = np.float16(rng.standard_normal((N, Cin, H, W)) * 0.5)
+    w = np.float16(rng.standard_normal((Cout, Cin, 1, 1)) * 0.2)
+    b = np.float16(rng.standard_normal(Cout) * 0.2)
+    before = ctx.launch_count()
+    got = conv_gpu(ctx, x, w, b, (1, 1), (0, 0), out_dtype=dt)
+    assert ctx.launch_count() - before == (N if scalar else 1)
+    # fp32 sums in another order (sqrt(Cin) eps32), then one fp16 rounding step
+    tol = 2e-3 if dt == np.float16 else 2e-5
+    ref = ora.conv2d(x, w, b, out_dtype=dt)
+    assert relerr(got, ref) < tol, describe(got, ref, tol)
 
 
 def test_im2col_bit_exact(ctx, ora):
