@@ -416,6 +416,145 @@ ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half*
     }
 }
 
+// Narrow rows (at most two vectors a lane) of launches of many waves: R rows per group of LPG lanes, so that a lane has R
+// or more 16-byte loads in flight (2 R with the residual add in front, ADD) and gamma and beta are read once for all of them.
+// Bound by HBM; with one row at a time the loads in flight were what bound it: 524288 x 112 fp16 69.0 -> 54.9 us (4.3 TB/s),
+// 131072 x 224 35.6 -> 29.9, 200000 x 200 53.0 -> 43.3; behind the add 524288 x 112 86.2 -> 78.9 (6.0 TB/s), 32768 x 448
+// 23.1 -> 20.6.  Eight rows lose (63.7: registers).  Alone, rows of two vectors a lane do not gain (32768 x 448 14.1 both
+// ways, 16384 x 448 7.1 -> 7.4) and stay with ln_warp_kernel.  A row is kept as read (fp16 stays packed,
+// also the sum x + h, which add.Tensor rounds to fp16), every operation and its order is that of the kernels
+// above, hence the same bits.  The R rows' statistics leave in one store each.
+template <typename InT, typename OutT, int VPL, int LPG, int R, bool ADD>
+__global__ void __launch_bounds__(128)
+ln_rows_kernel(const InT* a, InT* x, const InT* __restrict__ h, OutT* __restrict__ out, float* __restrict__ mean,
+               float* __restrict__ rstd, const InT* __restrict__ gamma, const InT* __restrict__ beta, int64_t groups, int C,
+               float eps, int use_clamp, float lo, float hi) {
+    constexpr int VN = Vec16<InT>::N;
+    constexpr int SIDE = 32 / LPG;   // rows side by side in a warp
+    static_assert(LPG == 32 || VPL == 1, "only single-vector groups share a warp");
+    static_assert(R <= LPG, "a lane per row writes the statistics");
+    const int lane = threadIdx.x & (LPG - 1);
+    const int64_t row0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (R * SIDE) + (threadIdx.x & 31) / LPG;
+    const int nvec = C / VN;
+    grid_dep_wait();     // the rows are the previous kernel's output
+    grid_dep_launch();
+    Vec16<InT> v[R][VPL], hv[ADD ? R : 1][ADD ? VPL : 1];
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+            const int64_t g = row0 + k * SIDE;
+            const int vi = lane + 32 * i;
+            if (vi < nvec && g < groups) {
+                v[k][i].raw = *(reinterpret_cast<const uint4*>((ADD ? x : a) + g * C) + vi);
+                if constexpr (ADD) hv[k][i].raw = __ldg(reinterpret_cast<const uint4*>(h + g * C) + vi);
+            } else {
+                v[k][i].raw = make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
+    Vec16<InT> gw[VPL], bw[VPL];
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+        const int vi = lane + 32 * i;
+        gw[i].raw = (gamma && vi < nvec) ? __ldg(reinterpret_cast<const uint4*>(gamma) + vi) : make_uint4(0u, 0u, 0u, 0u);
+        bw[i].raw = (beta && vi < nvec) ? __ldg(reinterpret_cast<const uint4*>(beta) + vi) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    float mu[R], r[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+            const int vi = lane + 32 * i;
+            if (vi < nvec) {
+                float f[VN];
+                v[k][i].to_f32(f);
+                if constexpr (ADD) {
+                    float fh[VN];
+                    hv[k][i].to_f32(fh);
+#pragma unroll
+                    for (int j = 0; j < VN; ++j) {
+                        f[j] = __half2float(__float2half_rn(f[j] + fh[j]));        // add.Tensor rounds here
+                        if (use_clamp) f[j] = __half2float(__float2half_rn(fminf(fmaxf(f[j], lo), hi)));
+                    }
+                    store_vec<VN>(reinterpret_cast<InT*>(&v[k][i].raw), f);         // exact: already fp16 values
+                    if (row0 + k * SIDE < groups)
+                        *(reinterpret_cast<uint4*>(x + (row0 + k * SIDE) * C) + vi) = v[k][i].raw;
+                }
+#pragma unroll
+                for (int j = 0; j < VN; ++j) s += f[j];
+            }
+        }
+        mu[k] = s;
+    }
+#pragma unroll
+    for (int o = LPG / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < R; ++k) mu[k] += __shfl_xor_sync(0xffffffffu, mu[k], o);
+    const float n = (float)C;
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        mu[k] /= n;
+        float s2 = 0.f;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i)
+            if (lane + 32 * i < nvec) {
+                float f[VN];
+                v[k][i].to_f32(f);
+#pragma unroll
+                for (int j = 0; j < VN; ++j) {
+                    const float d = f[j] - mu[k];
+                    s2 = fmaf(d, d, s2);
+                }
+            }
+        r[k] = s2;
+    }
+#pragma unroll
+    for (int o = LPG / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < R; ++k) r[k] += __shfl_xor_sync(0xffffffffu, r[k], o);
+#pragma unroll
+    for (int k = 0; k < R; ++k) r[k] = 1.0f / sqrtf(r[k] / n + eps);
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+        const int vi = lane + 32 * i;
+        float gf[VN], bf[VN];
+        gw[i].to_f32(gf);
+        bw[i].to_f32(bf);
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const int64_t g = row0 + k * SIDE;
+            if (vi < nvec && g < groups) {
+                float y[VN];
+                v[k][i].to_f32(y);
+#pragma unroll
+                for (int j = 0; j < VN; ++j) y[j] = (y[j] - mu[k]) * r[k];
+                if (gamma) {
+#pragma unroll
+                    for (int j = 0; j < VN; ++j) y[j] = __fmul_rn(y[j], gf[j]);
+                }
+                if (beta) {
+#pragma unroll
+                    for (int j = 0; j < VN; ++j) y[j] = __fadd_rn(y[j], bf[j]);
+                }
+                store_vec<VN>(out + g * C + (int64_t)vi * VN, y);
+            }
+        }
+    }
+    float m = mu[0], q = r[0];
+#pragma unroll
+    for (int k = 1; k < R; ++k)
+        if (lane == k) {
+            m = mu[k];
+            q = r[k];
+        }
+    const int64_t g = row0 + lane * SIDE;
+    if (lane < R && g < groups) {
+        mean[g] = m;
+        rstd[g] = q;
+    }
+}
+
 __device__ __forceinline__ float ldf(const __half* p, int64_t i) { return __half2float(p[i]); }
 __device__ __forceinline__ float ldf(const float* p, int64_t i) { return p[i]; }
 __device__ __forceinline__ void stf(__half* p, int64_t i, float v) { p[i] = __float2half_rn(v); }
@@ -562,6 +701,12 @@ static bool ln_packs(int64_t groups, int64_t C) { return groups * C >= (int64_t)
 // instructions save; five and six gain (50000 x 1280: 51.8 -> 49.1, 43000 x 1480: 55.2 -> 52.1).
 constexpr bool ln_pack_width(int vpl) { return vpl == 5 || vpl == 6; }
 
+// Rows of one vector a lane, `lpg` lanes each: four of them per group of lanes while that leaves eight blocks an SM, else two
+// (3000 x 112: 3.42 us one at a time, 3.04 two, 3.12 four; 524288 x 112: 69.0, 61.7, 54.9).
+static bool ln_four_rows(const b200_ctx* ctx, int64_t groups, int lpg) {
+    return groups >= (int64_t)8 * ctx->prop.multiProcessorCount * 4 * 4 * (32 / lpg);
+}
+
 template <typename InT, typename OutT>
 static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, void* out, float* mean,
                      float* rstd, const void* gamma, const void* beta, float eps) {
@@ -595,12 +740,27 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
             B200_CUDA(launch_dep(ln_warp_kernel<InT, OutT, V>, grid, block, 0, ctx->stream, 1, ap, op, mean, rstd, gp, bp, \
                                  groups, (int)C, eps));                                                     \
     } while (0)
+#define LN_GO_LAT(V)                                                                                        \
+    B200_CUDA(launch_dep(ln_warp_kernel<InT, OutT, V, 32, true>, grid, block, 0, ctx->stream, 1, ap, op, mean, rstd, gp, bp, \
+                         groups, (int)C, eps))
 #define LN_GO_SHARED(L)                                                                                     \
     B200_CUDA(launch_dep(ln_warp_kernel<InT, OutT, 1, L>, dim3((unsigned)cdiv(groups, wpb * (32 / L))), block, 0,   \
                          ctx->stream, 1, ap, op, mean, rstd, gp, bp, groups, (int)C, eps))
-        if (nvec <= 8) LN_GO_SHARED(8);
+#define LN_GO_ROWS(V, L, R)                                                                                 \
+    B200_CUDA(launch_dep(ln_rows_kernel<InT, OutT, V, L, R, false>, dim3((unsigned)cdiv(groups, wpb * R * (32 / L))), block, 0, \
+                         ctx->stream, 1, ap, (InT*)nullptr, (const InT*)nullptr, op, mean, rstd, gp, bp, groups, (int)C, eps, 0, \
+                         0.f, 0.f))
+#define LN_GO_ROWS1(L)                                                                                      \
+    do {                                                                                                    \
+        if (ln_four_rows(ctx, groups, L)) LN_GO_ROWS(1, L, 4);                                              \
+        else LN_GO_ROWS(1, L, 2);                                                                           \
+    } while (0)
+        if (!lat && nvec <= 8) LN_GO_ROWS1(8);
+        else if (!lat && nvec <= 16) LN_GO_ROWS1(16);
+        else if (!lat && vpl <= 1) LN_GO_ROWS1(32);
+        else if (nvec <= 8) LN_GO_SHARED(8);
         else if (nvec <= 16) LN_GO_SHARED(16);
-        else if (vpl <= 1) LN_GO(1);
+        else if (vpl <= 1) LN_GO_LAT(1);
         else if (vpl <= 2) LN_GO(2);
         else if (vpl <= 3) LN_GO(3);
         else if (vpl <= 4) LN_GO(4);
@@ -617,6 +777,9 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
                                  op, mean, rstd, gp, bp, (int)C, eps));
 #undef LN_GO
 #undef LN_GO_SHARED
+#undef LN_GO_LAT
+#undef LN_GO_ROWS
+#undef LN_GO_ROWS1
     } else {
         ln_block_kernel<InT, OutT><<<(unsigned)groups, 256, 0, ctx->stream>>>(ap, op, mean, rstd, gp, bp,
                                                                              C, eps);
@@ -668,14 +831,30 @@ extern "C" int b200_add_layernorm_f16(b200_ctx* ctx, int64_t groups, int64_t C, 
                                  (__half*)out, mean, rstd, (const __half*)gamma, (const __half*)beta, groups, (int)C, eps, \
                                  use_clamp, lo, hi));                                                             \
     } while (0)
+#define LNA_GO_LAT(V)                                                                                             \
+    B200_CUDA(launch_dep(ln_add_warp_kernel<V, 32, true>, grid, block, 0, ctx->stream, 1, (__half*)x, (const __half*)h, (__half*)out, \
+                         mean, rstd, (const __half*)gamma, (const __half*)beta, groups, (int)C, eps, use_clamp, lo, hi))
 #define LNA_GO_SHARED(L)                                                                                          \
     B200_CUDA(launch_dep(ln_add_warp_kernel<1, L>, dim3((unsigned)cdiv(groups, wpb * (32 / L))), block, 0, ctx->stream, 1, \
                          (__half*)x, (const __half*)h, (__half*)out, mean, rstd, (const __half*)gamma,             \
                          (const __half*)beta, groups, (int)C, eps, use_clamp, lo, hi))
-    if (nvec <= 8) LNA_GO_SHARED(8);
+#define LNA_GO_ROWS(V, L, R)                                                                                      \
+    B200_CUDA(launch_dep(ln_rows_kernel<__half, __half, V, L, R, true>, dim3((unsigned)cdiv(groups, wpb * R * (32 / L))), block, 0, \
+                         ctx->stream, 1, (const __half*)nullptr, (__half*)x, (const __half*)h, (__half*)out, mean, rstd, \
+                         (const __half*)gamma, (const __half*)beta, groups, (int)C, eps, use_clamp, lo, hi))
+#define LNA_GO_ROWS1(L)                                                                                           \
+    do {                                                                                                          \
+        if (ln_four_rows(ctx, groups, L)) LNA_GO_ROWS(1, L, 4);                                                   \
+        else LNA_GO_ROWS(1, L, 2);                                                                                \
+    } while (0)
+    if (!lat && nvec <= 8) LNA_GO_ROWS1(8);
+    else if (!lat && nvec <= 16) LNA_GO_ROWS1(16);
+    else if (!lat && vpl <= 1) LNA_GO_ROWS1(32);
+    else if (!lat && vpl <= 2) LNA_GO_ROWS(2, 32, 2);
+    else if (nvec <= 8) LNA_GO_SHARED(8);
     else if (nvec <= 16) LNA_GO_SHARED(16);
-    else if (vpl <= 1) LNA_GO(1);
-    else if (vpl <= 2) LNA_GO(2);
+    else if (vpl <= 1) LNA_GO_LAT(1);
+    else if (vpl <= 2) LNA_GO_LAT(2);
     else if (vpl <= 3) LNA_GO(3);
     else if (vpl <= 4) LNA_GO(4);
     else if (vpl <= 5) LNA_GO(5);
@@ -685,6 +864,9 @@ extern "C" int b200_add_layernorm_f16(b200_ctx* ctx, int64_t groups, int64_t C, 
     else LNA_GO(16);
 #undef LNA_GO
 #undef LNA_GO_SHARED
+#undef LNA_GO_LAT
+#undef LNA_GO_ROWS
+#undef LNA_GO_ROWS1
     ctx->launches++;
     B200_CUDA(cudaGetLastError());
     return B200_OK;

@@ -148,3 +148,42 @@ def test_only_the_widths_that_gain_take_the_packed_form(ctx, C, same):
     large = layernorm_gpu(ctx, np.tile(part, (-(-_packed_rows(C) // 4096), 1)), gam, bet, 1e-5)
     equal = [np.array_equal(a, b[:len(a)]) for a, b in zip(small, large)]
     assert equal == [True] * 3 if same else not all(equal)
+
+
+@pytest.mark.parametrize("dt,C,groups", [(np.float16, 8, 2369), (np.float16, 64, 75779), (np.float16, 72, 37887), (np.float16, 112, 37891),
+                                         (np.float16, 128, 2371), (np.float16, 136, 18943), (np.float16, 256, 18947),
+                                         (np.float32, 28, 37889), (np.float32, 128, 18945), (np.float16, 264, 2369),
+                                         (np.float16, 512, 2370)])
+def test_several_narrow_rows_at_a_time(ctx, ora, dt, C, groups):
+    """Widths at both ends of a row's lanes, row counts that leave a last group short and on either side of the rule for
+    four rows: the oracle's values, and bit for bit what one row at a time (a launch of few rows) gives; with fp16 also
+    behind the residual add."""
+    rng = np.random.default_rng(C + groups)
+    a = (rng.standard_normal((groups, C), dtype=np.float32) * 2 + 0.5).astype(dt)
+    gam, bet = ((o + 0.1 * rng.standard_normal(C)).astype(dt) for o in (1, 0))
+    part = slice(groups - 1999, groups)
+    for g, b in ((gam, bet), (gam, None), (None, bet)):
+        got, mean, rstd = layernorm_gpu(ctx, a, g, b, 1e-5)
+        few, fmean, frstd = layernorm_gpu(ctx, np.ascontiguousarray(a[part]), g, b, 1e-5)
+        assert np.array_equal(got[part], few) and np.array_equal(mean[part], fmean) and np.array_equal(rstd[part], frstd)
+    ref, rmean, rrstd = ora.layernorm(a[part], None, bet, 1e-5, out_dtype=dt)
+    tol = 1.5e-3 if dt == np.float16 else 2e-6      # as above: a few fp32 ulps of the sums, at most one output ulp
+    assert relerr(few, ref) < tol, describe(few, ref, tol)
+    assert np.max(np.abs(fmean - rmean)) < 1e-5 and relerr(frstd, rrstd) < 1e-5
+    if dt != np.float16:
+        return
+    h0 = rng.standard_normal((groups, C), dtype=np.float32).astype(dt)
+    gd, bd = ctx.toback(gam), ctx.toback(bet)
+    for clamp in (None, (-1.5, 2.0)):
+        xa, xb, ha = ctx.toback(a), ctx.toback(a), ctx.toback(h0)
+        m1, r1, m2, r2 = (ctx.allocate(np.float32, groups) for _ in range(4))
+        oa, ob = ctx.allocate(dt, C, groups), ctx.allocate(dt, C, groups)
+        jv.add_(ctx, xa, xa, ha)
+        if clamp:
+            jv.clamp_(ctx, xa, xa, *clamp)
+        jv.layernorm_(ctx, oa, m1, r1, xa, gd, bd, C, 1e-5)
+        ctx.fill_bytes(ob, 0xFF)
+        jv.add_layernorm_(ctx, ob, m2, r2, xb, ha, gd, bd, C, 1e-5, clamp=clamp)
+        ctx.synchronize()
+        for one, other in ((xa, xb), (oa, ob), (m1, m2), (r1, r2)):
+            assert np.array_equal(one.to_host(), other.to_host())
