@@ -21,6 +21,8 @@
 #include <stdio.h>
 #include <stdlib.h>
 
+#include <type_traits>
+
 #include "act.cuh"
 #include "internal.h"
 #include "ptx.cuh"
@@ -42,7 +44,7 @@ constexpr int SMEM_LIMIT = 232448; // 227 KB
 //           per K step (256 columns + the rest), the tile's width a launch parameter (a multiple of 16 in
 //           (256, 512]).  It is for launches whose 256-wide tiles would need a second, mostly empty round of
 //           the workers: the width is chosen so that every tile is some worker's only one.
-template <int BN, typename OutT, int NCTA> struct GemmCfg {
+template <int BN, typename OutT, int NCTA, int GC = 16> struct GemmCfg {
     static constexpr bool WIDE = BN == 512;
     static_assert(!WIDE || NCTA == 2, "the wide tile is built for CTA pairs");
     static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
@@ -50,9 +52,11 @@ template <int BN, typename OutT, int NCTA> struct GemmCfg {
     static constexpr int B_COLS = BN / NCTA;               // feature columns this CTA stages
     static constexpr int B_BYTES = B_COLS * GEMM_BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int OUT_COLS = 128 / (int)sizeof(OutT); // columns per 128-byte staging row
-    static constexpr int SUB_COLS = 64 / (int)sizeof(OutT);   // epilogue slab: 64 bytes of output per row
-    static constexpr int TAIL_BYTES = EPI_WARPS * (BN / (EPI_WARPS / 4) * 4 + 32 * 16 * (int)sizeof(OutT)) + 256; // per-warp fp32 bias of its own columns and one staged chunk; barriers
+    // the epilogue's slabs, one per warp: 32 rows of GC output columns, behind them each warp's bias of its own columns
+    // (fp32; fp16 beside the wide slabs, which would cost a stage otherwise) and the barriers
+    static constexpr int SLAB_BYTES = 32 * GC * (int)sizeof(OutT);
+    static constexpr int BIAS_BYTES = BN / (EPI_WARPS / 4) * (GC == 16 ? 4 : 2);
+    static constexpr int TAIL_BYTES = EPI_WARPS * (SLAB_BYTES + BIAS_BYTES) + 256;
     static constexpr int STAGES_RAW = (SMEM_LIMIT - TAIL_BYTES) / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + TAIL_BYTES;
@@ -62,8 +66,8 @@ template <int BN, typename OutT, int NCTA> struct GemmCfg {
     static_assert(SMEM_BYTES <= SMEM_LIMIT, "shared memory over budget");
     static_assert(TMEM_COLS == 128 || TMEM_COLS == 256 || TMEM_COLS == 512, "TMEM columns");
     static_assert(B_COLS % 64 == 0, "each CTA stages whole 64-column slabs of B");
-    static_assert((EPI_WARPS * (BN / (EPI_WARPS / 4)) * 4) % 512 == 0 && (STAGES * STAGE_BYTES) % 1024 == 0,
-                  "the epilogue slabs must start on the swizzle pattern's period");
+    static_assert((STAGES * STAGE_BYTES) % 1024 == 0, "the epilogue slabs must start on the swizzle pattern's period");
+    static_assert(GC == 16 || (sizeof(OutT) == 2 && !WIDE && BN / (EPI_WARPS / 4) % GC == 0), "slabs of whole column groups");
 };
 
 template <typename OutT> struct GemmParams {
@@ -180,13 +184,13 @@ __device__ __forceinline__ void st_release_gpu(int* p, int v) {
 // accumulators are laid over the drained operand ring and every CTA finishes its share of the tile's chunks from all
 // of them, read through distributed shared memory and added in rank order: no workspace, no flags, and a hand-off of
 // a cluster barrier where the stream-K one through L2 costs ~6 us.
-template <int BN, typename OutT, int NCTA, bool KSPLIT>
+template <int BN, typename OutT, int NCTA, bool KSPLIT, int GC>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, tokens, batch}
                    const __grid_constant__ CUtensorMap tmapW,   // A(M,K): {features, K, batch}
-                   const __grid_constant__ CUtensorMap tmapO,   // out(M,N): {features, tokens, batch}, boxes of 16 x 32
+                   const __grid_constant__ CUtensorMap tmapO,   // out(M,N): {features, tokens, batch}, boxes of GC x 32
                    const GemmParams<OutT> p) {
-    using Cfg = GemmCfg<BN, OutT, NCTA>;
+    using Cfg = GemmCfg<BN, OutT, NCTA, GC>;
     constexpr int TILE_N = GEMM_BM * NCTA; // tokens per tile
     // The swizzled tiles need a 1024-byte aligned base.  The declaration asks for it; should a
     // toolchain not honour that, every thread of the grid sees the same misaligned offset and
@@ -197,8 +201,9 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
         if (threadIdx.x == 0) atomicCAS(p.d_status, 0, KST_SMEM_LAYOUT);
         return;
     }
-    __half* sbias = reinterpret_cast<__half*>(smem + Cfg::STAGES * Cfg::STAGE_BYTES);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(sbias) + EPI_WARPS * (BN / (EPI_WARPS / 4) * 4 + 32 * 16 * (int)sizeof(OutT)));
+    uint8_t* slabs = smem + Cfg::STAGES * Cfg::STAGE_BYTES;
+    uint8_t* sbias = slabs + EPI_WARPS * Cfg::SLAB_BYTES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sbias + EPI_WARPS * Cfg::BIAS_BYTES);
     uint64_t* full = bars;                     // [STAGES]  (pair: only the leader's are used)
     uint64_t* empty = bars + Cfg::STAGES;      // [STAGES]
     uint64_t* tfull = bars + 2 * Cfg::STAGES;  // [2]
@@ -390,24 +395,24 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
         }
     } else {
         // ---------------------------------------------------------------- epilogue
-        // Sixteen warps, four per TMEM lane quadrant, each taking every fourth chunk of 16 columns.
-        // Per chunk: tcgen05.ld -> +bias, round, activation -> a warp-private shared slab (32 rows x 16
-        // columns, plain rows) -> one bulk tensor store of the 16 x 32 box, clipped at the ragged edges
+        // Sixteen warps, four per TMEM lane quadrant, each taking every fourth group of GC columns.
+        // Per group: tcgen05.ld -> +bias, round, activation -> a warp-private shared slab (32 rows x GC
+        // columns) -> one bulk tensor store of the GC x 32 box, clipped at the ragged edges
         // of the output.  Each step is a short dependent chain, so the throughput comes from the four
-        // warps per scheduler taking turns; warps never wait for one another.  What bounds a tile's ~4000 cycles
-        // here is the SM's way out to L2, ~23 bytes per clock measured (64 KB of fp16 per CTA and tile): wider
-        // chunks, two slabs per warp and stores straight from registers were each built and measured slower.
-        constexpr int CH = 16;                 // columns per chunk (one tcgen05.ld.32x32b.x16)
+        // warps per scheduler taking turns; warps never wait for one another.
+        constexpr int CH = GC >= 32 ? 32 : 16; // columns per chunk (one tcgen05.ld)
+        constexpr int CPG = GC / CH;           // chunks of a group
         constexpr int NPART = EPI_WARPS / 4;   // warps sharing a lane quadrant
         constexpr int NCH = BN / NPART / CH;   // chunks one warp owns of a tile
-        constexpr int RB = CH * (int)sizeof(OutT);  // staged bytes per row and chunk
+        constexpr int RB = GC * (int)sizeof(OutT);  // staged bytes per row and group
+        using BiasT = std::conditional_t<GC == 16, float, __half>;
         const int ew = warp - 2;               // 0..15
         const int quad = warp & 3;             // TMEM lane quadrant this warp may read
-        const int part = ew >> 2;              // which chunks of the quadrant's rows
+        const int part = ew >> 2;              // which groups of the quadrant's rows
         const int row = quad * 32 + lane;      // token row inside this CTA's half of the tile
-        uint8_t* wstg = reinterpret_cast<uint8_t*>(sbias) + EPI_WARPS * (BN / NPART) * 4 + ew * (32 * RB);
-        float* wbias = reinterpret_cast<float*>(sbias) + ew * (BN / NPART);   // fp32 bias of this warp's own columns
-        auto chunk_col = [&](int c) { return (NPART * c + part) * CH; };
+        uint8_t* wstg = slabs + ew * Cfg::SLAB_BYTES;
+        BiasT* wbias = reinterpret_cast<BiasT*>(sbias + ew * Cfg::BIAS_BYTES);   // bias of this warp's own columns
+        auto chunk_col = [&](int c) { return (NPART * (c / CPG) + part) * GC + (c % CPG) * CH; };
         int it = 0;
         SegIter seg;
         for (seg.init(p.total_tiles, p.num_kb, p.streamk, worker, nworkers); seg.valid(); seg.next(), ++it) {
@@ -459,7 +464,9 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
             __syncwarp(); // the previous tile's readers of wbias are done
             for (int j = lane; j < BN / NPART; j += 32) {   // wbias[c*CH + t] = bias of column chunk_col(c) + t
                 const int col = chunk_col(j / CH) + (j % CH);
-                wbias[j] = (p.bias != nullptr && !p.bias_per_n && m0 + col < p.M) ? __half2float(p.bias[m0 + col]) : 0.f;
+                const __half b = (p.bias != nullptr && !p.bias_per_n && m0 + col < p.M) ? p.bias[m0 + col] : __float2half_rn(0.f);
+                if constexpr (GC == 16) wbias[j] = __half2float(b);
+                else wbias[j] = b;
             }
             const bool row_bias = !contributor && p.bias != nullptr && p.bias_per_n;   // the finisher adds the bias
             const float rbias = (row_bias && n0 + row < p.N) ? __half2float(p.bias[n0 + row]) : 0.f;
@@ -472,10 +479,10 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
             const uint32_t tacc = tmem_base + (uint32_t(quad * 32) << 16) + acc * BN;
             const int act_kind = p.epilogue;
             uint8_t* rowp = wstg + lane * RB;
-            // The slab's rows are 32 B (fp16) or 64 B (fp32) apart, so lanes four (two) apart would hit the same
+            // The slab's rows are 32, 64 or 128 B apart, so lanes four (two, one) apart would hit the same
             // banks.  The store map swizzles at that width (16-byte chunk index ^= address bits from 7 up), which
-            // spreads a warp's 16-byte stores over all banks: four wavefronts per instruction instead of eight.
-            const int swz = RB == 32 ? ((lane >> 2) & 1) : ((lane >> 1) & 3);
+            // spreads a warp's 16-byte stores over all banks: four wavefronts per instruction.
+            const int swz = RB == 32 ? ((lane >> 2) & 1) : (RB == 64 ? ((lane >> 1) & 3) : (lane & 7));
 
             // KSPLIT: the accumulator over the operand ring, [chunk][quarter][row] of 16 bytes
             const uint32_t dump = smem_u32(smem) + row * 16;
@@ -514,7 +521,8 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
                     }
                 } else {
                     uint32_t r[CH];
-                    tmem_ld16(tacc + col0, r);
+                    if constexpr (CH == 32) tmem_ld32(tacc + col0, r);
+                    else tmem_ld16(tacc + col0, r);
                     tmem_wait_ld();
 #pragma unroll
                     for (int t = 0; t < CH; ++t) v[t] = __uint_as_float(r[t]);
@@ -555,20 +563,33 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
                         }
                     }
                 }
-                if (m0 + col0 >= p.M || rows_valid <= 0 || (Cfg::WIDE && col0 >= p.bn)) continue; // nothing to write to the output
+                // nothing of this group to write to the output
+                if (m0 + col0 - (c % CPG) * CH >= p.M || rows_valid <= 0 || (Cfg::WIDE && col0 >= p.bn)) continue;
 
-                // the engine must have read the previous chunk out of the slab before it is overwritten; that
+                // the engine must have read the previous group out of the slab before it is overwritten; that
                 // read ran under this chunk's tcgen05.ld and arithmetic
-                if (lane == 0) tma_store_wait_read<0>();
-                __syncwarp();
+                if (c % CPG == 0) {
+                    if (lane == 0) tma_store_wait_read<0>();
+                    __syncwarp();
+                }
                 // registers -> shared, lane = row
-                const float* bc = wbias + c * CH;
+                const BiasT* bc = wbias + c * CH;
                 if constexpr (sizeof(OutT) == 2) {
                     auto emit = [&](auto act) {
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) {
-                            const float4 b0 = *reinterpret_cast<const float4*>(bc + j * 8);
-                            const float4 b1 = *reinterpret_cast<const float4*>(bc + j * 8 + 4);
+                        for (int j = 0; j < CH / 8; ++j) {
+                            float4 b0, b1;
+                            if constexpr (GC == 16) {
+                                b0 = *reinterpret_cast<const float4*>(bc + j * 8);
+                                b1 = *reinterpret_cast<const float4*>(bc + j * 8 + 4);
+                            } else {
+                                const uint4 w = *reinterpret_cast<const uint4*>(bc + j * 8);
+                                const __half2* h2 = reinterpret_cast<const __half2*>(&w);
+                                const float2 f0 = __half22float2(h2[0]), f1 = __half22float2(h2[1]), f2 = __half22float2(h2[2]),
+                                             f3 = __half22float2(h2[3]);
+                                b0 = make_float4(f0.x, f0.y, f1.x, f1.y);
+                                b1 = make_float4(f2.x, f2.y, f3.x, f3.y);
+                            }
                             uint4 o;
                             __half2* h = reinterpret_cast<__half2*>(&o);
                             // Round to fp16 first; the activation sees the rounded value.
@@ -576,7 +597,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
                             h[1] = act(__floats2half2_rn(v[j * 8 + 2] + b0.z, v[j * 8 + 3] + b0.w));
                             h[2] = act(__floats2half2_rn(v[j * 8 + 4] + b1.x, v[j * 8 + 5] + b1.y));
                             h[3] = act(__floats2half2_rn(v[j * 8 + 6] + b1.z, v[j * 8 + 7] + b1.w));
-                            *reinterpret_cast<uint4*>(rowp + ((j ^ swz) << 4)) = o;
+                            *reinterpret_cast<uint4*>(rowp + ((((c % CPG) * (CH / 8) + j) ^ swz) << 4)) = o;
                         }
                     };
                     switch (act_kind) {
@@ -607,12 +628,13 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
                         *reinterpret_cast<float4*>(rowp + ((j ^ swz) << 4)) = o;
                     }
                 }
-                // shared -> global by the bulk-store engine: one instruction for the 16 x 32 box (the engine undoes
+                if (c % CPG != CPG - 1) continue;
+                // shared -> global by the bulk-store engine: one instruction for the GC x 32 box (the engine undoes
                 // the slab's swizzle), clipped at the ragged edges of the output.
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    tma_store_3d(&tmapO, wstg, m0 + col0, n0 + quad * 32, batch);
+                    tma_store_3d(&tmapO, wstg, m0 + col0 - (CPG - 1) * CH, n0 + quad * 32, batch);
                     tma_store_commit();
                 }
             }
@@ -679,6 +701,12 @@ __global__ void gemm_f16_scalar_kernel(int64_t M, int64_t N, int64_t K, const __
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+#ifndef GEMM_SLAB_KB
+#define GEMM_SLAB_KB 8
+#endif
+#ifndef GEMM_SLAB_128
+#define GEMM_SLAB_128 32
+#endif
 struct TilePick {
     int bn;      // feature columns per tile
     int ncta;    // 1: 128-token tiles, one CTA each; 2: 256-token tiles, one CTA pair each
@@ -819,7 +847,7 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
 // context's device whichever is current (the plan entry comes here without a launch), by one thread while others wait.
 static KsplitRoom ksplit_ask(b200_ctx* ctx) {
     using Cfg = GemmCfg<64, __half, 1>;
-    auto kern = gemm_f16_tc_kernel<64, __half, 1, true>;
+    auto kern = gemm_f16_tc_kernel<64, __half, 1, true, 16>;
     KsplitRoom got = {{ctx->prop.multiProcessorCount, 0, 0, 0}};
     if (cudaSetDevice(ctx->device) != cudaSuccess ||
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess) {
@@ -853,18 +881,18 @@ static const KsplitRoom& ksplit_room(b200_ctx* ctx) {
     return room[d];
 }
 
-template <int BN, typename OutT, int NCTA, bool KSPLIT = false>
+template <int BN, typename OutT, int NCTA, bool KSPLIT = false, int GC = 16>
 static int launch_tc(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda,
                      const void* B, int64_t ldb, const void* bias, int bias_per_n, void* out, int64_t ldo,
                      int epi, int64_t nbatch, int64_t sA, int64_t sB, int64_t sO, int streamk, int width,
                      int ksplit) {
-    using Cfg = GemmCfg<BN, OutT, NCTA>;
+    using Cfg = GemmCfg<BN, OutT, NCTA, GC>;
     if (Cfg::WIDE) {
         B200_REQUIRE(width > 256 && width <= 512 && width % 16 == 0, B200_EINVAL, "gemm: wide tile of %d columns", width);
         streamk = 0;
     }
     static bool attr_done[16] = {};
-    auto kern = gemm_f16_tc_kernel<BN, OutT, NCTA, KSPLIT>;
+    auto kern = gemm_f16_tc_kernel<BN, OutT, NCTA, KSPLIT, GC>;
     if (!attr_done[ctx->device & 15]) {
         B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
         attr_done[ctx->device & 15] = true;
@@ -891,9 +919,9 @@ static int launch_tc(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void*
         const uint64_t osz = sizeof(OutT);
         uint64_t dims[3] = {(uint64_t)M, (uint64_t)N, (uint64_t)nbatch};
         uint64_t str[2] = {(uint64_t)ldo * osz, (uint64_t)(nbatch > 1 ? sO : ldo * N) * osz};
-        uint32_t box[3] = {16, 32, 1};
+        uint32_t box[3] = {GC, 32, 1};
         int rc = make_tmap(ctx, &tO, sizeof(OutT) == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, out,
-                           dims, str, box, sizeof(OutT) == 2 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B);
+                           dims, str, box, GC * osz == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : GC * osz == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
         if (rc) return rc;
     }
     GemmParams<OutT> p;
@@ -1088,8 +1116,8 @@ int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, 
                                       strideA, strideB, strideO);
     }
     const TilePick t = pick_tile(M, N, K, nbatch, ctx->prop.multiProcessorCount, ksplit_room(ctx), use_workspace != 0, epilogue);
-#define GEMM_GO(BN_, T_, NC_)                                                                                     \
-    return launch_tc<BN_, T_, NC_>(ctx, M, N, K, A, lda, B, ldb, bias, bias_per_n, out, ldo, epilogue, nbatch, strideA, \
+#define GEMM_GO(...)                                                                                              \
+    return launch_tc<__VA_ARGS__>(ctx, M, N, K, A, lda, B, ldb, bias, bias_per_n, out, ldo, epilogue, nbatch, strideA, \
                                    strideB, strideO, t.streamk, t.width, t.ksplit)
 #define GEMM_GO_SPLIT(BN_, T_)                                                                                    \
     return launch_tc<BN_, T_, 1, true>(ctx, M, N, K, A, lda, B, ldb, bias, bias_per_n, out, ldo, epilogue, nbatch, strideA, \
@@ -1104,8 +1132,11 @@ int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, 
     }
     if (out_dtype == B200_F16) {
         if (t.bn == 512) GEMM_GO(512, __half, 2);
-        if (t.ncta == 2 && t.bn == 256) GEMM_GO(256, __half, 2);
-        if (t.ncta == 2) GEMM_GO(128, __half, 2);
+        if (t.ncta == 2 && t.bn == 256) {
+            if (cdiv(K, GEMM_BK) <= GEMM_SLAB_KB) GEMM_GO(256, __half, 2, false, 64);
+            GEMM_GO(256, __half, 2);
+        }
+        if (t.ncta == 2) GEMM_GO(128, __half, 2, false, GEMM_SLAB_128);
         if (t.bn == 256) GEMM_GO(256, __half, 1);
         if (t.bn == 128) GEMM_GO(128, __half, 1);
         GEMM_GO(64, __half, 1);
