@@ -16,7 +16,7 @@ namespace b200 {
 // brackets 7.1.26 step by step in fp32: over the fp16 grid 250 values round to another neighbour (458), fp32 results of
 // N(0, 0.1), N(0, 1) and N(0, 3) are off by 1.0e-7, 8.1e-8 and 4.7e-8 in the 2-norm (1.5e-7, 8.5e-8, 4.9e-8).  One
 // exponential an element and no sign to carry: a pair takes some 20 instructions where the steps take 32, two MUFU
-// operations instead of four, and those bound the GEMM store of a short-K product (GELU_TIMES).
+// operations instead of four, and those bound the GEMM store of a short-K product (524288 x 448 x 112: 239 -> 222 us).
 // Infinities and NaN give what the formula gives.
 // Every multiply, add and fused multiply-add is spelled out, so that the packed form below, which the GEMM
 // store uses, performs the same roundings and gives the same bits.

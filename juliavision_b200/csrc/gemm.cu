@@ -21,8 +21,6 @@
 #include <stdio.h>
 #include <stdlib.h>
 
-#include <type_traits>
-
 #include "act.cuh"
 #include "internal.h"
 #include "ptx.cuh"
@@ -52,10 +50,10 @@ template <int BN, typename OutT, int NCTA, int GC = 16> struct GemmCfg {
     static constexpr int B_COLS = BN / NCTA;               // feature columns this CTA stages
     static constexpr int B_BYTES = B_COLS * GEMM_BK * 2;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    // the epilogue's slabs, one per warp: 32 rows of GC output columns, behind them each warp's bias of its own columns
-    // (fp32; fp16 beside the wide slabs, which would cost a stage otherwise) and the barriers
+    // the epilogue's slabs, one per warp: 32 rows of GC output columns, behind them each warp's fp32 bias of its own columns
+    // and the barriers
     static constexpr int SLAB_BYTES = 32 * GC * (int)sizeof(OutT);
-    static constexpr int BIAS_BYTES = BN / (EPI_WARPS / 4) * (GC == 16 ? 4 : 2);
+    static constexpr int BIAS_BYTES = BN / (EPI_WARPS / 4) * 4;
     static constexpr int TAIL_BYTES = EPI_WARPS * (SLAB_BYTES + BIAS_BYTES) + 256;
     static constexpr int STAGES_RAW = (SMEM_LIMIT - TAIL_BYTES) / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
@@ -67,7 +65,7 @@ template <int BN, typename OutT, int NCTA, int GC = 16> struct GemmCfg {
     static_assert(TMEM_COLS == 128 || TMEM_COLS == 256 || TMEM_COLS == 512, "TMEM columns");
     static_assert(B_COLS % 64 == 0, "each CTA stages whole 64-column slabs of B");
     static_assert((STAGES * STAGE_BYTES) % 1024 == 0, "the epilogue slabs must start on the swizzle pattern's period");
-    static_assert(GC == 16 || (sizeof(OutT) == 2 && !WIDE && BN / (EPI_WARPS / 4) % GC == 0), "slabs of whole column groups");
+    static_assert(GC == 16 || (GC == 32 && sizeof(OutT) == 2 && !WIDE && BN / (EPI_WARPS / 4) % GC == 0), "slabs of whole chunks");
 };
 
 template <typename OutT> struct GemmParams {
@@ -170,6 +168,34 @@ __device__ __forceinline__ TileAt tile_at(uint32_t tile, uint32_t tiles_m, uint3
     t.tm = (int)(rem - (uint32_t)t.tn * tiles_m);
     return t;
 }
+
+// The same for a worker's tiles in turn.  Whole tiles are `step` apart: the place moves by a constant, carried over by
+// hand, where a division a tile was a tenth of what an epilogue warp issues on short K.
+struct TileWalk {
+    int dm, dn, tiles_m, tiles_n;
+    bool whole;
+    TileAt at;
+    __device__ __forceinline__ void init(const SegIter& seg, uint32_t step, int tiles_m_, int tiles_n_, bool one_plane) {
+        tiles_m = tiles_m_;
+        tiles_n = tiles_n_;
+        whole = !seg.streamk && one_plane;
+        dn = (int)(step / (uint32_t)tiles_m);
+        dm = (int)step - dn * tiles_m;
+        at = tile_at(seg.tile, (uint32_t)tiles_m, (uint32_t)tiles_m * (uint32_t)tiles_n, one_plane);
+    }
+    __device__ __forceinline__ void next(const SegIter& seg) {
+        if (whole) {
+            at.tm += dm;
+            at.tn += dn;
+            if (at.tm >= tiles_m) {
+                at.tm -= tiles_m;
+                ++at.tn;
+            }
+        } else {
+            at = tile_at(seg.tile, (uint32_t)tiles_m, (uint32_t)tiles_m * (uint32_t)tiles_n, false);
+        }
+    }
+};
 
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
     int v;
@@ -395,29 +421,49 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
         }
     } else {
         // ---------------------------------------------------------------- epilogue
-        // Sixteen warps, four per TMEM lane quadrant, each taking every fourth group of GC columns.
-        // Per group: tcgen05.ld -> +bias, round, activation -> a warp-private shared slab (32 rows x GC
+        // Sixteen warps, four per TMEM lane quadrant, each taking every fourth chunk of GC columns.
+        // Per chunk: tcgen05.ld -> +bias, round, activation -> a warp-private shared slab (32 rows x GC
         // columns) -> one bulk tensor store of the GC x 32 box, clipped at the ragged edges
         // of the output.  Each step is a short dependent chain, so the throughput comes from the four
-        // warps per scheduler taking turns; warps never wait for one another.
-        constexpr int CH = GC >= 32 ? 32 : 16; // columns per chunk (one tcgen05.ld)
-        constexpr int CPG = GC / CH;           // chunks of a group
+        // warps per scheduler taking turns; warps never wait for one another.  fp16 results of CTA pairs go 32 columns at
+        // a time: half the steps, and half the rows the store engine takes one by one (32 bytes each at 16 columns).
+        // Microseconds, 16 -> 32: 524288 x 336 x 112 126 -> 111, 131072 x 672 x 224 72 -> 65, 524288 x 448 x 112 with GELU
+        // 222 -> 201, 65536 x 5120 x 1280 727 -> 718; 64 columns do no better and cost a second stage.  The 256-wide pair pays
+        // with one of its six stages and goes without on long reductions (deep_ring).
+        constexpr int CH = GC;                 // columns per chunk (one tcgen05.ld)
         constexpr int NPART = EPI_WARPS / 4;   // warps sharing a lane quadrant
         constexpr int NCH = BN / NPART / CH;   // chunks one warp owns of a tile
         constexpr int RB = GC * (int)sizeof(OutT);  // staged bytes per row and group
-        using BiasT = std::conditional_t<GC == 16, float, __half>;
         const int ew = warp - 2;               // 0..15
         const int quad = warp & 3;             // TMEM lane quadrant this warp may read
-        const int part = ew >> 2;              // which groups of the quadrant's rows
+        const int part = ew >> 2;              // which chunks of the quadrant's rows
         const int row = quad * 32 + lane;      // token row inside this CTA's half of the tile
         uint8_t* wstg = slabs + ew * Cfg::SLAB_BYTES;
-        BiasT* wbias = reinterpret_cast<BiasT*>(sbias + ew * Cfg::BIAS_BYTES);   // bias of this warp's own columns
-        auto chunk_col = [&](int c) { return (NPART * (c / CPG) + part) * GC + (c % CPG) * CH; };
+        float* wbias = reinterpret_cast<float*>(sbias + ew * Cfg::BIAS_BYTES);   // bias of this warp's own columns
+        auto chunk_col = [&](int c) { return (NPART * c + part) * CH; };
         int it = 0;
-        SegIter seg;
-        for (seg.init(p.total_tiles, p.num_kb, p.streamk, worker, nworkers); seg.valid(); seg.next(), ++it) {
+        // A tile's place and its bias are looked up while the tile before it is worked on: in series they stood between a
+        // tile and the next, whose accumulator is long complete on short K, for 1000 to 2200 of some 7000 cycles
+        // (32768 x 1792 x 448 with GELU 75 -> 69 us, 131072 x 896 x 224 132 -> 127).
+        constexpr int BPL = (BN / NPART + 31) / 32;   // bias columns a lane looks up
+        __half nbias[BPL];
+        auto ask_bias = [&](int m0) {
+#pragma unroll
+            for (int i = 0; i < BPL; ++i) {
+                const int j = lane + 32 * i;
+                const int col = chunk_col(j / CH) + (j % CH);
+                nbias[i] = (p.bias != nullptr && !p.bias_per_n && j < BN / NPART && m0 + col < p.M) ? p.bias[m0 + col] : __float2half_rn(0.f);
+            }
+        };
+        SegIter seg, seg_next;
+        TileWalk walk;
+        seg_next.init(p.total_tiles, p.num_kb, p.streamk, worker, nworkers);
+        walk.init(seg_next, nworkers, p.tiles_m, p.tiles_n, one_plane);
+        if (seg_next.valid()) ask_bias(walk.at.tm * (Cfg::WIDE ? p.bn : BN));
+        for (; seg_next.valid(); ++it) {
+            seg = seg_next;
+            const TileAt at = walk.at;
             const uint32_t tile = seg.tile;
-            const TileAt at = tile_at(tile, (uint32_t)p.tiles_m, tiles_per_batch, one_plane);
             const int batch = at.batch;
             const int m0 = at.tm * (Cfg::WIDE ? p.bn : BN);
             const int n0 = at.tn * TILE_N + (int)rank * GEMM_BM;
@@ -462,11 +508,14 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
             const bool collect = ncontrib > 0 && sk_ok;
 
             __syncwarp(); // the previous tile's readers of wbias are done
-            for (int j = lane; j < BN / NPART; j += 32) {   // wbias[c*CH + t] = bias of column chunk_col(c) + t
-                const int col = chunk_col(j / CH) + (j % CH);
-                const __half b = (p.bias != nullptr && !p.bias_per_n && m0 + col < p.M) ? p.bias[m0 + col] : __float2half_rn(0.f);
-                if constexpr (GC == 16) wbias[j] = __half2float(b);
-                else wbias[j] = b;
+#pragma unroll
+            for (int i = 0; i < BPL; ++i)   // wbias[c*CH + t] = bias of column chunk_col(c) + t
+                if (lane + 32 * i < BN / NPART) wbias[lane + 32 * i] = __half2float(nbias[i]);
+            __syncwarp();
+            seg_next.next();
+            if (seg_next.valid()) {
+                walk.next(seg_next);
+                ask_bias(walk.at.tm * (Cfg::WIDE ? p.bn : BN));
             }
             const bool row_bias = !contributor && p.bias != nullptr && p.bias_per_n;   // the finisher adds the bias
             const float rbias = (row_bias && n0 + row < p.N) ? __half2float(p.bias[n0 + row]) : 0.f;
@@ -479,10 +528,10 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
             const uint32_t tacc = tmem_base + (uint32_t(quad * 32) << 16) + acc * BN;
             const int act_kind = p.epilogue;
             uint8_t* rowp = wstg + lane * RB;
-            // The slab's rows are 32, 64 or 128 B apart, so lanes four (two, one) apart would hit the same
+            // The slab's rows are 32 or 64 B apart, so lanes four (two) apart would hit the same
             // banks.  The store map swizzles at that width (16-byte chunk index ^= address bits from 7 up), which
             // spreads a warp's 16-byte stores over all banks: four wavefronts per instruction.
-            const int swz = RB == 32 ? ((lane >> 2) & 1) : (RB == 64 ? ((lane >> 1) & 3) : (lane & 7));
+            const int swz = RB == 32 ? ((lane >> 2) & 1) : ((lane >> 1) & 3);
 
             // KSPLIT: the accumulator over the operand ring, [chunk][quarter][row] of 16 bytes
             const uint32_t dump = smem_u32(smem) + row * 16;
@@ -563,41 +612,34 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
                         }
                     }
                 }
-                // nothing of this group to write to the output
-                if (m0 + col0 - (c % CPG) * CH >= p.M || rows_valid <= 0 || (Cfg::WIDE && col0 >= p.bn)) continue;
+                if (m0 + col0 >= p.M || rows_valid <= 0 || (Cfg::WIDE && col0 >= p.bn)) continue; // nothing to write to the output
 
-                // the engine must have read the previous group out of the slab before it is overwritten; that
+                // the engine must have read the previous chunk out of the slab before it is overwritten; that
                 // read ran under this chunk's tcgen05.ld and arithmetic
-                if (c % CPG == 0) {
-                    if (lane == 0) tma_store_wait_read<0>();
-                    __syncwarp();
-                }
+                if (lane == 0) tma_store_wait_read<0>();
+                __syncwarp();
                 // registers -> shared, lane = row
-                const BiasT* bc = wbias + c * CH;
+                const float* bc = wbias + c * CH;
                 if constexpr (sizeof(OutT) == 2) {
                     auto emit = [&](auto act) {
 #pragma unroll
                         for (int j = 0; j < CH / 8; ++j) {
-                            float4 b0, b1;
-                            if constexpr (GC == 16) {
-                                b0 = *reinterpret_cast<const float4*>(bc + j * 8);
-                                b1 = *reinterpret_cast<const float4*>(bc + j * 8 + 4);
-                            } else {
-                                const uint4 w = *reinterpret_cast<const uint4*>(bc + j * 8);
-                                const __half2* h2 = reinterpret_cast<const __half2*>(&w);
-                                const float2 f0 = __half22float2(h2[0]), f1 = __half22float2(h2[1]), f2 = __half22float2(h2[2]),
-                                             f3 = __half22float2(h2[3]);
-                                b0 = make_float4(f0.x, f0.y, f1.x, f1.y);
-                                b1 = make_float4(f2.x, f2.y, f3.x, f3.y);
-                            }
+                            // the bias of eight columns, four packed pairs
+                            const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(bc + j * 8);
+                            const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(bc + j * 8 + 4);
+                            auto biased = [&](int t, uint64_t b) {
+                                float lo, hi;
+                                unpack2(add2(pack2(v[j * 8 + t], v[j * 8 + t + 1]), b), lo, hi);
+                                return __floats2half2_rn(lo, hi);
+                            };
                             uint4 o;
                             __half2* h = reinterpret_cast<__half2*>(&o);
                             // Round to fp16 first; the activation sees the rounded value.
-                            h[0] = act(__floats2half2_rn(v[j * 8 + 0] + b0.x, v[j * 8 + 1] + b0.y));
-                            h[1] = act(__floats2half2_rn(v[j * 8 + 2] + b0.z, v[j * 8 + 3] + b0.w));
-                            h[2] = act(__floats2half2_rn(v[j * 8 + 4] + b1.x, v[j * 8 + 5] + b1.y));
-                            h[3] = act(__floats2half2_rn(v[j * 8 + 6] + b1.z, v[j * 8 + 7] + b1.w));
-                            *reinterpret_cast<uint4*>(rowp + ((((c % CPG) * (CH / 8) + j) ^ swz) << 4)) = o;
+                            h[0] = act(biased(0, b0.x));
+                            h[1] = act(biased(2, b0.y));
+                            h[2] = act(biased(4, b1.x));
+                            h[3] = act(biased(6, b1.y));
+                            *reinterpret_cast<uint4*>(rowp + ((j ^ swz) << 4)) = o;
                         }
                     };
                     switch (act_kind) {
@@ -628,13 +670,12 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
                         *reinterpret_cast<float4*>(rowp + ((j ^ swz) << 4)) = o;
                     }
                 }
-                if (c % CPG != CPG - 1) continue;
                 // shared -> global by the bulk-store engine: one instruction for the GC x 32 box (the engine undoes
                 // the slab's swizzle), clipped at the ragged edges of the output.
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    tma_store_3d(&tmapO, wstg, m0 + col0 - (CPG - 1) * CH, n0 + quad * 32, batch);
+                    tma_store_3d(&tmapO, wstg, m0 + col0, n0 + quad * 32, batch);
                     tma_store_commit();
                 }
             }
@@ -701,12 +742,10 @@ __global__ void gemm_f16_scalar_kernel(int64_t M, int64_t N, int64_t K, const __
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-#ifndef GEMM_SLAB_KB
-#define GEMM_SLAB_KB 8
-#endif
-#ifndef GEMM_SLAB_128
-#define GEMM_SLAB_128 32
-#endif
+// Whether a 256-wide pair stores 16 columns at a time and keeps a sixth stage instead (see the epilogue): reductions of 24
+// k-blocks and more (32768 x 448 x 1792: 55.5 us, 58 with 32 columns; of 20, 65536 x 5120 x 1280, 728 and 720).
+static bool deep_ring(int64_t K) { return cdiv(K, GEMM_BK) >= 24; }
+
 struct TilePick {
     int bn;      // feature columns per tile
     int ncta;    // 1: 128-token tiles, one CTA each; 2: 256-token tiles, one CTA pair each
@@ -921,7 +960,7 @@ static int launch_tc(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void*
         uint64_t str[2] = {(uint64_t)ldo * osz, (uint64_t)(nbatch > 1 ? sO : ldo * N) * osz};
         uint32_t box[3] = {GC, 32, 1};
         int rc = make_tmap(ctx, &tO, sizeof(OutT) == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, out,
-                           dims, str, box, GC * osz == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : GC * osz == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+                           dims, str, box, GC * osz == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
         if (rc) return rc;
     }
     GemmParams<OutT> p;
@@ -1042,8 +1081,8 @@ int b200_gemm_f16_plan(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, int64_t n
         plan->stages = GemmCfg<512, __half, 2>::STAGES;
         plan->smem_bytes = GemmCfg<512, __half, 2>::SMEM_BYTES;
     } else if (t.ncta == 2) {
-        plan->stages = bn == 256 ? GemmCfg<256, __half, 2>::STAGES : GemmCfg<128, __half, 2>::STAGES;
-        plan->smem_bytes = bn == 256 ? GemmCfg<256, __half, 2>::SMEM_BYTES : GemmCfg<128, __half, 2>::SMEM_BYTES;
+        plan->stages = bn == 128 ? GemmCfg<128, __half, 2, 32>::STAGES : deep_ring(K) ? GemmCfg<256, __half, 2>::STAGES : GemmCfg<256, __half, 2, 32>::STAGES;
+        plan->smem_bytes = bn == 128 ? GemmCfg<128, __half, 2, 32>::SMEM_BYTES : deep_ring(K) ? GemmCfg<256, __half, 2>::SMEM_BYTES : GemmCfg<256, __half, 2, 32>::SMEM_BYTES;
     } else {
         plan->stages = bn == 256 ? GemmCfg<256, __half, 1>::STAGES
                                  : (bn == 128 ? GemmCfg<128, __half, 1>::STAGES : GemmCfg<64, __half, 1>::STAGES);
@@ -1132,11 +1171,9 @@ int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, 
     }
     if (out_dtype == B200_F16) {
         if (t.bn == 512) GEMM_GO(512, __half, 2);
-        if (t.ncta == 2 && t.bn == 256) {
-            if (cdiv(K, GEMM_BK) <= GEMM_SLAB_KB) GEMM_GO(256, __half, 2, false, 64);
-            GEMM_GO(256, __half, 2);
-        }
-        if (t.ncta == 2) GEMM_GO(128, __half, 2, false, GEMM_SLAB_128);
+        if (t.ncta == 2 && t.bn == 256 && deep_ring(K)) GEMM_GO(256, __half, 2);
+        if (t.ncta == 2 && t.bn == 256) GEMM_GO(256, __half, 2, false, 32);
+        if (t.ncta == 2) GEMM_GO(128, __half, 2, false, 32);
         if (t.bn == 256) GEMM_GO(256, __half, 1);
         if (t.bn == 128) GEMM_GO(128, __half, 1);
         GEMM_GO(64, __half, 1);

@@ -464,3 +464,41 @@ def test_weight_operand_produced_by_the_previous_launch(ctx):
         y1 = Y1.to_host()                                        # torch (N1, M1)
         want = np.float32(X2.to_host()) @ np.float32(y1)         # (N2, N1) @ (N1, M1)
         assert relerr(Y2.to_host(), want) < 5e-3, f"round {round_}"
+
+
+@pytest.mark.parametrize("tile", ["256x2", "128x2"])
+@pytest.mark.parametrize("tokens,out,K", [(300, 8, 64), (700, 24, 1536), (520, 264, 1472), (4100, 1304, 72), (20000, 456, 40), (257, 40, 1528)])
+def test_pairs_of_ctas_store_wide_chunks(ctx, ora, tile, tokens, out, K, monkeypatch):
+    """Feature counts that end inside a stored chunk, reductions on both sides of the deeper ring's rule, one and many tiles
+    a worker with feature tiles that do not divide its step: results by rounding at the store only."""
+    monkeypatch.setenv("B200_GEMM_TILE", tile)
+    rng = np.random.default_rng(tokens + out + K)
+    X, Wt, b = _case(rng, tokens, out, K, scale=0.25)
+    for epi, bias in (("identity", b), ("gelu", b), ("relu", None)):
+        got = linear_gpu(ctx, X, Wt, bias, epi=epi)
+        ref = ora.linear(X, Wt, bias, epi=epi)
+        assert relerr(got, ref) < 2e-3, (epi, describe(got, ref, 2e-3))          # one rounding step of fp16
+
+
+def test_gelu_over_every_half(ctx, ora):
+    """The folded activation against the stand-alone op (equal bits) and the oracle (an fp16 step, and what 7.1.26 in fp32
+    is off by where it cancels), for every finite fp16 value; infinities and NaN as the formula has them."""
+    x = np.arange(65536, dtype=np.uint16).view(np.float16)
+    x = np.concatenate([x[np.isfinite(x)], np.float16([np.inf, -np.inf, np.nan, 0, 0, 0, 0, 0])])
+    d, o = ctx.toback(x), ctx.allocate(np.float16, x.size)
+    jv.act_(ctx, o, d, "gelu")
+    alone = o.to_host()
+    with np.errstate(over="ignore", invalid="ignore"):
+        ref = ora.act(x, "gelu")
+        fin = np.isfinite(x)
+        step = np.spacing(np.abs(ref[fin])).astype(np.float32)
+    assert np.all(np.abs(alone[fin].astype(np.float32) - ref[fin].astype(np.float32)) <= step + 1e-7)
+    assert alone[~fin][0] == np.inf and np.isnan(alone[~fin][1]) and np.isnan(alone[~fin][2])
+    finite = np.where(fin, x, np.float16(0))
+    one = np.zeros((300, 8), np.float16)
+    one[:, 0] = 1
+    weight = np.zeros((x.size, 8), np.float16)
+    weight[:, 0] = finite
+    got = linear_gpu(ctx, one, weight, None, epi="gelu")       # x * 1 + zeros: the values themselves, exactly
+    want = np.where(fin, alone, alone[np.flatnonzero(finite == 0)[0]])
+    assert np.all(got == want[None, :])
