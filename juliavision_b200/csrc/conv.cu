@@ -151,6 +151,22 @@ static int conv2d_group(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_
     bool implicit = conv_implicit_takes(W, H, Cin, N, KW, KH, Cout, P) &&
                     (onebyone ? !gemm_1x1 : !aligned || cdiv(P, 128) * N >= 2 * ctx->prop.multiProcessorCount);
     const size_t ws_mark = ctx->ws_used;
+    // An even stride over rows of whole words: the implicit kernel reads the image in words, whatever the image's size.  Its
+    // weight takes a workspace; refused (a graph recorded without an eager call before), the call goes on as it did.
+    const int words = conv_implicit_takes(W, H, Cin, N, KW > 8 ? KW : 8, KH, Cout, P) ? conv_words(W, KW, sx, px, dx, x, x_img) : 0;
+    if (words) {
+        void* wp = nullptr;
+        rc = ws_scratch(ctx, (size_t)(conv_words_ldw(Cin * KH, words) * Cout) * 2, &wp);
+        if (rc && rc != B200_ENOMEM) return rc;
+        if (!rc) {
+            rc = conv_words_weight(ctx, wp, w, KW, px, Cin * KH, Cout, words);
+            if (!rc)
+                rc = conv_implicit_launch(ctx, W, H, Cin, N, KW, KH, Cout, sx, sy, px, py, dx, dy, OW, P, x, x_img, wp,
+                                          conv_words_ldw(Cin * KH, words), bias, out, out_img, out_dtype, epilogue, words);
+            ctx->ws_used = ws_mark;   // the copy is not kept: what comes next on the stream runs after it was read
+            return rc;
+        }
+    }
     const bool padded = CRS % 8 != 0;
     if (padded || (implicit && !al16(w))) {
         ldw = (CRS + 7) / 8 * 8;
@@ -171,7 +187,7 @@ static int conv2d_group(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_
     }
     if (implicit) {
         rc = conv_implicit_launch(ctx, W, H, Cin, N, KW, KH, Cout, sx, sy, px, py, dx, dy, OW, P, x, x_img, wB, ldw, bias, out,
-                                  out_img, out_dtype, epilogue);
+                                  out_img, out_dtype, epilogue, 0);
         if (!padded) ctx->ws_used = ws_mark;   // that copy is not kept: what comes next on the stream runs after it was read
         return rc;
     }

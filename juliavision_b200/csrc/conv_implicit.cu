@@ -20,14 +20,26 @@
 // Measured (us, B200) against the im2col + GEMM route: 1024 x 1024 x 3 -> 112, 7 x 7 / 4: 35 -> 23.6; 300 x 296 x 16 -> 64,
 // 3 x 3: 42.5 -> 24.6; against the scalar GEMM odd pixel counts had: 43 x 42 x 256 -> 256, 3 x 3 / 2: 229 -> 14.2, two of
 // 230 x 225 x 32 -> 80, 3 x 3: 890 -> 43.  What is left is the gather's load latency.
+// An even stride takes the image in whole words instead (G): the pixels' first taps are then 8 (stride 4, 8, ...) or 4
+// bytes apart, so one pixel's taps of a kernel row, with the element or two before or after them that fill the words, are
+// two aligned loads, masked to the taps.  The reduction is laid out (cin, kh, G columns), G = 8 or 4, the weight the same
+// with zeros between, the tile K-major: a thread's pixel and eight columns are one 16-byte store.  A seventh and a third more
+// columns than taps (7 x 7 / 4, 3 x 3 / 2) and a tenth of the instructions: us, before and
+// now: 1024 x 1024 x 3 -> 112, 7 x 7 / 4 24.7 -> 15.9, eight of them 166 -> 93, 512 x 512 x 3 -> 64 18.4 -> 6.4, 3 x 3 / 2
+// 256 x 256 x 32 -> 128 19.4 -> 15.8, 128 x 128 x 128 -> 256 22.5 -> 18.1.  What is left is a CTA's chain of latencies.
 // A small image (fewer CTAs than the GPU holds) splits the reduction over the CTAs of a cluster, whose fp32 tiles
 // meet in distributed shared memory, added in rank order.
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "act.cuh"
 #include "internal.h"
 #include "ptx.cuh"
 
+#ifndef CI_SPLIT
+#define CI_SPLIT 4
+#endif
 namespace b200 {
 
 constexpr int CI_PIX = 128;              // pixels per CTA (TMEM lanes)
@@ -53,6 +65,8 @@ struct ConvParams {
     int W, H, CRS, Cout, OW, P, tiles;   // tiles of CI_PIX pixels per image
     int sx, sy, px, py, dx, dy;
     int KW, KH;
+    int rows;                 // G: kernel rows of all channels, Cin * KH
+    uint32_t mask[4];         // G: the words of a kernel row that are taps
     uint32_t mKW, mKH;        // ceil(2^32 / KW), ceil(2^32 / KH): exact quotients below 2^16
     int epi;
     int* d_status;
@@ -79,8 +93,34 @@ __device__ __forceinline__ uint32_t ldg_u16_if(const uint16_t* p, bool in) {
     return v;
 }
 
-// grid (K parts, pixel tiles of all images, channel tiles); the K parts of a tile form a cluster.
-template <int BN, typename OutT>
+// The words of a piece of a kernel row, or zeros: predicated loads, no branch.
+__device__ __forceinline__ void ldg_words_if(uint32_t (&v)[2], const uint16_t* p, bool in) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred P;\n\t"
+        "setp.ne.u32 P, %3, 0;\n\t"
+        "mov.b32 %0, 0;\n\t"
+        "mov.b32 %1, 0;\n\t"
+        "@P ld.global.nc.v2.b32 {%0, %1}, [%2];\n\t"
+        "}\n"
+        : "=&r"(v[0]), "=&r"(v[1])
+        : "l"(p), "r"((uint32_t)in));
+}
+__device__ __forceinline__ void ldg_words_if(uint32_t (&v)[1], const uint16_t* p, bool in) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred P;\n\t"
+        "setp.ne.u32 P, %2, 0;\n\t"
+        "mov.b32 %0, 0;\n\t"
+        "@P ld.global.nc.b32 %0, [%1];\n\t"
+        "}\n"
+        : "=&r"(v[0])
+        : "l"(p), "r"((uint32_t)in));
+}
+
+// grid (K parts, pixel tiles of all images, channel tiles); the K parts of a tile form a cluster.  G: columns of the
+// reduction per kernel row where the image is read in words, 0: tap by tap.
+template <int BN, typename OutT, int G>
 __global__ void __launch_bounds__(CI_THREADS, 2)
 conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Cout}, boxes of 64 x BN
                      const ConvParams p) {
@@ -150,8 +190,8 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
         }
     } else if (warp == 9) {
         if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc_f16(CI_PIX, BN, /*a MN-major*/ 1, /*b K-major*/ 0);
-            constexpr uint64_t adesc0 = make_smem_desc(64 * CI_BK * 2, 1024);
+            constexpr uint32_t idesc = make_idesc_f16(CI_PIX, BN, /*a MN-major, in words K-major*/ G == 0, /*b K-major*/ 0);
+            constexpr uint64_t adesc0 = G == 0 ? make_smem_desc(64 * CI_BK * 2, 1024) : make_smem_desc(16, 1024);
             constexpr uint64_t bdesc0 = make_smem_desc(16, 1024);
             bool ok = true;
             for (int kb = 0; kb < nkb; ++kb) {
@@ -160,8 +200,8 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
                 tc_fence_after();
                 const uint32_t a = smem_u32(smem + s * Cfg::STAGE_BYTES), b = a + CI_A_BYTES;
 #pragma unroll
-                for (int k = 0; k < CI_BK / 16; ++k)   // 16 k: two 8-row groups of A, 32 bytes inside B's swizzle row
-                    umma_ss(tmem_base, smem_desc_at(adesc0, a + k * 2048), smem_desc_at(bdesc0, b + k * 32), idesc, (kb | k) != 0);
+                for (int k = 0; k < CI_BK / 16; ++k)   // 16 k: two 8-row groups of an MN-major A, 32 bytes inside a K-major swizzle row
+                    umma_ss(tmem_base, smem_desc_at(adesc0, a + k * (G == 0 ? 2048 : 32)), smem_desc_at(bdesc0, b + k * 32), idesc, (kb | k) != 0);
                 umma_commit(&empty[s]);
             }
             if (ok) umma_commit(tfull);
@@ -169,6 +209,54 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
     } else {
         for (int j = tid; j < BN; j += CI_GATHER)   // read in the epilogue, a barrier among these warps later
             sbias[j] = p.bias != nullptr && c0 + j < p.Cout ? __half2float(p.bias[c0 + j]) : 0.f;
+        bool ok = true;
+        const uint16_t* xi = reinterpret_cast<const uint16_t*>(p.x) + (int64_t)img * p.x_img;
+        if constexpr (G > 0) {
+            // Pixel tid % 128; of a k-block's eight 16-byte pieces those of one parity.
+            constexpr int VL = G / 2, RPC = 8 / G;   // elements a load, kernel rows a piece
+            const int pix = tid & 127, par = tid >> 7, m = m0 + pix;
+            const int oh = m / p.OW, ow = m - oh * p.OW;
+            const int bx = ow * p.sx - p.px, by = m < p.P ? oh * p.sy - p.py : -(1 << 30);   // never inside the image
+            const bool in0 = (uint32_t)bx < (uint32_t)p.W, in1 = (uint32_t)(bx + VL) < (uint32_t)p.W;   // whole words: W is a multiple
+            const int base = by * p.W + bx;
+            uint32_t v[2][4][RPC][2][VL / 2];
+            auto load = [&](int kb, int b) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int u = 0; u < RPC; ++u) {
+                        const int r = ((kb0 + kb) * 8 + 2 * i + par) * RPC + u;   // the same for the warp
+                        const int cin = (int)div_magic((uint32_t)r, p.KH, p.mKH), ky = (r - cin * p.KH) * p.dy;
+                        const bool row = r < p.rows && (uint32_t)(by + ky) < (uint32_t)p.H;
+                        const uint16_t* src = xi + (base + (cin * p.H + ky) * p.W);
+                        ldg_words_if(v[b][i][u][0], src, row && in0);
+                        ldg_words_if(v[b][i][u][1], src + VL, row && in1);
+                    }
+            };
+            load(0, 0);
+            auto step = [&](int kb, int b) -> bool {
+                const int s = kb % Cfg::STAGES;
+                if (kb + 1 < nkb) load(kb + 1, b ^ 1);
+                if (ok && !mbar_wait(&empty[s], (uint32_t)((kb / Cfg::STAGES) & 1) ^ 1, p.d_status, KST_WAIT_EMPTY, abort_flag)) ok = false;
+                if (__any_sync(0xffffffffu, !ok)) return ok = false;
+                const uint32_t a = smem_u32(smem + s * Cfg::STAGE_BYTES) + pix * 128;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) w[e] = v[b][i][e / (4 / RPC)][(e / (VL / 2)) & 1][e % (VL / 2)] & p.mask[e];
+                    st_shared_v4(a + (((2 * i + par) ^ (pix & 7)) << 4), w);
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[s]);
+                return true;
+            };
+            for (int kb = 0; kb < nkb; kb += 2) {   // by twos: the registers of a step are named at compile time
+                if (!step(kb, 0)) break;
+                if (kb + 1 < nkb && !step(kb + 1, 1)) break;
+            }
+        } else {
         // Pixels 2 lane, 2 lane + 1 of either half of the tile.
         int bx[4], by[4], base[4];
 #pragma unroll
@@ -179,7 +267,6 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
             by[q] = m < p.P ? oh * p.sy - p.py : -(1 << 30);   // never inside the image
             base[q] = by[q] * p.W + bx[q];
         }
-        const uint16_t* xi = reinterpret_cast<const uint16_t*>(p.x) + (int64_t)img * p.x_img;
         const int row_off = warp * 128 + (((lane >> 2) ^ warp) << 4) + (lane & 3) * 4;   // row warp + 8 r: r * 1024 further
         // The taps of the warp's eight rows of a k-block, row r by lane r: offset in the image and (x, y) shift.  A row
         // past the reduction gets a shift that is never inside.
@@ -209,7 +296,6 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
                 for (int h = 0; h < 2; ++h)
                     *reinterpret_cast<uint32_t*>(a + h * (64 * CI_BK * 2) + i * 1024) = v[i][2 * h] | (v[i][2 * h + 1] << 16);
         };
-        bool ok = true;
         uint32_t va[4][4], vb[4][4];
         taps(0);
         load(va, 0);
@@ -227,6 +313,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(&full[s]);
+        }
         }
         // ------------------------------------------------------------------ epilogue
         named_bar_sync(1, CI_GATHER);   // sbias
@@ -308,11 +395,11 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
     }
 }
 
-template <int BN, typename OutT>
+template <int BN, typename OutT, int G>
 static int ci_launch(b200_ctx* ctx, const CUtensorMap& tw, const ConvParams& p, int64_t N, int parts) {
     using Cfg = CiCfg<BN>;
     static bool attr_done[16] = {};
-    auto kern = conv_implicit_kernel<BN, OutT>;
+    auto kern = conv_implicit_kernel<BN, OutT, G>;
     if (!attr_done[ctx->device & 15]) {
         B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
         attr_done[ctx->device & 15] = true;
@@ -328,10 +415,46 @@ bool conv_implicit_takes(int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t K
            Cout < (1 << 20) && W < (1 << 28) && H < (1 << 28);
 }
 
+// Whether the image can be read in words, and the columns of the reduction a kernel row then takes (0: no).  The pixels'
+// first taps have to lie `word` elements apart with every row of the image starting on one, and a row's taps in two words.
+// One word would do for narrow kernels and half of the reduction would be zeros; they stay with the taps.
+int conv_words(int64_t W, int64_t KW, int64_t sx, int64_t px, int64_t dx, const void* x, int64_t x_img) {
+    for (const int64_t word : {4, 2}) {
+        const int64_t lead = (word - px % word) % word;
+        if (sx % word == 0 && W % word == 0 && x_img % word == 0 && (dx == 1 || KW == 1) && reinterpret_cast<uintptr_t>(x) % (2 * word) == 0 &&
+            KW + lead > word && KW + lead <= 2 * word)
+            return (int)(2 * word);
+    }
+    return 0;
+}
+
+// The weight for it: (Cout, CRS) -> (Cout, Cin KH, g), each kernel row's taps behind `lead` zeros; rows in whole 16 bytes.
+int64_t conv_words_ldw(int64_t rows, int g) { return cdiv(rows * g, 8) * 8; }
+
+__global__ void conv_words_weight_kernel(__half* __restrict__ dst, const __half* __restrict__ src, int KW, int g, int lead, int rows,
+                                         int ldw, int64_t n) {
+    grid_dep_wait();     // the weight may be the previous kernel's output
+    grid_dep_launch();
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t co = i / ldw;
+        const int k = (int)(i - co * ldw), row = k / g, t = k - row * g - lead;
+        dst[i] = row < rows && t >= 0 && t < KW ? src[(co * rows + row) * KW + t] : __float2half_rn(0.f);
+    }
+}
+
+int conv_words_weight(b200_ctx* ctx, void* dst, const void* w, int64_t KW, int64_t px, int64_t rows, int64_t Cout, int g) {
+    const int64_t ldw = conv_words_ldw(rows, g), n = Cout * ldw, word = g / 2, cap = (int64_t)ctx->prop.multiProcessorCount * 8;
+    const int64_t blocks = cdiv(n, 256);
+    B200_CUDA(launch_dep(conv_words_weight_kernel, dim3((unsigned)(blocks < cap ? blocks : cap), 1, 1), dim3(256, 1, 1), 0, ctx->stream, 1,
+                         (__half*)dst, (const __half*)w, (int)KW, g, (int)((word - px % word) % word), (int)rows, (int)ldw, n));
+    ctx->launches++;
+    return B200_OK;
+}
+
 int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t KW, int64_t KH, int64_t Cout,
                          int64_t sx, int64_t sy, int64_t px, int64_t py, int64_t dx, int64_t dy, int64_t OW, int64_t P,
                          const void* x, int64_t x_img, const void* w, int64_t ldw, const void* bias, void* out,
-                         int64_t out_img, int out_dtype, int epilogue) {
+                         int64_t out_img, int out_dtype, int epilogue, int g) {
     ConvParams p;
     p.x = static_cast<const __half*>(x);
     p.bias = static_cast<const __half*>(bias);
@@ -345,23 +468,43 @@ int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64
     p.epi = epilogue;
     p.d_status = ctx->d_status;
     p.tiles = (int)cdiv(P, CI_PIX);
+    p.rows = (int)(Cin * KH);
+    if (g) {
+        const int64_t word = g / 2, lead = (word - px % word) % word;
+        p.CRS = (int)(Cin * KH * g);
+        p.px = (int)(px + lead);
+        for (int e = 0; e < 4; ++e) {
+            p.mask[e] = 0;
+            for (int h = 0; h < 2; ++h) {
+                const int64_t t = (2 * e + h) % g - lead;
+                if (t >= 0 && t < KW) p.mask[e] |= 0xFFFFu << (16 * h);
+            }
+        }
+    }
     // Channels per CTA: all of them up to 256, since every channel tile gathers the pixels again; but a launch that
     // leaves half of the GPU's CTAs unused splits the reduction, two k-blocks a part at least, which the 256-wide
     // tile has no shared memory for.
-    const int64_t tiles = p.tiles * N, room = 2 * (int64_t)ctx->prop.multiProcessorCount, nkb = cdiv(p.CRS, CI_BK);
+    const int64_t tiles = p.tiles * N, room = 2 * (int64_t)ctx->prop.multiProcessorCount, nkb = cdiv((int64_t)p.CRS, CI_BK);
     int bn = Cout <= 64 ? 64 : (Cout <= 128 || (2 * tiles * cdiv(Cout, 128) <= room && nkb >= 4) ? 128 : 256), parts = 1;
     if (bn < 256)
-        while (parts < 8 && 2 * parts * tiles * cdiv(Cout, bn) <= room && nkb >= 4 * parts) parts *= 2;
+        while (parts < 8 && 2 * parts * tiles * cdiv(Cout, bn) <= room && nkb >= (g ? CI_SPLIT : 4) * parts) parts *= 2;
     CUtensorMap tw;
     uint64_t dims[2] = {(uint64_t)p.CRS, (uint64_t)Cout};
     uint64_t str[1] = {(uint64_t)ldw * 2};
     uint32_t box[2] = {CI_BK, (uint32_t)bn};
     int rc = make_tmap(ctx, &tw, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, w, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
-    const bool h = out_dtype == B200_F16;
-    if (bn == 256) return h ? ci_launch<256, __half>(ctx, tw, p, N, 1) : ci_launch<256, float>(ctx, tw, p, N, 1);
-    if (bn == 128) return h ? ci_launch<128, __half>(ctx, tw, p, N, parts) : ci_launch<128, float>(ctx, tw, p, N, parts);
-    return h ? ci_launch<64, __half>(ctx, tw, p, N, parts) : ci_launch<64, float>(ctx, tw, p, N, parts);
+    auto go = [&](auto zero, auto G) -> int {
+        using T = decltype(zero);
+        constexpr int g = decltype(G)::value;
+        if (bn == 256) return ci_launch<256, T, g>(ctx, tw, p, N, 1);
+        if (bn == 128) return ci_launch<128, T, g>(ctx, tw, p, N, parts);
+        return ci_launch<64, T, g>(ctx, tw, p, N, parts);
+    };
+    auto typed = [&](auto G) { return out_dtype == B200_F16 ? go(__half(), G) : go(float(), G); };
+    if (g == 8) return typed(std::integral_constant<int, 8>());
+    if (g == 4) return typed(std::integral_constant<int, 4>());
+    return typed(std::integral_constant<int, 0>());
 }
 
 } // namespace b200

@@ -49,9 +49,22 @@ struct GrParams {
     int64_t lda, ldb, ldo;
     int64_t M, N, K;
     int bias_per_n, epi, b_vec;
+    int64_t block0;      // the launch's first row block
+    int tail;            // a second launch of the same product: nothing it reads waits for the first
     int steps_per_cta;   // steps of GR_STEP columns each CTA of a cluster takes
 };
 
+__device__ __forceinline__ uint4 ld_l2(const char* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L2::256B.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+#ifndef GR_LD
+#define GR_LD(q) __ldg(reinterpret_cast<const uint4*>(q))
+#endif
+#ifndef GR_TAIL
+#define GR_TAIL 1
+#endif
 // grid (K parts, row blocks, token blocks), the K parts of a row block forming a cluster; 256 threads.
 template <int NT, typename OutT>
 __global__ void __launch_bounds__(32 * GR_WARPS, GrCfg<NT>::MIN_BLOCKS)
@@ -63,6 +76,8 @@ gemm_rows_kernel(const GrParams p) {
     float* red = reinterpret_cast<float*>(gr_smem);                        // [warp][8 tokens][RP], after the main loop
     float* sums = reinterpret_cast<float*>(gr_smem + Cfg::SMEM_BYTES - Cfg::SUM_BYTES);   // [token][ROWS]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int64_t block = p.block0 + blockIdx.y;
+    grid_dep_launch();   // only the tail is launched to start early, and it reads what the first part reads
     const int64_t n0 = (int64_t)blockIdx.z * (NT * 8);
     const int ntok = (int)(p.N - n0 < NT * 8 ? p.N - n0 : NT * 8);
     const int64_t step0 = (int64_t)blockIdx.x * p.steps_per_cta;
@@ -83,7 +98,7 @@ gemm_rows_kernel(const GrParams p) {
     const char* col0 = reinterpret_cast<const char*>(p.A + (int64_t)warp * p.lda);
     const int s = (int)(reinterpret_cast<uintptr_t>(col0) & 15u) >> 1;
     const int64_t cstep = 8 * p.lda * 2;                                   // bytes from one of the warp's columns to its next
-    const int64_t jv = (int64_t)blockIdx.y * (Cfg::ROWS / 8);              // the block's first vector
+    const int64_t jv = block * (Cfg::ROWS / 8);              // the block's first vector
     bool live[MB];
 #pragma unroll
     for (int mi = 0; mi < MB; ++mi) live[mi] = 8 * (jv + 8 * mi + g) - s < p.M;   // the vector holds a row of A
@@ -98,7 +113,7 @@ gemm_rows_kernel(const GrParams p) {
             const char* v = vec0 + j * cstep;
 #pragma unroll
             for (int mi = 0; mi < MB; ++mi)
-                a[mi][c] = in && live[mi] ? __ldg(reinterpret_cast<const uint4*>(v + mi * 128)) : make_uint4(0u, 0u, 0u, 0u);
+                a[mi][c] = in && live[mi] ? GR_LD(v + mi * 128) : make_uint4(0u, 0u, 0u, 0u);
         }
     };
 
@@ -161,7 +176,7 @@ gemm_rows_kernel(const GrParams p) {
 
     // Sum over the warps, eight tokens at a time: row r of the block is accumulator row r + s of warp `warp`.
     const uint32_t nparts = cluster_nctarank();
-    const int64_t m0 = (int64_t)blockIdx.y * Cfg::ROWS;
+    const int64_t m0 = block * Cfg::ROWS;
     auto store = [&](int tok, int r, float v) {
         const int64_t m = m0 + r, n = n0 + tok;
         if (p.bias != nullptr) v += __half2float(p.bias[p.bias_per_n ? n : m]);
@@ -193,6 +208,7 @@ gemm_rows_kernel(const GrParams p) {
         }
     }
     if (nparts == 1) return;
+    if (p.tail) grid_dep_wait();   // what follows on the stream runs after the first part as well
     cluster_sync_all();   // every part's sums are in its shared memory
     const uint32_t rank = cluster_ctarank();
     const uint32_t mine = smem_u32(sums);
@@ -225,21 +241,38 @@ static int gr_launch(b200_ctx* ctx, GrParams p) {
     const int64_t room = (int64_t)ctx->prop.multiProcessorCount * Cfg::MIN_BLOCKS;
     int64_t parts = 1;
     while (parts < 8 && 2 * parts * blocks * tblocks <= room && steps >= 4 * parts) parts *= 2;
-    p.steps_per_cta = (int)cdiv(steps, parts);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)parts, (unsigned)blocks, (unsigned)tblocks);
-    cfg.blockDim = dim3(32 * GR_WARPS, 1, 1);
-    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)parts;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    B200_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
-    ctx->launches++;
+    // Row blocks past the last full round of the resident ones, less than half a round of them, are a launch of their own,
+    // split along K like few row blocks are: 433 blocks of 296 take a round and a half instead of two.  (A second launch may
+    // start as the first one's blocks leave: see the kernel.)  TAIL_TIMES.
+    int64_t tail = 0, tail_parts = 1;
+    if (parts == 1 && tblocks == 1 && blocks > room && GR_TAIL) {
+        tail = blocks % room;
+        while (tail_parts < 8 && 2 * tail_parts * tail <= room && steps >= 4 * tail_parts) tail_parts *= 2;
+        if (tail_parts == 1) tail = 0;
+    }
+    auto go = [&](int64_t first, int64_t n, int64_t k_parts, bool second) -> cudaError_t {
+        p.block0 = first;
+        p.tail = second;
+        p.steps_per_cta = (int)cdiv(steps, k_parts);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)k_parts, (unsigned)n, (unsigned)tblocks);
+        cfg.blockDim = dim3(32 * GR_WARPS, 1, 1);
+        cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+        cfg.stream = ctx->stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)k_parts;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = second ? 2 : 1;
+        ctx->launches++;
+        return cudaLaunchKernelEx(&cfg, kern, p);
+    };
+    if (blocks > tail) B200_CUDA(go(0, blocks - tail, parts, false));
+    if (tail) B200_CUDA(go(blocks - tail, tail, tail_parts, true));
     return B200_OK;
 }
 

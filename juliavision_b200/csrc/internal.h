@@ -135,7 +135,11 @@ bool conv_implicit_takes(int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t K
 int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t KW, int64_t KH, int64_t Cout,
                          int64_t sx, int64_t sy, int64_t px, int64_t py, int64_t dx, int64_t dy, int64_t OW, int64_t P,
                          const void* x, int64_t x_img, const void* w, int64_t ldw, const void* bias, void* out,
-                         int64_t out_img, int out_dtype, int epilogue);
+                         int64_t out_img, int out_dtype, int epilogue, int g);
+// Its form for even strides (g = conv_words, not 0), whose weight conv_words_weight lays out with leading dimension conv_words_ldw.
+int conv_words(int64_t W, int64_t KW, int64_t sx, int64_t px, int64_t dx, const void* x, int64_t x_img);
+int64_t conv_words_ldw(int64_t rows, int g);
+int conv_words_weight(b200_ctx* ctx, void* dst, const void* w, int64_t KW, int64_t px, int64_t rows, int64_t Cout, int g);
 
 // GEMM over operands a tensor map cannot express, from a few tens of thousands of elements of A up (gemm_rows.cu).
 bool gemm_rows_takes(int64_t M, int64_t N, int64_t K, int64_t nbatch);

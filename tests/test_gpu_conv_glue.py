@@ -190,6 +190,58 @@ def test_glue_bit_exact(ctx, ora):
         assert np.all(d <= np.spacing(np.abs(ref)).astype(np.float32) + 1e-7)   # fast exp: one fp16 ulp at most
 
 
+# (N, Cin, H, W, Cout, KH, KW, stride, padding, dilation): 8 and 4 columns a kernel row, taps before and behind the words'
+# ends, one and several k-blocks and parts of a cluster, odd kernel-row counts, dilated rows, pixels past the last tile
+WORDS = [(1, 3, 37, 64, 112, 7, 7, (4, 4), (3, 3), (1, 1)), (2, 3, 40, 44, 24, 7, 5, (3, 4), (2, 2), (2, 1)),
+         (1, 5, 24, 48, 130, 4, 8, (1, 8), (0, 0), (1, 1)), (2, 17, 31, 30, 64, 3, 3, (2, 2), (1, 1), (1, 1)),
+         (1, 7, 9, 22, 300, 1, 4, (2, 2), (0, 4), (1, 1)), (1, 64, 20, 26, 40, 3, 3, (2, 6), (1, 1), (1, 1)),
+         (3, 1, 50, 52, 16, 2, 2, (2, 4), (0, 5), (3, 1)), (1, 160, 16, 16, 72, 3, 3, (2, 2), (1, 1), (1, 1))]
+
+
+@pytest.mark.parametrize("N,Cin,H,W,Cout,KH,KW,stride,padding,dilation", WORDS)
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+def test_conv_of_even_stride_reads_whole_words(ctx, ora, N, Cin, H, W, Cout, KH, KW, stride, padding, dilation, dt):
+    rng = np.random.default_rng(Cin + Cout + W)
+    x = np.float16(rng.standard_normal((N, Cin, H, W)) * 0.5)
+    w = np.float16(rng.standard_normal((Cout, Cin, KH, KW)) * 0.2)
+    b = np.float16(rng.standard_normal(Cout) * 0.2)
+    ref = ora.conv2d(x, w, b, stride, padding, dilation, out_dtype=dt)
+    out = ctx.allocate(dt, *reversed(ref.shape))
+    ctx.fill_bytes(out, 0xFF)
+    ctx.ws.reset()
+    jv.convolution_(ctx, out, ctx.toback(x), ctx.toback(w), ctx.toback(b), stride[::-1], padding[::-1], dilation[::-1])
+    ctx.synchronize()
+    got = out.to_host()
+    tol = 2e-3 if dt == np.float16 else 2e-5      # as for the taps
+    assert relerr(got, ref) < tol, describe(got, ref, tol)
+
+
+def test_conv_in_words_keeps_to_its_taps(ctx, ora):
+    """An infinity or NaN beside a pixel's taps, inside the words that hold them, does not reach it."""
+    x = np.float16(np.random.default_rng(3).standard_normal((1, 2, 16, 64)))
+    w = np.float16(np.random.default_rng(4).standard_normal((8, 2, 3, 5)))
+    x[0, 0, :, 0::8] = np.inf
+    x[0, 1, :, 7::8] = np.nan
+    got = conv_gpu(ctx, x, w, None, (1, 8), (1, 0))         # taps 0..4 of words of 8: 0 is one, 7 is none
+    clean = x.copy()
+    clean[0, 1, :, 7::8] = 0
+    assert not np.isnan(got).all() and np.array_equal(np.isnan(got), np.isnan(conv_gpu(ctx, clean, w, None, (1, 8), (1, 0))))
+    got = conv_gpu(ctx, np.ascontiguousarray(x[:, 1:]), np.ascontiguousarray(w[:, 1:]), None, (1, 8), (1, 0))
+    ref = ora.conv2d(np.ascontiguousarray(clean[:, 1:]), np.ascontiguousarray(w[:, 1:]), None, (1, 8), (1, 0))
+    assert np.all(np.isfinite(got)) and relerr(got, ref) < 2e-3
+
+
+@pytest.mark.parametrize("n,d0,d1", [(2, 112, 264), (1, 8, 8), (3, 72, 56), (1, 64, 64), (1, 200, 4096)])
+def test_transposed_copy_in_words_is_exact(ctx, n, d0, d1):
+    """Tiles cut on either side, against numpy; a source one element off its boundary takes the narrow kernel, same result."""
+    a = np.float16(np.random.default_rng(d0 + d1).standard_normal((n, d0, d1)))
+    got = ctx.contiguous(ctx.toback(a).permute((1, 0, 2))).to_host()
+    assert np.array_equal(got, a.transpose(0, 2, 1))
+    flat = ctx.toback(np.concatenate([np.float16([0]), a.ravel()]))
+    off = jv.DeviceArray(ctx, flat.ptr + 2, np.float16, (d1, d0, n), owner=flat)
+    assert np.array_equal(ctx.contiguous(off.permute((1, 0, 2))).to_host(), a.transpose(0, 2, 1))
+
+
 def test_permute_bit_exact(ctx):
     rng = np.random.default_rng(5)
     a = np.float16(rng.standard_normal((2, 37, 5, 24)))         # torch (B,L,H,E) -> device (E,H,L,B)

@@ -497,8 +497,8 @@ def test_gelu_over_every_half(ctx, ora):
     finite = np.where(fin, x, np.float16(0))
     one = np.zeros((300, 8), np.float16)
     one[:, 0] = 1
-    weight = np.zeros((x.size, 8), np.float16)
-    weight[:, 0] = finite
+    weight = np.zeros((8, x.size), np.float16)
+    weight[0] = finite
     got = linear_gpu(ctx, one, weight, None, epi="gelu")       # x * 1 + zeros: the values themselves, exactly
     want = np.where(fin, alone, alone[np.flatnonzero(finite == 0)[0]])
     assert np.all(got == want[None, :])
