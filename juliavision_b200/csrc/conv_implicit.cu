@@ -26,7 +26,7 @@
 // with zeros between, the tile K-major: a thread's pixel and eight columns are one 16-byte store.  A seventh and a third more
 // columns than taps (7 x 7 / 4, 3 x 3 / 2) and a tenth of the instructions: us, before and
 // now: 1024 x 1024 x 3 -> 112, 7 x 7 / 4 24.7 -> 15.9, eight of them 166 -> 93, 512 x 512 x 3 -> 64 18.4 -> 6.4, 3 x 3 / 2
-// 256 x 256 x 32 -> 128 19.4 -> 15.8, 128 x 128 x 128 -> 256 22.5 -> 18.1.  What is left is a CTA's chain of latencies.
+// 256 x 256 x 32 -> 128 19.4 -> 9.2, 128 x 128 x 128 -> 256 22.5 -> 18.1.  What is left is a CTA's chain of latencies.
 // A small image (fewer CTAs than the GPU holds) splits the reduction over the CTAs of a cluster, whose fp32 tiles
 // meet in distributed shared memory, added in rank order.
 #include <cuda_fp16.h>
@@ -37,9 +37,6 @@
 #include "internal.h"
 #include "ptx.cuh"
 
-#ifndef CI_SPLIT
-#define CI_SPLIT 4
-#endif
 namespace b200 {
 
 constexpr int CI_PIX = 128;              // pixels per CTA (TMEM lanes)
@@ -210,8 +207,8 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
         for (int j = tid; j < BN; j += CI_GATHER)   // read in the epilogue, a barrier among these warps later
             sbias[j] = p.bias != nullptr && c0 + j < p.Cout ? __half2float(p.bias[c0 + j]) : 0.f;
         bool ok = true;
-        const uint16_t* xi = reinterpret_cast<const uint16_t*>(p.x) + (int64_t)img * p.x_img;
         if constexpr (G > 0) {
+            const uint16_t* xi = reinterpret_cast<const uint16_t*>(p.x) + (int64_t)img * p.x_img;
             // Pixel tid % 128; of a k-block's eight 16-byte pieces those of one parity.
             constexpr int VL = G / 2, RPC = 8 / G;   // elements a load, kernel rows a piece
             const int pix = tid & 127, par = tid >> 7, m = m0 + pix;
@@ -267,6 +264,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
             by[q] = m < p.P ? oh * p.sy - p.py : -(1 << 30);   // never inside the image
             base[q] = by[q] * p.W + bx[q];
         }
+        const uint16_t* xi = reinterpret_cast<const uint16_t*>(p.x) + (int64_t)img * p.x_img;
         const int row_off = warp * 128 + (((lane >> 2) ^ warp) << 4) + (lane & 3) * 4;   // row warp + 8 r: r * 1024 further
         // The taps of the warp's eight rows of a k-block, row r by lane r: offset in the image and (x, y) shift.  A row
         // past the reduction gets a shift that is never inside.
@@ -364,23 +362,25 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
             const uint32_t mine = smem_u32(smem) + (tid & 127) * 4;
             const int pix = m0 + (tid & 127);
             // four channels' loads from every part in flight together: a remote load takes a few hundred nanoseconds
-            for (int c = rank * (BN / parts) + (tid >> 7); c < (rank + 1) * (BN / parts); c += 8) {
-                float v[4][8];
+            by_act([&](auto act) {
+                for (int c = rank * (BN / parts) + (tid >> 7); c < (rank + 1) * (BN / parts); c += 8) {
+                    float v[4][8];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const uint32_t src = mapa_u32(mine + c * (CI_PIX * 4), q < parts ? q : 0);
+                    for (int q = 0; q < 8; ++q) {
+                        const uint32_t src = mapa_u32(mine + c * (CI_PIX * 4), q < parts ? q : 0);
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) v[u][q] = q < parts ? ld_cluster_f32(src + u * (2 * CI_PIX * 4)) : 0.f;
+                        for (int u = 0; u < 4; ++u) v[u][q] = q < parts ? ld_cluster_f32(src + u * (2 * CI_PIX * 4)) : 0.f;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        float o = 0.f;
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) o += v[u][q];
+                        if (pix < p.P && c0 + c + 2 * u < p.Cout)
+                            store(out0 + (int64_t)(c + 2 * u) * p.P + pix, o + sbias[c + 2 * u], act);
+                    }
                 }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    float o = 0.f;
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) o += v[u][q];
-                    if (pix < p.P && c0 + c + 2 * u < p.Cout)
-                        by_act([&](auto act) { store(out0 + (int64_t)(c + 2 * u) * p.P + pix, o + sbias[c + 2 * u], act); });
-                }
-            }
+            });
         }
         cluster_sync_all();   // nobody leaves while its tile may still be read
     }
@@ -483,11 +483,12 @@ int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64
     }
     // Channels per CTA: all of them up to 256, since every channel tile gathers the pixels again; but a launch that
     // leaves half of the GPU's CTAs unused splits the reduction, two k-blocks a part at least, which the 256-wide
-    // tile has no shared memory for.
+    // tile has no shared memory for; four a part where they are read in words and take less than a cluster's barriers
+    // (256 x 256 x 32 -> 128, 3 x 3 / 2: 15.8 us with two, 9.2).
     const int64_t tiles = p.tiles * N, room = 2 * (int64_t)ctx->prop.multiProcessorCount, nkb = cdiv((int64_t)p.CRS, CI_BK);
     int bn = Cout <= 64 ? 64 : (Cout <= 128 || (2 * tiles * cdiv(Cout, 128) <= room && nkb >= 4) ? 128 : 256), parts = 1;
     if (bn < 256)
-        while (parts < 8 && 2 * parts * tiles * cdiv(Cout, bn) <= room && nkb >= (g ? CI_SPLIT : 4) * parts) parts *= 2;
+        while (parts < 8 && 2 * parts * tiles * cdiv(Cout, bn) <= room && nkb >= (g ? 8 : 4) * parts) parts *= 2;
     CUtensorMap tw;
     uint64_t dims[2] = {(uint64_t)p.CRS, (uint64_t)Cout};
     uint64_t str[1] = {(uint64_t)ldw * 2};

@@ -4,8 +4,8 @@
 // misalignment) times a handful of tokens, where reading A once is all that should be paid.
 //
 // What bounds it: reading A, then the loads' latency (the accumulators leave room for fewer blocks per SM).  Measured
-// against the one-thread-per-output kernel that ran these before (whole calls, B200): 5 x 51865 x 1280 240 -> 37 us
-// (3.6 TB/s of A; the copy rate's floor is 20), 12 x 31751 x 928 172 -> 18.5, 17 x 1337 x 712 61 -> 8.6.
+// against the one-thread-per-output kernel that ran these before (whole calls, B200): 5 x 51865 x 1280 240 -> 34.8 us
+// (3.8 TB/s of A; the copy rate's floor is 20), 12 x 31751 x 928 172 -> 18.5, 17 x 1337 x 712 61 -> 8.6.
 //
 // Columns k and k + 8 of A are 8 * lda * 2 bytes apart, a multiple of 16, so all columns k = w (mod 8) sit at the same
 // offset s_w from a 16-byte boundary.  Warp w of a CTA takes exactly those columns and keeps its accumulators aligned
@@ -54,17 +54,6 @@ struct GrParams {
     int steps_per_cta;   // steps of GR_STEP columns each CTA of a cluster takes
 };
 
-__device__ __forceinline__ uint4 ld_l2(const char* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L2::256B.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-#ifndef GR_LD
-#define GR_LD(q) __ldg(reinterpret_cast<const uint4*>(q))
-#endif
-#ifndef GR_TAIL
-#define GR_TAIL 1
-#endif
 // grid (K parts, row blocks, token blocks), the K parts of a row block forming a cluster; 256 threads.
 template <int NT, typename OutT>
 __global__ void __launch_bounds__(32 * GR_WARPS, GrCfg<NT>::MIN_BLOCKS)
@@ -113,7 +102,7 @@ gemm_rows_kernel(const GrParams p) {
             const char* v = vec0 + j * cstep;
 #pragma unroll
             for (int mi = 0; mi < MB; ++mi)
-                a[mi][c] = in && live[mi] ? GR_LD(v + mi * 128) : make_uint4(0u, 0u, 0u, 0u);
+                a[mi][c] = in && live[mi] ? __ldg(reinterpret_cast<const uint4*>(v + mi * 128)) : make_uint4(0u, 0u, 0u, 0u);
         }
     };
 
@@ -243,9 +232,10 @@ static int gr_launch(b200_ctx* ctx, GrParams p) {
     while (parts < 8 && 2 * parts * blocks * tblocks <= room && steps >= 4 * parts) parts *= 2;
     // Row blocks past the last full round of the resident ones, less than half a round of them, are a launch of their own,
     // split along K like few row blocks are: 433 blocks of 296 take a round and a half instead of two.  (A second launch may
-    // start as the first one's blocks leave: see the kernel.)  TAIL_TIMES.
+    // start as the first one's blocks leave: see the kernel.)  5 x 51865 x 1280 37.4 -> 34.8 us, 17 x 20001 x 1024 31.5 -> 26.7,
+    // 64 x 51865 x 1280 143 -> 141.
     int64_t tail = 0, tail_parts = 1;
-    if (parts == 1 && tblocks == 1 && blocks > room && GR_TAIL) {
+    if (parts == 1 && tblocks == 1 && blocks > room) {
         tail = blocks % room;
         while (tail_parts < 8 && 2 * tail_parts * tail <= room && steps >= 4 * tail_parts) tail_parts *= 2;
         if (tail_parts == 1) tail = 0;
@@ -267,7 +257,7 @@ static int gr_launch(b200_ctx* ctx, GrParams p) {
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = second ? 2 : 1;
+        cfg.numAttrs = second && pdl_enabled() ? 2 : 1;
         ctx->launches++;
         return cudaLaunchKernelEx(&cfg, kern, p);
     };

@@ -502,3 +502,16 @@ def test_gelu_over_every_half(ctx, ora):
     got = linear_gpu(ctx, one, weight, None, epi="gelu")       # x * 1 + zeros: the values themselves, exactly
     want = np.where(fin, alone, alone[np.flatnonzero(finite == 0)[0]])
     assert np.all(got == want[None, :])
+
+
+@pytest.mark.parametrize("tokens,out,K", [(2, 35525, 512), (16, 35641, 515), (19, 20001, 1024), (33, 16577, 520), (5, 53279, 384)])
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+def test_unaligned_rows_past_the_last_full_round(ctx, ora, tokens, out, K, dt):
+    """Row blocks that fill the GPU once or more and leave one block, half a round and just more than that: the rest is a launch
+    of its own, split along K; with a bias, every row."""
+    rng = np.random.default_rng(tokens + out)
+    X, Wt, b = _case(rng, tokens, out, K, scale=0.25)
+    got = linear_gpu(ctx, X, Wt, b, out_dtype=dt)
+    ref = ora.linear(X, Wt, b, out_dtype=dt)
+    tol = 2e-3 if dt == np.float16 else 2e-5             # one rounding step of fp16; sqrt(K) eps32
+    assert relerr(got, ref) < tol, describe(got, ref, tol)
