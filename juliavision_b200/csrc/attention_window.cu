@@ -6,10 +6,11 @@
 // At this size the work per window is a megaflop and the operation is bound by HBM and by latency, not by
 // the tensor pipe: the 128-row TMEM tiles of the large kernel are mostly empty and its per-CTA set-up
 // (TMEM allocation, barriers, tensor maps) costs more than the window's arithmetic, with one CTA resident
-// per SM.  So this kernel is small instead: one CTA of four warps per 64 queries of one (window, head),
-// 27 KB of shared memory so that eight or more are resident per SM, operands fetched with plain 16-byte
-// loads (twelve in flight per thread), and each warp's 16 x 64 scores and 16 x 64 output held in registers
-// as warp-level m16n8k16 tiles.
+// per SM.  So this kernel is small instead: CTAs of four warps, four to an SM, each walking units of 64 queries of one
+// (window, head) with the next unit's operands on their way (cp.async, two buffers of 27 KB) under this one's arithmetic,
+// and each warp's 16 x 64 scores and 16 x 64 output held in registers as warp-level m16n8k16 tiles.  A CTA per unit, six to
+// an SM, alternated between loading and computing: 8192 windows x 2 heads of 64 x 64 x 56 (470 MB) 123.5 -> 115.8
+// us, 2000 x 4 of 49 x 49 x 64 57.8 -> 49.6, 4000 x 4 of 16 x 16 x 56 53.0 -> 50.3.
 #include <cuda_fp16.h>
 
 #include "internal.h"
@@ -27,6 +28,7 @@ struct WinParams {
     void* out;
     int64_t qsL, qsH, qsB, ksL, ksH, ksB, vsL, vsH, vsB, osL, osH, osB;
     int E, Lq, Lk, H, B, qtiles, out_f32;
+    int units;
     float scale_log2;
 };
 
@@ -42,50 +44,28 @@ __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// rows [0, rows) x E halves of a strided (E, L) slice into a zero-padded [64][AW_PITCH] shared tile
-__device__ __forceinline__ void win_fetch(uint4 (&r)[4], const __half* base, int64_t sL, int rows, int E, int tid) {
+__device__ __forceinline__ float win_ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// rows [0, rows) x E halves of a strided (E, L) slice on their way into a [64][AW_PITCH] shared tile, zeros elsewhere already
+__device__ __forceinline__ void win_fetch(__half* tile, const __half* base, int64_t sL, int rows, int E, int tid) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int idx = tid + i * AW_THREADS;          // 512 vectors: 64 rows x 8
         const int row = idx >> 3, vec = idx & 7;
-        r[i] = make_uint4(0u, 0u, 0u, 0u);
-        if (row < rows && vec * 8 < E) r[i] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)row * sL) + vec);
+        if (row < rows && vec * 8 < E)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(tile + row * AW_PITCH + vec * 8)),
+                         "l"(base + (int64_t)row * sL + vec * 8)
+                         : "memory");
     }
 }
 
-__device__ __forceinline__ void win_put(__half* tile, const uint4 (&r)[4], int tid) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int idx = tid + i * AW_THREADS;
-        *reinterpret_cast<uint4*>(tile + (idx >> 3) * AW_PITCH + (idx & 7) * 8) = r[i];
-    }
-}
-
-__global__ void __launch_bounds__(AW_THREADS, 6) attention_window_kernel(const WinParams p) {
-    __shared__ __align__(16) __half Qs[AW_BQ * AW_PITCH];
-    __shared__ __align__(16) __half Ks[AW_LK * AW_PITCH];
-    __shared__ __align__(16) __half Vs[AW_LK * AW_PITCH];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    int64_t u = blockIdx.x;
-    const int qt = (int)(u % p.qtiles);
-    u /= p.qtiles;
-    const int h = (int)(u % p.H);
-    const int b = (int)(u / p.H);
-    const int q0 = qt * AW_BQ;
-    const int qrows = min(AW_BQ, p.Lq - q0);
-
-    grid_dep_wait();
-    {
-        uint4 rq[4], rk[4], rv[4];
-        win_fetch(rq, p.q + (int64_t)q0 * p.qsL + (int64_t)h * p.qsH + (int64_t)b * p.qsB, p.qsL, qrows, p.E, tid);
-        win_fetch(rk, p.k + (int64_t)h * p.ksH + (int64_t)b * p.ksB, p.ksL, p.Lk, p.E, tid);
-        win_fetch(rv, p.v + (int64_t)h * p.vsH + (int64_t)b * p.vsB, p.vsL, p.Lk, p.E, tid);
-        win_put(Qs, rq, tid);
-        win_put(Ks, rk, tid);
-        win_put(Vs, rv, tid);
-    }
-    __syncthreads();
-    grid_dep_launch();
+// One unit: 64 queries of one (window, head) out of its shared tiles.
+__device__ __forceinline__ void window_unit(const WinParams& p, __half* Qs, const __half* Ks, const __half* Vs, int h, int b, int q0,
+                                            int qrows, int warp, int lane, int g, int t) {
     const int r0 = warp * 16;
     if (r0 >= qrows) return;
 
@@ -131,8 +111,8 @@ __global__ void __launch_bounds__(AW_THREADS, 6) attention_window_kernel(const W
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt) {
         // the row sum is taken over the fp16-rounded probabilities the second product uses
-        const __half2 lo = __floats2half2_rn(exp2f(s[nt][0] - m0), exp2f(s[nt][1] - m0));
-        const __half2 hi = __floats2half2_rn(exp2f(s[nt][2] - m1), exp2f(s[nt][3] - m1));
+        const __half2 lo = __floats2half2_rn(win_ex2(s[nt][0] - m0), win_ex2(s[nt][1] - m0));
+        const __half2 hi = __floats2half2_rn(win_ex2(s[nt][2] - m1), win_ex2(s[nt][3] - m1));
         const float2 flo = __half22float2(lo), fhi = __half22float2(hi);
         l0 += flo.x + flo.y;
         l1 += fhi.x + fhi.y;
@@ -183,6 +163,7 @@ __global__ void __launch_bounds__(AW_THREADS, 6) attention_window_kernel(const W
     __syncwarp();
 #pragma unroll
     for (int ne = 0; ne < 8; ++ne) {
+        if (ne * 8 >= p.E) continue;   // those columns stay zeros for the next unit, whatever this one's are
         __half* d = Qs + (r0 + g) * AW_PITCH + ne * 8 + 2 * t;
         *reinterpret_cast<uint32_t*>(d) = pack_h2(o[ne][0] * i0, o[ne][1] * i0);
         *reinterpret_cast<uint32_t*>(d + 8 * AW_PITCH) = pack_h2(o[ne][2] * i1, o[ne][3] * i1);
@@ -196,6 +177,54 @@ __global__ void __launch_bounds__(AW_THREADS, 6) attention_window_kernel(const W
         if (r0 + row < qrows && vec * 8 < p.E)
             *reinterpret_cast<uint4*>(out + (int64_t)(q0 + r0 + row) * p.osL + vec * 8) =
                 *reinterpret_cast<const uint4*>(Qs + (r0 + row) * AW_PITCH + vec * 8);
+    }
+}
+
+constexpr int AW_TILE = 64 * AW_PITCH;                 // halves of one operand's tile
+constexpr int AW_SMEM_BYTES = 2 * 3 * AW_TILE * 2;     // two buffers of Q, K and V
+constexpr int AW_CTAS_PER_SM = 4;
+static_assert(AW_BQ == 64 && AW_LK == 64, "tiles of 64 rows");
+
+__global__ void __launch_bounds__(AW_THREADS, AW_CTAS_PER_SM) attention_window_kernel(const WinParams p) {
+    extern __shared__ __align__(16) __half win_smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    struct Unit { int h, b, q0, qrows; };
+    auto unit = [&](int u) {
+        Unit a;
+        const int hb = u / p.qtiles;
+        a.b = hb / p.H;
+        a.h = hb - a.b * p.H;
+        a.q0 = (u - hb * p.qtiles) * AW_BQ;
+        a.qrows = min(AW_BQ, p.Lq - a.q0);
+        return a;
+    };
+    auto fetch = [&](const Unit& a, int buf) {
+        __half* tiles = win_smem + buf * 3 * AW_TILE;
+        win_fetch(tiles, p.q + (int64_t)a.q0 * p.qsL + (int64_t)a.h * p.qsH + (int64_t)a.b * p.qsB, p.qsL, a.qrows, p.E, tid);
+        win_fetch(tiles + AW_TILE, p.k + (int64_t)a.h * p.ksH + (int64_t)a.b * p.ksB, p.ksL, p.Lk, p.E, tid);
+        win_fetch(tiles + 2 * AW_TILE, p.v + (int64_t)a.h * p.vsH + (int64_t)a.b * p.vsB, p.vsL, p.Lk, p.E, tid);
+    };
+    // Once: what no unit's operands cover (columns past E, rows past Lk) is read as zeros, and stays so.
+    for (int i = tid; i < 6 * AW_TILE / 8; i += AW_THREADS) reinterpret_cast<uint4*>(win_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    grid_dep_wait();
+    grid_dep_launch();
+    Unit cur = unit(blockIdx.x);
+    fetch(cur, 0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    int buf = 0;
+    for (int u = blockIdx.x; u < p.units; u += gridDim.x, buf ^= 1) {
+        Unit next = cur;
+        if (u + (int)gridDim.x < p.units) {
+            next = unit(u + gridDim.x);
+            fetch(next, buf ^ 1);
+        }
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 1;" ::: "memory");
+        __syncthreads();   // every thread's copies of this unit have landed
+        __half* Qs = win_smem + buf * 3 * AW_TILE;
+        window_unit(p, Qs, Qs + AW_TILE, Qs + 2 * AW_TILE, cur.h, cur.b, cur.q0, cur.qrows, warp, lane, g, t);
+        __syncthreads();   // the buffer is free for the unit after the next
+        cur = next;
     }
 }
 
@@ -216,8 +245,16 @@ int attention_window_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     p.out_f32 = out_dtype == B200_F32;
     p.scale_log2 = scale * 1.4426950408889634f;
     const int64_t ctas = (int64_t)p.qtiles * H * B;
-    B200_REQUIRE(ctas < (1ll << 31), B200_DECLINE_EXTENT, "attention: too many windows");
-    B200_CUDA(launch_dep(attention_window_kernel, dim3((unsigned)ctas, 1, 1), dim3(AW_THREADS, 1, 1), 0, ctx->stream, 1, p));
+    B200_REQUIRE(ctas < (1ll << 30), B200_DECLINE_EXTENT, "attention: too many windows");
+    static bool attr_done[16] = {};
+    if (!attr_done[ctx->device & 15]) {
+        B200_CUDA(cudaFuncSetAttribute(attention_window_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AW_SMEM_BYTES));
+        attr_done[ctx->device & 15] = true;
+    }
+    p.units = (int)ctas;
+    const int64_t room = (int64_t)AW_CTAS_PER_SM * ctx->prop.multiProcessorCount;
+    B200_CUDA(launch_dep(attention_window_kernel, dim3((unsigned)(ctas < room ? ctas : room), 1, 1), dim3(AW_THREADS, 1, 1), AW_SMEM_BYTES,
+                         ctx->stream, 1, p));
     ctx->launches++;
     return B200_OK;
 }

@@ -1,3 +1,4 @@
+import math
 import os
 
 import numpy as np
@@ -510,3 +511,27 @@ def test_few_queries_with_smaller_clusters(ctx, ora, B, H, Lq, Lk, E, monkeypatc
         assert relerr(got, ref) < 2e-3, (most, describe(got, ref, 2e-3))     # P rounded to fp16
         assert not any(np.array_equal(got, s) for s in seen), most
         seen.append(got)
+
+
+@pytest.mark.parametrize("E,Lq,Lk,H,B,dt", [(56, 64, 64, 3, 500, np.float16), (64, 49, 49, 2, 700, np.float16), (8, 70, 5, 3, 333, np.float32),
+                                            (40, 16, 64, 5, 601, np.float16), (56, 129, 33, 2, 297, np.float16)])
+def test_windows_walked_in_turn(ctx, ora, E, Lq, Lk, H, B, dt):
+    """More units than CTAs, so that both buffers are used again: head dims and key counts that leave columns and rows of zeros,
+    query tiles of different fill next to each other, and a window of NaN that must not reach its neighbours."""
+    rng = np.random.default_rng(E + Lq + Lk)
+    q = np.float16(rng.standard_normal((B, H, Lq, E)))
+    k, v = (np.float16(rng.standard_normal((B, H, Lk, E))) for _ in range(2))
+    q[3] = np.nan
+    out = ctx.allocate(dt, E, Lq, H, B)
+    ctx.fill_bytes(out, 0xFF)
+    ctx.ws.reset()
+    jv.sdpa(ctx, ctx.toback(q), ctx.toback(k), ctx.toback(v), None, 1.0 / math.sqrt(E), out=out)
+    ctx.synchronize()
+    got = out.to_host().astype(np.float64)
+    s = np.einsum("bhqe,bhke->bhqk", q.astype(np.float64), k.astype(np.float64)) / math.sqrt(E)
+    pr = np.exp(s - s.max(-1, keepdims=True))
+    ref = np.einsum("bhqk,bhke->bhqe", pr / pr.sum(-1, keepdims=True), v.astype(np.float64))
+    assert np.all(np.isnan(got[3]))
+    keep = np.arange(B) != 3
+    # P rounded to fp16 (2^-11 relative, against values of order one), and one rounding of the result
+    assert np.all(np.isfinite(got[keep])) and np.max(np.abs(got[keep] - ref[keep])) < 5e-3
