@@ -70,7 +70,7 @@ template <int EP, bool BIAS = false, int NT_ = 2> struct AttCfg {
     static constexpr int S_V = S_K + K_STAGES * KV_BYTES;      // V_STAGES tiles
     static constexpr int S_END = S_V + V_STAGES * KV_BYTES;
     static constexpr int BIAS_TILE_BYTES = BIAS ? ATT_BR * BIAS_ROW_WORDS * 4 : 0;
-    static constexpr int SMEM_BYTES = S_END + NT * BIAS_TILE_BYTES + 320;
+    static constexpr int SMEM_BYTES = S_END + NT * BIAS_TILE_BYTES + 256;
     static_assert(CTAS_PER_SM * (SMEM_BYTES + 1024) <= 233472, "shared memory over budget");
 };
 // tensor-memory map of two tiles (512 columns): S of tile t, fp32, at [128 t, 128 t + 128); O of tile t, fp32, at
@@ -176,10 +176,11 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
     uint64_t* v_empty = v_full + V_STAGES;                 // [V_STAGES]
     uint64_t* s_full = v_empty + V_STAGES;                 // [2]
     uint64_t* s_empty = s_full + 2;                        // [2]
-    uint64_t* p_full = s_empty + 2;                        // [2 tiles][2 halves]
-    uint64_t* pv_done = p_full + 4;                        // [2]
+    uint64_t* p_full = s_empty + 2;                        // [2]
+    uint64_t* pv_done = p_full + 2;                        // [2]
     uint64_t* exp_turn = pv_done + 2;                      // [2]: whose turn it is to run its exponentials
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(exp_turn + 2);
+    uint64_t* p_half = exp_turn + 2;                       // [2]: HALVES, the first half of a block's P is written
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(exp_turn + (HALVES ? 4 : 2));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
@@ -218,8 +219,8 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             mbar_init(&q_full[t], 1);
             mbar_init(&s_full[t], 1);
             mbar_init(&s_empty[t], 4);   // one arrival per softmax warp
-            mbar_init(&p_full[2 * t], 4);
-            mbar_init(&p_full[2 * t + 1], 4);
+            mbar_init(&p_full[t], 4);
+            if (HALVES) mbar_init(&p_half[t], 4);
             mbar_init(&pv_done[t], 1);
             mbar_init(&exp_turn[t], 4);
         }
@@ -333,21 +334,24 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                 const int sv = j % V_STAGES;
                 if (!mbar_wait(&v_full[sv], (uint32_t)((j / V_STAGES) & 1), p.d_status, KST_WAIT_FULL, abort_flag)) break;
                 if (j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 7);   // issuer reaches its wait for P(j)
-                const uint32_t v_addr = smem_u32(smem + Cfg::S_V + sv * Cfg::KV_BYTES);
-                bool got = true;
-#pragma unroll
-                for (int hf = 0; hf < (HALVES ? 2 : 1); ++hf) {
-                    if (got) got = mbar_wait(&p_full[2 * t + (HALVES ? hf : 1)], (uint32_t)(j & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag);
-                    if (!got) break;
+                constexpr int FIRST = HALVES ? BC / 32 : 0;   // steps that do not wait for the whole of P
+                if constexpr (HALVES) {
+                    if (!mbar_wait(&p_half[t], (uint32_t)(j & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag)) break;
                     tc_fence_after();
+                    const uint32_t v_addr = smem_u32(smem + Cfg::S_V + sv * Cfg::KV_BYTES);
 #pragma unroll
-                    for (int k = hf * (BC / 32); k < (HALVES ? (hf + 1) * (BC / 32) : BC / 16); ++k) {
-                        // P comes from tensor memory: 16 keys = 8 packed columns per step.
-                        // V: 16 key rows = two 8-row groups = 2048 B.
+                    for (int k = 0; k < FIRST; ++k)
                         umma_ts(o_tmem, p_tmem + k * 8, smem_desc_at(vdesc0, v_addr + k * 2048), idesc_o, (j | k) != 0);
-                    }
                 }
-                if (!got) break;
+                if (!mbar_wait(&p_full[t], (uint32_t)(j & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag)) break;
+                tc_fence_after();
+                const uint32_t v_addr = smem_u32(smem + Cfg::S_V + sv * Cfg::KV_BYTES);
+#pragma unroll
+                for (int k = FIRST; k < BC / 16; ++k) {
+                    // P comes from tensor memory: 16 keys = 8 packed columns per step.
+                    // V: 16 key rows = two 8-row groups = 2048 B.
+                    umma_ts(o_tmem, p_tmem + k * 8, smem_desc_at(vdesc0, v_addr + k * 2048), idesc_o, (j | k) != 0);
+                }
                 umma_commit(&pv_done[t]);
                 umma_commit(&v_empty[sv]);   // one of `ntiles` arrivals that free this V stage
                 if (j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 1);   // P V(j) issued
@@ -590,7 +594,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                         tmem_wait_st();
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(&p_full[2 * t]);
+                        if (lane == 0) mbar_arrive(&p_half[t]);
                     }
                 }
                 tmem_wait_st();
@@ -600,7 +604,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                 m_run = m_new;
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&p_full[2 * t + 1]);
+                if (lane == 0) mbar_arrive(&p_full[t]);
                 if (lane == 0 && quad == 0 && j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 6);  // P written
                 if (lane == 0 && j == 3) ATT_TRACE(56 + 64 * t + quad);                  // per-warp P written, block 3
             }
