@@ -1,3 +1,4 @@
+import math
 import os
 
 import numpy as np
@@ -502,6 +503,23 @@ def test_gelu_over_every_half(ctx, ora):
     got = linear_gpu(ctx, one, weight, None, epi="gelu")       # x * 1 + zeros: the values themselves, exactly
     want = np.where(fin, alone, alone[np.flatnonzero(finite == 0)[0]])
     assert np.all(got == want[None, :])
+
+
+def test_gelu_of_large_negative_values_goes_to_zero(ctx):
+    """fp32 results below -6, from every product's store: no further from x Phi(x) than 0 is (the 7.1.26
+    steps give 0 there), but for one step of the smallest float times nine."""
+    x = -np.float16(2.0) ** np.linspace(np.log2(6.01), 15.9, 400).astype(np.float16)
+    x = np.concatenate([x, np.float16([-6.004, -8.992, -9.0, -9.008, -65504.0])])
+    x = np.concatenate([x, np.zeros(-x.size % 8, np.float16)])
+    exact = np.array([0.5 * float(t) * math.erfc(-float(t) / math.sqrt(2)) for t in x])
+    got = []
+    for tokens, out in ((1, x.size), (3, x.size), (300, x.size), (5, x.size - 1)):      # row, few rows, tiles, unaligned rows
+        one, weight = np.zeros((tokens, 128), np.float16), np.zeros((128, out), np.float16)
+        one[:, 0], weight[0] = 1, x[:out]
+        got += list(linear_gpu(ctx, one, weight, None, epi="gelu", out_dtype=np.float32)[[0, -1]])
+    for g in got:
+        e = exact[:g.size]
+        assert np.all(np.abs(g.astype(np.float64) - e) <= np.abs(e) + 2e-44)
 
 
 @pytest.mark.parametrize("tokens,out,K", [(2, 35525, 512), (16, 35641, 515), (19, 20001, 1024), (33, 16577, 520), (5, 53279, 384)])
