@@ -28,7 +28,7 @@ struct WinParams {
     void* out;
     int64_t qsL, qsH, qsB, ksL, ksH, ksB, vsL, vsH, vsB, osL, osH, osB;
     int E, Lq, Lk, H, B, qtiles, out_f32;
-    int units;
+    uint32_t units;
     float scale_log2;
 };
 
@@ -189,12 +189,12 @@ __global__ void __launch_bounds__(AW_THREADS, AW_CTAS_PER_SM) attention_window_k
     extern __shared__ __align__(16) __half win_smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     struct Unit { int h, b, q0, qrows; };
-    auto unit = [&](int u) {
+    auto unit = [&](uint32_t u) {
         Unit a;
-        const int hb = u / p.qtiles;
+        const int hb = (int)(u / (uint32_t)p.qtiles);
         a.b = hb / p.H;
         a.h = hb - a.b * p.H;
-        a.q0 = (u - hb * p.qtiles) * AW_BQ;
+        a.q0 = (int)(u - (uint32_t)hb * (uint32_t)p.qtiles) * AW_BQ;
         a.qrows = min(AW_BQ, p.Lq - a.q0);
         return a;
     };
@@ -213,9 +213,9 @@ __global__ void __launch_bounds__(AW_THREADS, AW_CTAS_PER_SM) attention_window_k
     fetch(cur, 0);
     asm volatile("cp.async.commit_group;" ::: "memory");
     int buf = 0;
-    for (int u = blockIdx.x; u < p.units; u += gridDim.x, buf ^= 1) {
+    for (uint32_t u = blockIdx.x; u < p.units; u += gridDim.x, buf ^= 1) {   // below 2^31 and a step: no wrap
         Unit next = cur;
-        if (u + (int)gridDim.x < p.units) {
+        if (u + gridDim.x < p.units) {
             next = unit(u + gridDim.x);
             fetch(next, buf ^ 1);
         }
@@ -245,13 +245,13 @@ int attention_window_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     p.out_f32 = out_dtype == B200_F32;
     p.scale_log2 = scale * 1.4426950408889634f;
     const int64_t ctas = (int64_t)p.qtiles * H * B;
-    B200_REQUIRE(ctas < (1ll << 30), B200_DECLINE_EXTENT, "attention: too many windows");
+    B200_REQUIRE(ctas < (1ll << 31), B200_DECLINE_EXTENT, "attention: too many windows");
     static bool attr_done[16] = {};
     if (!attr_done[ctx->device & 15]) {
         B200_CUDA(cudaFuncSetAttribute(attention_window_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AW_SMEM_BYTES));
         attr_done[ctx->device & 15] = true;
     }
-    p.units = (int)ctas;
+    p.units = (uint32_t)ctas;
     const int64_t room = (int64_t)AW_CTAS_PER_SM * ctx->prop.multiProcessorCount;
     B200_CUDA(launch_dep(attention_window_kernel, dim3((unsigned)(ctas < room ? ctas : room), 1, 1), dim3(AW_THREADS, 1, 1), AW_SMEM_BYTES,
                          ctx->stream, 1, p));

@@ -535,3 +535,19 @@ def test_windows_walked_in_turn(ctx, ora, E, Lq, Lk, H, B, dt):
     keep = np.arange(B) != 3
     # P rounded to fp16 (2^-11 relative, against values of order one), and one rounding of the result
     assert np.all(np.isfinite(got[keep])) and np.max(np.abs(got[keep] - ref[keep])) < 5e-3
+
+
+def test_more_than_2_to_the_30_windows(ctx):
+    """Heads x batch past 2^30, which the walk over the windows counts: one query and one key each, so that the result is v,
+    out of operands that overlap; 17 GB of results, a few planes of them read back."""
+    E, H, B = 8, 65535, 16385
+    v = np.float16(np.random.default_rng(30).standard_normal(8 * (H + B)))
+    d = ctx.toback(v)
+    view = jv.DeviceArray(ctx, d.ptr, np.float16, (E, 1, H, B), (1, 8, 8, 8), owner=d)
+    out = ctx.allocate(np.float16, E, 1, H, B)
+    ctx.fill_bytes(out, 0xFF)
+    jv.sdpa(ctx, view, view, view, None, 1.0, out=out)
+    ctx.synchronize()
+    for b in (0, 1, 8191, 8192, 16383, 16384):
+        plane = jv.DeviceArray(ctx, out.ptr + b * H * E * 2, np.float16, (E, H), owner=out)
+        assert np.array_equal(plane.to_host(), v[8 * b:8 * (b + H)].reshape(H, E)), b
