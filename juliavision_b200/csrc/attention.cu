@@ -1023,7 +1023,7 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
         attr_done[ctx->device & 15] = true;
     }
     // Many windows of at most 64 keys: bound by HBM and latency, not by the tensor pipe; the small-tile
-    // kernel keeps six CTAs per SM in flight where this one's set-up would cost more than the arithmetic.
+    // kernel keeps four or six CTAs per SM in flight where this one's set-up would cost more than the arithmetic.
     if (bptr == nullptr && E <= 64 && Lk <= 64 && B * H * cdiv(Lq, 64) > 2 * ctx->prop.multiProcessorCount)
         return attention_window_launch(ctx, E, Lq, Lk, H, B, q, k, v, o, out_dtype, scale);
     // A few queries: their tile would be mostly empty (see attention_few.cu).

@@ -6,11 +6,12 @@
 // At this size the work per window is a megaflop and the operation is bound by HBM and by latency, not by
 // the tensor pipe: the 128-row TMEM tiles of the large kernel are mostly empty and its per-CTA set-up
 // (TMEM allocation, barriers, tensor maps) costs more than the window's arithmetic, with one CTA resident
-// per SM.  So this kernel is small instead: CTAs of four warps, four to an SM, each walking units of 64 queries of one
-// (window, head) with the next unit's operands on their way (cp.async, two buffers of 27 KB) under this one's arithmetic,
-// and each warp's 16 x 64 scores and 16 x 64 output held in registers as warp-level m16n8k16 tiles.  A CTA per unit, six to
-// an SM, alternated between loading and computing: 8192 windows x 2 heads of 64 x 64 x 56 (470 MB) 123.5 -> 115.8
-// us, 2000 x 4 of 49 x 49 x 64 57.8 -> 49.6, 4000 x 4 of 16 x 16 x 56 53.0 -> 50.3.
+// per SM.  So this kernel is small instead: CTAs of four warps, operands fetched with cp.async, and each warp's 16 x 64 scores
+// and 16 x 64 output held in registers as warp-level m16n8k16 tiles.  A CTA takes one unit, 64 queries of one (window, head),
+// six CTAs to an SM; or, where there are more units of many keys than that, four CTAs to an SM walk the units with the next
+// one's operands on their way (two buffers of 27 KB) under this one's arithmetic.
+// Microseconds, replayed (a unit a CTA with loads through registers / walking / now): 8192 windows x 2 heads of 64 x 64 x 56
+// (470 MB) 118.6 / 107.1 / 106.3, 2000 x 4 of 49 x 49 x 64 57.2 / 49.9 / 49.6, 600 x 4 of 16 x 16 x 56 9.9 / 9.6 / 8.5.
 #include <cuda_fp16.h>
 
 #include "internal.h"
@@ -181,11 +182,14 @@ __device__ __forceinline__ void window_unit(const WinParams& p, __half* Qs, cons
 }
 
 constexpr int AW_TILE = 64 * AW_PITCH;                 // halves of one operand's tile
-constexpr int AW_SMEM_BYTES = 2 * 3 * AW_TILE * 2;     // two buffers of Q, K and V
-constexpr int AW_CTAS_PER_SM = 4;
+constexpr int AW_BUF_BYTES = 3 * AW_TILE * 2;          // one buffer of Q, K and V
+constexpr int AW_CTAS_PER_SM = 4;                      // walking, two buffers
+constexpr int AW_CTAS_PER_SM_ONE = 6;                  // a unit per CTA, one buffer
 static_assert(AW_BQ == 64 && AW_LK == 64, "tiles of 64 rows");
 
-__global__ void __launch_bounds__(AW_THREADS, AW_CTAS_PER_SM) attention_window_kernel(const WinParams p) {
+// WALK: the grid's CTAs walk the units, two buffers each; else a CTA takes the one unit of its index.
+template <bool WALK>
+__global__ void __launch_bounds__(AW_THREADS, WALK ? AW_CTAS_PER_SM : AW_CTAS_PER_SM_ONE) attention_window_kernel(const WinParams p) {
     extern __shared__ __align__(16) __half win_smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     struct Unit { int h, b, q0, qrows; };
@@ -203,23 +207,38 @@ __global__ void __launch_bounds__(AW_THREADS, AW_CTAS_PER_SM) attention_window_k
         win_fetch(tiles, p.q + (int64_t)a.q0 * p.qsL + (int64_t)a.h * p.qsH + (int64_t)a.b * p.qsB, p.qsL, a.qrows, p.E, tid);
         win_fetch(tiles + AW_TILE, p.k + (int64_t)a.h * p.ksH + (int64_t)a.b * p.ksB, p.ksL, p.Lk, p.E, tid);
         win_fetch(tiles + 2 * AW_TILE, p.v + (int64_t)a.h * p.vsH + (int64_t)a.b * p.vsB, p.vsL, p.Lk, p.E, tid);
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    // Once: what no unit's operands cover (columns past E, rows past Lk) is read as zeros, and stays so.
-    for (int i = tid; i < 6 * AW_TILE / 8; i += AW_THREADS) reinterpret_cast<uint4*>(win_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
+    // Once: what no unit's copies cover (columns past E, keys past Lk) is read as zeros, and stays so.  Queries past a tile's
+    // last give rows that are not stored.
+#pragma unroll
+    for (int tile = 0; tile < (WALK ? 6 : 3); ++tile)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = (tid >> 3) + 16 * i, vec = tid & 7;
+            if (vec * 8 >= p.E || (tile % 3 != 0 && row >= p.Lk))
+                *reinterpret_cast<uint4*>(win_smem + tile * AW_TILE + row * AW_PITCH + vec * 8) = make_uint4(0u, 0u, 0u, 0u);
+        }
     grid_dep_wait();
     grid_dep_launch();
     Unit cur = unit(blockIdx.x);
     fetch(cur, 0);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    if constexpr (!WALK) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        window_unit(p, win_smem, win_smem + AW_TILE, win_smem + 2 * AW_TILE, cur.h, cur.b, cur.q0, cur.qrows, warp, lane, g, t);
+        return;
+    }
     int buf = 0;
-    for (uint32_t u = blockIdx.x; u < p.units; u += gridDim.x, buf ^= 1) {   // below 2^31 and a step: no wrap
+    for (uint32_t u = blockIdx.x; u < p.units; u += gridDim.x, buf ^= 1) {
         Unit next = cur;
         if (u + gridDim.x < p.units) {
             next = unit(u + gridDim.x);
             fetch(next, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
-        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 1;" ::: "memory");
         __syncthreads();   // every thread's copies of this unit have landed
         __half* Qs = win_smem + buf * 3 * AW_TILE;
         window_unit(p, Qs, Qs + AW_TILE, Qs + 2 * AW_TILE, cur.h, cur.b, cur.q0, cur.qrows, warp, lane, g, t);
@@ -244,17 +263,28 @@ int attention_window_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     p.qtiles = (int)cdiv(Lq, AW_BQ);
     p.out_f32 = out_dtype == B200_F32;
     p.scale_log2 = scale * 1.4426950408889634f;
-    const int64_t ctas = (int64_t)p.qtiles * H * B;
-    B200_REQUIRE(ctas < (1ll << 31), B200_DECLINE_EXTENT, "attention: too many windows");
+    const int64_t units = (int64_t)p.qtiles * H * B, sms = ctx->prop.multiProcessorCount;
+    B200_REQUIRE(units < (1ll << 31), B200_DECLINE_EXTENT, "attention: too many windows");
+    p.units = (uint32_t)units;
+    // A walking CTA of a single unit only pays for its second buffer, and one of two takes longer than six CTAs side by side; of
+    // few keys there is little to fetch ahead.  Between three and four units an SM both take the same alone, and back to back
+    // walking CTAs, which leave no room for the next launch's, spread evenly.  Microseconds on 148 SMs, a unit a CTA / walking,
+    // each launch behind another kernel: 300 units of 64 x 64 x 56 6.2 / 6.2 (6.7 with every buffer zeroed whole), 592 7.1 / 7.2
+    // (back to back 7.0 / 5.8), 800 8.6 / 9.0, 888 8.7 / 9.8, 1040 11.1 / 10.7, 1200 12.4 / 11.7; 16 x 16 x 56: 300 4.5 / 4.6,
+    // 800 5.3 / 6.2, 1800 8.2 / 9.4, 16000 51.1 / 51.2.
+    if (Lk <= 32 || units <= 3 * sms || (units > AW_CTAS_PER_SM * sms && units <= AW_CTAS_PER_SM_ONE * sms)) {
+        B200_CUDA(launch_dep(attention_window_kernel<false>, dim3((unsigned)units, 1, 1), dim3(AW_THREADS, 1, 1), AW_BUF_BYTES, ctx->stream, 1, p));
+        ctx->launches++;
+        return B200_OK;
+    }
     static bool attr_done[16] = {};
     if (!attr_done[ctx->device & 15]) {
-        B200_CUDA(cudaFuncSetAttribute(attention_window_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AW_SMEM_BYTES));
+        B200_CUDA(cudaFuncSetAttribute(attention_window_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * AW_BUF_BYTES));
         attr_done[ctx->device & 15] = true;
     }
-    p.units = (uint32_t)ctas;
-    const int64_t room = (int64_t)AW_CTAS_PER_SM * ctx->prop.multiProcessorCount;
-    B200_CUDA(launch_dep(attention_window_kernel, dim3((unsigned)(ctas < room ? ctas : room), 1, 1), dim3(AW_THREADS, 1, 1), AW_SMEM_BYTES,
-                         ctx->stream, 1, p));
+    const int64_t room = AW_CTAS_PER_SM * sms;
+    B200_CUDA(launch_dep(attention_window_kernel<true>, dim3((unsigned)(units < room ? units : room), 1, 1), dim3(AW_THREADS, 1, 1),
+                         2 * AW_BUF_BYTES, ctx->stream, 1, p));
     ctx->launches++;
     return B200_OK;
 }
