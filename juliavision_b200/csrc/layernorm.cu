@@ -420,7 +420,7 @@ ln_add_warp_kernel(__half* __restrict__ x, const __half* __restrict__ h, __half*
 // or more 16-byte loads in flight (2 R with the residual add in front, ADD) and gamma and beta are read once for all of them.
 // Bound by HBM; with one row at a time the loads in flight were what bound it: 524288 x 112 fp16 69.0 -> 54.9 us (4.3 TB/s),
 // 131072 x 224 35.6 -> 29.9, 200000 x 200 53.0 -> 43.3; behind the add 524288 x 112 86.2 -> 78.9 (6.0 TB/s), 32768 x 448
-// 23.1 -> 20.6.  Eight rows lose (63.7: registers).  Alone, rows of two vectors a lane do not gain (32768 x 448 14.1 both
+// 23.1 -> 20.6; smaller launches: ln_fills.  Eight rows lose (63.7: registers).  Alone, rows of two vectors a lane do not gain (32768 x 448 14.1 both
 // ways, 16384 x 448 7.1 -> 7.4) and stay with ln_warp_kernel.  A row is kept as read (fp16 stays packed,
 // also the sum x + h, which add.Tensor rounds to fp16), every operation and its order is that of the kernels
 // above, hence the same bits.  The R rows' statistics leave in one store each.
@@ -701,10 +701,15 @@ static bool ln_packs(int64_t groups, int64_t C) { return groups * C >= (int64_t)
 // instructions save; five and six gain (50000 x 1280: 51.8 -> 49.1, 43000 x 1480: 55.2 -> 52.1).
 constexpr bool ln_pack_width(int vpl) { return vpl == 5 || vpl == 6; }
 
-// Rows of one vector a lane, `lpg` lanes each: four of them per group of lanes while that leaves eight blocks an SM, else two
-// (3000 x 112: 3.42 us one at a time, 3.04 two, 3.12 four; 524288 x 112: 69.0, 61.7, 54.9).
-static bool ln_four_rows(const b200_ctx* ctx, int64_t groups, int lpg) {
-    return groups >= (int64_t)8 * ctx->prop.multiProcessorCount * 4 * 4 * (32 / lpg);
+// Whether a launch of `rows` rows a group of `lpg` lanes fills every SM with `n` blocks of four warps: the rule for the kernel of
+// several rows.  Its loads in flight pay where bytes bound the launch, its longer chain costs where latency does.  Microseconds,
+// each launch behind another kernel, one row / two / four, 148 SMs: fp16 rows of 112 15000 4.1 / 4.7 / 5.2, 38000 (16 blocks of
+// two) 7.3 / 6.9 / 7.3, 60000 (12 blocks of four) 10.3 / 9.7 / 9.4, of 64 24000 3.9 / 4.0 / 4.4, 150000 12.8 / 12.3 / 11.6; fp32 of
+// 128 9500 (8 blocks of two) 4.5 / 4.5 / 4.9, 15000 5.7 / 5.2 / 5.9, 24000 8.1 / 6.6 / 6.7, 100000 28.7 / 21.4 / 20.4; behind the
+// add, 112 24000 6.2 / 6.5 / 7.0, 70000 (30) 14.8 / 14.4 / 14.5, 150000 27.3 / 26.2 / 25.4; two vectors a lane, 448 9500 (8)
+// 7.6 / 7.8, 14000 12.7 / 11.4.
+static bool ln_fills(const b200_ctx* ctx, int64_t groups, int rows, int lpg, int64_t n) {
+    return groups >= n * ctx->prop.multiProcessorCount * 4 * rows * (32 / lpg);
 }
 
 template <typename InT, typename OutT>
@@ -740,9 +745,6 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
             B200_CUDA(launch_dep(ln_warp_kernel<InT, OutT, V>, grid, block, 0, ctx->stream, 1, ap, op, mean, rstd, gp, bp, \
                                  groups, (int)C, eps));                                                     \
     } while (0)
-#define LN_GO_LAT(V)                                                                                        \
-    B200_CUDA(launch_dep(ln_warp_kernel<InT, OutT, V, 32, true>, grid, block, 0, ctx->stream, 1, ap, op, mean, rstd, gp, bp, \
-                         groups, (int)C, eps))
 #define LN_GO_SHARED(L)                                                                                     \
     B200_CUDA(launch_dep(ln_warp_kernel<InT, OutT, 1, L>, dim3((unsigned)cdiv(groups, wpb * (32 / L))), block, 0,   \
                          ctx->stream, 1, ap, op, mean, rstd, gp, bp, groups, (int)C, eps))
@@ -750,17 +752,15 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
     B200_CUDA(launch_dep(ln_rows_kernel<InT, OutT, V, L, R, false>, dim3((unsigned)cdiv(groups, wpb * R * (32 / L))), block, 0, \
                          ctx->stream, 1, ap, (InT*)nullptr, (const InT*)nullptr, op, mean, rstd, gp, bp, groups, (int)C, eps, 0, \
                          0.f, 0.f))
-#define LN_GO_ROWS1(L)                                                                                      \
+#define LN_GO_NARROW(L, ONE)                                                                                \
     do {                                                                                                    \
-        if (ln_four_rows(ctx, groups, L)) LN_GO_ROWS(1, L, 4);                                              \
-        else LN_GO_ROWS(1, L, 2);                                                                           \
+        if (ln_fills(ctx, groups, 4, L, 12)) LN_GO_ROWS(1, L, 4);                                           \
+        else if (ln_fills(ctx, groups, 2, L, sizeof(InT) == 4 ? 10 : 14)) LN_GO_ROWS(1, L, 2);              \
+        else ONE;                                                                                           \
     } while (0)
-        if (!lat && nvec <= 8) LN_GO_ROWS1(8);
-        else if (!lat && nvec <= 16) LN_GO_ROWS1(16);
-        else if (!lat && vpl <= 1) LN_GO_ROWS1(32);
-        else if (nvec <= 8) LN_GO_SHARED(8);
-        else if (nvec <= 16) LN_GO_SHARED(16);
-        else if (vpl <= 1) LN_GO_LAT(1);
+        if (nvec <= 8) LN_GO_NARROW(8, LN_GO_SHARED(8));
+        else if (nvec <= 16) LN_GO_NARROW(16, LN_GO_SHARED(16));
+        else if (vpl <= 1) LN_GO_NARROW(32, LN_GO(1));
         else if (vpl <= 2) LN_GO(2);
         else if (vpl <= 3) LN_GO(3);
         else if (vpl <= 4) LN_GO(4);
@@ -777,9 +777,8 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
                                  op, mean, rstd, gp, bp, (int)C, eps));
 #undef LN_GO
 #undef LN_GO_SHARED
-#undef LN_GO_LAT
 #undef LN_GO_ROWS
-#undef LN_GO_ROWS1
+#undef LN_GO_NARROW
     } else {
         ln_block_kernel<InT, OutT><<<(unsigned)groups, 256, 0, ctx->stream>>>(ap, op, mean, rstd, gp, bp,
                                                                              C, eps);
@@ -831,9 +830,6 @@ extern "C" int b200_add_layernorm_f16(b200_ctx* ctx, int64_t groups, int64_t C, 
                                  (__half*)out, mean, rstd, (const __half*)gamma, (const __half*)beta, groups, (int)C, eps, \
                                  use_clamp, lo, hi));                                                             \
     } while (0)
-#define LNA_GO_LAT(V)                                                                                             \
-    B200_CUDA(launch_dep(ln_add_warp_kernel<V, 32, true>, grid, block, 0, ctx->stream, 1, (__half*)x, (const __half*)h, (__half*)out, \
-                         mean, rstd, (const __half*)gamma, (const __half*)beta, groups, (int)C, eps, use_clamp, lo, hi))
 #define LNA_GO_SHARED(L)                                                                                          \
     B200_CUDA(launch_dep(ln_add_warp_kernel<1, L>, dim3((unsigned)cdiv(groups, wpb * (32 / L))), block, 0, ctx->stream, 1, \
                          (__half*)x, (const __half*)h, (__half*)out, mean, rstd, (const __half*)gamma,             \
@@ -842,19 +838,17 @@ extern "C" int b200_add_layernorm_f16(b200_ctx* ctx, int64_t groups, int64_t C, 
     B200_CUDA(launch_dep(ln_rows_kernel<__half, __half, V, L, R, true>, dim3((unsigned)cdiv(groups, wpb * R * (32 / L))), block, 0, \
                          ctx->stream, 1, (const __half*)nullptr, (__half*)x, (const __half*)h, (__half*)out, mean, rstd, \
                          (const __half*)gamma, (const __half*)beta, groups, (int)C, eps, use_clamp, lo, hi))
-#define LNA_GO_ROWS1(L)                                                                                           \
+#define LNA_GO_NARROW(L, ONE)                                                                                     \
     do {                                                                                                          \
-        if (ln_four_rows(ctx, groups, L)) LNA_GO_ROWS(1, L, 4);                                                   \
-        else LNA_GO_ROWS(1, L, 2);                                                                                \
+        if (ln_fills(ctx, groups, 4, L, 24)) LNA_GO_ROWS(1, L, 4);                                                \
+        else if (ln_fills(ctx, groups, 2, L, 20)) LNA_GO_ROWS(1, L, 2);                                           \
+        else ONE;                                                                                                 \
     } while (0)
-    if (!lat && nvec <= 8) LNA_GO_ROWS1(8);
-    else if (!lat && nvec <= 16) LNA_GO_ROWS1(16);
-    else if (!lat && vpl <= 1) LNA_GO_ROWS1(32);
-    else if (!lat && vpl <= 2) LNA_GO_ROWS(2, 32, 2);
-    else if (nvec <= 8) LNA_GO_SHARED(8);
-    else if (nvec <= 16) LNA_GO_SHARED(16);
-    else if (vpl <= 1) LNA_GO_LAT(1);
-    else if (vpl <= 2) LNA_GO_LAT(2);
+    if (nvec <= 8) LNA_GO_NARROW(8, LNA_GO_SHARED(8));
+    else if (nvec <= 16) LNA_GO_NARROW(16, LNA_GO_SHARED(16));
+    else if (vpl <= 1) LNA_GO_NARROW(32, LNA_GO(1));
+    else if (vpl <= 2 && ln_fills(ctx, groups, 2, 32, 10)) LNA_GO_ROWS(2, 32, 2);
+    else if (vpl <= 2) LNA_GO(2);
     else if (vpl <= 3) LNA_GO(3);
     else if (vpl <= 4) LNA_GO(4);
     else if (vpl <= 5) LNA_GO(5);
@@ -864,9 +858,8 @@ extern "C" int b200_add_layernorm_f16(b200_ctx* ctx, int64_t groups, int64_t C, 
     else LNA_GO(16);
 #undef LNA_GO
 #undef LNA_GO_SHARED
-#undef LNA_GO_LAT
 #undef LNA_GO_ROWS
-#undef LNA_GO_ROWS1
+#undef LNA_GO_NARROW
     ctx->launches++;
     B200_CUDA(cudaGetLastError());
     return B200_OK;

@@ -153,10 +153,14 @@ def test_only_the_widths_that_gain_take_the_packed_form(ctx, C, same):
 @pytest.mark.parametrize("dt,C,groups", [(np.float16, 8, 2369), (np.float16, 64, 75779), (np.float16, 72, 37887), (np.float16, 112, 37891),
                                          (np.float16, 128, 2371), (np.float16, 136, 18943), (np.float16, 256, 18947),
                                          (np.float32, 28, 37889), (np.float32, 128, 18945), (np.float16, 264, 2369),
-                                         (np.float16, 512, 2370)])
+                                         (np.float16, 512, 2370),
+                                         # two and four rows on either side of their rules, alone and behind the add
+                                         (np.float16, 8, 113665), (np.float16, 56, 227331), (np.float16, 120, 56831), (np.float16, 128, 113667),
+                                         (np.float16, 248, 28419), (np.float16, 256, 56835), (np.float32, 28, 113667), (np.float32, 60, 23681),
+                                         (np.float32, 128, 28417), (np.float16, 264, 11841), (np.float16, 512, 11845)])
 def test_several_narrow_rows_at_a_time(ctx, ora, dt, C, groups):
-    """Widths at both ends of a row's lanes, row counts that leave a last group short and on either side of the rule for
-    four rows: the oracle's values, and bit for bit what one row at a time (a launch of few rows) gives; with fp16 also
+    """Widths at both ends of a row's lanes, row counts that leave a last group short and on either side of the rules for
+    two and four rows: the oracle's values, and bit for bit what one row at a time (a launch of few rows) gives; with fp16 also
     behind the residual add."""
     rng = np.random.default_rng(C + groups)
     a = (rng.standard_normal((groups, C), dtype=np.float32) * 2 + 0.5).astype(dt)
