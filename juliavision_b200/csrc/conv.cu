@@ -151,11 +151,10 @@ static int conv2d_group(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_
     bool implicit = conv_implicit_takes(W, H, Cin, N, KW, KH, Cout, P) &&
                     (onebyone ? !gemm_1x1 : !aligned || cdiv(P, 128) * N >= 2 * ctx->prop.multiProcessorCount);
     const size_t ws_mark = ctx->ws_used;
-    // An even stride over rows of whole words: the implicit kernel reads the image in words, whatever the image's size.  Its
+    // An even stride over rows of whole words: the implicit kernel reads the image in words where that gains.  Its
     // weight takes a workspace; refused (a graph recorded without an eager call before), the call goes on as it did.
-    // Not where laying out the weight is more than reading the image (34 x 34 x 256 -> 256, 3 x 3 / 2: 14.3 us, 15.1 in words).
     const int words = conv_implicit_takes(W, H, Cin, N, KW > 8 ? KW : 8, KH, Cout, P) ? conv_words(W, KW, sx, px, dx, x, x_img) : 0;
-    if (words && conv_words_ldw(Cin * KH, words) * Cout <= N * Cin * W * H) {
+    if (words && conv_words_gains(ctx, W, H, Cin, N, KW, KH, Cout, P, words, implicit)) {
         void* wp = nullptr;
         rc = ws_scratch(ctx, (size_t)(conv_words_ldw(Cin * KH, words) * Cout) * 2, &wp);
         if (rc && rc != B200_ENOMEM) return rc;

@@ -421,7 +421,7 @@ bool conv_implicit_takes(int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t K
 int conv_words(int64_t W, int64_t KW, int64_t sx, int64_t px, int64_t dx, const void* x, int64_t x_img) {
     for (const int64_t word : {4, 2}) {
         const int64_t lead = (word - px % word) % word;
-        if (sx % word == 0 && W % word == 0 && x_img % word == 0 && (dx == 1 || KW == 1) && reinterpret_cast<uintptr_t>(x) % (2 * word) == 0 &&
+        if (sx % word == 0 && W % word == 0 && x_img % word == 0 && dx == 1 && reinterpret_cast<uintptr_t>(x) % (2 * word) == 0 &&
             KW + lead > word && KW + lead <= 2 * word)
             return (int)(2 * word);
     }
@@ -449,6 +449,41 @@ int conv_words_weight(b200_ctx* ctx, void* dst, const void* w, int64_t KW, int64
                          (__half*)dst, (const __half*)w, (int)KW, g, (int)((word - px % word) % word), (int)rows, (int)ldw, n));
     ctx->launches++;
     return B200_OK;
+}
+
+// Channels per CTA: all of them up to 256, since every channel tile gathers the pixels again; but a launch that
+// leaves half of the GPU's CTAs unused splits the reduction, two k-blocks a part at least, which the 256-wide
+// tile has no shared memory for; four a part where they are read in words and take less than a cluster's barriers
+// (256 x 256 x 32 -> 128, 3 x 3 / 2: 15.8 us with two, 9.2).  tiles: pixel tiles of all images; cols: of the reduction.
+struct CiTiles { int bn, parts; int64_t nkb; };
+static CiTiles ci_tiles(const b200_ctx* ctx, int64_t tiles, int64_t cols, int64_t Cout, int g) {
+    const int64_t room = 2 * (int64_t)ctx->prop.multiProcessorCount, nkb = cdiv(cols, CI_BK);
+    CiTiles t = {Cout <= 64 ? 64 : (Cout <= 128 || (2 * tiles * cdiv(Cout, 128) <= room && nkb >= 4) ? 128 : 256), 1, nkb};
+    if (t.bn < 256)
+        while (t.parts < 8 && 2 * t.parts * tiles * cdiv(Cout, t.bn) <= room && nkb >= (g ? 8 : 4) * t.parts) t.parts *= 2;
+    return t;
+}
+
+// Which of the convolutions that can be read in words gain by it.  Not where laying out the weight is more than reading the
+// image (34 x 34 x 256 -> 256, 3 x 3 / 2: 14.3 us, 15.1 in words), nor a kernel no wider than a word, half of whose columns are
+// zeros, on a short reduction (72 x 66 x 16 -> 8, 2 x 2 / 2 padded by 1: 4.5 us by taps, 5.2).  The implicit kernel by taps loses to
+// it otherwise (`taps`; 560 x 556 x 3 -> 32, 7 x 7 / 4: 12.2 us, 6.8); against the im2col matrix of a small image the cheaper one
+// is taken, in microseconds as fitted to 280 convolutions of 16 to 512 pixels a side, 1 to 384 -> 8 to 512 channels: the first
+// moves and multiplies more, the second has a long chain a CTA (64 x 60 x 64 -> 256, 3 x 3 / 2: 9.0 us, 12.6 in words; 128 x 128 x
+// 128 -> 128: 20.1, 15.2).  That is 0.3% off the faster of the two in the mean, always words was 1.7%, and 1.15 times it at worst (1.66).
+bool conv_words_gains(const b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t KW, int64_t KH, int64_t Cout, int64_t P,
+                      int g, bool taps) {
+    const int64_t cols = Cin * KH * g, tiles = cdiv(P, CI_PIX) * N;
+    if (conv_words_ldw(Cin * KH, g) * Cout > N * Cin * W * H || (2 * KW <= g && cols <= 4 * CI_BK)) return false;
+    if (taps) return true;
+    const CiTiles t = ci_tiles(ctx, tiles, cols, Cout, g);
+    const double load = (double)(tiles * cdiv(Cout, t.bn) * t.parts) / (2.0 * ctx->prop.multiProcessorCount);   // of the resident CTAs
+    const double crs = (double)(KW * KH * Cin);
+    const double words = 3.1 + 4.8e-6 * (double)(cols * Cout) + (double)cdiv(t.nkb, t.parts) * (0.41 + 0.84 * load) +
+                         0.0129 * t.bn * (load > 1.0 ? load : 1.0) + (t.parts > 1 ? 2.5 + 1.8 * load : 0.0);
+    const double matrix = (double)N * (6.9 + 2.36e-6 * (double)P * crs + 1.3e-9 * (double)P * crs * (double)Cout + 0.0012 * crs) +
+                          (KW * KH * Cin % 8 != 0 ? 1.2 : 0.0);
+    return 1.04 * words < matrix;
 }
 
 int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t KW, int64_t KH, int64_t Cout,
@@ -481,14 +516,8 @@ int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64
             }
         }
     }
-    // Channels per CTA: all of them up to 256, since every channel tile gathers the pixels again; but a launch that
-    // leaves half of the GPU's CTAs unused splits the reduction, two k-blocks a part at least, which the 256-wide
-    // tile has no shared memory for; four a part where they are read in words and take less than a cluster's barriers
-    // (256 x 256 x 32 -> 128, 3 x 3 / 2: 15.8 us with two, 9.2).
-    const int64_t tiles = p.tiles * N, room = 2 * (int64_t)ctx->prop.multiProcessorCount, nkb = cdiv((int64_t)p.CRS, CI_BK);
-    int bn = Cout <= 64 ? 64 : (Cout <= 128 || (2 * tiles * cdiv(Cout, 128) <= room && nkb >= 4) ? 128 : 256), parts = 1;
-    if (bn < 256)
-        while (parts < 8 && 2 * parts * tiles * cdiv(Cout, bn) <= room && nkb >= (g ? 8 : 4) * parts) parts *= 2;
+    const CiTiles t = ci_tiles(ctx, p.tiles * N, p.CRS, Cout, g);
+    const int bn = t.bn, parts = t.parts;
     CUtensorMap tw;
     uint64_t dims[2] = {(uint64_t)p.CRS, (uint64_t)Cout};
     uint64_t str[1] = {(uint64_t)ldw * 2};

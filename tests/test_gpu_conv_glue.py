@@ -190,15 +190,24 @@ def test_glue_bit_exact(ctx, ora):
         assert np.all(d <= np.spacing(np.abs(ref)).astype(np.float32) + 1e-7)   # fast exp: one fp16 ulp at most
 
 
-# (N, Cin, H, W, Cout, KH, KW, stride, padding, dilation): 8 and 4 columns a kernel row, taps before and behind the words'
-# ends, one and several k-blocks and parts of a cluster, odd kernel-row counts, dilated rows, pixels past the last tile
-WORDS = [(1, 3, 37, 64, 112, 7, 7, (4, 4), (3, 3), (1, 1)), (2, 3, 40, 44, 24, 7, 5, (3, 4), (2, 2), (2, 1)),
-         (1, 5, 24, 48, 130, 4, 8, (1, 8), (0, 0), (1, 1)), (2, 17, 31, 30, 64, 3, 3, (2, 2), (1, 1), (1, 1)),
-         (1, 7, 9, 22, 300, 1, 4, (2, 2), (0, 4), (1, 1)), (1, 64, 20, 26, 40, 3, 3, (2, 6), (1, 1), (1, 1)),
-         (3, 1, 50, 52, 16, 2, 2, (2, 4), (0, 5), (3, 1)), (1, 160, 16, 16, 72, 3, 3, (2, 2), (1, 1), (1, 1))]
+# (N, Cin, H, W, Cout, KH, KW, stride, padding, dilation): 8 and 4 columns a kernel row, each with tiles of 64, 128 and 256
+# channels and two channel tiles; taps before and behind the words' ends, one and several k-blocks and images, clusters of 1, 2,
+# 4 and 8 parts, odd kernel-row counts, dilated rows, strides past a word, pixels past the last tile
+WORDS = [(1, 3, 75, 100, 112, 7, 7, (4, 4), (3, 3), (1, 1)), (2, 3, 40, 44, 24, 7, 5, (3, 4), (2, 2), (2, 1)),
+         (1, 3, 90, 132, 200, 7, 7, (4, 4), (3, 3), (1, 1)), (1, 5, 70, 104, 66, 4, 8, (1, 8), (0, 0), (1, 1)),
+         (1, 20, 51, 52, 40, 7, 6, (4, 4), (3, 3), (1, 1)), (1, 40, 83, 88, 112, 7, 7, (4, 4), (3, 3), (1, 1)),
+         (3, 1, 50, 52, 16, 3, 5, (2, 4), (0, 5), (3, 1)), (2, 17, 31, 30, 64, 3, 3, (2, 2), (1, 1), (1, 1)),
+         (1, 64, 20, 26, 40, 3, 3, (2, 6), (1, 1), (1, 1)), (1, 24, 45, 62, 104, 3, 3, (2, 2), (1, 1), (1, 1)),
+         (1, 15, 61, 66, 300, 3, 3, (2, 2), (1, 1), (1, 1)), (1, 48, 45, 50, 130, 3, 3, (2, 2), (1, 1), (1, 1)),
+         (1, 172, 44, 30, 72, 3, 3, (2, 2), (1, 1), (1, 1)), (1, 16, 64, 64, 128, 3, 3, (2, 2), (1, 1), (1, 1)),
+         (1, 96, 33, 38, 24, 1, 4, (2, 2), (0, 4), (1, 1))]
+# the same kernels where reading in words does not gain: a weight larger than the image, half of the columns zeros on a short
+# reduction, a long chain a CTA against a small im2col matrix
+NOT_WORDS = [(1, 3, 37, 64, 112, 7, 7, (4, 4), (3, 3), (1, 1)), (1, 16, 37, 38, 8, 2, 2, (2, 2), (1, 1), (1, 1)),
+             (1, 64, 60, 64, 256, 3, 3, (2, 2), (1, 1), (1, 1))]
 
 
-@pytest.mark.parametrize("N,Cin,H,W,Cout,KH,KW,stride,padding,dilation", WORDS)
+@pytest.mark.parametrize("N,Cin,H,W,Cout,KH,KW,stride,padding,dilation", WORDS + NOT_WORDS)
 @pytest.mark.parametrize("dt", [np.float16, np.float32])
 def test_conv_of_even_stride_reads_whole_words(ctx, ora, N, Cin, H, W, Cout, KH, KW, stride, padding, dilation, dt):
     rng = np.random.default_rng(Cin + Cout + W)
@@ -209,11 +218,54 @@ def test_conv_of_even_stride_reads_whole_words(ctx, ora, N, Cin, H, W, Cout, KH,
     out = ctx.allocate(dt, *reversed(ref.shape))
     ctx.fill_bytes(out, 0xFF)
     ctx.ws.reset()
-    jv.convolution_(ctx, out, ctx.toback(x), ctx.toback(w), ctx.toback(b), stride[::-1], padding[::-1], dilation[::-1])
+    args = ctx.toback(x), ctx.toback(w), ctx.toback(b)
+    before = ctx.launch_count()
+    jv.convolution_(ctx, out, *args, stride[::-1], padding[::-1], dilation[::-1])
+    # in words: the weight laid out and the convolution, whose scratch is given back; by taps no scratch and one launch, or, as
+    # by an im2col matrix, scratch that stays until the reset
+    route = ctx.launch_count() - before, ctx.ws.stats()[0]
+    assert (route == (2, 0)) == ((N, Cin, H, W, Cout, KH, KW, stride, padding, dilation) in WORDS), route
     ctx.synchronize()
     got = out.to_host()
     tol = 2e-3 if dt == np.float16 else 2e-5      # as for the taps
     assert relerr(got, ref) < tol, describe(got, ref, tol)
+
+
+@pytest.mark.parametrize("Cin,Cout,H,W,scratch", [(24, 104, 45, 62, 0), (3, 64, 90, 132, None), (16, 64, 64, 64, None)])
+def test_conv_in_words_does_not_depend_on_the_workspace(ora, Cin, Cout, H, W, scratch):
+    """Recorded on a context that has no workspace yet, the laid-out weight is refused: the call goes by taps as it would have
+    without the words, or says that it has no room where that route wants scratch of its own; then in words all the same."""
+    rng = np.random.default_rng(Cout + W)
+    x = np.float16(rng.standard_normal((1, Cin, H, W)) * 0.5)
+    w = np.float16(rng.standard_normal((Cout, Cin, 3, 3)) * 0.2)
+    ref = ora.conv2d(x, w, None, (2, 2), (1, 1), out_dtype=np.float32)
+    with jv.Ctx(0) as c:
+        dx, dw = c.toback(x), c.toback(w)
+        out = c.allocate(np.float32, *reversed(ref.shape))
+        c.fill_bytes(out, 0xFF)
+        c.synchronize()
+        call = lambda: jv.convolution_(c, out, dx, dw, None, (2, 2), (1, 1), (1, 1))
+        before = c.launch_count()
+        if scratch == 0:
+            g = c.capture(call)
+            assert c.launch_count() - before == 1 and c.ws.stats()[1] == 0
+            g.replay()
+            c.synchronize()
+            assert relerr(out.to_host(), ref) < 2e-5
+            del g
+        else:
+            with pytest.raises(jv.B200Error):
+                c.capture(call)
+        c.fill_bytes(out, 0xFF)
+        before = c.launch_count()
+        call()
+        assert c.launch_count() - before == 2
+        g = c.capture(call)
+        c.fill_bytes(out, 0xFF)
+        g.replay()
+        c.synchronize()
+        assert relerr(out.to_host(), ref) < 2e-5
+        del g
 
 
 def test_conv_in_words_keeps_to_its_taps(ctx, ora):
