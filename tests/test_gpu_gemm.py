@@ -522,14 +522,59 @@ def test_gelu_of_large_negative_values_goes_to_zero(ctx):
         assert np.all(np.abs(g.astype(np.float64) - e) <= np.abs(e) + 2e-44)
 
 
-@pytest.mark.parametrize("tokens,out,K", [(2, 35525, 512), (16, 35641, 515), (19, 20001, 1024), (33, 16577, 520), (5, 53279, 384)])
+# (tokens, out features, K, launches on 148 SMs): what is left past the full rounds is one block, some, exactly half a round, just
+# more than that; of a short reduction, which is not split; split in two, four and eight parts, some of those without a step
+@pytest.mark.parametrize("tokens,out,K,launches", [(2, 35525, 512, 2), (16, 35641, 515, 2), (19, 20001, 1024, 2), (33, 16577, 520, 2),
+                                                   (5, 53279, 384, 1), (5, 53279, 512, 2), (5, 53401, 512, 1), (33, 8289, 2100, 2)])
 @pytest.mark.parametrize("dt", [np.float16, np.float32])
-def test_unaligned_rows_past_the_last_full_round(ctx, ora, tokens, out, K, dt):
-    """Row blocks that fill the GPU once or more and leave one block, half a round and just more than that: the rest is a launch
-    of its own, split along K; with a bias, every row."""
+def test_unaligned_rows_past_the_last_full_round(ctx, ora, tokens, out, K, launches, dt):
+    """Row blocks that fill the GPU once or more and leave some: at most half a round of them is a launch of its own, split
+    along K; with a bias, every row."""
     rng = np.random.default_rng(tokens + out)
     X, Wt, b = _case(rng, tokens, out, K, scale=0.25)
+    before = ctx.launch_count()
     got = linear_gpu(ctx, X, Wt, b, out_dtype=dt)
+    if ctx.dev.cores == 148:
+        assert ctx.launch_count() - before == launches
     ref = ora.linear(X, Wt, b, out_dtype=dt)
     tol = 2e-3 if dt == np.float16 else 2e-5             # one rounding step of fp16; sqrt(K) eps32
     assert relerr(got, ref) < tol, describe(got, ref, tol)
+
+
+def test_what_follows_a_product_in_two_launches_waits_for_both(ctx):
+    """A layer norm that is launched early behind the second launch, eagerly and recorded, gives the bits it gives behind a
+    finished product, over results that are poisoned before each."""
+    rng = np.random.default_rng(8)
+    M, K, tokens, C = 35840, 1024, 5, 112
+    base = ctx.toback(np.concatenate([np.float16([0]), (rng.standard_normal(M * K, dtype=np.float32) * 0.05).astype(np.float16)]))
+    w = jv.DeviceArray(ctx, base.ptr + 2, np.float16, (M, K), owner=base)            # off a 16-byte boundary: by row blocks
+    x = ctx.toback((rng.standard_normal((tokens, K)) * 0.25).astype(np.float16))
+    y, z = ctx.allocate(np.float16, M, tokens), ctx.allocate(np.float16, M, tokens)
+    rows = M * tokens // C
+    mean, rstd = ctx.allocate(np.float32, rows), ctx.allocate(np.float32, rows)
+    view = lambda a: jv.DeviceArray(ctx, a.ptr, np.float16, (C, rows), owner=a)
+
+    def norm():
+        jv.layernorm_(ctx, view(z), mean, rstd, view(y), None, None, C, 1e-5)
+
+    def both():
+        ctx.fill_bytes(y, 0xFF)
+        jv.matmul_(ctx, y, w, x, None)
+        norm()
+
+    ctx.fill_bytes(y, 0xFF)
+    before = ctx.launch_count()
+    jv.matmul_(ctx, y, w, x, None)
+    assert ctx.launch_count() - before == 2
+    ctx.synchronize()
+    norm()
+    ctx.synchronize()
+    product, want = y.to_host(), z.to_host()
+    assert np.all(np.isfinite(want))
+    g = ctx.capture(both)
+    for run in (both, g.replay) * 4:
+        ctx.fill_bytes(z, 0xFF)
+        run()
+        ctx.synchronize()
+        assert np.array_equal(z.to_host(), want) and np.array_equal(y.to_host(), product)
+    del g
