@@ -253,16 +253,15 @@ static int launch_permute(b200_ctx* ctx, const void* src, void* out, const int64
 // lowest value.  Both arrays are indexed (x, y, c, n) through element strides, so the planar layout
 // of the reference's call and a channels-last token array go through the same kernel; VEC = 8 takes
 // eight channels per thread when the channel axis is contiguous in both.
-// I: as for the permuted copy.  A 2 x 2 window without padding, an image encoder's, is inside the image wherever it lies: its
+// I: as for the permuted copy.  TWO: a 2 x 2 window without padding, an image encoder's, is inside the image wherever it lies: its
 // four loads go out together.  The six pools of an image encoder's pass over eight images (560 MB): 253 -> 167 us; its eight
 // permuted copies 155 -> 108.
-template <int VEC, typename I>
+template <int VEC, bool TWO, typename I>
 __global__ void __launch_bounds__(256)
 maxpool2d_kernel(const __half* __restrict__ x, __half* __restrict__ out, int W, int H, int C, int OW, int OH, I total,
                  int64_t xs0, int64_t xs1, int64_t xs2, int64_t xs3, int64_t os0, int64_t os1, int64_t os2, int64_t os3,
                  int kx, int ky, int sx, int sy, int px, int py, int c_fast) {
     const I CV = C / VEC, ow = OW, oh = OH;
-    const bool two = kx == 2 && ky == 2 && px == 0 && py == 0;
     for (I i = blockIdx.x * (I)blockDim.x + threadIdx.x; i < total; i += (I)gridDim.x * blockDim.x) {
         int ox, oy, c, n;
         I t = i;
@@ -286,7 +285,7 @@ maxpool2d_kernel(const __half* __restrict__ x, __half* __restrict__ out, int W, 
 #pragma unroll
                 for (int u = 0; u < 4; ++u) acc[u] = __hmax2_nan(acc[u], hh[u]);
             };
-            if (two) {
+            if constexpr (TWO) {
                 const __half* p0 = xp + (int64_t)bx * xs0 + (int64_t)by * xs1;
                 uint4 w[4];
 #pragma unroll
@@ -297,10 +296,13 @@ maxpool2d_kernel(const __half* __restrict__ x, __half* __restrict__ out, int W, 
                 for (int dy = 0; dy < ky; ++dy) {
                     const int iy = by + dy;
                     if (iy < 0 || iy >= H) continue;
+#pragma unroll 2   // two loads in flight: 5 x 5 / 2 over 4 of 14 x 14 x 64 6.5 -> 5.6 us
                     for (int dx = 0; dx < kx; ++dx) {
                         const int ix = bx + dx;
                         if (ix < 0 || ix >= W) continue;
-                        take(*reinterpret_cast<const uint4*>(xp + (int64_t)ix * xs0 + (int64_t)iy * xs1));
+                        // by value: a reference costs the loads their width (3 x 3 / 1 over 2 of 56 x 56 x 256: 6.4 -> 5.3 us)
+                        const uint4 w = *reinterpret_cast<const uint4*>(xp + (int64_t)ix * xs0 + (int64_t)iy * xs1);
+                        take(w);
                     }
                 }
             }
@@ -358,12 +360,15 @@ int b200_maxpool2d_f16(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cn, int64_t 
             xstride[2], xstride[3], ostride[0], ostride[1], ostride[2], ostride[3], (int)kx, (int)ky, (int)sx, (int)sy,
             (int)px, (int)py, c_fast);
     };
+    const bool two = kx == 2 && ky == 2 && px == 0 && py == 0;
     if (total < (1ll << 31)) {
-        if (vec) go(maxpool2d_kernel<8, uint32_t>, (uint32_t)total);
-        else go(maxpool2d_kernel<1, uint32_t>, (uint32_t)total);
+        if (vec && two) go(maxpool2d_kernel<8, true, uint32_t>, (uint32_t)total);
+        else if (vec) go(maxpool2d_kernel<8, false, uint32_t>, (uint32_t)total);
+        else go(maxpool2d_kernel<1, false, uint32_t>, (uint32_t)total);
     } else {
-        if (vec) go(maxpool2d_kernel<8, int64_t>, total);
-        else go(maxpool2d_kernel<1, int64_t>, total);
+        if (vec && two) go(maxpool2d_kernel<8, true, int64_t>, total);
+        else if (vec) go(maxpool2d_kernel<8, false, int64_t>, total);
+        else go(maxpool2d_kernel<1, false, int64_t>, total);
     }
     ctx->launches++;
     B200_CUDA(cudaGetLastError());
