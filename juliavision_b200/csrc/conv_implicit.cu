@@ -25,7 +25,7 @@
 // two aligned loads, masked to the taps.  The reduction is laid out (cin, kh, G columns), G = 8 or 4, the weight the same
 // with zeros between, the tile K-major: a thread's pixel and eight columns are one 16-byte store.  A seventh and a third more
 // columns than taps (7 x 7 / 4, 3 x 3 / 2) and a tenth of the instructions: us, before and
-// now: 1024 x 1024 x 3 -> 112, 7 x 7 / 4 24.7 -> 15.9, eight of them 166 -> 93, 512 x 512 x 3 -> 64 18.4 -> 6.4, 3 x 3 / 2
+// now: 1024 x 1024 x 3 -> 112, 7 x 7 / 4 24.8 -> 17.0, eight of them 166 -> 93, 512 x 512 x 3 -> 64 18.4 -> 6.4, 3 x 3 / 2
 // 256 x 256 x 32 -> 128 19.4 -> 9.2, 128 x 128 x 128 -> 256 22.5 -> 18.1.  What is left is a CTA's chain of latencies.
 // A small image (fewer CTAs than the GPU holds) splits the reduction over the CTAs of a cluster, whose fp32 tiles
 // meet in distributed shared memory, added in rank order.

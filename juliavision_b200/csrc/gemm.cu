@@ -428,7 +428,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
         // warps per scheduler taking turns; warps never wait for one another.  fp16 results of CTA pairs go 32 columns at
         // a time: half the steps, and half the rows the store engine takes one by one (32 bytes each at 16 columns).
         // Microseconds, 16 -> 32: 524288 x 336 x 112 126 -> 111, 131072 x 672 x 224 72 -> 65, 524288 x 448 x 112 with GELU
-        // 222 -> 201, 65536 x 5120 x 1280 727 -> 718; 64 columns do no better and cost a second stage.  The 256-wide pair pays
+        // 222 -> 201; 64 columns do no better and cost a second stage.  The 256-wide pair pays
         // with one of its six stages and goes without on long reductions (deep_ring).
         constexpr int CH = GC;                 // columns per chunk (one tcgen05.ld)
         constexpr int NPART = EPI_WARPS / 4;   // warps sharing a lane quadrant
@@ -743,7 +743,9 @@ __global__ void gemm_f16_scalar_kernel(int64_t M, int64_t N, int64_t K, const __
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Whether a 256-wide pair stores 16 columns at a time and keeps a sixth stage instead (see the epilogue): reductions of 24
-// k-blocks and more (32768 x 448 x 1792: 55.5 us, 58 with 32 columns; of 20, 65536 x 5120 x 1280, 728 and 720).
+// k-blocks and more.  Over 90 products of 8192 to 65536 tokens 32 columns took 1.01 of 16's time in the mean at 10 to 23
+// k-blocks, single ones 0.94 to 1.17, which is what repeats of one differ by under the power cap, and 1.03 at 24 to 28, none less
+// than 1.01 (32768 x 448 x 1792: 57.1 us, 59.3 with 32); 1.01 at 32 to 40.  What shorter ones gain stands there.
 static bool deep_ring(int64_t K) { return cdiv(K, GEMM_BK) >= 24; }
 
 struct TilePick {
@@ -788,8 +790,10 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
     TilePick best{256, 1, 0, 0, 1};
     double best_cost = 1e300;
     // What a tile costs beside its k-blocks, fitted to 1150 products of 8 to 300,000 tokens and 16 to 500,000 features, K = 1
-    // to 4600, timed on every tile (the tile chosen is 1.2% slower than the fastest in the mean; with one t_tile for
-    // all of them 2.1%).
+    // to 4600, timed on every tile with 16-column stores, the bias looked up in series and the steps of 7.1.26 for GELU (the
+    // tile chosen was 1.2% slower than the fastest in the mean; with one t_tile for all of them 2.1%; the figures of single
+    // products below are of that time).  With the present epilogue it is 1.1% over 200 others, 32% at worst (75993 x 272 x
+    // 208 with GELU: 36.2 us on 256x2 tiles, 27.5 on 128x2).
     // A launch of up to three rounds: t_tile, and a pair's set-up and hand-overs where a tile is only a few k-blocks long
     // (1067 x 1224 x 144: 5.9 us on 128x2 tiles, 5.2 on 128x1; 18600 x 160 x 192: 6.6 on 256x2, 5.6 on 256x1), which
     // show once, so not over several rounds of one feature tile (51442 x 184 x 168: 18.2 us on 256x1, 15.1 on 256x2).
