@@ -8,10 +8,11 @@
 // (TMEM allocation, barriers, tensor maps) costs more than the window's arithmetic, with one CTA resident
 // per SM.  So this kernel is small instead: CTAs of four warps, operands fetched with cp.async, and each warp's 16 x 64 scores
 // and 16 x 64 output held in registers as warp-level m16n8k16 tiles.  A CTA takes one unit, 64 queries of one (window, head),
-// six CTAs to an SM; or, where there are more units of many keys than that, four CTAs to an SM walk the units with the next
+// six CTAs to an SM; or, where there are many more units of more than a few keys, four CTAs to an SM walk the units with the next
 // one's operands on their way (two buffers of 27 KB) under this one's arithmetic.
-// Microseconds, replayed (a unit a CTA with loads through registers / walking / now): 8192 windows x 2 heads of 64 x 64 x 56
-// (470 MB) 118.6 / 107.1 / 106.3, 2000 x 4 of 49 x 49 x 64 57.2 / 49.9 / 49.6, 600 x 4 of 16 x 16 x 56 9.9 / 9.6 / 8.5.
+// Microseconds, replayed (a unit a CTA with loads through registers / always walking / now): 8192 windows x 2 heads of 64 x 64 x
+// 56 (470 MB) 118.6 / 107.1 / 106.3, 1024 x 2 in the L2 15.3 / 17.1 / 14.6, 2000 x 4 of 49 x 49 x 64 57.2 / 49.9 / 49.6, 600 x 4 of
+// 16 x 16 x 56 9.9 / 9.6 / 8.5.
 #include <cuda_fp16.h>
 
 #include "internal.h"
@@ -266,13 +267,14 @@ int attention_window_launch(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     const int64_t units = (int64_t)p.qtiles * H * B, sms = ctx->prop.multiProcessorCount;
     B200_REQUIRE(units < (1ll << 31), B200_DECLINE_EXTENT, "attention: too many windows");
     p.units = (uint32_t)units;
-    // A walking CTA of a single unit only pays for its second buffer, and one of two takes longer than six CTAs side by side; of
-    // few keys there is little to fetch ahead.  Between three and four units an SM both take the same alone, and back to back
-    // walking CTAs, which leave no room for the next launch's, spread evenly.  Microseconds on 148 SMs, a unit a CTA / walking,
-    // each launch behind another kernel: 300 units of 64 x 64 x 56 6.2 / 6.2 (6.7 with every buffer zeroed whole), 592 7.1 / 7.2
-    // (back to back 7.0 / 5.8), 800 8.6 / 9.0, 888 8.7 / 9.8, 1040 11.1 / 10.7, 1200 12.4 / 11.7; 16 x 16 x 56: 300 4.5 / 4.6,
-    // 800 5.3 / 6.2, 1800 8.2 / 9.4, 16000 51.1 / 51.2.
-    if (Lk <= 32 || units <= 3 * sms || (units > AW_CTAS_PER_SM * sms && units <= AW_CTAS_PER_SM_ONE * sms)) {
+    // A walking CTA of a single unit only pays for its second buffer, one of two or three takes longer than six CTAs side by side
+    // with others behind them, and of few keys there is little to fetch ahead.  Between three and four units an SM both take the
+    // same alone, and back to back walking CTAs, which leave no room for the next launch's, spread evenly.  Microseconds on 148
+    // SMs, a unit a CTA / walking, each launch behind another kernel: 300 units of 64 x 64 x 56 6.2 / 6.2 (6.7 with every buffer
+    // zeroed whole), 592 7.1 / 7.2 (back to back 7.0 / 5.8), 800 8.6 / 9.0, 888 8.7 / 9.8, 1600 in the L2 13.1 / 14.5, 2048
+    // 16.1 / 17.3; of 49 x 49 x 64 2048 in the L2 14.0 / 14.7, 4096 27.5 / 26.5; of 36 x 36 x 48 2400 from memory 15.3 / 14.7; of
+    // 16 x 16 x 56 300 4.5 / 4.6, 1800 8.2 / 9.4, 16000 51.1 / 51.2.
+    if (Lk <= 32 || (units <= 14 * sms && (units <= 3 * sms || units > AW_CTAS_PER_SM * sms))) {
         B200_CUDA(launch_dep(attention_window_kernel<false>, dim3((unsigned)units, 1, 1), dim3(AW_THREADS, 1, 1), AW_BUF_BYTES, ctx->stream, 1, p));
         ctx->launches++;
         return B200_OK;

@@ -513,12 +513,13 @@ def test_few_queries_with_smaller_clusters(ctx, ora, B, H, Lq, Lk, E, monkeypatc
         seen.append(got)
 
 
-# walking CTAs of many units, of at most one (three to four units an SM) and of two; and, up to three units an SM, between four
-# and six, or of few keys, a CTA each
+# a CTA each, on either side of the rule's lines (three, four and fourteen units an SM) and of few keys, and walking CTAs of at
+# most one unit and of many
 @pytest.mark.parametrize("E,Lq,Lk,H,B,dt", [(56, 64, 64, 3, 500, np.float16), (64, 49, 49, 2, 700, np.float16), (8, 70, 5, 3, 333, np.float32),
                                             (40, 16, 64, 5, 601, np.float16), (56, 129, 33, 2, 297, np.float16),
                                             (56, 64, 64, 5, 100, np.float16), (64, 50, 64, 7, 127, np.float16), (40, 65, 33, 4, 40, np.float32),
-                                            (56, 64, 64, 4, 111, np.float32), (24, 17, 1, 6, 148, np.float16), (64, 100, 32, 3, 900, np.float16)])
+                                            (56, 64, 64, 4, 111, np.float32), (24, 17, 1, 6, 148, np.float16), (64, 100, 32, 3, 900, np.float16),
+                                            (64, 49, 49, 3, 700, np.float16), (8, 70, 33, 4, 300, np.float32), (56, 129, 40, 2, 360, np.float16)])
 def test_windows_walked_in_turn(ctx, ora, E, Lq, Lk, H, B, dt):
     """Both forms on either side of their rule: head dims and key counts that leave columns and rows of zeros, buffers used
     again, query tiles of different fill next to each other, and a window of NaN that must not reach its neighbours."""
