@@ -205,7 +205,7 @@ def kernel_figures(ctx, jv, pk, quick: bool):
     ctx.synchronize()
     ms = time_region(ctx, conv, 20)
     out["conv_stem_1024x1024x3_7x7s4_to_112"] = dict(ms=round(ms, 5), tflops=round(2.0 * 65536 * 147 * 112 / ms / 1e9, 2),
-                                                     note="im2col (19 MB) + GEMM; HBM/latency-bound, not tensor-bound")
+                                                     note="the image read in words straight into the tiles; latency-bound, not tensor-bound")
     Bw, Hw, Lw, Ew = 1024, 2, 64, 56
     # operands as the image encoder hands them over: one token-major q/k/v projection (3d, tokens) with the
     # tokens of a window adjacent, read through strides; the result token-major as well
