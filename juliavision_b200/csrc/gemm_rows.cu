@@ -54,7 +54,8 @@ struct GrParams {
     int steps_per_cta;   // steps of GR_STEP columns each CTA of a cluster takes
 };
 
-// Out of line: inlined, its registers change the main loop's of the two-tile form (115 for 96), 9 x 45001 x 2000 62.6 -> 64.3 us.
+// Out of line, and not called for nothing, in the two-tile form: inlined, its registers change the main loop's (115 for 96), 9 x
+// 45001 x 2000 61.1 -> 62.8 us.  The other forms lose by it (4 x 20001 x 1280 18.8 -> 19.5).
 __device__ __noinline__ float gr_act(int epi, float v) { return apply_act(epi, v); }
 
 // grid (K parts, row blocks, token blocks), the K parts of a row block forming a cluster; 256 threads.  TWO: one of two
@@ -176,7 +177,7 @@ gemm_rows_kernel(const GrParams p) {
         const int64_t m = m0 + r, n = n0 + tok;
         if (p.bias != nullptr) v += __half2float(p.bias[p.bias_per_n ? n : m]);
         OutT* o = static_cast<OutT*>(p.out) + n * p.ldo + m;
-        auto act = [&](float u) { return NT == 2 ? gr_act(p.epi, u) : apply_act(p.epi, u); };
+        auto act = [&](float u) { return NT != 2 ? apply_act(p.epi, u) : p.epi == B200_EPI_NONE ? u : gr_act(p.epi, u); };
         if constexpr (sizeof(OutT) == 2) *o = __float2half_rn(act(__half2float(__float2half_rn(v))));
         else *o = act(v);
     };
