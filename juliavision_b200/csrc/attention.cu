@@ -24,14 +24,14 @@ namespace b200 {
 
 constexpr int ATT_BR = 128;  // queries per tile (TMEM lanes)
 constexpr int ATT_TILE_BYTES = 128 * 128; // one swizzle atom of an operand tile: 128 rows x 128 B (64 fp16 of E)
-#ifndef ATT_TURN_AT
-#define ATT_TURN_AT 2   // after which quarter (0..3) of its exponentials a tile passes the turn
-#endif
 // Two shapes of CTA, chosen by the head dimension, and a third for short keys:
 //   EP = 64, NT = 1:           one query tile, key blocks of 64, P over S, 128 tensor-memory columns and 48 KB, so that
 //                              four CTAs share an SM
 //   EP = 64  (E <= 64):        two query tiles of 128 per CTA, K/V rings of 4 stages x 16 KB
-//   EP = 128 (64 < E <= 128):  two query tiles of 128 per CTA as well; every operand tile is two swizzle atoms along
+//   EP = 80  (64 < E <= 80):   as EP = 128, but O has 80 columns per tile, which leaves P 48 columns of its own: 96 of a
+//                              block's 128 keys, the other 32 go through shared memory (A operand of the last two steps
+//                              of P V).  8 heads x 4096 x 72: 70.9 us with P over S, 58.0 so; no mask (no room for it)
+//   EP = 128 (80 < E <= 128, with a mask 64 < E):  two query tiles of 128 per CTA as well; every operand tile is two swizzle atoms along
 //                              E (columns 0-63, 64-127, the second zero-filled past E by the tensor map), S = Q K'
 //                              runs over both, O has 128 columns per tile — S 2 x 128 + O 2 x 128 fill the tensor
 //                              memory, so P is written over the first 64 columns of its tile's S once the softmax
@@ -46,10 +46,11 @@ constexpr int ATT_TILE_BYTES = 128 * 128; // one swizzle atom of an operand tile
 // boundary at or one entry before the first, 65 words apart (odd, for the same reason).
 constexpr int BIAS_ROW_WORDS = 66;
 template <int EP, bool BIAS = false, int NT_ = 2> struct AttCfg {
-    static_assert(EP == 64 || EP == 128, "head dim is padded to one or two swizzle atoms");
-    static constexpr int ATOMS = EP / 64;              // 16 KB atoms per operand tile
+    static_assert(EP == 64 || EP == 80 || EP == 128, "head dim is padded to one or two swizzle atoms, O to EP columns");
+    static constexpr int ATOMS = EP == 64 ? 1 : 2;     // 16 KB atoms per operand tile
     static constexpr int NT = NT_;                     // query tiles per CTA
     static_assert(NT == 2 || (NT == 1 && EP == 64 && !BIAS), "one tile per CTA is built for E <= 64 without a mask");
+    static_assert(EP != 80 || !BIAS, "a mask leaves no room for the tail of P");
     static constexpr int BC = NT == 2 ? 128 : 64;      // keys per block
     static constexpr int CTAS_PER_SM = NT == 2 ? 1 : 4;
     static constexpr int THREADS = 128 * NT + 128;     // NT softmax warpgroups, then TMA, UMMA and idle warps
@@ -57,8 +58,10 @@ template <int EP, bool BIAS = false, int NT_ = 2> struct AttCfg {
     // registers of a softmax thread and of the others: (NT x 128 x one + 128 x the other) is what the launch holds
     static constexpr int SOFTMAX_REGS = NT == 2 ? 232 : 96, OTHER_REGS = NT == 2 ? 40 : 32;
     static constexpr int TMEM_COLS = NT == 2 ? 512 : 128;
-    // S of tile t at BC t, O at O_COL + EP t, P of its own at P_COL + 64 t
-    static constexpr int O_COL = NT * BC, P_COL = 384;
+    // S of tile t at BC t, O at O_COL + EP t, P of its own at P_COL + P_COLS t
+    static constexpr int O_COL = NT * BC, P_COL = O_COL + NT * EP;
+    static constexpr bool P_TAIL = EP == 80;               // the last 32 keys of a block's P lie in shared memory
+    static constexpr int P_COLS = P_TAIL ? 48 : 64;
     static constexpr int K_STAGES = NT == 2 && EP == 64 ? 4 : 2;
     static constexpr int V_STAGES = NT == 2 && EP == 64 ? 4 : (BIAS ? 1 : 2);
     static constexpr bool P_IN_S = EP == 128 || NT == 1;   // P shares its tile's S columns (tensor memory is full otherwise)
@@ -68,14 +71,17 @@ template <int EP, bool BIAS = false, int NT_ = 2> struct AttCfg {
     static constexpr int S_Q = 0;                              // NT tiles
     static constexpr int S_K = NT * Q_BYTES;                   // K_STAGES tiles
     static constexpr int S_V = S_K + K_STAGES * KV_BYTES;      // V_STAGES tiles
-    static constexpr int S_END = S_V + V_STAGES * KV_BYTES;
+    static constexpr int S_P = S_V + V_STAGES * KV_BYTES;      // P_TAIL: NT tiles of 128 rows x 128 B, the first 64 used
+    static constexpr int S_END = S_P + (P_TAIL ? NT * ATT_TILE_BYTES : 0);
     static constexpr int BIAS_TILE_BYTES = BIAS ? ATT_BR * BIAS_ROW_WORDS * 4 : 0;
-    static constexpr int SMEM_BYTES = S_END + NT * BIAS_TILE_BYTES + 256;
+    static constexpr int S_BARS = S_END + NT * BIAS_TILE_BYTES;   // the barriers, then the tensor-memory address and the abort flag
+    static constexpr int BARRIERS = 2 + 2 * K_STAGES + 2 * V_STAGES + 10 + (EP == 128 ? 2 : 0);
+    static constexpr int SMEM_BYTES = S_BARS + (BARRIERS + 1) * 8;
     static_assert(CTAS_PER_SM * (SMEM_BYTES + 1024) <= 233472, "shared memory over budget");
 };
 // tensor-memory map of two tiles (512 columns): S of tile t, fp32, at [128 t, 128 t + 128); O of tile t, fp32, at
-// [256 + EP t, ... + EP); P of tile t, fp16 packed two keys per column, at [384 + 64 t, ... + 64) for EP = 64 and
-// over the first 64 columns of S_t for EP = 128
+// [256 + EP t, ... + EP); P of tile t, fp16 packed two keys per column, at [384 + 64 t, ... + 64) for EP = 64, at
+// [416 + 48 t, ... + 48) for EP = 80 and over the first 64 columns of S_t for EP = 128
 
 struct AttnParams {
     int E, Lq, Lk, H, B;
@@ -121,6 +127,11 @@ __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void st_shared16(uint32_t at, const uint32_t* v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -160,6 +171,8 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
     // half's exponentials.  8 heads x 4096 x 72: 71.7 -> 70.3 us, 12 x 1500 x 96 32.2 -> 31.7, masked 8 x 2048 x 72 50.6 -> 49.9;
     // with columns of its own the turns hide as much and the extra hand-over costs (12 x 4096 x 64: 85.9 -> 88.1).
     constexpr bool HALVES = EP == 128;
+    constexpr bool OWN_P = !Cfg::P_IN_S;     // P in columns (and shared memory) of its own
+    constexpr bool FREE = OWN_P && !BIAS;    // its tiles go their own ways after the start, see the softmax
     constexpr int ITEM_ROWS = NT * ATT_BR;   // queries one whole work item covers
     extern __shared__ __align__(1024) uint8_t smem[];
     // Uniform across the grid: a base that is not 1024-aligned makes every thread leave before
@@ -168,7 +181,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
         if (threadIdx.x == 0) atomicCAS(p.d_status, 0, KST_SMEM_LAYOUT);
         return;
     }
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::S_END + NT * Cfg::BIAS_TILE_BYTES);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::S_BARS);
     uint64_t* q_full = bars + 0;                           // [2]
     uint64_t* k_full = bars + 2;                           // [K_STAGES]
     uint64_t* k_empty = k_full + K_STAGES;                 // [K_STAGES]
@@ -182,6 +195,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
     uint64_t* p_half = exp_turn + 2;                       // [2]: HALVES, the first half of a block's P is written
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(exp_turn + (HALVES ? 4 : 2));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    static_assert(Cfg::BARRIERS == 2 + 2 * K_STAGES + 2 * V_STAGES + 10 + (HALVES ? 2 : 0), "barriers counted by the layout");
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -282,80 +296,96 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
         }
     } else if (warp == Cfg::ISSUE_WARP || (NT == 2 && warp == Cfg::ISSUE_WARP + 1)) {
         // ------------------------------------------------------------- UMMA issuers
-        // One issuing lane per query tile (warp 9: tile 0, warp 10: tile 1).  Each walks its own
+        // One issuing warp per query tile (warp 9: tile 0, warp 10: tile 1).  Each walks its own
         // chain  S_t(j+1) = Q_t K(j+1)'  as soon as the softmax has pulled S_t(j) into registers,
         // then  O_t += P_t(j) V(j)  once P_t(j) is written.  The two chains share only the
-        // K/V rings.  (Issuing a UMMA blocks while the tensor pipe is busy, so the issuing lanes
-        // are not softmax threads.)
+        // K/V rings.  (Issuing a UMMA blocks while the tensor pipe is busy, so the issuing warps
+        // are not softmax warps.)
+        // The whole warp walks the chain and waits; the thread elect.sync picks (the same one every time) issues, every
+        // operand being the same for the warp.  With one lane running it under `if (lane == 0)`, P written -> P V
+        // issued took 1000 clocks and S taken -> Q K' issued 1300, with nothing else on the tensor core; now 290 and
+        // 430.  16 heads x 2048 x 128 35.4 -> 33.7 us, masked 8 x 2048 x 72 49.9 -> 45.1, 1024 x 8 windows of 256 x 56 374 -> 359.
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::OTHER_REGS));
         const int t = warp - Cfg::ISSUE_WARP;
-        if (lane == 0 && t < ntiles) {
+        if (t < ntiles) {
             // S = Q K': both operands K-major (E contiguous), from shared memory.  O += P V: P from
-            // tensor memory, V MN-major (E contiguous per key) from shared memory.
+            // tensor memory (P_TAIL: its last 32 keys K-major from shared memory), V MN-major (E contiguous per key) from
+            // shared memory.
             constexpr uint32_t idesc_s = make_idesc_f16(ATT_BR, BC, 0, 0);
             constexpr uint32_t idesc_o = make_idesc_f16(ATT_BR, EP, 0, 1);
             constexpr uint64_t kdesc0 = make_smem_desc(16, 1024);
             constexpr uint64_t vdesc0 = make_smem_desc(Cfg::KV_ATOM, 1024);
             const uint32_t q_addr = smem_u32(smem + Cfg::S_Q + t * Cfg::Q_BYTES);
+            const uint32_t tail_addr = smem_u32(smem + Cfg::S_P + t * ATT_TILE_BYTES);
             const uint32_t s_tmem = tmem_base + t * BC;
             const uint32_t o_tmem = tmem_base + Cfg::O_COL + t * EP;
-            const uint32_t p_tmem = Cfg::P_IN_S ? s_tmem : tmem_base + Cfg::P_COL + t * 64;
+            const uint32_t p_tmem = OWN_P ? tmem_base + Cfg::P_COL + t * Cfg::P_COLS : s_tmem;
 
+            auto wait = [&](uint64_t* bar, uint32_t parity, int code) -> bool {   // one answer per warp
+                return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.d_status, code, abort_flag));
+            };
             auto issue_qk = [&](int j) -> bool {
                 const int sk = j % K_STAGES;
-                if (!mbar_wait(&k_full[sk], (uint32_t)((j / K_STAGES) & 1), p.d_status, KST_WAIT_FULL, abort_flag))
-                    return false;
+                if (!wait(&k_full[sk], (uint32_t)((j / K_STAGES) & 1), KST_WAIT_FULL)) return false;
                 // With P in S's columns this product is issued after P V(j-1), which read P after the softmax had taken
                 // S(j-1), and UMMAs of one thread run in issue order: nothing else to wait for.
-                if (!Cfg::P_IN_S && j > 0 &&
-                    !mbar_wait(&s_empty[t], (uint32_t)((j - 1) & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag))
-                    return false;
+                if (OWN_P && j > 0 && !wait(&s_empty[t], (uint32_t)((j - 1) & 1), KST_WAIT_SOFTMAX)) return false;
                 tc_fence_after();
-                const uint32_t k_addr = smem_u32(smem + Cfg::S_K + sk * Cfg::KV_BYTES);
+                if (elect_one()) {
+                    const uint32_t k_addr = smem_u32(smem + Cfg::S_K + sk * Cfg::KV_BYTES);
 #pragma unroll
-                for (int k = 0; k < EP / 16; ++k) {
-                    // past the head dim both operands are zeros (E = 72: five of eight steps; the fifth always has some)
-                    if (EP == 128 && k >= 5 && k * 16 >= p.E) break;
-                    // 16 elements of E = 32 B inside the swizzle row; every fourth step moves to the next atom
-                    const uint32_t in = (uint32_t)(k & 3) * 32;
-                    umma_ss(s_tmem, smem_desc_at(kdesc0, q_addr + (uint32_t)(k >> 2) * ATT_TILE_BYTES + in),
-                            smem_desc_at(kdesc0, k_addr + (uint32_t)(k >> 2) * Cfg::KV_ATOM + in), idesc_s, k != 0);
+                    for (int k = 0; k < EP / 16; ++k) {
+                        // past the head dim both operands are zeros
+                        if (EP == 128 && k >= 5 && k * 16 >= p.E) break;
+                        // 16 elements of E = 32 B inside the swizzle row; every fourth step moves to the next atom
+                        const uint32_t in = (uint32_t)(k & 3) * 32;
+                        umma_ss(s_tmem, smem_desc_at(kdesc0, q_addr + (uint32_t)(k >> 2) * ATT_TILE_BYTES + in),
+                                smem_desc_at(kdesc0, k_addr + (uint32_t)(k >> 2) * Cfg::KV_ATOM + in), idesc_s, k != 0);
+                    }
+                    umma_commit(&s_full[t]);
+                    umma_commit(&k_empty[sk]);   // one of `ntiles` arrivals that free this K stage
+                    if (j >= 1 && j < 7) ATT_TRACE(64 * t + 8 + 8 * (j - 1) + 0);   // Q K'(j) issued, filed under block j-1
                 }
-                umma_commit(&s_full[t]);
-                umma_commit(&k_empty[sk]);   // one of `ntiles` arrivals that free this K stage
-                if (j >= 1 && j < 7) ATT_TRACE(64 * t + 8 + 8 * (j - 1) + 0);   // Q K'(j) issued, filed under block j-1
+                __syncwarp();
                 return true;
             };
-
-            bool ok = mbar_wait(&q_full[t], 0, p.d_status, KST_WAIT_FULL, abort_flag);
-            if (ok && nblk > 0) ok = issue_qk(0);
-            for (int j = 0; ok && j < nblk; ++j) {
-                if (!Cfg::P_IN_S && j + 1 < nblk && !issue_qk(j + 1)) break;
-                const int sv = j % V_STAGES;
-                if (!mbar_wait(&v_full[sv], (uint32_t)((j / V_STAGES) & 1), p.d_status, KST_WAIT_FULL, abort_flag)) break;
-                if (j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 7);   // issuer reaches its wait for P(j)
-                constexpr int FIRST = HALVES ? BC / 32 : 0;   // steps that do not wait for the whole of P
-                if constexpr (HALVES) {
-                    if (!mbar_wait(&p_half[t], (uint32_t)(j & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag)) break;
-                    tc_fence_after();
-                    const uint32_t v_addr = smem_u32(smem + Cfg::S_V + sv * Cfg::KV_BYTES);
-#pragma unroll
-                    for (int k = 0; k < FIRST; ++k)
-                        umma_ts(o_tmem, p_tmem + k * 8, smem_desc_at(vdesc0, v_addr + k * 2048), idesc_o, (j | k) != 0);
-                }
-                if (!mbar_wait(&p_full[t], (uint32_t)(j & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag)) break;
-                tc_fence_after();
+            // P V of block j, steps [k0, k1) of 16 keys.
+            auto issue_pv = [&](int j, int sv, int k0, int k1) {
                 const uint32_t v_addr = smem_u32(smem + Cfg::S_V + sv * Cfg::KV_BYTES);
 #pragma unroll
-                for (int k = FIRST; k < BC / 16; ++k) {
+                for (int k = k0; k < k1; ++k) {
                     // P comes from tensor memory: 16 keys = 8 packed columns per step.
                     // V: 16 key rows = two 8-row groups = 2048 B.
-                    umma_ts(o_tmem, p_tmem + k * 8, smem_desc_at(vdesc0, v_addr + k * 2048), idesc_o, (j | k) != 0);
+                    const uint64_t vdesc = smem_desc_at(vdesc0, v_addr + k * 2048);
+                    if (Cfg::P_TAIL && k >= BC / 16 - 2) umma_ss(o_tmem, smem_desc_at(kdesc0, tail_addr + (k - (BC / 16 - 2)) * 32), vdesc, idesc_o, 1);
+                    else umma_ts(o_tmem, p_tmem + k * 8, vdesc, idesc_o, (j | k) != 0);
                 }
-                umma_commit(&pv_done[t]);
-                umma_commit(&v_empty[sv]);   // one of `ntiles` arrivals that free this V stage
-                if (j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 1);   // P V(j) issued
-                if (Cfg::P_IN_S && j + 1 < nblk && !issue_qk(j + 1)) break;   // overwrites P(j): after the product that reads it
+            };
+
+            bool ok = wait(&q_full[t], 0, KST_WAIT_FULL);
+            if (ok && nblk > 0) ok = issue_qk(0);
+            for (int j = 0; ok && j < nblk; ++j) {
+                if (OWN_P && j + 1 < nblk && !issue_qk(j + 1)) break;
+                const int sv = j % V_STAGES;
+                if (!wait(&v_full[sv], (uint32_t)((j / V_STAGES) & 1), KST_WAIT_FULL)) break;
+                if (j < 6 && lane == 0) ATT_TRACE(64 * t + 8 + 8 * j + 7);   // issuer reaches its wait for P(j)
+                constexpr int FIRST = HALVES ? BC / 32 : 0;   // steps that do not wait for the whole of P
+                if constexpr (HALVES) {
+                    if (!wait(&p_half[t], (uint32_t)(j & 1), KST_WAIT_SOFTMAX)) break;
+                    tc_fence_after();
+                    if (elect_one()) issue_pv(j, sv, 0, FIRST);
+                    __syncwarp();
+                }
+                if (!wait(&p_full[t], (uint32_t)(j & 1), KST_WAIT_SOFTMAX)) break;
+                tc_fence_after();
+                if (elect_one()) {
+                    issue_pv(j, sv, FIRST, BC / 16);
+                    umma_commit(&pv_done[t]);
+                    umma_commit(&v_empty[sv]);   // one of `ntiles` arrivals that free this V stage
+                    if (j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 1);   // P V(j) issued
+                }
+                __syncwarp();
+                if (!OWN_P && j + 1 < nblk && !issue_qk(j + 1)) break;   // overwrites P(j): after the product that reads it
             }
         }
     } else {
@@ -368,17 +398,20 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             const uint32_t lane_base = uint32_t(quad * 32) << 16;
             const uint32_t s_tmem = tmem_base + lane_base + t * BC;
             const uint32_t o_tmem = tmem_base + lane_base + Cfg::O_COL + t * EP;
-            const uint32_t p_tmem = Cfg::P_IN_S ? s_tmem : tmem_base + lane_base + Cfg::P_COL + t * 64;
+            const uint32_t p_tmem = OWN_P ? tmem_base + lane_base + Cfg::P_COL + t * Cfg::P_COLS : s_tmem;
             const float sc = BIAS ? p.scale : p.scale_log2;
             const float sce = BIAS ? 1.4426950408889634f : sc;   // with a bias the scores are scaled when it is added
             float m_run = -INFINITY, l_run = 0.f;
             bool ok = true;
-            // Both tiles take the same time per block, and left alone they fall into step: both
-            // want the MUFU pipe in the same half of every period and leave it idle in the other.
-            // So the exponential phases take turns (tile 0 block j, tile 1 block j, tile 0 block
-            // j+1, ...): while one tile owns the MUFU pipe the other does its max / rescale / waits
-            // and its tensor-core work runs.
-            const bool pingpong = ntiles == 2 && ATT_TURN_AT >= 0;
+            // Both tiles take the same time per block, and in step both would want the MUFU pipe in the same half of
+            // every period and leave it idle in the other.  Where P has a place of its own and there is no mask it is enough that tile 1
+            // starts behind: nothing brings the two together again (12 heads x 4096 x 64: 79.6 us, 84.5 in step, 86.3 with a turn
+            // handed over every block; started after the last quarter instead of the first, 8 x 4096 x 72 takes 63.4 for 58.0).
+            // With P over S, or a mask, a tile's block is one long chain and the exponential phases take turns (tile 0 block j, tile 1
+            // block j, tile 0 block j+1, ...): while one tile owns the MUFU pipe the other does its max / rescale / waits
+            // and its tensor-core work runs (16 heads x 2048 x 128: 33.7 us, 38.5 without).
+            const bool pingpong = ntiles == 2;
+            constexpr int TURN_AT = FREE ? 0 : 3;   // after which quarter of its exponentials a tile passes the turn
             // The mask, when its keys are contiguous: each warp copies the next block's entries of its own 32 rows to
             // shared memory (cp.async, a row's entries across the lanes) while it works on this block, and every thread
             // then reads its row back.  Nothing but the warp itself is involved, so no barrier is.  Rows may start at
@@ -421,21 +454,27 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             };
             if (bias_async) bias_fetch(0);
 
-            for (int j = 0; ok && j < nblk; ++j) {
-                if (!mbar_wait(&s_full[t], (uint32_t)(j & 1), p.d_status, KST_WAIT_TMEM_FULL, abort_flag)) { ok = false; break; }
+            uint32_t r[NC][32];
+            // The whole row of S (128 fp32) comes into registers in one round trip.
+            auto scores = [&](int j) -> bool {
+                if (!mbar_wait(&s_full[t], (uint32_t)(j & 1), p.d_status, KST_WAIT_TMEM_FULL, abort_flag)) return false;
                 tc_fence_after();
-                const int nvalid = p.Lk - (jb0 + j) * BC; // keys of this block that exist (>= BC when full)
-                if (lane == 0 && quad == 0 && j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 2);  // S(0, j) ready
-
-                // The whole row of S (128 fp32) comes into registers in one round trip; S is then
-                // free for the next Q K' of this tile.
-                uint32_t r[NC][32];
 #pragma unroll
                 for (int c = 0; c < NC; ++c) tmem_ld32(s_tmem + c * 32, r[c]);
+                return true;
+            };
+            for (int j = 0; ok && j < nblk; ++j) {
+                if (!scores(j)) { ok = false; break; }
+                const int nvalid = p.Lk - (jb0 + j) * BC; // keys of this block that exist (>= BC when full)
+                if (lane == 0 && quad == 0 && j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 2);  // S(0, j) ready
                 tmem_wait_ld();
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(r[c][i]));   // in registers from here on
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&s_empty[t]);
+                if (lane == 0) mbar_arrive(&s_empty[t]);   // free for the next Q K' of this tile
                 if (lane == 0 && quad == 0 && j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 3);  // S in registers
 
                 if constexpr (BIAS) {
@@ -531,21 +570,22 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                 const float m_blk = mx * sce;
                 const float slack = (BC < 128 && j == 1) ? 0.0f : 8.0f;
                 const float m_new = (m_blk > m_run + slack) ? m_blk : m_run;
-                // 0 on the first block (m_run = -inf), else 1 or < 2^-8.  With a mask a row may have seen
-                // nothing but -inf so far: then the reference point stays -inf and nothing is rescaled.
-                const float alpha = (BIAS && m_run == m_new) ? 1.0f : ex2(m_run - m_new);
+                // With a mask a row may have seen nothing but -inf so far: then the reference point stays -inf.
                 const float m_sub = (BIAS && m_new == -INFINITY) ? 0.f : m_new;
-
-                // P's shared tile and O are both still in use by the previous block's P V.
-                if (j > 0 && !mbar_wait(&pv_done[t], (uint32_t)((j - 1) & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
-                if (lane == 0 && quad == 0 && j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 4);  // max done, PV(j-1) done
-                // Rescale O (and the running sum in its column 64) when this row's maximum moved;
-                // skipped warp-wide when no row's did — exact, the factor would be 1.
-                if (j > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+                float alpha = 1.0f;
+                bool pv_known = false;
+                // O is in use by the previous block's P V; so are P's columns where nothing else says that it is done.
+                auto pv_wait = [&]() -> bool {
+                    if (j > 0 && !pv_known && !mbar_wait(&pv_done[t], (uint32_t)((j - 1) & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag)) return false;
+                    pv_known = true;
+                    tc_fence_after();
+                    return true;
+                };
+                if (!FREE && !pv_wait()) { ok = false; break; }
+                auto rescale = [&]() -> bool {
+                    alpha = (BIAS && m_run == m_new) ? 1.0f : ex2(m_run - m_new);   // 0 on the first block (m_run = -inf), else 1 or < 2^-8
+                    if (j == 0) return true;
+                    if (!pv_wait()) return false;
 #pragma unroll 1
                     for (int c = 0; c < EP / 16; ++c) {   // 16 columns at a time: S is live in registers
                         uint32_t o16[16];
@@ -556,9 +596,11 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                         tmem_st16_raw(o_tmem + c * 16, o16);
                     }
                     tmem_wait_st();
-                }
-
-                if (pingpong && (t == 1 || j > 0)) {
+                    return true;
+                };
+                if (!FREE && __any_sync(0xffffffffu, m_new != m_run) && !rescale()) { ok = false; break; }
+                if (lane == 0 && quad == 0 && j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 4);  // max done
+                if (pingpong && (FREE ? t == 1 && j == 0 : t == 1 || j > 0)) {
                     // tile 0 waits for tile 1's block j-1, tile 1 for tile 0's block j
                     const uint32_t par = (uint32_t)((t == 1 ? j : j - 1) & 1);
                     if (!mbar_wait(&exp_turn[t], par, p.d_status, KST_WAIT_SOFTMAX, abort_flag)) { ok = false; break; }
@@ -568,9 +610,11 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                 // (two keys per 32-bit column) straight into tensor memory for the P V product.
                 const uint64_t sc2 = pack2(sce, sce), nm2 = pack2(-m_sub, -m_sub);
                 uint64_t lsa = pack2(0.f, 0.f), lsb = pack2(0.f, 0.f);
+                uint32_t pk[NC][16];
+                bool pv_seen = false;   // asked half way, so that the answer is there when it is needed
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    uint32_t pk[16];
+                    if (FREE && c == NC / 2) pv_seen = j == 0 || mbar_test_wait(&pv_done[t], (uint32_t)((j - 1) & 1));
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         // two scores per FMA and per add (packed fp32 pairs), one ex2 each, one convert for the pair
@@ -581,12 +625,10 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                         if (i & 1) lsb = add2(lsb, pack2(e0, e1));
                         else lsa = add2(lsa, pack2(e0, e1));
                         const __half2 h2 = __floats2half2_rn(e0, e1);
-                        pk[i] = *reinterpret_cast<const uint32_t*>(&h2);
+                        pk[c][i] = *reinterpret_cast<const uint32_t*>(&h2);
                     }
-                    tmem_st16_raw(p_tmem + c * 16, pk);
-                    // Hand the turn over part way: the other tile's exponentials then overlap the
-                    // rest of these, which keeps the MUFU pipe fed without falling in step.
-                    if (c == ATT_TURN_AT && NC == 4 && pingpong) {
+                    if (!FREE) tmem_st16_raw(p_tmem + c * 16, pk[c]);
+                    if (c == TURN_AT && NC == 4 && pingpong && (!FREE || j == 0)) {
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&exp_turn[1 - t]);
                     }
@@ -595,6 +637,19 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&p_half[t]);
+                    }
+                }
+                if constexpr (FREE) {
+                    pv_known = __all_sync(0xffffffffu, pv_seen);   // one answer per warp
+                    if (__any_sync(0xffffffffu, m_new != m_run) && !rescale()) { ok = false; break; }
+                    if (!pv_wait()) { ok = false; break; }
+#pragma unroll
+                    for (int c = 0; c < (Cfg::P_TAIL ? NC - 1 : NC); ++c) tmem_st16_raw(p_tmem + c * 16, pk[c]);
+                    if (Cfg::P_TAIL) {
+                        const uint32_t at = smem_u32(smem + Cfg::S_P + t * ATT_TILE_BYTES) + row * 128;
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) st_shared16(at + ((c ^ (row & 7)) << 4), &pk[NC - 1][4 * c]);
+                        fence_proxy_async_smem();
                     }
                 }
                 tmem_wait_st();
@@ -613,6 +668,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             if (ok && nblk > 0)
                 ok = mbar_wait(&pv_done[t], (uint32_t)((nblk - 1) & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag);
             if (ok) {
+                constexpr int W = EP % 32 ? 16 : 32;   // columns a step
                 tc_fence_after();
                 const int lq = q0 + t * ATT_BR + row;
                 if (nsp > 1) {
@@ -622,15 +678,15 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                     const int64_t prow = ((int64_t)split * p.ntail + tailpair) * ITEM_ROWS + t * ATT_BR + row;
                     float* po = p.part_o + prow * p.E;
 #pragma unroll 1
-                    for (int c = 0; c < EP / 32; ++c) {
-                        uint32_t r[32];
-                        tmem_ld32(o_tmem + c * 32, r);
+                    for (int c = 0; c < EP / W; ++c) {
+                        uint32_t r[W];
+                        tmem_ld(o_tmem + c * W, r);
                         tmem_wait_ld();
                         if (lq < p.Lq) {
 #pragma unroll
-                            for (int i = 0; i < 32; i += 4)
-                                if (c * 32 + i < p.E)
-                                    *reinterpret_cast<float4*>(po + c * 32 + i) =
+                            for (int i = 0; i < W; i += 4)
+                                if (c * W + i < p.E)
+                                    *reinterpret_cast<float4*>(po + c * W + i) =
                                         make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]), __uint_as_float(r[i + 2]),
                                                     __uint_as_float(r[i + 3]));
                         }
@@ -643,25 +699,25 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                 const float inv = 1.0f / (l_run == 0.f ? 1.0f : l_run);
                 const int64_t obase = lq * p.osL + h * p.osH + b * p.osB;
 #pragma unroll 1
-                for (int c = 0; c < EP / 32; ++c) {
-                    uint32_t r[32];
-                    tmem_ld32(o_tmem + c * 32, r);
+                for (int c = 0; c < EP / W; ++c) {
+                    uint32_t r[W];
+                    tmem_ld(o_tmem + c * W, r);
                     tmem_wait_ld();
                     if (lq < p.Lq) {
                         if (p.out_f32) {
-                            float* o = static_cast<float*>(p.out) + obase + c * 32;
+                            float* o = static_cast<float*>(p.out) + obase + c * W;
 #pragma unroll
-                            for (int i = 0; i < 32; i += 4) {
-                                if (c * 32 + i < p.E)
+                            for (int i = 0; i < W; i += 4) {
+                                if (c * W + i < p.E)
                                     *reinterpret_cast<float4*>(o + i) =
                                         make_float4(__uint_as_float(r[i]) * inv, __uint_as_float(r[i + 1]) * inv,
                                                     __uint_as_float(r[i + 2]) * inv, __uint_as_float(r[i + 3]) * inv);
                             }
                         } else {
-                            __half* o = static_cast<__half*>(p.out) + obase + c * 32;
+                            __half* o = static_cast<__half*>(p.out) + obase + c * W;
 #pragma unroll
-                            for (int i = 0; i < 32; i += 8) {
-                                if (c * 32 + i < p.E) {
+                            for (int i = 0; i < W; i += 8) {
+                                if (c * W + i < p.E) {
                                     uint4 w;
                                     __half2* hh = reinterpret_cast<__half2*>(&w);
 #pragma unroll
@@ -1016,6 +1072,8 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
                                        AttCfg<64>::SMEM_BYTES));
         B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<64, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        AttCfg<64, true>::SMEM_BYTES));
+        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<80, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       AttCfg<80>::SMEM_BYTES));
         B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<128, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        AttCfg<128>::SMEM_BYTES));
         B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<128, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1061,6 +1119,7 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
             return launch_dep(kern, grid, dim3(threads, 1, 1), smem, ctx->stream, 1, tq, tk, tv, p);
         };
         if (single) return go(attention_f16_tc_kernel<64, false, 1>, AttCfg<64, false, 1>::THREADS, AttCfg<64, false, 1>::SMEM_BYTES);
+        if (wide && E <= 80 && !bptr) return go(attention_f16_tc_kernel<80, false, 2>, AttCfg<80>::THREADS, AttCfg<80>::SMEM_BYTES);
         if (wide)
             return bptr ? go(attention_f16_tc_kernel<128, true, 2>, AttCfg<128, true>::THREADS, AttCfg<128, true>::SMEM_BYTES)
                         : go(attention_f16_tc_kernel<128, false, 2>, AttCfg<128>::THREADS, AttCfg<128>::SMEM_BYTES);

@@ -556,3 +556,23 @@ def test_more_than_2_to_the_30_windows(ctx):
     for b in (0, 1, 8191, 8192, 16383, 16384):
         plane = jv.DeviceArray(ctx, out.ptr + b * H * E * 2, np.float16, (E, H), owner=out)
         assert np.array_equal(plane.to_host(), v[8 * b:8 * (b + H)].reshape(H, E)), b
+
+
+@pytest.mark.parametrize("E", [56, 64, 72, 80, 96])
+@pytest.mark.parametrize("Lq,Lk", [(300, 33), (129, 97), (128, 128), (257, 225), (1, 700), (300, 1025)])
+def test_reference_point_that_moves_in_later_blocks(ctx, E, Lq, Lk):
+    """Scores that grow from key block to key block, slowly enough to be let through or by more than 2^8 at once; the
+    last 32 keys of a block take another way to the product for some head dims."""
+    rng = np.random.default_rng(E + 7 * Lq + Lk)
+    q, k, v = (np.float16(rng.standard_normal((2, 3, n, E))) for n in (Lq, Lk, Lk))
+    grow = np.where(np.arange(Lk) // 128 % 3 == 2, 1.0 + np.arange(Lk) // 128, 1.0) * np.where(np.arange(Lk) % 128 >= 96, 1.5, 1.0)
+    k = np.float16(k * grow[None, None, :, None])
+    got, plan = attention_gpu(ctx, q, k, v, 0.5, np.float32)
+    assert isinstance(plan, jv.FlashTCPlan)
+    s = np.einsum("bhqe,bhke->bhqk", np.float64(q), np.float64(k)) * 0.5
+    p = np.exp(s - s.max(-1, keepdims=True))
+    ref = np.einsum("bhqk,bhke->bhqe", p / p.sum(-1, keepdims=True), np.float64(v))
+    # P is rounded to fp16 (2^-11 of each weight, none rounded further: they lie within 2^8 of the reference point or
+    # below 2^-14 of it, 2^-25 each), sums are fp32 over Lk terms
+    vmax = np.abs(np.float64(v)).max()
+    assert np.abs(got - ref).max() < vmax * (2.0 ** -11 + Lk * 2.0 ** -25 + 1e-5)
