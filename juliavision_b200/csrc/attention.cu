@@ -41,7 +41,10 @@ constexpr int ATT_TILE_BYTES = 128 * 128; // one swizzle atom of an operand tile
 // With an additive mask each tile also stages a block's 128 x 128 mask entries (BIAS_ROW_WORDS words per row, see
 // the softmax); at EP = 128 the room for it comes from the V ring, which keeps one stage: V(j+1) is asked for when
 // both tiles' P V(j) are done and needed a softmax later, more than a fetch takes.
-// A staged mask row: 128 entries.  Rows on 8-byte boundaries are copied and read 8 bytes at a time, 66 words apart
+// Through a tensor map the entries come as two boxes of 64 keys, swizzled, asked for by a warp of their own as soon as the
+// block before is read.  Copied by the softmax's own warps, they cost a block 1800 clocks of standing in front of a full queue
+// (4 heads x 4000 x 56: 69.3 -> 51.0 us, 8 x 2048 x 72 49.8 -> 37.6); copies of 8 bytes by warps of their own were no faster.
+// A row staged by the softmax's warps: 128 entries.  Rows on 8-byte boundaries are copied and read 8 bytes at a time, 66 words apart
 // (an odd number of 8-byte units, so that a warp's 32 rows lie in all banks); others word by word, from the 4-byte
 // boundary at or one entry before the first, 65 words apart (odd, for the same reason).
 constexpr int BIAS_ROW_WORDS = 66;
@@ -75,7 +78,7 @@ template <int EP, bool BIAS = false, int NT_ = 2> struct AttCfg {
     static constexpr int S_END = S_P + (P_TAIL ? NT * ATT_TILE_BYTES : 0);
     static constexpr int BIAS_TILE_BYTES = BIAS ? ATT_BR * BIAS_ROW_WORDS * 4 : 0;
     static constexpr int S_BARS = S_END + NT * BIAS_TILE_BYTES;   // the barriers, then the tensor-memory address and the abort flag
-    static constexpr int BARRIERS = 2 + 2 * K_STAGES + 2 * V_STAGES + 10 + (EP == 128 ? 2 : 0);
+    static constexpr int BARRIERS = 2 + 2 * K_STAGES + 2 * V_STAGES + 10 + (EP == 128 ? 2 : 0) + (BIAS ? 4 : 0);
     static constexpr int SMEM_BYTES = S_BARS + (BARRIERS + 1) * 8;
     static_assert(CTAS_PER_SM * (SMEM_BYTES + 1024) <= 233472, "shared memory over budget");
 };
@@ -97,8 +100,7 @@ struct AttnParams {
     // strides (0 on a broadcast axis); null when absent.
     const __half* bias;
     int64_t bsK, bsQ, bsH, bsB;
-    int bias_async;     // keys contiguous: the mask's blocks are copied to shared memory ahead of use, 1: by words,
-                        // 2: every row starts on an 8-byte boundary
+    int mask;           // how the mask's blocks reach the softmax: one of MASK_*
     // Keys split over nsplit CTAs per query pair (few queries, many keys): each writes its unnormalised
     // fp32 O rows to part_o[split][tail pair][256 rows][E] and (reference point, row sum) to part_ml[...][2];
     // attention_merge_kernel combines them (the reference's attn_flash_cm_merge!, flash.jl:1398-1421).
@@ -107,6 +109,10 @@ struct AttnParams {
     float* part_o;
     float* part_ml;
 };
+
+// Entry by entry from global memory (keys not contiguous); copied to shared memory ahead of use by words, or 8 bytes at
+// a time where every row starts on an 8-byte boundary; through a tensor map.
+enum { MASK_DIRECT = 0, MASK_WORDS = 1, MASK_EIGHTS = 2, MASK_TMA = 3 };
 
 #define ATT_TRACE(slot)                                                                              \
     do {                                                                                             \
@@ -162,7 +168,8 @@ template <int EP, bool BIAS, int NT_>
 __global__ void __launch_bounds__(AttCfg<EP, BIAS, NT_>::THREADS, AttCfg<EP, BIAS, NT_>::CTAS_PER_SM)
 attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                         const __grid_constant__ CUtensorMap tmapK,
-                        const __grid_constant__ CUtensorMap tmapV, const AttnParams p) {
+                        const __grid_constant__ CUtensorMap tmapV,
+                        const __grid_constant__ CUtensorMap tmapM, const AttnParams p) {
     using Cfg = AttCfg<EP, BIAS, NT_>;
     constexpr int K_STAGES = Cfg::K_STAGES, V_STAGES = Cfg::V_STAGES;
     constexpr int BC = Cfg::BC, NC = BC / 32;   // keys per block, and per-thread pieces of 32 of them
@@ -193,9 +200,11 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
     uint64_t* pv_done = p_full + 2;                        // [2]
     uint64_t* exp_turn = pv_done + 2;                      // [2]: whose turn it is to run its exponentials
     uint64_t* p_half = exp_turn + 2;                       // [2]: HALVES, the first half of a block's P is written
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(exp_turn + (HALVES ? 4 : 2));
+    uint64_t* mask_full = p_half + (HALVES ? 2 : 0);       // [2]: BIAS, a block's mask entries have landed (MASK_TMA)
+    uint64_t* mask_empty = mask_full + 2;                  // [2]: and have been read
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mask_full + (BIAS ? 4 : 0));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    static_assert(Cfg::BARRIERS == 2 + 2 * K_STAGES + 2 * V_STAGES + 10 + (HALVES ? 2 : 0), "barriers counted by the layout");
+    static_assert(Cfg::BARRIERS == 2 + 2 * K_STAGES + 2 * V_STAGES + 10 + (HALVES ? 2 : 0) + (BIAS ? 4 : 0), "barriers counted by the layout");
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -237,6 +246,10 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             if (HALVES) mbar_init(&p_half[t], 4);
             mbar_init(&pv_done[t], 1);
             mbar_init(&exp_turn[t], 4);
+            if (BIAS) {
+                mbar_init(&mask_full[t], 1);
+                mbar_init(&mask_empty[t], 4);
+            }
         }
         for (int s = 0; s < K_STAGES; ++s) {
             mbar_init(&k_full[s], 1);
@@ -269,6 +282,21 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
     // share over (setmaxnreg at the head of each role's branch).
     if (warp == 4 * NT + 3 || (NT == 1 && warp == 6)) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::OTHER_REGS));
+        if (BIAS && p.mask == MASK_TMA && lane == 0) {   // a block's 128 x 128 entries per tile, as soon as the block before is read
+            bool ok = true;
+            for (int j = 0; ok && j < nblk; ++j)
+                for (int t = 0; ok && t < ntiles; ++t) {
+                    if (j > 0 && !mbar_wait(&mask_empty[t], (uint32_t)((j - 1) & 1), p.d_status, KST_WAIT_EMPTY, abort_flag)) {
+                        ok = false;
+                        break;
+                    }
+                    mbar_arrive_expect_tx(&mask_full[t], 2 * ATT_TILE_BYTES);
+#pragma unroll
+                    for (int a = 0; a < 2; ++a)
+                        tma_load_4d(smem + Cfg::S_END + t * Cfg::BIAS_TILE_BYTES + a * ATT_TILE_BYTES, &tmapM, &mask_full[t],
+                                    (jb0 + j) * BC + 64 * a, q0 + t * ATT_BR, p.bsH ? h : 0, p.bsB ? b : 0);
+                }
+        }
     } else if (warp == Cfg::TMA_WARP) {
         // ------------------------------------------------------------- TMA producer
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::OTHER_REGS));
@@ -412,7 +440,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             // and its tensor-core work runs (16 heads x 2048 x 128: 33.7 us, 38.5 without).
             const bool pingpong = ntiles == 2;
             constexpr int TURN_AT = FREE ? 0 : 3;   // after which quarter of its exponentials a tile passes the turn
-            // The mask, when its keys are contiguous: each warp copies the next block's entries of its own 32 rows to
+            // A mask no tensor map is over, its keys contiguous: each warp copies the next block's entries of its own 32 rows to
             // shared memory (cp.async, a row's entries across the lanes) while it works on this block, and every thread
             // then reads its row back.  Nothing but the warp itself is involved, so no barrier is.  Rows may start at
             // any element: when not all of them lie on 8-byte boundaries (an odd number of keys puts every other row in
@@ -421,8 +449,8 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             // row per thread, 20 heads x 1500 x 1500 took 152 us, with words copied 56, with 8 bytes at a time 45 (24
             // without a mask: adding it is 64 more packed FMAs, 128 conversions and the reads per thread and block).
             uint32_t* bias_rows = reinterpret_cast<uint32_t*>(smem + Cfg::S_END) + (t * ATT_BR + quad * 32) * BIAS_ROW_WORDS;
-            const bool bias_async = BIAS && p.bias != nullptr && p.bias_async;
-            const bool bias8 = BIAS && p.bias_async == 2;
+            const bool bias_async = BIAS && (p.mask == MASK_WORDS || p.mask == MASK_EIGHTS);
+            const bool bias8 = BIAS && p.mask == MASK_EIGHTS;
             auto bias_fetch = [&](int j) {
                 const int keys = min(BC, p.Lk - (jb0 + j) * BC);
                 const int rows = min(32, p.Lq - (q0 + t * ATT_BR + quad * 32));   // rows of this warp that exist
@@ -458,12 +486,14 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             // The whole row of S (128 fp32) comes into registers in one round trip.
             auto scores = [&](int j) -> bool {
                 if (!mbar_wait(&s_full[t], (uint32_t)(j & 1), p.d_status, KST_WAIT_TMEM_FULL, abort_flag)) return false;
+                __syncwarp();
                 tc_fence_after();
 #pragma unroll
                 for (int c = 0; c < NC; ++c) tmem_ld32(s_tmem + c * 32, r[c]);
                 return true;
             };
             for (int j = 0; ok && j < nblk; ++j) {
+                if (BIAS && p.mask == MASK_TMA && !mbar_wait(&mask_full[t], (uint32_t)(j & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag)) { ok = false; break; }
                 if (!scores(j)) { ok = false; break; }
                 const int nvalid = p.Lk - (jb0 + j) * BC; // keys of this block that exist (>= BC when full)
                 if (lane == 0 && quad == 0 && j < 6) ATT_TRACE(64 * t + 8 + 8 * j + 2);  // S(0, j) ready
@@ -482,27 +512,34 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                     // (A reference point beyond 2^12, where every key of a row carries the type's lowest value, is itself
                     // rounded by more than fp16 tells from one: there the heaviest key's P is rounded like the others'.)
                     const int lq = q0 + t * ATT_BR + row;
-                    if (p.bias == nullptr) {
-#pragma unroll
-                        for (int c = 0; c < NC; ++c)
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) r[c][i] = __float_as_uint(__uint_as_float(r[c][i]) * sc);
-                    } else {
+                    {
                         const __half* brow = p.bias + (int64_t)(lq < p.Lq ? lq : 0) * p.bsQ + (int64_t)h * p.bsH +
                                              (int64_t)b * p.bsB + (int64_t)(jb0 + j) * BC * p.bsK;
-                        if (bias_async) {
+                        const uint64_t sc2b = pack2(sc, sc);
+                        // score * scale + mask for two keys: the mask's units, the exponent's factor follows later
+                        auto add = [&](int c, int i, uint32_t two) {
+                            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&two));
+                            float x0, x1;
+                            unpack2(fma2(pack2(__uint_as_float(r[c][2 * i]), __uint_as_float(r[c][2 * i + 1])), sc2b, pack2(f.x, f.y)),
+                                    x0, x1);
+                            r[c][2 * i] = __float_as_uint(x0);
+                            r[c][2 * i + 1] = __float_as_uint(x1);
+                        };
+                        if (p.mask == MASK_TMA) {
+                            const uint8_t* w = smem + Cfg::S_END + t * Cfg::BIAS_TILE_BYTES + row * 128;   // rows of 64 entries, 128-byte swizzle
+#pragma unroll
+                            for (int c = 0; c < BC / 8; ++c) {
+                                const uint4 eight = *reinterpret_cast<const uint4*>(w + (c >> 3) * ATT_TILE_BYTES + (((c & 7) ^ (row & 7)) << 4));
+                                add(c >> 2, (c & 3) * 4, eight.x);
+                                add(c >> 2, (c & 3) * 4 + 1, eight.y);
+                                add(c >> 2, (c & 3) * 4 + 2, eight.z);
+                                add(c >> 2, (c & 3) * 4 + 3, eight.w);
+                            }
+                            __syncwarp();   // every lane has read its row
+                            if (lane == 0) mbar_arrive(&mask_empty[t]);
+                        } else if (bias_async) {
                             cp_async_wait_all();
                             __syncwarp();
-                            const uint64_t sc2b = pack2(sc, sc);
-                            // score * scale + mask for two keys: the mask's units, the exponent's factor follows later
-                            auto add = [&](int c, int i, uint32_t two) {
-                                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&two));
-                                float x0, x1;
-                                unpack2(fma2(pack2(__uint_as_float(r[c][2 * i]), __uint_as_float(r[c][2 * i + 1])), sc2b, pack2(f.x, f.y)),
-                                        x0, x1);
-                                r[c][2 * i] = __float_as_uint(x0);
-                                r[c][2 * i + 1] = __float_as_uint(x1);
-                            };
                             if (bias8) {
                                 const uint2* w = reinterpret_cast<const uint2*>(bias_rows + lane * 66);
 #pragma unroll
@@ -974,6 +1011,84 @@ static int make_qkv_map(b200_ctx* ctx, CUtensorMap* m, const b200_strided4* t, i
                      CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+// A mask whose rows lie on 16-byte boundaries, zero-filled to a multiple of 8 keys: one warp a row.  Any strides; rows of
+// contiguous keys are read by words from the 4-byte boundary at or below each eight's first entry, every word holding one.
+__global__ void __launch_bounds__(256)
+mask_rows_kernel(const __half* __restrict__ mask, uint4* __restrict__ out, int Lq, int Lk, int64_t rows, int planesH, int64_t bsK,
+                 int64_t bsQ, int64_t bsH, int64_t bsB) {
+    grid_dep_wait();
+    grid_dep_launch();
+    const int lane = threadIdx.x & 31;
+    const int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    const int64_t plane = row / Lq;
+    const __half* src = mask + (row - plane * Lq) * bsQ + (plane % planesH) * bsH + (plane / planesH) * bsB;
+    const int n8 = (Lk + 7) / 8;
+    uint4* dst = out + row * n8;
+    for (int c = lane; c < n8; c += 32) {
+        const int n = min(8, Lk - c * 8);
+        uint32_t v[4] = {0, 0, 0, 0};
+        if (bsK == 1) {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(src + c * 8);
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
+            const int odd = (int)(a >> 1) & 1, words = (n + odd + 1) >> 1;
+            uint32_t x[5];
+#pragma unroll
+            for (int i = 0; i < 5; ++i) x[i] = i < words ? __ldg(w + i) : 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = __funnelshift_r(x[i], x[i + 1], 16 * odd);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (i < n) v[i >> 1] |= (uint32_t)__half_as_ushort(src[(int64_t)(c * 8 + i) * bsK]) << (16 * (i & 1));
+        }
+        dst[c] = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+// The mask's tensor map, over the mask itself where its rows lie on 16-byte boundaries, else over a copy of it whose rows do
+// where that is worth a launch.  Leaves p->mask as it is where neither is to be had.
+// The copy costs 2 us and 0.9 per million entries; a CTA gains 0.95 us a key block over copies of 8 bytes by the softmax's own
+// warps (1.6 with its wider heads, and over copies of words), less where its 256 rows are not all there.  20 heads x 1500 x 1500
+// 42.1 -> 36.9 us, 2 x 8 x 1001 x 1001 31.1 -> 26.7, 4 x 20 x 1001 x 1001 x 32 88.8 -> 62.6; 2 x 2001 x 2001 x 128 would
+// go 24.6 -> 26.8 and 8 x 100 x 3001 16.2 -> 17.9.  Keys apart, 20 x 1500 x 1500 193 -> 92, 4 x 300 x 300 44.6 -> 14.5.  `serial`: key blocks a CTA walks.
+static int mask_map(b200_ctx* ctx, const __half* bptr, const int64_t* bs, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B,
+                    int64_t serial, AttnParams* p, CUtensorMap* tm) {
+    const uint64_t Hm = bs[2] != 0 ? (uint64_t)H : 1, Bm = bs[3] != 0 ? (uint64_t)B : 1;
+    const int64_t ext[4] = {Lk, Lq, (int64_t)Hm, (int64_t)Bm};
+    uint64_t dims[4] = {(uint64_t)Lk, (uint64_t)Lq, Hm, Bm}, str[3];
+    bool lies = (bs[0] == 1 || Lk == 1) && reinterpret_cast<uintptr_t>(bptr) % 16 == 0;
+    uint64_t dense = (uint64_t)(Lk + 7) / 8 * 16;   // a legal stride for an axis of extent one
+    for (int d = 1; d < 4; ++d) {
+        lies = lies && (ext[d] == 1 || (bs[d] > 0 && bs[d] % 8 == 0 && bs[d] < (1ll << 38)));
+        str[d - 1] = ext[d] == 1 ? dense : (uint64_t)bs[d] * 2;
+        dense *= (uint64_t)ext[d];
+    }
+    const void* base = bptr;
+    if (!lies) {
+        const int64_t rows = Lq * (int64_t)(Hm * Bm), n8 = (Lk + 7) / 8;
+        const bool apart = p->mask == MASK_DIRECT;
+        const double gain = (apart ? 6.0 : p->mask == MASK_EIGHTS && E <= 64 ? 0.95 : 1.6) * (double)serial;
+        if (gain * (Lq < 2 * ATT_BR ? (double)Lq / (2 * ATT_BR) : 1.0) < 2.0 + (apart ? 8e-6 : 0.9e-6) * (double)(rows * Lk)) return B200_OK;
+        void* ws = nullptr;
+        const int rc = ws_scratch(ctx, (size_t)(rows * n8) * 16, &ws);
+        if (rc == B200_ENOMEM) return B200_OK;
+        if (rc) return rc;
+        B200_CUDA(launch_dep(mask_rows_kernel, dim3((unsigned)cdiv(rows, 8), 1, 1), dim3(256, 1, 1), 0, ctx->stream, 1, bptr, (uint4*)ws,
+                             (int)Lq, (int)Lk, rows, (int)Hm, bs[0], bs[1], bs[2], bs[3]));
+        ctx->launches++;
+        base = ws;
+        str[0] = (uint64_t)n8 * 16;
+        str[1] = str[0] * (uint64_t)Lq;
+        str[2] = str[1] * Hm;
+    }
+    uint32_t box[4] = {64, ATT_BR, 1, 1};
+    const int rc = make_tmap(ctx, tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, base, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (rc) return rc;
+    p->mask = MASK_TMA;
+    return B200_OK;
+}
+
 } // namespace b200
 
 using namespace b200;
@@ -1111,12 +1226,14 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     p.trace = ctx->gemm_trace;
     p.bias = bptr;
     p.bsK = bs[0]; p.bsQ = bs[1]; p.bsH = bs[2]; p.bsB = bs[3];
-    p.bias_async = !bptr || !(bs[0] == 1 || Lk == 1) ? 0 : 1 + (reinterpret_cast<uintptr_t>(bptr) % 8 == 0 && bs[1] % 4 == 0 && bs[2] % 4 == 0 && bs[3] % 4 == 0);
+    p.mask = !(bs[0] == 1 || Lk == 1) ? MASK_DIRECT
+             : reinterpret_cast<uintptr_t>(bptr) % 8 == 0 && bs[1] % 4 == 0 && bs[2] % 4 == 0 && bs[3] % 4 == 0 ? MASK_EIGHTS : MASK_WORDS;
+    CUtensorMap tm = tq;   // not read unless there is a mask
     const int64_t nblk_all = cdiv(Lk, block);
     const int64_t item_rows = single ? ATT_BR : 2 * ATT_BR;
     auto launch = [&](dim3 grid) -> cudaError_t {
         auto go = [&](auto kern, int threads, size_t smem) {
-            return launch_dep(kern, grid, dim3(threads, 1, 1), smem, ctx->stream, 1, tq, tk, tv, p);
+            return launch_dep(kern, grid, dim3(threads, 1, 1), smem, ctx->stream, 1, tq, tk, tv, tm, p);
         };
         if (single) return go(attention_f16_tc_kernel<64, false, 1>, AttCfg<64, false, 1>::THREADS, AttCfg<64, false, 1>::SMEM_BYTES);
         if (wide && E <= 80 && !bptr) return go(attention_f16_tc_kernel<80, false, 2>, AttCfg<80>::THREADS, AttCfg<80>::SMEM_BYTES);
@@ -1166,6 +1283,11 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
             }
         }
     }
+    if (bptr) {
+        const int64_t waves = p.nsplit > 1 ? (pairs - p.ntail) / sms : cdiv(pairs, sms);
+        const int64_t serial = waves * nblk_all + (p.nsplit > 1 ? cdiv(nblk_all, p.nsplit) : 0);
+        if ((rc = mask_map(ctx, bptr, bs, E, Lq, Lk, H, B, serial, &p, &tm))) return rc;
+    }
     if (p.nsplit > 1) {
         p.pair_ctas = (int)(pairs - p.ntail);
         const int64_t ctas = p.pair_ctas + (int64_t)p.ntail * p.nsplit;
@@ -1184,6 +1306,7 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     p.pair_ctas = (int)(pairs - nsplit);
     B200_CUDA(launch(dim3((unsigned)(pairs + nsplit), 1, 1)));
     ctx->launches++;
+    if (frugal) ctx->ws_used = ws_mark;   // a repacked mask, as above
     return B200_OK;
 }
 

@@ -576,3 +576,47 @@ def test_reference_point_that_moves_in_later_blocks(ctx, E, Lq, Lk):
     # below 2^-14 of it, 2^-25 each), sums are fp32 over Lk terms
     vmax = np.abs(np.float64(v)).max()
     assert np.abs(got - ref).max() < vmax * (2.0 ** -11 + Lk * 2.0 ** -25 + 1e-5)
+
+
+@pytest.mark.parametrize("B,H,Lq,Lk,E", [(1, 8, 300, 1001, 64), (2, 6, 513, 640, 56), (1, 20, 129, 1500, 72), (3, 4, 260, 2050, 128), (1, 6, 1000, 127, 64)])
+@pytest.mark.parametrize("planes", ["all", "batch", "head", "keys"])
+def test_however_a_mask_lies_the_result_is_the_same(ctx, ora, B, H, Lq, Lk, E, planes):
+    """The same mask on 16-byte boundaries (read through a tensor map where its strides allow one), behind an odd number of
+    entries, on 8-byte boundaries, and with its keys apart: read in place or by way of a copy, every bit is the same."""
+    rng = np.random.default_rng(Lq + Lk + E)
+    q, k, v = (np.float16(rng.standard_normal((B, H, n, E))) for n in (Lq, Lk, Lk))
+    shape = {"all": (1, 1, Lq, Lk), "batch": (B, 1, Lq, Lk), "head": (1, H, Lq, Lk), "keys": (B, 1, 1, Lk)}[planes]
+    bias = np.float16(rng.standard_normal(shape))
+    bias[rng.random(shape) < 0.2] = -np.inf
+    if planes != "keys":
+        bias[..., Lq - 1, : Lk // 2] = -np.inf
+        bias[..., 0, :] = -np.inf
+    dq, dk, dv = qkv_views(ctx, q, k, v)
+
+    def run(pitch, offset, apart):
+        """`bias` in a device array whose rows are `pitch` entries apart (keys apart: whose keys are), `offset` entries in."""
+        n0, n1, n2, n3 = shape
+        inner, outer = (n2, n3) if apart else (n3, n2)
+        flat = np.full(offset + n0 * n1 * outer * pitch, np.nan, np.float16)
+        rows = flat[offset:].reshape(n0, n1, outer, pitch)[..., :inner]
+        rows[...] = bias.swapaxes(2, 3) if apart else bias
+        d = ctx.toback(flat)
+        plane = outer * pitch
+        st = (pitch, 1) if apart else (1, pitch)
+        db = jv.DeviceArray(ctx, d.ptr + 2 * offset, np.float16, (n3, n2, n1, n0), st + (plane, plane * n1), owner=d)
+        out = ctx.allocate(np.float32, E, Lq, H, B)
+        ctx.fill_bytes(out, 0xFF)
+        ctx.ws.reset()
+        jv.sdpa(ctx, dq, dk, dv, db, 1 / np.sqrt(E), out=out)
+        ctx.synchronize()
+        return out.to_host()
+
+    aligned = (Lk + 7) // 8 * 8
+    got = run(aligned, 0, False)
+    assert np.all(np.isfinite(got))
+    ref = ora.attention_ref(q, k, v, 1 / np.sqrt(E), bias=bias)
+    assert relerr(got, ref) < TOL, describe(got, ref, TOL)
+    if planes != "keys":
+        assert np.all(got[:, :, 0] == 0)
+    for pitch, offset, apart in ((aligned, 5, False), (aligned + 1, 0, False), (aligned + 4, 4, False), (Lq + 3, 1, True)):
+        assert np.array_equal(run(pitch, offset, apart), got), (pitch, offset, apart)
