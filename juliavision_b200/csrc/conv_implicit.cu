@@ -17,6 +17,7 @@
 //              Afterwards the epilogue, TMEM -> +bias, round, act -> global
 //   warp 8     TMA producer of the weight tile (K-major, straight from w)
 //   warp 9     UMMA issuer
+// In words, launches of more CTAs than that take four smaller ones per SM (CiCfg).
 // Measured (us, B200) against the im2col + GEMM route: 1024 x 1024 x 3 -> 112, 7 x 7 / 4: 35 -> 23.6; 300 x 296 x 16 -> 64,
 // 3 x 3: 42.5 -> 24.6; against the scalar GEMM odd pixel counts had: 43 x 42 x 256 -> 256, 3 x 3 / 2: 229 -> 14.2, two of
 // 230 x 225 x 32 -> 80, 3 x 3: 890 -> 43.  What is left is the gather's load latency.
@@ -41,17 +42,22 @@ namespace b200 {
 
 constexpr int CI_PIX = 128;              // pixels per CTA (TMEM lanes)
 constexpr int CI_BK = 64;                // one 128-byte swizzle row of the weight tile
-constexpr int CI_GATHER = 256;           // gather / epilogue threads
-constexpr int CI_THREADS = CI_GATHER + 64;
 constexpr int CI_A_BYTES = CI_PIX * CI_BK * 2;
 
-template <int BN> struct CiCfg {
-    static constexpr int STAGES = BN == 256 ? 2 : (BN == 128 ? 3 : 4);
+// SMALL: half the gather warps and a third to half of the ring, four CTAs to an SM, for launches of more than two an SM read in
+// words: a CTA's chain of waits is what takes the time, and four run beside each other (us on the device, two and four:
+// 1024 x 1024 x 3 -> 112, 7 x 7 / 4 15.7, 14.2, eight of them 92.8, 72.6; 512 x 512 x 16 -> 64, 3 x 3 / 2 12.9, 12.0; launches that
+// two an SM hold lose, 256 x 256 x 3 -> 96, 7 x 7 / 4 5.8, 6.9).  Issue slots are 45 % used then, the longest wait is for loads.
+template <int BN, bool SMALL = false> struct CiCfg {
+    static constexpr int GATHER = SMALL ? 128 : 256;   // gather / epilogue threads
+    static constexpr int THREADS = GATHER + 64;
+    static constexpr int CTAS = SMALL ? 4 : 2;
+    static constexpr int STAGES = SMALL ? (BN == 64 ? 2 : 1) : BN == 256 ? 2 : (BN == 128 ? 3 : 4);
     static constexpr int B_BYTES = BN * CI_BK * 2;
     static constexpr int STAGE_BYTES = CI_A_BYTES + B_BYTES;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + BN * 4 + 128;
-    static constexpr bool SPLITS = BN * CI_PIX * 4 <= STAGES * STAGE_BYTES;   // the fp32 tile fits over the drained ring
-    static_assert(2 * (SMEM_BYTES + 1024) <= 233472, "two CTAs per SM");
+    static constexpr bool SPLITS = !SMALL && BN * CI_PIX * 4 <= STAGES * STAGE_BYTES;   // the fp32 tile fits over the drained ring
+    static_assert(CTAS * (SMEM_BYTES + 1024) <= 233472 && CTAS * BN <= 512, "shared or tensor memory over budget");
 };
 
 struct ConvParams {
@@ -117,11 +123,13 @@ __device__ __forceinline__ void ldg_words_if(uint32_t (&v)[1], const uint16_t* p
 
 // grid (K parts, pixel tiles of all images, channel tiles); the K parts of a tile form a cluster.  G: columns of the
 // reduction per kernel row where the image is read in words, 0: tap by tap.
-template <int BN, typename OutT, int G>
-__global__ void __launch_bounds__(CI_THREADS, 2)
+template <int BN, typename OutT, int G, bool SMALL>
+__global__ void __launch_bounds__((CiCfg<BN, SMALL>::THREADS), (CiCfg<BN, SMALL>::CTAS))
 conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Cout}, boxes of 64 x BN
                      const ConvParams p) {
-    using Cfg = CiCfg<BN>;
+    using Cfg = CiCfg<BN, SMALL>;
+    constexpr int CI_GATHER = Cfg::GATHER, TMA_WARP = CI_GATHER / 32, ISSUE_WARP = TMA_WARP + 1;
+    static_assert(!SMALL || G > 0, "the small CTA reads the image in words");
     extern __shared__ __align__(1024) uint8_t smem[];
     if ((smem_u32(smem) & 1023u) != 0) {
         if (threadIdx.x == 0) atomicCAS(p.d_status, 0, KST_SMEM_LAYOUT);
@@ -150,7 +158,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
         fence_barrier_init();
         prefetch_tmap(&tmapW);
     }
-    if (warp == 8) {
+    if (warp == TMA_WARP) {
         tmem_alloc(tmem_slot, BN);
         tmem_relinquish();
     }
@@ -158,7 +166,10 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    grid_dep_wait();
+    // In words the kernel before this one lays out the weight, and lets this one start when all before it is done: the image
+    // and the bias are there, and only the weight has to be waited for
+    // (256 x 256 x 32 -> 128, 3 x 3 / 2, with the issuing warp below: 9.07 -> 8.18 us; 1024 x 1024 x 3 -> 112, 7 x 7 / 4: 15.83 -> 15.66).
+    if (G == 0 || warp == TMA_WARP) grid_dep_wait();
     grid_dep_launch();
 
     // Channel c of the tile at pixel pix, rounded before the activation sees it.  The activation is a template
@@ -176,7 +187,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
             default: body([](float v) { return apply_act(B200_EPI_GELU_TANH, v); }); break;
         }
     };
-    if (warp == 8) {
+    if (warp == TMA_WARP) {
         if (lane == 0) {
             for (int kb = 0; kb < nkb; ++kb) {
                 const int s = kb % Cfg::STAGES;
@@ -185,23 +196,26 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
                 tma_load_2d(smem + s * Cfg::STAGE_BYTES + CI_A_BYTES, &tmapW, &full[s], (kb0 + kb) * CI_BK, c0);
             }
         }
-    } else if (warp == 9) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc_f16(CI_PIX, BN, /*a MN-major, in words K-major*/ G == 0, /*b K-major*/ 0);
-            constexpr uint64_t adesc0 = G == 0 ? make_smem_desc(64 * CI_BK * 2, 1024) : make_smem_desc(16, 1024);
-            constexpr uint64_t bdesc0 = make_smem_desc(16, 1024);
-            bool ok = true;
-            for (int kb = 0; kb < nkb; ++kb) {
-                const int s = kb % Cfg::STAGES;
-                if (!mbar_wait(&full[s], (uint32_t)((kb / Cfg::STAGES) & 1), p.d_status, KST_WAIT_FULL, abort_flag)) { ok = false; break; }
-                tc_fence_after();
+    } else if (warp == ISSUE_WARP) {
+        // the warp waits together and the thread elect.sync picks issues, as in the GEMM
+        constexpr uint32_t idesc = make_idesc_f16(CI_PIX, BN, /*a MN-major, in words K-major*/ G == 0, /*b K-major*/ 0);
+        constexpr uint64_t adesc0 = G == 0 ? make_smem_desc(64 * CI_BK * 2, 1024) : make_smem_desc(16, 1024);
+        constexpr uint64_t bdesc0 = make_smem_desc(16, 1024);
+        bool ok = true;
+        for (int kb = 0; kb < nkb; ++kb) {
+            const int s = kb % Cfg::STAGES;
+            ok = mbar_wait(&full[s], (uint32_t)((kb / Cfg::STAGES) & 1), p.d_status, KST_WAIT_FULL, abort_flag);
+            if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+            tc_fence_after();
+            if (elect_one()) {
                 const uint32_t a = smem_u32(smem + s * Cfg::STAGE_BYTES), b = a + CI_A_BYTES;
 #pragma unroll
                 for (int k = 0; k < CI_BK / 16; ++k)   // 16 k: two 8-row groups of an MN-major A, 32 bytes inside a K-major swizzle row
                     umma_ss(tmem_base, smem_desc_at(adesc0, a + k * (G == 0 ? 2048 : 32)), smem_desc_at(bdesc0, b + k * 32), idesc, (kb | k) != 0);
                 umma_commit(&empty[s]);
+                if (kb + 1 == nkb) umma_commit(tfull);
             }
-            if (ok) umma_commit(tfull);
+            __syncwarp();
         }
     } else {
         for (int j = tid; j < BN; j += CI_GATHER)   // read in the epilogue, a barrier among these warps later
@@ -209,20 +223,22 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
         bool ok = true;
         if constexpr (G > 0) {
             const uint16_t* xi = reinterpret_cast<const uint16_t*>(p.x) + (int64_t)img * p.x_img;
-            // Pixel tid % 128; of a k-block's eight 16-byte pieces those of one parity.
+            // Pixel tid % 128; of a k-block's eight 16-byte pieces those of one parity, in SMALL all, the even ones first.
             constexpr int VL = G / 2, RPC = 8 / G;   // elements a load, kernel rows a piece
+            constexpr int HALVES = SMALL ? 2 : 1;   // SMALL: a thread takes all eight pieces of its pixel, four at a time
             const int pix = tid & 127, par = tid >> 7, m = m0 + pix;
             const int oh = m / p.OW, ow = m - oh * p.OW;
             const int bx = ow * p.sx - p.px, by = m < p.P ? oh * p.sy - p.py : -(1 << 30);   // never inside the image
             const bool in0 = (uint32_t)bx < (uint32_t)p.W, in1 = (uint32_t)(bx + VL) < (uint32_t)p.W;   // whole words: W is a multiple
             const int base = by * p.W + bx;
             uint32_t v[2][4][RPC][2][VL / 2];
-            auto load = [&](int kb, int b) {
+            auto load = [&](int st, int b) {
+                const int kb = st / HALVES, par1 = SMALL ? st & 1 : par;
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
 #pragma unroll
                     for (int u = 0; u < RPC; ++u) {
-                        const int r = ((kb0 + kb) * 8 + 2 * i + par) * RPC + u;   // the same for the warp
+                        const int r = ((kb0 + kb) * 8 + 2 * i + par1) * RPC + u;   // the same for the warp
                         const int cin = (int)div_magic((uint32_t)r, p.KH, p.mKH), ky = (r - cin * p.KH) * p.dy;
                         const bool row = r < p.rows && (uint32_t)(by + ky) < (uint32_t)p.H;
                         const uint16_t* src = xi + (base + (cin * p.H + ky) * p.W);
@@ -231,10 +247,11 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
                     }
             };
             load(0, 0);
-            auto step = [&](int kb, int b) -> bool {
-                const int s = kb % Cfg::STAGES;
-                if (kb + 1 < nkb) load(kb + 1, b ^ 1);
-                if (ok && !mbar_wait(&empty[s], (uint32_t)((kb / Cfg::STAGES) & 1) ^ 1, p.d_status, KST_WAIT_EMPTY, abort_flag)) ok = false;
+            const int nsteps = nkb * HALVES;
+            auto step = [&](int st, int b) -> bool {
+                const int kb = st / HALVES, s = kb % Cfg::STAGES, par1 = SMALL ? b : par;
+                if (st + 1 < nsteps) load(st + 1, b ^ 1);
+                if ((!SMALL || b == 0) && ok && !mbar_wait(&empty[s], (uint32_t)((kb / Cfg::STAGES) & 1) ^ 1, p.d_status, KST_WAIT_EMPTY, abort_flag)) ok = false;
                 if (__any_sync(0xffffffffu, !ok)) return ok = false;
                 const uint32_t a = smem_u32(smem + s * Cfg::STAGE_BYTES) + pix * 128;
 #pragma unroll
@@ -242,16 +259,17 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
                     uint32_t w[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) w[e] = v[b][i][e / (4 / RPC)][(e / (VL / 2)) & 1][e % (VL / 2)] & p.mask[e];
-                    st_shared_v4(a + (((2 * i + par) ^ (pix & 7)) << 4), w);
+                    st_shared_v4(a + (((2 * i + par1) ^ (pix & 7)) << 4), w);
                 }
+                if (SMALL && b == 0) return true;
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&full[s]);
                 return true;
             };
-            for (int kb = 0; kb < nkb; kb += 2) {   // by twos: the registers of a step are named at compile time
-                if (!step(kb, 0)) break;
-                if (kb + 1 < nkb && !step(kb + 1, 1)) break;
+            for (int st = 0; st < nsteps; st += 2) {   // by twos: the registers of a step are named at compile time
+                if (!step(st, 0)) break;
+                if (st + 1 < nsteps && !step(st + 1, 1)) break;
             }
         } else {
         // Pixels 2 lane, 2 lane + 1 of either half of the tile.
@@ -318,14 +336,15 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
         if (ok && !mbar_wait(tfull, 0, p.d_status, KST_WAIT_TMEM_FULL, abort_flag)) ok = false;
         if (!__any_sync(0xffffffffu, !ok)) {
             tc_fence_after();
-            const int quad = warp & 3, part = warp >> 2;   // tensor-memory lane quadrant, half of the channels
+            constexpr int SHARES = CI_GATHER / 128;
+            const int quad = warp & 3, part = warp >> 2;   // tensor-memory lane quadrant, share of the channels
             const int pix = m0 + quad * 32 + lane;
             const uint32_t tacc = tmem_base + (uint32_t(quad * 32) << 16);
-            const int cend = min((part + 1) * (BN / 2), p.Cout - c0);
+            const int cend = min((part + 1) * (BN / SHARES), p.Cout - c0);
             if (Cfg::SPLITS && parts > 1) {
                 float* acc = reinterpret_cast<float*>(smem) + quad * 32 + lane;   // [channel][pixel], over the drained ring
 #pragma unroll 1
-                for (int c = part * (BN / 2); c < cend; c += 16) {
+                for (int c = part * (BN / SHARES); c < cend; c += 16) {
                     uint32_t r[16];
                     tmem_ld16(tacc + c, r);
                     tmem_wait_ld();
@@ -335,7 +354,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
             } else {
                 by_act([&](auto act) {
 #pragma unroll 1
-                    for (int c = part * (BN / 2); c < cend; c += 16) {
+                    for (int c = part * (BN / SHARES); c < cend; c += 16) {
                         uint32_t r[16];
                         tmem_ld16(tacc + c, r);
                         tmem_wait_ld();
@@ -358,7 +377,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
     }
     if (Cfg::SPLITS && parts > 1) {
         cluster_sync_all();   // every part's tile is in its shared memory
-        if (warp < 8) {
+        if (warp < TMA_WARP) {
             const uint32_t mine = smem_u32(smem) + (tid & 127) * 4;
             const int pix = m0 + (tid & 127);
             // four channels' loads from every part in flight together: a remote load takes a few hundred nanoseconds
@@ -389,23 +408,23 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 8) {
+    if (warp == TMA_WARP) {
         tc_fence_after();
         tmem_dealloc(tmem_base, BN);
     }
 }
 
-template <int BN, typename OutT, int G>
+template <int BN, typename OutT, int G, bool SMALL = false>
 static int ci_launch(b200_ctx* ctx, const CUtensorMap& tw, const ConvParams& p, int64_t N, int parts) {
-    using Cfg = CiCfg<BN>;
+    using Cfg = CiCfg<BN, SMALL>;
     static bool attr_done[16] = {};
-    auto kern = conv_implicit_kernel<BN, OutT, G>;
+    auto kern = conv_implicit_kernel<BN, OutT, G, SMALL>;
     if (!attr_done[ctx->device & 15]) {
         B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
         attr_done[ctx->device & 15] = true;
     }
     dim3 grid((unsigned)parts, (unsigned)(p.tiles * N), (unsigned)cdiv(p.Cout, BN));
-    B200_CUDA(launch_dep(kern, grid, dim3(CI_THREADS, 1, 1), Cfg::SMEM_BYTES, ctx->stream, parts, tw, p));
+    B200_CUDA(launch_dep(kern, grid, dim3(Cfg::THREADS, 1, 1), Cfg::SMEM_BYTES, ctx->stream, parts, tw, p));
     ctx->launches++;
     return B200_OK;
 }
@@ -518,6 +537,7 @@ int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64
     }
     const CiTiles t = ci_tiles(ctx, p.tiles * N, p.CRS, Cout, g);
     const int bn = t.bn, parts = t.parts;
+    const bool small = parts == 1 && p.tiles * N * cdiv(Cout, bn) > 2 * ctx->prop.multiProcessorCount;
     CUtensorMap tw;
     uint64_t dims[2] = {(uint64_t)p.CRS, (uint64_t)Cout};
     uint64_t str[1] = {(uint64_t)ldw * 2};
@@ -527,6 +547,10 @@ int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64
     auto go = [&](auto zero, auto G) -> int {
         using T = decltype(zero);
         constexpr int g = decltype(G)::value;
+        if constexpr (g > 0) {
+            if (small && bn == 128) return ci_launch<128, T, g, true>(ctx, tw, p, N, 1);
+            if (small && bn == 64) return ci_launch<64, T, g, true>(ctx, tw, p, N, 1);
+        }
         if (bn == 256) return ci_launch<256, T, g>(ctx, tw, p, N, 1);
         if (bn == 128) return ci_launch<128, T, g>(ctx, tw, p, N, parts);
         return ci_launch<64, T, g>(ctx, tw, p, N, parts);

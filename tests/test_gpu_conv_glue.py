@@ -268,6 +268,28 @@ def test_conv_in_words_does_not_depend_on_the_workspace(ora, Cin, Cout, H, W, sc
         del g
 
 
+# more pixel tiles than two CTAs an SM take: 64 and 128 channels a CTA, ragged, one and several k-blocks, words of 4 and 2, two images
+@pytest.mark.parametrize("N,Cin,H,W,Cout,K,stride", [(1, 3, 808, 804, 112, 7, 4), (2, 3, 600, 608, 40, 7, 4), (1, 5, 395, 396, 72, 3, 2), (1, 24, 390, 400, 64, 3, 2)])
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+@pytest.mark.parametrize("act", ["identity", "gelu"])
+def test_conv_in_words_of_many_tiles(ctx, ora, N, Cin, H, W, Cout, K, stride, dt, act):
+    rng = np.random.default_rng(Cin + Cout + W)
+    x = np.float16(rng.standard_normal((N, Cin, H, W)) * 0.5)
+    w = np.float16(rng.standard_normal((Cout, Cin, K, K)) * 0.2)
+    b = np.float16(rng.standard_normal(Cout) * 0.2)
+    ref = ora.conv2d(x, w, b, (stride,) * 2, (K // 2,) * 2, epi={"identity": "none"}.get(act, act), out_dtype=dt)
+    out = ctx.allocate(dt, *reversed(ref.shape))
+    ctx.fill_bytes(out, 0xFF)
+    ctx.ws.reset()
+    half, dx, dw, db = ctx.toback(x * np.float16(0.5)), ctx.allocate(np.float16, W, H, Cin, N), ctx.toback(w), ctx.toback(b)
+    ctx.fill_bytes(dx, 0xFF)
+    jv.add_(ctx, dx, half, half)          # the image is the output of the kernel right before
+    jv.convolution_(ctx, out, dx, dw, db, (stride,) * 2, (K // 2,) * 2, (1, 1), 1, act=act)
+    ctx.synchronize()
+    tol = 2e-3 if dt == np.float16 else 2e-5      # as above
+    assert relerr(out.to_host(), ref) < tol, describe(out.to_host(), ref, tol)
+
+
 def test_conv_in_words_keeps_to_its_taps(ctx, ora):
     """An infinity or NaN beside a pixel's taps, inside the words that hold them, does not reach it."""
     x = np.float16(np.random.default_rng(3).standard_normal((1, 2, 16, 64)))
