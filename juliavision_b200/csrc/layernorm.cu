@@ -570,10 +570,101 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
     return warp_sum(t);
 }
 
-// Rows too wide for one warp's registers (more than 16 vectors per lane): one block per row, the row in registers as
-// above, the two sums over the block through shared memory.  Bound by HBM; with scalar accesses and the row read three
-// times these rows took 71.6 us for 7112 x 4280 in fp32, now 44.5 (5.5 TB/s); 79 x 3168 5.4 -> 3.3, 20000 x 5120 in fp16
-// 206 -> 106 (replayed over four operand sets).
+// Rows of more than some 224 vectors: a block per row, a thread four to six vectors of it, kept as read (fp16 stays packed, 28 to
+// 46 registers), moments and output two elements an instruction, the two sums through shared memory with one barrier each.
+// Bound by HBM; a warp a row (ln_warp_kernel) holds 8 registers a vector and then has too few rows in flight, 256 threads a row
+// too little each.  Microseconds, a warp or 256 threads a row before -> now, 80 Mi elements of fp16: 1800 wide 70.5 -> 66.8, 2056
+// 89.3 -> 68.8, 2560 84.6 -> 58.1 (5.5 TB/s), 3072 76.5 -> 60.8, 4096 112.3 -> 63.2, 5120 85.9 -> 59.7; 40 Mi of fp32: 1280 53.8 -> 51.6,
+// 2048 60.1 -> 52.3; in the L2, 1953 x 4096 16.8 -> 8.8; 64 x 4096 6.7 -> 3.2; behind the add 9765 x 4096 105 -> 51.7
+// (6.2 TB/s), 600 x 4096 11.7 -> 6.1.  Narrower rows lose (52083 x 1536: 59.2 -> 64.8).  gamma and beta asked for with
+// the row cost a fifth (registers), and so did rings of rows in shared memory that bulk copies fill, a warp a row (20480 x 4096: 98).
+// With ADD the residual add (and clamp) of ln_add_warp_kernel comes first, for the same widths and the same bits.
+template <typename InT, typename OutT, int VPT, bool ADD>
+__global__ void __launch_bounds__(1024)
+ln_split_kernel(const InT* a, InT* x, const InT* __restrict__ h, OutT* __restrict__ out, float* __restrict__ mean,
+                float* __restrict__ rstd, const InT* __restrict__ gamma, const InT* __restrict__ beta, int C, float eps,
+                int use_clamp, float lo, float hi) {
+    constexpr int VN = Vec16<InT>::N;
+    __shared__ float red[2][32];
+    const int64_t g = blockIdx.x;
+    const int nvec = C / VN, tid = threadIdx.x, T = blockDim.x, warp = tid >> 5, lane = tid & 31, warps = T >> 5;
+    const uint4* src = reinterpret_cast<const uint4*>((ADD ? x : a) + g * (int64_t)C);
+    grid_dep_wait();     // the input is the previous kernel's output
+    grid_dep_launch();
+    Vec16<InT> raw[VPT], hv[ADD ? VPT : 1];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+        if (tid + T * i < nvec) {
+            raw[i].raw = src[tid + T * i];
+            if constexpr (ADD) hv[i].raw = __ldg(reinterpret_cast<const uint4*>(h + g * (int64_t)C) + tid + T * i);
+        }
+    uint64_t s = pack2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+        if (tid + T * i < nvec) {
+            float f[VN];
+            raw[i].to_f32(f);
+            if constexpr (ADD) {
+                float fh[VN];
+                hv[i].to_f32(fh);
+#pragma unroll
+                for (int j = 0; j < VN; ++j) {
+                    f[j] = __half2float(__float2half_rn(f[j] + fh[j]));        // add.Tensor rounds here
+                    if (use_clamp) f[j] = __half2float(__float2half_rn(fminf(fmaxf(f[j], lo), hi)));
+                }
+                store_vec<VN>(reinterpret_cast<InT*>(&raw[i].raw), f);          // exact: already fp16 values
+                *(reinterpret_cast<uint4*>(x + g * (int64_t)C) + tid + T * i) = raw[i].raw;
+            }
+#pragma unroll
+            for (int j = 0; j < VN; j += 2) s = add2(s, pack2(f[j], f[j + 1]));
+        }
+    auto block_total = [&](float v, float* r) {
+        v = warp_sum(v);
+        if (lane == 0) r[warp] = v;
+        __syncthreads();
+        return warp_sum(lane < warps ? r[lane] : 0.f);
+    };
+    const float n = (float)C;
+    const float mu = block_total(pairs_sum(s), red[0]) / n;
+    const uint64_t nmu = pack2(-mu, -mu);
+    s = pack2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+        if (tid + T * i < nvec) {
+            float f[VN];
+            raw[i].to_f32(f);
+#pragma unroll
+            for (int j = 0; j < VN; j += 2) {
+                const uint64_t d = add2(pack2(f[j], f[j + 1]), nmu);
+                s = fma2(d, d, s);
+            }
+        }
+    const float r = 1.0f / sqrtf(block_total(pairs_sum(s), red[1]) / n + eps);
+    OutT* dst = out + g * (int64_t)C;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int v = tid + T * i;
+        if (v < nvec) {
+            float f[VN];
+            uint64_t d[VN / 2];
+            raw[i].to_f32(f);
+#pragma unroll
+            for (int j = 0; j < VN / 2; ++j) d[j] = add2(pack2(f[2 * j], f[2 * j + 1]), nmu);
+            uint4 gv = make_uint4(0u, 0u, 0u, 0u), bv = gv;
+            if (gamma) gv = __ldg(reinterpret_cast<const uint4*>(gamma) + v);
+            if (beta) bv = __ldg(reinterpret_cast<const uint4*>(beta) + v);
+            ln_write<InT, OutT>(dst + (int64_t)v * VN, d, r, gamma != nullptr, gv, beta != nullptr, bv);
+        }
+    }
+    if (tid == 0) {
+        mean[g] = mu;
+        rstd[g] = r;
+    }
+}
+
+// fp32 rows of more than 512 vectors, and as wide fp16 ones in launches of few rows: 256 threads a row, the row in registers,
+// the two sums over the block through shared memory.  Bound by HBM; with scalar accesses and the row read three
+// times these rows took 71.6 us for 7112 x 4280 in fp32, now 44.5 (5.5 TB/s; replayed over four operand sets).
 template <typename InT, typename OutT, int VPT>
 __global__ void __launch_bounds__(LN_WIDE_THREADS)
 ln_wide_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restrict__ mean, float* __restrict__ rstd,
@@ -712,6 +803,15 @@ static bool ln_fills(const b200_ctx* ctx, int64_t groups, int rows, int lpg, int
     return groups >= n * ctx->prop.multiProcessorCount * 4 * rows * (32 / lpg);
 }
 
+// Vectors a thread of ln_split_kernel, 0 for rows that stay with the other kernels.  Past 512 vectors 256 threads a row are as fast
+// in fp32 (2400 x 2600: 12.6 us, 13.8; 11111 x 3600 50.5, 52.9), and in fp16 where a launch waits for a block or two (64 x
+// 5120: 3.4 us, 3.7; 1200 x 5120 7.1, 6.4): the last bits of a row of more than 4096 depend on that.
+template <typename InT> static int ln_split(const b200_ctx* ctx, int64_t groups, int nvec) {
+    if (sizeof(InT) == 4) return nvec > 256 && nvec <= 512 ? 6 : 0;
+    if (nvec <= 224 || (nvec > 512 && groups <= (int64_t)4 * ctx->prop.multiProcessorCount)) return 0;
+    return cdiv(cdiv(nvec, 5), 32) < cdiv(cdiv(nvec, 4), 32) ? 5 : 4;
+}
+
 template <typename InT, typename OutT>
 static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, void* out, float* mean,
                      float* rstd, const void* gamma, const void* beta, float eps) {
@@ -758,7 +858,16 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
         else if (ln_fills(ctx, groups, 2, L, sizeof(InT) == 4 ? 10 : 14)) LN_GO_ROWS(1, L, 2);              \
         else ONE;                                                                                           \
     } while (0)
-        if (nvec <= 8) LN_GO_NARROW(8, LN_GO_SHARED(8));
+        // A block a row: the vectors a thread that leave fewer lanes idle (320 vectors: five of 64 threads, four would be of 96).
+        const int split = ln_split<InT>(ctx, groups, nvec);
+        auto go_split = [&](auto kern) {
+            return launch_dep(kern, dim3((unsigned)groups), dim3((unsigned)cdiv(cdiv(nvec, split), 32) * 32), 0, ctx->stream, 1, ap,
+                              (InT*)nullptr, (const InT*)nullptr, op, mean, rstd, gp, bp, (int)C, eps, 0, 0.f, 0.f);
+        };
+        if (split == 4) B200_CUDA(go_split(ln_split_kernel<InT, OutT, 4, false>));
+        else if (split == 5) B200_CUDA(go_split(ln_split_kernel<InT, OutT, 5, false>));
+        else if (split == 6) B200_CUDA(go_split(ln_split_kernel<InT, OutT, 6, false>));
+        else if (nvec <= 8) LN_GO_NARROW(8, LN_GO_SHARED(8));
         else if (nvec <= 16) LN_GO_NARROW(16, LN_GO_SHARED(16));
         else if (vpl <= 1) LN_GO_NARROW(32, LN_GO(1));
         else if (vpl <= 2) LN_GO(2);
@@ -767,8 +876,6 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
         else if (vpl <= 5) LN_GO(5);
         else if (vpl <= 6) LN_GO(6);
         else if (vpl <= 8) LN_GO(8);
-        else if (vpl <= 12) LN_GO(12);
-        else if (vpl <= 16) LN_GO(16);
         else if (nvec <= 4 * LN_WIDE_THREADS)
             B200_CUDA(launch_dep(ln_wide_kernel<InT, OutT, 4>, dim3((unsigned)groups), dim3(LN_WIDE_THREADS), 0, ctx->stream, 1, ap,
                                  op, mean, rstd, gp, bp, (int)C, eps));
@@ -844,7 +951,15 @@ extern "C" int b200_add_layernorm_f16(b200_ctx* ctx, int64_t groups, int64_t C, 
         else if (ln_fills(ctx, groups, 2, L, 20)) LNA_GO_ROWS(1, L, 2);                                           \
         else ONE;                                                                                                 \
     } while (0)
-    if (nvec <= 8) LNA_GO_NARROW(8, LNA_GO_SHARED(8));
+    const int split = ln_split<__half>(ctx, groups, nvec);
+    auto go_split = [&](auto kern) {
+        return launch_dep(kern, dim3((unsigned)groups), dim3((unsigned)cdiv(cdiv(nvec, split), 32) * 32), 0, ctx->stream, 1,
+                          (const __half*)nullptr, (__half*)x, (const __half*)h, (__half*)out, mean, rstd, (const __half*)gamma,
+                          (const __half*)beta, (int)C, eps, use_clamp, lo, hi);
+    };
+    if (split == 4) B200_CUDA(go_split(ln_split_kernel<__half, __half, 4, true>));
+    else if (split == 5) B200_CUDA(go_split(ln_split_kernel<__half, __half, 5, true>));
+    else if (nvec <= 8) LNA_GO_NARROW(8, LNA_GO_SHARED(8));
     else if (nvec <= 16) LNA_GO_NARROW(16, LNA_GO_SHARED(16));
     else if (vpl <= 1) LNA_GO_NARROW(32, LNA_GO(1));
     else if (vpl <= 2 && ln_fills(ctx, groups, 2, 32, 10)) LNA_GO_ROWS(2, 32, 2);
@@ -853,9 +968,7 @@ extern "C" int b200_add_layernorm_f16(b200_ctx* ctx, int64_t groups, int64_t C, 
     else if (vpl <= 4) LNA_GO(4);
     else if (vpl <= 5) LNA_GO(5);
     else if (vpl <= 6) LNA_GO(6);
-    else if (vpl <= 8) LNA_GO(8);
-    else if (vpl <= 12) LNA_GO(12);
-    else LNA_GO(16);
+    else LNA_GO(8);
 #undef LNA_GO
 #undef LNA_GO_SHARED
 #undef LNA_GO_ROWS

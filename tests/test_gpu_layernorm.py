@@ -191,3 +191,38 @@ def test_several_narrow_rows_at_a_time(ctx, ora, dt, C, groups):
         ctx.synchronize()
         for one, other in ((xa, xb), (oa, ob), (m1, m2), (r1, r2)):
             assert np.array_equal(one.to_host(), other.to_host())
+
+
+# the narrowest and widest rows of the form of a block a row, those next to them, four and five vectors a thread, idle lanes
+SPLIT = [(np.float16, 1792, 70), (np.float16, 1800, 70), (np.float16, 2056, 600), (np.float16, 2560, 70), (np.float16, 3080, 70),
+         (np.float16, 4096, 2400), (np.float16, 4104, 592), (np.float16, 4104, 593), (np.float16, 5120, 600), (np.float16, 16384, 600),
+         (np.float32, 1024, 70), (np.float32, 1028, 70), (np.float32, 1540, 600), (np.float32, 2048, 70)]
+
+
+@pytest.mark.parametrize("dt,C,groups", SPLIT)
+def test_a_block_a_row(ctx, ora, dt, C, groups):
+    rng = np.random.default_rng(C + groups)
+    a = (rng.standard_normal((groups, C), dtype=np.float32) * 2 + 0.5).astype(dt)
+    gam, bet = ((o + 0.1 * rng.standard_normal(C)).astype(dt) for o in (1, 0))
+    tol = 1.5e-3 if dt == np.float16 else 2e-6      # as above: a few fp32 ulps of the sums, at most one output ulp
+    for g, b in ((gam, bet), (gam, None), (None, bet), (None, None)):
+        got, mean, rstd = layernorm_gpu(ctx, a, g, b, 1e-5)
+        ref, rmean, rrstd = ora.layernorm(a, g, b, 1e-5, out_dtype=dt)
+        assert relerr(got, ref) < tol, describe(got, ref, tol)
+        assert np.max(np.abs(mean - rmean)) < 1e-5 and relerr(rstd, rrstd) < 1e-5
+    if dt != np.float16:
+        return
+    h = (rng.standard_normal((groups, C), dtype=np.float32)).astype(dt)     # behind the add: the three ops, bit for bit
+    for clamp in (None, (-1.5, 2.0)):
+        xa, xb, dh, dg, db = (ctx.toback(t) for t in (a, a, h, gam, bet))
+        m1, r1, m2, r2 = (ctx.allocate(np.float32, groups) for _ in range(4))
+        oa, ob = ctx.allocate(dt, C, groups), ctx.allocate(dt, C, groups)
+        jv.add_(ctx, xa, xa, dh)
+        if clamp:
+            jv.clamp_(ctx, xa, xa, *clamp)
+        jv.layernorm_(ctx, oa, m1, r1, xa, dg, db, C, 1e-5)
+        ctx.fill_bytes(ob, 0xFF)
+        jv.add_layernorm_(ctx, ob, m2, r2, xb, dh, dg, db, C, 1e-5, clamp=clamp)
+        ctx.synchronize()
+        for one, other in ((xa, xb), (oa, ob), (m1, m2), (r1, r2)):
+            assert np.array_equal(one.to_host(), other.to_host())
