@@ -17,6 +17,9 @@
 // windows of up to 256 keys, one tile in blocks of 64; the kernel comment below gives the roles and the pipeline.
 #include <cuda_fp16.h>
 
+#include <mutex>
+#include <type_traits>
+
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -81,7 +84,16 @@ template <int EP, bool BIAS = false, int NT_ = 2> struct AttCfg {
     static constexpr int BARRIERS = 2 + 2 * K_STAGES + 2 * V_STAGES + 10 + (EP == 128 ? 2 : 0) + (BIAS ? 4 : 0);
     static constexpr int SMEM_BYTES = S_BARS + (BARRIERS + 1) * 8;
     static_assert(CTAS_PER_SM * (SMEM_BYTES + 1024) <= 233472, "shared memory over budget");
+    // Joining: a CTA's share of an item's rows from all of them, over the operand tiles, [part][four columns][row] of 16 bytes (16 more
+    // between columns, so that neighbouring fours of a row lie in other banks); behind them [part][row] (reference point, sum).
+    static constexpr int join_bytes(int parts) {
+        const int share = (NT * ATT_BR + parts - 1) / parts;
+        return parts * (EP / 4 * (share * 16 + 16) + share * 8);
+    }
+    static_assert(NT == 1 || (join_bytes(2) <= S_V + V_STAGES * KV_BYTES && join_bytes(8) <= S_V + V_STAGES * KV_BYTES),
+                  "the rows to join fit over the operand tiles");
 };
+constexpr int JOIN_MOST = 8;   // CTAs of a portable cluster
 // tensor-memory map of two tiles (512 columns): S of tile t, fp32, at [128 t, 128 t + 128); O of tile t, fp32, at
 // [256 + EP t, ... + EP); P of tile t, fp16 packed two keys per column, at [384 + 64 t, ... + 64) for EP = 64, at
 // [416 + 48 t, ... + 48) for EP = 80 and over the first 64 columns of S_t for EP = 128
@@ -164,7 +176,9 @@ __device__ __forceinline__ void tmem_st16_raw(uint32_t taddr, const uint32_t* r)
 // the P V product takes its A operand from there, so the shared-memory port only feeds K and V.
 // BIAS: the scaled score gets an additive fp16 mask before the softmax; a row whose keys are all
 // blocked (-inf everywhere) comes out as zeros, as in attn_softmax (attention.jl:73-100).
-template <int EP, bool BIAS, int NT_>
+// JOIN: the CTAs an item's keys are cut over are a cluster, which joins their rows through distributed shared memory: an instance of
+// its own (in one with the others its code cost their loop 13 %).
+template <int EP, bool BIAS, int NT_, bool JOIN>
 __global__ void __launch_bounds__(AttCfg<EP, BIAS, NT_>::THREADS, AttCfg<EP, BIAS, NT_>::CTAS_PER_SM)
 attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                         const __grid_constant__ CUtensorMap tmapK,
@@ -276,6 +290,8 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
     // Everything above overlapped the previous kernel's tail; from here on its results are needed.
     grid_dep_wait();
     grid_dep_launch();
+
+    bool met = false;   // joining: this warp has passed the barrier behind which the rows are there
 
     // Register budget: the two softmax warpgroups hold a full score row per thread; the third
     // warpgroup (one TMA lane, one UMMA lane, two idle warps) needs almost nothing and hands its
@@ -706,8 +722,28 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             // Epilogue: O / l to global through the caller's output strides.
             if (ok && nblk > 0)
                 ok = mbar_wait(&pv_done[t], (uint32_t)((nblk - 1) & 1), p.d_status, KST_WAIT_SOFTMAX, abort_flag);
-            if (ok) {
-                constexpr int W = EP % 32 ? 16 : 32;   // columns a step
+            constexpr int W = EP % 32 ? 16 : 32;   // columns a step
+            if (JOIN) {
+                cluster_sync_all();       // nobody in the cluster reads its K, V or Q any more
+                met = true;
+                const int share = (ITEM_ROWS + nsp - 1) / nsp, nch = p.E >> 2;   // rows a CTA finishes, fours of a row
+                const int r = t * ATT_BR + row, owner = r / share, col = share * 16 + 16;
+                const uint32_t to = mapa_u32(smem_u32(smem), owner);
+                if (ok) {
+                    tc_fence_after();
+                    const uint32_t at = to + split * nch * col + (r - owner * share) * 16;
+#pragma unroll 1
+                    for (int c = 0; c < EP / W; ++c) {
+                        uint32_t v[W];
+                        tmem_ld(o_tmem + c * W, v);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int i = 0; i < W; i += 4)
+                            if (c * W + i < p.E) st_cluster_v4(at + (c * W + i) / 4 * col, v[i], v[i + 1], v[i + 2], v[i + 3]);
+                    }
+                    st_cluster_f32x2(to + nsp * nch * col + (split * share + r - owner * share) * 8, m_run, l_run);
+                }
+            } else if (ok) {
                 tc_fence_after();
                 const int lq = q0 + t * ATT_BR + row;
                 if (nsp > 1) {
@@ -772,8 +808,64 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
                 }   // nsplit == 1
             }
         }
+        if constexpr (JOIN) {
+            // Each CTA of the cluster finishes its share of the rows, in split order, as attention_merge_kernel does:
+            // out = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M), M the largest reference point.
+            if (!met) cluster_sync_all();
+            met = true;
+            cluster_sync_all();   // every part's rows are there
+            // share <= 128 rows, so at least two threads a row, each every per-th four of it
+            const int share = (ITEM_ROWS + nsp - 1) / nsp, nch = p.E >> 2;
+            const int r0 = split * share, n = min(min(share, ITEM_ROWS - r0), p.Lq - q0 - r0), col = share * 16 + 16;
+            const int per = 128 * NT / share, r = threadIdx.x / per;
+            if (r < n) {
+                const float2* ml = reinterpret_cast<const float2*>(smem + nsp * nch * col + r * 8);
+                float w[JOIN_MOST], M = -INFINITY, den = 0.f;
+                float2 f[JOIN_MOST];
+#pragma unroll
+                for (int s = 0; s < JOIN_MOST; ++s) f[s] = s < nsp ? ml[s * share] : make_float2(-INFINITY, 0.f);
+#pragma unroll
+                for (int s = 0; s < JOIN_MOST; ++s) M = fmaxf(M, f[s].x);
+#pragma unroll
+                for (int s = 0; s < JOIN_MOST; ++s) {
+                    w[s] = (f[s].x == -INFINITY) ? 0.f : exp2f(f[s].x - M);
+                    den = fmaf(f[s].y, w[s], den);
+                }
+                const float inv = 1.0f / (den == 0.f ? 1.0f : den);
+                const int64_t at0 = (q0 + r0 + r) * p.osL + h * p.osH + b * p.osB;
+#pragma unroll 2
+                for (int c = threadIdx.x - r * per; c < nch; c += per) {
+                    const uint8_t* o = smem + c * col + r * 16;
+                    float4 v[JOIN_MOST], num = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int s = 0; s < JOIN_MOST; ++s)
+                        if (s < nsp) v[s] = *reinterpret_cast<const float4*>(o + s * nch * col);
+#pragma unroll
+                    for (int s = 0; s < JOIN_MOST; ++s)
+                        if (s < nsp) {
+                            num.x = fmaf(v[s].x, w[s], num.x);
+                            num.y = fmaf(v[s].y, w[s], num.y);
+                            num.z = fmaf(v[s].z, w[s], num.z);
+                            num.w = fmaf(v[s].w, w[s], num.w);
+                        }
+                    const int64_t at = at0 + 4 * c;
+                    if (p.out_f32) {
+                        *reinterpret_cast<float4*>(static_cast<float*>(p.out) + at) = make_float4(num.x * inv, num.y * inv, num.z * inv, num.w * inv);
+                    } else {
+                        uint2 h2;
+                        *reinterpret_cast<__half2*>(&h2.x) = __floats2half2_rn(num.x * inv, num.y * inv);
+                        *reinterpret_cast<__half2*>(&h2.y) = __floats2half2_rn(num.z * inv, num.w * inv);
+                        *reinterpret_cast<uint2*>(static_cast<__half*>(p.out) + at) = h2;
+                    }
+                }
+            }
+        }
     }
 
+    if (JOIN && !met) {   // the roles without rows: the two barriers of a join
+        cluster_sync_all();
+        cluster_sync_all();
+    }
     if (*abort_flag) {
         for (int i = 0; i < 4; ++i) __nanosleep(1000000);
     }
@@ -1013,6 +1105,74 @@ static int make_qkv_map(b200_ctx* ctx, CUtensorMap* m, const b200_strided4* t, i
                      CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+// How many clusters of 2 to JOIN_MOST CTAs of an SM each the GPU holds at once (a GPC's SMs do not divide without a rest: 45 of
+// three, not 49): asked once per device.
+struct AttRooms { int clusters[JOIN_MOST + 1]; };
+static const AttRooms& att_rooms(b200_ctx* ctx) {
+    static std::once_flag once[16];
+    static AttRooms rooms[16];
+    const int d = ctx->device & 15;
+    std::call_once(once[d], [&] {
+        using Cfg = AttCfg<64>;
+        auto kern = attention_f16_tc_kernel<64, false, 2, false>;
+        AttRooms& got = rooms[d];
+        got = {};
+        if (cudaSetDevice(ctx->device) != cudaSuccess ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        for (int n = 2; n <= JOIN_MOST; ++n) {
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)n;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)(ctx->prop.multiProcessorCount / n * n), 1, 1);
+            cfg.blockDim = dim3(Cfg::THREADS, 1, 1);
+            cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int fit = 0;
+            if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) == cudaSuccess) got.clusters[n] = fit;
+            else cudaGetLastError();
+        }
+    });
+    return rooms[d];
+}
+
+// Over how many CTAs the keys of each of `pairs` items are cut, and whether those are a cluster that joins its rows in the launch.
+// The estimate beside a call's start, in us, fitted to 250 shapes of 2 to 18 heads and 400 to 2040 keys (2 to 7 % off): `block` and
+// `load` x the SMs used per key block, a cluster's `join`, or a second launch that merges (`merge` and `rows` x the parts' rows / 256).
+// Items of one tile have few rows to merge and do not join (16 heads, 40 x 8192 x 128: 24.9 us merged, 29.0); clusters that would
+// fill their room exactly may take two rounds (45 of three: 14.9 us and 23).
+// A join is the cheapest cut wherever its clusters are resident at once: 1.05 to 1.65 times as fast as merging, 1.29 in the mean
+// (9 heads x 2040 x 64 28.0 -> 21.5 us, 18 x 1020 22.2 -> 15.0, 12 x 900 x 128 23.2 -> 18.9); two and three key blocks, and many
+// pairs of four, stay whole (12 heads x 400: 9.9 us, 13.0 merged).  More than eight parts are worth a merge where pairs are few.
+struct AttSplit { int parts; bool join; };
+static AttSplit att_split(b200_ctx* ctx, int64_t pairs, int64_t nblk, int64_t Lq, int64_t E, bool masked) {
+    struct Cost { double block, load, join, merge, rows; };
+    static const Cost costs[5] = {{1.35, 0.37, 3.65, 4.15, 0.035}, {1.44, 0.57, 4.4, 4.75, 0.038}, {1.83, 0.46, 4.7, 5.4, 0.038},
+                                  {2.07, 0.56, 3.9, 5.15, 0.035}, {2.44, 0.77, 4.7, 5.6, 0.042}};
+    const Cost& c = costs[masked ? 3 + (E > 64) : (E > 64) + (E > 80)];
+    const int64_t sms = ctx->prop.multiProcessorCount;
+    auto walk = [&](int64_t n) { return (double)cdiv(nblk, n) * (c.block + c.load * (double)(pairs * n) / (double)sms); };
+    const AttRooms& rooms = att_rooms(ctx);
+    AttSplit best = {1, false};
+    double least = walk(1);
+    for (int n = 2; n <= JOIN_MOST && n <= nblk && Lq > ATT_BR; ++n)
+        if (pairs < rooms.clusters[n] + (n == 2) && walk(n) + c.join < least) {
+            least = walk(n) + c.join;
+            best = {n, true};
+        }
+    int64_t n = sms / pairs;
+    if (n > nblk / 2) n = nblk / 2;
+    if (n > 64) n = 64;
+    if (n >= 2 && walk(n) + c.merge + c.rows * (double)(pairs * n) * (Lq < 2 * ATT_BR ? (double)Lq / (2 * ATT_BR) : 1.0) < least) best = {(int)n, false};
+    return best;
+}
+
 // A mask whose rows lie on 16-byte boundaries, zero-filled to a multiple of 8 keys: one warp a row.  Any strides; rows of
 // contiguous keys are read by words from the 4-byte boundary at or below each eight's first entry, every word holding one.
 __global__ void __launch_bounds__(256)
@@ -1069,13 +1229,18 @@ static int mask_map(b200_ctx* ctx, const __half* bptr, const int64_t* bs, int64_
     const void* base = bptr;
     if (!lies) {
         const int64_t rows = Lq * (int64_t)(Hm * Bm), n8 = (Lk + 7) / 8;
-        const bool apart = p->mask == MASK_DIRECT;
-        const double gain = (apart ? 6.0 : p->mask == MASK_EIGHTS && E <= 64 ? 0.95 : 1.6) * (double)serial;
-        if (gain * (Lq < 2 * ATT_BR ? (double)Lq / (2 * ATT_BR) : 1.0) < 2.0 + (apart ? 8e-6 : 0.9e-6) * (double)(rows * Lk)) return B200_OK;
+        // Its room is asked for before it is weighed, so that a context gets it with its first masked call.
+        const size_t mark = ctx->ws_used;
         void* ws = nullptr;
         const int rc = ws_scratch(ctx, (size_t)(rows * n8) * 16, &ws);
         if (rc == B200_ENOMEM) return B200_OK;
         if (rc) return rc;
+        const bool apart = p->mask == MASK_DIRECT;
+        const double gain = (apart ? 6.0 : p->mask == MASK_EIGHTS && E <= 64 ? 0.95 : 1.6) * (double)serial;
+        if (gain * (Lq < 2 * ATT_BR ? (double)Lq / (2 * ATT_BR) : 1.0) < 2.0 + (apart ? 8e-6 : 0.9e-6) * (double)(rows * Lk)) {
+            ctx->ws_used = mark;
+            return B200_OK;
+        }
         B200_CUDA(launch_dep(mask_rows_kernel, dim3((unsigned)cdiv(rows, 8), 1, 1), dim3(256, 1, 1), 0, ctx->stream, 1, bptr, (uint4*)ws,
                              (int)Lq, (int)Lk, rows, (int)Hm, bs[0], bs[1], bs[2], bs[3]));
         ctx->launches++;
@@ -1183,18 +1348,18 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     }
     static bool attr_done[16] = {};
     if (!attr_done[ctx->device & 15]) {
-        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<64, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       AttCfg<64, false, 1>::SMEM_BYTES));
-        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<64, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       AttCfg<64>::SMEM_BYTES));
-        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<64, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       AttCfg<64, true>::SMEM_BYTES));
-        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<80, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       AttCfg<80>::SMEM_BYTES));
-        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<128, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       AttCfg<128>::SMEM_BYTES));
-        B200_CUDA(cudaFuncSetAttribute(attention_f16_tc_kernel<128, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       AttCfg<128, true>::SMEM_BYTES));
+        auto allow = [](auto kern, int bytes) { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
+        B200_CUDA(allow(attention_f16_tc_kernel<64, false, 1, false>, AttCfg<64, false, 1>::SMEM_BYTES));
+        B200_CUDA(allow(attention_f16_tc_kernel<64, false, 2, false>, AttCfg<64>::SMEM_BYTES));
+        B200_CUDA(allow(attention_f16_tc_kernel<64, false, 2, true>, AttCfg<64>::SMEM_BYTES));
+        B200_CUDA(allow(attention_f16_tc_kernel<64, true, 2, false>, AttCfg<64, true>::SMEM_BYTES));
+        B200_CUDA(allow(attention_f16_tc_kernel<64, true, 2, true>, AttCfg<64, true>::SMEM_BYTES));
+        B200_CUDA(allow(attention_f16_tc_kernel<80, false, 2, false>, AttCfg<80>::SMEM_BYTES));
+        B200_CUDA(allow(attention_f16_tc_kernel<80, false, 2, true>, AttCfg<80>::SMEM_BYTES));
+        B200_CUDA(allow(attention_f16_tc_kernel<128, false, 2, false>, AttCfg<128>::SMEM_BYTES));
+        B200_CUDA(allow(attention_f16_tc_kernel<128, false, 2, true>, AttCfg<128>::SMEM_BYTES));
+        B200_CUDA(allow(attention_f16_tc_kernel<128, true, 2, false>, AttCfg<128, true>::SMEM_BYTES));
+        B200_CUDA(allow(attention_f16_tc_kernel<128, true, 2, true>, AttCfg<128, true>::SMEM_BYTES));
         attr_done[ctx->device & 15] = true;
     }
     // Many windows of at most 64 keys: bound by HBM and latency, not by the tensor pipe; the small-tile
@@ -1233,43 +1398,51 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     CUtensorMap tm = tq;   // not read unless there is a mask
     const int64_t nblk_all = cdiv(Lk, block);
     const int64_t item_rows = single ? ATT_BR : 2 * ATT_BR;
-    auto launch = [&](dim3 grid) -> cudaError_t {
+    auto launch = [&](dim3 grid, int cluster = 1) -> cudaError_t {
         auto go = [&](auto kern, int threads, size_t smem) {
-            return launch_dep(kern, grid, dim3(threads, 1, 1), smem, ctx->stream, 1, tq, tk, tv, tm, p);
+            return launch_dep(kern, grid, dim3(threads, 1, 1), smem, ctx->stream, cluster, tq, tk, tv, tm, p);
         };
-        if (single) return go(attention_f16_tc_kernel<64, false, 1>, AttCfg<64, false, 1>::THREADS, AttCfg<64, false, 1>::SMEM_BYTES);
-        if (wide && E <= 80 && !bptr) return go(attention_f16_tc_kernel<80, false, 2>, AttCfg<80>::THREADS, AttCfg<80>::SMEM_BYTES);
-        if (wide)
-            return bptr ? go(attention_f16_tc_kernel<128, true, 2>, AttCfg<128, true>::THREADS, AttCfg<128, true>::SMEM_BYTES)
-                        : go(attention_f16_tc_kernel<128, false, 2>, AttCfg<128>::THREADS, AttCfg<128>::SMEM_BYTES);
-        return bptr ? go(attention_f16_tc_kernel<64, true, 2>, AttCfg<64, true>::THREADS, AttCfg<64, true>::SMEM_BYTES)
-                    : go(attention_f16_tc_kernel<64, false, 2>, AttCfg<64>::THREADS, AttCfg<64>::SMEM_BYTES);
+        if (single) return go(attention_f16_tc_kernel<64, false, 1, false>, AttCfg<64, false, 1>::THREADS, AttCfg<64, false, 1>::SMEM_BYTES);
+        auto either = [&](auto ep, auto bias) {
+            using Cfg = AttCfg<decltype(ep)::value, decltype(bias)::value>;
+            return cluster > 1 ? go(attention_f16_tc_kernel<decltype(ep)::value, decltype(bias)::value, 2, true>, Cfg::THREADS, Cfg::SMEM_BYTES)
+                               : go(attention_f16_tc_kernel<decltype(ep)::value, decltype(bias)::value, 2, false>, Cfg::THREADS, Cfg::SMEM_BYTES);
+        };
+        using Int64 = std::integral_constant<int, 64>;
+        using Int80 = std::integral_constant<int, 80>;
+        using Int128 = std::integral_constant<int, 128>;
+        if (bptr) return wide ? either(Int128(), std::true_type()) : either(Int64(), std::true_type());
+        return !wide ? either(Int64(), std::false_type()) : E <= 80 ? either(Int80(), std::false_type()) : either(Int128(), std::false_type());
     };
     p.qpairs = (int)cdiv(Lq, item_rows);
     const int64_t pairs = (int64_t)p.qpairs * H * B;      // work items: pairs of query tiles, or single tiles of short keys
     B200_REQUIRE(pairs < (1ll << 30), B200_DECLINE_EXTENT, "attention: too many query tiles");
-    // Two cases cut pairs along the keys (at least two key blocks per piece) and merge afterwards:
-    // fewer pairs than half the SMs (a few hundred queries over many keys: every pair is cut so that
-    // the SMs are all used), and a last wave that would leave most SMs idle (its pairs are cut so that
-    // the wave is as short as the cut allows instead of a whole pair long).  Masked calls, uncut and
-    // cut: 4 heads x 300 x 2000 52.6 -> 17.3 us, 2 x 512 x 4096 98 -> 21, 24 x 1800 x 1800 101 -> 81.
+    // Pairs that do not fill the SMs are cut along the keys (att_split): over a cluster's CTAs, which join their rows in the same
+    // launch, or over more of them with a merge behind.  A last wave that would leave most SMs idle has its pairs cut
+    // (at least two key blocks per piece) so that the wave is as short as that allows instead of a whole pair long.
     p.nsplit = 1;
     p.ntail = 0;
     p.part_o = p.part_ml = nullptr;
+    int join = 1;   // CTAs of a cluster an item's keys are cut over
     const int64_t rem = pairs % sms;
     const size_t ws_mark = ctx->ws_used;
     const bool frugal = bptr != nullptr || Lq <= (E <= 64 ? 32 : 16);
-    if (!single && nblk_all >= 4) {
+    if (!single) {
         int64_t ntail = 0, ns = 1;
         if (2 * pairs <= sms) {
-            ntail = pairs;
-            ns = sms / pairs;
-        } else if (pairs > sms && rem > 0 && 2 * rem <= sms) {
+            const AttSplit cut = att_split(ctx, pairs, nblk_all, Lq, E, bptr != nullptr);
+            if (cut.join) {
+                join = cut.parts;
+            } else {
+                ntail = pairs;
+                ns = cut.parts;
+            }
+        } else if (nblk_all >= 4 && pairs > sms && rem > 0 && 2 * rem <= sms) {
             ntail = rem;
             ns = sms / rem;
+            if (ns > nblk_all / 2) ns = nblk_all / 2;
+            if (ns > 64) ns = 64;
         }
-        if (ns > nblk_all / 2) ns = nblk_all / 2;
-        if (ns > 64) ns = 64;
         if (ntail > 0 && ns >= 2) {
             const int64_t rows = ntail * item_rows;
             void* ws = nullptr;
@@ -1286,9 +1459,18 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
         }
     }
     if (bptr) {
-        const int64_t waves = p.nsplit > 1 ? (pairs - p.ntail) / sms : cdiv(pairs, sms);
-        const int64_t serial = waves * nblk_all + (p.nsplit > 1 ? cdiv(nblk_all, p.nsplit) : 0);
+        const int64_t waves = join > 1 ? 0 : p.nsplit > 1 ? (pairs - p.ntail) / sms : cdiv(pairs, sms);
+        const int64_t serial = waves * nblk_all + (join > 1 ? cdiv(nblk_all, join) : p.nsplit > 1 ? cdiv(nblk_all, p.nsplit) : 0);
         if ((rc = mask_map(ctx, bptr, bs, E, Lq, Lk, H, B, serial, &p, &tm))) return rc;
+    }
+    if (join > 1) {
+        p.pair_ctas = 0;
+        p.nsplit = join;
+        p.ntail = (int)pairs;
+        B200_CUDA(launch(dim3((unsigned)(pairs * join), 1, 1), join));
+        ctx->launches++;
+        if (frugal) ctx->ws_used = ws_mark;
+        return B200_OK;
     }
     if (p.nsplit > 1) {
         p.pair_ctas = (int)(pairs - p.ntail);

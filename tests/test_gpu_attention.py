@@ -620,3 +620,41 @@ def test_however_a_mask_lies_the_result_is_the_same(ctx, ora, B, H, Lq, Lk, E, p
         assert np.all(got[:, :, 0] == 0)
     for pitch, offset, apart in ((aligned, 5, False), (aligned + 1, 0, False), (aligned + 4, 4, False), (Lq + 3, 1, True)):
         assert np.array_equal(run(pitch, offset, apart), got), (pitch, offset, apart)
+
+
+# items of two tiles, few enough to be cut over a cluster's CTAs: 2 to 8 of them, parts of uneven length, shares of rows that do
+# not divide 256, a second tile of one row, every width of head
+JOINED = [(1, 1, 257, 385, 64), (1, 2, 300, 900, 56), (2, 3, 500, 1700, 64), (1, 1, 256, 1100, 72), (1, 5, 700, 700, 80),
+          (1, 2, 1000, 1300, 128), (1, 18, 1020, 1020, 64), (3, 1, 129, 900, 104), (1, 9, 2040, 2040, 32)]
+
+
+@pytest.mark.parametrize("B,H,Lq,Lk,E", JOINED)
+@pytest.mark.parametrize("masked", [False, True])
+def test_keys_cut_over_a_cluster(ctx, ora, B, H, Lq, Lk, E, masked):
+    rng = np.random.default_rng(B + H + Lq + Lk + E)
+    q, k, v = (np.float16(rng.standard_normal((B, H, n, E))) for n in (Lq, Lk, Lk))
+    k[:, :, Lk // 3:Lk // 3 + 3] *= 4                                     # the reference points of the parts differ
+    bias = None
+    if masked:
+        bias = np.float16(rng.standard_normal((B, 1, Lq, Lk)))
+        bias[rng.random(bias.shape) < 0.2] = -np.inf
+        bias[:, :, 0, : Lk // 2] = -np.inf                                # parts that see nothing of a row
+        bias[:, :, Lq - 1] = -np.inf
+    ref = ora.attention_ref(q, k, v, 1 / np.sqrt(E), bias=bias)
+    buf = ctx.allocate(np.float16, H * E, Lq * B)                         # the result token-major as well
+    for out in (ctx.allocate(np.float32, E, Lq, H, B),
+                jv.DeviceArray(ctx, buf.ptr, np.float16, (E, Lq, H, B), (1, H * E, E, H * E * Lq), owner=buf)):
+        dq, dk, dv = qkv_views(ctx, q, k, v)
+        db = None if bias is None else ctx.toback(bias)
+        ctx.fill_bytes(buf if out.ptr == buf.ptr else out, 0xFF)
+        ctx.ws.reset()
+        n0 = ctx.launch_count()
+        jv.sdpa(ctx, dq, dk, dv, db, 1 / np.sqrt(E), out=out)
+        assert ctx.launch_count() - n0 <= (2 if masked else 1) and (masked or ctx.ws.stats()[0] == 0)
+        ctx.synchronize()
+        got = out.to_host() if out.ptr != buf.ptr else buf.to_host().reshape(B, Lq, H, E).transpose(0, 2, 1, 3)
+        assert np.all(np.isfinite(got))
+        # P is rounded to fp16 (2^-11 per key, averaged over them) and, for fp16, the result once more
+        assert relerr(got, ref) < 2e-3, describe(got, ref, 2e-3)
+        if masked:
+            assert np.all(got[:, :, Lq - 1] == 0)
