@@ -16,8 +16,8 @@ from importlib.machinery import EXTENSION_SUFFIXES
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 SO = os.path.join(CSRC, "libb200dnn.so")
-SOURCES = ["ctx.cu", "layernorm.cu", "gemm.cu", "attention.cu", "glue.cu", "conv.cu", "conv_implicit.cu", "gemv.cu", "gemm_rows.cu", "attention_window.cu", "attention_few.cu", "selftest.cu"]
-HEADERS = ["internal.h", "ptx.cuh", "act.cuh", os.path.join("..", "..", "include", "b200dnn.h")]
+SOURCES = ["ctx.cu", "layernorm.cu", "gemm.cu", "attention.cu", "glue.cu", "conv.cu", "conv_implicit.cu", "gemv.cu", "gemm_rows.cu", "gemm_rows_tc.cu", "attention_window.cu", "attention_few.cu", "selftest.cu"]
+HEADERS = ["internal.h", "ptx.cuh", "act.cuh", "gemm_rows.cuh", os.path.join("..", "..", "include", "b200dnn.h")]
 HOST_SRC = os.path.join(CSRC, "hostcalls.c")   # the entry points' host side, a CPython extension
 HOST_SO = os.path.join(CSRC, "hostcalls" + EXTENSION_SUFFIXES[0])   # for this interpreter: another builds its own
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")

@@ -4,23 +4,26 @@
 // misalignment) times a handful of tokens, where reading A once is all that should be paid.
 //
 // What bounds it: reading A, then the loads' latency (the accumulators leave room for fewer blocks per SM).  Measured
-// against the one-thread-per-output kernel that ran these before (whole calls, B200): 5 x 51865 x 1280 240 -> 34.8 us
-// (3.8 TB/s of A; the copy rate's floor is 20), 12 x 31751 x 928 172 -> 18.5, 17 x 1337 x 712 61 -> 8.6.
+// against the one-thread-per-output kernel that ran these before (whole calls, B200): 17 x 1337 x 712 61 -> 8.6 us; 5 x 35519 x 1280
+// takes 20.7 (4.4 TB/s of A).
 //
 // Columns k and k + 8 of A are 8 * lda * 2 bytes apart, a multiple of 16, so all columns k = w (mod 8) sit at the same
 // offset s_w from a 16-byte boundary.  Warp w of a CTA takes exactly those columns and keeps its accumulators aligned
 // to memory rather than to rows, as gemv_kernel does: the 16-byte vector at position j of a column holds rows
 // 8 j - s_w ... 8 j - s_w + 7, and only the sum over the eight warps, through shared memory, shifts by s_w.  The order
 // of a reduction axis and the names of a tile's rows are free, so the vectors become tensor-core fragments (m16n8k16,
-// warp-level: an unaligned operand can reach neither TMA nor a swizzled tile) with two byte permutes per register and
+// warp-level) with two byte permutes per register and
 // no trip through shared memory: lane (g, t) holds four columns' vectors of rows 8 g ... 8 g + 7, and word p of them
 // gives rows 2 p and 2 p + 1 of the group as the fragment's rows g and g + 8.
+//
+// Where A is long the product goes to gemm_rows_tc.cu, which finds tiles for tcgen05 in the same classes of columns.
 //
 // When row blocks alone do not fill the GPU the K axis is split over the CTAs of a cluster and the partial sums meet
 // through distributed shared memory, added in rank order: no workspace, and the result does not depend on timing.
 #include <cuda_fp16.h>
 
 #include "act.cuh"
+#include "gemm_rows.cuh"
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -41,17 +44,6 @@ template <int NT> struct GrCfg {
     static constexpr int SUM_BYTES = NT * 8 * ROWS * 4;               // this CTA's sums, for the cluster
     static constexpr int SMEM_BYTES = (X_BYTES > RED_BYTES ? X_BYTES : RED_BYTES) + SUM_BYTES;
     static constexpr int MIN_BLOCKS = NT <= 4 ? 2 : 1;
-};
-
-struct GrParams {
-    const __half *A, *B, *bias;
-    void* out;
-    int64_t lda, ldb, ldo;
-    int64_t M, N, K;
-    int bias_per_n, epi, b_vec;
-    int64_t block0;      // TWO: the launch's first row block
-    int tail;            // TWO: the second launch of the product: nothing it reads waits for the first
-    int steps_per_cta;   // steps of GR_STEP columns each CTA of a cluster takes
 };
 
 // Out of line, and not called for nothing, in the two-tile form: inlined, its registers change the main loop's (115 for 96), 9 x
@@ -240,8 +232,7 @@ static int gr_launch(b200_ctx* ctx, GrParams p) {
     while (parts < 8 && 2 * parts * blocks * tblocks <= room && steps >= 4 * parts) parts *= 2;
     // Row blocks past the last full round of the resident ones, less than half a round of them, are a launch of their own,
     // split along K like few row blocks are: 433 blocks of 296 take a round and a half instead of two.  (A second launch may
-    // start as the first one's blocks leave: see the kernel.)  5 x 51865 x 1280 37.4 -> 34.8 us, 17 x 20001 x 1024 31.5 -> 26.7,
-    // 64 x 51865 x 1280 143 -> 141.
+    // start as the first one's blocks leave: see the kernel.)  17 x 20001 x 1024 31.5 -> 26.7 us.
     int64_t tail = 0, tail_parts = 1;
     if (parts == 1 && tblocks == 1 && blocks > room) {
         tail = blocks % room;
@@ -295,6 +286,7 @@ int gemm_rows_launch(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void*
     p.b_vec = ldb % 8 == 0 && (reinterpret_cast<uintptr_t>(B) & 15u) == 0;
     p.steps_per_cta = 0;
     const bool h = out_dtype == B200_F16;
+    if (const int nt = gemm_rows_tc_tokens(ctx, M, N, K)) return gemm_rows_tc_launch(ctx, p, nt, h);
     if (N <= 8) return h ? gr_launch<1, __half>(ctx, p) : gr_launch<1, float>(ctx, p);
     if (N <= 16) return h ? gr_launch<2, __half>(ctx, p) : gr_launch<2, float>(ctx, p);
     if (N <= 32) return h ? gr_launch<4, __half>(ctx, p) : gr_launch<4, float>(ctx, p);

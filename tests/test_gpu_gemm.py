@@ -541,6 +541,32 @@ def test_unaligned_rows_past_the_last_full_round(ctx, ora, tokens, out, K, launc
     assert relerr(got, ref) < tol, describe(got, ref, tol)
 
 
+# (tokens, out features, K, elements between columns, elements off the boundary): a token block of 16, 32, 48 and 64, and more than
+# one; the last class without its last column, a reduction that ends inside sixteen of a class, and B off 16 bytes; one row block a
+# CTA and several, the last one cut; rows 0 ... 7 elements off in turn, or all the same; few columns to a class, and many
+@pytest.mark.parametrize("tokens,out,K,lda,off", [(5, 50001, 801, 50003, 1), (8, 36000, 1112, 36000, 1), (9, 28673, 736, 28675, 7),
+                                                  (16, 85001, 257, 85004, 2), (17, 21001, 1024, 21001, 0), (32, 328001, 65, 328002, 5),
+                                                  (33, 8291, 1103, 8297, 3), (48, 9001, 1280, 9001, 1), (49, 140001, 66, 140003, 6),
+                                                  (64, 9001, 1280, 9003, 0), (50, 11003, 2000, 11005, 4), (70, 9005, 1000, 9006, 3)])
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+def test_unaligned_rows_of_long_products(ctx, ora, tokens, out, K, lda, off, dt):
+    """Weights that long go to the form in tensor memory: with a bias, every row, and what lies between the columns and around
+    them (NaN here) stays out of the results."""
+    rng = np.random.default_rng(out)
+    X, Wt, b = _case(rng, tokens, out, K, scale=0.25)
+    room = np.full(off + K * lda + 8, np.nan, np.float16)
+    np.lib.stride_tricks.as_strided(room[off:], (K, out), (2 * lda, 2))[...] = Wt
+    base, x, bias = ctx.toback(room), ctx.toback(X), ctx.toback(b)
+    w = jv.DeviceArray(ctx, base.ptr + 2 * off, np.float16, (out, K), (1, lda), owner=base)
+    y = ctx.allocate(dt, out, tokens)
+    ctx.fill_bytes(y, 0xFF)
+    jv.matmul_(ctx, y, w, x, bias)
+    ctx.synchronize()
+    got, ref = y.to_host(), ora.linear(X, Wt, b, out_dtype=dt)
+    tol = 2e-3 if dt == np.float16 else 2e-5             # one rounding step of fp16; sqrt(K) eps32
+    assert relerr(got, ref) < tol, describe(got, ref, tol)
+
+
 def test_what_follows_a_product_in_two_launches_waits_for_both(ctx):
     """A layer norm that is launched early behind the second launch, eagerly and recorded, gives the bits it gives behind a
     finished product, over results that are poisoned before each."""
