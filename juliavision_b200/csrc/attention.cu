@@ -228,7 +228,8 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
     // CTAs [0, pair_ctas) own a whole pair.  The pairs after those are the tail: either each is cut along
     // the keys into nsplit CTAs whose partial results are merged afterwards (nsplit > 1), or each is
     // handed out as two single tiles.
-    int item = blockIdx.x, half = -1, split = 0, nsp = 1;
+    // A join's CTAs all belong to the tail; the whole pairs before it, if any, are a launch of their own.
+    int item = blockIdx.x + (JOIN ? p.pair_ctas : 0), half = -1, split = 0, nsp = 1;
     if (item >= p.pair_ctas) {
         const int t = item - p.pair_ctas;
         if (p.nsplit > 1) {
@@ -288,7 +289,9 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // Everything above overlapped the previous kernel's tail; from here on its results are needed.
-    grid_dep_wait();
+    // (A joined tail reads only what its whole pairs' launch has waited for, so it starts as that one's CTAs leave; what follows the
+    // tail on the stream waits for it to end, hence, by the wait at its end, for both.)
+    if (!JOIN || p.pair_ctas == 0) grid_dep_wait();
     grid_dep_launch();
 
     bool met = false;   // joining: this warp has passed the barrier behind which the rows are there
@@ -866,6 +869,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
         cluster_sync_all();
         cluster_sync_all();
     }
+    if (JOIN && p.pair_ctas > 0) grid_dep_wait();
     if (*abort_flag) {
         for (int i = 0; i < 4; ++i) __nanosleep(1000000);
     }
@@ -1150,8 +1154,13 @@ static const AttRooms& att_rooms(b200_ctx* ctx) {
 // A join is the cheapest cut wherever its clusters are resident at once: 1.05 to 1.65 times as fast as merging, 1.29 in the mean
 // (9 heads x 2040 x 64 28.0 -> 21.5 us, 18 x 1020 22.2 -> 15.0, 12 x 900 x 128 23.2 -> 18.9); two and three key blocks, and many
 // pairs of four, stay whole (12 heads x 400: 9.9 us, 13.0 merged).  More than eight parts are worth a merge where pairs are few.
+// The tail of `waves` full rounds of items is cut the same way.  Its clusters wait for SMs of one group that fall free one by one, up
+// to 7 % of the rounds apart: joined rather than merged, 12 heads x 4096 x 4096 x 64 80.3 -> 76.9 us, x 1200 39.3 -> 34.1, 10 heads x
+// 4096 x 4096 x 72 80.0 -> 71.9, but x 8000 138.6 -> 140.7.  Wider heads take three-CTA clusters up to one short of their room
+// (44 of 45, 12 heads x 4096 x 4096 x 72: 89.5 -> 103.5, two rounds of them).  Masked tails go on merging, their CTAs' ends lie
+// further apart (12 heads x 4096 x 4096 111.6 -> 117.3, 14 x 2900 86.1 -> 89.8; short ones would gain, 38 x 1024 x 640 31.1 -> 29.4).
 struct AttSplit { int parts; bool join; };
-static AttSplit att_split(b200_ctx* ctx, int64_t pairs, int64_t nblk, int64_t Lq, int64_t E, bool masked) {
+static AttSplit att_split(b200_ctx* ctx, int64_t pairs, int64_t nblk, int64_t Lq, int64_t E, bool masked, int64_t waves) {
     struct Cost { double block, load, join, merge, rows; };
     static const Cost costs[5] = {{1.35, 0.37, 3.65, 4.15, 0.035}, {1.44, 0.57, 4.4, 4.75, 0.038}, {1.83, 0.46, 4.7, 5.4, 0.038},
                                   {2.07, 0.56, 3.9, 5.15, 0.035}, {2.44, 0.77, 4.7, 5.6, 0.042}};
@@ -1161,9 +1170,11 @@ static AttSplit att_split(b200_ctx* ctx, int64_t pairs, int64_t nblk, int64_t Lq
     const AttRooms& rooms = att_rooms(ctx);
     AttSplit best = {1, false};
     double least = walk(1);
-    for (int n = 2; n <= JOIN_MOST && n <= nblk && Lq > ATT_BR; ++n)
-        if (pairs < rooms.clusters[n] + (n == 2) && walk(n) + c.join < least) {
-            least = walk(n) + c.join;
+    const double apart = 0.07 * ((double)(waves * nblk) * (c.block + c.load) - 20.0);
+    const double join = c.join + (apart > 0.0 ? apart : 0.0);
+    for (int n = 2; n <= JOIN_MOST && n <= nblk && Lq > ATT_BR && !(waves && masked); ++n)
+        if (pairs + (waves && E > 64) < rooms.clusters[n] + (n == 2) && walk(n) + join < least) {
+            least = walk(n) + join;
             best = {n, true};
         }
     int64_t n = sms / pairs;
@@ -1425,23 +1436,19 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     p.part_o = p.part_ml = nullptr;
     int join = 1;   // CTAs of a cluster an item's keys are cut over
     const int64_t rem = pairs % sms;
+    const bool tail = nblk_all >= 4 && pairs > sms && rem > 0 && 2 * rem <= sms;
     const size_t ws_mark = ctx->ws_used;
     const bool frugal = bptr != nullptr || Lq <= (E <= 64 ? 32 : 16);
     if (!single) {
         int64_t ntail = 0, ns = 1;
-        if (2 * pairs <= sms) {
-            const AttSplit cut = att_split(ctx, pairs, nblk_all, Lq, E, bptr != nullptr);
+        if (2 * pairs <= sms || tail) {
+            const AttSplit cut = att_split(ctx, tail ? rem : pairs, nblk_all, Lq, E, bptr != nullptr, tail ? pairs / sms : 0);
             if (cut.join) {
                 join = cut.parts;
             } else {
-                ntail = pairs;
+                ntail = tail ? rem : pairs;
                 ns = cut.parts;
             }
-        } else if (nblk_all >= 4 && pairs > sms && rem > 0 && 2 * rem <= sms) {
-            ntail = rem;
-            ns = sms / rem;
-            if (ns > nblk_all / 2) ns = nblk_all / 2;
-            if (ns > 64) ns = 64;
         }
         if (ntail > 0 && ns >= 2) {
             const int64_t rows = ntail * item_rows;
@@ -1459,15 +1466,19 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
         }
     }
     if (bptr) {
-        const int64_t waves = join > 1 ? 0 : p.nsplit > 1 ? (pairs - p.ntail) / sms : cdiv(pairs, sms);
+        const int64_t waves = join > 1 ? (tail ? pairs / sms : 0) : p.nsplit > 1 ? (pairs - p.ntail) / sms : cdiv(pairs, sms);
         const int64_t serial = waves * nblk_all + (join > 1 ? cdiv(nblk_all, join) : p.nsplit > 1 ? cdiv(nblk_all, p.nsplit) : 0);
         if ((rc = mask_map(ctx, bptr, bs, E, Lq, Lk, H, B, serial, &p, &tm))) return rc;
     }
     if (join > 1) {
-        p.pair_ctas = 0;
+        p.ntail = (int)(tail ? rem : pairs);
+        p.pair_ctas = (int)(pairs - p.ntail);
+        if (tail) {
+            B200_CUDA(launch(dim3((unsigned)p.pair_ctas, 1, 1)));
+            ctx->launches++;
+        }
         p.nsplit = join;
-        p.ntail = (int)pairs;
-        B200_CUDA(launch(dim3((unsigned)(pairs * join), 1, 1), join));
+        B200_CUDA(launch(dim3((unsigned)(p.ntail * join), 1, 1), join));
         ctx->launches++;
         if (frugal) ctx->ws_used = ws_mark;
         return B200_OK;

@@ -658,3 +658,46 @@ def test_keys_cut_over_a_cluster(ctx, ora, B, H, Lq, Lk, E, masked):
         assert relerr(got, ref) < 2e-3, describe(got, ref, 2e-3)
         if masked:
             assert np.all(got[:, :, Lq - 1] == 0)
+
+
+# one full round of items and a few (148 SMs), two rounds and 40, most that three CTAs an item leave room for, and every width
+@pytest.mark.parametrize("B,H,Lq,Lk,E", [(1, 19, 2040, 900, 64), (3, 14, 1999, 700, 32), (1, 12, 4096, 520, 64), (2, 19, 1100, 1200, 72),
+                                         (1, 38, 1024, 1100, 128)])
+def test_a_last_round_cut_over_clusters(ctx, ora, B, H, Lq, Lk, E):
+    """The items past the last full round are a second launch, whose clusters join their rows: no scratch, every row; and a layer
+    norm that is launched early behind it, eagerly and recorded, finds both launches' rows over a poisoned result."""
+    rng = np.random.default_rng(H + Lk)
+    q, k, v = (np.float16(rng.standard_normal((B, H, n, E))) for n in (Lq, Lk, Lk))
+    dq, dk, dv = qkv_views(ctx, q, k, v)
+    out, z = ctx.allocate(np.float16, E, Lq, H, B), ctx.allocate(np.float16, E, Lq * H * B)
+    mean, rstd = ctx.allocate(np.float32, Lq * H * B), ctx.allocate(np.float32, Lq * H * B)
+    flat = jv.DeviceArray(ctx, out.ptr, np.float16, (E, Lq * H * B), owner=out)
+
+    def norm():
+        jv.layernorm_(ctx, z, mean, rstd, flat, None, None, E, 1e-5)
+
+    def both():
+        ctx.fill_bytes(out, 0xFF)
+        jv.sdpa(ctx, dq, dk, dv, None, 1 / np.sqrt(E), out=out)
+        norm()
+
+    ctx.ws.reset()
+    ctx.fill_bytes(out, 0xFF)
+    n0 = ctx.launch_count()
+    jv.sdpa(ctx, dq, dk, dv, None, 1 / np.sqrt(E), out=out)
+    if ctx.dev.cores == 148:
+        assert ctx.launch_count() - n0 == 2 and ctx.ws.stats()[0] == 0
+    ctx.synchronize()
+    norm()
+    ctx.synchronize()
+    got, want = out.to_host(), z.to_host()
+    ref = ora.attention_ref(q, k, v, 1 / np.sqrt(E))
+    # P is rounded to fp16 (2^-11 per key, averaged over them) and the result once more
+    assert relerr(got, ref) < 2e-3, describe(got, ref, 2e-3)
+    g = ctx.capture(both)
+    for run in (both, g.replay) * 3:
+        ctx.fill_bytes(z, 0xFF)
+        run()
+        ctx.synchronize()
+        assert np.array_equal(z.to_host(), want) and np.array_equal(out.to_host(), got)
+    del g
