@@ -59,7 +59,6 @@ template <int BN, typename OutT, int NCTA, int GC = 16> struct GemmCfg {
     static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + TAIL_BYTES;
     static constexpr int TMEM_COLS = WIDE ? 512 : (2 * BN < 32 ? 32 : 2 * BN);
-    static_assert(NCTA == 2 || STAGES * STAGE_BYTES >= GEMM_BM * BN * 4, "a tile's fp32 accumulator fits over the ring");
     static_assert(STAGES >= 2, "ring too shallow");
     static_assert(SMEM_BYTES <= SMEM_LIMIT, "shared memory over budget");
     static_assert(TMEM_COLS == 128 || TMEM_COLS == 256 || TMEM_COLS == 512, "TMEM columns");
@@ -79,7 +78,7 @@ template <typename OutT> struct GemmParams {
     const __half* bias;
     int bias_per_n;        // 0: bias[i] over features (M); 1: bias[j] over tokens (N)
     int epilogue;
-    int ksplit;            // KSPLIT: CTAs (a cluster) per tile
+    int ksplit;            // KSPLIT: CTAs or pairs (a cluster) per tile
     int streamk;           // 0: whole tiles, strided over the workers; 1 + lean: contiguous k-block ranges per worker (see SegIter)
     float* sk_part;        // stream-K: fp32 partial accumulators, one 128 x BN block per (worker, CTA rank)
     int* sk_flag;          // stream-K: one flag per (worker, CTA rank, epilogue warp), zero between launches
@@ -206,7 +205,7 @@ __device__ __forceinline__ void st_release_gpu(int* p, int v) {
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// KSPLIT: a cluster of p.ksplit CTAs (NCTA = 1) takes one tile, each a contiguous part of its k-blocks.  The fp32
+// KSPLIT: a cluster of p.ksplit CTAs (NCTA = 1) or CTA pairs (NCTA = 2) takes one tile, each a contiguous part of its k-blocks.  The fp32
 // accumulators are laid over the drained operand ring and every CTA finishes its share of the tile's chunks from all
 // of them, read through distributed shared memory and added in rank order: no workspace, no flags, and a hand-off of
 // a cluster barrier where the stream-K one through L2 costs ~6 us.
@@ -239,11 +238,14 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // warp-uniform, and known to be
     const int lane = threadIdx.x & 31;
-    static_assert(!KSPLIT || NCTA == 1, "a K split is over single CTAs");
-    const uint32_t rank = NCTA == 2 ? cluster_ctarank() : 0u;  // 0 = the CTA that issues the UMMAs
-    const uint32_t kpart = KSPLIT ? cluster_ctarank() : 0u;    // which part of the tile's k-blocks
-    const uint32_t worker = NCTA == 2 ? (blockIdx.x >> 1) : (KSPLIT ? blockIdx.x / (uint32_t)p.ksplit : blockIdx.x);
-    const uint32_t nworkers = NCTA == 2 ? (gridDim.x >> 1) : (KSPLIT ? gridDim.x / (uint32_t)p.ksplit : gridDim.x);
+    static_assert(!KSPLIT || Cfg::STAGES * Cfg::STAGE_BYTES >= GEMM_BM * BN * 4, "the accumulator fits over the ring");
+    const uint32_t crank = NCTA == 2 || KSPLIT ? cluster_ctarank() : 0u;
+    const uint32_t rank = NCTA == 2 ? (KSPLIT ? crank & 1u : crank) : 0u;  // 0 = the CTA that issues the UMMAs
+    const uint32_t lead = NCTA == 2 && KSPLIT ? crank & ~1u : 0u;          // its rank in the cluster
+    const uint32_t kpart = KSPLIT ? crank / NCTA : 0u;                     // which part of the tile's k-blocks
+    const uint32_t per = KSPLIT ? NCTA * (uint32_t)p.ksplit : NCTA;        // CTAs a worker is
+    const uint32_t worker = KSPLIT || NCTA == 2 ? blockIdx.x / per : blockIdx.x;
+    const uint32_t nworkers = KSPLIT || NCTA == 2 ? gridDim.x / per : gridDim.x;
 
     if (threadIdx.x == 0) {
         GEMM_TRACE(0); // kernel entry
@@ -320,7 +322,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
                     if constexpr (NCTA == 2) {
                         // Both CTAs' bytes are counted on the leader's barrier; the leader posts
                         // the expectation for the pair.
-                        const uint32_t bar = mapa_u32(smem_u32(&full[s]), 0);
+                        const uint32_t bar = mapa_u32(smem_u32(&full[s]), lead);
                         if constexpr (Cfg::WIDE) {
                             if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * (Cfg::A_BYTES + (2 + slabs2) * Cfg::B_CHUNK_BYTES));
                             tma_load_3d_pair(sa, &tmapX, bar, kb * GEMM_BK, n0, batch);
@@ -405,14 +407,14 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
                                         idesc, accum);
                             }
                         }
-                        if constexpr (NCTA == 2) umma_commit_pair(&empty[s], 3); // frees the stage in both CTAs
+                        if constexpr (NCTA == 2) umma_commit_pair(&empty[s], (uint16_t)(3u << lead)); // frees the stage in both CTAs
                         else umma_commit(&empty[s]);
                     }
                     __syncwarp();
                     if (++s == Cfg::STAGES) { s = 0; ph ^= 1; }
                 }
                 if (ok && elect_one()) {
-                    if constexpr (NCTA == 2) umma_commit_pair(&tfull[acc], 3);
+                    if constexpr (NCTA == 2) umma_commit_pair(&tfull[acc], (uint16_t)(3u << lead));
                     else umma_commit(&tfull[acc]);
                     GEMM_TRACE(4 + (it < 4 ? it : 3)); // all UMMAs of tile `it` issued
                 }
@@ -558,7 +560,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
                     for (int t = 0; t < CH; ++t) v[t] = 0.f;
 #pragma unroll 4
                     for (uint32_t k = 0; k < (uint32_t)p.ksplit; ++k) {
-                        const uint32_t src = mapa_u32(dump + (uint32_t)(col0 / 4) * (GEMM_BM * 16), k);
+                        const uint32_t src = mapa_u32(dump + (uint32_t)(col0 / 4) * (GEMM_BM * 16), NCTA * k + rank);
 #pragma unroll
                         for (int q = 0; q < CH / 4; ++q) {
                             const float4 f = ld_cluster_f32x4(src + q * (GEMM_BM * 16));
@@ -581,7 +583,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapX,   // B(K,N): {K, t
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) {
-                        if constexpr (NCTA == 2) mbar_arrive_cluster_cta_release(mapa_u32(smem_u32(&tempty[acc]), 0));
+                        if constexpr (NCTA == 2) mbar_arrive_cluster_cta_release(mapa_u32(smem_u32(&tempty[acc]), lead));
                         else mbar_arrive(&tempty[acc]);
                     }
                 }
@@ -753,7 +755,7 @@ struct TilePick {
     int ncta;    // 1: 128-token tiles, one CTA each; 2: 256-token tiles, one CTA pair each
     int streamk; // 1: equal k-block ranges per worker instead of whole tiles
     int width;   // bn == 512 (the wide tile): feature columns per tile, a multiple of 16 in (256, 512]
-    int ksplit;  // > 1: CTAs of a cluster that share a tile's k-blocks (ncta == 1)
+    int ksplit;  // > 1: CTAs or pairs of a cluster that share a tile's k-blocks
 };
 
 // Tile planner.  Candidates are (BN, NCTA, whole-tile | stream-K); the estimate for each is
@@ -776,6 +778,9 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
         int bn = 0, nc = 0, ks = 1;
         char sk = 0;
         const int got = sscanf(f, "%dx%d%c%d", &bn, &nc, &sk, &ks);
+        if (got == 4 && sk == 'k' && nc == 2 && bn == 256 && (ks == 2 || ks == 4) && ks <= cdiv(K, GEMM_BK) &&
+            cdiv(M, 256) * cdiv(N, (int64_t)GEMM_BM * 2) * nbatch <= room.clusters[ks / 2 + 1])
+            return {256, 2, 0, 0, ks};
         if (got == 4 && sk == 'k' && nc == 1 && (bn == 128 || bn == 64) && ks >= 2 && ks <= 8 && ks <= cdiv(K, GEMM_BK) &&
             cdiv(M, bn) * cdiv(N, (int64_t)GEMM_BM) * nbatch * ks <= sms)
             return {bn, 1, 0, 0, ks};
@@ -863,6 +868,19 @@ static TilePick pick_tile(int64_t M, int64_t N, int64_t K, int64_t nbatch, int s
                 best_cost = cost;
                 best = {bn, 1, 0, 0, 1 << l};
             }
+        }
+    }
+    // The same over two or four pairs, for tiles that leave half of the SMs or more idle as pairs and that the clusters above cannot
+    // hold or hold in two parts only.  Against the estimates of what it replaces, whole 128-wide pair tiles of long reductions (which
+    // come out ahead of the truth: 26.3 for 20.3 us at 64 k-blocks) and two parts, t_join is 7.3 and 6: 1500 x 1280 x 5120 21.9 -> 20.9
+    // us, x 4096 20.4 -> 18.5, 512 x 4096 x 4096 20.3 -> 18.9, 500 x 1280 x 5120 17.3 -> 15.2, 995 x 664 x 4720 18.1 -> 15.5; whole it
+    // stays at 768 x 2560 x 2560 (14.5, 15.3), in two parts at 1148 x 704 x 2760 (12.5, 13.5); with GELU, whose arithmetic the join leaves in the open, 7699 x 160 x 3120 (17.3, 17.6).
+    for (int l = 1; l <= 2 && nkb >= 24; ++l) {
+        if (cdiv(M, 256) * cdiv(N, (int64_t)GEMM_BM * 2) * nbatch > room.clusters[l + 1]) break;
+        const double cost = (double)cdiv(nkb, (int64_t)1 << l) * cands[0].t_kb + t_tile + (l == 1 ? 7.3 : 6.0) + (gelu ? 0.6 : 0.0);
+        if (cost < 0.95 * best_cost) {
+            best_cost = cost;
+            best = {256, 2, 0, 0, 1 << l};
         }
     }
     best_cost *= 0.85;
@@ -1018,7 +1036,7 @@ static int launch_tc(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void*
     int workers = (int)((int64_t)p.total_tiles < workers_max ? (int64_t)p.total_tiles : workers_max);
     p.ksplit = 1;
     if (KSPLIT) {
-        B200_REQUIRE(ksplit >= 2 && ksplit <= 8 && ksplit <= p.num_kb && (int64_t)p.total_tiles * ksplit <= ctx->prop.multiProcessorCount,
+        B200_REQUIRE(ksplit >= 2 && ksplit <= 8 && ksplit <= p.num_kb && (int64_t)p.total_tiles * ksplit * NCTA <= ctx->prop.multiProcessorCount,
                      B200_EINVAL, "gemm: K split in %d", ksplit);
         p.ksplit = ksplit;
         workers = (int)p.total_tiles;
@@ -1085,8 +1103,8 @@ int b200_gemm_f16_plan(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, int64_t n
         plan->stages = GemmCfg<512, __half, 2>::STAGES;
         plan->smem_bytes = GemmCfg<512, __half, 2>::SMEM_BYTES;
     } else if (t.ncta == 2) {
-        plan->stages = bn == 128 ? GemmCfg<128, __half, 2, 32>::STAGES : deep_ring(K) ? GemmCfg<256, __half, 2>::STAGES : GemmCfg<256, __half, 2, 32>::STAGES;
-        plan->smem_bytes = bn == 128 ? GemmCfg<128, __half, 2, 32>::SMEM_BYTES : deep_ring(K) ? GemmCfg<256, __half, 2>::SMEM_BYTES : GemmCfg<256, __half, 2, 32>::SMEM_BYTES;
+        plan->stages = bn == 128 ? GemmCfg<128, __half, 2, 32>::STAGES : deep_ring(K) || t.ksplit > 1 ? GemmCfg<256, __half, 2>::STAGES : GemmCfg<256, __half, 2, 32>::STAGES;
+        plan->smem_bytes = bn == 128 ? GemmCfg<128, __half, 2, 32>::SMEM_BYTES : deep_ring(K) || t.ksplit > 1 ? GemmCfg<256, __half, 2>::SMEM_BYTES : GemmCfg<256, __half, 2, 32>::SMEM_BYTES;
     } else {
         plan->stages = bn == 256 ? GemmCfg<256, __half, 1>::STAGES
                                  : (bn == 128 ? GemmCfg<128, __half, 1>::STAGES : GemmCfg<64, __half, 1>::STAGES);
@@ -1162,16 +1180,20 @@ int gemm_f16_run(b200_ctx* ctx, int64_t M, int64_t N, int64_t K, const void* A, 
 #define GEMM_GO(...)                                                                                              \
     return launch_tc<__VA_ARGS__>(ctx, M, N, K, A, lda, B, ldb, bias, bias_per_n, out, ldo, epilogue, nbatch, strideA, \
                                    strideB, strideO, t.streamk, t.width, t.ksplit)
-#define GEMM_GO_SPLIT(BN_, T_)                                                                                    \
-    return launch_tc<BN_, T_, 1, true>(ctx, M, N, K, A, lda, B, ldb, bias, bias_per_n, out, ldo, epilogue, nbatch, strideA, \
+#define GEMM_GO_SPLIT(BN_, T_, NCTA_)                                                                                    \
+    return launch_tc<BN_, T_, NCTA_, true>(ctx, M, N, K, A, lda, B, ldb, bias, bias_per_n, out, ldo, epilogue, nbatch, strideA, \
                                        strideB, strideO, 0, 0, t.ksplit)
+    if (t.ksplit > 1 && t.ncta == 2) {
+        if (out_dtype == B200_F16) GEMM_GO_SPLIT(256, __half, 2);
+        GEMM_GO_SPLIT(256, float, 2);
+    }
     if (t.ksplit > 1) {
         if (out_dtype == B200_F16) {
-            if (t.bn == 128) GEMM_GO_SPLIT(128, __half);
-            GEMM_GO_SPLIT(64, __half);
+            if (t.bn == 128) GEMM_GO_SPLIT(128, __half, 1);
+            GEMM_GO_SPLIT(64, __half, 1);
         }
-        if (t.bn == 128) GEMM_GO_SPLIT(128, float);
-        GEMM_GO_SPLIT(64, float);
+        if (t.bn == 128) GEMM_GO_SPLIT(128, float, 1);
+        GEMM_GO_SPLIT(64, float, 1);
     }
     if (out_dtype == B200_F16) {
         if (t.bn == 512) GEMM_GO(512, __half, 2);

@@ -224,6 +224,12 @@ def test_tiles_shared_by_a_cluster(ctx, ora, tile, tokens, out, K, monkeypatch):
     assert relerr(two.to_host(), np.stack([zero, -2 * zero])) < 2e-5
 
 
+@pytest.mark.parametrize("tile", ["256x2k2", "256x2k4"])
+@pytest.mark.parametrize("tokens,out,K", [(2, 8, 512), (129, 264, 530), (300, 200, 1288), (517, 1000, 4264), (1500, 1280, 5120)])
+def test_tiles_shared_by_the_pairs_of_a_cluster(ctx, ora, tile, tokens, out, K, monkeypatch):
+    test_tiles_shared_by_a_cluster(ctx, ora, tile, tokens, out, K, monkeypatch)
+
+
 def test_plans_made_by_several_threads_agree(ctx):
     """The plan entry asks the runtime once per device and keeps the answer for every thread."""
     import ctypes as C
