@@ -138,7 +138,8 @@ static int conv2d_group(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_
     const void* wB = w;
     int64_t ldw = CRS;
     // The implicit kernel where the GEMM cannot store the result, and where it has two pixel tiles per SM or more; a small
-    // image the GEMM can store is as fast through a small im2col matrix (64 x 58 x 24 -> 64: 7.5 us, implicit 12).
+    // image the GEMM can store is as fast through a small im2col matrix (64 x 58 x 24 -> 64: 7.5 us, by taps 12), but where it is
+    // read in runs and gains (conv_runs_gain).
     const bool aligned = P % 8 == 0 && out_img * osz % 16 == 0 && al16(out);   // the GEMM can store the result
     const bool gemm_1x1 = onebyone && aligned && x_img % 8 == 0 && al16(x);
     if (onebyone && !gemm_1x1 && scalar_1x1_is_faster(ctx, P, Cin, Cout, N)) {
@@ -149,7 +150,8 @@ static int conv2d_group(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_
         return B200_OK;
     }
     bool implicit = conv_implicit_takes(W, H, Cin, N, KW, KH, Cout, P) &&
-                    (onebyone ? !gemm_1x1 : !aligned || cdiv(P, 128) * N >= 2 * ctx->prop.multiProcessorCount);
+                    (onebyone ? !gemm_1x1 : !aligned || cdiv(P, 128) * N >= 2 * ctx->prop.multiProcessorCount ||
+                                             (conv_runs(W, KW, KH, sx, sy, OW) && conv_runs_gain(ctx, Cin, N, KW, KH, Cout, P)));
     const size_t ws_mark = ctx->ws_used;
     // An even stride over rows of whole words: the implicit kernel reads the image in words where that gains.  Its
     // weight takes a workspace; refused (a graph recorded without an eager call before), the call goes on as it did.

@@ -17,7 +17,7 @@
 //              Afterwards the epilogue, TMEM -> +bias, round, act -> global
 //   warp 8     TMA producer of the weight tile (K-major, straight from w)
 //   warp 9     UMMA issuer
-// In words, launches of more CTAs than that take four smaller ones per SM (CiCfg).
+// In words and in runs, launches of more CTAs than that take four smaller ones per SM (CiCfg).
 // Measured (us, B200) against the im2col + GEMM route: 1024 x 1024 x 3 -> 112, 7 x 7 / 4: 35 -> 23.6; 300 x 296 x 16 -> 64,
 // 3 x 3: 42.5 -> 24.6; against the scalar GEMM odd pixel counts had: 43 x 42 x 256 -> 256, 3 x 3 / 2: 229 -> 14.2, two of
 // 230 x 225 x 32 -> 80, 3 x 3: 890 -> 43.  What is left is the gather's load latency.
@@ -28,6 +28,13 @@
 // columns than taps (7 x 7 / 4, 3 x 3 / 2) and a tenth of the instructions: us, before and
 // now: 1024 x 1024 x 3 -> 112, 7 x 7 / 4 24.8 -> 17.0, eight of them 166 -> 93, 512 x 512 x 3 -> 64 18.4 -> 6.4, 3 x 3 / 2
 // 256 x 256 x 32 -> 128 19.4 -> 9.2, 128 x 128 x 128 -> 256 22.5 -> 18.1.  What is left is a CTA's chain of latencies.
+// A convolution of stride one whose rows of results are as long as the image's (3 x 3 padded by 1) is read in runs: the taps of eight
+// neighbouring pixels are eight elements in a row in memory, over the ends of image rows as well, so a thread reads the two aligned
+// vectors they lie in, shifts them into place, blanks what is outside the image by bits it has worked out once, and stores a whole
+// 16-byte piece of the tile; the reduction's order and bits are the taps'.  500 x 495 x 16 -> 40: 837 warp instructions a k-block and
+// warp by taps; us, by taps and in runs: 64.6, 42.1, 1000 x 991 x 16 -> 32 267, 165, two of 106 x 97 x 136 -> 80 47.7, 35.4, two of 185 x
+// 181 x 16 -> 56 19.4, 12.8, 300 x 296 x 16 -> 64 24.1, 17.5 (with the four smaller CTAs an SM; 57.3, -, 40.2, 18.9, 22.5 with two and
+// dearer masks).
 // A small image (fewer CTAs than the GPU holds) splits the reduction over the CTAs of a cluster, whose fp32 tiles
 // meet in distributed shared memory, added in rank order.
 #include <cuda_fp16.h>
@@ -121,15 +128,24 @@ __device__ __forceinline__ void ldg_words_if(uint32_t (&v)[1], const uint16_t* p
         : "l"(p), "r"((uint32_t)in));
 }
 
+// Bits 0 ... 7 of m as halves of ones or zeros.  (Bit i of four goes to the top of byte i, whose sign prmt repeats.)
+__device__ __forceinline__ void halves_of_bits(uint32_t (&w)[4], uint32_t m) {
+    const uint32_t lo = ((m & 15u) * 0x10204080u) & 0x80808080u, hi = ((m >> 4) * 0x10204080u) & 0x80808080u;
+    asm("prmt.b32 %0, %1, %1, 0x9988;" : "=r"(w[0]) : "r"(lo));
+    asm("prmt.b32 %0, %1, %1, 0xBBAA;" : "=r"(w[1]) : "r"(lo));
+    asm("prmt.b32 %0, %1, %1, 0x9988;" : "=r"(w[2]) : "r"(hi));
+    asm("prmt.b32 %0, %1, %1, 0xBBAA;" : "=r"(w[3]) : "r"(hi));
+}
+
 // grid (K parts, pixel tiles of all images, channel tiles); the K parts of a tile form a cluster.  G: columns of the
-// reduction per kernel row where the image is read in words, 0: tap by tap.
+// reduction per kernel row where the image is read in words, 0: tap by tap, -1: tap by tap in runs of eight pixels.
 template <int BN, typename OutT, int G, bool SMALL>
 __global__ void __launch_bounds__((CiCfg<BN, SMALL>::THREADS), (CiCfg<BN, SMALL>::CTAS))
 conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Cout}, boxes of 64 x BN
                      const ConvParams p) {
     using Cfg = CiCfg<BN, SMALL>;
     constexpr int CI_GATHER = Cfg::GATHER, TMA_WARP = CI_GATHER / 32, ISSUE_WARP = TMA_WARP + 1;
-    static_assert(!SMALL || G > 0, "the small CTA reads the image in words");
+    static_assert(!SMALL || G != 0, "the small CTA reads the image in words or runs");
     extern __shared__ __align__(1024) uint8_t smem[];
     if ((smem_u32(smem) & 1023u) != 0) {
         if (threadIdx.x == 0) atomicCAS(p.d_status, 0, KST_SMEM_LAYOUT);
@@ -169,7 +185,7 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
     // In words the kernel before this one lays out the weight, and lets this one start when all before it is done: the image
     // and the bias are there, and only the weight has to be waited for
     // (256 x 256 x 32 -> 128, 3 x 3 / 2, with the issuing warp below: 9.07 -> 8.18 us; 1024 x 1024 x 3 -> 112, 7 x 7 / 4: 15.83 -> 15.66).
-    if (G == 0 || warp == TMA_WARP) grid_dep_wait();
+    if (G <= 0 || warp == TMA_WARP) grid_dep_wait();
     grid_dep_launch();
 
     // Channel c of the tile at pixel pix, rounded before the activation sees it.  The activation is a template
@@ -198,8 +214,8 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
         }
     } else if (warp == ISSUE_WARP) {
         // the warp waits together and the thread elect.sync picks issues, as in the GEMM
-        constexpr uint32_t idesc = make_idesc_f16(CI_PIX, BN, /*a MN-major, in words K-major*/ G == 0, /*b K-major*/ 0);
-        constexpr uint64_t adesc0 = G == 0 ? make_smem_desc(64 * CI_BK * 2, 1024) : make_smem_desc(16, 1024);
+        constexpr uint32_t idesc = make_idesc_f16(CI_PIX, BN, /*a MN-major, in words K-major*/ G <= 0, /*b K-major*/ 0);
+        constexpr uint64_t adesc0 = G <= 0 ? make_smem_desc(64 * CI_BK * 2, 1024) : make_smem_desc(16, 1024);
         constexpr uint64_t bdesc0 = make_smem_desc(16, 1024);
         bool ok = true;
         for (int kb = 0; kb < nkb; ++kb) {
@@ -210,8 +226,10 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
             if (elect_one()) {
                 const uint32_t a = smem_u32(smem + s * Cfg::STAGE_BYTES), b = a + CI_A_BYTES;
 #pragma unroll
-                for (int k = 0; k < CI_BK / 16; ++k)   // 16 k: two 8-row groups of an MN-major A, 32 bytes inside a K-major swizzle row
-                    umma_ss(tmem_base, smem_desc_at(adesc0, a + k * (G == 0 ? 2048 : 32)), smem_desc_at(bdesc0, b + k * 32), idesc, (kb | k) != 0);
+                for (int k = 0; k < CI_BK / 16; ++k) {   // 16 k: two 8-row groups of an MN-major A, 32 bytes inside a K-major swizzle row
+                    if (G < 0 && (kb0 + kb) * CI_BK + k * 16 >= p.CRS) break;   // not gathered
+                    umma_ss(tmem_base, smem_desc_at(adesc0, a + k * (G <= 0 ? 2048 : 32)), smem_desc_at(bdesc0, b + k * 32), idesc, (kb | k) != 0);
+                }
                 umma_commit(&empty[s]);
                 if (kb + 1 == nkb) umma_commit(tfull);
             }
@@ -270,6 +288,97 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
             for (int st = 0; st < nsteps; st += 2) {   // by twos: the registers of a step are named at compile time
                 if (!step(st, 0)) break;
                 if (st + 1 < nsteps && !step(st + 1, 1)) break;
+            }
+        } else if constexpr (G < 0) {
+            // Pixels 8 (lane % 16) ... of the tile, a run of memory for every tap.  What of it lies outside the image is masked: byte
+            // kx of `xm` are the eight pixels' columns that are inside with that tap, byte ky of `ym` the rows.
+            const uint16_t* xi = reinterpret_cast<const uint16_t*>(p.x) + (int64_t)img * p.x_img;
+            const int c = lane & 15, up = lane >> 4, m = m0 + 8 * c, y0 = m / p.W, x0 = m - y0 * p.W;
+            uint32_t xm = 0, ym = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int wrap = x0 + j >= p.W, x = x0 + j - (wrap ? p.W : 0) - p.px;   // W is eight at the least
+                const int y = m + j < p.P ? y0 + wrap - p.py : -(1 << 30);
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {   // bits of taps that are not there are not looked at
+                    xm |= (uint32_t)((uint32_t)(x + t * p.dx) < (uint32_t)p.W) << (8 * t + j);
+                    ym |= (uint32_t)((uint32_t)(y + t * p.dy) < (uint32_t)p.H) << (8 * t + j);
+                }
+            }
+            const int base = m - p.py * p.W - p.px, total = p.CRS / (p.KW * p.KH) * p.H * p.W;
+            // A warp takes rows warp + WARPS r of a k-block, four at a time, a half of it each of two.
+            constexpr int WARPS = CI_GATHER / 32, STEPS = 16 / WARPS;
+            const int row = WARPS == 8 ? warp : warp + 4 * up;   // in its eight rows
+            uint8_t* const to = smem + (c >> 3) * (64 * CI_BK * 2) + (WARPS == 8 ? up * 1024 : 0) + row * 128 + (((c & 7) ^ row) << 4);
+            int koff, kxy;   // of row r by lane r: offset in the image, and 8 kx, 8 ky; past the reduction negative
+            auto taps = [&](int kb) {
+                const uint32_t k = (uint32_t)((kb0 + kb) * CI_BK + warp + WARPS * (lane & (64 / WARPS - 1)));
+                const uint32_t t = div_magic(k, p.KW, p.mKW), cin = div_magic(t, p.KH, p.mKH);
+                const int kx = (int)(k - t * p.KW), ky = (int)(t - cin * p.KH);
+                koff = ((int)cin * p.H + ky * p.dy) * p.W + kx * p.dx;
+                kxy = k < (uint32_t)p.CRS ? 8 * kx | 8 * ky << 8 : -1;
+            };
+            struct Run { uint4 v[2]; uint32_t how; };   // the vectors the run lies in; its first element there, and the mask << 8
+            auto load = [&](Run (&run)[2], int step) {   // r = 4 step + 2 i + up of the k-block whose taps are held
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int o = __shfl_sync(0xffffffffu, koff, 4 * step + 2 * i + up), t = __shfl_sync(0xffffffffu, kxy, 4 * step + 2 * i + up);
+                    const uint32_t mask = t < 0 ? 0u : xm >> (t & 255) & ym >> (t >> 8) & 255u;
+                    const int e = base + o;
+                    const uint16_t* a = xi + e;
+                    const int s = (int)(reinterpret_cast<uintptr_t>(a) >> 1) & 7, ev = e - s;
+                    const uint4* v = reinterpret_cast<const uint4*>(a - s);
+                    run[i].how = (uint32_t)s | mask << 8;
+                    // a vector is read if it holds an element of the image
+                    run[i].v[0] = mask != 0 && ev > -8 && ev < total ? __ldg(v) : make_uint4(0u, 0u, 0u, 0u);
+                    run[i].v[1] = mask != 0 && s != 0 && ev > -16 && ev + 8 < total ? __ldg(v + 1) : make_uint4(0u, 0u, 0u, 0u);
+                }
+            };
+            auto put = [&](const Run (&run)[2], int stage, int step) {
+                uint8_t* a = to + stage * Cfg::STAGE_BYTES + step * (512 * WARPS);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t s = run[i].how & 7u, mask = run[i].how >> 8;
+                    const uint4 v0 = run[i].v[0], v1 = run[i].v[1];
+                    // by two words, one word, one element
+                    const bool b2 = s & 4, b1 = s & 2;
+                    const uint32_t t0 = b2 ? v0.z : v0.x, t1 = b2 ? v0.w : v0.y, t2 = b2 ? v1.x : v0.z, t3 = b2 ? v1.y : v0.w, t4 = b2 ? v1.z : v1.x,
+                                   t5 = b2 ? v1.w : v1.y;
+                    const uint32_t u[5] = {b1 ? t1 : t0, b1 ? t2 : t1, b1 ? t3 : t2, b1 ? t4 : t3, b1 ? t5 : t4};
+                    uint32_t w[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) w[q] = __funnelshift_r(u[q], u[q + 1], (s & 1u) << 4);
+                    uint32_t in[4];
+                    halves_of_bits(in, mask);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) w[q] &= in[q];
+                    *reinterpret_cast<uint4*>(a + i * (256 * WARPS)) = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+            };
+            Run ra[2], rb[2];
+            taps(0);
+            load(ra, 0);
+            for (int kb = 0; kb < nkb; ++kb) {
+                const int s = kb % Cfg::STAGES;
+                const int n = (p.CRS - (kb0 + kb) * CI_BK + CI_BK / STEPS - 1) / (CI_BK / STEPS);   // steps with a row of the reduction
+                if (n > 1) load(rb, 1);
+                if (ok && !mbar_wait(&empty[s], (uint32_t)((kb / Cfg::STAGES) & 1) ^ 1, p.d_status, KST_WAIT_EMPTY, abort_flag)) ok = false;
+                if (__any_sync(0xffffffffu, !ok)) { ok = false; break; }
+                put(ra, s, 0);
+                if constexpr (STEPS == 4) {
+                    if (n > 2) load(ra, 2);
+                    if (n > 1) put(rb, s, 1);
+                    if (n > 3) load(rb, 3);
+                    if (n > 2) put(ra, s, 2);
+                }
+                if (kb + 1 < nkb) {
+                    taps(kb + 1);
+                    load(ra, 0);
+                }
+                if (n >= STEPS) put(rb, s, STEPS - 1);
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[s]);
             }
         } else {
         // Pixels 2 lane, 2 lane + 1 of either half of the tile.
@@ -473,14 +582,21 @@ int conv_words_weight(b200_ctx* ctx, void* dst, const void* w, int64_t KW, int64
 // Channels per CTA: all of them up to 256, since every channel tile gathers the pixels again; but a launch that
 // leaves half of the GPU's CTAs unused splits the reduction, two k-blocks a part at least, which the 256-wide
 // tile has no shared memory for; four a part where they are read in words and take less than a cluster's barriers
-// (256 x 256 x 32 -> 128, 3 x 3 / 2: 15.8 us with two, 9.2).  tiles: pixel tiles of all images; cols: of the reduction.
+// (256 x 256 x 32 -> 128, 3 x 3 / 2: 15.8 us with two, 9.2).  Eight parts up to the clusters a GPC's SMs hold at once (48 x 44 x
+// 256 -> 256, 3 x 3, 34 clusters: 25.5 us, with four parts 21.1).  tiles: pixel tiles of all images; cols: of the reduction.
 struct CiTiles { int bn, parts; int64_t nkb; };
 static CiTiles ci_tiles(const b200_ctx* ctx, int64_t tiles, int64_t cols, int64_t Cout, int g) {
     const int64_t room = 2 * (int64_t)ctx->prop.multiProcessorCount, nkb = cdiv(cols, CI_BK);
     CiTiles t = {Cout <= 64 ? 64 : (Cout <= 128 || (2 * tiles * cdiv(Cout, 128) <= room && nkb >= 4) ? 128 : 256), 1, nkb};
     if (t.bn < 256)
-        while (t.parts < 8 && 2 * t.parts * tiles * cdiv(Cout, t.bn) <= room && nkb >= (g ? 8 : 4) * t.parts) t.parts *= 2;
+        while (t.parts < 8 && (2 * t.parts + (t.parts == 4)) * tiles * cdiv(Cout, t.bn) <= room && nkb >= (g ? 8 : 4) * t.parts) t.parts *= 2;
     return t;
+}
+
+// What a convolution takes through the im2col matrix of a small image, one after the other, in microseconds (fitted as below).
+static double ci_matrix(int64_t N, int64_t P, int64_t crs, int64_t Cout) {
+    return (double)N * (6.9 + 2.36e-6 * (double)P * (double)crs + 1.3e-9 * (double)P * (double)crs * (double)Cout + 0.0012 * (double)crs) +
+           (crs % 8 != 0 ? 1.2 : 0.0);
 }
 
 // Which of the convolutions that can be read in words gain by it.  Not where laying out the weight is more than reading the
@@ -497,12 +613,29 @@ bool conv_words_gains(const b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, in
     if (taps) return true;
     const CiTiles t = ci_tiles(ctx, tiles, cols, Cout, g);
     const double load = (double)(tiles * cdiv(Cout, t.bn) * t.parts) / (2.0 * ctx->prop.multiProcessorCount);   // of the resident CTAs
-    const double crs = (double)(KW * KH * Cin);
     const double words = 3.1 + 4.8e-6 * (double)(cols * Cout) + (double)cdiv(t.nkb, t.parts) * (0.41 + 0.84 * load) +
                          0.0129 * t.bn * (load > 1.0 ? load : 1.0) + (t.parts > 1 ? 2.5 + 1.8 * load : 0.0);
-    const double matrix = (double)N * (6.9 + 2.36e-6 * (double)P * crs + 1.3e-9 * (double)P * crs * (double)Cout + 0.0012 * crs) +
-                          (KW * KH * Cin % 8 != 0 ? 1.2 : 0.0);
-    return 1.04 * words < matrix;
+    return 1.04 * words < ci_matrix(N, P, KW * KH * Cin, Cout);
+}
+
+// Whether the pixels' taps are runs of memory as the pixels are: a row of results as long as the image's, pixel by pixel.
+bool conv_runs(int64_t W, int64_t KW, int64_t KH, int64_t sx, int64_t sy, int64_t OW) {
+    return sx == 1 && sy == 1 && OW == W && W >= 8 && KW <= 4 && KH <= 4;
+}
+
+// Whether a small image read in runs beats its im2col matrix, by an estimate fitted to 190 of 3 x 3, 16 to 512 pixels a side and 1 to
+// 384 -> 8 to 512 channels, in microseconds: the route it picks is 0.3 % off the faster one in the mean and 8 % at worst (always runs
+// 2.5 and 46 %, always the matrix 73 % in the mean).  64 x 60 x 64 -> 64: 12.8 -> 8.2 us, two images 25.2 -> 11.2, 128 x 124 x 128 ->
+// 128 50.8 -> 24.2, 128 x 124 x 64 -> 64 29.2 -> 15.1; a reduction off eights, whose weight either route copies, stays with the matrix
+// more often (48 x 47 x 133 -> 488: 20.1, 29.3).
+bool conv_runs_gain(const b200_ctx* ctx, int64_t Cin, int64_t N, int64_t KW, int64_t KH, int64_t Cout, int64_t P) {
+    const int64_t crs = KW * KH * Cin, tiles = cdiv(P, CI_PIX) * N;
+    const CiTiles t = ci_tiles(ctx, tiles, crs, Cout, 0);
+    const double load = (double)(tiles * cdiv(Cout, t.bn) * t.parts) / (2.0 * ctx->prop.multiProcessorCount), rounds = load > 1.0 ? load : 1.0;
+    const double blocks = t.parts > 1 ? (double)cdiv(t.nkb, t.parts) : (double)crs / CI_BK;
+    const double runs = 0.81 + blocks * (0.55 + 1.65 * load) + (0.012 * t.bn + 2.47) * rounds + (t.parts > 1 ? 2.44 + 0.7 * load : 0.0) +
+                        (crs % 8 != 0 ? 1.75 + 4.3e-6 * (double)(crs * Cout) : 0.0);
+    return 0.95 * runs < ci_matrix(N, P, crs, Cout);
 }
 
 int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t KW, int64_t KH, int64_t Cout,
@@ -547,7 +680,7 @@ int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64
     auto go = [&](auto zero, auto G) -> int {
         using T = decltype(zero);
         constexpr int g = decltype(G)::value;
-        if constexpr (g > 0) {
+        if constexpr (g != 0) {
             if (small && bn == 128) return ci_launch<128, T, g, true>(ctx, tw, p, N, 1);
             if (small && bn == 64) return ci_launch<64, T, g, true>(ctx, tw, p, N, 1);
         }
@@ -558,6 +691,7 @@ int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64
     auto typed = [&](auto G) { return out_dtype == B200_F16 ? go(__half(), G) : go(float(), G); };
     if (g == 8) return typed(std::integral_constant<int, 8>());
     if (g == 4) return typed(std::integral_constant<int, 4>());
+    if (conv_runs(W, KW, KH, sx, sy, OW)) return typed(std::integral_constant<int, -1>());
     return typed(std::integral_constant<int, 0>());
 }
 

@@ -138,6 +138,8 @@ int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64
                          int64_t out_img, int out_dtype, int epilogue, int g);
 // Its form for even strides (g = conv_words, not 0), whose weight conv_words_weight lays out with leading dimension conv_words_ldw.
 int conv_words(int64_t W, int64_t KW, int64_t sx, int64_t px, int64_t dx, const void* x, int64_t x_img);
+bool conv_runs(int64_t W, int64_t KW, int64_t KH, int64_t sx, int64_t sy, int64_t OW);
+bool conv_runs_gain(const b200_ctx* ctx, int64_t Cin, int64_t N, int64_t KW, int64_t KH, int64_t Cout, int64_t P);
 bool conv_words_gains(const b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64_t N, int64_t KW, int64_t KH, int64_t Cout, int64_t P,
                       int g, bool taps);
 int64_t conv_words_ldw(int64_t rows, int g);

@@ -2,6 +2,7 @@ import os
 
 import numpy as np
 import pytest
+import torch
 
 import juliavision_b200 as jv
 
@@ -266,6 +267,36 @@ def test_conv_in_words_does_not_depend_on_the_workspace(ora, Cin, Cout, H, W, sc
         c.synchronize()
         assert relerr(out.to_host(), ref) < 2e-5
         del g
+
+
+# (N, Cin, H, W, Cout, (KH, KW), (py, px), (dy, dx)), every row of results as long as the image's: the narrowest image, one and two
+# k-blocks' ends inside sixteen rows, more pixel tiles than two CTAs an SM take (64 and 128 channels), a split reduction, 256 channels
+# a CTA, 1 x 1, four taps and two (dilated, so that the lengths agree), an image the GEMM could store as well
+RUNS = [(1, 3, 9, 8, 5, (3, 3), (1, 1), (1, 1)), (2, 5, 17, 11, 70, (3, 3), (1, 1), (1, 1)), (1, 40, 37, 131, 200, (1, 1), (0, 0), (1, 1)),
+        (2, 8, 201, 255, 40, (3, 3), (1, 1), (1, 1)), (1, 9, 261, 255, 100, (3, 3), (1, 1), (1, 1)), (1, 200, 33, 31, 300, (3, 3), (1, 1), (1, 1)),
+        (1, 16, 51, 49, 24, (4, 2), (0, 1), (1, 2)), (3, 7, 21, 23, 16, (2, 4), (3, 3), (5, 2)), (1, 64, 60, 64, 64, (3, 3), (1, 1), (1, 1)),
+        (1, 12, 40, 45, 72, (3, 3), (2, 9), (1, 9))]
+
+
+@pytest.mark.parametrize("N,Cin,H,W,Cout,K,pad,dil", RUNS)
+@pytest.mark.parametrize("off", [0, 1, 6])
+def test_conv_in_runs(ctx, ora, N, Cin, H, W, Cout, K, pad, dil, off):
+    """Stride one and rows of the same length, the image at any distance from 16 bytes, NaN before and behind it."""
+    rng = np.random.default_rng(Cin + Cout + W)
+    x = np.float16(rng.standard_normal((N, Cin, H, W)) * 0.5)
+    w = np.float16(rng.standard_normal((Cout, Cin) + K) * 0.2)
+    b = np.float16(rng.standard_normal(Cout) * 0.2)
+    ref = torch.nn.functional.conv2d(*(torch.from_numpy(a).double() for a in (x, w, b)), padding=pad, dilation=dil).numpy()
+    assert ref.shape[-1] == W
+    base = ctx.toback(np.concatenate([np.full(off, np.nan, np.float16), x.reshape(-1), np.full(8, np.nan, np.float16)]))
+    dx = jv.DeviceArray(ctx, base.ptr + 2 * off, np.float16, (W, H, Cin, N), owner=base)
+    dw, db = ctx.toback(w), ctx.toback(b)
+    for dt, tol in ((np.float16, 2e-3), (np.float32, 2e-5)):      # one rounding step of fp16; sqrt(CRS) eps32
+        out = ctx.allocate(dt, *reversed(ref.shape))
+        ctx.fill_bytes(out, 0xFF)
+        jv.convolution_(ctx, out, dx, dw, db, (1, 1), pad[::-1], dil[::-1], 1)
+        ctx.synchronize()
+        assert relerr(out.to_host(), ref) < tol, describe(out.to_host(), ref, tol)
 
 
 # more pixel tiles than two CTAs an SM take: 64 and 128 channels a CTA, ragged, one and several k-blocks, words of 4 and 2, two images
