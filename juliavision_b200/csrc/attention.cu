@@ -1429,8 +1429,8 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     const int64_t pairs = (int64_t)p.qpairs * H * B;      // work items: pairs of query tiles, or single tiles of short keys
     B200_REQUIRE(pairs < (1ll << 30), B200_DECLINE_EXTENT, "attention: too many query tiles");
     // Pairs that do not fill the SMs are cut along the keys (att_split): over a cluster's CTAs, which join their rows in the same
-    // launch, or over more of them with a merge behind.  A last wave that would leave most SMs idle has its pairs cut
-    // (at least two key blocks per piece) so that the wave is as short as that allows instead of a whole pair long.
+    // launch, or over more of them with a merge behind.  A last wave that would leave most SMs idle has its pairs cut the same way,
+    // so that the wave is as short as that allows instead of a whole pair long.
     p.nsplit = 1;
     p.ntail = 0;
     p.part_o = p.part_ml = nullptr;
