@@ -76,7 +76,6 @@ struct ConvParams {
     int sx, sy, px, py, dx, dy;
     int KW, KH;
     int rows;                 // G: kernel rows of all channels, Cin * KH
-    int late;                 // G, 256 channels: the gather waits for what runs before it
     uint32_t mask[4];         // G: the words of a kernel row that are taps
     uint32_t mKW, mKH;        // ceil(2^32 / KW), ceil(2^32 / KH): exact quotients below 2^16
     int epi;
@@ -183,11 +182,9 @@ conv_implicit_kernel(const __grid_constant__ CUtensorMap tmapW,   // w: {CRS, Co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    // In words the kernel before this one lays out the weight, and lets this one start when all before it is done: the image
-    // and the bias are there, and only the weight has to be waited for
-    // (256 x 256 x 32 -> 128, 3 x 3 / 2, with the issuing warp below: 9.07 -> 8.18 us; 1024 x 1024 x 3 -> 112, 7 x 7 / 4: 15.83 -> 15.66).
-    // Not at 256 channels and more CTAs than SMs (700 x 700 x 3 -> 200: 13.6 us early, 12.9; 512 x 512 x 3 -> 160, 128 CTAs: 8.7, 9.2).
-    if (G <= 0 || (BN == 256 && p.late) || warp == TMA_WARP) grid_dep_wait();
+    // Every warp, in words too: the launch before lays out the weight and has itself waited for the image, but a kernel's writes are
+    // visible to the grid that waits, and the gather reads past the L1's coherence (ld.global.nc).
+    grid_dep_wait();
     grid_dep_launch();
 
     // Channel c of the tile at pixel pix, rounded before the activation sees it.  The activation is a template
@@ -673,7 +670,6 @@ int conv_implicit_launch(b200_ctx* ctx, int64_t W, int64_t H, int64_t Cin, int64
     const CiTiles t = ci_tiles(ctx, p.tiles * N, p.CRS, Cout, g);
     const int bn = t.bn, parts = t.parts;
     const bool small = parts == 1 && p.tiles * N * cdiv(Cout, bn) > 2 * ctx->prop.multiProcessorCount;
-    p.late = p.tiles * N * cdiv(Cout, bn) > ctx->prop.multiProcessorCount;
     CUtensorMap tw;
     uint64_t dims[2] = {(uint64_t)p.CRS, (uint64_t)Cout};
     uint64_t str[1] = {(uint64_t)ldw * 2};

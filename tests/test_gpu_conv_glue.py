@@ -321,6 +321,42 @@ def test_conv_in_words_of_many_tiles(ctx, ora, N, Cin, H, W, Cout, K, stride, dt
     assert relerr(out.to_host(), ref) < tol, describe(out.to_host(), ref, tol)
 
 
+# 64, 128 and 256 channels a CTA: up to a CTA an SM and more of them, four smaller CTAs an SM among them, words of 4 and 2
+@pytest.mark.parametrize("N,Cin,H,W,Cout,K,stride", [(1, 3, 256, 256, 64, 7, 4), (1, 3, 808, 804, 112, 7, 4), (1, 16, 130, 132, 100, 3, 2),
+                                                     (1, 16, 180, 180, 200, 3, 2), (1, 3, 512, 512, 160, 7, 4), (1, 3, 700, 700, 200, 7, 4)])
+def test_conv_in_words_reads_what_was_written_last(ctx, ora, N, Cin, H, W, Cout, K, stride):
+    """One buffer, rewritten by the kernel right before and convolved again and again: every result is that of the image and bias
+    it was called on, eagerly and recorded."""
+    rng = np.random.default_rng(Cin + Cout + W)
+    images = [np.float16(rng.standard_normal((N, Cin, H, W)) * 0.5) for _ in range(3)]
+    w = np.float16(rng.standard_normal((Cout, Cin, K, K)) * 0.2)
+    biases = [np.float16(rng.standard_normal(Cout) * 0.2) for _ in images]
+    dw, x, b = ctx.toback(w), ctx.allocate(np.float16, W, H, Cin, N), ctx.allocate(np.float16, Cout)
+    hx, hb = ([ctx.toback(a * np.float16(0.5)) for a in part] for part in (images, biases))
+    refs = [ora.conv2d(a, w, v, (stride,) * 2, (K // 2,) * 2, out_dtype=np.float32) for a, v in zip(images, biases)]
+    outs = [ctx.allocate(np.float32, *reversed(refs[0].shape)) for _ in range(6)]
+
+    def rounds():
+        for i, out in enumerate(outs):
+            jv.add_(ctx, b, hb[i % 3], hb[i % 3])
+            jv.add_(ctx, x, hx[i % 3], hx[i % 3])
+            jv.convolution_(ctx, out, x, dw, b, (stride,) * 2, (K // 2,) * 2, (1, 1), 1)
+
+    ctx.ws.reset()
+    before = ctx.launch_count()
+    rounds()
+    assert ctx.launch_count() - before == 4 * len(outs)     # two sums, the weight laid out, the convolution in words
+    g = ctx.capture(rounds)
+    for run in (rounds, g.replay):
+        for out in outs:
+            ctx.fill_bytes(out, 0xFF)
+        run()
+        ctx.synchronize()
+        for i, out in enumerate(outs):
+            assert relerr(out.to_host(), refs[i % 3]) < 2e-5, i      # as above
+    del g
+
+
 def test_conv_in_words_keeps_to_its_taps(ctx, ora):
     """An infinity or NaN beside a pixel's taps, inside the words that hold them, does not reach it."""
     x = np.float16(np.random.default_rng(3).standard_normal((1, 2, 16, 64)))
