@@ -570,11 +570,11 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
     return warp_sum(t);
 }
 
-// Rows of more than some 224 vectors: a block per row, a thread four to six vectors of it, kept as read (fp16 stays packed, 28 to
+// Rows of some 224 to 512 vectors: a block per row, a thread four to six vectors of it, kept as read (fp16 stays packed, 28 to
 // 46 registers), moments and output two elements an instruction, the two sums through shared memory with one barrier each.
-// Bound by HBM; a warp a row (ln_warp_kernel) holds 8 registers a vector and then has too few rows in flight, 256 threads a row
-// too little each.  Microseconds, a warp or 256 threads a row before -> now, 80 Mi elements of fp16: 1800 wide 70.5 -> 66.8, 2056
-// 89.3 -> 68.8, 2560 84.6 -> 58.1 (5.5 TB/s), 3072 76.5 -> 60.8, 4096 112.3 -> 63.2, 5120 85.9 -> 59.7; 40 Mi of fp32: 1280 53.8 -> 51.6,
+// Bound by HBM; a warp a row (ln_warp_kernel) holds 8 registers a vector and then has too few rows in flight.  Microseconds, a
+// warp a row before -> now, 80 Mi elements of fp16: 1800 wide 70.5 -> 66.8, 2056
+// 89.3 -> 68.8, 2560 84.6 -> 58.1 (5.5 TB/s), 3072 76.5 -> 60.8, 4096 112.3 -> 63.2; 40 Mi of fp32: 1280 53.8 -> 51.6,
 // 2048 60.1 -> 52.3; in the L2, 1953 x 4096 16.8 -> 8.8; 64 x 4096 6.7 -> 3.2; behind the add 9765 x 4096 105 -> 51.7
 // (6.2 TB/s), 600 x 4096 11.7 -> 6.1.  Narrower rows lose (52083 x 1536: 59.2 -> 64.8).  gamma and beta asked for with
 // the row cost a fifth (registers), and so did rings of rows in shared memory that bulk copies fill, a warp a row (20480 x 4096: 98).
@@ -662,9 +662,12 @@ ln_split_kernel(const InT* a, InT* x, const InT* __restrict__ h, OutT* __restric
     }
 }
 
-// fp32 rows of more than 512 vectors, and as wide fp16 ones in launches of few rows: 256 threads a row, the row in registers,
-// the two sums over the block through shared memory.  Bound by HBM; with scalar accesses and the row read three
-// times these rows took 71.6 us for 7112 x 4280 in fp32, now 44.5 (5.5 TB/s; replayed over four operand sets).
+// Rows of more than 512 vectors: 256 threads a row, the row in registers as it was read (fp16 stays packed: an SM holds twice the
+// blocks that it does with the row in fp32), the two sums over the block through shared memory.  One order of sums whatever
+// the number of rows, so that a row's bits do not depend on the rows beside it.  Bound by HBM; with scalar accesses and the row read
+// three times 7112 x 4280 in fp32 took 71.6 us, now 44.5 (5.5 TB/s; replayed over four operand sets).  fp16, microseconds with the
+// row in fp32 and now: 64 x 4104 3.3, 3.0; 592 x 5120 behind another kernel 5.3, 5.0; 1600 x 6144 13.8, 11.1; 10000 x 5120 56.0, 41.3;
+// 4000 x 16384 75.9, 46.3.  The block a row above took 3.7, 5.6, 12.9, 39.4 and 64.6 there (700 x 5120: 6.0, here 4.6).
 template <typename InT, typename OutT, int VPT>
 __global__ void __launch_bounds__(LN_WIDE_THREADS)
 ln_wide_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restrict__ mean, float* __restrict__ rstd,
@@ -680,14 +683,14 @@ ln_wide_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
 #pragma unroll
     for (int i = 0; i < VPT; ++i)
         if (tid + LN_WIDE_THREADS * i < nvec) raw[i].raw = __ldg(src + tid + LN_WIDE_THREADS * i);
-    float x[VPT][VN];
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < VPT; ++i)
         if (tid + LN_WIDE_THREADS * i < nvec) {
-            raw[i].to_f32(x[i]);
+            float x[VN];
+            raw[i].to_f32(x);
 #pragma unroll
-            for (int j = 0; j < VN; ++j) s += x[i][j];
+            for (int j = 0; j < VN; ++j) s += x[j];
         }
     const float n = (float)C;
     const float mu = block_sum(s, red) / n;
@@ -695,9 +698,11 @@ ln_wide_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
 #pragma unroll
     for (int i = 0; i < VPT; ++i)
         if (tid + LN_WIDE_THREADS * i < nvec) {
+            float x[VN];
+            raw[i].to_f32(x);
 #pragma unroll
             for (int j = 0; j < VN; ++j) {
-                const float d = x[i][j] - mu;
+                const float d = x[j] - mu;
                 s2 += d * d;
             }
         }
@@ -707,9 +712,10 @@ ln_wide_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
     for (int i = 0; i < VPT; ++i) {
         const int v = tid + LN_WIDE_THREADS * i;
         if (v < nvec) {
-            float y[VN];
+            float x[VN], y[VN];
+            raw[i].to_f32(x);
 #pragma unroll
-            for (int j = 0; j < VN; ++j) y[j] = (x[i][j] - mu) * r;
+            for (int j = 0; j < VN; ++j) y[j] = (x[j] - mu) * r;
             if (sizeof(OutT) == 4 && gamma && beta) {
                 // gamma and beta in one rounding, as in ln_block_kernel: with two, fp32 results were 7 % further from 64
                 // bits (rounded to fp16 it does not show, and there both vectors at once cost registers and 17 % of the time)
@@ -739,7 +745,7 @@ ln_wide_kernel(const InT* __restrict__ a, OutT* __restrict__ out, float* __restr
                 t.to_f32(bf);
 #pragma unroll
                 for (int j = 0; j < VN; ++j)   // fp32 without gamma: one rounding too (with two, 14 % further)
-                    if constexpr (sizeof(OutT) == 4) y[j] = fmaf(x[i][j] - mu, r, bf[j]);
+                    if constexpr (sizeof(OutT) == 4) y[j] = fmaf(x[j] - mu, r, bf[j]);
                     else y[j] += bf[j];
             }
             store_vec<VN>(dst + (int64_t)v * VN, y);
@@ -803,13 +809,12 @@ static bool ln_fills(const b200_ctx* ctx, int64_t groups, int rows, int lpg, int
     return groups >= n * ctx->prop.multiProcessorCount * 4 * rows * (32 / lpg);
 }
 
-// Vectors a thread of ln_split_kernel, 0 for rows that stay with the other kernels.  Past 512 vectors 256 threads a row are as fast
-// in fp32 (2400 x 2600: 12.6 us, 13.8; 11111 x 3600 50.5, 52.9), and in fp16 where a launch waits for a block or two (64 x
-// 5120: 3.4 us, 3.7; 1200 x 5120 7.1, 6.4): the last bits of a row of more than 4096 depend on that.
-template <typename InT> static int ln_split(const b200_ctx* ctx, int64_t groups, int nvec) {
-    if (sizeof(InT) == 4) return nvec > 256 && nvec <= 512 ? 6 : 0;
-    if (nvec <= 224 || (nvec > 512 && groups <= (int64_t)4 * ctx->prop.multiProcessorCount)) return 0;
-    return cdiv(cdiv(nvec, 5), 32) < cdiv(cdiv(nvec, 4), 32) ? 5 : 4;
+// Vectors a thread of ln_split_kernel, 0 for rows that stay with the other kernels.  Past 512 vectors 256 threads a row are as fast or
+// faster: in fp32 2400 x 2600 12.6 us, 13.8, 11111 x 3600 50.5, 52.9; in fp16 see ln_wide_kernel.
+template <typename InT> static int ln_split(int nvec) {
+    if (nvec > 512) return 0;
+    if (sizeof(InT) == 4) return nvec > 256 ? 6 : 0;
+    return nvec <= 224 ? 0 : cdiv(cdiv(nvec, 5), 32) < cdiv(cdiv(nvec, 4), 32) ? 5 : 4;
 }
 
 template <typename InT, typename OutT>
@@ -858,8 +863,11 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
         else if (ln_fills(ctx, groups, 2, L, sizeof(InT) == 4 ? 10 : 14)) LN_GO_ROWS(1, L, 2);              \
         else ONE;                                                                                           \
     } while (0)
+#define LN_GO_WIDE(V)                                                                                       \
+    B200_CUDA(launch_dep(ln_wide_kernel<InT, OutT, V>, dim3((unsigned)groups), dim3(LN_WIDE_THREADS), 0, ctx->stream, 1, ap, op, \
+                         mean, rstd, gp, bp, (int)C, eps))
         // A block a row: the vectors a thread that leave fewer lanes idle (320 vectors: five of 64 threads, four would be of 96).
-        const int split = ln_split<InT>(ctx, groups, nvec);
+        const int split = ln_split<InT>(nvec);
         auto go_split = [&](auto kern) {
             return launch_dep(kern, dim3((unsigned)groups), dim3((unsigned)cdiv(cdiv(nvec, split), 32) * 32), 0, ctx->stream, 1, ap,
                               (InT*)nullptr, (const InT*)nullptr, op, mean, rstd, gp, bp, (int)C, eps, 0, 0.f, 0.f);
@@ -876,12 +884,11 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
         else if (vpl <= 5) LN_GO(5);
         else if (vpl <= 6) LN_GO(6);
         else if (vpl <= 8) LN_GO(8);
-        else if (nvec <= 4 * LN_WIDE_THREADS)
-            B200_CUDA(launch_dep(ln_wide_kernel<InT, OutT, 4>, dim3((unsigned)groups), dim3(LN_WIDE_THREADS), 0, ctx->stream, 1, ap,
-                                 op, mean, rstd, gp, bp, (int)C, eps));
-        else
-            B200_CUDA(launch_dep(ln_wide_kernel<InT, OutT, 8>, dim3((unsigned)groups), dim3(LN_WIDE_THREADS), 0, ctx->stream, 1, ap,
-                                 op, mean, rstd, gp, bp, (int)C, eps));
+        else if (nvec <= 3 * LN_WIDE_THREADS) LN_GO_WIDE(3);
+        else if (nvec <= 4 * LN_WIDE_THREADS) LN_GO_WIDE(4);
+        else if (nvec <= 6 * LN_WIDE_THREADS) LN_GO_WIDE(6);
+        else LN_GO_WIDE(8);
+#undef LN_GO_WIDE
 #undef LN_GO
 #undef LN_GO_SHARED
 #undef LN_GO_ROWS
@@ -951,7 +958,7 @@ extern "C" int b200_add_layernorm_f16(b200_ctx* ctx, int64_t groups, int64_t C, 
         else if (ln_fills(ctx, groups, 2, L, 20)) LNA_GO_ROWS(1, L, 2);                                           \
         else ONE;                                                                                                 \
     } while (0)
-    const int split = ln_split<__half>(ctx, groups, nvec);
+    const int split = ln_split<__half>(nvec);
     auto go_split = [&](auto kern) {
         return launch_dep(kern, dim3((unsigned)groups), dim3((unsigned)cdiv(cdiv(nvec, split), 32) * 32), 0, ctx->stream, 1,
                           (const __half*)nullptr, (__half*)x, (const __half*)h, (__half*)out, mean, rstd, (const __half*)gamma,

@@ -226,3 +226,17 @@ def test_a_block_a_row(ctx, ora, dt, C, groups):
         ctx.synchronize()
         for one, other in ((xa, xb), (oa, ob), (m1, m2), (r1, r2)):
             assert np.array_equal(one.to_host(), other.to_host())
+
+
+@pytest.mark.parametrize("dt,C,groups", [(np.float16, 1800, 800), (np.float16, 4096, 800), (np.float16, 4104, 800), (np.float16, 5120, 800),
+                                         (np.float16, 6152, 800), (np.float16, 8200, 800), (np.float16, 16384, 600), (np.float32, 2048, 600),
+                                         (np.float32, 3076, 600)])
+def test_a_wide_rows_bits_do_not_depend_on_the_rows_beside_it(ctx, dt, C, groups):
+    """The rows of a shard are those of the whole: below and above four rows an SM, and one alone."""
+    rng = np.random.default_rng(C)
+    a = (rng.standard_normal((groups, C), dtype=np.float32) * 2 + 0.5).astype(dt)
+    gam, bet = ((o + 0.1 * rng.standard_normal(C)).astype(dt) for o in (1, 0))
+    whole = layernorm_gpu(ctx, a, gam, bet, 1e-5)
+    for n in (1, 148, 592):
+        for one, other in zip(layernorm_gpu(ctx, a[:n], gam, bet, 1e-5), whole):
+            assert np.array_equal(one, other[:n])
