@@ -1224,7 +1224,10 @@ mask_rows_kernel(const __half* __restrict__ mask, uint4* __restrict__ out, int L
 // The copy costs 2 us and 0.9 per million entries; a CTA gains 0.95 us a key block over copies of 8 bytes by the softmax's own
 // warps (1.6 with its wider heads, and over copies of words), less where its 256 rows are not all there.  20 heads x 1500 x 1500
 // 42.1 -> 36.9 us, 2 x 8 x 1001 x 1001 31.1 -> 26.7, 4 x 20 x 1001 x 1001 x 32 88.8 -> 62.6; 2 x 2001 x 2001 x 128 would
-// go 24.6 -> 26.8 and 8 x 100 x 3001 16.2 -> 17.9.  Keys apart, 20 x 1500 x 1500 193 -> 92, 4 x 300 x 300 44.6 -> 14.5.  `serial`: key blocks a CTA walks.
+// go 24.6 -> 26.8 and 8 x 100 x 3001 16.2 -> 17.9.  Keys apart, 20 x 1500 x 1500 193 -> 92, 4 x 300 x 300 44.6 -> 14.5.
+// The workspace keeps what a copy took and half as much again, so there is a most to it: 256 MiB are 11584 x 11584 entries, and a
+// larger mask is read in place, as every one that is not copied.  `serial`: key blocks a CTA walks.
+constexpr size_t MASK_COPY_MOST = (size_t)256 << 20;
 static int mask_map(b200_ctx* ctx, const __half* bptr, const int64_t* bs, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B,
                     int64_t serial, AttnParams* p, CUtensorMap* tm) {
     const uint64_t Hm = bs[2] != 0 ? (uint64_t)H : 1, Bm = bs[3] != 0 ? (uint64_t)B : 1;
@@ -1240,18 +1243,19 @@ static int mask_map(b200_ctx* ctx, const __half* bptr, const int64_t* bs, int64_
     const void* base = bptr;
     if (!lies) {
         const int64_t rows = Lq * (int64_t)(Hm * Bm), n8 = (Lk + 7) / 8;
-        // Its room is asked for before it is weighed, so that a context gets it with its first masked call.
-        const size_t mark = ctx->ws_used;
-        void* ws = nullptr;
-        const int rc = ws_scratch(ctx, (size_t)(rows * n8) * 16, &ws);
-        if (rc == B200_ENOMEM) return B200_OK;
-        if (rc) return rc;
+        const size_t bytes = (size_t)(rows * n8) * 16, mark = ctx->ws_used;
         const bool apart = p->mask == MASK_DIRECT;
         const double gain = (apart ? 6.0 : p->mask == MASK_EIGHTS && E <= 64 ? 0.95 : 1.6) * (double)serial;
-        if (gain * (Lq < 2 * ATT_BR ? (double)Lq / (2 * ATT_BR) : 1.0) < 2.0 + (apart ? 8e-6 : 0.9e-6) * (double)(rows * Lk)) {
-            ctx->ws_used = mark;
+        void* ws = nullptr;
+        if (bytes > MASK_COPY_MOST ||
+            gain * (Lq < 2 * ATT_BR ? (double)Lq / (2 * ATT_BR) : 1.0) < 2.0 + (apart ? 8e-6 : 0.9e-6) * (double)(rows * Lk)) {
+            // A context's first masked call leaves it a workspace, if only the smallest: one recorded later finds room for a small copy.
+            if (ctx->ws_buf == nullptr && ws_scratch(ctx, 0, &ws) == B200_OK) ctx->ws_used = mark;
             return B200_OK;
         }
+        const int rc = ws_scratch(ctx, bytes, &ws);
+        if (rc == B200_ENOMEM) return B200_OK;
+        if (rc) return rc;
         B200_CUDA(launch_dep(mask_rows_kernel, dim3((unsigned)cdiv(rows, 8), 1, 1), dim3(256, 1, 1), 0, ctx->stream, 1, bptr, (uint4*)ws,
                              (int)Lq, (int)Lk, rows, (int)Hm, bs[0], bs[1], bs[2], bs[3]));
         ctx->launches++;

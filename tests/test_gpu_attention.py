@@ -701,3 +701,40 @@ def test_a_last_round_cut_over_clusters(ctx, ora, B, H, Lq, Lk, E):
         ctx.synchronize()
         assert np.array_equal(z.to_host(), want) and np.array_equal(out.to_host(), got)
     del g
+
+
+def test_a_mask_that_is_not_copied_takes_no_workspace(ora):
+    """Masks off 16-byte boundaries: a plane a head, which is dearer to copy than to read in place, and one of more entries than are
+    ever copied.  The workspace stays as it was found."""
+    rng = np.random.default_rng(12)
+    with jv.Ctx(0) as c:
+        c.scratch(np.float16, 8)
+        c.ws.reset()
+        found = c.ws.stats()
+        B, H, L, E = 2, 8, 1001, 64
+        q, k, v = (np.float16(rng.standard_normal((B, H, L, E))) for _ in range(3))
+        bias = np.float16(rng.standard_normal((B, H, L, L)))
+        bias[rng.random(bias.shape) < 0.2] = -np.inf
+        dq, dk, dv = qkv_views(c, q, k, v)
+        db, out = c.toback(bias), c.allocate(np.float32, E, L, H, B)
+        c.fill_bytes(out, 0xFF)
+        jv.sdpa(c, dq, dk, dv, db, 1 / np.sqrt(E), out=out)
+        c.synchronize()
+        ref = ora.attention_ref(q, k, v, 1 / np.sqrt(E), bias=bias)
+        assert relerr(out.to_host(), ref) < TOL, describe(out.to_host(), ref, TOL)
+        assert c.ws.stats() == found
+
+        H, L = 3, 11601
+        dq, dk, dv = (c.toback(np.float16(rng.standard_normal((1, H, L, E)))) for _ in range(3))
+        room = c.allocate(np.float16, L * L + 1)
+        c.fill_bytes(room, 0)
+        zeros = jv.DeviceArray(c, room.ptr + 2, np.float16, (L, L, 1, 1), owner=room)
+        got, ref = (c.allocate(np.float32, E, L, H, 1) for _ in range(2))
+        c.fill_bytes(got, 0xFF)
+        jv.sdpa(c, dq, dk, dv, zeros, 1 / np.sqrt(E), out=got)
+        c.synchronize()
+        assert c.ws.stats() == found
+        jv.sdpa(c, dq, dk, dv, None, 1 / np.sqrt(E), out=ref)
+        c.synchronize()
+        # either side rounds P to fp16 about a reference point of its own: 2^-11 of each of 11601 weights
+        assert relerr(got.to_host(), ref.to_host()) < 2e-3
