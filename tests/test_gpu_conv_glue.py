@@ -299,6 +299,25 @@ def test_conv_in_runs(ctx, ora, N, Cin, H, W, Cout, K, pad, dil, off):
         assert relerr(out.to_host(), ref) < tol, describe(out.to_host(), ref, tol)
 
 
+@pytest.mark.parametrize("N,Cin,H,W,K,pad", [(2, 5, 17, 11, (3, 3), (1, 1)), (2, 9, 201, 255, (3, 3), (1, 1)), (1, 33, 21, 25, (3, 3), (1, 1)),
+                                             (1, 6, 19, 13, (1, 3), (0, 1))])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_conv_in_runs_keeps_to_its_taps(ctx, N, Cin, H, W, K, pad, bad):
+    """What a run crosses and a pixel's taps do not reach stays out of it: the other end of the row above or below, the next channel's
+    first row, the last row of the one before, another image.  The rest has the bits it has with zeros there."""
+    rng = np.random.default_rng(W)
+    x = np.float16(rng.standard_normal((N, Cin, H, W)) * 0.5)
+    w = np.float16((0.1 + rng.random((24, Cin) + K)) * 0.2)
+    for where in (np.s_[:, :, :, 0], np.s_[:, :, :, W - 1], np.s_[:, :, 0], np.s_[:, 1, H - 1]) + (np.s_[0],) * (N > 1):
+        spoilt, clean, marks = x.copy(), x.copy(), np.zeros_like(x)
+        spoilt[where], clean[where], marks[where] = bad, 0, 1
+        reached = torch.nn.functional.conv2d(torch.from_numpy(marks).float(), torch.ones((1, Cin) + K), padding=pad).numpy() > 0
+        reached = np.broadcast_to(reached, (N, 24) + reached.shape[2:])
+        got, want = conv_gpu(ctx, spoilt, w, None, (1, 1), pad), conv_gpu(ctx, clean, w, None, (1, 1), pad)
+        assert np.all(np.isfinite(want)) and not np.any(np.isfinite(got[reached]))
+        assert not np.all(reached) and np.array_equal(got[~reached], want[~reached])
+
+
 # more pixel tiles than two CTAs an SM take: 64 and 128 channels a CTA, ragged, one and several k-blocks, words of 4 and 2, two images
 @pytest.mark.parametrize("N,Cin,H,W,Cout,K,stride", [(1, 3, 808, 804, 112, 7, 4), (2, 3, 600, 608, 40, 7, 4), (1, 5, 395, 396, 72, 3, 2), (1, 24, 390, 400, 64, 3, 2)])
 @pytest.mark.parametrize("dt", [np.float16, np.float32])

@@ -224,10 +224,40 @@ def test_tiles_shared_by_a_cluster(ctx, ora, tile, tokens, out, K, monkeypatch):
     assert relerr(two.to_host(), np.stack([zero, -2 * zero])) < 2e-5
 
 
-@pytest.mark.parametrize("tile", ["256x2k2", "256x2k4"])
-@pytest.mark.parametrize("tokens,out,K", [(2, 8, 512), (129, 264, 530), (300, 200, 1288), (517, 1000, 4264), (1500, 1280, 5120)])
-def test_tiles_shared_by_the_pairs_of_a_cluster(ctx, ora, tile, tokens, out, K, monkeypatch):
+def _pair_parts(ctx, tokens, out, K, nbatch=1):
+    """Over how many CTA pairs the plan cuts a 256 x 256 tile's reduction."""
+    import ctypes as C
+    from juliavision_b200 import _lib
+    p = _lib.GemmPlan()
+    _lib.check(_lib.lib().b200_gemm_f16_plan(ctx.handle, out, tokens, K, nbatch, C.byref(p)))
+    assert (p.block_m, p.block_n) == (256, 256)
+    return p.ctas / (2 * -(-tokens // 256) * -(-out // 256) * nbatch)
+
+
+# `one`, `two`: the pairs a tile of the product, and of two of them at once, is shared by; 1 where the clusters would not all be
+# resident, and the tiles stay whole
+@pytest.mark.parametrize("tile,tokens,out,K,one,two", [
+    ("256x2k2", 2, 8, 512, 2, 2), ("256x2k2", 129, 264, 530, 2, 2), ("256x2k2", 300, 200, 1288, 2, 2), ("256x2k2", 517, 1000, 4264, 2, 2),
+    ("256x2k2", 1000, 1000, 5120, 2, 2), ("256x2k2", 1500, 1280, 5120, 2, 1),
+    ("256x2k4", 2, 8, 512, 4, 4), ("256x2k4", 129, 264, 530, 4, 4), ("256x2k4", 300, 200, 1288, 4, 4), ("256x2k4", 300, 700, 4264, 4, 4),
+    ("256x2k4", 517, 1000, 4264, 4, 1), ("256x2k4", 1500, 1280, 5120, 1, 1)])
+def test_tiles_shared_by_the_pairs_of_a_cluster(ctx, ora, tile, tokens, out, K, one, two, monkeypatch):
+    monkeypatch.setenv("B200_GEMM_TILE", tile)
+    if ctx.dev.cores == 148:
+        assert (_pair_parts(ctx, tokens, out, K), _pair_parts(ctx, tokens, out, K, 2)) == (one, two)
     test_tiles_shared_by_a_cluster(ctx, ora, tile, tokens, out, K, monkeypatch)
+
+
+@pytest.mark.parametrize("tokens,out,K,parts", [(1500, 1280, 5120, 2), (1500, 1280, 4096, 2), (512, 4096, 4096, 2), (500, 1280, 5120, 4),
+                                                (995, 664, 4720, 4)])
+def test_the_planner_shares_tiles_of_long_reductions_among_pairs(ctx, ora, tokens, out, K, parts):
+    """Its own choice, no override, and what it gives."""
+    if ctx.dev.cores == 148:
+        assert _pair_parts(ctx, tokens, out, K) == parts
+    rng = np.random.default_rng(tokens + K)
+    X, Wt, b = _case(rng, tokens, out, K, scale=0.25)
+    got, ref = linear_gpu(ctx, X, Wt, b, out_dtype=np.float32), ora.linear(X, Wt, b, out_dtype=np.float32)
+    assert relerr(got, ref) < 2e-5, describe(got, ref, 2e-5)             # sqrt(K) eps32
 
 
 def test_plans_made_by_several_threads_agree(ctx):
@@ -569,6 +599,33 @@ def test_unaligned_rows_of_long_products(ctx, ora, tokens, out, K, lda, off, dt)
     jv.matmul_(ctx, y, w, x, bias)
     ctx.synchronize()
     got, ref = y.to_host(), ora.linear(X, Wt, b, out_dtype=dt)
+    tol = 2e-3 if dt == np.float16 else 2e-5             # one rounding step of fp16; sqrt(K) eps32
+    assert relerr(got, ref) < tol, describe(got, ref, tol)
+
+
+# a token block of 16, 32, 48 and 64; rows past a last full round of gemm_rows.cu's, which would be a second launch there
+@pytest.mark.parametrize("tokens,out,K", [(8, 35777, 1200), (16, 16701, 1280), (27, 16701, 1280), (48, 8403, 1100), (61, 8403, 1100)])
+@pytest.mark.parametrize("dt", [np.float16, np.float32])
+@pytest.mark.parametrize("epi,with_bias", [("gelu", True), ("relu", False), ("identity", False)])
+def test_unaligned_rows_of_long_products_end_in_their_activation(ctx, ora, tokens, out, K, dt, epi, with_bias):
+    """In one launch; A and the output one element into allocations whose neighbours hold NaN."""
+    rng = np.random.default_rng(out + tokens)
+    X, Wt, b = _case(rng, tokens, out, K, scale=0.25)
+    pad = np.full(K * out + 16, np.nan, np.float16)
+    pad[1:1 + K * out] = Wt.reshape(-1)
+    base, x, bias = ctx.toback(pad), ctx.toback(X), ctx.toback(b) if with_bias else None
+    w = jv.DeviceArray(ctx, base.ptr + 2, np.float16, (out, K), owner=base)
+    dest = ctx.allocate(dt, out * tokens + 2)
+    ctx.fill_bytes(dest, 0xFF)
+    y = jv.DeviceArray(ctx, dest.ptr + np.dtype(dt).itemsize, dt, (out, tokens), owner=dest)
+    before = ctx.launch_count()
+    jv.matmul_(ctx, y, w, x, bias, epi=epi)
+    if ctx.dev.cores == 148:
+        assert ctx.launch_count() - before == 1
+    ctx.synchronize()
+    flat = dest.to_host()
+    got, ref = flat[1:-1].reshape(tokens, out), ora.linear(X, Wt, b if with_bias else None, epi=epi if epi != "identity" else "none", out_dtype=dt)
+    assert np.isnan(flat[0]) and np.isnan(flat[-1]), "wrote outside the output"
     tol = 2e-3 if dt == np.float16 else 2e-5             # one rounding step of fp16; sqrt(K) eps32
     assert relerr(got, ref) < tol, describe(got, ref, tol)
 

@@ -51,6 +51,26 @@ def test_matches_the_allocating_entry_point_twice_in_a_row(ctx, geom):
         assert np.max(np.abs(got - ref)) / np.max(np.abs(ref)) < 5e-3, f"round {round_}"
 
 
+@pytest.mark.parametrize("W,H,Cin,Cout", [(123, 125, 600, 64), (149, 149, 960, 10), (131, 129, 1280, 31), (105, 123, 784, 47)])
+def test_large_images_off_eight_pixels_have_a_bias_per_channel(ctx, W, H, Cin, Cout):
+    """A 1 x 1 convolution whose pixels are a product's unaligned rows and whose channels its tokens: 64, 10, 31 and 47 of them."""
+    L = _lib.lib()
+    rng = np.random.default_rng(W + Cin)
+    x = np.float16(rng.standard_normal((Cin, H * W), dtype=np.float32) * 0.5)
+    w = np.float16(rng.standard_normal((Cout, Cin), dtype=np.float32) * 0.1)
+    b = np.float16(rng.standard_normal(Cout) * 4)
+    ref = np.maximum(w.astype(np.float64) @ x.astype(np.float64) + b.astype(np.float64)[:, None], 0)
+    dx, dw, db = ctx.toback(x), ctx.toback(w), ctx.toback(b)
+    for bias, want in ((db, ref), (None, np.maximum(w.astype(np.float64) @ x.astype(np.float64), 0))):
+        out = ctx.allocate(np.float32, W, H, Cout, 1)
+        ctx.fill_bytes(out, 0xFF)
+        _lib.check(L.b200_conv2d_f16_noalloc(ctx.handle, W, H, Cin, 1, 1, 1, Cout, 1, 1, 0, 0, 1, 1, dx.ptr, dw.ptr,
+                                             bias.ptr if bias is not None else None, out.ptr, _lib.F32, _lib.EPI["relu"]))
+        ctx.synchronize()
+        got = out.to_host().astype(np.float64).reshape(want.shape)
+        assert np.max(np.abs(got - want)) / np.max(np.abs(want)) < 2e-5          # sqrt(K) eps32
+
+
 def _stats(c):
     import ctypes as C
     L = _lib.lib()
