@@ -884,9 +884,9 @@ static int launch_ln(b200_ctx* ctx, int64_t groups, int64_t C, const void* a, vo
         else if (vpl <= 5) LN_GO(5);
         else if (vpl <= 6) LN_GO(6);
         else if (vpl <= 8) LN_GO(8);
-        else if (nvec <= 3 * LN_WIDE_THREADS) LN_GO_WIDE(3);
+        else if (sizeof(InT) == 2 && nvec <= 3 * LN_WIDE_THREADS) LN_GO_WIDE(3);
         else if (nvec <= 4 * LN_WIDE_THREADS) LN_GO_WIDE(4);
-        else if (nvec <= 6 * LN_WIDE_THREADS) LN_GO_WIDE(6);
+        else if (sizeof(InT) == 2 && nvec <= 6 * LN_WIDE_THREADS) LN_GO_WIDE(6);
         else LN_GO_WIDE(8);
 #undef LN_GO_WIDE
 #undef LN_GO
