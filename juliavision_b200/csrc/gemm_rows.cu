@@ -4,8 +4,8 @@
 // misalignment) times a handful of tokens, where reading A once is all that should be paid.
 //
 // What bounds it: reading A, then the loads' latency (the accumulators leave room for fewer blocks per SM).  Measured
-// against the one-thread-per-output kernel that ran these before (whole calls, B200): 17 x 1337 x 712 61 -> 8.6 us; 5 x 35519 x 1280
-// takes 20.7 (4.4 TB/s of A).
+// against the one-thread-per-output kernel that ran these before (whole calls, B200): 17 x 1337 x 712 61 -> 8.6 us; 5 x 17579 x 4096
+// takes 31.4 (4.6 TB/s of A).
 //
 // Columns k and k + 8 of A are 8 * lda * 2 bytes apart, a multiple of 16, so all columns k = w (mod 8) sit at the same
 // offset s_w from a 16-byte boundary.  Warp w of a CTA takes exactly those columns and keeps its accumulators aligned
@@ -47,7 +47,7 @@ template <int NT> struct GrCfg {
 };
 
 // Out of line, and not called for nothing, in the two-tile form: inlined, its registers change the main loop's (115 for 96), 9 x
-// 45001 x 2000 61.1 -> 62.8 us.  The other forms lose by it (4 x 20001 x 1280 18.8 -> 19.5).
+// 45001 x 2000, which gemm_rows_tc.cu takes now, 61.1 -> 62.8 us.  The other forms lose by it (4 x 20001 x 1280 18.8 -> 19.5).
 __device__ __noinline__ float gr_act(int epi, float v) { return apply_act(epi, v); }
 
 // grid (K parts, row blocks, token blocks), the K parts of a row block forming a cluster; 256 threads.  TWO: one of two

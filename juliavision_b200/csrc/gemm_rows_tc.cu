@@ -333,22 +333,33 @@ static int gt_launch(b200_ctx* ctx, const GrParams& g) {
 }
 
 // This form turns all of B in every CTA and ends with a sum that nothing hides, some 4 us of a call; A has to be long enough to pay for
-// it, more so for few tokens, whose row blocks cost gemm_rows.cu little.  Both sides, us:
-// 5 tokens: x 51865 x 1280 32.4 -> 26.7, x 35841 x 1160 24.9 -> 23.3, x 40001 x 1000 22.7 -> 22.3, x 51865 x 384 15.6 -> 16.8,
-//   x 300001 x 136 45 -> 69;  16: x 51865 x 1280 47.7 -> 27.4, x 24001 x 1200 25.6 -> 19.2, x 111865 x 256 33.4 -> 33.6,
-//   x 151865 x 72 31 -> 41;  32: x 51865 x 1280 62.9 -> 29.5, x 12001 x 1000 16.7 -> 12.9;  48: x 51865 x 1280 129 -> 33.4,
-//   x 9001 x 1280 27.2 -> 15.5;  64: x 51865 x 1280 139 -> 46.0, x 9001 x 1280 28.7 -> 19.9.
-// And a CTA has to have rows: 16 x 2001 x 4800, 16 rows a CTA, 15.0 -> 34.4.
+// it, more so for few tokens, whose row blocks cost gemm_rows.cu little.  B stays in shared memory, so a long reduction takes the ring's
+// room, and then the copies stand.  By gemm_rows.cu and by this form, us:
+// 5 tokens: x 51865 x 1280 32.4, 26.7; x 54687 x 768 25.2, 23.6; x 42001 x 1000 23.2, 23.5; x 51865 x 384 15.6, 16.8; x 300001 x 136 45, 69.  Where
+//   the ring is not whole: x 13125 x 3200 24.8, 25.8; x 17579 x 4096 31.4, 34.7; x 8301 x 5120 20.9, 41.6.  And many rows, which the other
+//   form reads at 4.8 TB/s and this one at 4.0: x 171875 x 1280 92.5, 95.9; x 300001 x 1000 135, 153;
+// 16: x 51865 x 1280 47.7, 27.4; x 24001 x 1200 25.6, 19.2; x 147657 x 256 42.5, 45.6; x 112251 x 259 41.3, 37.0; x 10921 x 4150 50.6, 46.5;
+//   x 11825 x 4879 59.8, 60.9; x 14407 x 5162 63.6, 72.1;
+// 32: x 51865 x 1280 62.9, 29.5; x 14765 x 2560 34.8, 29.1;  18: x 11641 x 2764 49.9, 53.9;
+// 48: x 51865 x 1280 129, 33.4; x 9001 x 1280 27.2, 15.5;  64: x 51865 x 1280 139, 46.0; x 9001 x 1280 28.7, 19.9, and where B leaves the
+//   least ring x 9001 x 1350 41.4, 42.8 (49 tokens 36.4, 42.0), x 15121 x 1321 59.6, 44.0;
+// A read twice, by blocks of 32: 64 x 17001 x 2000 73.9, 40.4; 40 x 17007 x 2315 91.2, 71.6; 34 x 12241 x 2406 64.0, 67.5; 48 x 9951 x 2199 57.9, 68.9;
+//   60 x 18749 x 2759 136, 151.
+// Over 1700 products of 2 to 150 tokens drawn beside those that the lines were laid by, no call is more than 1.05 times as slow as by
+// gemm_rows.cu; of the others 2 x 36001 x 2000 (34.0, 36.9: little more there than one round of row blocks).
+// The lines of 9 and 21 million elements do not lie where the forms meet but above: 33 x 16577 x 520 (8.6 million) takes 27 us and would
+// take 13, 32 x 12001 x 1000 16.7 and 12.9.  Under them the other form's two launches are what runs and is tested.
+// And a CTA has to have rows: 16 x 2001 x 4800, 16 rows a CTA, 15.0, 34.4.
 int gemm_rows_tc_tokens(const b200_ctx* ctx, int64_t M, int64_t N, int64_t K) {
-    const int64_t per = cdiv(N, cdiv(N, 64));   // tokens of a token block
-    if (M < 56 * (int64_t)ctx->prop.multiProcessorCount || K < (N <= 8 ? 768 : N <= 16 ? 256 : 64) ||
-        M * K < (N <= 8 ? 40000000 : N <= 32 ? 21000000 : 9000000))
-        return 0;
-    if (per <= 16 && GtCfg<16>::fits(K)) return 16;
-    if (per <= 32) return GtCfg<32>::fits(K) ? 32 : 0;
+    const int64_t per = cdiv(N, cdiv(N, 64)), steps = cdiv(K, 128), size = M * K;   // tokens of a token block
+    if (M < 56 * (int64_t)ctx->prop.multiProcessorCount) return 0;
+    if (N <= 8) return K >= 768 && size >= 45000000 && M < 170000 && GtCfg<16>::ring(K, 2) >= GT_RING ? 16 : 0;
+    if (N <= 16) return K > 256 && steps <= 36 && size >= 21000000 ? 16 : 0;
+    if (K < 64 || size < (N <= 32 ? 21000000 : 9000000)) return 0;
+    if (N <= 32) return steps <= 21 ? 32 : 0;
     if (per <= 48 && GtCfg<48>::fits(K)) return 48;
-    if (GtCfg<64>::fits(K)) return 64;
-    return M * K >= 21000000 && GtCfg<32>::fits(K) ? 32 : 0;   // A twice: 64 x 17001 x 2000 73.9 -> 40.4
+    if (GtCfg<64>::fits(K) && (steps <= 10 || size >= 16000000)) return 64;
+    return steps <= 20 && size >= (steps > 16 && N <= 64 ? 30000000 : 21000000) ? 32 : 0;
 }
 
 int gemm_rows_tc_launch(b200_ctx* ctx, const GrParams& p, int tokens, bool half_out) {

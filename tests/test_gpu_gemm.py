@@ -559,9 +559,12 @@ def test_gelu_of_large_negative_values_goes_to_zero(ctx):
 
 
 # (tokens, out features, K, launches on 148 SMs): what is left past the full rounds is one block, some, exactly half a round, just
-# more than that; of a short reduction, which is not split; split in two, four and eight parts, some of those without a step
+# more than that; of a short reduction, which is not split; split in two, four and eight parts, some of those without a step; weights
+# that are long, and which the form in tensor memory would take longer for: reductions that leave it a small ring, very many rows
 @pytest.mark.parametrize("tokens,out,K,launches", [(2, 35525, 512, 2), (16, 35641, 515, 2), (19, 20001, 1024, 2), (33, 16577, 520, 2),
-                                                   (5, 53279, 384, 1), (5, 53279, 512, 2), (5, 53401, 512, 1), (33, 8289, 2100, 2)])
+                                                   (5, 53279, 384, 1), (5, 53279, 512, 2), (5, 53401, 512, 1), (33, 8289, 2100, 2),
+                                                   (5, 37001, 3300, 2), (2, 250001, 900, 2), (16, 16801, 5000, 2),
+                                                   (20, 17001, 2800, 2), (60, 9001, 1350, 2), (36, 9951, 2199, 2)])
 @pytest.mark.parametrize("dt", [np.float16, np.float32])
 def test_unaligned_rows_past_the_last_full_round(ctx, ora, tokens, out, K, launches, dt):
     """Row blocks that fill the GPU once or more and leave some: at most half a round of them is a launch of its own, split
@@ -580,7 +583,7 @@ def test_unaligned_rows_past_the_last_full_round(ctx, ora, tokens, out, K, launc
 # (tokens, out features, K, elements between columns, elements off the boundary): a token block of 16, 32, 48 and 64, and more than
 # one; the last class without its last column, a reduction that ends inside sixteen of a class, and B off 16 bytes; one row block a
 # CTA and several, the last one cut; rows 0 ... 7 elements off in turn, or all the same; few columns to a class, and many
-@pytest.mark.parametrize("tokens,out,K,lda,off", [(5, 50001, 801, 50003, 1), (8, 36000, 1112, 36000, 1), (9, 28673, 736, 28675, 7),
+@pytest.mark.parametrize("tokens,out,K,lda,off", [(5, 56251, 801, 56253, 1), (8, 40501, 1112, 40501, 1), (7, 15001, 3072, 15003, 5), (9, 28673, 736, 28675, 7),
                                                   (16, 85001, 257, 85004, 2), (17, 21001, 1024, 21001, 0), (32, 328001, 65, 328002, 5),
                                                   (33, 8291, 1103, 8297, 3), (48, 9001, 1280, 9001, 1), (49, 140001, 66, 140003, 6),
                                                   (64, 9001, 1280, 9003, 0), (50, 11003, 2000, 11005, 4), (70, 9005, 1000, 9006, 3)])
@@ -604,7 +607,7 @@ def test_unaligned_rows_of_long_products(ctx, ora, tokens, out, K, lda, off, dt)
 
 
 # a token block of 16, 32, 48 and 64; rows past a last full round of gemm_rows.cu's, which would be a second launch there
-@pytest.mark.parametrize("tokens,out,K", [(8, 35777, 1200), (16, 16701, 1280), (27, 16701, 1280), (48, 8403, 1100), (61, 8403, 1100)])
+@pytest.mark.parametrize("tokens,out,K", [(8, 37601, 1200), (16, 16701, 1280), (27, 16701, 1280), (48, 8403, 1100), (61, 8403, 1100)])
 @pytest.mark.parametrize("dt", [np.float16, np.float32])
 @pytest.mark.parametrize("epi,with_bias", [("gelu", True), ("relu", False), ("identity", False)])
 def test_unaligned_rows_of_long_products_end_in_their_activation(ctx, ora, tokens, out, K, dt, epi, with_bias):
