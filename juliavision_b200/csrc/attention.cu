@@ -1160,13 +1160,13 @@ static const AttRooms& att_rooms(b200_ctx* ctx) {
 // (44 of 45, 12 heads x 4096 x 4096 x 72: 89.5 -> 103.5, two rounds of them).  Masked tails go on merging, their CTAs' ends lie
 // further apart (12 heads x 4096 x 4096 111.6 -> 117.3, 14 x 2900 86.1 -> 89.8; short ones would gain, 38 x 1024 x 640 31.1 -> 29.4).
 struct AttSplit { int parts; bool join; };
-static AttSplit att_split(b200_ctx* ctx, int64_t pairs, int64_t nblk, int64_t Lq, int64_t E, bool masked, int64_t waves) {
+static AttSplit att_split(b200_ctx* ctx, int64_t pairs, int64_t nblk, int64_t Lq, int64_t E, bool masked, int64_t waves, double staged) {
     struct Cost { double block, load, join, merge, rows; };
     static const Cost costs[5] = {{1.35, 0.37, 3.65, 4.15, 0.035}, {1.44, 0.57, 4.4, 4.75, 0.038}, {1.83, 0.46, 4.7, 5.4, 0.038},
                                   {2.07, 0.56, 3.9, 5.15, 0.035}, {2.44, 0.77, 4.7, 5.6, 0.042}};
     const Cost& c = costs[masked ? 3 + (E > 64) : (E > 64) + (E > 80)];
     const int64_t sms = ctx->prop.multiProcessorCount;
-    auto walk = [&](int64_t n) { return (double)cdiv(nblk, n) * (c.block + c.load * (double)(pairs * n) / (double)sms); };
+    auto walk = [&](int64_t n) { return (double)cdiv(nblk, n) * (c.block + staged + c.load * (double)(pairs * n) / (double)sms); };
     const AttRooms& rooms = att_rooms(ctx);
     AttSplit best = {1, false};
     double least = walk(1);
@@ -1219,50 +1219,79 @@ mask_rows_kernel(const __half* __restrict__ mask, uint4* __restrict__ out, int L
     }
 }
 
+// What a mask's way to the softmax costs, in us.
+// The softmax warps' own staging: `block` for every key block of a CTA, 0.3 of it for the first, whose entries are waited for either way.
+// 1.1 by copies of 8 bytes, 1.4 so beside wider heads, 2.2 by words, less for the warps of a tile that have no rows (0.55 of it for 32
+// queries); entry by entry, keys apart, 6 and for the first as well.
+// `copy`: a launch that lays the rows on 16-byte boundaries for the tensor map, 2.2, 0.9 per million entries and 0.1 for every trip of a
+// row's warp, 256 keys (keys apart 2 and 8 per million).
+// Fitted to 700 masks of 9 to 3900 queries and 50 to 4500 keys, either way taken: the cheaper one by this is 0.2 % off in the mean and 1.07
+// at worst.  20 heads x 1500 x 1500 42.1 -> 36.9 us, 2 x 8 x 1001 x 1001 31.1 -> 26.7, 4 x 20 x 1001 x 1001 x 32 88.8 -> 62.6; 2 x 2001 x
+// 2001 x 128 would go 24.6 -> 26.8, 8 x 100 x 3001 16.2 -> 17.9, 16 x 35 x 4391 x 128 26.5 -> 32.2 and one block, 2 x 32 x 575 x 50, 14.4 -> 16.3.
+// Keys apart, 20 x 1500 x 1500 193 -> 92, 4 x 300 x 300 44.6 -> 14.5.  The workspace keeps what a copy took and half as much again, so
+// there is a most to it: 256 MiB are 11584 x 11584 entries, and a larger mask is read in place, as every one that is not copied.
+constexpr int64_t MASK_COPY_MOST = (int64_t)256 << 20;
+struct MaskWay {
+    bool lies;      // rows on 16-byte boundaries: the map is over the mask itself
+    bool apart;
+    double block, copy;
+    int64_t rows, bytes;   // of a copy
+    bool copied(int64_t blocks, int64_t walks) const {
+        return block * ((double)blocks - (apart ? 0.0 : 0.7 * (double)walks)) >= copy && bytes <= MASK_COPY_MOST;
+    }
+};
+static MaskWay mask_way(const __half* bptr, const int64_t* bs, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B, int mask) {
+    const int64_t ext[4] = {Lk, Lq, bs[2] != 0 ? H : 1, bs[3] != 0 ? B : 1};
+    MaskWay w;
+    w.lies = (bs[0] == 1 || Lk == 1) && reinterpret_cast<uintptr_t>(bptr) % 16 == 0;
+    for (int d = 1; d < 4; ++d) w.lies = w.lies && (ext[d] == 1 || (bs[d] > 0 && bs[d] % 8 == 0 && bs[d] < (1ll << 38)));
+    w.apart = mask == MASK_DIRECT;
+    w.rows = Lq * ext[2] * ext[3];
+    w.bytes = w.rows * cdiv(Lk, 8) * 16;
+    const double entries = (double)(w.rows * Lk);
+    if (w.apart) {
+        w.block = Lq < 2 * ATT_BR ? 6.0 * (double)Lq / (2 * ATT_BR) : 6.0;
+        w.copy = 2.0 + 8e-6 * entries;
+    } else {
+        w.block = (mask == MASK_WORDS ? 2.2 : E <= 64 ? 1.1 : 1.4) * (Lq < ATT_BR ? 0.4 + 0.6 * (double)Lq / ATT_BR : 1.0);
+        w.copy = 2.2 + 0.9e-6 * entries + 0.1 * (double)cdiv(Lk, 256);
+    }
+    return w;
+}
+
 // The mask's tensor map, over the mask itself where its rows lie on 16-byte boundaries, else over a copy of it whose rows do
 // where that is worth a launch.  Leaves p->mask as it is where neither is to be had.
-// The copy costs 2 us and 0.9 per million entries; a CTA gains 0.95 us a key block over copies of 8 bytes by the softmax's own
-// warps (1.6 with its wider heads, and over copies of words), less where its 256 rows are not all there.  20 heads x 1500 x 1500
-// 42.1 -> 36.9 us, 2 x 8 x 1001 x 1001 31.1 -> 26.7, 4 x 20 x 1001 x 1001 x 32 88.8 -> 62.6; 2 x 2001 x 2001 x 128 would
-// go 24.6 -> 26.8 and 8 x 100 x 3001 16.2 -> 17.9.  Keys apart, 20 x 1500 x 1500 193 -> 92, 4 x 300 x 300 44.6 -> 14.5.
-// The workspace keeps what a copy took and half as much again, so there is a most to it: 256 MiB are 11584 x 11584 entries, and a
-// larger mask is read in place, as every one that is not copied.  `serial`: key blocks a CTA walks.
-constexpr size_t MASK_COPY_MOST = (size_t)256 << 20;
-static int mask_map(b200_ctx* ctx, const __half* bptr, const int64_t* bs, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B,
-                    int64_t serial, AttnParams* p, CUtensorMap* tm) {
-    const uint64_t Hm = bs[2] != 0 ? (uint64_t)H : 1, Bm = bs[3] != 0 ? (uint64_t)B : 1;
-    const int64_t ext[4] = {Lk, Lq, (int64_t)Hm, (int64_t)Bm};
-    uint64_t dims[4] = {(uint64_t)Lk, (uint64_t)Lq, Hm, Bm}, str[3];
-    bool lies = (bs[0] == 1 || Lk == 1) && reinterpret_cast<uintptr_t>(bptr) % 16 == 0;
-    uint64_t dense = (uint64_t)(Lk + 7) / 8 * 16;   // a legal stride for an axis of extent one
-    for (int d = 1; d < 4; ++d) {
-        lies = lies && (ext[d] == 1 || (bs[d] > 0 && bs[d] % 8 == 0 && bs[d] < (1ll << 38)));
-        str[d - 1] = ext[d] == 1 ? dense : (uint64_t)bs[d] * 2;
+// Nor where many CTAs fetch boxes of few keys, rows of parts of a line, the same ones at the same time, and each waits for its first: 80
+// items of 144 queries x 8 keys 7.2 us staged, 10.7; x 24 7.3, 9.0; of 29 queries x 72 5.8, 6.7; x 64 and x 128 gain (0.95, 0.94 of
+// the staged time), and so do launches of up to some 48 items (16 x 99 x 96: 5.5, 5.0).
+// `blocks`: key blocks a CTA walks, `walks`: from how many first ones; `items`: of two tiles.
+static int mask_map(b200_ctx* ctx, const __half* bptr, const int64_t* bs, const MaskWay& way, int64_t Lq, int64_t Lk, int64_t H, int64_t B,
+                    int64_t blocks, int64_t walks, int64_t items, AttnParams* p, CUtensorMap* tm) {
+    const int64_t ext[4] = {Lk, Lq, bs[2] != 0 ? H : 1, bs[3] != 0 ? B : 1};
+    uint64_t dims[4], str[3], dense = (uint64_t)cdiv(Lk, 8) * 16;   // a legal stride for an axis of extent one
+    for (int d = 0; d < 4; ++d) {
+        dims[d] = (uint64_t)ext[d];
+        if (d == 0) continue;
+        str[d - 1] = way.lies && ext[d] != 1 ? (uint64_t)bs[d] * 2 : dense;
         dense *= (uint64_t)ext[d];
     }
+    if (way.lies && items > 48 && Lk < 128 && Lk != 64 && (Lk < 64 || Lq < ATT_BR)) return B200_OK;
     const void* base = bptr;
-    if (!lies) {
-        const int64_t rows = Lq * (int64_t)(Hm * Bm), n8 = (Lk + 7) / 8;
-        const size_t bytes = (size_t)(rows * n8) * 16, mark = ctx->ws_used;
-        const bool apart = p->mask == MASK_DIRECT;
-        const double gain = (apart ? 6.0 : p->mask == MASK_EIGHTS && E <= 64 ? 0.95 : 1.6) * (double)serial;
+    if (!way.lies) {
+        const size_t mark = ctx->ws_used;
         void* ws = nullptr;
-        if (bytes > MASK_COPY_MOST ||
-            gain * (Lq < 2 * ATT_BR ? (double)Lq / (2 * ATT_BR) : 1.0) < 2.0 + (apart ? 8e-6 : 0.9e-6) * (double)(rows * Lk)) {
+        if (!way.copied(blocks, walks)) {
             // A context's first masked call leaves it a workspace, if only the smallest: one recorded later finds room for a small copy.
             if (ctx->ws_buf == nullptr && ws_scratch(ctx, 0, &ws) == B200_OK) ctx->ws_used = mark;
             return B200_OK;
         }
-        const int rc = ws_scratch(ctx, bytes, &ws);
+        const int rc = ws_scratch(ctx, (size_t)way.bytes, &ws);
         if (rc == B200_ENOMEM) return B200_OK;
         if (rc) return rc;
-        B200_CUDA(launch_dep(mask_rows_kernel, dim3((unsigned)cdiv(rows, 8), 1, 1), dim3(256, 1, 1), 0, ctx->stream, 1, bptr, (uint4*)ws,
-                             (int)Lq, (int)Lk, rows, (int)Hm, bs[0], bs[1], bs[2], bs[3]));
+        B200_CUDA(launch_dep(mask_rows_kernel, dim3((unsigned)cdiv(way.rows, 8), 1, 1), dim3(256, 1, 1), 0, ctx->stream, 1, bptr, (uint4*)ws,
+                             (int)Lq, (int)Lk, way.rows, (int)ext[2], bs[0], bs[1], bs[2], bs[3]));
         ctx->launches++;
         base = ws;
-        str[0] = (uint64_t)n8 * 16;
-        str[1] = str[0] * (uint64_t)Lq;
-        str[2] = str[1] * Hm;
     }
     uint32_t box[4] = {64, ATT_BR, 1, 1};
     const int rc = make_tmap(ctx, tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, base, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
@@ -1411,6 +1440,8 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     p.mask = !(bs[0] == 1 || Lk == 1) ? MASK_DIRECT
              : reinterpret_cast<uintptr_t>(bptr) % 8 == 0 && bs[1] % 4 == 0 && bs[2] % 4 == 0 && bs[3] % 4 == 0 ? MASK_EIGHTS : MASK_WORDS;
     CUtensorMap tm = tq;   // not read unless there is a mask
+    MaskWay way = {};
+    if (bptr) way = mask_way(bptr, bs, E, Lq, Lk, H, B, p.mask);
     const int64_t nblk_all = cdiv(Lk, block);
     const int64_t item_rows = single ? ATT_BR : 2 * ATT_BR;
     auto launch = [&](dim3 grid, int cluster = 1) -> cudaError_t {
@@ -1446,7 +1477,8 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     if (!single) {
         int64_t ntail = 0, ns = 1;
         if (2 * pairs <= sms || tail) {
-            const AttSplit cut = att_split(ctx, tail ? rem : pairs, nblk_all, Lq, E, bptr != nullptr, tail ? pairs / sms : 0);
+            const double staged = bptr && !way.lies && !way.apart && !way.copied(cdiv(pairs, sms) * nblk_all, cdiv(pairs, sms)) ? way.block : 0.0;
+            const AttSplit cut = att_split(ctx, tail ? rem : pairs, nblk_all, Lq, E, bptr != nullptr, tail ? pairs / sms : 0, staged);
             if (cut.join) {
                 join = cut.parts;
             } else {
@@ -1472,7 +1504,7 @@ int b200_attention_f16_bias(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, in
     if (bptr) {
         const int64_t waves = join > 1 ? (tail ? pairs / sms : 0) : p.nsplit > 1 ? (pairs - p.ntail) / sms : cdiv(pairs, sms);
         const int64_t serial = waves * nblk_all + (join > 1 ? cdiv(nblk_all, join) : p.nsplit > 1 ? cdiv(nblk_all, p.nsplit) : 0);
-        if ((rc = mask_map(ctx, bptr, bs, E, Lq, Lk, H, B, serial, &p, &tm))) return rc;
+        if ((rc = mask_map(ctx, bptr, bs, way, Lq, Lk, H, B, serial, waves + (join > 1 || p.nsplit > 1), pairs, &p, &tm))) return rc;
     }
     if (join > 1) {
         p.ntail = (int)(tail ? rem : pairs);

@@ -578,7 +578,8 @@ def test_reference_point_that_moves_in_later_blocks(ctx, E, Lq, Lk):
     assert np.abs(got - ref).max() < vmax * (2.0 ** -11 + Lk * 2.0 ** -25 + 1e-5)
 
 
-@pytest.mark.parametrize("B,H,Lq,Lk,E", [(1, 8, 300, 1001, 64), (2, 6, 513, 640, 56), (1, 20, 129, 1500, 72), (3, 4, 260, 2050, 128), (1, 6, 1000, 127, 64)])
+@pytest.mark.parametrize("B,H,Lq,Lk,E", [(1, 8, 300, 1001, 64), (2, 6, 513, 640, 56), (1, 20, 129, 1500, 72), (3, 4, 260, 2050, 128), (1, 6, 1000, 127, 64),
+                                           (2, 30, 144, 24, 64), (2, 30, 29, 72, 80)])
 @pytest.mark.parametrize("planes", ["all", "batch", "head", "keys"])
 def test_however_a_mask_lies_the_result_is_the_same(ctx, ora, B, H, Lq, Lk, E, planes):
     """The same mask on 16-byte boundaries (read through a tensor map where its strides allow one), behind an odd number of
