@@ -810,10 +810,13 @@ static bool ln_fills(const b200_ctx* ctx, int64_t groups, int rows, int lpg, int
 }
 
 // Vectors a thread of ln_split_kernel, 0 for rows that stay with the other kernels.  Past 512 vectors 256 threads a row are as fast or
-// faster: in fp32 2400 x 2600 12.6 us, 13.8, 11111 x 3600 50.5, 52.9; in fp16 see ln_wide_kernel.
+// faster: in fp32 2400 x 2600 12.6 us, 13.8, 11111 x 3600 50.5, 52.9; in fp16 see ln_wide_kernel.  fp32, six and four: 50000 x 1032 69, 77,
+// 20000 x 1280 34.6, 36.3, 2400 x 1664 8.4, 7.8, 3200 x 2048 13.8, 12.6.  By the row's width alone, so that its bits do not depend on
+// the rows beside it; what a launch of some 19 rows an SM of the narrowest loses, one round of warps and two of blocks (2800 x 2048 in
+// fp16 5.0 us, 6.7; 3200 x 1032 in fp32 5.7, 7.6), it gives back at any other size (64 rows 4.0, 3.2; 20000 35.8, 32.4).
 template <typename InT> static int ln_split(int nvec) {
     if (nvec > 512) return 0;
-    if (sizeof(InT) == 4) return nvec > 256 ? 6 : 0;
+    if (sizeof(InT) == 4) return nvec <= 256 ? 0 : nvec <= 352 ? 6 : 4;
     return nvec <= 224 ? 0 : cdiv(cdiv(nvec, 5), 32) < cdiv(cdiv(nvec, 4), 32) ? 5 : 4;
 }
 
