@@ -1220,13 +1220,13 @@ mask_rows_kernel(const __half* __restrict__ mask, uint4* __restrict__ out, int L
 }
 
 // What a mask's way to the softmax costs, in us.
-// The softmax warps' own staging: `block` for every key block of a CTA, 0.3 of it for the first, whose entries are waited for either way.
-// 1.1 by copies of 8 bytes, 1.4 so beside wider heads, 2.2 by words, less for the warps of a tile that have no rows (0.55 of it for 32
+// The softmax warps' own staging: `block` for every key block of a CTA, 0.2 of it for the first, whose entries are waited for either way.
+// 1.1 by copies of 8 bytes, 1.2 so beside wider heads, 2.5 by words, less for the warps of a tile that have no rows (0.4 of it for 32
 // queries); entry by entry, keys apart, 6 and for the first as well.
-// `copy`: a launch that lays the rows on 16-byte boundaries for the tensor map, 2.2, 0.9 per million entries and 0.1 for every trip of a
+// `copy`: a launch that lays the rows on 16-byte boundaries for the tensor map, 1.4, 0.9 per million entries and 0.3 for every trip of a
 // row's warp, 256 keys (keys apart 2 and 8 per million).
-// Fitted to 700 masks of 9 to 3900 queries and 50 to 4500 keys, either way taken: the cheaper one by this is 0.2 % off in the mean and 1.07
-// at worst.  20 heads x 1500 x 1500 42.1 -> 36.9 us, 2 x 8 x 1001 x 1001 31.1 -> 26.7, 4 x 20 x 1001 x 1001 x 32 88.8 -> 62.6; 2 x 2001 x
+// Fitted to 930 masks of 9 to 3900 queries and 50 to 9000 keys, either way taken: the cheaper one by this is 0.4 % off in the mean and 1.13
+// at worst (always the copy 5 %, never 7 %).  20 heads x 1500 x 1500 42.1 -> 36.9 us, 2 x 8 x 1001 x 1001 31.1 -> 26.7, 4 x 20 x 1001 x 1001 x 32 88.8 -> 62.6; 2 x 2001 x
 // 2001 x 128 would go 24.6 -> 26.8, 8 x 100 x 3001 16.2 -> 17.9, 16 x 35 x 4391 x 128 26.5 -> 32.2 and one block, 2 x 32 x 575 x 50, 14.4 -> 16.3.
 // Keys apart, 20 x 1500 x 1500 193 -> 92, 4 x 300 x 300 44.6 -> 14.5.  The workspace keeps what a copy took and half as much again, so
 // there is a most to it: 256 MiB are 11584 x 11584 entries, and a larger mask is read in place, as every one that is not copied.
@@ -1237,7 +1237,7 @@ struct MaskWay {
     double block, copy;
     int64_t rows, bytes;   // of a copy
     bool copied(int64_t blocks, int64_t walks) const {
-        return block * ((double)blocks - (apart ? 0.0 : 0.7 * (double)walks)) >= copy && bytes <= MASK_COPY_MOST;
+        return block * ((double)blocks - (apart ? 0.0 : 0.8 * (double)walks)) >= copy && bytes <= MASK_COPY_MOST;
     }
 };
 static MaskWay mask_way(const __half* bptr, const int64_t* bs, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B, int mask) {
@@ -1253,8 +1253,8 @@ static MaskWay mask_way(const __half* bptr, const int64_t* bs, int64_t E, int64_
         w.block = Lq < 2 * ATT_BR ? 6.0 * (double)Lq / (2 * ATT_BR) : 6.0;
         w.copy = 2.0 + 8e-6 * entries;
     } else {
-        w.block = (mask == MASK_WORDS ? 2.2 : E <= 64 ? 1.1 : 1.4) * (Lq < ATT_BR ? 0.4 + 0.6 * (double)Lq / ATT_BR : 1.0);
-        w.copy = 2.2 + 0.9e-6 * entries + 0.1 * (double)cdiv(Lk, 256);
+        w.block = (mask == MASK_WORDS ? 2.5 : E <= 64 ? 1.1 : 1.2) * (Lq < ATT_BR ? 0.2 + 0.8 * (double)Lq / ATT_BR : 1.0);
+        w.copy = 1.4 + 0.9e-6 * entries + 0.3 * (double)cdiv(Lk, 256);
     }
     return w;
 }
