@@ -27,13 +27,14 @@ namespace b200 {
 
 constexpr int ATT_BR = 128;  // queries per tile (TMEM lanes)
 constexpr int ATT_TILE_BYTES = 128 * 128; // one swizzle atom of an operand tile: 128 rows x 128 B (64 fp16 of E)
-// Two shapes of CTA, chosen by the head dimension, and a third for short keys:
+// Four forms of CTA, by the head dimension, the mask and, the first, by short keys:
 //   EP = 64, NT = 1:           one query tile, key blocks of 64, P over S, 128 tensor-memory columns and 48 KB, so that
 //                              four CTAs share an SM
 //   EP = 64  (E <= 64):        two query tiles of 128 per CTA, K/V rings of 4 stages x 16 KB
 //   EP = 80  (64 < E <= 80):   as EP = 128, but O has 80 columns per tile, which leaves P 48 columns of its own: 96 of a
 //                              block's 128 keys, the other 32 go through shared memory (A operand of the last two steps
-//                              of P V).  8 heads x 4096 x 72: 70.9 us with P over S, 58.0 so; no mask (no room for it)
+//                              of P V).  8 heads x 4096 x 72 replayed: 70.9 us with P over S, 58.5 so (70.6 and 61.7 by
+//                              calls); no mask (no room for it)
 //   EP = 128 (80 < E <= 128, with a mask 64 < E):  two query tiles of 128 per CTA as well; every operand tile is two swizzle atoms along
 //                              E (columns 0-63, 64-127, the second zero-filled past E by the tensor map), S = Q K'
 //                              runs over both, O has 128 columns per tile — S 2 x 128 + O 2 x 128 fill the tensor
@@ -59,7 +60,7 @@ template <int EP, bool BIAS = false, int NT_ = 2> struct AttCfg {
     static_assert(EP != 80 || !BIAS, "a mask leaves no room for the tail of P");
     static constexpr int BC = NT == 2 ? 128 : 64;      // keys per block
     static constexpr int CTAS_PER_SM = NT == 2 ? 1 : 4;
-    static constexpr int THREADS = 128 * NT + 128;     // NT softmax warpgroups, then TMA, UMMA and idle warps
+    static constexpr int THREADS = 128 * NT + 128;     // NT softmax warpgroups, then TMA and UMMA warps and one that fetches the mask or idles
     static constexpr int TMA_WARP = 4 * NT, ISSUE_WARP = 4 * NT + 1;
     // registers of a softmax thread and of the others: (NT x 128 x one + 128 x the other) is what the launch holds
     static constexpr int SOFTMAX_REGS = NT == 2 ? 232 : 96, OTHER_REGS = NT == 2 ? 40 : 32;
@@ -168,12 +169,13 @@ __device__ __forceinline__ void tmem_st16_raw(uint32_t taddr, const uint32_t* r)
 //   warps 0-3  softmax of tile 0, warps 4-7 softmax of tile 1: one thread per query row, the whole
 //              128-score row in registers (these two warpgroups take registers from the third)
 //   warp 8     TMA producer: both Q tiles once, then K and V blocks through the rings of AttCfg
-//   warps 9,10 UMMA issuers, one lane per tile: S_t = Q_t K' and O_t += P_t V per key block;
+//   warps 9,10 UMMA issuers, one warp per tile, which waits together and has one thread issue: S_t = Q_t K' and O_t += P_t V per key block;
 //              the two chains are independent, so the tensor core works on one tile while the
 //              other tile's softmax runs
+//   warp 11    asks for the mask's entries where a tensor map is over them
 // One tile (NT = 1): warps 0-3 its softmax, 64 scores a thread, warp 4 the producer, warp 5 the issuer; four CTAs per SM.
-// P never touches shared memory: the softmax threads write it as packed fp16 into tensor memory and
-// the P V product takes its A operand from there, so the shared-memory port only feeds K and V.
+// P stays out of shared memory, but for a quarter of it at EP = 80: the softmax threads write it as packed fp16 into tensor memory
+// and the P V product takes its A operand from there, so the shared-memory port feeds K and V.
 // BIAS: the scaled score gets an additive fp16 mask before the softmax; a row whose keys are all
 // blocked (-inf everywhere) comes out as zeros, as in attn_softmax (attention.jl:73-100).
 // JOIN: the CTAs an item's keys are cut over are a cluster, which joins their rows through distributed shared memory: an instance of
@@ -189,7 +191,7 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
     constexpr int BC = Cfg::BC, NC = BC / 32;   // keys per block, and per-thread pieces of 32 of them
     constexpr int NT = Cfg::NT;
     // Where P lies over S, everything after P waits for P V: it is issued in two halves of the block, the first under the second
-    // half's exponentials.  8 heads x 4096 x 72: 71.7 -> 70.3 us, 12 x 1500 x 96 32.2 -> 31.7, masked 8 x 2048 x 72 50.6 -> 49.9;
+    // half's exponentials.  12 x 1500 x 96 32.2 -> 31.7 us, masked 8 x 2048 x 72 50.6 -> 49.9 (before the whole warp issued);
     // with columns of its own the turns hide as much and the extra hand-over costs (12 x 4096 x 64: 85.9 -> 88.1).
     constexpr bool HALVES = EP == 128;
     constexpr bool OWN_P = !Cfg::P_IN_S;     // P in columns (and shared memory) of its own
@@ -289,15 +291,15 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // Everything above overlapped the previous kernel's tail; from here on its results are needed.
-    // (A joined tail reads only what its whole pairs' launch has waited for, so it starts as that one's CTAs leave; what follows the
-    // tail on the stream waits for it to end, hence, by the wait at its end, for both.)
+    // (A joined tail reads only what its whole pairs' launch has waited for, and by TMA alone, which reads the L2, so it starts as that
+    // one's CTAs leave; what follows the tail on the stream waits for it to end, hence, by the wait at its end, for both.)
     if (!JOIN || p.pair_ctas == 0) grid_dep_wait();
     grid_dep_launch();
 
     bool met = false;   // joining: this warp has passed the barrier behind which the rows are there
 
     // Register budget: the two softmax warpgroups hold a full score row per thread; the third
-    // warpgroup (one TMA lane, one UMMA lane, two idle warps) needs almost nothing and hands its
+    // warpgroup (a TMA lane, the warps that issue and the mask's lane) needs almost nothing and hands its
     // share over (setmaxnreg at the head of each role's branch).
     if (warp == 4 * NT + 3 || (NT == 1 && warp == 6)) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::OTHER_REGS));
@@ -452,14 +454,16 @@ attention_f16_tc_kernel(const __grid_constant__ CUtensorMap tmapQ,
             bool ok = true;
             // Both tiles take the same time per block, and in step both would want the MUFU pipe in the same half of
             // every period and leave it idle in the other.  Where P has a place of its own and there is no mask it is enough that tile 1
-            // starts behind: nothing brings the two together again (12 heads x 4096 x 64: 79.6 us, 84.5 in step, 86.3 with a turn
-            // handed over every block; started after the last quarter instead of the first, 8 x 4096 x 72 takes 63.4 for 58.0).
+            // starts behind: nothing brings the two together again (12 heads x 4096 x 64, its tail not joined: 79.6 us, 84.5 in step, 86.3
+            // with a turn handed over every block).
             // With P over S, or a mask, a tile's block is one long chain and the exponential phases take turns (tile 0 block j, tile 1
             // block j, tile 0 block j+1, ...): while one tile owns the MUFU pipe the other does its max / rescale / waits
             // and its tensor-core work runs (16 heads x 2048 x 128: 33.7 us, 38.5 without).
             const bool pingpong = ntiles == 2;
-            // After which quarter of its exponentials a tile passes the turn (the 32-layer encoder: 3290 us after the first, 3240 after the
-            // third; 12 heads x 4096 x 64 alone 79.6 and 80.3).
+            // After which quarter of its exponentials a tile passes the turn.  The mean over 12 shapes of 2 to 40 heads and 800 to 16384
+            // keys, after the first, second, third and last: 64 wide 1, 1.05, 0.99, 0.98, and the 32-layer encoder 3189 us, 3234, 3148, 3150;
+            // 72 wide 1, 0.99, 1.03, 1.04 (8 heads x 4096: 58.5, 58.2, 62.7, 63.5); 128 wide 1, 0.99, 0.96, 0.96; masked 64 wide alike within 1 %,
+            // 80 wide 1, 0.99, 0.95, 0.97.
             constexpr int TURN_AT = !FREE ? 3 : EP == 64 ? 2 : 0;
             // A mask no tensor map is over, its keys contiguous: each warp copies the next block's entries of its own 32 rows to
             // shared memory (cp.async, a row's entries across the lanes) while it works on this block, and every thread
@@ -1184,8 +1188,9 @@ static AttSplit att_split(b200_ctx* ctx, int64_t pairs, int64_t nblk, int64_t Lq
     return best;
 }
 
-// A mask whose rows lie on 16-byte boundaries, zero-filled to a multiple of 8 keys: one warp a row.  Any strides; rows of
-// contiguous keys are read by words from the 4-byte boundary at or below each eight's first entry, every word holding one.
+// A mask whose rows lie on 16-byte boundaries: one warp a row.  Any strides; rows of contiguous keys are read by words from the 4-byte
+// boundary at or below each eight's first entry, every word holding one.  What is behind a row's last key in its last eight is what
+// the last word had there or zero; the tensor map's extent ends before it.
 __global__ void __launch_bounds__(256)
 mask_rows_kernel(const __half* __restrict__ mask, uint4* __restrict__ out, int Lq, int Lk, int64_t rows, int planesH, int64_t bsK,
                  int64_t bsQ, int64_t bsH, int64_t bsB) {

@@ -395,8 +395,10 @@ template <typename F> static auto af_dispatch(int64_t E, int64_t Lq, bool masked
 // 32 queries, 16 to 8192 keys): the large kernel takes as long for 128 keys as this one for 64, but sets up tensor memory
 // and merges.  16 to 32 queries over up to 384 keys are its (20 heads, 32 x 128: 4.4 us there, 7.2 here; 32 x 256 5.7, 6.7),
 // and many heads over long keys with more than 16 queries (36 heads, 32 x 8192: 31, 36); up to 8 queries are nearly always
-// this one's (8 heads, 1 x 1000: 9.5, 5.0).  Over 4154 further shapes the choice leaves three more than 4 % behind the large
-// kernel, where taking every call here left 350, by up to three quarters.
+// this one's (8 heads, 1 x 1000: 9.5, 5.0).  The large kernel's constants, and that it cuts whatever leaves SMs idle into parts of two
+// blocks or more, are of its form before whole warps issued and a cut was weighed; against the present one the choice is 0.4 % off the
+// faster in the mean over 420 shapes (always here 5 %, always there 25 %), 26 of them more than 4 %, up to 1.3 times for a
+// few queries' long masks (4 x 4, 3 x 6849 x 128: 35.3 us, 27.4 there).
 bool attention_few_takes(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64_t H, int64_t B, bool masked) {
     if (Lq > (E <= 64 ? 32 : 16)) return false;
     if (af_forced()) return true;
@@ -410,7 +412,7 @@ bool attention_few_takes(b200_ctx* ctx, int64_t E, int64_t Lq, int64_t Lk, int64
     const Large& m = large[E > 64][masked];
     double there = m.wave * (double)cdiv(items, sms) + m.block * (double)(blocks * cdiv(items, sms));
     const int64_t rem = items % sms, cut = 2 * items <= sms ? items : (items > sms && rem > 0 && 2 * rem <= sms ? rem : 0);
-    if (blocks >= 4 && cut > 0) {   // the keys of `cut` items over ns CTAs each, as the large kernel's launch does
+    if (blocks >= 4 && cut > 0) {   // the keys of `cut` items over ns CTAs each
         int64_t ns = sms / cut;
         if (ns > blocks / 2) ns = blocks / 2;
         if (ns > 64) ns = 64;
